@@ -48,6 +48,9 @@ SIGNATURES = {
     "cf_infinite_attn_fwd_sorted": [P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, F64, F64, P, F64, I32,
                                     I32, P, P, P, P],
     "cf_serve_submit": [P, P, P, P, P, P, I64, I64, I64, I64, I32, P, P],
+    "cf_dense_image_bytes": [I64],
+    "cf_dense_pack_layer": [P, P, P, P, P, P, I64, P, P],
+    "cf_dense_pack_embedding": [P, I64, P, P],
     "cf_row_cost": [P, P, I64, I64, F64, P, P],
     "cf_row_order": [P, P, I64, I64, F64, P, P],
     "cf_reci_phase": [P, P, P, P, I64, P, P],
@@ -134,6 +137,7 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
+        lib.cf_dense_image_bytes.restype = c_int64
         _lib = lib
     return _lib
 

@@ -1,0 +1,433 @@
+// The dense part of an encoder layer boundary in ONE kernel, forward:
+//
+//     tail of layer l      y  = x + attn Wo^T + bo
+//                          x' = y + relu(y W1^T + b1) W2^T + b2            (hidden units in chunks of 128)
+//     head of layer l+1    q|k|v = x' Wqkv^T + bqkv ;  a = width(q . w_pos) ;  q <- q / sqrt(16)
+//
+// (models/indexed_latticeformer_encoder.py:848-890 without LayerNorm, and the in-projection and Gaussian-width
+// pipeline of models/indexed_lattice_multi_head_attention_cuda.py:582-722.)  See dense_tc_core.cuh for the organisation
+// of a block and the arithmetic.  The chain of a tile alternates products and epilogues; the two products of
+// consecutive feed-forward chunks are kept in flight against each other's epilogues (accumulators D0 / D1 for the hidden
+// units, DX for the output), so the tensor pipe only waits at y, at x' and at the end of a tile.
+#include "dense_tc_core.cuh"
+
+__device__ unsigned g_dense_forward_status;  // set by a block whose waits ran out (never in a working build)
+
+namespace cf {
+namespace {
+using namespace tc5;
+
+__global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const DenseForward p)
+{
+    extern __shared__ __align__(1024) unsigned char smem_tc[];
+    uint32_t tmem;
+    const Shared s = block_begin(smem_tc, tmem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long tiles = (p.N + 127) / 128;
+    const int chunks = p.ff / 128;
+    const bool tail = p.tail != nullptr, embed = p.embed != nullptr, head = p.head != nullptr;
+    grid_launch_dependents();
+
+    if (warp == STREAM_WARP) {
+        if (p.weights_fresh) grid_dependency_wait();
+        if (lane == 0) {
+            Producer pr;
+            for (long long tile = blockIdx.x; tile < tiles && pr.ok; tile += gridDim.x) {
+                if (tail) pr.stream(s, p.tail, 0, 1 + 2 * chunks);
+                else if (embed) pr.stream(s, p.embed, 0, 1);
+                if (head) pr.stream(s, p.head, 1 + 2 * chunks, 3);
+            }
+            if (!pr.ok) pr.drain(s);
+        }
+        grid_dependency_wait();
+    } else if (warp == ISSUE_WARP) {
+        grid_dependency_wait();
+        if (lane == 0) {
+            Issuer is;
+            Phase ph;
+            for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
+                bool ok = true;
+                auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
+                auto product = [&](int d, int a, bool acc, int done) {
+                    if (ok) is.product(s, tmem, d, a, acc);
+                    ok = ok && is.ok;
+                    mma_commit(s.bar(done));
+                };
+                if (tail || embed) {
+                    ready(B_A0);
+                    product(D0, OFF_A0, false, B_D0);
+                }
+                if (tail) {
+                    ready(B_A0);
+                    product(D0, OFF_A0, false, B_D0);
+                    if (chunks > 1) product(D1, OFF_A0, false, B_D1);
+                    for (int c = 0; c < chunks && ok; ++c) {
+                        ready(B_A1);
+                        product(DX, OFF_A1, c > 0, B_A1_FREE);
+                        if (c + 1 == chunks) mma_commit(s.bar(B_DX));
+                        if (c + 2 < chunks) product((c & 1) ? D1 : D0, OFF_A0, false, (c & 1) ? B_D1 : B_D0);
+                    }
+                }
+                if (head) {
+                    ready(B_A0);
+                    product(D0, OFF_A0, false, B_D0);
+                    product(D1, OFF_A0, false, B_D1);
+                    product(DX, OFF_A0, false, B_DX);
+                }
+                is.ok = is.ok && ok;
+            }
+            if (!is.ok) is.drain(s);
+        }
+    } else {
+        const Place pl;
+        unsigned char *A0 = s.mem + OFF_A0, *A1 = s.mem + OFF_A1;
+        const float *tail_inv = reinterpret_cast<const float *>(p.tail), *head_inv = reinterpret_cast<const float *>(p.head);
+        if (p.weights_fresh) grid_dependency_wait();
+        // constants of the weights: 1 / s of each matrix, and a bound of the hidden units' biases
+        float wo_i = 0.f, w1_i = 0.f, w2_i = 0.f, wh_i = 0.f, we_i = 0.f, b1_max = 0.f;
+        if (tail) {
+            wo_i = tail_inv[0]; w1_i = tail_inv[1]; w2_i = tail_inv[2 * chunks];
+            for (int i = threadIdx.x; i < p.ff; i += EPI_THREADS) b1_max = fmaxf(b1_max, fabsf(p.b1[i]));
+            b1_max = warp_max(b1_max);
+            if (lane == 0) s.warp_floats()[warp] = b1_max;
+            epilogue_sync();
+#pragma unroll
+            for (int w = 0; w < EPI_WARPS; ++w) b1_max = fmaxf(b1_max, s.warp_floats()[w]);
+        }
+        if (embed) we_i = *reinterpret_cast<const float *>(p.embed);
+        if (head) wh_i = head_inv[1 + 2 * chunks];
+        grid_dependency_wait();
+        Phase ph;
+        for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            const long long row_base = tile * 128;
+            epilogue_sync();  // the previous tile's readers are done with the per-row scales
+            float x[2][16];   // the thread's 32 features: x, then y, then x'
+            float xi[4];      // 1 / scale of its four rows in the current operand
+            // largest magnitude of the rows -> scales, then operand 0
+            auto publish = [&]() {
+                float m[4] = {0.f, 0.f, 0.f, 0.f}, xs[4];
+#pragma unroll
+                for (int half = 0; half < 2; ++half)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) m[2 * half + ((i >> 1) & 1)] = fmaxf(m[2 * half + ((i >> 1) & 1)], fabsf(x[half][i]));
+                row_maxima(s, pl, m);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xs[i] = power_of_two(m[i], xi[i]);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) store_operand(A0, pl, half, x[half], xs[2 * half], xs[2 * half + 1]);
+                fence_async_smem();
+                fence_before();
+                mbar_arrive(s.bar(B_A0));
+            };
+            if (tail || embed) {
+                if (tail) {
+                    load_operand(s, A0, [&](int row, int ln) {
+                        return row_base + row < p.N ? *reinterpret_cast<const float4 *>(p.attn + (row_base + row) * 128 + 4 * ln)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                    });
+                } else {
+                    load_operand(s, A0, [&](int row, int ln) {
+                        float e[4] = {0.f, 0.f, 0.f, 0.f};
+                        if (row_base + row < p.N) {
+                            if (p.features != nullptr) {
+                                const float *f = p.features + (row_base + row) * p.feature_dim;
+#pragma unroll
+                                for (int u = 0; u < 4; ++u)
+                                    if (4 * ln + u < p.feature_dim) e[u] = f[4 * ln + u];
+                            } else {
+                                const long long z = p.species[row_base + row] - 4 * ln;
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) e[u] = z == u ? 1.0f : 0.0f;
+                            }
+                        }
+                        return make_float4(e[0], e[1], e[2], e[3]);
+                    });
+                }
+                fence_async_smem();
+                fence_before();
+                mbar_arrive(s.bar(B_A0));
+                if (tail) {  // the residual and its bias arrive during the product
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float2 b = *reinterpret_cast<const float2 *>(p.bo + pl.col0 + 8 * j);
+                            x[half][4 * j] += b.x; x[half][4 * j + 1] += b.y; x[half][4 * j + 2] += b.x; x[half][4 * j + 3] += b.y;
+                        }
+                    }
+                }
+                epilogue_sync();  // (the loading warps' scales)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
+                ph.wait(s, B_D0);
+                fence_after();
+                const float wi = tail ? wo_i : we_i;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float d[16];
+                    tmem_load_16x32(pl.tmem(tmem, D0, half), d);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const float sc = xi[2 * half + ((i >> 1) & 1)] * wi;
+                        x[half][i] = tail ? fmaf(d[i], sc, x[half][i]) : d[i] * sc;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+            }
+            if (tail) {
+                publish();  // y
+                if (p.y_save != nullptr) {
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) store_rows(p.y_save, 128, row_base, p.N, pl, half, x[half]);
+                }
+                // The hidden units of all chunks share one scale per row (their products with W2 meet in one accumulator),
+                // from a bound known beforehand: |h| <= 128 max|y| max|W1| + max|b1|, with both operands below 2^15 in
+                // their scaled form.  A bound some 2^8 above the largest unit still leaves 2^-31 of it as resolution.
+                float hs[4], hi[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) hs[i] = power_of_two(fmaf(137438953472.0f * xi[i], w1_i, b1_max), hi[i]);
+                for (int c = 0; c < chunks; ++c) {
+                    const int d_col = (c & 1) ? D1 : D0;
+                    float2 bias[4];
+                    load_columns(p.b1 + 128 * c, pl, bias);
+                    ph.wait(s, (c & 1) ? B_D1 : B_D0);
+                    fence_after();
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        float h[16];
+                        tmem_load_16x32(pl.tmem(tmem, d_col, half), h);
+                        const float sa = xi[2 * half] * w1_i, sb = xi[2 * half + 1] * w1_i;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float2 b = bias[j];
+                            h[4 * j] = fmaxf(fmaf(h[4 * j], sa, b.x), 0.f);
+                            h[4 * j + 1] = fmaxf(fmaf(h[4 * j + 1], sa, b.y), 0.f);
+                            h[4 * j + 2] = fmaxf(fmaf(h[4 * j + 2], sb, b.x), 0.f);
+                            h[4 * j + 3] = fmaxf(fmaf(h[4 * j + 3], sb, b.y), 0.f);
+                        }
+                        if (half == 0 && c > 0) ph.wait(s, B_A1_FREE);  // the previous chunk has been multiplied
+                        store_operand(A1, pl, half, h, hs[2 * half], hs[2 * half + 1]);
+                        if (p.h_save != nullptr) store_rows(p.h_save + 128 * c, p.ff, row_base, p.N, pl, half, h);
+                    }
+                    fence_async_smem();
+                    fence_before();
+                    mbar_arrive(s.bar(B_A1));
+                }
+                float2 bias[4];
+                load_columns(p.b2, pl, bias);
+                ph.wait(s, B_A1_FREE);
+                ph.wait(s, B_DX);
+                fence_after();
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float d[16];
+                    tmem_load_16x32(pl.tmem(tmem, DX, half), d);
+                    const float sa = hi[2 * half] * w2_i, sb = hi[2 * half + 1] * w2_i;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 b = bias[j];
+                        x[half][4 * j] += fmaf(d[4 * j], sa, b.x);
+                        x[half][4 * j + 1] += fmaf(d[4 * j + 1], sa, b.y);
+                        x[half][4 * j + 2] += fmaf(d[4 * j + 2], sb, b.x);
+                        x[half][4 * j + 3] += fmaf(d[4 * j + 3], sb, b.y);
+                    }
+                }
+            }
+            if (head) publish();
+            if (tail || embed) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
+            }
+            if (!head) continue;
+#pragma unroll
+            for (int which = 0; which < 3; ++which) {
+                float2 bias[4];
+                load_columns(p.bqkv + 128 * which, pl, bias);
+                ph.wait(s, which == 0 ? B_D0 : which == 1 ? B_D1 : B_DX);
+                fence_after();
+                float *dst = which == 0 ? p.q : which == 1 ? p.k : p.v;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float d[16];
+                    tmem_load_16x32(pl.tmem(tmem, which == 0 ? D0 : which == 1 ? D1 : DX, half), d);
+                    const float sa = xi[2 * half] * wh_i, sb = xi[2 * half + 1] * wh_i;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 b = bias[j];
+                        d[4 * j] = fmaf(d[4 * j], sa, b.x); d[4 * j + 1] = fmaf(d[4 * j + 1], sa, b.y);
+                        d[4 * j + 2] = fmaf(d[4 * j + 2], sb, b.x); d[4 * j + 3] = fmaf(d[4 * j + 3], sb, b.y);
+                    }
+                    if (which == 0) {
+                        // the heads' Gaussian widths from alpha = q . w_pos (…attention_cuda.py:647-722), then q / sqrt(16)
+#pragma unroll
+                        for (int hh = 0; hh < 2; ++hh) {
+                            float al[2] = {0.f, 0.f};
+#pragma unroll
+                            for (int jj = 0; jj < 2; ++jj) {
+                                const int j = 2 * hh + jj;
+                                const float2 w = *reinterpret_cast<const float2 *>(p.w_pos + pl.col0 + 8 * j);
+                                al[0] = fmaf(d[4 * j + 1], w.y, fmaf(d[4 * j], w.x, al[0]));
+                                al[1] = fmaf(d[4 * j + 3], w.y, fmaf(d[4 * j + 2], w.x, al[1]));
+                            }
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                al[e] += __shfl_xor_sync(FULL, al[e], 1);
+                                al[e] += __shfl_xor_sync(FULL, al[e], 2);
+                                const long long row = row_base + pl.row0 + 16 * half + 8 * e;
+                                if (pl.t == 0 && row < p.N) {
+                                    const float tt = (al[e] + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - p.lower_bound));
+                                    const float elu = tt > 0.f ? tt : expm1f(tt);
+                                    p.a[row * HEADS + 2 * pl.group + hh] = ((1.0f - p.lower_bound) * elu + 1.0f) * p.a_factor;
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) d[i] *= 0.25f;
+                    }
+                    store_rows(dst, 128, row_base, p.N, pl, half, d);
+                }
+            }
+        }
+    }
+    block_end(s, tmem, &g_dense_forward_status);
+}
+
+// ---- packing -------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) dense_pack_kernel(const PackJob job)
+{
+    const PackBlock &b = job.b[blockIdx.x];
+    __shared__ float warp_m[8];
+    const int tid = threadIdx.x;
+    float m = 0.f;
+#pragma unroll
+    for (int gi = 0; gi < 3; ++gi)
+        if (b.group[gi] != nullptr)
+            for (int i = tid; i < b.group_elems; i += 256) m = fmaxf(m, fabsf(b.group[gi][i]));
+    m = warp_max(m);
+    if ((tid & 31) == 0) warp_m[tid >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, warp_m[w]);
+    float inv;
+    const float sc = power_of_two(m, inv);
+    if (tid == 0) reinterpret_cast<float *>(b.image)[b.block] = inv;
+    unsigned char *out = b.image + TC_HEADER_BYTES + (size_t)b.block * TC_BLOCK_BYTES;
+    for (int idx = tid; idx < 128 * 16; idx += 256) {
+        const int n = idx & 127, k0 = (idx >> 7) * 8;  // a 16-byte chunk: eight k of output row n
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = k0 + u;
+            v[u] = (n < b.rows && k < b.cols) ? (b.trans ? b.src[(size_t)k * b.ld + n] : b.src[(size_t)n * b.ld + k]) * sc : 0.f;
+        }
+        uint4 h0, h1;
+        split_pair(v[0], v[1], h0.x, h1.x);
+        split_pair(v[2], v[3], h0.y, h1.y);
+        split_pair(v[4], v[5], h0.z, h1.z);
+        split_pair(v[6], v[7], h0.w, h1.w);
+        unsigned char *at = out + (k0 >> 6) * STAGE_BYTES + n * 128 + ((((k0 & 63) >> 3) ^ (n & 7)) << 4);
+        *reinterpret_cast<uint4 *>(at) = h0;
+        *reinterpret_cast<uint4 *>(at + 16384) = h1;
+    }
+}
+
+}  // namespace
+
+int launch_dense_forward(const DenseForward &p, cudaStream_t s)
+{
+    if (p.N == 0) return CF_OK;
+    if (p.ff <= 0 || p.ff % 128 != 0 || p.ff > TC_MAX_FF)
+        return fail(CF_ERR_UNSUPPORTED, "dense forward: ff_dim=%d must be a multiple of 128 up to %d", p.ff, TC_MAX_FF);
+    static thread_local bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!configured[dev & 63]) {
+        if (cudaFuncSetAttribute(dense_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc5::SMEM_BYTES) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(CF_ERR_CUDA, "dense forward: %d bytes of shared memory not available", tc5::SMEM_BYTES);
+        }
+        configured[dev & 63] = true;
+    }
+    const long long tiles = (p.N + 127) / 128, cap = sm_count();
+    launch_chained(dense_forward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
+                   p.chained, p);
+    return launch_status("dense_forward_kernel");
+}
+
+int launch_pack(const PackJob &job, int count, cudaStream_t s)
+{
+    if (count == 0) return CF_OK;
+    dense_pack_kernel<<<count, 256, 0, s>>>(job);
+    return launch_status("dense_pack_kernel");
+}
+
+static PackBlock &pack_add(PackJob &job, int &count, unsigned char *image, int block, const float *src, int ld, int trans)
+{
+    PackBlock &b = job.b[count++];
+    b = PackBlock{};
+    b.src = src; b.ld = ld; b.trans = (short)trans; b.rows = 128; b.cols = 128; b.block = (short)block; b.image = image;
+    return b;
+}
+
+void pack_layer_forward(PackJob &job, int &count, unsigned char *image, int ff, const float *Wq, const float *Wk, const float *Wv,
+                        const float *Wo, const float *W1, const float *W2)
+{
+    const int chunks = ff / 128;
+    int at = 0;
+    auto one = [&](const float *src, int ld, const float *g0, const float *g1, const float *g2, int elems) {
+        PackBlock &b = pack_add(job, count, image, at++, src, ld, 0);
+        b.group[0] = g0; b.group[1] = g1; b.group[2] = g2; b.group_elems = elems;
+    };
+    auto w1 = [&](int c) { one(W1 + (size_t)c * 128 * 128, 128, W1, nullptr, nullptr, ff * 128); };
+    one(Wo, 128, Wo, nullptr, nullptr, 128 * 128);
+    w1(0);
+    if (chunks > 1) w1(1);
+    for (int c = 0; c < chunks; ++c) {
+        one(W2 + (size_t)c * 128, ff, W2, nullptr, nullptr, ff * 128);
+        if (c + 2 < chunks) w1(c + 2);
+    }
+    one(Wq, 128, Wq, Wk, Wv, 128 * 128);
+    one(Wk, 128, Wq, Wk, Wv, 128 * 128);
+    one(Wv, 128, Wq, Wk, Wv, 128 * 128);
+}
+
+void pack_embedding(PackJob &job, int &count, unsigned char *image, const float *W, int feature_dim)
+{
+    PackBlock &b = pack_add(job, count, image, 0, W, feature_dim, 0);
+    b.cols = (short)feature_dim;
+    b.group[0] = W;
+    b.group_elems = 128 * feature_dim;
+}
+
+}  // namespace cf
+
+extern "C" int64_t cf_dense_image_bytes(int64_t ff_dim) { return (int64_t)cf::tc_image_bytes(ff_dim > 0 ? cf::tc_layer_blocks((int)ff_dim) : 1); }
+
+extern "C" int cf_dense_pack_layer(const float *Wq, const float *Wk, const float *Wv, const float *Wo, const float *W1,
+                                   const float *W2, int64_t ff_dim, void *image, void *stream)
+{
+    using namespace cf;
+    CF_REQUIRE(Wq && Wk && Wv && Wo && W1 && W2 && image, CF_ERR_INVALID, "cf_dense_pack_layer: null pointer");
+    CF_REQUIRE(ff_dim > 0 && ff_dim % 128 == 0 && ff_dim <= TC_MAX_FF, CF_ERR_UNSUPPORTED,
+               "cf_dense_pack_layer: ff_dim=%lld must be a multiple of 128 up to %d", (long long)ff_dim, TC_MAX_FF);
+    CF_REQUIRE((reinterpret_cast<uintptr_t>(image) & 15) == 0, CF_ERR_INVALID, "cf_dense_pack_layer: image must be 16-byte aligned");
+    PackJob job;
+    int count = 0;
+    pack_layer_forward(job, count, static_cast<unsigned char *>(image), (int)ff_dim, Wq, Wk, Wv, Wo, W1, W2);
+    return launch_pack(job, count, as_stream(stream));
+}
+
+extern "C" int cf_dense_pack_embedding(const float *W, int64_t feature_dim, void *image, void *stream)
+{
+    using namespace cf;
+    CF_REQUIRE(W && image, CF_ERR_INVALID, "cf_dense_pack_embedding: null pointer");
+    CF_REQUIRE(feature_dim >= 1 && feature_dim <= 128, CF_ERR_UNSUPPORTED, "cf_dense_pack_embedding: %lld features (1..128)", (long long)feature_dim);
+    CF_REQUIRE((reinterpret_cast<uintptr_t>(image) & 15) == 0, CF_ERR_INVALID, "cf_dense_pack_embedding: image must be 16-byte aligned");
+    PackJob job;
+    int count = 0;
+    pack_embedding(job, count, static_cast<unsigned char *>(image), W, (int)feature_dim);
+    return launch_pack(job, count, as_stream(stream));
+}

@@ -1,0 +1,74 @@
+// Dense products of an encoder layer boundary on the fifth-generation tensor cores (dense_tc.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include "common.cuh"
+
+namespace cf {
+
+// Weight images.  A layer's projections are cut into 128 x 128 blocks; a block is 64 KB, the shared-memory image that
+// the tensor instruction reads: two 64-deep k panels, each { h0, h1 } of 128 rows x 128 bytes with the 128-byte swizzle
+// (tc5.cuh), so that a stage of the weight stream is one contiguous 32 KB copy.  Blocks are stored in the order in
+// which the kernel consumes them; in front of them 1 KB of scales (float, 1 / s of every block).
+constexpr int TC_BLOCK_BYTES = 65536;
+constexpr int TC_HEADER_BYTES = 1024;
+inline size_t tc_image_bytes(int blocks) { return (size_t)TC_HEADER_BYTES + (size_t)blocks * TC_BLOCK_BYTES; }
+inline int tc_tail_blocks(int ff) { return 1 + 2 * (ff / 128); }  // Wo, then W1 / W2 chunks interleaved
+inline int tc_layer_blocks(int ff) { return tc_tail_blocks(ff) + 3; }
+
+// One block to pack: element (n, k) is src[n ld + k] (or src[k ld + n] with trans), zero outside rows x cols; the scale
+// is that of the largest magnitude among `group` arrays of group_elems values each.
+struct PackBlock {
+    const float *src, *group[3];
+    int group_elems, ld;
+    short rows, cols, trans, block;   // block: index in the image
+    unsigned char *image;
+};
+constexpr int PACK_MAX = 56;                          // blocks of one launch (the job is a kernel parameter)
+constexpr int TC_MAX_FF = 128 * ((PACK_MAX - 4) / 2);  // a layer is packed by one launch
+struct PackJob {
+    PackBlock b[PACK_MAX];
+};
+int launch_pack(const PackJob &job, int count, cudaStream_t s);
+// The blocks of one layer, forward order: [Wo, W1_0, W1_1, W2_0, W1_2, W2_1, ..., Wq, Wk, Wv].  Appends to job.
+void pack_layer_forward(PackJob &job, int &count, unsigned char *image, int ff, const float *Wq, const float *Wk, const float *Wv,
+                        const float *Wo, const float *W1, const float *W2);
+void pack_embedding(PackJob &job, int &count, unsigned char *image, const float *W, int feature_dim);
+
+struct DenseForward {
+    long long N;
+    int ff;
+    bool chained, weights_fresh;    // weights_fresh: the images were written earlier on this stream by a kernel that may still run
+    // tail of the layer whose attention just ran (image null: none)
+    const unsigned char *tail;
+    const float *attn, *bo, *b1, *b2;
+    // embedding (only without a tail): x = features W^T
+    const unsigned char *embed;
+    const float *features;
+    const int64_t *species;
+    int feature_dim;
+    // head of the next layer (image null: none)
+    const unsigned char *head;
+    const float *bqkv, *w_pos;
+    float gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound;
+    // activations
+    const float *x_in;   // (N,128) features the tail's residual (or, without tail and embedding, the head) reads
+    float *x_out;        // (N,128) features after the tail / embedding
+    float *q, *k, *v, *a;
+    float *y_save, *h_save;  // training: y (N,128) and the hidden units (N, ff), or null
+};
+
+// The packed-weight pointers of the one-call forwards (slot 10 of a layer, W_embed_packed) carry bit 0 set when they name
+// such an image rather than fragments for the warp-level dense block (dense_block.cu).
+inline bool is_tc_image(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 1) != 0; }
+inline const unsigned char *tc_image(const void *p) { return reinterpret_cast<const unsigned char *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)1); }
+inline bool dense_tc_images(int num_layers, const float *const *weights)
+{
+    bool all = num_layers > 0;
+    for (int l = 0; l < num_layers; ++l) all = all && is_tc_image(weights[11 * l + 10]);
+    return all;
+}
+
+int launch_dense_forward(const DenseForward &p, cudaStream_t s);
+
+}  // namespace cf

@@ -19,6 +19,7 @@
 #include "blas_dyn.cuh"
 #include "common.cuh"
 #include "dense_block.cuh"
+#include "dense_tc.cuh"
 #include "row_list.cuh"
 #include "term_list.cuh"
 
@@ -196,6 +197,8 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     const bool fused = dense_path_available(num_layers, weights, ff_dim);  // one launch per layer boundary, no cuBLAS
     CF_REQUIRE(fused || embed == nullptr, CF_ERR_INVALID, "cf_encoder_forward: embedding stage without the dense path");
     CF_REQUIRE(fused || cublas_handle, CF_ERR_INVALID, "cf_encoder_forward: null cuBLAS handle");
+    CF_REQUIRE(embed == nullptr || is_tc_image(embed->packed) == dense_tc_images(num_layers, weights), CF_ERR_INVALID,
+               "cf_encoder_forward: embedding and layers packed in different ways");
     cudaStream_t s = as_stream(stream);
 
     float *qkv = workspace;
@@ -271,6 +274,37 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     // Fused dense path: every layer brings its weights packed for the tensor-core kernel (slot 10) and the
     // feed-forward width is a multiple of 128.  One launch per layer boundary instead of four GEMMs and two
     // element-wise passes; see dense_block.cu.
+    if (fused && dense_tc_images(num_layers, weights)) {
+        // the weights as images for the block-level tensor instructions (dense_tc.cu)
+        auto boundary = [&](int l) {  // the kernel before layer l's attention (tail of layer l - 1, head of layer l)
+            DenseForward d{};
+            d.N = N; d.ff = ff; d.chained = l > 0; d.x_in = d.x_out = x; d.q = q; d.k = k; d.v = v; d.a = a;
+            if (l > 0) {
+                const float *const *w = weights + 11 * (l - 1);
+                d.tail = tc_image(w[10]); d.attn = attn; d.bo = w[5]; d.b1 = w[7]; d.b2 = w[9];
+            } else if (embed != nullptr) {
+                d.embed = tc_image(embed->packed); d.features = embed->features; d.species = embed->species; d.feature_dim = embed->feature_dim;
+            }
+            if (l < num_layers) {
+                const float *const *w = weights + 11 * l;
+                const double *sc = scalars + 6 * l;
+                d.head = tc_image(w[10]); d.bqkv = w[1]; d.w_pos = w[2];
+                d.gauss_scale = (float)sc[0]; d.gauss_shift = (float)sc[1]; d.a_factor = (float)sc[2];
+                d.elu_beta = (float)sc[3]; d.lower_bound = (float)sc[4];
+            }
+            return launch_dense_forward(d, s);
+        };
+        rc = boundary(0);
+        if (forked) cudaStreamWaitEvent(s, side_stream().join, 0);
+        for (int l = 0; l < num_layers && rc == CF_OK; ++l) {
+            if (attn_events) cudaEventRecord(reinterpret_cast<cudaEvent_t>(attn_events[2 * l]), s);
+            rc = attention(l, scalars[6 * l + 5], weights[11 * l + 3], attn, lse);
+            if (attn_events) cudaEventRecord(reinterpret_cast<cudaEvent_t>(attn_events[2 * l + 1]), s);
+            if (rc == CF_OK) rc = boundary(l + 1);
+        }
+        if (rc != CF_OK) return rc;
+        return launch_status("cf_encoder_forward");
+    }
     if (fused) {
         auto head_of = [&](DenseArgs &d, int l) {
             const float *const *w = weights + 11 * l;

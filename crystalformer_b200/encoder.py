@@ -60,6 +60,33 @@ def pack_dense_weight(W: Tensor) -> Tensor:
     return torch.cat((frag(hi), frag(corr)), dim=-1).contiguous().reshape(-1)
 
 
+MAX_IMAGE_FF = 3328  # widest feed-forward of a layer image (cf_dense_pack_layer)
+
+
+def pack_dense_layer(wqkv: Tensor, wo: Tensor, w1: Tensor, w2: Tensor) -> Tensor:
+    """The image of a layer's projections that the dense kernel streams (cf_dense_pack_layer), as a byte tensor."""
+    lib = _lib.load()
+    ff = w1.shape[0]
+    image = torch.empty(int(lib.cf_dense_image_bytes(ff)), dtype=torch.uint8, device=wqkv.device)
+    with torch.cuda.device(wqkv.device):
+        _lib.call("cf_dense_pack_layer", *(wqkv[128 * i:].data_ptr() for i in range(3)), wo.data_ptr(), w1.data_ptr(), w2.data_ptr(),
+                  ff, image.data_ptr(), torch.cuda.current_stream(wqkv.device).cuda_stream)
+    return image
+
+
+def pack_dense_embedding(W: Tensor) -> Tensor:
+    """The image of the embedding weight (128, features <= 128), see ``pack_dense_layer``."""
+    image = torch.empty(int(_lib.load().cf_dense_image_bytes(0)), dtype=torch.uint8, device=W.device)
+    with torch.cuda.device(W.device):
+        _lib.call("cf_dense_pack_embedding", W.data_ptr(), W.shape[1], image.data_ptr(), torch.cuda.current_stream(W.device).cuda_stream)
+    return image
+
+
+def image_pointer(image: Optional[Tensor]) -> int:
+    """The address handed to the one-call forwards: bit 0 marks an image (as opposed to ``pack_dense_weight`` fragments)."""
+    return 0 if image is None else image.data_ptr() | int(image.dtype == torch.uint8)
+
+
 class BatchGeometry:
     """Everything the attention layers need besides the atom features, computed once per batch on the device."""
 
@@ -207,12 +234,15 @@ class CrystalformerEncoderCUDA(Module):
                        att.headed_pe_proj(), att.out_proj.weight, att.out_proj.bias,
                        layer.linear1.weight, layer.linear1.bias, layer.linear2.weight, layer.linear2.bias, None]
             tensors = [None if t is None else t.detach().float().contiguous() for t in tensors]
-            if self.dense_fused and layer.linear1.weight.shape[0] % 128 == 0:
-                # slot 10: in-projection, out-projection and feed-forward weights packed for the fused dense kernel
-                tensors[10] = torch.cat([pack_dense_weight(m) for m in
-                                         (wqkv, att.out_proj.weight, layer.linear1.weight, layer.linear2.weight)])
+            ff = layer.linear1.weight.shape[0]
+            if self.dense_fused and ff % 128 == 0:
+                # slot 10: in-projection, out-projection and feed-forward weights packed for the fused dense kernels
+                if ff <= MAX_IMAGE_FF:
+                    tensors[10] = pack_dense_layer(wqkv, tensors[4], tensors[6], tensors[8])
+                else:
+                    tensors[10] = torch.cat([pack_dense_weight(m) for m in (wqkv, tensors[4], tensors[6], tensors[8])])
             keep.append(tensors)
-            ptrs += [0 if t is None else t.data_ptr() for t in tensors]
+            ptrs += [0 if t is None else t.data_ptr() for t in tensors[:10]] + [image_pointer(tensors[10])]
             beta = float(P.positive_func.split("=")[1]) if "=" in P.positive_func else 1.0
             dist_max = P.value_pe_dist_max
             if dist_max < 0:

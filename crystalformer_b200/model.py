@@ -15,7 +15,7 @@ import torch.nn as nn
 
 from . import _lib
 from .cuda_funcs import IrregularMeanCUDA
-from .encoder import BatchGeometry, CrystalformerEncoderCUDA, pack_dense_weight
+from .encoder import MAX_IMAGE_FF, BatchGeometry, CrystalformerEncoderCUDA, image_pointer, pack_dense_embedding, pack_dense_weight
 from .params import DEFAULT_MODEL_PARAMS, LatticeformerParams
 
 
@@ -120,18 +120,20 @@ class Latticeformer(nn.Module):
         return self.input_embeddings.out_features == 128 and self.encoder.native and self.encoder._native_ok()
 
     def _embedding_packed(self, device) -> Optional[torch.Tensor]:
-        """The embedding weight, input columns zero-padded to 128, in the fragment order of the fused dense kernel
-        (which then computes the embedding inside the encoder's first launch); None when that kernel is not in use.
-        Rebuilt only when the weight changed."""
+        """The embedding weight, packed like the layers' projections (the fused dense kernel then computes the embedding
+        inside the encoder's first launch); None when that kernel is not in use.  Rebuilt only when the weight changed."""
         W = self.input_embeddings.weight
         if not self.encoder.dense_fused or W.shape[1] > 128:
             return None
         key = (device, W._version, W.data_ptr())
         cache = getattr(self, "_embed_cache", None)
         if cache is None or cache[0] != key:
-            padded = torch.zeros((128, 128), dtype=torch.float32, device=device)
-            padded[:, :W.shape[1]] = W.detach().float()
-            self._embed_cache = cache = (key, pack_dense_weight(padded))
+            if self.encoder.layers[0].linear1.weight.shape[0] <= MAX_IMAGE_FF:
+                self._embed_cache = cache = (key, pack_dense_embedding(W.detach().float().contiguous()))
+            else:
+                padded = torch.zeros((128, 128), dtype=torch.float32, device=device)
+                padded[:, :W.shape[1]] = W.detach().float()
+                self._embed_cache = cache = (key, pack_dense_weight(padded))
         return cache[1]
 
     def native_plan(self, device) -> dict:
@@ -152,7 +154,7 @@ class Latticeformer(nn.Module):
         plan["hidden"], plan["targets"] = plan["w1"].shape[0], plan["w2"].shape[0]
         if plan["emb_packed"] is not None:  # the description of the model for cf_serve_submit
             plan["desc"] = _lib.ModelDesc(
-                feature_dim=plan["emb"].shape[1], W_embed=plan["emb"].data_ptr(), W_embed_packed=plan["emb_packed"].data_ptr(),
+                feature_dim=plan["emb"].shape[1], W_embed=plan["emb"].data_ptr(), W_embed_packed=image_pointer(plan["emb_packed"]),
                 num_layers=len(enc.layers), lattice_range=int(P.lattice_range),
                 minimum_range=int(P.lattice_range) if P.minimum_range else 0, dense_tile_rows=0,
                 weights=ctypes.cast(w["ptrs"], ctypes.c_void_p), scalars=ctypes.cast(w["scalars"], ctypes.c_void_p),
@@ -211,7 +213,7 @@ class Latticeformer(nn.Module):
                 stream.wait_event(slot[1])  # (a no-op in effect unless the workspace was last used on another stream)
             _lib.call("cf_model_forward", ctypes.c_void_p(torch.cuda.current_blas_handle()),
                       feats.data_ptr(), feats.shape[1], pos.data_ptr(), trans.data_ptr(), sizes.data_ptr(), n_atoms, B,
-                      n_edges, max_atoms, plan["emb"].data_ptr(), None if emb_packed is None else emb_packed.data_ptr(),
+                      n_edges, max_atoms, plan["emb"].data_ptr(), image_pointer(emb_packed) or None,
                       *plan["tail"], work.data_ptr(), y.data_ptr(), self.encoder._attention_events(),
                       None if desc is None else ctypes.byref(desc),
                       None if slot is None else ctypes.c_void_p(inputs_ready.cuda_event),

@@ -323,6 +323,8 @@ int cf_infinite_attn_fwd_sorted(const float *q, const float *k, const float *v, 
  *             bfloat16(hi(w)), upper half: bfloat16(w - hi(w)) }.  When every layer has it and ff_dim is a multiple
  *             of 128, the four products and the element-wise steps of a layer boundary run as ONE tensor-core kernel
  *             (TF32 main product + bfloat16 correction product: fp32-level accuracy) instead of cuBLAS SGEMMs.
+ *             Alternatively the address of an image made by cf_dense_pack_layer with bit 0 set (address | 1), for all
+ *             layers: the same kernel on the block-level tensor instructions.
  *   scalars : HOST array of num_layers x 6 doubles: gauss_scale, gauss_shift, -0.5/scale_real^2, elu beta,
  *             gauss_lb_real, dist_max
  *   x       : (N,128) atom features, updated in place
@@ -331,6 +333,14 @@ int cf_infinite_attn_fwd_sorted(const float *q, const float *k, const float *v, 
  *             after each layer's attention kernels (lets a caller time them without splitting the call)
  * Geometry arguments as in cf_infinite_attn_fwd.  No gradient support (training uses the autograd path).
  * ---------------------------------------------------------------------------------------------------------- */
+/* Images of the dense weights for the one-call forwards.  cf_dense_image_bytes(ff_dim): bytes of a layer's image, or of
+ * the embedding's with ff_dim = 0; 16-byte aligned device memory.  Weights as in the layer's state: Wq, Wk, Wv, Wo
+ * (128,128), W1 (ff,128), W2 (128,ff), row-major (out, in); W (128, feature_dim <= 128).  ff_dim: a multiple of 128 up
+ * to 3328.  One launch each on `stream`; an image stays valid until the weights change. */
+int64_t cf_dense_image_bytes(int64_t ff_dim);
+int cf_dense_pack_layer(const float *Wq, const float *Wk, const float *Wv, const float *Wo, const float *W1,
+                        const float *W2, int64_t ff_dim, void *image, void *stream);
+int cf_dense_pack_embedding(const float *W, int64_t feature_dim, void *image, void *stream);
 int64_t cf_encoder_workspace_floats(int64_t N, int64_t E, int64_t ff_dim);
 int cf_encoder_forward(void *cublas_handle, int num_layers, const float *const *weights, const double *scalars, float *x,
                        const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
@@ -380,7 +390,8 @@ int cf_peer_gather_collect(const uint64_t *cells, uint32_t step, const int64_t *
  * integers the caller knows from the sizes.  workspace: cf_model_workspace_bytes(N, B, E, ff_dim) bytes, 256-byte
  * aligned.  order_reach: the reach handed to cf_row_order (about dist_max).
  * W_embed_packed (optional, NULL to skip): W_embed with its input columns zero-padded to 128, packed like slot 10 of
- * the layer weights (feature_dim <= 128).  When it is given and every layer brings packed weights, the embedding runs
+ * the layer weights (feature_dim <= 128; an image from cf_dense_pack_embedding, address | 1, if the layers bring
+ * images).  When it is given and every layer brings packed weights, the embedding runs
  * inside the first dense block, the whole forward runs in this library's kernels and cublas_handle may be NULL.
  * gather (optional, NULL to skip): the pooling + head kernel also stores y into every rank's gather buffer (see
  * cf_peer_gather above; B <= gather->rows_per_rank).
