@@ -51,6 +51,10 @@ SIGNATURES = {
     "cf_dense_image_bytes": [I64],
     "cf_dense_pack_layer": [P, P, P, P, P, P, I64, P, P],
     "cf_dense_pack_embedding": [P, I64, P, P],
+    "cf_train_saved_bytes": [P, I64, I64, I64],
+    "cf_train_scratch_bytes": [P, I64, I64, I64],
+    "cf_train_forward": [P, P, P, P],
+    "cf_train_backward": [P, P, P, P, P, P],
     "cf_row_cost": [P, P, I64, I64, F64, P, P],
     "cf_row_order": [P, P, I64, I64, F64, P, P],
     "cf_reci_phase": [P, P, P, P, I64, P, P],
@@ -78,6 +82,20 @@ class ModelDesc(ctypes.Structure):
                 ("dense_tile_rows", ctypes.c_int32), ("weights", c_void_p), ("scalars", c_void_p), ("K", c_int64),
                 ("ff_dim", c_int64), ("wscale", c_double), ("cutoff_radius", c_double), ("W1", c_void_p), ("b1", c_void_p),
                 ("hidden", c_int64), ("W2", c_void_p), ("b2", c_void_p), ("targets", c_int64), ("order_reach", c_double)]
+
+
+class TrainDesc(ctypes.Structure):
+    """``cf_train_desc``: the batch-independent arguments of a training step."""
+    _fields_ = [("num_layers", ctypes.c_int32), ("lattice_range", ctypes.c_int32), ("minimum_range", ctypes.c_int32),
+                ("feature_dim", ctypes.c_int32), ("K", c_int64), ("ff_dim", c_int64), ("hidden", c_int64), ("targets", c_int64),
+                ("wscale", c_double), ("cutoff_radius", c_double), ("order_reach", c_double), ("weights", c_void_p),
+                ("scalars", c_void_p)]
+
+
+class TrainBatch(ctypes.Structure):
+    """``cf_train_batch``: a batch and the memory its step keeps between forward and backward."""
+    _fields_ = [("features", c_void_p), ("pos", c_void_p), ("trans", c_void_p), ("sizes", c_void_p), ("N", c_int64), ("B", c_int64),
+                ("E", c_int64), ("max_atoms", c_int64), ("saved", c_void_p)]
 
 
 class ServeSlot(ctypes.Structure):
@@ -137,7 +155,8 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
-        lib.cf_dense_image_bytes.restype = c_int64
+        for name in ("cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_scratch_bytes"):
+            getattr(lib, name).restype = c_int64
         _lib = lib
     return _lib
 

@@ -394,6 +394,28 @@ void pack_layer_forward(PackJob &job, int &count, unsigned char *image, int ff, 
     one(Wv, 128, Wq, Wk, Wv, 128 * 128);
 }
 
+void pack_layer_backward(PackJob &job, int &count, unsigned char *image, int ff, const float *Wq, const float *Wk, const float *Wv,
+                         const float *Wo, const float *W1, const float *W2)
+{
+    const int chunks = ff / 128;
+    int at = 0;
+    auto one = [&](const float *src, int ld, const float *g0, const float *g1, const float *g2, int elems) {
+        PackBlock &b = pack_add(job, count, image, at++, src, ld, 1);
+        b.group[0] = g0; b.group[1] = g1; b.group[2] = g2; b.group_elems = elems;
+    };
+    auto w2 = [&](int c) { one(W2 + (size_t)c * 128, ff, W2, nullptr, nullptr, ff * 128); };
+    one(Wq, 128, Wq, Wk, Wv, 128 * 128);
+    one(Wk, 128, Wq, Wk, Wv, 128 * 128);
+    one(Wv, 128, Wq, Wk, Wv, 128 * 128);
+    w2(0);
+    if (chunks > 1) w2(1);
+    for (int c = 0; c < chunks; ++c) {
+        one(W1 + (size_t)c * 128 * 128, 128, W1, nullptr, nullptr, ff * 128);
+        if (c + 2 < chunks) w2(c + 2);
+    }
+    one(Wo, 128, Wo, nullptr, nullptr, 128 * 128);
+}
+
 void pack_embedding(PackJob &job, int &count, unsigned char *image, const float *W, int feature_dim)
 {
     PackBlock &b = pack_add(job, count, image, 0, W, feature_dim, 0);

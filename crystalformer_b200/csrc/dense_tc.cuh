@@ -71,4 +71,48 @@ inline bool dense_tc_images(int num_layers, const float *const *weights)
 
 int launch_dense_forward(const DenseForward &p, cudaStream_t s);
 
+// ---- training (dense_tc_bwd.cu) ---------------------------------------------------------------------------------------
+// The blocks of one layer in the backward kernel's order, every one transposed: [Wq, Wk, Wv] and
+// [W2_0, W2_1, W1_0, W2_2, W1_1, ..., Wo].  Appends to job.
+void pack_layer_backward(PackJob &job, int &count, unsigned char *image, int ff, const float *Wq, const float *Wk, const float *Wv,
+                         const float *Wo, const float *W1, const float *W2);
+
+// Backward of a boundary: the head of layer l + 1, then the tail of layer l.
+struct DenseBackward {
+    long long N;
+    int ff;
+    bool chained;
+    // head (image null: none): gx = g_res + gq' Wq + gk Wk + gv Wv, gq' = gq / 4 + galpha w_pos
+    const unsigned char *head;
+    const float *q, *w_pos;      // the saved query (scaled by 1/4)
+    float gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound;
+    float *gq, *ga;              // in: gradients of the scaled query and of a; out: gq' and galpha
+    const float *gk, *gv, *g_res;
+    float *gx;                   // (N,128) out (with a head), in (without)
+    // tail (image null: none): gh = (gx W2) [h > 0], gy = gx + gh W1, gattn = gy Wo
+    const unsigned char *tail;
+    const float *h;              // (N, ff) the saved hidden units
+    float *gh, *gy, *gattn;
+};
+int launch_dense_backward(const DenseBackward &p, cudaStream_t s);
+
+// One 128 x 128 block of a weight gradient: out[i ld + j] = sum_n g[n ldg + i] x[n ldx + j] (j < cols), and, where bias is
+// not null, bias[i] = sum_n g[n ldg + i].
+struct GradJob {
+    const float *g, *x;
+    long long rows;
+    int ldg, ldx, x_cols, ldo;
+    float *out, *bias;
+};
+constexpr int GRAD_MAX = 56;            // jobs of one launch (a kernel parameter)
+constexpr int GRAD_MAX_SPLITS = 16;
+constexpr int GRAD_PARTIAL = 128 * 128 + 128;
+struct GradJobs {
+    GradJob j[GRAD_MAX];
+};
+// Launches the jobs with the rows split so that the blocks fill the SMs; partial holds grad_partial_floats(count, rows of
+// job 0).
+size_t grad_partial_floats(int count, long long rows);
+int launch_weight_grads(const GradJobs &jobs, int count, float *partial, cudaStream_t s);
+
 }  // namespace cf

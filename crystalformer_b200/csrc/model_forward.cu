@@ -33,14 +33,16 @@ constexpr int HEAD_THREADS = 128;
 constexpr int HEAD_MAX_HIDDEN = 1024;
 
 // One thread block per crystal: mean of the atoms' features, hidden = relu(W1 mean + b1), y = W2 hidden + b2.
-// GATHER: y also goes into every rank's gather buffer (peer_gather.cuh).
+// GATHER: y also goes into every rank's gather buffer (peer_gather.cuh).  pooled_out, hid_out (training, or null): the
+// mean and the hidden units are kept.
 template <bool GATHER>
 __global__ void __launch_bounds__(HEAD_THREADS) pool_head_kernel(const float *__restrict__ x,
                                                                  const int64_t *__restrict__ atom_start,
                                                                  const float *__restrict__ W1, const float *__restrict__ b1,
                                                                  const float *__restrict__ W2, const float *__restrict__ b2,
                                                                  int hidden, int targets, float *__restrict__ y,
-                                                                 const cf_peer_gather gather)
+                                                                 const cf_peer_gather gather, float *__restrict__ pooled_out,
+                                                                 float *__restrict__ hid_out)
 {
     __shared__ __align__(16) float pooled[MODEL_DIM];
     __shared__ float hid[HEAD_MAX_HIDDEN];
@@ -49,6 +51,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) pool_head_kernel(const float *__
     grid_dependency_wait();  // (chained launch behind the last dense block)
     const long long s = atom_start[c], len = atom_start[c + 1] - s;
     pooled[tid] = len > 0 ? segment_mean_channel(x + s * MODEL_DIM + tid, MODEL_DIM, len) : 0.f;
+    if (pooled_out != nullptr) pooled_out[c * MODEL_DIM + tid] = pooled[tid];
     __syncthreads();
     const float4 *p4 = reinterpret_cast<const float4 *>(pooled);
     for (int u = tid; u < hidden; u += HEAD_THREADS) {
@@ -60,6 +63,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) pool_head_kernel(const float *__
             a0 = fmaf(w.x, v.x, a0); a1 = fmaf(w.y, v.y, a1); a2 = fmaf(w.z, v.z, a2); a3 = fmaf(w.w, v.w, a3);
         }
         hid[u] = fmaxf((a0 + a1) + (a2 + a3) + b1[u], 0.f);
+        if (hid_out != nullptr) hid_out[c * hidden + u] = hid[u];
     }
     __syncthreads();
     for (int t = warp; t < targets; t += HEAD_THREADS / 32) {
@@ -122,6 +126,15 @@ extern "C" int64_t cf_model_workspace_bytes(int64_t N, int64_t B, int64_t E, int
 
 namespace cf {
 
+int launch_pool_head(const float *x, const int64_t *atom_start, const float *W1, const float *b1, const float *W2,
+                     const float *b2, int hidden, int targets, long long B, float *y, float *pooled, float *hid, bool chained,
+                     cudaStream_t s)
+{
+    launch_chained(pool_head_kernel<false>, dim3((unsigned)B), dim3(HEAD_THREADS), 0, s, chained, x, atom_start, W1, b1, W2, b2, hidden,
+                   targets, y, cf_peer_gather{}, pooled, hid);
+    return launch_status("pool_head_kernel");
+}
+
 // cf_model_forward with the species of the atoms given either as feature rows (`features`, the reference's interface)
 // or as indices (`species`: the embedding of atom i is column species[i] of W_embed, i.e. what a one-hot feature row
 // gives; only with packed weights, where the first dense block builds the one-hot rows in shared memory).
@@ -183,10 +196,9 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
     const bool chained = num_layers > 0 && N > 0;  // behind the encoder's last dense block
     if (gather != nullptr)
         launch_chained(pool_head_kernel<true>, dim3((unsigned)B), dim3(HEAD_THREADS), 0, s, chained, (const float *)w.x,
-                       (const int64_t *)w.atom_start, W1, b1, W2, b2, (int)hidden, (int)targets, y, *gather);
+                       (const int64_t *)w.atom_start, W1, b1, W2, b2, (int)hidden, (int)targets, y, *gather, (float *)nullptr, (float *)nullptr);
     else
-        launch_chained(pool_head_kernel<false>, dim3((unsigned)B), dim3(HEAD_THREADS), 0, s, chained, (const float *)w.x,
-                       (const int64_t *)w.atom_start, W1, b1, W2, b2, (int)hidden, (int)targets, y, cf_peer_gather{});
+        return launch_pool_head(w.x, w.atom_start, W1, b1, W2, b2, (int)hidden, (int)targets, B, y, nullptr, nullptr, chained, s);
     return launch_status("cf_model_forward");
 }
 

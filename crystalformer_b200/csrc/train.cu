@@ -1,0 +1,516 @@
+// One training step of the whole model in two host calls: the forward (keeping what the backward needs) and the backward
+// (gradients of every parameter).
+//
+// The autograd path records some sixty framework operations per layer; on a batch of crystals each of them is a few
+// microseconds of device work, and the host needs about 5 ms to issue them.  Here a step is about forty launches of this
+// library's kernels:
+//   forward    weight images (both directions), batch geometry, term lists, then per layer the dense boundary
+//              (dense_tc.cu) and the fused attention (infinite_attn_fwd.cu), pooling + head
+//   backward   head and pooling, then per layer the dense boundary (dense_tc_bwd.cu) and the attention backward
+//              (infinite_attn_bwd.cu), and at the end every weight gradient of the model in one launch each for the
+//              projections and for the value encoding
+// (models/latticeformer.py:211-302 with pooling "avr", a Linear - ReLU - Linear head and LayerNorm = Identity.)
+#include "common.cuh"
+#include "dense_tc.cuh"
+#include "term_list.cuh"
+
+namespace cf {
+int launch_prepare_all(const float *pos, const float *trans, const int64_t *sizes, int64_t *atom_start,
+                       int64_t *edge_start, long long B, long long N, long long E, int64_t *batch, int64_t *edges,
+                       int64_t *row_start, float *pos_ij, float *rvlen, double reach, int32_t *row_order, bool *ordered,
+                       cudaStream_t s);
+int infinite_attn_fwd_impl(const float *q, const float *k, const float *v, const float *a, const float *pos,
+                           const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
+                           const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t H, int64_t D,
+                           int64_t E, int64_t K, int64_t max_atoms, double dist_max, double wscale, const float *W,
+                           double cutoff_radius, int lattice_range, int minimum_range, float *out, float *logit,
+                           float *lse, float *psi_row, const int32_t *row_order, const TermList *list,
+                           unsigned *ticket_ready, void *stream, bool chained);
+int infinite_attn_bwd_impl(const float *q, const float *k, const float *v, const float *a, const float *pos,
+                           const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
+                           const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t H, int64_t D,
+                           int64_t E, int64_t K, int64_t max_atoms, double dist_max, double wscale, const float *W,
+                           double cutoff_radius, int lattice_range, int minimum_range, const float *logit,
+                           const float *lse, const float *out, const float *gout, float *gq, float *gk, float *gv,
+                           float *ga, float *glogit, const int32_t *row_order, const TermList *list, void *stream);
+int launch_pool_head(const float *x, const int64_t *atom_start, const float *W1, const float *b1, const float *W2,
+                     const float *b2, int hidden, int targets, long long B, float *y, float *pooled, float *hid, bool chained,
+                     cudaStream_t s);
+namespace {
+
+constexpr int CH = HEADS * HEAD_DIM;  // 128
+
+// ---- head and pooling, backward: one block per crystal ------------------------------------------------------------------
+__global__ void __launch_bounds__(128) head_backward_kernel(const float *__restrict__ gy, const float *__restrict__ hid,
+                                                            const float *__restrict__ W1, const float *__restrict__ W2,
+                                                            const int64_t *__restrict__ atom_start, int hidden, int targets,
+                                                            float *__restrict__ ghid, float *__restrict__ gx)
+{
+    __shared__ float gh[1024];
+    const long long c = blockIdx.x;
+    const int tid = threadIdx.x;
+    for (int u = tid; u < hidden; u += 128) {
+        float g = 0.f;
+        for (int t = 0; t < targets; ++t) g = fmaf(gy[c * targets + t], __ldg(W2 + (size_t)t * hidden + u), g);
+        g = hid[c * hidden + u] > 0.f ? g : 0.f;
+        gh[u] = g;
+        ghid[c * hidden + u] = g;
+    }
+    __syncthreads();
+    float g0 = 0.f, g1 = 0.f;
+#pragma unroll 8
+    for (int u = 0; u < hidden; u += 2) {
+        g0 = fmaf(gh[u], __ldg(W1 + (size_t)u * CH + tid), g0);
+        g1 = fmaf(gh[u + 1], __ldg(W1 + (size_t)(u + 1) * CH + tid), g1);
+    }
+    const long long s = atom_start[c], n = atom_start[c + 1] - s;
+    const float g = (g0 + g1) / (float)n;
+    for (long long r = 0; r < n; ++r) gx[(s + r) * CH + tid] = g;
+}
+
+// gradient of the head's last layer: gW2[t][u] = sum_c gy[c][t] hid[c][u], gb2[t] = sum_c gy[c][t].  Block = (32 units,
+// target); the warps take every eighth crystal and meet in shared memory in a fixed order.
+__global__ void __launch_bounds__(256) head_weight_grad_kernel(const float *__restrict__ gy, const float *__restrict__ hid, long long B,
+                                                               int hidden, int targets, float *__restrict__ gW2, float *__restrict__ gb2)
+{
+    __shared__ float part[2][8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, u = blockIdx.x * 32 + lane, t = blockIdx.y;
+    float acc = 0.f, bias = 0.f;
+    for (long long c = w; c < B; c += 8) {
+        const float g = gy[c * targets + t];
+        acc = fmaf(g, u < hidden ? hid[c * hidden + u] : 0.f, acc);
+        bias += g;
+    }
+    part[0][w][lane] = acc;
+    part[1][w][lane] = bias;
+    __syncthreads();
+    if (w == 0) {
+        float a = 0.f, b = 0.f;
+        for (int i = 0; i < 8; ++i) { a += part[0][i][lane]; b += part[1][i][lane]; }
+        if (u < hidden) gW2[(size_t)t * hidden + u] = a;
+        if (blockIdx.x == 0 && lane == 0) gb2[t] = b;
+    }
+}
+
+// ---- gradients of the value encoding's projection and of the width weights, all layers ------------------------------------
+//     gWpe[h][m][k] = sum_n gattn[n][h][m] psi[n][h][k],   gwpos[c] = sum_n galpha[n][c / 16] q[n][c]
+// Block = (a share of the rows, layer); thread = (head, bin) with the head's sixteen channels in registers: psi is read
+// once, coalesced, and bounds the kernel (2 KB per row and layer); gattn comes as shared-memory broadcasts.
+constexpr int PE_ROWS = 16;  // rows staged at a time
+constexpr int PE_PARTIAL = CH * 64 + CH;
+constexpr int MAX_LAYERS = 32;
+struct PeArgs {
+    const float *gattn[MAX_LAYERS], *psi[MAX_LAYERS], *q[MAX_LAYERS], *galpha[MAX_LAYERS];
+    float *gW[MAX_LAYERS], *gwpos[MAX_LAYERS];
+    long long N;
+    int shares;
+    float *partial;
+};
+
+template <bool PSI>
+__global__ void __launch_bounds__(512) pe_grad_kernel(const PeArgs p)
+{
+    __shared__ __align__(16) float go[PE_ROWS * CH];
+    const int tid = threadIdx.x, l = blockIdx.y, h = tid >> 6;
+    const long long lo = p.N * blockIdx.x / p.shares, hi = p.N * (blockIdx.x + 1) / p.shares;
+    const float *gattn = p.gattn[l], *psi = PSI ? p.psi[l] : nullptr, *q = p.q[l], *galpha = p.galpha[l];
+    float acc[16], wpos = 0.f;
+#pragma unroll
+    for (int m = 0; m < 16; ++m) acc[m] = 0.f;
+    for (long long n0 = lo; n0 < hi; n0 += PE_ROWS) {
+        const int rows = (int)min((long long)PE_ROWS, hi - n0);
+        if (PSI) {
+            __syncthreads();
+            for (int i = tid; i < rows * CH; i += 512) go[i] = gattn[n0 * CH + i];
+            __syncthreads();
+            float ps[PE_ROWS];
+#pragma unroll
+            for (int r = 0; r < PE_ROWS; ++r) ps[r] = r < rows ? psi[(n0 + r) * 512 + tid] : 0.f;
+#pragma unroll
+            for (int r = 0; r < PE_ROWS; ++r) {
+                if (r >= rows) break;
+                const float4 *g4 = reinterpret_cast<const float4 *>(go + r * CH + h * 16);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const float4 g = g4[m];
+                    acc[4 * m] = fmaf(g.x, ps[r], acc[4 * m]); acc[4 * m + 1] = fmaf(g.y, ps[r], acc[4 * m + 1]);
+                    acc[4 * m + 2] = fmaf(g.z, ps[r], acc[4 * m + 2]); acc[4 * m + 3] = fmaf(g.w, ps[r], acc[4 * m + 3]);
+                }
+            }
+        }
+        if (tid < CH)
+            for (int r = 0; r < rows; ++r) wpos = fmaf(galpha[(n0 + r) * HEADS + (tid >> 4)], 4.0f * q[(n0 + r) * CH + tid], wpos);
+    }
+    float *out = p.partial + ((size_t)l * p.shares + blockIdx.x) * PE_PARTIAL;
+    if (PSI) {
+#pragma unroll
+        for (int m = 0; m < 16; ++m) out[(h * 16 + m) * 64 + (tid & 63)] = acc[m];
+    }
+    if (tid < CH) out[CH * 64 + tid] = wpos;
+}
+
+__global__ void __launch_bounds__(256) pe_grad_sum_kernel(const PeArgs p, int with_psi)
+{
+    const int l = blockIdx.y, idx = (with_psi ? 0 : CH * 64) + blockIdx.x * 256 + threadIdx.x;
+    if (idx >= PE_PARTIAL) return;
+    const float *in = p.partial + (size_t)l * p.shares * PE_PARTIAL + idx;
+    float t = 0.f;
+#pragma unroll 4
+    for (int sh = 0; sh < p.shares; ++sh) t += in[(size_t)sh * PE_PARTIAL];
+    if (idx < CH * 64) p.gW[l][idx] = t;
+    else p.gwpos[l][idx - CH * 64] = t;
+}
+
+// ---- memory ----------------------------------------------------------------------------------------------------------------
+struct Carver {
+    char *base;
+    size_t used = 0;
+    template <class T>
+    T *take(size_t count)
+    {
+        T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (count * sizeof(T) + 255) & ~(size_t)255;
+        return p;
+    }
+};
+
+struct LayerSaved {
+    unsigned char *forward, *backward;  // weight images
+    float *q, *k, *v, *a, *lse, *logit, *attn, *psi, *y, *h;
+};
+struct Saved {
+    int64_t *atom_start, *edge_start, *batch, *row_start, *edges;
+    float *pos_ij, *rvlen;
+    int32_t *row_order;
+    unsigned *tickets;
+    unsigned char *embed;
+    void *lists;
+    float *x[MAX_LAYERS + 1];
+    LayerSaved layer[MAX_LAYERS];
+    float *pooled, *hid;
+    size_t bytes;
+};
+Saved carve_saved(const cf_train_desc &d, void *memory, int64_t N, int64_t B, int64_t E)
+{
+    Carver c{static_cast<char *>(memory)};
+    Saved s{};
+    s.atom_start = c.take<int64_t>(B + 1);
+    s.edge_start = c.take<int64_t>(B + 1);
+    s.batch = c.take<int64_t>(N);
+    s.row_start = c.take<int64_t>(N + 1);
+    s.edges = c.take<int64_t>(2 * E);
+    s.pos_ij = c.take<float>(3 * E);
+    s.rvlen = c.take<float>(3 * B);
+    s.row_order = c.take<int32_t>(N);
+    s.tickets = c.take<unsigned>(MAX_LAYERS);
+    s.embed = c.take<unsigned char>(tc_image_bytes(1));
+    s.lists = c.take<char>(term_list_workspace_bytes(N, E));
+    const size_t image = tc_image_bytes(tc_layer_blocks((int)d.ff_dim));
+    for (int l = 0; l < d.num_layers; ++l) {
+        LayerSaved &y = s.layer[l];
+        s.x[l] = c.take<float>(N * CH);
+        y.forward = c.take<unsigned char>(image);
+        y.backward = c.take<unsigned char>(image);
+        y.q = c.take<float>(N * CH); y.k = c.take<float>(N * CH); y.v = c.take<float>(N * CH);
+        y.a = c.take<float>(N * HEADS); y.lse = c.take<float>(N * HEADS); y.logit = c.take<float>(E * HEADS);
+        y.attn = c.take<float>(N * CH);
+        y.psi = d.K > 0 ? c.take<float>(N * HEADS * d.K) : nullptr;
+        y.y = c.take<float>(N * CH);
+        y.h = c.take<float>(N * d.ff_dim);
+    }
+    s.x[d.num_layers] = c.take<float>(N * CH);
+    s.pooled = c.take<float>(B * CH);
+    s.hid = c.take<float>(B * d.hidden);
+    s.bytes = c.used;
+    return s;
+}
+
+struct LayerGrads {
+    float *gh, *gy, *gattn, *gq, *gk, *gv, *ga;
+};
+struct Scratch {
+    float *gx[MAX_LAYERS + 1];
+    LayerGrads layer[MAX_LAYERS];
+    float *glogit, *ghid, *partial, *pe_partial;
+    int shares;
+    size_t bytes;
+};
+int train_jobs(const cf_train_desc &d) { return d.num_layers * (4 + 2 * (int)(d.ff_dim / 128)) + 1 + (int)(d.hidden / 128); }
+Scratch carve_scratch(const cf_train_desc &d, void *memory, int64_t N, int64_t B, int64_t E)
+{
+    Carver c{static_cast<char *>(memory)};
+    Scratch s{};
+    for (int l = 0; l < d.num_layers; ++l) {
+        LayerGrads &g = s.layer[l];
+        s.gx[l] = c.take<float>(N * CH);
+        g.gh = c.take<float>(N * d.ff_dim);
+        g.gy = c.take<float>(N * CH); g.gattn = c.take<float>(N * CH);
+        g.gq = c.take<float>(N * CH); g.gk = c.take<float>(N * CH); g.gv = c.take<float>(N * CH);
+        g.ga = c.take<float>(N * HEADS);
+    }
+    s.gx[d.num_layers] = c.take<float>(N * CH);
+    s.glogit = c.take<float>(E * HEADS);
+    s.ghid = c.take<float>(B * d.hidden);
+    const int jobs = train_jobs(d);
+    size_t most = 0;
+    for (int at = 0; at < jobs; at += GRAD_MAX) {
+        const size_t f = grad_partial_floats(jobs - at < GRAD_MAX ? jobs - at : GRAD_MAX, N);
+        most = f > most ? f : most;
+    }
+    s.partial = c.take<float>(most);
+    // shares of the rows per layer for the value-encoding gradient: one wave of blocks, at least one stage of rows each
+    long long shares = sm_count() * 3 / (d.num_layers > 0 ? d.num_layers : 1);
+    const long long most_shares = (N + PE_ROWS - 1) / PE_ROWS;
+    shares = shares < most_shares ? shares : most_shares;
+    s.shares = (int)(shares > 1 ? shares : 1);
+    s.pe_partial = c.take<float>((size_t)d.num_layers * s.shares * PE_PARTIAL);
+    s.bytes = c.used;
+    return s;
+}
+
+int check_desc(const cf_train_desc *d, const char *who)
+{
+    CF_REQUIRE(d != nullptr && d->weights && d->scalars, CF_ERR_INVALID, "%s: null description", who);
+    CF_REQUIRE(d->num_layers >= 1 && d->num_layers <= MAX_LAYERS, CF_ERR_UNSUPPORTED, "%s: %d layers (1..%d)", who, (int)d->num_layers, MAX_LAYERS);
+    CF_REQUIRE(d->ff_dim > 0 && d->ff_dim % 128 == 0 && d->ff_dim <= TC_MAX_FF, CF_ERR_UNSUPPORTED,
+               "%s: ff_dim=%lld must be a multiple of 128 up to %d", who, (long long)d->ff_dim, TC_MAX_FF);
+    CF_REQUIRE(d->hidden > 0 && d->hidden % 128 == 0 && d->hidden <= 1024 && d->targets > 0, CF_ERR_UNSUPPORTED,
+               "%s: head of %lld hidden units, %lld targets (a multiple of 128 up to 1024)", who, (long long)d->hidden, (long long)d->targets);
+    CF_REQUIRE(d->feature_dim >= 1 && d->feature_dim <= 128, CF_ERR_UNSUPPORTED, "%s: %d features (1..128)", who, (int)d->feature_dim);
+    CF_REQUIRE(d->K == 0 || d->K == 64, CF_ERR_UNSUPPORTED, "%s: K=%lld, only K in {0,64} is compiled", who, (long long)d->K);
+    CF_REQUIRE(d->lattice_range >= 0 && d->lattice_range <= CF_MAX_RANGE && d->minimum_range >= 0, CF_ERR_RANGE,
+               "%s: lattice_range %d outside [0,%d]", who, (int)d->lattice_range, CF_MAX_RANGE);
+    return CF_OK;
+}
+int check_batch(const cf_train_batch *b, const char *who)
+{
+    CF_REQUIRE(b != nullptr, CF_ERR_INVALID, "%s: null batch", who);
+    CF_REQUIRE(b->N >= 1 && b->B >= 1 && b->E >= 1 && b->B <= (1 << 20), CF_ERR_INVALID, "%s: empty batch or too many crystals", who);
+    CF_REQUIRE(b->max_atoms >= 1 && b->max_atoms <= 1024, CF_ERR_RANGE, "%s: max_atoms=%lld outside [1,1024]", who, (long long)b->max_atoms);
+    CF_REQUIRE(b->features && b->pos && b->trans && b->sizes && b->saved, CF_ERR_INVALID, "%s: null pointer", who);
+    return CF_OK;
+}
+
+// Weights of layer l: Wq Wk Wv b_in w_pos Wpe Wo bo W1 b1 W2 b2; after the layers: W_embed, the head's W1 b1 W2 b2.
+enum { W_Q, W_K, W_V, B_IN, W_POS, W_PE, W_O, B_O, W_1, B_1, W_2, B_2, PER_LAYER };
+
+bool lists_of(const cf_train_desc &d, const Saved &s, int64_t N, int64_t E, TermList &list, float &a_widest)
+{
+    a_widest = -INFINITY;
+    for (int l = 0; l < d.num_layers; ++l) a_widest = fmaxf(a_widest, (float)(d.scalars[6 * l + 4] * d.scalars[6 * l + 2]));
+    if (!(weight_floor_log2() > -200.0f) || !(a_widest < 0.0f)) return false;
+    int *start, *count;
+    float *dmin;
+    unsigned long long *cursor;
+    float2 *pool;
+    term_list_carve(s.lists, N, E, &start, &count, &dmin, &cursor, &pool);
+    list.pool = pool; list.start = start; list.count = count; list.dmin = dmin;
+    list.window = term_window(weight_floor_log2(), a_widest);
+    return true;
+}
+
+}  // namespace
+}  // namespace cf
+
+extern "C" int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E)
+{
+    if (cf::check_desc(desc, "cf_train_saved_bytes") != CF_OK) return -1;
+    return (int64_t)cf::carve_saved(*desc, nullptr, N, B, E).bytes;
+}
+
+extern "C" int64_t cf_train_scratch_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E)
+{
+    if (cf::check_desc(desc, "cf_train_scratch_bytes") != CF_OK) return -1;
+    return (int64_t)cf::carve_scratch(*desc, nullptr, N, B, E).bytes;
+}
+
+extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, float *y, void *stream)
+{
+    using namespace cf;
+    int rc = check_desc(desc, "cf_train_forward");
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward");
+    if (rc != CF_OK) return rc;
+    CF_REQUIRE(y != nullptr, CF_ERR_INVALID, "cf_train_forward: null pointer");
+    const cf_train_desc &d = *desc;
+    const cf_train_batch &b = *batch;
+    const int64_t N = b.N, B = b.B, E = b.E;
+    const int L = d.num_layers, ff = (int)d.ff_dim;
+    cudaStream_t s = as_stream(stream);
+    Saved w = carve_saved(d, b.saved, N, B, E);
+    const float *const *tail_weights = d.weights + PER_LAYER * L;
+
+    // ---- weight images, both directions
+    {
+        static thread_local PackJob job;
+        int count = 0;
+        auto flush = [&](int need) {
+            if (rc == CF_OK && count + need > PACK_MAX) {
+                rc = launch_pack(job, count, s);
+                count = 0;
+            }
+        };
+        pack_embedding(job, count, w.embed, tail_weights[0], (int)d.feature_dim);
+        const int blocks = tc_layer_blocks(ff);
+        for (int dir = 0; dir < 2; ++dir)
+            for (int l = 0; l < L; ++l) {
+                const float *const *p = d.weights + PER_LAYER * l;
+                flush(blocks);
+                if (dir == 0) pack_layer_forward(job, count, w.layer[l].forward, ff, p[W_Q], p[W_K], p[W_V], p[W_O], p[W_1], p[W_2]);
+                else pack_layer_backward(job, count, w.layer[l].backward, ff, p[W_Q], p[W_K], p[W_V], p[W_O], p[W_1], p[W_2]);
+            }
+        if (rc == CF_OK) rc = launch_pack(job, count, s);
+        if (rc != CF_OK) return rc;
+    }
+    // ---- geometry and term lists
+    if (cudaMemsetAsync(w.tickets, 0, sizeof(unsigned) * MAX_LAYERS, s) != cudaSuccess) return launch_status("cf_train_forward: tickets");
+    bool ordered = false;
+    rc = launch_prepare_all(b.pos, b.trans, b.sizes, w.atom_start, w.edge_start, B, N, E, w.batch, w.edges, w.row_start, w.pos_ij, w.rvlen,
+                            d.order_reach, w.row_order, &ordered, s);
+    if (rc != CF_OK) return rc;
+    const int32_t *order = ordered ? w.row_order : nullptr;
+    const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
+    TermList list{};
+    float a_widest;
+    const bool listed = lists_of(d, w, N, E, list, a_widest);
+    if (listed) {
+        TermListBuild tb{};
+        tb.pos_ij = w.pos_ij; tb.tvecs = b.trans; tb.rvlen = rvlen; tb.batch = w.batch; tb.edges = w.edges; tb.row_start = w.row_start;
+        tb.row_order = order; tb.N = N; tb.E = E; tb.max_atoms = (int)b.max_atoms;
+        tb.rule = BoxRule{(float)d.cutoff_radius, d.lattice_range, d.minimum_range};
+        tb.a_widest = a_widest;
+        tb.window = list.window;
+        term_list_carve(w.lists, N, E, &tb.start, &tb.count, &tb.dmin, &tb.cursor, &tb.pool);
+        tb.capacity = (long long)term_pool_entries(N, E);
+        rc = launch_term_list_build(tb, s);
+        if (rc != CF_OK) return rc;
+    }
+    // ---- layers
+    for (int l = 0; l <= L && rc == CF_OK; ++l) {
+        DenseForward t{};
+        t.N = N; t.ff = ff; t.chained = l > 0; t.weights_fresh = true;
+        t.x_out = w.x[l];
+        if (l > 0) {
+            const LayerSaved &y = w.layer[l - 1];
+            const float *const *p = d.weights + PER_LAYER * (l - 1);
+            t.tail = y.forward; t.attn = y.attn; t.bo = p[B_O]; t.b1 = p[B_1]; t.b2 = p[B_2];
+            t.x_in = w.x[l - 1]; t.y_save = y.y; t.h_save = y.h;
+        } else {
+            t.embed = w.embed; t.features = b.features; t.feature_dim = (int)d.feature_dim;
+        }
+        if (l < L) {
+            const LayerSaved &y = w.layer[l];
+            const float *const *p = d.weights + PER_LAYER * l;
+            const double *sc = d.scalars + 6 * l;
+            t.head = y.forward; t.bqkv = p[B_IN]; t.w_pos = p[W_POS];
+            t.gauss_scale = (float)sc[0]; t.gauss_shift = (float)sc[1]; t.a_factor = (float)sc[2];
+            t.elu_beta = (float)sc[3]; t.lower_bound = (float)sc[4];
+            t.q = y.q; t.k = y.k; t.v = y.v; t.a = y.a;
+        }
+        rc = launch_dense_forward(t, s);
+        if (rc != CF_OK || l == L) break;
+        const LayerSaved &y = w.layer[l];
+        rc = infinite_attn_fwd_impl(y.q, y.k, y.v, y.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
+                                    HEAD_DIM, E, d.K, b.max_atoms, d.scalars[6 * l + 5], d.wscale, d.weights[PER_LAYER * l + W_PE],
+                                    d.cutoff_radius, d.lattice_range, d.minimum_range, y.attn, y.logit, y.lse, y.psi, order,
+                                    listed ? &list : nullptr, w.tickets + l, s, true);
+    }
+    if (rc != CF_OK) return rc;
+    return launch_pool_head(w.x[L], w.atom_start, tail_weights[1], tail_weights[2], tail_weights[3], tail_weights[4], (int)d.hidden,
+                            (int)d.targets, B, y, w.pooled, w.hid, true, s);
+}
+
+extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, const float *gy, void *scratch,
+                                 float *const *grads, void *stream)
+{
+    using namespace cf;
+    int rc = check_desc(desc, "cf_train_backward");
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_backward");
+    if (rc != CF_OK) return rc;
+    CF_REQUIRE(gy && scratch && grads, CF_ERR_INVALID, "cf_train_backward: null pointer");
+    const cf_train_desc &d = *desc;
+    const cf_train_batch &b = *batch;
+    const int64_t N = b.N, B = b.B, E = b.E;
+    const int L = d.num_layers, ff = (int)d.ff_dim, hidden = (int)d.hidden, targets = (int)d.targets;
+    cudaStream_t s = as_stream(stream);
+    const Saved w = carve_saved(d, b.saved, N, B, E);
+    Scratch g = carve_scratch(d, scratch, N, B, E);
+    const float *const *tail_weights = d.weights + PER_LAYER * L;
+    float *const *tail_grads = grads + PER_LAYER * L;
+    const bool ordered = N < (1ll << 31) && B <= 2048;
+    const int32_t *order = ordered ? w.row_order : nullptr;
+    const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
+    TermList list{};
+    float a_widest;
+    const bool listed = lists_of(d, w, N, E, list, a_widest);
+
+    head_backward_kernel<<<(unsigned)B, 128, 0, s>>>(gy, w.hid, tail_weights[1], tail_weights[3], w.atom_start, hidden, targets, g.ghid, g.gx[L]);
+    head_weight_grad_kernel<<<dim3((hidden + 31) / 32, targets), 256, 0, s>>>(gy, w.hid, B, hidden, targets, tail_grads[3], tail_grads[4]);
+    for (int l = L - 1; l >= -1 && rc == CF_OK; --l) {
+        DenseBackward t{};
+        t.N = N; t.ff = ff;
+        t.gx = g.gx[l + 1];
+        if (l + 1 < L) {  // head of layer l + 1
+            const LayerSaved &y = w.layer[l + 1];
+            const LayerGrads &gg = g.layer[l + 1];
+            const double *sc = d.scalars + 6 * (l + 1);
+            t.head = y.backward; t.q = y.q; t.w_pos = d.weights[PER_LAYER * (l + 1) + W_POS];
+            t.gauss_scale = (float)sc[0]; t.gauss_shift = (float)sc[1]; t.a_factor = (float)sc[2];
+            t.elu_beta = (float)sc[3]; t.lower_bound = (float)sc[4];
+            t.gq = gg.gq; t.gk = gg.gk; t.gv = gg.gv; t.ga = gg.ga; t.g_res = gg.gy;
+        }
+        if (l >= 0) {
+            const LayerSaved &y = w.layer[l];
+            const LayerGrads &gg = g.layer[l];
+            t.tail = y.backward; t.h = y.h; t.gh = gg.gh; t.gy = gg.gy; t.gattn = gg.gattn;
+        }
+        rc = launch_dense_backward(t, s);
+        if (rc != CF_OK || l < 0) break;
+        const LayerSaved &y = w.layer[l];
+        const LayerGrads &gg = g.layer[l];
+        rc = infinite_attn_bwd_impl(y.q, y.k, y.v, y.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
+                                    HEAD_DIM, E, d.K, b.max_atoms, d.scalars[6 * l + 5], d.wscale, d.weights[PER_LAYER * l + W_PE],
+                                    d.cutoff_radius, d.lattice_range, d.minimum_range, y.logit, y.lse, y.attn, gg.gattn, gg.gq, gg.gk,
+                                    gg.gv, gg.ga, g.glogit, order, listed ? &list : nullptr, s);
+    }
+    if (rc != CF_OK) return rc;
+    // ---- value encoding and width weights
+    PeArgs pe{};
+    pe.N = N; pe.shares = g.shares; pe.partial = g.pe_partial;
+    for (int l = 0; l < L; ++l) {
+        pe.gattn[l] = g.layer[l].gattn; pe.psi[l] = w.layer[l].psi; pe.q[l] = w.layer[l].q; pe.galpha[l] = g.layer[l].ga;
+        pe.gW[l] = grads[PER_LAYER * l + W_PE]; pe.gwpos[l] = grads[PER_LAYER * l + W_POS];
+    }
+    if (d.K > 0) pe_grad_kernel<true><<<dim3(g.shares, L), 512, 0, s>>>(pe);
+    else pe_grad_kernel<false><<<dim3(g.shares, L), 512, 0, s>>>(pe);
+    pe_grad_sum_kernel<<<dim3(((d.K > 0 ? PE_PARTIAL : CH) + 255) / 256, L), 256, 0, s>>>(pe, d.K > 0 ? 1 : 0);
+    // ---- projections
+    static thread_local GradJobs jobs;
+    int count = 0;
+    auto add = [&](const float *gm, int ldg, const float *xm, int ldx, long long rows, int x_cols, float *out, int ldo, float *bias) {
+        if (rc == CF_OK && count == GRAD_MAX) {
+            rc = launch_weight_grads(jobs, count, g.partial, s);
+            count = 0;
+        }
+        GradJob &j = jobs.j[count++];
+        j.g = gm; j.ldg = ldg; j.x = xm; j.ldx = ldx; j.rows = rows; j.x_cols = x_cols; j.out = out; j.ldo = ldo; j.bias = bias;
+    };
+    for (int l = 0; l < L; ++l) {
+        const LayerSaved &y = w.layer[l];
+        const LayerGrads &gg = g.layer[l];
+        float *const *o = grads + PER_LAYER * l;
+        add(gg.gq, CH, w.x[l], CH, N, CH, o[W_Q], CH, o[B_IN]);
+        add(gg.gk, CH, w.x[l], CH, N, CH, o[W_K], CH, o[B_IN] + CH);
+        add(gg.gv, CH, w.x[l], CH, N, CH, o[W_V], CH, o[B_IN] + 2 * CH);
+        add(gg.gy, CH, y.attn, CH, N, CH, o[W_O], CH, o[B_O]);
+        for (int c = 0; c < ff / CH; ++c) {
+            add(gg.gh + c * CH, ff, y.y, CH, N, CH, o[W_1] + (size_t)c * CH * CH, CH, o[B_1] + c * CH);
+            add(g.gx[l + 1], CH, y.h + c * CH, ff, N, CH, o[W_2] + c * CH, ff, c == 0 ? o[B_2] : nullptr);
+        }
+    }
+    add(g.gx[0], CH, b.features, (int)d.feature_dim, N, (int)d.feature_dim, tail_grads[0], (int)d.feature_dim, nullptr);
+    for (int u = 0; u < hidden / CH; ++u)
+        add(g.ghid + u * CH, hidden, w.pooled, CH, B, CH, tail_grads[1] + (size_t)u * CH * CH, CH, tail_grads[2] + u * CH);
+    if (rc == CF_OK) rc = launch_weight_grads(jobs, count, g.partial, s);
+    if (rc != CF_OK) return rc;
+    return launch_status("cf_train_backward");
+}

@@ -203,7 +203,11 @@ class CrystalformerEncoderCUDA(Module):
     # Inference fast path: the whole stack in one call into the library (cf_encoder_forward).
     # -----------------------------------------------------------------------------------------------------------
     def _native_ok(self) -> bool:
-        if self.training or torch.is_grad_enabled() or self.norm is not None or self.d_model != 128 or self.nhead != 8:
+        return not self.training and not torch.is_grad_enabled() and self._native_model()
+
+    def _native_model(self) -> bool:
+        """Whether the layers are what the one-call paths implement (inference and training)."""
+        if self.norm is not None or self.d_model != 128 or self.nhead != 8:
             return False
         for layer in self.layers:
             att, P = layer.self_attn, layer.self_attn.params

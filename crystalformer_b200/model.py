@@ -17,6 +17,7 @@ from . import _lib
 from .cuda_funcs import IrregularMeanCUDA
 from .encoder import MAX_IMAGE_FF, BatchGeometry, CrystalformerEncoderCUDA, image_pointer, pack_dense_embedding, pack_dense_weight
 from .params import DEFAULT_MODEL_PARAMS, LatticeformerParams
+from .training import train_step
 
 
 def default_params(**overrides) -> types.SimpleNamespace:
@@ -110,6 +111,10 @@ class Latticeformer(nn.Module):
     # (cf_model_forward); taken in eval mode without autograd when the configuration is the one it implements.
     # ---------------------------------------------------------------------------------------------------------------
     def _native_ok(self) -> bool:
+        return self._native_shell() and self.encoder._native_ok()
+
+    def _native_shell(self) -> bool:
+        """Whether embedding, pooling and head are what the one-call paths implement (inference and training)."""
         if not getattr(self, "native", True) or self.pooling != "avr" or isinstance(self.proj_before_pooling, nn.Module):
             return False
         m = self.mlp
@@ -117,7 +122,7 @@ class Latticeformer(nn.Module):
                 and isinstance(m[2], nn.ReLU) and isinstance(m[3], nn.Linear) and m[0].in_features == 128
                 and m[0].out_features <= 1024 and m[0].bias is not None and m[3].bias is not None):
             return False
-        return self.input_embeddings.out_features == 128 and self.encoder.native and self.encoder._native_ok()
+        return self.input_embeddings.out_features == 128 and self.encoder.native
 
     def _embedding_packed(self, device) -> Optional[torch.Tensor]:
         """The embedding weight, packed like the layers' projections (the fused dense kernel then computes the embedding
@@ -147,10 +152,7 @@ class Latticeformer(nn.Module):
         w = enc._packed_weights(device)
         plan = dict(w=w, emb=f32(self.input_embeddings.weight), w1=f32(self.mlp[0].weight), b1=f32(self.mlp[0].bias),
                     w2=f32(self.mlp[3].weight), b2=f32(self.mlp[3].bias), emb_packed=self._embedding_packed(device))
-        dist_max = P.value_pe_dist_max
-        if dist_max < 0:
-            sr = P.scale_real[0] if isinstance(P.scale_real, (list, tuple)) else P.scale_real
-            dist_max = -dist_max * sr
+        reach = self.native_reach()
         plan["hidden"], plan["targets"] = plan["w1"].shape[0], plan["w2"].shape[0]
         if plan["emb_packed"] is not None:  # the description of the model for cf_serve_submit
             plan["desc"] = _lib.ModelDesc(
@@ -160,12 +162,21 @@ class Latticeformer(nn.Module):
                 weights=ctypes.cast(w["ptrs"], ctypes.c_void_p), scalars=ctypes.cast(w["scalars"], ctypes.c_void_p),
                 K=int(P.value_pe_dist_real), ff_dim=w["ff"], wscale=float(P.value_pe_width_scale), cutoff_radius=enc._cutoff(),
                 W1=plan["w1"].data_ptr(), b1=plan["b1"].data_ptr(), hidden=plan["hidden"], W2=plan["w2"].data_ptr(),
-                b2=plan["b2"].data_ptr(), targets=plan["targets"], order_reach=float(dist_max) + 1.0)
+                b2=plan["b2"].data_ptr(), targets=plan["targets"], order_reach=reach)
         plan["tail"] = (len(enc.layers), w["ptrs"], w["scalars"], int(P.value_pe_dist_real), w["ff"],
                         float(P.value_pe_width_scale), enc._cutoff(), int(P.lattice_range),
                         int(P.lattice_range) if P.minimum_range else 0, plan["w1"].data_ptr(), plan["b1"].data_ptr(),
-                        plan["hidden"], plan["w2"].data_ptr(), plan["b2"].data_ptr(), plan["targets"], float(dist_max) + 1.0)
+                        plan["hidden"], plan["w2"].data_ptr(), plan["b2"].data_ptr(), plan["targets"], reach)
         return plan
+
+    def native_reach(self) -> float:
+        """The reach that orders the rows of a batch (ops.row_order)."""
+        P = self.encoder.lattice_params
+        dist_max = P.value_pe_dist_max
+        if dist_max < 0:
+            sr = P.scale_real[0] if isinstance(P.scale_real, (list, tuple)) else P.scale_real
+            dist_max = -dist_max * sr
+        return float(dist_max) + 1.0
 
     WORKSPACE_RING = 4  # forwards whose preparation may be in flight at a time (see _forward_native, inputs_ready)
 
@@ -238,6 +249,14 @@ class Latticeformer(nn.Module):
                 host = data.sizes.tolist()  # the one device->host read per batch (the reference does the same)
                 counts = (sum(host), sum(n * n for n in host), max(host) if host else 1)
             return self._forward_native(data, counts, gather, inputs_ready=inputs_ready)
+        if geometry is None and torch.is_grad_enabled() and data.pos.is_cuda and self._native_shell() \
+                and self.encoder._native_model():
+            y = train_step(self, data, counts)
+            if y is not None:
+                if gather is not None:
+                    gather.store(y)
+                    return gather.collect()
+                return y
         x = self.input_embeddings(data.x)
         if geometry is None:
             geometry = BatchGeometry(data.pos, data.trans_vec, data.sizes, *(counts if counts is not None else ()))

@@ -1,0 +1,165 @@
+"""Training step of the model shell in two library calls (cf_train_forward / cf_train_backward) behind one autograd node.
+
+``Latticeformer.forward`` takes it whenever gradients are enabled and the configuration is the one the calls implement:
+the node's inputs are the model's parameters, its backward returns all of their gradients.  Same values as the
+operation-by-operation autograd path (models/latticeformer.py:211-302 and its backward), which stays for everything else."""
+from __future__ import annotations
+
+import ctypes
+from typing import Optional, Tuple
+
+import torch
+
+from . import _lib
+
+
+class TrainPlan:
+    """What a step needs and the batch does not change: the parameters in the library's order with their addresses, the
+    scalar settings, and where every gradient lies in one flat buffer.  Valid while the parameters keep their storage."""
+
+    def __init__(self, model):
+        enc = model.encoder
+        P = enc.lattice_params
+        ordered, scalars = [], []
+        for layer in enc.layers:
+            att, Q = layer.self_attn, layer.self_attn.params
+            ordered += [att.q_proj_weight, att.k_proj_weight, att.v_proj_weight, att.in_proj_bias, att.lattice_pos_weights,
+                        att.pe_dist_proj, att.out_proj.weight, att.out_proj.bias, layer.linear1.weight, layer.linear1.bias,
+                        layer.linear2.weight, layer.linear2.bias]
+            beta = float(Q.positive_func.split("=")[1]) if "=" in Q.positive_func else 1.0
+            dist_max = Q.value_pe_dist_max if Q.value_pe_dist_max >= 0 else -Q.value_pe_dist_max * Q.scale_real
+            gs = att.gauss_scale.detach().cpu().tolist()
+            scalars += [gs[0], gs[1], -0.5 * Q.scale_real ** -2, beta, Q.gauss_lb_real, dist_max]
+        ordered += [model.input_embeddings.weight, model.mlp[0].weight, model.mlp[0].bias, model.mlp[3].weight, model.mlp[3].bias]
+        self.params = [p for p in ordered if p is not None]
+        # the places where the model holds them (and its submodules): a step checks that they are still the same objects
+        at = {id(p): (m._parameters, n) for m in model.modules() for n, p in m._parameters.items() if p is not None}
+        self.places = [(*at[id(p)], p) for p in self.params]
+        self.children = [(m._modules, n, c) for m in model.modules() for n, c in m._modules.items()]
+        self.scales = [layer.self_attn.gauss_scale for layer in enc.layers]
+        self.key = self.current_key()
+        sizes = [p.numel() for p in self.params]
+        # gradients start on 256-byte boundaries of one buffer (the kernels store rows of them as vectors)
+        offsets, at = [], 0
+        for n in sizes:
+            offsets.append(at)
+            at += (n + 63) // 64 * 64
+        self.spans = list(zip(offsets, sizes, [p.shape for p in self.params]))
+        self.floats = at
+        where = iter(range(len(self.params)))
+        self.slots = [None if p is None else next(where) for p in ordered]
+        self.offsets = offsets
+        self.pointers = (ctypes.c_void_p * len(ordered))(*[None if p is None else p.data_ptr() for p in ordered])
+        self.scalars = (ctypes.c_double * len(scalars))(*scalars)
+        self.targets = model.mlp[3].out_features
+        order_reach = model.native_reach()
+        self.desc = _lib.TrainDesc(
+            num_layers=len(enc.layers), lattice_range=int(P.lattice_range),
+            minimum_range=int(P.lattice_range) if P.minimum_range else 0, feature_dim=model.input_embeddings.in_features,
+            K=int(P.value_pe_dist_real), ff_dim=enc.layers[0].linear1.out_features, hidden=model.mlp[0].out_features,
+            targets=self.targets, wscale=float(P.value_pe_width_scale), cutoff_radius=enc._cutoff(), order_reach=order_reach,
+            weights=ctypes.cast(self.pointers, ctypes.c_void_p), scalars=ctypes.cast(self.scalars, ctypes.c_void_p))
+
+    def current(self) -> bool:
+        return all(d.get(n) is c for d, n, c in self.children) and all(d.get(n) is p for d, n, p in self.places) \
+            and self.current_key() == self.key
+
+    # a copy of the model makes its own plan (addresses cannot be copied)
+    def __deepcopy__(self, memo):
+        return None
+
+    def __reduce__(self):
+        return type(None), ()
+
+    def current_key(self) -> tuple:
+        return tuple([p.data_ptr() for p in self.params] + [g._version for g in self.scales] + [g.data_ptr() for g in self.scales])
+
+    def versions(self) -> list:
+        return [p._version for p in self.params]
+
+
+def supported(model) -> bool:
+    """Whether the parameters are what the kernels read: float32, contiguous, on one GPU, one projection per head."""
+    enc = model.encoder
+    ff = enc.layers[0].linear1.out_features if len(enc.layers) else 0
+    hidden = model.mlp[0].out_features
+    dev = model.input_embeddings.weight.device
+    if dev.type != "cuda" or not 1 <= len(enc.layers) <= 32 or ff % 128 or not 0 < ff <= 3328 or hidden % 128 \
+            or not 0 < hidden <= 1024 or model.input_embeddings.in_features > 128:
+        return False
+    for layer in enc.layers:
+        att = layer.self_attn
+        if layer.linear1.out_features != ff or att.params.value_pe_dist_real not in (0, 64) or att.params.gauss_lb_real <= 0 \
+                or att.out_proj.bias is None or (att.pe_dist_proj is not None and tuple(att.pe_dist_proj.shape) != (1, 8, 16, 64)) \
+                or (att.pe_dist_proj is None) != (att.params.value_pe_dist_real == 0):
+            return False
+        if any(isinstance(m, torch.nn.Dropout) and m.p > 0 for m in (layer.dropout, layer.dropout1, layer.dropout2)) or att.dropout > 0:
+            return False
+    return all(p.dtype == torch.float32 and p.is_contiguous() and p.device == dev for p in model.parameters())
+
+
+class TrainStep(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, plan: TrainPlan, inputs, counts: Tuple[int, int, int], *params):
+        feats, pos, trans, sizes = inputs
+        dev = pos.device
+        N, E, max_atoms = (int(c) for c in counts)
+        B = sizes.shape[0]
+        lib = _lib.load()
+        nbytes = int(lib.cf_train_saved_bytes(ctypes.byref(plan.desc), N, B, E))
+        saved = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        batch = _lib.TrainBatch(features=feats.data_ptr(), pos=pos.data_ptr(), trans=trans.data_ptr(), sizes=sizes.data_ptr(), N=N, B=B,
+                                E=E, max_atoms=max_atoms, saved=saved.data_ptr())
+        y = torch.empty((B, plan.targets), dtype=torch.float32, device=dev)
+        with torch.cuda.device(dev):
+            _lib.call("cf_train_forward", ctypes.byref(plan.desc), ctypes.byref(batch), y.data_ptr(),
+                      torch.cuda.current_stream(dev).cuda_stream)
+        ctx.save_for_backward(saved, feats, pos, trans, sizes)
+        ctx.step = (plan, batch, plan.versions())
+        return y
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, gy):
+        plan, batch, versions = ctx.step
+        keep = ctx.saved_tensors  # (the memory `batch` points into; released with the graph)
+        if plan.versions() != versions:
+            raise RuntimeError("a parameter of the model was modified by an in-place operation between the forward and the "
+                               "backward of a training step")
+        dev = gy.device
+        gy = gy.contiguous()
+        scratch = torch.empty(int(_lib.load().cf_train_scratch_bytes(ctypes.byref(plan.desc), batch.N, batch.B, batch.E)),
+                              dtype=torch.uint8, device=dev)
+        flat = torch.empty(plan.floats, dtype=torch.float32, device=dev)
+        base = flat.data_ptr()
+        where = (ctypes.c_void_p * len(plan.slots))(*[None if s is None else base + 4 * plan.offsets[s] for s in plan.slots])
+        with torch.cuda.device(dev):
+            _lib.call("cf_train_backward", ctypes.byref(plan.desc), ctypes.byref(batch), gy.data_ptr(), scratch.data_ptr(),
+                      ctypes.cast(where, ctypes.c_void_p), torch.cuda.current_stream(dev).cuda_stream)
+        del keep
+        return (None, None, None, *[flat[at:at + n].view(shape) for at, n, shape in plan.spans])
+
+
+def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[torch.Tensor]:
+    """The model's output on ``data`` with the step's autograd node behind it, or None when the calls do not apply."""
+    plan = getattr(model, "_train_plan", None)
+    if plan is None or not plan.current():
+        if not supported(model):
+            return None
+        plan = model._train_plan = TrainPlan(model)
+    if not all(layer.self_attn.term_lists for layer in model.encoder.layers):
+        return None
+    if any(t.requires_grad for t in (data.x, data.pos, data.trans_vec)) or torch.is_autocast_enabled():
+        return None
+    f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()
+    feats, pos, trans = f32(data.x), f32(data.pos), f32(data.trans_vec)
+    dev = pos.device
+    sizes = data.sizes
+    if sizes.device != dev or sizes.dtype != torch.int64 or not sizes.is_contiguous():
+        sizes = sizes.to(device=dev, dtype=torch.int64).contiguous()
+    if counts is None:
+        host = data.sizes.tolist()
+        counts = (sum(host), sum(n * n for n in host), max(host) if host else 1)
+    if counts[0] < 1 or counts[2] > 1024 or feats.data_ptr() % 16 or plan.params[0].device != dev:
+        return None
+    return TrainStep.apply(plan, (feats, pos, trans, sizes), counts, *plan.params)

@@ -1,0 +1,76 @@
+"""The training step in two library calls (crystalformer_b200.training) against the autograd path of the same model."""
+import copy
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from crystalformer_b200.synthetic import make_crystals
+
+pytestmark = pytest.mark.gpu
+
+
+def step(model, data, target, native):
+    model.native = native
+    for p in model.parameters():
+        p.grad = None
+    y = model(data)
+    (y - target).abs().mean().backward()
+    return y.detach(), {n: p.grad for n, p in model.named_parameters() if p.requires_grad}
+
+
+def setup(sizes, lengths=(4.0, 12.0), **params):
+    from crystalformer_b200.model import Latticeformer, default_params
+    torch.manual_seed(len(sizes))
+    model = Latticeformer(default_params(**params)).cuda().train()
+    for p in model.parameters():
+        if p.requires_grad:
+            p.data.add_(torch.randn_like(p) * 0.02)
+    cb = make_crystals(5, len(sizes), lambda rng, b: np.array(sizes), length_range=lengths)
+    t = lambda x: torch.as_tensor(x).cuda()
+    data = types.SimpleNamespace(x=t(cb.x), pos=t(cb.pos), trans_vec=t(cb.trans_vec), sizes=t(cb.sizes))
+    with torch.no_grad():
+        model(data)  # sets the width statistics
+    return model, data, torch.randn((len(sizes), model.mlp[3].out_features), device="cuda")
+
+
+@pytest.mark.parametrize("params", [dict(num_layers=2), dict(num_layers=3, value_pe_dist_real=0), dict(num_layers=1, ff_dim=128),
+                                    dict(num_layers=2, ff_dim=256, targets=["a", "b", "c"], embedding_dim=[256])])
+@pytest.mark.parametrize("sizes", [[1], [3, 60, 64], [33] * 4 + [1], [100, 128, 129], [7] * 130])
+def test_gradients_equal_the_autograd_path(params, sizes):
+    """Row tiles of 128 (one row, a full tile, one more), chunks of 64 rows, crystals of one atom and of more than 64."""
+    model, data, target = setup(sizes, lengths=(8.0, 14.0) if max(sizes) > 64 else (4.0, 12.0), **params)
+    y0, ref = step(model, data, target, native=False)
+    y1, got = step(model, data, target, native=True)
+    assert getattr(model, "_train_plan", None) is not None
+    assert (y0 - y1).abs().max() < 2e-6
+    for name in ref:
+        scale = ref[name].norm()
+        # a hidden unit within rounding of zero may fall on either side of the ReLU: one column of one gradient moves
+        assert (got[name] - ref[name]).norm() <= 2e-3 * scale + 1e-9, (name, float((got[name] - ref[name]).norm() / scale))
+    again = step(model, data, target, native=True)[1]
+    assert all(torch.equal(got[n], again[n]) for n in got)  # no atomics in any sum
+
+
+def test_step_follows_the_model():
+    """In-place updates, replaced parameters, copies and frozen parameters; a modified weight between the two halves."""
+    model, data, target = setup([9, 20, 5], num_layers=2)
+    step(model, data, target, native=True)
+    with torch.no_grad():
+        for p in model.parameters():
+            if p.requires_grad:
+                p.sub_(0.01 * p.grad)
+    model.mlp[3].weight = torch.nn.Parameter(model.mlp[3].weight.detach() * 1.5)
+    model.encoder.layers[0].linear1.weight.requires_grad_(False)
+    clone = copy.deepcopy(model)
+    for m in (model, clone):
+        ref, got = step(m, data, target, native=False)[1], step(m, data, target, native=True)[1]
+        assert "encoder.layers.0.linear1.weight" not in got
+        for name in ref:
+            assert (got[name] - ref[name]).norm() <= 2e-3 * ref[name].norm() + 1e-9, name
+    loss = model(data).sum()
+    with torch.no_grad():
+        model.mlp[0].bias.add_(1.0)
+    with pytest.raises(RuntimeError, match="in-place"):
+        loss.backward()
