@@ -22,6 +22,8 @@ SIGNATURES = {
     "cf_lattice_box": [P, I32, P, P, I64, I64, I64, P, F64, I32, I32, P, P],
     "cf_lattice_sum_fwd": [P, I32, P, P, P, P, I64, I64, I64, I64, F64, F64, P, I64, I64, P, F64, I32, I32, P, P, P],
     "cf_lattice_sum_bwd": [P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, F64, F64, P, F64, I32, I32, P, P, P, P],
+    "cf_lattice_sum_bwd_proj_floats": [I64],
+    "cf_lattice_sum_bwd_proj": [P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, F64, F64, P, F64, I32, I32, P, P, P, P],
     "cf_lattice_sum_bwd_static": [P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, F64, F64, P, F64, I32, I32, P, P, P],
     "cf_fused_attn_fwd": [P, P, P, P, P, P, P, I64, I64, I64, I64, P, P, P],
     "cf_fused_attn_bwd": [P, P, P, P, P, P, I64, I64, I64, I64, P, P, P, P, P, P, P, P, P],
@@ -155,7 +157,7 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
-        for name in ("cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_scratch_bytes"):
+        for name in ("cf_lattice_sum_bwd_proj_floats", "cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_scratch_bytes"):
             getattr(lib, name).restype = c_int64
         _lib = lib
     return _lib

@@ -1,14 +1,12 @@
 // Real-space lattice sum, forward: phi (E,H) and psi (E,H,K) or W psi (E,H,16) per edge.
 //
-// Two kernels (building blocks in lattice_core.cuh):
-//   lattice_phi_kernel   one thread per edge, all eight heads: z = log sum_n exp(a |r + n.T|^2).  MUFU-bound.
-//   lattice_psi_kernel   one warp per edge: the radial-basis expansion psi, with the Gaussian weights already
-//                        normalised by z, so no second reduction is needed.  The reference gives every (edge, head)
-//                        its own thread and so repeats the geometry and the 64 basis exponentials eight times; here
-//                        they are evaluated once per (edge, translation) and shared by the heads.
+// lattice_edge_kernel: one warp per edge, phi and psi from one walk over the box (building blocks in lattice_edge.cuh and
+// lattice_core.cuh).  The reference gives every (edge, head) its own thread and so repeats the geometry and the 64 basis
+// exponentials eight times; here they are evaluated once per (edge, translation) and shared by the heads.
+// lattice_phi_kernel: one thread per edge, phi alone; serves the fused attention where no term lists exist.
 // The box of a head follows the reference rule exactly; heads of one edge may have different boxes, in which case
 // the union box is enumerated and each head masks the translations outside its own.
-#include "lattice_core.cuh"
+#include "lattice_edge.cuh"
 
 namespace cf {
 
@@ -18,7 +16,6 @@ constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr int PSI_STRIDE = 68;                            // floats per head row of the per-warp psi tile (bank skew)
 constexpr int WT_HEAD_STRIDE = 64 * HEAD_DIM + 16;        // floats per head of the transposed projection (bank skew)
-constexpr int WARP_SMEM_FLOATS = STAGE_FLOATS + 8 * PSI_STRIDE;
 
 struct FwdArgs {
     const float *a;
@@ -34,48 +31,56 @@ struct FwdArgs {
     BoxRule rule;
     BasisParams basis;
     int a_per_edge;
-    int stage_w;      // 1: W (1,H,16,K) is staged transposed in shared memory
 };
 
-// out[h][4 mq .. 4 mq + 3] = sum_k W[h][m][k] psi[h][k] for the lane's (h, mq); psi in shared memory.
-template <int K, bool STAGED>
+// out[h][4 mq .. 4 mq + 3] = sum_k W[h][m][k] psi[h][k] for the lane's (h, mq), W in global memory, psi in shared memory.
+template <int K>
 __device__ __forceinline__ float4 project(const float *__restrict__ Wsrc, const float *__restrict__ psi, int lane)
 {
     const int h = lane >> 2, mq = lane & 3;
     float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
     const float *ps = psi + h * PSI_STRIDE;
-    if (STAGED) {
-        const float *wt = Wsrc + h * WT_HEAD_STRIDE + 4 * mq;  // [k][m]
-#pragma unroll 4
-        for (int k = 0; k < K; k += 4) {
-            const float4 pv = *reinterpret_cast<const float4 *>(ps + k);
-            const float4 w0 = *reinterpret_cast<const float4 *>(wt + (k + 0) * HEAD_DIM);
-            const float4 w1 = *reinterpret_cast<const float4 *>(wt + (k + 1) * HEAD_DIM);
-            const float4 w2 = *reinterpret_cast<const float4 *>(wt + (k + 2) * HEAD_DIM);
-            const float4 w3 = *reinterpret_cast<const float4 *>(wt + (k + 3) * HEAD_DIM);
-            o0 = fmaf(w0.x, pv.x, o0); o1 = fmaf(w0.y, pv.x, o1); o2 = fmaf(w0.z, pv.x, o2); o3 = fmaf(w0.w, pv.x, o3);
-            o0 = fmaf(w1.x, pv.y, o0); o1 = fmaf(w1.y, pv.y, o1); o2 = fmaf(w1.z, pv.y, o2); o3 = fmaf(w1.w, pv.y, o3);
-            o0 = fmaf(w2.x, pv.z, o0); o1 = fmaf(w2.y, pv.z, o1); o2 = fmaf(w2.z, pv.z, o2); o3 = fmaf(w2.w, pv.z, o3);
-            o0 = fmaf(w3.x, pv.w, o0); o1 = fmaf(w3.y, pv.w, o1); o2 = fmaf(w3.z, pv.w, o2); o3 = fmaf(w3.w, pv.w, o3);
-        }
-    } else {
-        const float *w = Wsrc + (size_t)(h * HEAD_DIM + 4 * mq) * K;  // [m][k], global memory
+    const float *w = Wsrc + (size_t)(h * HEAD_DIM + 4 * mq) * K;  // [m][k]
 #pragma unroll 2
-        for (int k = 0; k < K; k += 4) {
-            const float4 pv = *reinterpret_cast<const float4 *>(ps + k);
-            const float4 w0 = __ldg(reinterpret_cast<const float4 *>(w + 0 * K + k));
-            const float4 w1 = __ldg(reinterpret_cast<const float4 *>(w + 1 * K + k));
-            const float4 w2 = __ldg(reinterpret_cast<const float4 *>(w + 2 * K + k));
-            const float4 w3 = __ldg(reinterpret_cast<const float4 *>(w + 3 * K + k));
-            o0 += w0.x * pv.x + w0.y * pv.y + w0.z * pv.z + w0.w * pv.w;
-            o1 += w1.x * pv.x + w1.y * pv.y + w1.z * pv.z + w1.w * pv.w;
-            o2 += w2.x * pv.x + w2.y * pv.y + w2.z * pv.z + w2.w * pv.w;
-            o3 += w3.x * pv.x + w3.y * pv.y + w3.z * pv.z + w3.w * pv.w;
-        }
+    for (int k = 0; k < K; k += 4) {
+        const float4 pv = *reinterpret_cast<const float4 *>(ps + k);
+        const float4 w0 = __ldg(reinterpret_cast<const float4 *>(w + 0 * K + k));
+        const float4 w1 = __ldg(reinterpret_cast<const float4 *>(w + 1 * K + k));
+        const float4 w2 = __ldg(reinterpret_cast<const float4 *>(w + 2 * K + k));
+        const float4 w3 = __ldg(reinterpret_cast<const float4 *>(w + 3 * K + k));
+        o0 += w0.x * pv.x + w0.y * pv.y + w0.z * pv.z + w0.w * pv.w;
+        o1 += w1.x * pv.x + w1.y * pv.y + w1.z * pv.z + w1.w * pv.w;
+        o2 += w2.x * pv.x + w2.y * pv.y + w2.z * pv.z + w2.w * pv.w;
+        o3 += w3.x * pv.x + w3.y * pv.y + w3.z * pv.z + w3.w * pv.w;
     }
     return make_float4(o0, o1, o2, o3);
 }
 
+// The same for GROUP tiles at once with W staged as wt[h][k][m].
+template <int K>
+__device__ __forceinline__ void project_group(const float *__restrict__ wt_all, const float *__restrict__ psi, int lane, float4 (&o)[4])
+{
+    const int h = lane >> 2, mq = lane & 3;
+    const float *wt = wt_all + h * WT_HEAD_STRIDE + 4 * mq;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        float4 w[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) w[t] = *reinterpret_cast<const float4 *>(wt + (k + t) * HEAD_DIM);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float4 pv = *reinterpret_cast<const float4 *>(psi + (u * 8 + h) * PSI_STRIDE + k);
+            const float ps[4] = {pv.x, pv.y, pv.z, pv.w};
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                o[u].x = fmaf(w[t].x, ps[t], o[u].x); o[u].y = fmaf(w[t].y, ps[t], o[u].y);
+                o[u].z = fmaf(w[t].z, ps[t], o[u].z); o[u].w = fmaf(w[t].w, ps[t], o[u].w);
+            }
+        }
+    }
+}
 
 template <int TPE>
 __global__ void __launch_bounds__(128) lattice_phi_kernel(const PhiArgs p)
@@ -111,16 +116,25 @@ __global__ void __launch_bounds__(128) lattice_phi_kernel(const PhiArgs p)
     }
 }
 
-template <int K>
-__global__ void __launch_bounds__(THREADS, 5) lattice_psi_kernel(const FwdArgs p)
+// One warp per edge: phi and, with K > 0, the radial-basis expansion (MODE: as psi; projected with one W staged in shared
+// memory, four edges at a time; projected with a W per edge or atom).  Weights are taken relative to the nearest image,
+//     w_n = exp(a (d2_n - m)),   phi = a m + log sum w_n,   psi = sum w_n g(d_n) / sum w_n,
+// so one walk over the box gives both (an edge whose sum comes out empty - a head whose box misses the nearest image by
+// far - is repeated with the normaliser of that head's own minimum).
+enum { AS_PSI = 0, ONE_W = 1, MANY_W = 2 };
+constexpr int GROUP = 4;  // edges projected together: W is read from shared memory once for all of them
+
+template <int K, int MODE>
+__global__ void __launch_bounds__(THREADS, K == 0 ? 6 : 4) lattice_edge_kernel(const FwdArgs p)
 {
     extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int TILES = K == 0 ? 0 : MODE == ONE_W ? GROUP : 1;
+    constexpr int WARP_FLOATS = EDGE_TERM_FLOATS + (K > 0 ? STAGE_FLOATS : 0) + TILES * 8 * PSI_STRIDE;
     float *wt = smem;
-    float *mine = smem + (p.stage_w ? HEADS * WT_HEAD_STRIDE : 0) + warp * WARP_SMEM_FLOATS;
-    float *psi = mine + STAGE_FLOATS;
-
-    if (p.stage_w) {
+    float *mine = smem + (MODE == ONE_W ? HEADS * WT_HEAD_STRIDE : 0) + warp * WARP_FLOATS;
+    float *psi = mine + EDGE_TERM_FLOATS + STAGE_FLOATS;
+    if (MODE == ONE_W) {
         // W[h][m][k] -> wt[h][k][m] so that a lane reads its four outputs' weights as one float4
         for (int idx = threadIdx.x; idx < HEADS * HEAD_DIM * K; idx += THREADS) {
             const int h = idx / (HEAD_DIM * K), m = (idx / K) % HEAD_DIM, k = idx % K;
@@ -129,81 +143,150 @@ __global__ void __launch_bounds__(THREADS, 5) lattice_psi_kernel(const FwdArgs p
         __syncthreads();
     }
     BinAccumulator<K> bins;
-    bins.init(mine, lane, p.basis);
+    if (K > 0) bins.init(mine + EDGE_TERM_FLOATS, lane, p.basis);
+    EdgeTerms terms;
+    terms.buf = reinterpret_cast<float2 *>(mine); terms.count = 0; terms.lane = lane;
+    BoxWalk w5;
+    w5.init(lane);
+    EdgeStream es;
+    es.a = p.a; es.pos_ij = p.pos_ij; es.tvecs = p.tvecs; es.rvlen = p.rvlen; es.batch = p.batch; es.edges = p.edges;
+    es.E = p.E; es.a_per_edge = p.a_per_edge;
+    const long long stride = (long long)gridDim.x * WARPS;
+    es.begin((long long)blockIdx.x * WARPS + warp, stride, lane);
+    long long group_e[GROUP];
+    float group_inv[GROUP];
+    int in_group = 0;
 
-    for (long long e = (long long)blockIdx.x * WARPS + warp; e < p.E; e += (long long)gridDim.x * WARPS) {
-        const long long i = p.edges[e];
-        const long long c = p.batch[i];
-        const float rx = p.pos_ij[3 * e], ry = p.pos_ij[3 * e + 1], rz = p.pos_ij[3 * e + 2];
+    for (; es.e < p.E; es.next()) {
         Cell cell;
-        cell.load(p.tvecs + 9 * c);
-
-        // lanes 0..7 (and their copies) hold head (lane & 7): its width, its box and the log-normaliser from phi
-        const float a_own = p.a[(p.a_per_edge ? e : i) * HEADS + (lane & 7)];
-        const float z_own = p.z[e * HEADS + (lane & 7)];
-        const int pk_own = packed_box(p.rule, a_own, p.rvlen ? p.rvlen + 3 * c : nullptr);
+        float rx, ry, rz, rvl[3];
+        es.unpack(cell, rx, ry, rz, rvl);
+        const float a_own = es.a_own;
+        const int pk_own = packed_box(p.rule, a_own, p.rvlen ? rvl : nullptr);
         int uni = pk_own;
+        float a2max = a_own;
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) uni = box_union(uni, __shfl_xor_sync(FULL, uni, o));
+        for (int o = 4; o > 0; o >>= 1) {
+            uni = box_union(uni, __shfl_xor_sync(FULL, uni, o));
+            a2max = fmaxf(a2max, __shfl_xor_sync(FULL, a2max, o));
+        }
+        a2max *= LOG2E;
         const bool masked = !__all_sync(FULL, pk_own == uni);
-        float a2[8], off[8];
+        float a2[8];
         int pk[8];
 #pragma unroll
         for (int h = 0; h < 8; ++h) {
             a2[h] = __shfl_sync(FULL, a_own, h) * LOG2E;
-            off[h] = -__shfl_sync(FULL, z_own, h) * LOG2E;
             pk[h] = __shfl_sync(FULL, pk_own, h);
         }
-        const int R1 = box_r1(uni), R2 = box_r2(uni), R3 = box_r3(uni);
-        const int count = (2 * R1 + 1) * (2 * R2 + 1) * (2 * R3 + 1);
-        TermWalker walk;
-        walk.init(R1, R2, R3, (unsigned)lane);
-        const float F1 = (float)R1, F2 = (float)R2, F3 = (float)R3;
-        bins.clear();
-        for (int base = 0; base < count; base += 32) {
-            const bool valid = base + lane < count;
-            const float f1 = walk.u1 - F1, f2 = walk.u2 - F2, f3 = walk.u3 - F3;
-            const float dx = fmaf(cell.t3x, f3, fmaf(cell.t2x, f2, fmaf(cell.t1x, f1, rx)));
-            const float dy = fmaf(cell.t3y, f3, fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, ry)));
-            const float dz = fmaf(cell.t3z, f3, fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, rz)));
-            const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-            int i1 = 0, i2 = 0, i3 = 0;
-            if (masked) {
-                i1 = abs(__float2int_rn(f1)); i2 = abs(__float2int_rn(f2)); i3 = abs(__float2int_rn(f3));
-            }
+        // ---- nearest image of the union box, then the terms whose largest weight is above the floor
+        float S[8];
+#pragma unroll
+        for (int h = 0; h < 8; ++h) S[h] = 0.f;
+        if (K > 0) bins.clear();
+        float m = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
+        auto weigh = [&](bool got, float d2, int key) {
+            const float rel = d2 - m;
             float w[8];
-            float emax = -INFINITY;
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
-                float eh = fmaf(a2[h], d2, off[h]);
-                if (masked && !(i1 <= box_r1(pk[h]) && i2 <= box_r2(pk[h]) && i3 <= box_r3(pk[h]))) eh = -INFINITY;
-                w[h] = ex2(eh);
-                emax = fmaxf(emax, eh);
+                w[h] = ex2(a2[h] * rel);
+                if (!got || (masked && !key_in_box(key, pk[h]))) w[h] = 0.f;
+                S[h] += w[h];
             }
-            const float x = fast_sqrt(d2) * p.basis.bin_scale;
-            bins.push(valid && emax > p.basis.floor_log2 && d2 < p.basis.d2_cut, x, w);
-            walk.step();
+            if (K > 0) bins.push(got && d2 < p.basis.d2_cut, fast_sqrt(d2) * p.basis.bin_scale, w);
+        };
+        if (uni == BOX222) {
+            float d2v[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                d2v[b] = term_d2(cell, rx, ry, rz, w5.f1[b], w5.f2[b], w5.f3[b]);
+                if (b == 3 && lane >= 29) d2v[b] = INFINITY;
+                m = fminf(m, d2v[b]);
+            }
+            m = warp_min(m);
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                terms.add(a2max * (d2v[b] - m) > p.basis.floor_log2, d2v[b], masked ? term_key(w5.f1[b], w5.f2[b], w5.f3[b]) : 0);
+        } else {
+            walk_box(w5, uni, cell, rx, ry, rz, lane,
+                     [&](bool valid, float d2, float, float, float) { m = valid ? fminf(m, d2) : m; }, []() {});
+            m = warp_min(m);
+            walk_box(w5, uni, cell, rx, ry, rz, lane,
+                     [&](bool valid, float d2, float f1, float f2, float f3) {
+                         terms.add(valid && a2max * (d2 - m) > p.basis.floor_log2, d2, masked ? term_key(f1, f2, f3) : 0);
+                     },
+                     [&]() { if (terms.count >= 32) terms.consume(false, weigh); });
         }
-
-        bins.flush(psi, PSI_STRIDE);
-        if (p.W == nullptr) {
-            float *dst = p.v + (size_t)e * HEADS * K + lane;
+        terms.consume(true, weigh);
+        const int g = lane >> 2;
+        const float S_g = warp_sum_of_8(S, lane), a_g = __shfl_sync(FULL, a_own, g);
+        const int pk_g = __shfl_sync(FULL, pk_own, g);
+        float z_g = fmaf(m, a_g, logf(S_g)), inv_g = __frcp_rn(S_g);
+        if (__any_sync(FULL, !(S_g > 1e-30f))) {
+            // a head's box misses the nearest image by hundreds of square Angstrom: phi from its own minimum, and the
+            // expansion once more with normalised weights
+            if (!(S_g > 1e-30f)) z_g = head_phi_own_min(cell, rx, ry, rz, a_g, pk_g);
+            if (K > 0) {
+                float off[8];
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                dst[h * K] = psi[h * PSI_STRIDE + lane];
-                dst[h * K + 32] = psi[h * PSI_STRIDE + lane + 32];
+                for (int h = 0; h < 8; ++h) off[h] = -__shfl_sync(FULL, z_g, 4 * h) * LOG2E;
+                bins.clear();
+                auto again = [&](bool got, float d2, int key) {
+                    float w[8], top = -INFINITY;
+#pragma unroll
+                    for (int h = 0; h < 8; ++h) {
+                        float eh = fmaf(a2[h], d2, off[h]);
+                        if (!got || !key_in_box(key, pk[h])) eh = -INFINITY;
+                        w[h] = ex2(eh);
+                        top = fmaxf(top, eh);
+                    }
+                    bins.push(top > p.basis.floor_log2 && d2 < p.basis.d2_cut, fast_sqrt(d2) * p.basis.bin_scale, w);
+                };
+                walk_box(w5, uni, cell, rx, ry, rz, lane,
+                         [&](bool valid, float d2, float f1, float f2, float f3) { terms.add(valid, d2, term_key(f1, f2, f3)); },
+                         [&]() { if (terms.count >= 32) terms.consume(uni == BOX222, again); });
+                terms.consume(true, again);
+                inv_g = 1.0f;
             }
+        }
+        if ((lane & 3) == 0) p.z[es.e * HEADS + g] = z_g;
+        if (K == 0) continue;
+        if (MODE == AS_PSI) {
+            bins.flush(psi, PSI_STRIDE);
+            float4 *dst = reinterpret_cast<float4 *>(p.v + (size_t)es.e * HEADS * K) + lane;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {  // float4 lane + 32 t of the 8 x 64 block: head 2 t + lane / 16
+                const int h = 2 * t + (lane >> 4);
+                const float inv = __shfl_sync(FULL, inv_g, 4 * h);
+                float4 v = *reinterpret_cast<const float4 *>(psi + h * PSI_STRIDE + 4 * (lane & 15));
+                v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+                dst[32 * t] = v;
+            }
+            __syncwarp();
+        } else if (MODE == MANY_W) {
+            bins.flush(psi, PSI_STRIDE);
+            const long long wi = p.W_num == p.E ? es.e : es.i;
+            float4 o = project<K>(p.W + (size_t)wi * HEADS * HEAD_DIM * K, psi, lane);  // (lane = head lane / 4)
+            o.x *= inv_g; o.y *= inv_g; o.z *= inv_g; o.w *= inv_g;
+            reinterpret_cast<float4 *>(p.v + (size_t)es.e * HEADS * HEAD_DIM)[lane] = o;
             __syncwarp();
         } else {
-            float4 o;
-            if (p.stage_w) {
-                o = project<K, true>(wt, psi, lane);
-            } else {
-                const long long wi = (p.W_num == 1) ? 0 : (p.W_num == p.E ? e : i);
-                o = project<K, false>(p.W + (size_t)wi * HEADS * HEAD_DIM * K, psi, lane);
+            bins.flush(psi + in_group * 8 * PSI_STRIDE, PSI_STRIDE);
+#pragma unroll
+            for (int u = 0; u < GROUP; ++u)
+                if (u == in_group) { group_e[u] = es.e; group_inv[u] = inv_g; }
+            if (++in_group == GROUP || es.e + stride >= p.E) {
+                float4 o[GROUP];
+                project_group<K>(wt, psi, lane, o);
+#pragma unroll
+                for (int u = 0; u < GROUP; ++u)
+                    if (u < in_group)
+                        reinterpret_cast<float4 *>(p.v + (size_t)group_e[u] * HEADS * HEAD_DIM)[lane] =
+                            make_float4(o[u].x * group_inv[u], o[u].y * group_inv[u], o[u].z * group_inv[u], o[u].w * group_inv[u]);
+                in_group = 0;
+                __syncwarp();
             }
-            reinterpret_cast<float4 *>(p.v + (size_t)e * HEADS * HEAD_DIM)[lane] = o;
-            __syncwarp();
         }
     }
 }
@@ -227,25 +310,21 @@ __global__ void lattice_box_kernel(const float *a, int a_per_edge, const int64_t
 
 int launch_fwd(const FwdArgs &p, long long K, cudaStream_t stream)
 {
-    PhiArgs phi{};
-    phi.a = p.a; phi.pos_ij = p.pos_ij; phi.tvecs = p.tvecs; phi.batch = p.batch; phi.edges = p.edges;
-    phi.rvlen = p.rvlen; phi.z = p.z; phi.E = p.E; phi.rule = p.rule; phi.a_per_edge = p.a_per_edge;
-    phi.floor_log2 = p.basis.floor_log2;
-    launch_lattice_phi(phi, stream);
-    if (K > 0) {
-        const size_t smem = sizeof(float) * ((p.stage_w ? HEADS * WT_HEAD_STRIDE : 0) + WARPS * WARP_SMEM_FLOATS);
-        static thread_local int per_sm[2] = {0, 0};
-        int &occ = per_sm[p.stage_w ? 1 : 0];
-        if (occ == 0) {
-            cudaFuncSetAttribute(lattice_psi_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(float) * (HEADS * WT_HEAD_STRIDE + WARPS * WARP_SMEM_FLOATS)));
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lattice_psi_kernel<64>, THREADS, smem) != cudaSuccess || occ <= 0)
-                occ = 4;
-        }
-        const long long want = (p.E + WARPS - 1) / WARPS;
-        const long long cap = (long long)sm_count() * occ;
-        lattice_psi_kernel<64><<<(int)(want < cap ? want : cap), THREADS, smem, stream>>>(p);
+    const int mode = K == 0 ? 3 : p.W == nullptr ? AS_PSI : p.W_num == 1 ? ONE_W : MANY_W;
+    void (*const kernels[4])(const FwdArgs) = {lattice_edge_kernel<64, AS_PSI>, lattice_edge_kernel<64, ONE_W>,
+                                               lattice_edge_kernel<64, MANY_W>, lattice_edge_kernel<0, AS_PSI>};
+    const int tiles = mode == 3 ? 0 : mode == ONE_W ? GROUP : 1;
+    const size_t smem = sizeof(float) * ((mode == ONE_W ? HEADS * WT_HEAD_STRIDE : 0) +
+                                         WARPS * (EDGE_TERM_FLOATS + (K > 0 ? STAGE_FLOATS : 0) + tiles * 8 * PSI_STRIDE));
+    static thread_local int per_sm[4] = {0, 0, 0, 0};
+    int &occ = per_sm[mode];
+    if (occ == 0) {
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kernels[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernels[mode], THREADS, smem) != cudaSuccess || occ <= 0) occ = 2;
     }
+    const long long want = (p.E + WARPS - 1) / WARPS;
+    const long long cap = (long long)sm_count() * occ;
+    kernels[mode]<<<(int)(want < cap ? want : cap), THREADS, smem, stream>>>(p);
     return launch_status("cf_lattice_sum_fwd");
 }
 
@@ -318,6 +397,5 @@ extern "C" int cf_lattice_sum_fwd(const float *a, int a_per_edge, const float *p
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     p.a_per_edge = a_per_edge;
     p.basis = make_basis_params(K, dist_max, wscale, weight_floor_log2());
-    p.stage_w = (p.W != nullptr && W_num == 1) ? 1 : 0;
     return launch_fwd(p, K, as_stream(stream));
 }

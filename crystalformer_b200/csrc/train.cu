@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(512) pe_grad_kernel(const PeArgs p)
                 }
             }
         }
-        if (tid < CH)
+        if (tid < CH && q != nullptr)
             for (int r = 0; r < rows; ++r) wpos = fmaf(galpha[(n0 + r) * HEADS + (tid >> 4)], 4.0f * q[(n0 + r) * CH + tid], wpos);
     }
     float *out = p.partial + ((size_t)l * p.shares + blockIdx.x) * PE_PARTIAL;
@@ -158,7 +158,13 @@ __global__ void __launch_bounds__(256) pe_grad_sum_kernel(const PeArgs p, int wi
 #pragma unroll 4
     for (int sh = 0; sh < p.shares; ++sh) t += in[(size_t)sh * PE_PARTIAL];
     if (idx < CH * 64) p.gW[l][idx] = t;
-    else p.gwpos[l][idx - CH * 64] = t;
+    else if (p.gwpos[l] != nullptr) p.gwpos[l][idx - CH * 64] = t;
+}
+
+int projection_shares(long long rows)
+{
+    const long long most = (rows + PE_ROWS - 1) / PE_ROWS, cap = 2ll * sm_count();
+    return (int)(most < 1 ? 1 : most < cap ? most : cap);
 }
 
 // ---- memory ----------------------------------------------------------------------------------------------------------------
@@ -310,6 +316,20 @@ bool lists_of(const cf_train_desc &d, const Saved &s, int64_t N, int64_t E, Term
 }
 
 }  // namespace
+}  // namespace cf
+
+namespace cf {
+// gW[h][m][k] = sum over rows of gv[row][h][m] psi[row][h][k] (the drop-in operator's projection gradient, rows = edges).
+size_t projection_grad_floats(long long rows) { return (size_t)projection_shares(rows) * PE_PARTIAL; }
+int launch_projection_grad(const float *gv, const float *psi, long long rows, float *gW, float *partial, cudaStream_t s)
+{
+    PeArgs pe{};
+    pe.gattn[0] = gv; pe.psi[0] = psi; pe.gW[0] = gW;
+    pe.N = rows; pe.shares = projection_shares(rows); pe.partial = partial;
+    pe_grad_kernel<true><<<dim3(pe.shares, 1), 512, 0, s>>>(pe);
+    pe_grad_sum_kernel<<<dim3((CH * 64 + 255) / 256, 1), 256, 0, s>>>(pe, 1);
+    return launch_status("projection gradient");
+}
 }  // namespace cf
 
 extern "C" int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E)

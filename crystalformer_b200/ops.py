@@ -149,8 +149,8 @@ def lattice_sum_fwd(a, pos_ij, tvecs, batch, edges, K, dist_max, wscale, W=None,
 def lattice_sum_bwd(a, pos_ij, tvecs, batch, edges, row_start, z, gz, gv, K, dist_max, wscale, W=None, rvlen=None,
                     cutoff_radius=0.0, lattice_range=2, minimum_range=2):
     """ga (N,H) and gW (shape of W; None without W).  gv is the gradient of psi (E,H,K) when W is None, else of
-    W psi (E,H,Dv).  The projection is handled around the kernel with two GEMM-shaped torch calls:
-    gpsi = W^T gv before it, gW = sum_e gv_e (x) psi_e after it (psi recomputed by the kernel)."""
+    W psi (E,H,Dv).  With one projection for all edges everything is one library call; projections per edge or atom are
+    handled around the kernel: gpsi = W^T gv before it, gW = gv_e (x) psi_e after it (psi recomputed by the kernel)."""
     dev = a.device
     a = _want(a, torch.float32, "a")
     pos_ij = _want(pos_ij, torch.float32, "pos_ij", dev)
@@ -161,6 +161,16 @@ def lattice_sum_bwd(a, pos_ij, tvecs, batch, edges, row_start, z, gz, gv, K, dis
     W, rvlen = _want(W, torch.float32, "W", dev), _want(rvlen, torch.float32, "rvlen", dev)
     E, H, N = edges.shape[1], a.shape[1], batch.shape[0]
     ga = torch.empty((N, H), dtype=torch.float32, device=dev)
+    if K == 64 and W is not None and W.numel() == H * HEAD_DIM * K and H == HEADS:
+        # one projection for all edges: its parts run inside the call
+        gW = torch.empty(W.shape, dtype=torch.float32, device=dev)
+        work = torch.empty(int(_lib.load().cf_lattice_sum_bwd_proj_floats(E)), dtype=torch.float32, device=dev)
+        with torch.cuda.device(dev):
+            _lib.call("cf_lattice_sum_bwd_proj", _ptr(a), _ptr(pos_ij), _ptr(tvecs), _ptr(batch), _ptr(edges), _ptr(row_start),
+                      _ptr(z), _ptr(gz), _ptr(gv), _ptr(W), c_int64(N), c_int64(H), c_int64(E), c_int64(K), c_double(dist_max),
+                      c_double(wscale), _ptr(rvlen), c_double(cutoff_radius or 0.0), c_int(lattice_range), c_int(minimum_range),
+                      _ptr(ga), _ptr(gW), _ptr(work), _stream(dev))
+        return ga, gW
     scratch = torch.empty((E, H), dtype=torch.float32, device=dev)
     gpsi = psi = None
     if K > 0:
@@ -169,9 +179,7 @@ def lattice_sum_bwd(a, pos_ij, tvecs, batch, edges, row_start, z, gz, gv, K, dis
         else:
             W4 = W if W.dim() == 4 else W[None]
             W_num = W4.shape[0]
-            if W_num == 1:
-                gpsi = torch.einsum("ehd,hdk->ehk", gv, W4[0]).contiguous()
-            elif W_num == E:
+            if W_num == E:
                 gpsi = torch.einsum("ehd,ehdk->ehk", gv, W4).contiguous()
             elif W_num == N:
                 gpsi = torch.einsum("ehd,ehdk->ehk", gv, W4[edges[0]]).contiguous()
@@ -185,15 +193,11 @@ def lattice_sum_bwd(a, pos_ij, tvecs, batch, edges, row_start, z, gz, gv, K, dis
                   c_int(minimum_range), _ptr(ga), _ptr(psi), _ptr(scratch), _stream(dev))
     gW = None
     if psi is not None:
-        if W_num == 1:
-            gW = torch.einsum("ehd,ehk->hdk", gv, psi)[None]
-        elif W_num == E:
+        if W_num == E:
             gW = gv[..., :, None] * psi[..., None, :]
         else:
             gW = torch.zeros((N,) + tuple(W4.shape[1:]), dtype=torch.float32, device=dev)
             gW.index_add_(0, edges[0], gv[..., :, None] * psi[..., None, :])
-        if W.dim() == 3:
-            gW = gW[0]
     return ga, gW
 
 

@@ -150,6 +150,16 @@ int cf_lattice_sum_bwd(const float *a, const float *pos_ij, const float *tvecs, 
                        const float *rvlen, double cutoff_radius, int lattice_range, int minimum_range, float *ga,
                        float *psi_out, float *edge_scratch, void *stream);
 
+/* cf_lattice_sum_bwd with one projection W (8,16,64) shared by all edges, its two GEMM-shaped parts included: gv (E,8,16)
+ * is the gradient of W psi; writes ga (N,8) and gW (8,16,64).  K = 64 only.  workspace:
+ * cf_lattice_sum_bwd_proj_floats(E) floats. */
+int64_t cf_lattice_sum_bwd_proj_floats(int64_t E);
+int cf_lattice_sum_bwd_proj(const float *a, const float *pos_ij, const float *tvecs, const int64_t *batch,
+                            const int64_t *edges, const int64_t *row_start, const float *z, const float *gz,
+                            const float *gv, const float *W, int64_t N, int64_t H, int64_t E, int64_t K, double dist_max,
+                            double wscale, const float *rvlen, double cutoff_radius, int lattice_range, int minimum_range,
+                            float *ga, float *gW, float *workspace, void *stream);
+
 /* ------------------------------------------------------------------------------------------------------------
  * cf_lattice_sum_bwd without a scratch argument.  No counterpart in the reference (its wrappers always allocate
  * their temporaries with torch).
