@@ -100,7 +100,7 @@ __device__ __forceinline__ float term_d2(const Cell &cell, float rx, float ry, f
     return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 
-// Collected terms of a warp: (d2, |n1| | |n2| << 6 | |n3| << 12 as for key_in_box with no key index).
+// Collected terms of a warp: (d2, |n1| | |n2| << 8 | |n3| << 16).
 constexpr int EDGE_TERMS = 128;
 constexpr int EDGE_TERM_FLOATS = 2 * EDGE_TERMS;
 struct EdgeTerms {
@@ -162,7 +162,10 @@ __device__ __forceinline__ void walk_box(const BoxWalk &w5, int uni, const Cell 
 
 __device__ __forceinline__ int term_key(float f1, float f2, float f3)
 {
-    return pack_key(0, abs(__float2int_rn(f1)), abs(__float2int_rn(f2)), abs(__float2int_rn(f3)));
+    return abs(__float2int_rn(f1)) | (abs(__float2int_rn(f2)) << 8) | (abs(__float2int_rn(f3)) << 16);
 }
+// whether a term's digits are all within the box whose packed half-widths are box (boxor = box | 0x808080): byte-wise
+// 128 + R - |n| keeps its top bit exactly when |n| <= R
+__device__ __forceinline__ bool term_in_box(int key, int boxor) { return ((boxor - key) & 0x808080) == 0x808080; }
 
 }  // namespace cf

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(THREADS, 4) lattice_bwd_edges_kernel(const Bwd
         for (int h = 0; h < 8; ++h) {
             a2[h] = __shfl_sync(FULL, a_own, h) * LOG2E;
             off[h] = __shfl_sync(FULL, off_own, h);
-            pk[h] = __shfl_sync(FULL, pk_own, h);
+            pk[h] = __shfl_sync(FULL, pk_own, h) | 0x808080;
         }
         float C0[8], C1[8], C2[8];
 #pragma unroll
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(THREADS, 4) lattice_bwd_edges_kernel(const Bwd
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
                 float eh = fmaf(a2[h], d2, off[h]);
-                if (!got || (masked && !key_in_box(key, pk[h]))) eh = -INFINITY;
+                if (!got || (masked && !term_in_box(key, pk[h]))) eh = -INFINITY;
                 w[h] = ex2(eh);
                 top = fmaxf(top, eh);
                 C1[h] = fmaf(w[h], d2, C1[h]);

@@ -12,8 +12,8 @@ namespace cf {
 
 namespace {
 
-constexpr int THREADS = 128;
-constexpr int WARPS = THREADS / 32;
+enum { AS_PSI = 0, ONE_W = 1, MANY_W = 2 };
+constexpr int GROUP = 2;  // edges projected together: W is read from shared memory once for both
 constexpr int PSI_STRIDE = 68;                            // floats per head row of the per-warp psi tile (bank skew)
 constexpr int WT_HEAD_STRIDE = 64 * HEAD_DIM + 16;        // floats per head of the transposed projection (bank skew)
 
@@ -58,19 +58,19 @@ __device__ __forceinline__ float4 project(const float *__restrict__ Wsrc, const 
 
 // The same for GROUP tiles at once with W staged as wt[h][k][m].
 template <int K>
-__device__ __forceinline__ void project_group(const float *__restrict__ wt_all, const float *__restrict__ psi, int lane, float4 (&o)[4])
+__device__ __forceinline__ void project_group(const float *__restrict__ wt_all, const float *__restrict__ psi, int lane, float4 (&o)[GROUP])
 {
     const int h = lane >> 2, mq = lane & 3;
     const float *wt = wt_all + h * WT_HEAD_STRIDE + 4 * mq;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < GROUP; ++u) o[u] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 2
     for (int k = 0; k < K; k += 4) {
         float4 w[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) w[t] = *reinterpret_cast<const float4 *>(wt + (k + t) * HEAD_DIM);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < GROUP; ++u) {
             const float4 pv = *reinterpret_cast<const float4 *>(psi + (u * 8 + h) * PSI_STRIDE + k);
             const float ps[4] = {pv.x, pv.y, pv.z, pv.w};
 #pragma unroll
@@ -121,12 +121,14 @@ __global__ void __launch_bounds__(128) lattice_phi_kernel(const PhiArgs p)
 //     w_n = exp(a (d2_n - m)),   phi = a m + log sum w_n,   psi = sum w_n g(d_n) / sum w_n,
 // so one walk over the box gives both (an edge whose sum comes out empty - a head whose box misses the nearest image by
 // far - is repeated with the normaliser of that head's own minimum).
-enum { AS_PSI = 0, ONE_W = 1, MANY_W = 2 };
-constexpr int GROUP = 4;  // edges projected together: W is read from shared memory once for all of them
+
+// (the blocks that stage W have eight warps: 16 warps per SM then fit beside two copies of it)
+__host__ __device__ constexpr int edge_warps(int mode) { return mode == ONE_W ? 8 : 4; }
 
 template <int K, int MODE>
-__global__ void __launch_bounds__(THREADS, K == 0 ? 6 : 4) lattice_edge_kernel(const FwdArgs p)
+__global__ void __launch_bounds__(32 * edge_warps(MODE), K == 0 ? 6 : 16 / edge_warps(MODE)) lattice_edge_kernel(const FwdArgs p)
 {
+    constexpr int WARPS = edge_warps(MODE), THREADS = 32 * WARPS;
     extern __shared__ __align__(16) float smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int TILES = K == 0 ? 0 : MODE == ONE_W ? GROUP : 1;
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(THREADS, K == 0 ? 6 : 4) lattice_edge_kernel(c
 #pragma unroll
         for (int h = 0; h < 8; ++h) {
             a2[h] = __shfl_sync(FULL, a_own, h) * LOG2E;
-            pk[h] = __shfl_sync(FULL, pk_own, h);
+            pk[h] = __shfl_sync(FULL, pk_own, h) | 0x808080;
         }
         // ---- nearest image of the union box, then the terms whose largest weight is above the floor
         float S[8];
@@ -191,7 +193,7 @@ __global__ void __launch_bounds__(THREADS, K == 0 ? 6 : 4) lattice_edge_kernel(c
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
                 w[h] = ex2(a2[h] * rel);
-                if (!got || (masked && !key_in_box(key, pk[h]))) w[h] = 0.f;
+                if (!got || (masked && !term_in_box(key, pk[h]))) w[h] = 0.f;
                 S[h] += w[h];
             }
             if (K > 0) bins.push(got && d2 < p.basis.d2_cut, fast_sqrt(d2) * p.basis.bin_scale, w);
@@ -237,7 +239,7 @@ __global__ void __launch_bounds__(THREADS, K == 0 ? 6 : 4) lattice_edge_kernel(c
 #pragma unroll
                     for (int h = 0; h < 8; ++h) {
                         float eh = fmaf(a2[h], d2, off[h]);
-                        if (!got || !key_in_box(key, pk[h])) eh = -INFINITY;
+                        if (!got || !term_in_box(key, pk[h])) eh = -INFINITY;
                         w[h] = ex2(eh);
                         top = fmaxf(top, eh);
                     }
@@ -313,18 +315,19 @@ int launch_fwd(const FwdArgs &p, long long K, cudaStream_t stream)
     const int mode = K == 0 ? 3 : p.W == nullptr ? AS_PSI : p.W_num == 1 ? ONE_W : MANY_W;
     void (*const kernels[4])(const FwdArgs) = {lattice_edge_kernel<64, AS_PSI>, lattice_edge_kernel<64, ONE_W>,
                                                lattice_edge_kernel<64, MANY_W>, lattice_edge_kernel<0, AS_PSI>};
+    const int warps = edge_warps(mode), threads = 32 * warps;
     const int tiles = mode == 3 ? 0 : mode == ONE_W ? GROUP : 1;
     const size_t smem = sizeof(float) * ((mode == ONE_W ? HEADS * WT_HEAD_STRIDE : 0) +
-                                         WARPS * (EDGE_TERM_FLOATS + (K > 0 ? STAGE_FLOATS : 0) + tiles * 8 * PSI_STRIDE));
+                                         warps * (EDGE_TERM_FLOATS + (K > 0 ? STAGE_FLOATS : 0) + tiles * 8 * PSI_STRIDE));
     static thread_local int per_sm[4] = {0, 0, 0, 0};
     int &occ = per_sm[mode];
     if (occ == 0) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(kernels[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernels[mode], THREADS, smem) != cudaSuccess || occ <= 0) occ = 2;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernels[mode], threads, smem) != cudaSuccess || occ <= 0) occ = 2;
     }
-    const long long want = (p.E + WARPS - 1) / WARPS;
+    const long long want = (p.E + warps - 1) / warps;
     const long long cap = (long long)sm_count() * occ;
-    kernels[mode]<<<(int)(want < cap ? want : cap), THREADS, smem, stream>>>(p);
+    kernels[mode]<<<(int)(want < cap ? want : cap), threads, smem, stream>>>(p);
     return launch_status("cf_lattice_sum_fwd");
 }
 

@@ -149,16 +149,23 @@ __global__ void __launch_bounds__(512) pe_grad_kernel(const PeArgs p)
     if (tid < CH) out[CH * 64 + tid] = wpos;
 }
 
-__global__ void __launch_bounds__(256) pe_grad_sum_kernel(const PeArgs p, int with_psi)
+// the shares added in a fixed order: block = 32 values, warp w the shares w, w + 8, ..., then the eight partial sums
+__global__ void __launch_bounds__(256) pe_grad_sum_kernel(const PeArgs p, int first)
 {
-    const int l = blockIdx.y, idx = (with_psi ? 0 : CH * 64) + blockIdx.x * 256 + threadIdx.x;
-    if (idx >= PE_PARTIAL) return;
+    __shared__ float part[8][32];
+    const int l = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5, idx = first + blockIdx.x * 32 + lane;
     const float *in = p.partial + (size_t)l * p.shares * PE_PARTIAL + idx;
     float t = 0.f;
 #pragma unroll 4
-    for (int sh = 0; sh < p.shares; ++sh) t += in[(size_t)sh * PE_PARTIAL];
+    for (int sh = w; sh < p.shares; sh += 8) t += in[(size_t)sh * PE_PARTIAL];
+    part[w][lane] = t;
+    __syncthreads();
+    if (w != 0) return;
+    t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += part[i][lane];
     if (idx < CH * 64) p.gW[l][idx] = t;
-    else if (p.gwpos[l] != nullptr) p.gwpos[l][idx - CH * 64] = t;
+    else p.gwpos[l][idx - CH * 64] = t;
 }
 
 int projection_shares(long long rows)
@@ -327,7 +334,7 @@ int launch_projection_grad(const float *gv, const float *psi, long long rows, fl
     pe.gattn[0] = gv; pe.psi[0] = psi; pe.gW[0] = gW;
     pe.N = rows; pe.shares = projection_shares(rows); pe.partial = partial;
     pe_grad_kernel<true><<<dim3(pe.shares, 1), 512, 0, s>>>(pe);
-    pe_grad_sum_kernel<<<dim3((CH * 64 + 255) / 256, 1), 256, 0, s>>>(pe, 1);
+    pe_grad_sum_kernel<<<dim3(CH * 64 / 32, 1), 256, 0, s>>>(pe, 0);
     return launch_status("projection gradient");
 }
 }  // namespace cf
@@ -502,7 +509,7 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
     }
     if (d.K > 0) pe_grad_kernel<true><<<dim3(g.shares, L), 512, 0, s>>>(pe);
     else pe_grad_kernel<false><<<dim3(g.shares, L), 512, 0, s>>>(pe);
-    pe_grad_sum_kernel<<<dim3(((d.K > 0 ? PE_PARTIAL : CH) + 255) / 256, L), 256, 0, s>>>(pe, d.K > 0 ? 1 : 0);
+    pe_grad_sum_kernel<<<dim3((d.K > 0 ? PE_PARTIAL : CH) / 32, L), 256, 0, s>>>(pe, d.K > 0 ? 0 : CH * 64);
     // ---- projections
     static thread_local GradJobs jobs;
     int count = 0;
