@@ -53,6 +53,9 @@ SIGNATURES = {
     "cf_dense_image_bytes": [I64],
     "cf_dense_pack_layer": [P, P, P, P, P, P, I64, P, P],
     "cf_dense_pack_embedding": [P, I64, P, P],
+    "cf_model_head_floats": [I64],
+    "cf_model_begin": [P, P, P, I64, I64, P, P, P, P],
+    "cf_model_finish": [P, P, P, P, P, I64, I64, I64, I64, P, P, P, P, P, P, P],
     "cf_train_saved_bytes": [P, I64, I64, I64],
     "cf_train_scratch_bytes": [P, I64, I64, I64],
     "cf_train_forward": [P, P, P, P],
@@ -157,7 +160,7 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
-        for name in ("cf_lattice_sum_bwd_proj_floats", "cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_scratch_bytes"):
+        for name in ("cf_model_head_floats", "cf_lattice_sum_bwd_proj_floats", "cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_scratch_bytes"):
             getattr(lib, name).restype = c_int64
         _lib = lib
     return _lib

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "crystalformer_b200.h"
+#include "dense_tc.cuh"
 
 namespace cf {
 
@@ -44,7 +45,7 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
                        const double *scalars, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius, int lattice_range,
                        int minimum_range, const float *W1, const float *b1, int64_t hidden, const float *W2, const float *b2,
                        int64_t targets, double order_reach, void *workspace, float *y, void *const *attn_events,
-                       const cf_peer_gather *gather, void *inputs_ready, void *slot_free, void *stream);
+                       const cf_peer_gather *gather, void *inputs_ready, void *slot_free, void *stream, float *head = nullptr);
 
 inline bool dense_path_available(int num_layers, const float *const *weights, long long ff_dim)
 {
@@ -60,5 +61,9 @@ struct EmbedStage {
     int feature_dim;         // <= 128
     const float4 *packed;    // W_embed packed as a 128 x 128 weight (input columns beyond feature_dim zero)
 };
+inline void dense_embed_of(DenseForward &d, const EmbedStage &e)
+{
+    d.embed = tc_image(e.packed); d.features = e.features; d.species = e.species; d.feature_dim = e.feature_dim;
+}
 
 }  // namespace cf

@@ -71,6 +71,27 @@ inline bool dense_tc_images(int num_layers, const float *const *weights)
 
 int launch_dense_forward(const DenseForward &p, cudaStream_t s);
 
+// A forward whose first boundary (embedding and the first layer's head) has been launched ahead of the rest, with what it
+// wrote; head_stage carves it from N (4 x 128 + 8) floats.
+struct HeadStage {
+    float *x, *q, *k, *v, *a;
+};
+inline HeadStage head_stage(float *memory, long long N)
+{
+    HeadStage h;
+    h.x = memory; h.q = h.x + N * 128; h.k = h.q + N * 128; h.v = h.k + N * 128; h.a = h.v + N * 128;
+    return h;
+}
+// head of a layer (11 weight pointers, 6 scalars, as in cf_encoder_forward)
+inline void dense_head_of(DenseForward &d, const float *const *w, const double *sc)
+{
+    d.head = tc_image(w[10]); d.bqkv = w[1]; d.w_pos = w[2];
+    d.gauss_scale = (float)sc[0]; d.gauss_shift = (float)sc[1]; d.a_factor = (float)sc[2];
+    d.elu_beta = (float)sc[3]; d.lower_bound = (float)sc[4];
+}
+// Host read of a batch's sizes beside the work that `launch` queues (encoder_forward.cu).
+int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *), void *arg, void **inputs_event);
+
 // ---- training (dense_tc_bwd.cu) ---------------------------------------------------------------------------------------
 // The blocks of one layer in the backward kernel's order, every one transposed: [Wq, Wk, Wv] and
 // [W2_0, W2_1, W1_0, W2_2, W1_1, ..., Wo].  Appends to job.

@@ -29,7 +29,7 @@ int encoder_forward_impl(void *cublas_handle, int num_layers, const float *const
                          const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t E,
                          int64_t max_atoms, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius,
                          int lattice_range, int minimum_range, float *workspace, const int32_t *row_order,
-                         void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep);
+                         void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun);
 int infinite_attn_fwd_impl(const float *q, const float *k, const float *v, const float *a, const float *pos,
                            const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
                            const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t H, int64_t D,
@@ -49,7 +49,7 @@ namespace {
 // process: the term-list build of a forward depends on the geometry only and runs beside the first dense block.
 struct SideStream {
     cudaStream_t stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, inputs = nullptr;
     bool ok = false;
 };
 SideStream &side_stream()
@@ -61,7 +61,8 @@ SideStream &side_stream()
     if (!s.ok && s.stream == nullptr) {
         s.ok = cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) == cudaSuccess &&
                cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) == cudaSuccess &&
-               cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) == cudaSuccess;
+               cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&s.inputs, cudaEventDisableTiming) == cudaSuccess;
         if (!s.ok) {
             cudaGetLastError();
             s.stream = reinterpret_cast<cudaStream_t>(1);  // do not try again
@@ -71,6 +72,53 @@ SideStream &side_stream()
 }
 
 }  // namespace
+
+// The host's copy of a batch's sizes, for callers that only have them on the device: the copy is queued first, then
+// `launch` queues work that needs the number of atoms only, and the host waits for the copy while that runs.  counts =
+// { atoms, edges, largest crystal }.  Pinned staging memory and the event are this thread's (at most 8 MiB, returned
+// when the thread ends).
+namespace {
+struct PinnedSizes {
+    int64_t *at = nullptr;
+    int64_t capacity = 0;
+    ~PinnedSizes() { if (at != nullptr) cudaFreeHost(at); }
+    bool reserve(int64_t n)
+    {
+        if (n <= capacity) return true;
+        if (at != nullptr) cudaFreeHost(at);
+        at = nullptr;
+        capacity = 0;
+        const int64_t want = n < 1024 ? 1024 : n + n / 4;
+        if (cudaHostAlloc(reinterpret_cast<void **>(&at), sizeof(int64_t) * (size_t)want, cudaHostAllocPortable) != cudaSuccess) return false;
+        capacity = want;
+        return true;
+    }
+};
+}  // namespace
+int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *), void *arg, void **inputs_event)
+{
+    static thread_local PinnedSizes pinned;
+    SideStream &side = side_stream();
+    CF_REQUIRE(side.ok, CF_ERR_CUDA, "the side stream could not be created");
+    CF_REQUIRE(B >= 1 && B <= (1 << 20), CF_ERR_RANGE, "B=%lld outside [1, 2^20]", (long long)B);
+    const bool read = counts[0] < 0;
+    if (read) {
+        CF_REQUIRE(pinned.reserve(B), CF_ERR_CUDA, "no pinned memory for %lld sizes", (long long)B);
+        if (cudaMemcpyAsync(pinned.at, sizes, sizeof(int64_t) * (size_t)B, cudaMemcpyDeviceToHost, s) != cudaSuccess) return launch_status("sizes to the host");
+    }
+    if (cudaEventRecord(side.inputs, s) != cudaSuccess) return launch_status("sizes to the host");
+    *inputs_event = side.inputs;
+    const int rc = launch(arg);
+    if (rc != CF_OK || !read) return rc;
+    if (cudaEventSynchronize(side.inputs) != cudaSuccess) return launch_status("sizes to the host");
+    int64_t n = 0, e = 0, m = 0;
+    for (int64_t c = 0; c < B; ++c) {
+        const int64_t v = pinned.at[c];
+        n += v; e += v * v; m = v > m ? v : m;
+    }
+    counts[0] = n; counts[1] = e; counts[2] = m;
+    return CF_OK;
+}
 
 // The side stream made to wait for the caller's events (either may be NULL), for cf_model_forward's early preparation;
 // NULL if the side stream could not be created.
@@ -177,7 +225,7 @@ extern "C" int cf_encoder_forward(void *cublas_handle, int num_layers, const flo
 {
     return cf::encoder_forward_impl(cublas_handle, num_layers, weights, scalars, x, pos_ij, tvecs, rvlen, batch, edges,
                                     row_start, N, B, E, max_atoms, K, ff_dim, wscale, cutoff_radius, lattice_range,
-                                    minimum_range, workspace, row_order, attn_events, stream, nullptr, false);
+                                    minimum_range, workspace, row_order, attn_events, stream, nullptr, false, nullptr);
 }
 
 // cf_encoder_forward with an optional embedding stage (dense path only): x is then written by the first dense block.
@@ -186,7 +234,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                              const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t E,
                              int64_t max_atoms, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius,
                              int lattice_range, int minimum_range, float *workspace, const int32_t *row_order,
-                             void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep)
+                             void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun)
 {
     CF_REQUIRE(N >= 0 && E >= 0 && num_layers >= 0, CF_ERR_INVALID, "cf_encoder_forward: negative size");
     CF_REQUIRE(ff_dim > 0 && ff_dim % 4 == 0, CF_ERR_UNSUPPORTED, "cf_encoder_forward: ff_dim must be a positive multiple of 4");
@@ -204,6 +252,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     float *qkv = workspace;
     float *q = qkv + N * 384, *k = q + N * 128, *v = k + N * 128, *attn = v + N * 128;
     float *a = attn + N * 128, *lse = a + N * 8, *hidden = lse + N * 8, *logit = hidden + N * ff_dim;
+    if (begun != nullptr) { q = begun->q; k = begun->k; v = begun->v; a = begun->a; }  // (x is the caller's)
     int rc = CF_OK;
 
     // Term lists (term_list.cuh): the geometry is the same for every layer, so the (key, translation) pairs that can
@@ -277,21 +326,16 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     if (fused && dense_tc_images(num_layers, weights)) {
         // the weights as images for the block-level tensor instructions (dense_tc.cu)
         auto boundary = [&](int l) {  // the kernel before layer l's attention (tail of layer l - 1, head of layer l)
+            if (l == 0 && begun != nullptr) return (int)CF_OK;
             DenseForward d{};
             d.N = N; d.ff = ff; d.chained = l > 0; d.x_in = d.x_out = x; d.q = q; d.k = k; d.v = v; d.a = a;
             if (l > 0) {
                 const float *const *w = weights + 11 * (l - 1);
                 d.tail = tc_image(w[10]); d.attn = attn; d.bo = w[5]; d.b1 = w[7]; d.b2 = w[9];
             } else if (embed != nullptr) {
-                d.embed = tc_image(embed->packed); d.features = embed->features; d.species = embed->species; d.feature_dim = embed->feature_dim;
+                dense_embed_of(d, *embed);
             }
-            if (l < num_layers) {
-                const float *const *w = weights + 11 * l;
-                const double *sc = scalars + 6 * l;
-                d.head = tc_image(w[10]); d.bqkv = w[1]; d.w_pos = w[2];
-                d.gauss_scale = (float)sc[0]; d.gauss_shift = (float)sc[1]; d.a_factor = (float)sc[2];
-                d.elu_beta = (float)sc[3]; d.lower_bound = (float)sc[4];
-            }
+            if (l < num_layers) dense_head_of(d, weights + 11 * l, scalars + 6 * l);
             return launch_dense_forward(d, s);
         };
         rc = boundary(0);

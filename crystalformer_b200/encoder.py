@@ -20,6 +20,7 @@ from . import _lib, ops
 from .attention import CrystalformerMultiheadAttentionCUDA, heaviest_first, register_edge_info
 from .cuda_funcs import compile_kernels
 from .params import LatticeformerParams
+from .training import OfThisModel
 
 
 def _get_activation_fn(activation):
@@ -228,8 +229,8 @@ class CrystalformerEncoderCUDA(Module):
         params = [p for p in self.parameters()] + [b for b in self.buffers()]  # (gauss_scale is a buffer)
         key = (device, self.dense_fused, tuple(p._version for p in params), tuple(p.data_ptr() for p in params))
         cache = getattr(self, "_native_cache", None)
-        if cache is not None and cache[0] == key:
-            return cache[1]
+        if cache is not None and cache.values[0] == key:
+            return cache.values[1]
         keep, ptrs, scalars = [], [], []
         for layer in self.layers:
             att, P = layer.self_attn, layer.self_attn.params
@@ -255,7 +256,7 @@ class CrystalformerEncoderCUDA(Module):
             scalars += [gs[0], gs[1], -0.5 * P.scale_real ** -2, beta, P.gauss_lb_real, dist_max]
         packed = dict(keep=keep, ptrs=(ctypes.c_void_p * len(ptrs))(*ptrs), scalars=(ctypes.c_double * len(scalars))(*scalars),
                       ff=self.layers[0].linear1.weight.shape[0])
-        self._native_cache = (key, packed)
+        self._native_cache = OfThisModel(key, packed)
         return packed
 
     def _cutoff(self) -> float:

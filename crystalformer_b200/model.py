@@ -17,7 +17,7 @@ from . import _lib
 from .cuda_funcs import IrregularMeanCUDA
 from .encoder import MAX_IMAGE_FF, BatchGeometry, CrystalformerEncoderCUDA, image_pointer, pack_dense_embedding, pack_dense_weight
 from .params import DEFAULT_MODEL_PARAMS, LatticeformerParams
-from .training import train_step
+from .training import ModelWatch, OfThisModel, train_step
 
 
 def default_params(**overrides) -> types.SimpleNamespace:
@@ -154,6 +154,7 @@ class Latticeformer(nn.Module):
                     w2=f32(self.mlp[3].weight), b2=f32(self.mlp[3].bias), emb_packed=self._embedding_packed(device))
         reach = self.native_reach()
         plan["hidden"], plan["targets"] = plan["w1"].shape[0], plan["w2"].shape[0]
+        plan["images"] = plan["emb_packed"] is not None and plan["emb_packed"].dtype == torch.uint8
         if plan["emb_packed"] is not None:  # the description of the model for cf_serve_submit
             plan["desc"] = _lib.ModelDesc(
                 feature_dim=plan["emb"].shape[1], W_embed=plan["emb"].data_ptr(), W_embed_packed=image_pointer(plan["emb_packed"]),
@@ -194,11 +195,26 @@ class Latticeformer(nn.Module):
             slot = ring["slots"][at] = [torch.empty(nbytes, dtype=torch.uint8, device=dev), torch.cuda.Event(), False]
         return slot
 
-    def _forward_native(self, data, counts: Tuple[int, int, int], gather=None, plan: Optional[dict] = None,
+    def _current_plan(self, dev) -> dict:
+        """``native_plan``, rebuilt only when a parameter, a buffer or a module of the model is another one or has changed."""
+        cache = getattr(self, "_plan_cache", None)
+        key = (dev, self.encoder.dense_fused)
+        if cache is None or cache.values[0] != key or not cache.values[1].current():
+            plan = self.native_plan(dev)
+            self._plan_cache = cache = OfThisModel(key, ModelWatch(self, versions=True), plan)
+        return cache.values[2]
+
+    def _forward_native(self, data, counts: Optional[Tuple[int, int, int]], gather=None, plan: Optional[dict] = None,
                         inputs_ready: Optional[torch.cuda.Event] = None) -> torch.Tensor:
         dev = data.pos.device
         if plan is None:
-            plan = self.native_plan(dev)
+            plan = self._current_plan(dev)
+        if counts is None:
+            if "desc" in plan and plan["images"] and data.pos.shape[0] > 0 and data.sizes.device == dev \
+                    and data.sizes.dtype == torch.int64 and data.sizes.is_contiguous() and data.sizes.shape[0] > 0:
+                return self._forward_begun(data, gather, plan)
+            host = data.sizes.tolist()  # the one device->host read per batch (the reference does the same)
+            counts = (sum(host), sum(n * n for n in host), max(host) if host else 1)
         n_atoms, n_edges, max_atoms = (int(v) for v in counts)
         f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()
         feats, pos, trans = f32(data.x), f32(data.pos), f32(data.trans_vec)
@@ -234,20 +250,42 @@ class Latticeformer(nn.Module):
                 slot[2] = True
         return y if gather is None else gather.collect()
 
+    def _forward_begun(self, data, gather, plan: dict) -> torch.Tensor:
+        """The one-call forward for sizes that only the device knows: their read-back and the first dense block are queued
+        together, and the host waits for the former while the latter runs."""
+        dev = data.pos.device
+        f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()
+        feats, pos, trans, sizes = f32(data.x), f32(data.pos), f32(data.trans_vec), data.sizes
+        N, B = pos.shape[0], sizes.shape[0]
+        lib = _lib.load()
+        desc = ctypes.byref(plan["desc"])
+        head = torch.empty(N * 520, dtype=torch.float32, device=dev)  # cf_model_head_floats(N)
+        counts, event = (ctypes.c_int64 * 3)(-1, 0, 0), ctypes.c_void_p()
+        with torch.cuda.device(dev):
+            stream = torch.cuda.current_stream(dev).cuda_stream
+            _lib.call("cf_model_begin", desc, feats.data_ptr(), sizes.data_ptr(), N, B, head.data_ptr(), counts, ctypes.byref(event), stream)
+            n_atoms, n_edges, max_atoms = counts
+            if n_atoms != N:  # (atoms beyond the crystals: their rows are not part of the batch)
+                return self._forward_native(data, (n_atoms, n_edges, max_atoms), gather, plan)
+            work = torch.empty(int(lib.cf_model_workspace_bytes(N, B, n_edges, plan["w"]["ff"])), dtype=torch.uint8, device=dev)
+            y = torch.empty((B, plan["targets"]), dtype=torch.float32, device=dev)
+            step = None if gather is None else gather.next_descriptor()
+            _lib.call("cf_model_finish", desc, feats.data_ptr(), pos.data_ptr(), trans.data_ptr(), sizes.data_ptr(), N, B, n_edges,
+                      max_atoms, head.data_ptr(), event, work.data_ptr(), y.data_ptr(), self.encoder._attention_events(),
+                      None if step is None else ctypes.byref(step), stream)
+        return y if gather is None else gather.collect()
+
     def forward(self, data, geometry: Optional[BatchGeometry] = None, counts: Optional[Tuple[int, int, int]] = None,
                 gather=None, inputs_ready: Optional[torch.cuda.Event] = None):
         """``data`` carries x (N,98), pos (N,3), batch (N), trans_vec (B,3,3), sizes (B) like the reference's PyG batch.
         ``counts`` = (atoms, edges = sum n^2, largest crystal), when the caller knows them on the host, saves the
-        device->host read of ``sizes``.  ``gather`` (a ``sharding.PeerGather``, inference only): the outputs of every
+        device->host read of ``sizes`` (which inference overlaps with the first dense block).  ``gather`` (a ``sharding.PeerGather``, inference only): the outputs of every
         rank's crystals are returned, in the order of the unsharded batch.  ``inputs_ready`` (inference through the
         one-call path only): a CUDA event after which the tensors of ``data`` are valid.  The batch preparation, which
         depends on the inputs alone, is then not ordered behind the work already queued on the current stream and
         overlaps the previous batch's forward; the tensors must stay unchanged until this forward has run."""
         if geometry is None and not self.training and not torch.is_grad_enabled() and data.pos.is_cuda \
                 and self._native_ok():
-            if counts is None:
-                host = data.sizes.tolist()  # the one device->host read per batch (the reference does the same)
-                counts = (sum(host), sum(n * n for n in host), max(host) if host else 1)
             return self._forward_native(data, counts, gather, inputs_ready=inputs_ready)
         if geometry is None and torch.is_grad_enabled() and data.pos.is_cuda and self._native_shell() \
                 and self.encoder._native_model():

@@ -13,6 +13,47 @@ import torch
 from . import _lib
 
 
+class OfThisModel:
+    """A cache that belongs to one model object: copies and pickles of the model carry None instead (addresses and ctypes
+    structures cannot be copied)."""
+
+    def __init__(self, *values):
+        self.values = values
+
+    def __deepcopy__(self, memo):
+        return None
+
+    def __reduce__(self):
+        return type(None), ()
+
+
+class ModelWatch:
+    """Notices when a model is no longer the one a plan was made for: a submodule, parameter or buffer replaced, moved or
+    (with ``versions``) modified in place, or a setting changed."""
+
+    def __init__(self, model, versions: bool):
+        self.children = [(m._modules, n, c) for m in model.modules() for n, c in m._modules.items()]
+        self.places = [(d, n, t) for m in model.modules() for d in (m._parameters, m._buffers) for n, t in d.items() if t is not None]
+        self.tensors = [t for _, _, t in self.places]
+        self.versions = versions
+        self.settings = model.encoder.lattice_params
+        self.layer_settings = [layer.self_attn.params for layer in model.encoder.layers]
+        self.key = self.now()
+
+    def now(self) -> list:
+        P = self.settings  # the scalar settings that the plans of a model contain
+        key = [P.lattice_range, P.minimum_range, P.adaptive_cutoff_sigma, P.gauss_lb_real, str(P.scale_real), P.value_pe_dist_real,
+               P.value_pe_width_scale, P.value_pe_dist_max]
+        for Q in self.layer_settings:
+            key += (Q.positive_func, Q.gauss_lb_real, Q.scale_real, Q.value_pe_dist_max)
+        key += [t.data_ptr() for t in self.tensors]
+        return key + [t._version for t in self.tensors] if self.versions else key
+
+    def current(self) -> bool:
+        return all([d.get(n) is c for d, n, c in self.children]) and all([d.get(n) is t for d, n, t in self.places]) \
+            and self.now() == self.key
+
+
 class TrainPlan:
     """What a step needs and the batch does not change: the parameters in the library's order with their addresses, the
     scalar settings, and where every gradient lies in one flat buffer.  Valid while the parameters keep their storage."""
@@ -32,20 +73,17 @@ class TrainPlan:
             scalars += [gs[0], gs[1], -0.5 * Q.scale_real ** -2, beta, Q.gauss_lb_real, dist_max]
         ordered += [model.input_embeddings.weight, model.mlp[0].weight, model.mlp[0].bias, model.mlp[3].weight, model.mlp[3].bias]
         self.params = [p for p in ordered if p is not None]
-        # the places where the model holds them (and its submodules): a step checks that they are still the same objects
-        at = {id(p): (m._parameters, n) for m in model.modules() for n, p in m._parameters.items() if p is not None}
-        self.places = [(*at[id(p)], p) for p in self.params]
-        self.children = [(m._modules, n, c) for m in model.modules() for n, c in m._modules.items()]
+        self.watch = ModelWatch(model, versions=False)
         self.scales = [layer.self_attn.gauss_scale for layer in enc.layers]
-        self.key = self.current_key()
+        self.scale_versions = [g._version for g in self.scales]
         sizes = [p.numel() for p in self.params]
-        # gradients start on 256-byte boundaries of one buffer (the kernels store rows of them as vectors)
+        # gradients lie one after the other in one buffer
         offsets, at = [], 0
         for n in sizes:
             offsets.append(at)
-            at += (n + 63) // 64 * 64
-        self.spans = list(zip(offsets, sizes, [p.shape for p in self.params]))
+            at += n
         self.floats = at
+        self.like = [p.detach() for p in self.params]
         where = iter(range(len(self.params)))
         self.slots = [None if p is None else next(where) for p in ordered]
         self.offsets = offsets
@@ -61,18 +99,7 @@ class TrainPlan:
             weights=ctypes.cast(self.pointers, ctypes.c_void_p), scalars=ctypes.cast(self.scalars, ctypes.c_void_p))
 
     def current(self) -> bool:
-        return all(d.get(n) is c for d, n, c in self.children) and all(d.get(n) is p for d, n, p in self.places) \
-            and self.current_key() == self.key
-
-    # a copy of the model makes its own plan (addresses cannot be copied)
-    def __deepcopy__(self, memo):
-        return None
-
-    def __reduce__(self):
-        return type(None), ()
-
-    def current_key(self) -> tuple:
-        return tuple([p.data_ptr() for p in self.params] + [g._version for g in self.scales] + [g.data_ptr() for g in self.scales])
+        return self.watch.current() and [g._version for g in self.scales] == self.scale_versions
 
     def versions(self) -> list:
         return [p._version for p in self.params]
@@ -137,16 +164,18 @@ class TrainStep(torch.autograd.Function):
             _lib.call("cf_train_backward", ctypes.byref(plan.desc), ctypes.byref(batch), gy.data_ptr(), scratch.data_ptr(),
                       ctypes.cast(where, ctypes.c_void_p), torch.cuda.current_stream(dev).cuda_stream)
         del keep
-        return (None, None, None, *[flat[at:at + n].view(shape) for at, n, shape in plan.spans])
+        return (None, None, None, *torch._utils._unflatten_dense_tensors(flat, plan.like))
 
 
 def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[torch.Tensor]:
     """The model's output on ``data`` with the step's autograd node behind it, or None when the calls do not apply."""
-    plan = getattr(model, "_train_plan", None)
+    cache = getattr(model, "_train_plan", None)
+    plan = None if cache is None else cache.values[0]
     if plan is None or not plan.current():
         if not supported(model):
             return None
-        plan = model._train_plan = TrainPlan(model)
+        plan = TrainPlan(model)
+        model._train_plan = OfThisModel(plan)
     if not all(layer.self_attn.term_lists for layer in model.encoder.layers):
         return None
     if any(t.requires_grad for t in (data.x, data.pos, data.trans_vec)) or torch.is_autocast_enabled():

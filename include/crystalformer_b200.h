@@ -424,6 +424,16 @@ int cf_model_forward(void *cublas_handle, const float *features, int64_t feature
                      void *stream);
 
 /* ------------------------------------------------------------------------------------------------------------
+ * cf_model_forward in two halves, for callers whose sizes are on the device only (declared below cf_model_desc):
+ * cf_model_begin queues the read-back of the sizes, then the first dense block (which needs the number of atoms only),
+ * waits for the sizes while that runs and returns counts = { atoms, edges, largest crystal } (nothing is read or waited
+ * for if counts[0] >= 0 on entry); cf_model_finish queues the rest, its batch preparation beside the first block.  Only
+ * with weight images.  head: cf_model_head_floats(N) floats of device memory, kept between the two; inputs_event: an
+ * event of the library's, valid until this thread's next cf_model_begin / cf_train_begin.
+ * ---------------------------------------------------------------------------------------------------------- */
+int64_t cf_model_head_floats(int64_t N);
+
+/* ------------------------------------------------------------------------------------------------------------
  * A training step of the whole model (what autograd does through Latticeformer.forward and its backward,
  * models/latticeformer.py:211-302, same configuration as cf_model_forward) in two host calls.
  *   cf_train_desc  : weights = HOST array of 12 num_layers + 5 device pointers: per layer Wq, Wk, Wv (128,128),
@@ -507,6 +517,11 @@ typedef struct cf_model_desc {
     int64_t targets;
     double order_reach;
 } cf_model_desc;
+int cf_model_begin(const cf_model_desc *desc, const float *features, const int64_t *sizes, int64_t N, int64_t B, float *head,
+                   int64_t *counts, void **inputs_event, void *stream);
+int cf_model_finish(const cf_model_desc *desc, const float *features, const float *pos, const float *trans, const int64_t *sizes,
+                    int64_t N, int64_t B, int64_t E, int64_t max_atoms, float *head, void *inputs_event, void *workspace, float *y,
+                    void *const *attn_events, const cf_peer_gather *gather, void *stream);
 typedef struct cf_serve_slot {
     void *copy_stream, *compute_stream;
     void *copied, *inputs_free, *done;
