@@ -56,9 +56,11 @@ SIGNATURES = {
     "cf_model_head_floats": [I64],
     "cf_model_begin": [P, P, P, I64, I64, P, P, P, P],
     "cf_model_finish": [P, P, P, P, P, I64, I64, I64, I64, P, P, P, P, P, P, P],
-    "cf_train_saved_bytes": [P, I64, I64, I64],
+    "cf_train_saved_bytes": [P, I64, I64],
+    "cf_train_edge_bytes": [P, I64, I64, I64],
     "cf_train_scratch_bytes": [P, I64, I64, I64],
-    "cf_train_forward": [P, P, P, P],
+    "cf_train_begin": [P, P, P, P, P],
+    "cf_train_forward": [P, P, P, P, P],
     "cf_train_backward": [P, P, P, P, P, P],
     "cf_row_cost": [P, P, I64, I64, F64, P, P],
     "cf_row_order": [P, P, I64, I64, F64, P, P],
@@ -100,7 +102,7 @@ class TrainDesc(ctypes.Structure):
 class TrainBatch(ctypes.Structure):
     """``cf_train_batch``: a batch and the memory its step keeps between forward and backward."""
     _fields_ = [("features", c_void_p), ("pos", c_void_p), ("trans", c_void_p), ("sizes", c_void_p), ("N", c_int64), ("B", c_int64),
-                ("E", c_int64), ("max_atoms", c_int64), ("saved", c_void_p)]
+                ("E", c_int64), ("max_atoms", c_int64), ("saved", c_void_p), ("saved_edges", c_void_p)]
 
 
 class ServeSlot(ctypes.Structure):
@@ -160,7 +162,8 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.argtypes = argtypes
             fn.restype = c_int
-        for name in ("cf_model_head_floats", "cf_lattice_sum_bwd_proj_floats", "cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_scratch_bytes"):
+        for name in ("cf_model_head_floats", "cf_lattice_sum_bwd_proj_floats", "cf_dense_image_bytes", "cf_train_saved_bytes", "cf_train_edge_bytes",
+                     "cf_train_scratch_bytes"):
             getattr(lib, name).restype = c_int64
         _lib = lib
     return _lib

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(ORDER_THREADS) prepare_all_kernel(const Prepar
 int launch_prepare_all(const float *pos, const float *trans, const int64_t *sizes, int64_t *atom_start,
                        int64_t *edge_start, long long B, long long N, long long E, int64_t *batch, int64_t *edges,
                        int64_t *row_start, float *pos_ij, float *rvlen, double reach, int32_t *row_order, bool *ordered,
-                       cudaStream_t s)
+                       cudaStream_t s, float *rvecs, float *vcell)
 {
     PrepareAll p{};
     p.pos = pos; p.trans = trans; p.atom_start = atom_start; p.edge_start = edge_start; p.B = B; p.N = N; p.E = E;
@@ -314,7 +314,7 @@ int launch_prepare_all(const float *pos, const float *trans, const int64_t *size
     } else {
         crystal_offsets_kernel<<<1, SCAN_THREADS, 0, s>>>(sizes, B, atom_start, edge_start);
     }
-    p.batch = batch; p.edges = edges; p.row_start = row_start; p.pos_ij = pos_ij; p.rvlen = rvlen;
+    p.batch = batch; p.edges = edges; p.row_start = row_start; p.pos_ij = pos_ij; p.rvlen = rvlen; p.rvecs = rvecs; p.vcell = vcell;
     *ordered = row_order != nullptr && B <= ORDER_MAX_CRYSTALS && N < (1ll << 31);
     p.order = *ordered ? row_order : nullptr;
     p.padded = 2;

@@ -278,9 +278,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                                 al[e] += __shfl_xor_sync(FULL, al[e], 2);
                                 const long long row = row_base + pl.row0 + 16 * half + 8 * e;
                                 if (pl.t == 0 && row < p.N) {
-                                    const float tt = (al[e] + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - p.lower_bound));
-                                    const float elu = tt > 0.f ? tt : expm1f(tt);
-                                    p.a[row * HEADS + 2 * pl.group + hh] = ((1.0f - p.lower_bound) * elu + 1.0f) * p.a_factor;
+                                    const float lb = pl.group < 2 ? p.lower_bound : p.lower_bound_hi;
+                                    const float tt = (al[e] + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - lb));
+                                    const float elu = tt > 0.f ? tt : expm1f(tt), f = (1.0f - lb) * elu + 1.0f;
+                                    const float factor = pl.group < 2 ? p.a_factor : p.a_factor_hi;
+                                    p.a[row * HEADS + 2 * pl.group + hh] = p.inverse ? factor / f : f * factor;
                                 }
                             }
                         }

@@ -51,6 +51,8 @@ struct DenseForward {
     const unsigned char *head;
     const float *bqkv, *w_pos;
     float gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound;
+    float a_factor_hi, lower_bound_hi;  // heads 4-7 (domain "multihead": the reciprocal-space half; else as heads 0-3)
+    bool inverse;                       // a = a_factor / f instead of a_factor f (domain "RECI")
     // activations
     const float *x_in;   // (N,128) features the tail's residual (or, without tail and embedding, the head) reads
     float *x_out;        // (N,128) features after the tail / embedding
@@ -88,6 +90,7 @@ inline void dense_head_of(DenseForward &d, const float *const *w, const double *
     d.head = tc_image(w[10]); d.bqkv = w[1]; d.w_pos = w[2];
     d.gauss_scale = (float)sc[0]; d.gauss_shift = (float)sc[1]; d.a_factor = (float)sc[2];
     d.elu_beta = (float)sc[3]; d.lower_bound = (float)sc[4];
+    d.a_factor_hi = d.a_factor; d.lower_bound_hi = d.lower_bound;
 }
 // Host read of a batch's sizes beside the work that `launch` queues (encoder_forward.cu).
 int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *), void *arg, void **inputs_event);
@@ -106,7 +109,8 @@ struct DenseBackward {
     // head (image null: none): gx = g_res + gq' Wq + gk Wk + gv Wv, gq' = gq / 4 + galpha w_pos
     const unsigned char *head;
     const float *q, *w_pos;      // the saved query (scaled by 1/4)
-    float gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound;
+    float gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound, a_factor_hi, lower_bound_hi;  // as in DenseForward
+    bool inverse;
     float *gq, *ga;              // in: gradients of the scaled query and of a; out: gq' and galpha
     const float *gk, *gv, *g_res;
     float *gx;                   // (N,128) out (with a head), in (without)

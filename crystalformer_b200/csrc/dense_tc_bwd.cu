@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 // ---- gq' and gk as operands 0 and 1, with one scale per row for the three of them (their products meet in
                 //      one accumulator); warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (head l / 4)
                 const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
-                const float slope = p.gauss_scale * p.a_factor * p.elu_beta;
+                const float lb = lane < 16 ? p.lower_bound : p.lower_bound_hi;
+                const float slope = p.gauss_scale * (lane < 16 ? p.a_factor : p.a_factor_hi) * p.elu_beta;
                 float *inv_out = s.row_floats(0);
                 const uint32_t lane_at = (lane >> 4) * 16384 + (lane & 1) * 8;
                 auto put = [&](unsigned char *buf, int row, const float4 v, float sc) {
@@ -138,8 +139,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                         float al = 4.0f * fmaf(qv.w, wp.w, fmaf(qv.z, wp.z, fmaf(qv.y, wp.y, qv.x * wp.x)));
                         al += __shfl_xor_sync(FULL, al, 1);
                         al += __shfl_xor_sync(FULL, al, 2);
-                        const float tt = (al + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - p.lower_bound));
-                        const float galpha = ga * slope * (tt > 0.f ? 1.0f : expf(tt));
+                        const float tt = (al + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - lb));
+                        float galpha = ga * slope * (tt > 0.f ? 1.0f : expf(tt));
+                        if (p.inverse) {
+                            const float f = (1.0f - lb) * (tt > 0.f ? tt : expm1f(tt)) + 1.0f;
+                            galpha = -galpha / (f * f);
+                        }
                         gq[u].x = fmaf(galpha, wp.x, 0.25f * gq[u].x); gq[u].y = fmaf(galpha, wp.y, 0.25f * gq[u].y);
                         gq[u].z = fmaf(galpha, wp.z, 0.25f * gq[u].z); gq[u].w = fmaf(galpha, wp.w, 0.25f * gq[u].w);
                         __syncwarp();  // (the lanes of a head have read ga)

@@ -131,6 +131,15 @@ cudaStream_t early_prep_stream(void *inputs_ready, void *slot_free)
     return side.stream;
 }
 
+// `s` made to wait for what has been queued on the side stream so far.
+int join_early_prep(cudaStream_t s)
+{
+    SideStream &side = side_stream();
+    if (cudaEventRecord(side.join, side.stream) != cudaSuccess || cudaStreamWaitEvent(s, side.join, 0) != cudaSuccess)
+        return launch_status("side stream join");
+    return CF_OK;
+}
+
 namespace {
 
 struct LayerScalars {

@@ -18,7 +18,7 @@ int validate_peer_gather(const cf_peer_gather *g, long long rows, const char *wh
 int launch_prepare_all(const float *pos, const float *trans, const int64_t *sizes, int64_t *atom_start,
                        int64_t *edge_start, long long B, long long N, long long E, int64_t *batch, int64_t *edges,
                        int64_t *row_start, float *pos_ij, float *rvlen, double reach, int32_t *row_order, bool *ordered,
-                       cudaStream_t s);
+                       cudaStream_t s, float *rvecs = nullptr, float *vcell = nullptr);
 int encoder_forward_impl(void *cublas_handle, int num_layers, const float *const *weights, const double *scalars,
                          float *x, const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
                          const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t E,

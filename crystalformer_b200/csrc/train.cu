@@ -15,10 +15,12 @@
 #include "term_list.cuh"
 
 namespace cf {
+cudaStream_t early_prep_stream(void *inputs_ready, void *slot_free);
+int join_early_prep(cudaStream_t s);
 int launch_prepare_all(const float *pos, const float *trans, const int64_t *sizes, int64_t *atom_start,
                        int64_t *edge_start, long long B, long long N, long long E, int64_t *batch, int64_t *edges,
                        int64_t *row_start, float *pos_ij, float *rvlen, double reach, int32_t *row_order, bool *ordered,
-                       cudaStream_t s);
+                       cudaStream_t s, float *rvecs = nullptr, float *vcell = nullptr);
 int infinite_attn_fwd_impl(const float *q, const float *k, const float *v, const float *a, const float *pos,
                            const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
                            const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t H, int64_t D,
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(512) pe_grad_kernel(const PeArgs p)
     for (int m = 0; m < 16; ++m) acc[m] = 0.f;
     for (long long n0 = lo; n0 < hi; n0 += PE_ROWS) {
         const int rows = (int)min((long long)PE_ROWS, hi - n0);
-        if (PSI) {
+        if (PSI && psi != nullptr) {
             __syncthreads();
             for (int i = tid; i < rows * CH; i += 512) go[i] = gattn[n0 * CH + i];
             __syncthreads();
@@ -164,8 +166,44 @@ __global__ void __launch_bounds__(256) pe_grad_sum_kernel(const PeArgs p, int fi
     t = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) t += part[i][lane];
+    if (idx < CH * 64 && p.psi[l] == nullptr) return;  // (the layer's operators have written it, or it has none)
     if (idx < CH * 64) p.gW[l][idx] = t;
     else p.gwpos[l][idx - CH * 64] = t;
+}
+
+// ---- layers with a reciprocal-space half (domains "reci", "RECI", "multihead"): phi of either half, gradients of either ----
+// phi = phi_real for heads below `real`, phi_reci for the others; the value encoding of the latter is zero
+__global__ void merge_phi_kernel(const float4 *__restrict__ phi_real, const float4 *__restrict__ phi_reci, float4 *__restrict__ phi,
+                                 float4 *__restrict__ values, long long E)
+{
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // (edge, half of the heads) x 16 float4
+    const long long e = idx >> 4;
+    const int t = (int)(idx & 15);
+    if (e >= E) return;
+    if (t < 2) phi[2 * e + t] = t == 0 ? phi_real[2 * e] : phi_reci[2 * e + 1];
+    if (values != nullptr) values[32 * e + 16 + t] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// the other way round: the gradient of phi split by heads, that of the reciprocal half's (zero) value encoding dropped
+__global__ void split_gphi_kernel(const float4 *__restrict__ gphi, float4 *__restrict__ g_real, float4 *__restrict__ g_reci,
+                                  float4 *__restrict__ gvalues, long long E)
+{
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long e = idx >> 4;
+    const int t = (int)(idx & 15);
+    if (e >= E) return;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < 2) {
+        const float4 g = gphi[2 * e + t];
+        g_real[2 * e + t] = t == 0 ? g : zero;
+        g_reci[2 * e + t] = t == 0 ? zero : g;
+    }
+    if (gvalues != nullptr) gvalues[32 * e + 16 + t] = zero;
+}
+// ga of the halves side by side: heads 4-7 from the reciprocal sum
+__global__ void merge_ga_kernel(const float4 *__restrict__ ga_reci, float4 *__restrict__ ga, long long N)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N) ga[2 * i + 1] = ga_reci[2 * i + 1];
 }
 
 int projection_shares(long long rows)
@@ -187,23 +225,35 @@ struct Carver {
     }
 };
 
+enum Domain { REAL = 0, RECI = 1, RECI_INVERSE = 2, MULTIHEAD = 3 };
+constexpr int SCALARS = 9;  // gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound, dist_max, a_factor_hi, lower_bound_hi, domain
+Domain domain_of(const cf_train_desc &d, int l) { return (Domain)(int)d.scalars[SCALARS * l + 8]; }
+bool has_values(const cf_train_desc &d, int l) { return d.K > 0 && (domain_of(d, l) == REAL || domain_of(d, l) == MULTIHEAD); }
+
 struct LayerSaved {
     unsigned char *forward, *backward;  // weight images
-    float *q, *k, *v, *a, *lse, *logit, *attn, *psi, *y, *h;
+    float *q, *k, *v, *a, *attn, *psi, *y, *h;
+    float *lse, *logit;                              // domain real: the fused attention
+    float *phi_real, *sum_reci, *phi, *values, *prob;  // others: the operator pair
 };
 struct Saved {
-    int64_t *atom_start, *edge_start, *batch, *row_start, *edges;
-    float *pos_ij, *rvlen;
+    // memory whose size depends on atoms and crystals only
+    int64_t *atom_start, *edge_start, *batch, *row_start;
+    float *rvlen, *rvecs, *vcell;
     int32_t *row_order;
     unsigned *tickets;
     unsigned char *embed;
-    void *lists;
     float *x[MAX_LAYERS + 1];
     LayerSaved layer[MAX_LAYERS];
     float *pooled, *hid;
     size_t bytes;
+    // memory whose size depends on the edges
+    int64_t *edges;
+    float *pos_ij, *kr, *phi_reci;
+    void *lists;
+    size_t edge_bytes;
 };
-Saved carve_saved(const cf_train_desc &d, void *memory, int64_t N, int64_t B, int64_t E)
+Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64_t N, int64_t B, int64_t E)
 {
     Carver c{static_cast<char *>(memory)};
     Saved s{};
@@ -211,13 +261,12 @@ Saved carve_saved(const cf_train_desc &d, void *memory, int64_t N, int64_t B, in
     s.edge_start = c.take<int64_t>(B + 1);
     s.batch = c.take<int64_t>(N);
     s.row_start = c.take<int64_t>(N + 1);
-    s.edges = c.take<int64_t>(2 * E);
-    s.pos_ij = c.take<float>(3 * E);
     s.rvlen = c.take<float>(3 * B);
+    s.rvecs = c.take<float>(9 * B);
+    s.vcell = c.take<float>(B);
     s.row_order = c.take<int32_t>(N);
     s.tickets = c.take<unsigned>(MAX_LAYERS);
     s.embed = c.take<unsigned char>(tc_image_bytes(1));
-    s.lists = c.take<char>(term_list_workspace_bytes(N, E));
     const size_t image = tc_image_bytes(tc_layer_blocks((int)d.ff_dim));
     for (int l = 0; l < d.num_layers; ++l) {
         LayerSaved &y = s.layer[l];
@@ -225,9 +274,9 @@ Saved carve_saved(const cf_train_desc &d, void *memory, int64_t N, int64_t B, in
         y.forward = c.take<unsigned char>(image);
         y.backward = c.take<unsigned char>(image);
         y.q = c.take<float>(N * CH); y.k = c.take<float>(N * CH); y.v = c.take<float>(N * CH);
-        y.a = c.take<float>(N * HEADS); y.lse = c.take<float>(N * HEADS); y.logit = c.take<float>(E * HEADS);
+        y.a = c.take<float>(N * HEADS); y.lse = c.take<float>(N * HEADS);
         y.attn = c.take<float>(N * CH);
-        y.psi = d.K > 0 ? c.take<float>(N * HEADS * d.K) : nullptr;
+        y.psi = d.K > 0 && domain_of(d, l) == REAL ? c.take<float>(N * HEADS * d.K) : nullptr;
         y.y = c.take<float>(N * CH);
         y.h = c.take<float>(N * d.ff_dim);
     }
@@ -235,6 +284,29 @@ Saved carve_saved(const cf_train_desc &d, void *memory, int64_t N, int64_t B, in
     s.pooled = c.take<float>(B * CH);
     s.hid = c.take<float>(B * d.hidden);
     s.bytes = c.used;
+    Carver e{static_cast<char *>(edge_memory)};
+    s.edges = e.take<int64_t>(2 * E);
+    s.pos_ij = e.take<float>(3 * E);
+    bool fused = false, split = false;
+    for (int l = 0; l < d.num_layers; ++l) {
+        LayerSaved &y = s.layer[l];
+        const Domain dom = domain_of(d, l);
+        fused = fused || dom == REAL;
+        split = split || dom != REAL;
+        if (dom == REAL) {
+            y.logit = e.take<float>(E * HEADS);
+        } else {
+            y.phi_real = dom == MULTIHEAD ? e.take<float>(E * HEADS) : nullptr;
+            y.sum_reci = e.take<float>(E * HEADS);
+            y.phi = e.take<float>(E * HEADS);
+            y.values = has_values(d, l) ? e.take<float>(E * CH) : nullptr;
+            y.prob = e.take<float>(E * HEADS);
+        }
+    }
+    s.kr = split ? e.take<float>(3 * E) : nullptr;
+    s.phi_reci = split ? e.take<float>(E * HEADS) : nullptr;
+    s.lists = fused ? e.take<char>(term_list_workspace_bytes(N, E)) : nullptr;
+    s.edge_bytes = e.used;
     return s;
 }
 
@@ -245,6 +317,7 @@ struct Scratch {
     float *gx[MAX_LAYERS + 1];
     LayerGrads layer[MAX_LAYERS];
     float *glogit, *ghid, *partial, *pe_partial;
+    float *gphi, *g_real, *g_reci, *gvalues, *ga_reci, *pair;  // the operator pair's backward
     int shares;
     size_t bytes;
 };
@@ -263,6 +336,17 @@ Scratch carve_scratch(const cf_train_desc &d, void *memory, int64_t N, int64_t B
     }
     s.gx[d.num_layers] = c.take<float>(N * CH);
     s.glogit = c.take<float>(E * HEADS);
+    bool split = false, values = false;
+    for (int l = 0; l < d.num_layers; ++l) {
+        split = split || domain_of(d, l) != REAL;
+        values = values || (domain_of(d, l) != REAL && has_values(d, l));
+    }
+    if (split) {
+        s.gphi = c.take<float>(E * HEADS); s.g_real = c.take<float>(E * HEADS); s.g_reci = c.take<float>(E * HEADS);
+        s.ga_reci = c.take<float>(N * HEADS);
+        s.gvalues = values ? c.take<float>(E * CH) : nullptr;
+        s.pair = c.take<float>(values ? (size_t)cf_lattice_sum_bwd_proj_floats(E) : (size_t)E * HEADS);
+    }
     s.ghid = c.take<float>(B * d.hidden);
     const int jobs = train_jobs(d);
     size_t most = 0;
@@ -291,16 +375,24 @@ int check_desc(const cf_train_desc *d, const char *who)
                "%s: head of %lld hidden units, %lld targets (a multiple of 128 up to 1024)", who, (long long)d->hidden, (long long)d->targets);
     CF_REQUIRE(d->feature_dim >= 1 && d->feature_dim <= 128, CF_ERR_UNSUPPORTED, "%s: %d features (1..128)", who, (int)d->feature_dim);
     CF_REQUIRE(d->K == 0 || d->K == 64, CF_ERR_UNSUPPORTED, "%s: K=%lld, only K in {0,64} is compiled", who, (long long)d->K);
+    for (int l = 0; l < d->num_layers; ++l) {
+        const double dom = d->scalars[SCALARS * l + 8];
+        CF_REQUIRE(dom == REAL || ((dom == RECI || dom == RECI_INVERSE || dom == MULTIHEAD) && d->lattice_range <= 6), CF_ERR_UNSUPPORTED,
+                   "%s: layer %d has domain code %g (0..3; lattice_range up to 6 for the reciprocal ones)", who, l, dom);
+    }
     CF_REQUIRE(d->lattice_range >= 0 && d->lattice_range <= CF_MAX_RANGE && d->minimum_range >= 0, CF_ERR_RANGE,
                "%s: lattice_range %d outside [0,%d]", who, (int)d->lattice_range, CF_MAX_RANGE);
     return CF_OK;
 }
-int check_batch(const cf_train_batch *b, const char *who)
+int check_batch(const cf_train_batch *b, const char *who, bool edges_known)
 {
     CF_REQUIRE(b != nullptr, CF_ERR_INVALID, "%s: null batch", who);
-    CF_REQUIRE(b->N >= 1 && b->B >= 1 && b->E >= 1 && b->B <= (1 << 20), CF_ERR_INVALID, "%s: empty batch or too many crystals", who);
-    CF_REQUIRE(b->max_atoms >= 1 && b->max_atoms <= 1024, CF_ERR_RANGE, "%s: max_atoms=%lld outside [1,1024]", who, (long long)b->max_atoms);
+    CF_REQUIRE(b->N >= 1 && b->B >= 1 && b->B <= (1 << 20), CF_ERR_INVALID, "%s: empty batch or too many crystals", who);
     CF_REQUIRE(b->features && b->pos && b->trans && b->sizes && b->saved, CF_ERR_INVALID, "%s: null pointer", who);
+    if (!edges_known) return CF_OK;
+    CF_REQUIRE(b->E >= 1 && b->max_atoms >= 1 && b->max_atoms <= 1024, CF_ERR_RANGE, "%s: E=%lld, max_atoms=%lld (1..1024)", who,
+               (long long)b->E, (long long)b->max_atoms);
+    CF_REQUIRE(b->saved_edges, CF_ERR_INVALID, "%s: null pointer", who);
     return CF_OK;
 }
 
@@ -310,8 +402,9 @@ enum { W_Q, W_K, W_V, B_IN, W_POS, W_PE, W_O, B_O, W_1, B_1, W_2, B_2, PER_LAYER
 bool lists_of(const cf_train_desc &d, const Saved &s, int64_t N, int64_t E, TermList &list, float &a_widest)
 {
     a_widest = -INFINITY;
-    for (int l = 0; l < d.num_layers; ++l) a_widest = fmaxf(a_widest, (float)(d.scalars[6 * l + 4] * d.scalars[6 * l + 2]));
-    if (!(weight_floor_log2() > -200.0f) || !(a_widest < 0.0f)) return false;
+    for (int l = 0; l < d.num_layers; ++l)
+        if (domain_of(d, l) == REAL) a_widest = fmaxf(a_widest, (float)(d.scalars[SCALARS * l + 4] * d.scalars[SCALARS * l + 2]));
+    if (s.lists == nullptr || !(weight_floor_log2() > -200.0f) || !(a_widest < 0.0f)) return false;
     int *start, *count;
     float *dmin;
     unsigned long long *cursor;
@@ -339,10 +432,16 @@ int launch_projection_grad(const float *gv, const float *psi, long long rows, fl
 }
 }  // namespace cf
 
-extern "C" int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E)
+extern "C" int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B)
 {
     if (cf::check_desc(desc, "cf_train_saved_bytes") != CF_OK) return -1;
-    return (int64_t)cf::carve_saved(*desc, nullptr, N, B, E).bytes;
+    return (int64_t)cf::carve_saved(*desc, nullptr, nullptr, N, B, 0).bytes;
+}
+
+extern "C" int64_t cf_train_edge_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E)
+{
+    if (cf::check_desc(desc, "cf_train_edge_bytes") != CF_OK) return -1;
+    return (int64_t)cf::carve_saved(*desc, nullptr, nullptr, N, B, E).edge_bytes;
 }
 
 extern "C" int64_t cf_train_scratch_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E)
@@ -351,48 +450,114 @@ extern "C" int64_t cf_train_scratch_bytes(const cf_train_desc *desc, int64_t N, 
     return (int64_t)cf::carve_scratch(*desc, nullptr, N, B, E).bytes;
 }
 
-extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, float *y, void *stream)
+namespace cf {
+namespace {
+
+// weight images of all layers, one direction (with the embedding's in the forward one)
+int pack_all(const cf_train_desc &d, const Saved &w, bool forward, cudaStream_t s)
+{
+    static thread_local PackJob job;
+    const int L = d.num_layers, ff = (int)d.ff_dim, blocks = tc_layer_blocks(ff);
+    int count = 0, rc = CF_OK;
+    if (forward) pack_embedding(job, count, w.embed, d.weights[PER_LAYER * L], d.feature_dim);
+    for (int l = 0; l < L && rc == CF_OK; ++l) {
+        const float *const *p = d.weights + PER_LAYER * l;
+        if (count + blocks > PACK_MAX) {
+            rc = launch_pack(job, count, s);
+            count = 0;
+        }
+        (forward ? pack_layer_forward : pack_layer_backward)(job, count, forward ? w.layer[l].forward : w.layer[l].backward, ff, p[W_Q],
+                                                             p[W_K], p[W_V], p[W_O], p[W_1], p[W_2]);
+    }
+    return rc == CF_OK ? launch_pack(job, count, s) : rc;
+}
+
+template <class Args>
+void width_scalars(Args &t, const cf_train_desc &d, int l)
+{
+    const double *sc = d.scalars + SCALARS * l;
+    t.gauss_scale = (float)sc[0]; t.gauss_shift = (float)sc[1]; t.a_factor = (float)sc[2];
+    t.elu_beta = (float)sc[3]; t.lower_bound = (float)sc[4];
+    t.a_factor_hi = (float)sc[6]; t.lower_bound_hi = (float)sc[7];
+    t.inverse = domain_of(d, l) == RECI_INVERSE;
+}
+
+// the dense kernel before layer l's attention (l = num_layers: after the last one)
+int forward_boundary(const cf_train_desc &d, const cf_train_batch &b, const Saved &w, int l, cudaStream_t s)
+{
+    DenseForward t{};
+    t.N = b.N; t.ff = (int)d.ff_dim; t.chained = l > 0; t.weights_fresh = true;
+    t.x_out = w.x[l];
+    if (l > 0) {
+        const LayerSaved &y = w.layer[l - 1];
+        const float *const *p = d.weights + PER_LAYER * (l - 1);
+        t.tail = y.forward; t.attn = y.attn; t.bo = p[B_O]; t.b1 = p[B_1]; t.b2 = p[B_2];
+        t.x_in = w.x[l - 1]; t.y_save = y.y; t.h_save = y.h;
+    } else {
+        t.embed = w.embed; t.features = b.features; t.feature_dim = d.feature_dim;
+    }
+    if (l < d.num_layers) {
+        const LayerSaved &y = w.layer[l];
+        const float *const *p = d.weights + PER_LAYER * l;
+        t.head = y.forward; t.bqkv = p[B_IN]; t.w_pos = p[W_POS];
+        width_scalars(t, d, l);
+        t.q = y.q; t.k = y.k; t.v = y.v; t.a = y.a;
+    }
+    return launch_dense_forward(t, s);
+}
+
+struct TrainBegin {
+    const cf_train_desc *d;
+    const cf_train_batch *b;
+    const Saved *w;
+    cudaStream_t s;
+};
+int train_begin_launch(void *arg)
+{
+    const TrainBegin &t = *static_cast<const TrainBegin *>(arg);
+    const int rc = pack_all(*t.d, *t.w, true, t.s);
+    return rc == CF_OK ? forward_boundary(*t.d, *t.b, *t.w, 0, t.s) : rc;
+}
+
+unsigned blocks_of(long long threads) { return (unsigned)((threads + 255) / 256); }
+
+}  // namespace
+}  // namespace cf
+
+extern "C" int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **inputs_event, void *stream)
+{
+    using namespace cf;
+    int rc = check_desc(desc, "cf_train_begin");
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_begin", false);
+    if (rc != CF_OK) return rc;
+    CF_REQUIRE(counts && inputs_event, CF_ERR_INVALID, "cf_train_begin: null pointer");
+    const Saved w = carve_saved(*desc, batch->saved, nullptr, batch->N, batch->B, 0);
+    TrainBegin arg{desc, batch, &w, as_stream(stream)};
+    return read_sizes_beside(batch->sizes, batch->B, counts, as_stream(stream), train_begin_launch, &arg, inputs_event);
+}
+
+extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *inputs_event, float *y, void *stream)
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_forward");
-    if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward");
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward", true);
     if (rc != CF_OK) return rc;
-    CF_REQUIRE(y != nullptr, CF_ERR_INVALID, "cf_train_forward: null pointer");
+    CF_REQUIRE(y && inputs_event, CF_ERR_INVALID, "cf_train_forward: null pointer");
     const cf_train_desc &d = *desc;
     const cf_train_batch &b = *batch;
     const int64_t N = b.N, B = b.B, E = b.E;
-    const int L = d.num_layers, ff = (int)d.ff_dim;
+    const int L = d.num_layers;
     cudaStream_t s = as_stream(stream);
-    Saved w = carve_saved(d, b.saved, N, B, E);
+    const Saved w = carve_saved(d, b.saved, b.saved_edges, N, B, E);
     const float *const *tail_weights = d.weights + PER_LAYER * L;
 
-    // ---- weight images, both directions
-    {
-        static thread_local PackJob job;
-        int count = 0;
-        auto flush = [&](int need) {
-            if (rc == CF_OK && count + need > PACK_MAX) {
-                rc = launch_pack(job, count, s);
-                count = 0;
-            }
-        };
-        pack_embedding(job, count, w.embed, tail_weights[0], (int)d.feature_dim);
-        const int blocks = tc_layer_blocks(ff);
-        for (int dir = 0; dir < 2; ++dir)
-            for (int l = 0; l < L; ++l) {
-                const float *const *p = d.weights + PER_LAYER * l;
-                flush(blocks);
-                if (dir == 0) pack_layer_forward(job, count, w.layer[l].forward, ff, p[W_Q], p[W_K], p[W_V], p[W_O], p[W_1], p[W_2]);
-                else pack_layer_backward(job, count, w.layer[l].backward, ff, p[W_Q], p[W_K], p[W_V], p[W_O], p[W_1], p[W_2]);
-            }
-        if (rc == CF_OK) rc = launch_pack(job, count, s);
-        if (rc != CF_OK) return rc;
-    }
-    // ---- geometry and term lists
-    if (cudaMemsetAsync(w.tickets, 0, sizeof(unsigned) * MAX_LAYERS, s) != cudaSuccess) return launch_status("cf_train_forward: tickets");
+    // ---- geometry, term lists and the backward's weight images beside the first dense block
+    cudaStream_t prep = early_prep_stream(inputs_event, nullptr);
+    CF_REQUIRE(prep != nullptr, CF_ERR_CUDA, "cf_train_forward: the side stream could not be created");
+    if (cudaMemsetAsync(w.tickets, 0, sizeof(unsigned) * MAX_LAYERS, prep) != cudaSuccess) return launch_status("cf_train_forward: tickets");
     bool ordered = false;
     rc = launch_prepare_all(b.pos, b.trans, b.sizes, w.atom_start, w.edge_start, B, N, E, w.batch, w.edges, w.row_start, w.pos_ij, w.rvlen,
-                            d.order_reach, w.row_order, &ordered, s);
+                            d.order_reach, w.row_order, &ordered, prep, w.rvecs, w.vcell);
     if (rc != CF_OK) return rc;
     const int32_t *order = ordered ? w.row_order : nullptr;
     const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
@@ -408,42 +573,42 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
         tb.window = list.window;
         term_list_carve(w.lists, N, E, &tb.start, &tb.count, &tb.dmin, &tb.cursor, &tb.pool);
         tb.capacity = (long long)term_pool_entries(N, E);
-        rc = launch_term_list_build(tb, s);
+        rc = launch_term_list_build(tb, prep);
         if (rc != CF_OK) return rc;
     }
+    if (w.kr != nullptr) rc = cf_reci_phase(w.pos_ij, w.rvecs, w.batch, w.edges, E, w.kr, prep);
+    if (rc == CF_OK) rc = join_early_prep(s);
+    if (rc == CF_OK) rc = pack_all(d, w, false, prep);  // (joined before the backward, below)
     // ---- layers
-    for (int l = 0; l <= L && rc == CF_OK; ++l) {
-        DenseForward t{};
-        t.N = N; t.ff = ff; t.chained = l > 0; t.weights_fresh = true;
-        t.x_out = w.x[l];
-        if (l > 0) {
-            const LayerSaved &y = w.layer[l - 1];
-            const float *const *p = d.weights + PER_LAYER * (l - 1);
-            t.tail = y.forward; t.attn = y.attn; t.bo = p[B_O]; t.b1 = p[B_1]; t.b2 = p[B_2];
-            t.x_in = w.x[l - 1]; t.y_save = y.y; t.h_save = y.h;
+    for (int l = 0; l < L && rc == CF_OK; ++l) {
+        const LayerSaved &t = w.layer[l];
+        const Domain dom = domain_of(d, l);
+        const double dist_max = d.scalars[SCALARS * l + 5];
+        if (dom == REAL) {
+            rc = infinite_attn_fwd_impl(t.q, t.k, t.v, t.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
+                                        HEAD_DIM, E, d.K, b.max_atoms, dist_max, d.wscale, d.weights[PER_LAYER * l + W_PE],
+                                        d.cutoff_radius, d.lattice_range, d.minimum_range, t.attn, t.logit, t.lse, t.psi, order,
+                                        listed ? &list : nullptr, w.tickets + l, s, true);
         } else {
-            t.embed = w.embed; t.features = b.features; t.feature_dim = (int)d.feature_dim;
+            if (dom == MULTIHEAD)
+                rc = cf_lattice_sum_fwd(t.a, 0, w.pos_ij, b.trans, w.batch, w.edges, N, HEADS, E, d.K, dist_max, d.wscale,
+                                        d.weights[PER_LAYER * l + W_PE], 1, HEAD_DIM, rvlen, d.cutoff_radius, d.lattice_range,
+                                        d.minimum_range, t.phi_real, t.values, s);
+            float *phi_reci = dom == MULTIHEAD ? w.phi_reci : t.phi;
+            if (rc == CF_OK)
+                rc = cf_reci_sum_fwd(t.a, w.kr, w.rvecs, w.vcell, w.batch, w.row_start, N, HEADS, E, d.lattice_range, phi_reci, t.sum_reci, s);
+            if (dom == MULTIHEAD && rc == CF_OK)
+                merge_phi_kernel<<<blocks_of(16 * E), 256, 0, s>>>(reinterpret_cast<const float4 *>(t.phi_real),
+                                                                   reinterpret_cast<const float4 *>(phi_reci),
+                                                                   reinterpret_cast<float4 *>(t.phi), reinterpret_cast<float4 *>(t.values), E);
+            if (rc == CF_OK) rc = cf_fused_attn_fwd(t.q, t.k, t.v, t.phi, t.values, w.edges, w.row_start, N, HEADS, HEAD_DIM, E, t.prob, t.attn, s);
         }
-        if (l < L) {
-            const LayerSaved &y = w.layer[l];
-            const float *const *p = d.weights + PER_LAYER * l;
-            const double *sc = d.scalars + 6 * l;
-            t.head = y.forward; t.bqkv = p[B_IN]; t.w_pos = p[W_POS];
-            t.gauss_scale = (float)sc[0]; t.gauss_shift = (float)sc[1]; t.a_factor = (float)sc[2];
-            t.elu_beta = (float)sc[3]; t.lower_bound = (float)sc[4];
-            t.q = y.q; t.k = y.k; t.v = y.v; t.a = y.a;
-        }
-        rc = launch_dense_forward(t, s);
-        if (rc != CF_OK || l == L) break;
-        const LayerSaved &y = w.layer[l];
-        rc = infinite_attn_fwd_impl(y.q, y.k, y.v, y.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
-                                    HEAD_DIM, E, d.K, b.max_atoms, d.scalars[6 * l + 5], d.wscale, d.weights[PER_LAYER * l + W_PE],
-                                    d.cutoff_radius, d.lattice_range, d.minimum_range, y.attn, y.logit, y.lse, y.psi, order,
-                                    listed ? &list : nullptr, w.tickets + l, s, true);
+        if (rc == CF_OK) rc = forward_boundary(d, b, w, l + 1, s);
     }
-    if (rc != CF_OK) return rc;
-    return launch_pool_head(w.x[L], w.atom_start, tail_weights[1], tail_weights[2], tail_weights[3], tail_weights[4], (int)d.hidden,
-                            (int)d.targets, B, y, w.pooled, w.hid, true, s);
+    if (rc == CF_OK)
+        rc = launch_pool_head(w.x[L], w.atom_start, tail_weights[1], tail_weights[2], tail_weights[3], tail_weights[4], (int)d.hidden,
+                              (int)d.targets, B, y, w.pooled, w.hid, true, s);
+    return rc == CF_OK ? join_early_prep(s) : rc;
 }
 
 extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, const float *gy, void *scratch,
@@ -451,7 +616,7 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_backward");
-    if (rc == CF_OK) rc = check_batch(batch, "cf_train_backward");
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_backward", true);
     if (rc != CF_OK) return rc;
     CF_REQUIRE(gy && scratch && grads, CF_ERR_INVALID, "cf_train_backward: null pointer");
     const cf_train_desc &d = *desc;
@@ -459,7 +624,7 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
     const int64_t N = b.N, B = b.B, E = b.E;
     const int L = d.num_layers, ff = (int)d.ff_dim, hidden = (int)d.hidden, targets = (int)d.targets;
     cudaStream_t s = as_stream(stream);
-    const Saved w = carve_saved(d, b.saved, N, B, E);
+    const Saved w = carve_saved(d, b.saved, b.saved_edges, N, B, E);
     Scratch g = carve_scratch(d, scratch, N, B, E);
     const float *const *tail_weights = d.weights + PER_LAYER * L;
     float *const *tail_grads = grads + PER_LAYER * L;
@@ -479,10 +644,8 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
         if (l + 1 < L) {  // head of layer l + 1
             const LayerSaved &y = w.layer[l + 1];
             const LayerGrads &gg = g.layer[l + 1];
-            const double *sc = d.scalars + 6 * (l + 1);
             t.head = y.backward; t.q = y.q; t.w_pos = d.weights[PER_LAYER * (l + 1) + W_POS];
-            t.gauss_scale = (float)sc[0]; t.gauss_shift = (float)sc[1]; t.a_factor = (float)sc[2];
-            t.elu_beta = (float)sc[3]; t.lower_bound = (float)sc[4];
+            width_scalars(t, d, l + 1);
             t.gq = gg.gq; t.gk = gg.gk; t.gv = gg.gv; t.ga = gg.ga; t.g_res = gg.gy;
         }
         if (l >= 0) {
@@ -494,10 +657,34 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
         if (rc != CF_OK || l < 0) break;
         const LayerSaved &y = w.layer[l];
         const LayerGrads &gg = g.layer[l];
-        rc = infinite_attn_bwd_impl(y.q, y.k, y.v, y.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
-                                    HEAD_DIM, E, d.K, b.max_atoms, d.scalars[6 * l + 5], d.wscale, d.weights[PER_LAYER * l + W_PE],
-                                    d.cutoff_radius, d.lattice_range, d.minimum_range, y.logit, y.lse, y.attn, gg.gattn, gg.gq, gg.gk,
-                                    gg.gv, gg.ga, g.glogit, order, listed ? &list : nullptr, s);
+        const double dist_max = d.scalars[SCALARS * l + 5];
+        if (domain_of(d, l) == REAL) {
+            rc = infinite_attn_bwd_impl(y.q, y.k, y.v, y.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
+                                        HEAD_DIM, E, d.K, b.max_atoms, dist_max, d.wscale, d.weights[PER_LAYER * l + W_PE],
+                                        d.cutoff_radius, d.lattice_range, d.minimum_range, y.logit, y.lse, y.attn, gg.gattn, gg.gq, gg.gk,
+                                        gg.gv, gg.ga, g.glogit, order, listed ? &list : nullptr, s);
+            continue;
+        }
+        const bool multi = domain_of(d, l) == MULTIHEAD;
+        rc = cf_fused_attn_bwd(y.q, y.k, y.v, y.values, w.edges, w.row_start, N, HEADS, HEAD_DIM, E, y.prob, y.attn, gg.gattn, gg.gq, gg.gk,
+                               gg.gv, g.gphi, y.values != nullptr ? g.gvalues : nullptr, s);
+        if (multi && rc == CF_OK) {
+            split_gphi_kernel<<<blocks_of(16 * E), 256, 0, s>>>(reinterpret_cast<const float4 *>(g.gphi), reinterpret_cast<float4 *>(g.g_real),
+                                                                reinterpret_cast<float4 *>(g.g_reci),
+                                                                reinterpret_cast<float4 *>(y.values != nullptr ? g.gvalues : nullptr), E);
+            if (y.values != nullptr)
+                rc = cf_lattice_sum_bwd_proj(y.a, w.pos_ij, b.trans, w.batch, w.edges, w.row_start, y.phi_real, g.g_real, g.gvalues,
+                                             d.weights[PER_LAYER * l + W_PE], N, HEADS, E, d.K, dist_max, d.wscale, rvlen, d.cutoff_radius,
+                                             d.lattice_range, d.minimum_range, gg.ga, grads[PER_LAYER * l + W_PE], g.pair, s);
+            else
+                rc = cf_lattice_sum_bwd(y.a, w.pos_ij, b.trans, w.batch, w.edges, w.row_start, y.phi_real, g.g_real, nullptr, N, HEADS, E, 0,
+                                        dist_max, d.wscale, rvlen, d.cutoff_radius, d.lattice_range, d.minimum_range, gg.ga, nullptr, g.pair, s);
+        }
+        if (rc == CF_OK)
+            rc = cf_reci_sum_bwd(y.a, w.kr, w.rvecs, w.batch, w.row_start, multi ? g.g_reci : g.gphi, y.sum_reci, N, HEADS, E, d.lattice_range,
+                                 multi ? g.ga_reci : gg.ga, s);
+        if (multi && rc == CF_OK)
+            merge_ga_kernel<<<blocks_of(N), 256, 0, s>>>(reinterpret_cast<const float4 *>(g.ga_reci), reinterpret_cast<float4 *>(gg.ga), N);
     }
     if (rc != CF_OK) return rc;
     // ---- value encoding and width weights

@@ -206,13 +206,13 @@ class CrystalformerEncoderCUDA(Module):
     def _native_ok(self) -> bool:
         return not self.training and not torch.is_grad_enabled() and self._native_model()
 
-    def _native_model(self) -> bool:
-        """Whether the layers are what the one-call paths implement (inference and training)."""
+    def _native_model(self, domains=("real",)) -> bool:
+        """Whether the layers are what the one-call paths implement (inference: real-space layers; training: any domain)."""
         if self.norm is not None or self.d_model != 128 or self.nhead != 8:
             return False
         for layer in self.layers:
             att, P = layer.self_attn, layer.self_attn.params
-            if not (P.domain == "real" and P.positive_func.startswith("elu") and P.gauss_state == "q" and P.normalize_gauss and att.fused
+            if not (P.domain in domains and P.positive_func.startswith("elu") and P.gauss_state == "q" and P.normalize_gauss and att.fused
                     and P.value_pe_condproj == "no" and P.norm_func_mode == 0 and att.kdim == 128 and att.vdim == 128
                     and att.in_proj_bias is not None and layer.activation is F.relu and not layer.norm_first
                     and isinstance(layer.norm1, Identity)):

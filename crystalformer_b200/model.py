@@ -17,7 +17,7 @@ from . import _lib
 from .cuda_funcs import IrregularMeanCUDA
 from .encoder import MAX_IMAGE_FF, BatchGeometry, CrystalformerEncoderCUDA, image_pointer, pack_dense_embedding, pack_dense_weight
 from .params import DEFAULT_MODEL_PARAMS, LatticeformerParams
-from .training import ModelWatch, OfThisModel, train_step
+from .training import DOMAINS, ModelWatch, OfThisModel, train_step
 
 
 def default_params(**overrides) -> types.SimpleNamespace:
@@ -288,7 +288,7 @@ class Latticeformer(nn.Module):
                 and self._native_ok():
             return self._forward_native(data, counts, gather, inputs_ready=inputs_ready)
         if geometry is None and torch.is_grad_enabled() and data.pos.is_cuda and self._native_shell() \
-                and self.encoder._native_model():
+                and self.encoder._native_model(DOMAINS):
             y = train_step(self, data, counts)
             if y is not None:
                 if gather is not None:

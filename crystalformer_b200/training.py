@@ -45,13 +45,16 @@ class ModelWatch:
         key = [P.lattice_range, P.minimum_range, P.adaptive_cutoff_sigma, P.gauss_lb_real, str(P.scale_real), P.value_pe_dist_real,
                P.value_pe_width_scale, P.value_pe_dist_max]
         for Q in self.layer_settings:
-            key += (Q.positive_func, Q.gauss_lb_real, Q.scale_real, Q.value_pe_dist_max)
+            key += (Q.positive_func, Q.gauss_lb_real, Q.scale_real, Q.value_pe_dist_max, Q.gauss_lb_reci, Q.scale_reci)
         key += [t.data_ptr() for t in self.tensors]
         return key + [t._version for t in self.tensors] if self.versions else key
 
     def current(self) -> bool:
         return all([d.get(n) is c for d, n, c in self.children]) and all([d.get(n) is t for d, n, t in self.places]) \
             and self.now() == self.key
+
+
+DOMAINS = ("real", "reci", "RECI", "multihead")  # in the order of the library's codes
 
 
 class TrainPlan:
@@ -70,7 +73,9 @@ class TrainPlan:
             beta = float(Q.positive_func.split("=")[1]) if "=" in Q.positive_func else 1.0
             dist_max = Q.value_pe_dist_max if Q.value_pe_dist_max >= 0 else -Q.value_pe_dist_max * Q.scale_real
             gs = att.gauss_scale.detach().cpu().tolist()
-            scalars += [gs[0], gs[1], -0.5 * Q.scale_real ** -2, beta, Q.gauss_lb_real, dist_max]
+            real, reci = (-0.5 * Q.scale_real ** -2, Q.gauss_lb_real), (-0.5 * Q.scale_reci ** 2, Q.gauss_lb_reci)
+            low, high = {"real": (real, real), "multihead": (real, reci)}.get(Q.domain, (reci, reci))
+            scalars += [gs[0], gs[1], low[0], beta, low[1], dist_max, *high, DOMAINS.index(Q.domain)]
         ordered += [model.input_embeddings.weight, model.mlp[0].weight, model.mlp[0].bias, model.mlp[3].weight, model.mlp[3].bias]
         self.params = [p for p in ordered if p is not None]
         self.watch = ModelWatch(model, versions=False)
@@ -116,32 +121,45 @@ def supported(model) -> bool:
         return False
     for layer in enc.layers:
         att = layer.self_attn
-        if layer.linear1.out_features != ff or att.params.value_pe_dist_real not in (0, 64) or att.params.gauss_lb_real <= 0 \
-                or att.out_proj.bias is None or (att.pe_dist_proj is not None and tuple(att.pe_dist_proj.shape) != (1, 8, 16, 64)) \
-                or (att.pe_dist_proj is None) != (att.params.value_pe_dist_real == 0):
+        Q = att.params
+        bins = Q.value_pe_dist_real if Q.domain in ("real", "multihead") else 0
+        if layer.linear1.out_features != ff or bins not in (0, 64) or Q.gauss_lb_real <= 0 or Q.gauss_lb_reci <= 0 \
+                or isinstance(Q.scale_real, (list, tuple)) or isinstance(Q.scale_reci, (list, tuple)) \
+                or (Q.domain != "real" and Q.lattice_range > 6) or att.out_proj.bias is None \
+                or (tuple(att.pe_dist_proj.shape) if att.pe_dist_proj is not None else None) != ((1, 8, 16, 64) if bins else None):
             return False
         if any(isinstance(m, torch.nn.Dropout) and m.p > 0 for m in (layer.dropout, layer.dropout1, layer.dropout2)) or att.dropout > 0:
             return False
     return all(p.dtype == torch.float32 and p.is_contiguous() and p.device == dev for p in model.parameters())
 
 
+class NotThisBatch(Exception):
+    """The calls do not take the batch (a crystal of more than 1024 atoms, atoms outside every crystal)."""
+
+
 class TrainStep(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, plan: TrainPlan, inputs, counts: Tuple[int, int, int], *params):
+    def forward(ctx, plan: TrainPlan, inputs, counts: Optional[Tuple[int, int, int]], *params):
         feats, pos, trans, sizes = inputs
         dev = pos.device
-        N, E, max_atoms = (int(c) for c in counts)
-        B = sizes.shape[0]
+        N, B = pos.shape[0], sizes.shape[0]
         lib = _lib.load()
-        nbytes = int(lib.cf_train_saved_bytes(ctypes.byref(plan.desc), N, B, E))
-        saved = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        desc = ctypes.byref(plan.desc)
+        saved = torch.empty(int(lib.cf_train_saved_bytes(desc, N, B)), dtype=torch.uint8, device=dev)
         batch = _lib.TrainBatch(features=feats.data_ptr(), pos=pos.data_ptr(), trans=trans.data_ptr(), sizes=sizes.data_ptr(), N=N, B=B,
-                                E=E, max_atoms=max_atoms, saved=saved.data_ptr())
+                                saved=saved.data_ptr())
+        known, event = (ctypes.c_int64 * 3)(*((-1, 0, 0) if counts is None else counts)), ctypes.c_void_p()
         y = torch.empty((B, plan.targets), dtype=torch.float32, device=dev)
         with torch.cuda.device(dev):
-            _lib.call("cf_train_forward", ctypes.byref(plan.desc), ctypes.byref(batch), y.data_ptr(),
-                      torch.cuda.current_stream(dev).cuda_stream)
-        ctx.save_for_backward(saved, feats, pos, trans, sizes)
+            stream = torch.cuda.current_stream(dev).cuda_stream
+            _lib.call("cf_train_begin", desc, ctypes.byref(batch), known, ctypes.byref(event), stream)
+            if known[0] != N or known[2] > 1024:
+                raise NotThisBatch
+            batch.E, batch.max_atoms = known[1], known[2]
+            edges = torch.empty(int(lib.cf_train_edge_bytes(desc, N, B, batch.E)), dtype=torch.uint8, device=dev)
+            batch.saved_edges = edges.data_ptr()
+            _lib.call("cf_train_forward", desc, ctypes.byref(batch), event, y.data_ptr(), stream)
+        ctx.save_for_backward(saved, edges, feats, pos, trans, sizes)
         ctx.step = (plan, batch, plan.versions())
         return y
 
@@ -186,9 +204,10 @@ def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[
     sizes = data.sizes
     if sizes.device != dev or sizes.dtype != torch.int64 or not sizes.is_contiguous():
         sizes = sizes.to(device=dev, dtype=torch.int64).contiguous()
-    if counts is None:
-        host = data.sizes.tolist()
-        counts = (sum(host), sum(n * n for n in host), max(host) if host else 1)
-    if counts[0] < 1 or counts[2] > 1024 or feats.data_ptr() % 16 or plan.params[0].device != dev:
+    if pos.shape[0] < 1 or feats.data_ptr() % 16 or plan.params[0].device != dev or (counts is not None and (
+            counts[0] != pos.shape[0] or counts[2] > 1024)):
         return None
-    return TrainStep.apply(plan, (feats, pos, trans, sizes), counts, *plan.params)
+    try:
+        return TrainStep.apply(plan, (feats, pos, trans, sizes), counts, *plan.params)
+    except NotThisBatch:
+        return None

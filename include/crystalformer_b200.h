@@ -435,20 +435,24 @@ int64_t cf_model_head_floats(int64_t N);
 
 /* ------------------------------------------------------------------------------------------------------------
  * A training step of the whole model (what autograd does through Latticeformer.forward and its backward,
- * models/latticeformer.py:211-302, same configuration as cf_model_forward) in two host calls.
+ * models/latticeformer.py:211-302, same configuration as cf_model_forward, any of the domains) in three host calls.
  *   cf_train_desc  : weights = HOST array of 12 num_layers + 5 device pointers: per layer Wq, Wk, Wv (128,128),
  *                    in_proj_bias (384), lattice_pos_weights (128), pe_dist_proj (8,16,K) or NULL, out_proj.weight,
  *                    out_proj.bias, linear1.weight (ff,128), linear1.bias, linear2.weight (128,ff), linear2.bias; then
- *                    W_embed (128, feature_dim), head W1 (hidden,128), b1, W2 (targets,hidden), b2.  scalars as in
- *                    cf_encoder_forward (6 per layer).  ff_dim a multiple of 128 up to 3328, hidden of 128 up to 1024,
- *                    feature_dim <= 128, up to 32 layers.
- *   cf_train_batch : the inputs of cf_model_forward (N, B, E >= 1, max_atoms <= 1024) and `saved`,
- *                    cf_train_saved_bytes(desc, N, B, E) bytes of 256-byte aligned device memory that the forward fills
- *                    and the backward reads.
- * cf_train_forward writes y (B, targets).  cf_train_backward takes gy (B, targets), scratch of
- * cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of device pointers to the gradients, in the order of the
- * weights (the entry of a NULL weight is not used); every gradient is written, none accumulated.  The weights must not
- * change between the two calls.
+ *                    W_embed (128, feature_dim), head W1 (hidden,128), b1, W2 (targets,hidden), b2.  scalars = HOST array
+ *                    of 9 doubles per layer: gauss_scale, gauss_shift, width factor and elu beta and lower bound of
+ *                    heads 0-3, dist_max, width factor and lower bound of heads 4-7, domain (0 "real", 1 "reci", 2 "RECI",
+ *                    3 "multihead"; the factor is -0.5 / scale_real^2 for real-space heads, -0.5 scale_reci^2 for
+ *                    reciprocal-space ones).  ff_dim a multiple of 128 up to 3328, hidden of 128 up to 1024, feature_dim
+ *                    <= 128, up to 32 layers; lattice_range up to 6 with a reciprocal domain.
+ *   cf_train_batch : the inputs of cf_model_forward and 256-byte aligned device memory that the forward fills and the
+ *                    backward reads: `saved`, cf_train_saved_bytes(desc, N, B) bytes, and `saved_edges`,
+ *                    cf_train_edge_bytes(desc, N, B, E) bytes (E = sum n^2 >= 1, largest crystal max_atoms <= 1024).
+ * cf_train_begin needs N, B and `saved` only: it queues the read-back of the sizes, packs the weights and runs the first
+ * dense block, and returns counts and inputs_event as cf_model_begin does; cf_train_forward then writes y (B, targets).
+ * cf_train_backward takes gy (B, targets), scratch of cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of
+ * device pointers to the gradients, in the order of the weights (the entry of a NULL weight is not used); every gradient
+ * is written, none accumulated.  The weights must not change between the calls.
  * ---------------------------------------------------------------------------------------------------------- */
 typedef struct cf_train_desc {
     int32_t num_layers, lattice_range, minimum_range, feature_dim;
@@ -461,11 +465,13 @@ typedef struct cf_train_batch {
     const float *features, *pos, *trans;
     const int64_t *sizes;
     int64_t N, B, E, max_atoms;
-    void *saved;
+    void *saved, *saved_edges;
 } cf_train_batch;
-int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
+int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B);
+int64_t cf_train_edge_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
 int64_t cf_train_scratch_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
-int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, float *y, void *stream);
+int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **inputs_event, void *stream);
+int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *inputs_event, float *y, void *stream);
 int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, const float *gy, void *scratch,
                       float *const *grads, void *stream);
 

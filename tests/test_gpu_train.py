@@ -36,7 +36,10 @@ def setup(sizes, lengths=(4.0, 12.0), **params):
 
 
 @pytest.mark.parametrize("params", [dict(num_layers=2), dict(num_layers=3, value_pe_dist_real=0), dict(num_layers=1, ff_dim=128),
-                                    dict(num_layers=2, ff_dim=256, targets=["a", "b", "c"], embedding_dim=[256])])
+                                    dict(num_layers=2, ff_dim=256, targets=["a", "b", "c"], embedding_dim=[256]),
+                                    dict(num_layers=2, domain="multihead"), dict(num_layers=1, domain="multihead", value_pe_dist_real=0),
+                                    dict(num_layers=2, domain="reci"), dict(num_layers=2, domain="RECI"),
+                                    dict(num_layers=2, domain="real-reci")])
 @pytest.mark.parametrize("sizes", [[1], [3, 60, 64], [33] * 4 + [1], [100, 128, 129], [7] * 130])
 def test_gradients_equal_the_autograd_path(params, sizes):
     """Row tiles of 128 (one row, a full tile, one more), chunks of 64 rows, crystals of one atom and of more than 64."""
@@ -45,10 +48,12 @@ def test_gradients_equal_the_autograd_path(params, sizes):
     y1, got = step(model, data, target, native=True)
     assert getattr(model, "_train_plan", None) is not None
     assert (y0 - y1).abs().max() < 2e-6
+    # (a single atom's soft-max has no gradient: what is left of q's and k's is rounding of the others)
+    noise = 1e-6 * max(float(g.norm()) for g in ref.values())
     for name in ref:
         scale = ref[name].norm()
         # a hidden unit within rounding of zero may fall on either side of the ReLU: one column of one gradient moves
-        assert (got[name] - ref[name]).norm() <= 2e-3 * scale + 1e-9, (name, float((got[name] - ref[name]).norm() / scale))
+        assert (got[name] - ref[name]).norm() <= 2e-3 * scale + noise, (name, float((got[name] - ref[name]).norm() / scale))
     again = step(model, data, target, native=True)[1]
     assert all(torch.equal(got[n], again[n]) for n in got)  # no atomics in any sum
 
