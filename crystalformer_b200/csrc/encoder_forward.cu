@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "dense_block.cuh"
 #include "dense_tc.cuh"
+#include "infinite_attn_block.cuh"
 #include "row_list.cuh"
 #include "term_list.cuh"
 
@@ -222,7 +223,8 @@ extern "C" int64_t cf_encoder_workspace_floats(int64_t N, int64_t E, int64_t ff_
     // then the term lists: directory (2 ints per edge), allocation cursor, pool (2 floats per entry)
     // (or, for batches of small crystals, the row lists: whichever is larger)
     const size_t lists = cf::term_list_workspace_bytes(N, E), rows = cf::row_list_workspace_bytes(N, E);
-    return N * (384 + 384 + 128 + 8 + 8 + ff_dim) + E * 8 + 64 + (int64_t)((lists > rows ? lists : rows) + 3) / 4;
+    return N * (384 + 384 + 128 + 8 + 8 + ff_dim) + E * 8 + 64 + (int64_t)((lists > rows ? lists : rows) + 3) / 4 +
+           (int64_t)cf::row_blocks_words(N) + 64;
 }
 
 extern "C" int cf_encoder_forward(void *cublas_handle, int num_layers, const float *const *weights, const double *scalars,
@@ -275,6 +277,8 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     // to wait for this stream here.
     bool forked = early_prep;
     unsigned *tickets = nullptr;
+    RowBlocks row_blocks{};
+    bool by_blocks = false;  // term lists and crystals of up to ROW_BLOCK_MAX_ATOMS: the row block kernel
     if (pos_ij != nullptr && weight_floor_log2() > -200.0f) {
         float a_widest = -INFINITY;
         for (int l = 0; l < num_layers; ++l) a_widest = fmaxf(a_widest, (float)(scalars[6 * l + 4] * scalars[6 * l + 2]));
@@ -306,9 +310,14 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                 term_list_carve(logit + E * 8 + 64, N, E, &tb.start, &tb.count, &tb.dmin, &tb.cursor, &tb.pool);
                 tb.capacity = (long long)term_pool_entries(N, E);
                 rc = launch_term_list_build(tb, forked ? side.stream : s);
+                by_blocks = max_atoms > ROW_BLOCK_MIN_ATOMS && max_atoms <= ROW_BLOCK_MAX_ATOMS && num_layers <= ROW_BLOCK_LAYERS && N < (1ll << 31);
+                if (by_blocks && rc == CF_OK) {
+                    row_blocks = row_blocks_carve(workspace + ((cf_encoder_workspace_floats(N, E, ff_dim) - (int64_t)row_blocks_words(N) - 32) & ~3ll), N);
+                    rc = launch_row_blocks(row_blocks, row_order, row_start, edges, N, E, forked ? side.stream : s);
+                }
                 // the row tickets of all layers, zeroed once here instead of by a phi launch per layer (on the main
                 // stream, ahead of the first dense block: the list build is the longer of the two branches)
-                if (K > 0 && num_layers <= 16 && (tickets = row_ticket_block(num_layers)) != nullptr &&
+                if (!by_blocks && K > 0 && num_layers <= 16 && (tickets = row_ticket_block(num_layers)) != nullptr &&
                     cudaMemsetAsync(tickets, 0, sizeof(unsigned) * num_layers, s) != cudaSuccess)
                     tickets = nullptr;
                 lists.pool = tb.pool; lists.start = tb.start; lists.count = tb.count; lists.dmin = tb.dmin; lists.window = tb.window;
@@ -324,6 +333,9 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
             return sorted_attn_impl(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, N, E, max_atoms, dist_max, wscale,
                                     W, cutoff_radius, lattice_range, minimum_range, attn_out, lse_out, row_lists,
                                     l < ROW_SCHED_SLOTS - 1 ? l : ROW_SCHED_SLOTS - 1, l < ROW_SCHED_SLOTS - 1, K, s);
+        if (by_blocks)
+            return block_attn_impl(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, N, B, E, K, max_atoms, dist_max, wscale, W,
+                                   cutoff_radius, lattice_range, minimum_range, attn_out, logit, lse_out, nullptr, lists, row_blocks, l, s);
         return infinite_attn_fwd_impl(q, k, v, a, nullptr, pos_ij, tvecs, rvlen, batch, edges, row_start, N, B, HEADS, HEAD_DIM,
                                       E, K, max_atoms, dist_max, wscale, W, cutoff_radius, lattice_range, minimum_range,
                                       attn_out, logit, lse_out, nullptr, row_order, list, tickets ? tickets + l : nullptr, s, true);

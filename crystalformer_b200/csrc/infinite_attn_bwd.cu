@@ -9,12 +9,11 @@
 // hoisted projection.  The gradient of W is sum_i gout_i (x) psi_row_i, a GEMM done by the caller.
 //
 //   infinite_attn_bwd_rows_kernel  CTA per atom i: recompute q.k, p_ij, then each warp takes a contiguous range of the
-//                                  row's keys; lanes run over (key, translation) terms, survivors are compacted and each
-//                                  lane contracts the 64 basis values of its own term with u_i (shared memory, broadcast
-//                                  reads).  Per-key sums are formed by walking the staged entries in order, so nothing
-//                                  depends on scheduling.  Writes glogit (E,H), ga (N,H), gq (N,H,D).
-//   infinite_attn_bwd_cols_kernel  warp per (key j, head): gk_j, gv_j from glogit and p_ij = exp(logit - lse_i), reading
-//                                  the crystal's n x n block in column order by index arithmetic.
+//                                  row's keys.  Lanes run over (key, translation) terms; those within reach of the widest
+//                                  head are collected, and every lane takes one: its eight joint weights, the contraction
+//                                  of the basis with u_i, and a segmented scan for the sums per key (fixed order, one warp
+//                                  per key).  Writes glogit (E,H), ga (N,H), gq (N,H,D).
+//   infinite_attn_bwd_cols_kernel  gk_j, gv_j from glogit and p_ij = exp(logit - lse_i), eight keys per block.
 #include "lattice_bwd_core.cuh"
 #include "term_list.cuh"
 
@@ -24,6 +23,7 @@ namespace {
 constexpr int THREADS = 128;
 constexpr int WARPS = THREADS / 32;
 constexpr int KBINS = 64;
+constexpr int BWD_RING = 64;  // candidates of a warp: up to 31 left over + 32 offered
 
 struct BwdRowArgs {
     const float *q, *k, *v, *a, *pos, *pos_ij, *tvecs, *rvlen, *W, *logit, *lse, *out, *gout;
@@ -39,12 +39,12 @@ struct BwdRowArgs {
 
 __host__ __device__ inline size_t bwd_row_smem_floats(int max_atoms, bool with_basis)
 {
-    // per atom: rel (4) + c (8) + p (8) + gov (8) + s0 (8); then u (8 x 64), per-warp staging and results, ga partials
-    return (size_t)max_atoms * 36 + (with_basis ? HEADS * U_STRIDE + WARPS * (BWD_STAGE_FLOATS + 32 * 8) : 0) + WARPS * 8 + 16;
+    // per atom: rel (4) + c (8) + p (8) + gov (8) + s0 (8); then u (8 x 64), per-warp candidates, ga partials
+    return (size_t)max_atoms * 36 + (with_basis ? HEADS * U_STRIDE : 0) + WARPS * 2 * BWD_RING + WARPS * 8 + 16;
 }
 
 template <int K>
-__global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const BwdRowArgs p)
+__global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(const BwdRowArgs p)
 {
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -54,10 +54,11 @@ __global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const B
     float *gov = pj + (size_t)p.max_atoms * 8;                         // [max_atoms][8] gout_i . v_j - delta_i
     float *s0 = gov + (size_t)p.max_atoms * 8;                         // [max_atoms][8] sum_n P c, then glogit
     float *u = s0 + (size_t)p.max_atoms * 8;                           // [8][64]
-    float *stage = u + (K > 0 ? HEADS * U_STRIDE : 0) + (K > 0 ? warp * (BWD_STAGE_FLOATS + 32 * 8) : 0);
-    float *res = stage + BWD_STAGE_FLOATS;                             // [32][8] P c of the staged entries
-    float *ga_part = u + (K > 0 ? HEADS * U_STRIDE + WARPS * (BWD_STAGE_FLOATS + 32 * 8) : 0);  // [WARPS][8]
+    float *rings = u + (K > 0 ? HEADS * U_STRIDE : 0);                 // [WARPS][2 BWD_RING]
+    float *ga_part = rings + WARPS * 2 * BWD_RING;                     // [WARPS][8]
     float *delta_s = ga_part + WARPS * 8;                              // [8]
+    CandidateRingOf<BWD_RING> ring;
+    ring.init(rings + warp * 2 * BWD_RING, lane);
 
     for (long long slot = blockIdx.x; slot < p.N; slot += gridDim.x) {
         const long long i = p.row_order ? p.row_order[slot] : slot;
@@ -145,14 +146,18 @@ __global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const B
             a2[h] = __shfl_sync(FULL, a_own, h) * LOG2E;
             pk[h] = __shfl_sync(FULL, pk_own, h);
         }
+        float a2max = a2[0], cmax = -INFINITY;
+#pragma unroll
+        for (int h = 1; h < 8; ++h) a2max = fmaxf(a2max, a2[h]);
+        for (int idx = lane; idx < n * HEADS; idx += 32) cmax = fmaxf(cmax, cj[idx]);
+        cmax = warp_max(cmax);
         float G[8];
 #pragma unroll
         for (int h = 0; h < 8; ++h) G[h] = 0.f;
-        // lanes 0..7 carry the running per-key sum of head (lane) while walking the staged entries in order
-        float run = 0.f;
-        int run_key = -1;
-        // one term per lane: the eight joint weights, their part of ga, and (K > 0) the contraction of the basis with u
-        auto term = [&](bool valid, int j, float d2, int key) {
+        // one term per lane, terms of a key contiguous: the eight joint weights, their part of ga, and (K > 0) the contraction
+        // of the basis with u, summed per key by a segmented scan (a fixed tree over the batch; the last lane of a key's run
+        // adds it to the key's total, which no other warp touches)
+        auto weigh = [&](bool got, int j, float d2, int key) {
             const float4 ca = *reinterpret_cast<const float4 *>(cj + j * 8);
             const float4 cb = *reinterpret_cast<const float4 *>(cj + j * 8 + 4);
             const float4 ga4 = *reinterpret_cast<const float4 *>(gov + j * 8);
@@ -164,47 +169,51 @@ __global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const B
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
                 float eh = fmaf(a2[h], d2, off[h]);
-                if (!valid || (masked && !key_in_box(key, pk[h]))) eh = -INFINITY;
+                if (!got || (masked && !key_in_box(key, pk[h]))) eh = -INFINITY;
                 w[h] = ex2(eh);
                 emax = fmaxf(emax, eh);
                 G[h] = fmaf(w[h] * d2, gj[h], G[h]);
             }
             if (K > 0) {
-                const float x = fast_sqrt(d2) * p.basis.bin_scale;
                 const bool keep = emax > p.basis.floor_log2 && d2 < p.basis.d2_cut;
-                const int cnt = stage_terms(stage, lane, keep, x, d2, j, w);
-                if (cnt > 0) {
-                    if (lane < cnt) {
-                        const float4 *row = reinterpret_cast<const float4 *>(stage + BWD_ENTRY_FLOATS * lane);
-                        const float4 hd = row[0], pa = row[1], pb = row[2];
-                        const float pw[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
-                        float cd[8];
-                        if (K == 64 && p.basis.windowed) basis_dot_window(u, hd.x, p.basis.bin_step, cd);
-                        else basis_dot<(K > 0 ? K : 4)>(u, hd.x, p.basis.bin_step, cd);
-                        float pc[8];
+                if (!__any_sync(FULL, keep)) return;
+                const float x = fast_sqrt(d2) * p.basis.bin_scale;
+                float pc[8];
+                if (keep) {
+                    if (K == 64 && p.basis.windowed) basis_dot_window(u, x, p.basis.bin_step, pc);
+                    else basis_dot<(K > 0 ? K : 4)>(u, x, p.basis.bin_step, pc);
+                }
 #pragma unroll
-                        for (int h = 0; h < 8; ++h) {
-                            pc[h] = pw[h] * cd[h];
-                            G[h] = fmaf(pc[h], hd.y, G[h]);
-                        }
-                        reinterpret_cast<float4 *>(res + 8 * lane)[0] = make_float4(pc[0], pc[1], pc[2], pc[3]);
-                        reinterpret_cast<float4 *>(res + 8 * lane)[1] = make_float4(pc[4], pc[5], pc[6], pc[7]);
+                for (int h = 0; h < 8; ++h) {
+                    pc[h] = keep ? w[h] * pc[h] : 0.f;
+                    G[h] = fmaf(pc[h], d2, G[h]);
+                }
+                const int id = got ? j : -1;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const bool same = __shfl_up_sync(FULL, id, o) == id && lane >= o;
+#pragma unroll
+                    for (int h = 0; h < 8; ++h) {
+                        const float up = __shfl_up_sync(FULL, pc[h], o);
+                        pc[h] += same ? up : 0.f;
                     }
-                    __syncwarp();
-                    if (lane < 8) {  // ordered walk: entries are sorted by key
-                        for (int m = 0; m < cnt; ++m) {
-                            const int key_m = __float_as_int(stage[BWD_ENTRY_FLOATS * m + 2]);
-                            if (key_m != run_key) {
-                                if (run_key >= 0) s0[run_key * 8 + lane] = run;
-                                run = 0.f;
-                                run_key = key_m;
-                            }
-                            run += res[8 * m + lane];
-                        }
-                    }
+                }
+                const int id_next = __shfl_down_sync(FULL, id, 1);  // (every lane takes part; lane 31 gets its own)
+                if (got && (lane == 31 || id_next != id)) {
+                    float4 *dst = reinterpret_cast<float4 *>(s0 + j * 8);
+                    const float4 x0 = dst[0], x1 = dst[1];
+                    dst[0] = make_float4(x0.x + pc[0], x0.y + pc[1], x0.z + pc[2], x0.w + pc[3]);
+                    dst[1] = make_float4(x1.x + pc[4], x1.y + pc[5], x1.z + pc[6], x1.w + pc[7]);
                 }
                 __syncwarp();
             }
+        };
+        // candidates: terms that the widest head and the row's largest offset could bring above the floor
+        auto consume = [&]() {
+            float d2;
+            int key;
+            const bool got = ring.take(d2, key);
+            weigh(got, got ? (key & 2047) : 0, got ? d2 : 0.f, key);  // (a lane without an entry reads whatever the ring held)
         };
         const int list_first = (p.list.pool != nullptr && n > 0) ? p.list.start[e0] : -1;
         if (list_first >= 0) {
@@ -233,7 +242,8 @@ __global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const B
                 if (at + 32 + lane < w_hi) ahead = __ldg(p.list.pool + at + 32 + lane);
                 const int key = __float_as_int(en.y);
                 // (the lists are built for a box that contains every head's: terms outside this row's boxes drop out here)
-                term(live && key_in_box(key, uni), live ? (key & 2047) : k_lo, en.x, key);
+                ring.offer(live && key_in_box(key, uni) && fmaf(a2max, en.x, cmax) > p.basis.floor_log2, en.x, key);
+                while (ring.ready()) consume();
             }
         } else {
             const int R1 = box_r1(uni), R2 = box_r2(uni), R3 = box_r3(uni);
@@ -255,13 +265,14 @@ __global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const B
                 const float dy = fmaf(cell.t3y, f3, fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, r.y)));
                 const float dz = fmaf(cell.t3z, f3, fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, r.z)));
                 const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                int key = 0;
-                if (masked) key = pack_key(0, abs(__float2int_rn(f1)), abs(__float2int_rn(f2)), abs(__float2int_rn(f3)));
-                term(valid, j, d2, key);
+                int key = j;
+                if (masked) key = pack_key(j, abs(__float2int_rn(f1)), abs(__float2int_rn(f2)), abs(__float2int_rn(f3)));
+                ring.offer(valid && fmaf(a2max, d2, cmax) > p.basis.floor_log2, d2, key);
+                while (ring.ready()) consume();
                 walk.step();
             }
         }
-        if (K > 0 && lane < 8 && run_key >= 0) s0[run_key * 8 + lane] = run;
+        while (ring.count > 0) consume();
 #pragma unroll
         for (int h = 0; h < 8; ++h) G[h] = warp_sum(G[h]);
         if (lane < 8) ga_part[warp * 8 + lane] = pick8(G, lane);
@@ -286,30 +297,66 @@ __global__ void __launch_bounds__(THREADS) infinite_attn_bwd_rows_kernel(const B
     }
 }
 
-// gk_j = sum_i glogit_ij q_i, gv_j = sum_i p_ij gout_i with p_ij = exp(logit_ij - lse_i); warp per (key, head).
+// gk_j = sum_i glogit_ij q_i, gv_j = sum_i p_ij gout_i with p_ij = exp(logit_ij - lse_i).  Block = eight consecutive keys (of
+// one crystal at a time), warp = head: a row's values of the eight keys are contiguous in the n x n block, so they are read
+// coalesced, thirty-two rows at a time, and q and gout once for the eight keys (a warp per key and head read them, and the
+// columns with a stride, once per key: 0.11 ms against 0.02 ms at crystals of 100-200 atoms).
+constexpr int COL_KEYS = 8, COL_ROWS = 32;
+constexpr int COL_LD = COL_ROWS * COL_KEYS + 4;  // floats per head (bank skew)
 __global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRowArgs p)
 {
-    const int lane = threadIdx.x & 31, h = threadIdx.x >> 5;
-    const int d = lane & 15, half = lane >> 4;
-    for (long long j = blockIdx.x; j < p.N; j += gridDim.x) {
-        const long long r0 = p.row_start[j];
-        const int n = (int)(p.row_start[j + 1] - r0);
-        if (n == 0) continue;
-        const long long first = p.edges[p.E + r0];
-        const long long c0 = p.row_start[first];
-        const long long jl = j - first;
-        float av = 0.f, ak = 0.f;
-        for (int il = half; il < n; il += 2) {
-            const long long i = first + il, e = c0 + (long long)il * n + jl;
-            const float pr = ex2((p.logit[e * HEADS + h] - p.lse[i * HEADS + h]) * LOG2E);
-            av = fmaf(pr, __ldg(p.gout + (i * HEADS + h) * HEAD_DIM + d), av);
-            ak = fmaf(p.glogit[e * HEADS + h], __ldg(p.q + (i * HEADS + h) * HEAD_DIM + d), ak);
-        }
-        av += __shfl_xor_sync(FULL, av, 16);
-        ak += __shfl_xor_sync(FULL, ak, 16);
-        if (half == 0) {
-            p.gv[(j * HEADS + h) * HEAD_DIM + d] = av;
-            p.gk[(j * HEADS + h) * HEAD_DIM + d] = ak;
+    __shared__ __align__(16) float gs[HEADS * COL_LD], ps[HEADS * COL_LD];
+    const int tid = threadIdx.x, lane = tid & 31, h = tid >> 5;
+    const int d = lane & 15, par = lane >> 4;
+    for (long long tile = blockIdx.x; tile * COL_KEYS < p.N; tile += gridDim.x) {
+        long long j0 = tile * COL_KEYS;
+        const long long tile_end = min(j0 + COL_KEYS, p.N);
+        while (j0 < tile_end) {
+            const long long r0 = p.row_start[j0];
+            const int n = (int)(p.row_start[j0 + 1] - r0);
+            if (n == 0) { ++j0; continue; }
+            const long long first = p.edges[p.E + r0];
+            const long long c0 = p.row_start[first];
+            const int jl = (int)(j0 - first), keys = (int)(min(tile_end, first + n) - j0);
+            float ak[COL_KEYS], av[COL_KEYS];
+#pragma unroll
+            for (int u = 0; u < COL_KEYS; ++u) ak[u] = av[u] = 0.f;
+            for (int i0 = 0; i0 < n; i0 += COL_ROWS) {
+                const int rows = min(COL_ROWS, n - i0);
+                __syncthreads();  // (the previous chunk has been read)
+                for (int idx = tid; idx < rows * 64; idx += 256) {
+                    const int i = idx >> 6, jj = (idx >> 3) & 7, hh = idx & 7;
+                    float g = 0.f, pr = 0.f;
+                    if (jj < keys) {
+                        const long long e = (c0 + (long long)(i0 + i) * n + jl + jj) * HEADS + hh;
+                        g = p.glogit[e];
+                        pr = ex2((p.logit[e] - p.lse[(first + i0 + i) * HEADS + hh]) * LOG2E);
+                    }
+                    gs[hh * COL_LD + i * COL_KEYS + jj] = g;
+                    ps[hh * COL_LD + i * COL_KEYS + jj] = pr;
+                }
+                __syncthreads();
+                const float *qp = p.q + (first + i0) * HEADS * HEAD_DIM + h * HEAD_DIM + d;
+                const float *gp = p.gout + (first + i0) * HEADS * HEAD_DIM + h * HEAD_DIM + d;
+#pragma unroll 4
+                for (int i = par; i < rows; i += 2) {
+                    const float qv = __ldg(qp + (size_t)i * HEADS * HEAD_DIM), gv = __ldg(gp + (size_t)i * HEADS * HEAD_DIM);
+                    const float4 *g4 = reinterpret_cast<const float4 *>(gs + h * COL_LD + i * COL_KEYS);
+                    const float4 *p4 = reinterpret_cast<const float4 *>(ps + h * COL_LD + i * COL_KEYS);
+                    const float4 g0 = g4[0], g1 = g4[1], p0 = p4[0], p1 = p4[1];
+                    ak[0] = fmaf(g0.x, qv, ak[0]); ak[1] = fmaf(g0.y, qv, ak[1]); ak[2] = fmaf(g0.z, qv, ak[2]); ak[3] = fmaf(g0.w, qv, ak[3]);
+                    ak[4] = fmaf(g1.x, qv, ak[4]); ak[5] = fmaf(g1.y, qv, ak[5]); ak[6] = fmaf(g1.z, qv, ak[6]); ak[7] = fmaf(g1.w, qv, ak[7]);
+                    av[0] = fmaf(p0.x, gv, av[0]); av[1] = fmaf(p0.y, gv, av[1]); av[2] = fmaf(p0.z, gv, av[2]); av[3] = fmaf(p0.w, gv, av[3]);
+                    av[4] = fmaf(p1.x, gv, av[4]); av[5] = fmaf(p1.y, gv, av[5]); av[6] = fmaf(p1.z, gv, av[6]); av[7] = fmaf(p1.w, gv, av[7]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < COL_KEYS; ++u) {
+                ak[u] += __shfl_xor_sync(FULL, ak[u], 16);
+                av[u] += __shfl_xor_sync(FULL, av[u], 16);
+                if (u < keys) (par == 0 ? p.gk : p.gv)[(j0 + u) * HEADS * HEAD_DIM + h * HEAD_DIM + d] = par == 0 ? ak[u] : av[u];
+            }
+            j0 += keys;
         }
     }
 }
@@ -410,7 +457,7 @@ int cf::infinite_attn_bwd_impl(const float *q, const float *k, const float *v, c
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, smem) != cudaSuccess || occ <= 0) occ = 1;
     const long long cap = (long long)sm_count() * occ;
     kernel<<<(int)(N < cap ? N : cap), THREADS, smem, s>>>(p);
-    const long long cap2 = (long long)sm_count() * 8;
-    infinite_attn_bwd_cols_kernel<<<(int)(N < cap2 ? N : cap2), 256, 0, s>>>(p);
+    const long long tiles = (N + COL_KEYS - 1) / COL_KEYS, cap2 = (long long)sm_count() * 8;
+    infinite_attn_bwd_cols_kernel<<<(int)(tiles < cap2 ? tiles : cap2), 256, 0, s>>>(p);
     return launch_status("cf_infinite_attn_bwd");
 }

@@ -859,6 +859,25 @@ int launch_leftover_rows(const float *q, const float *k, const float *v, const f
     // left-over rows are rare: a grid of one block per SM draws them through the ticket
     return launch_rows(p, K, (long long)sm_count() * (max_atoms <= 12 ? WARPS : 1), s, true);
 }
+
+// The rows that the block kernel (infinite_attn_block.cu) met without a term list: phi is in the logit array already.
+int launch_listless_rows(const float *q, const float *k, const float *v, const float *a, const float *pos_ij, const float *tvecs,
+                         const float *rvlen, const int64_t *batch, const int64_t *edges, const int64_t *row_start, int64_t N, int64_t E,
+                         int64_t max_atoms, double dist_max, double wscale, const float *W, double cutoff_radius, int lattice_range,
+                         int minimum_range, float *out, float *logit, float *lse, float *psi_row, const TermList &list, const int *rows,
+                         const unsigned *count, unsigned *ticket, int64_t K, cudaStream_t s)
+{
+    RowArgs p{};
+    p.q = q; p.k = k; p.v = v; p.a = a; p.pos_ij = pos_ij; p.tvecs = tvecs; p.rvlen = rvlen; p.W = W;
+    p.batch = batch; p.edges = edges; p.row_start = row_start; p.row_order = rows; p.rows_on_device = count; p.E = E;
+    p.out = out; p.logit = logit; p.lse = lse; p.psi_row = psi_row; p.N = N; p.max_atoms = (int)max_atoms;
+    p.keep_logit = 1;
+    p.ticket = ticket;
+    if (K > 0) p.list = list;
+    p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
+    p.basis = make_basis_params(K, dist_max, wscale, weight_floor_log2());
+    return launch_rows(p, K, (long long)sm_count() * (max_atoms <= 12 ? WARPS : 1), s, true);
+}
 }  // namespace cf
 
 unsigned *cf::row_ticket_block(int count) { return next_ticket_block(count); }

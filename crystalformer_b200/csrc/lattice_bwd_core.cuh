@@ -12,8 +12,6 @@
 namespace cf {
 
 constexpr int U_STRIDE = 64;                  // floats per head row of the u tile
-constexpr int BWD_ENTRY_FLOATS = 12;          // x, d2, key index, pad, p0..7
-constexpr int BWD_STAGE_FLOATS = 32 * BWD_ENTRY_FLOATS;
 
 // c[h] = sum_k u[h][k] 2^(-((k+1) step - x)^2); u in shared memory, [8][U_STRIDE].
 template <int K>
@@ -63,22 +61,6 @@ __device__ __forceinline__ void basis_dot_window(const float *__restrict__ u, fl
             c[h] = fmaf(uv.w, g3, c[h]);
         }
     }
-}
-
-// Compacts the lanes' surviving terms into the warp's staging area; returns how many were staged.
-__device__ __forceinline__ int stage_terms(float *stage, int lane, bool keep, float x, float d2, int key,
-                                           const float (&p)[8])
-{
-    const unsigned mask = __ballot_sync(FULL, keep);
-    if (keep) {
-        const int slot = __popc(mask & ((1u << lane) - 1u));
-        float4 *row = reinterpret_cast<float4 *>(stage + BWD_ENTRY_FLOATS * slot);
-        row[0] = make_float4(x, d2, __int_as_float(key), 0.f);
-        row[1] = make_float4(p[0], p[1], p[2], p[3]);
-        row[2] = make_float4(p[4], p[5], p[6], p[7]);
-    }
-    __syncwarp();
-    return __popc(mask);
 }
 
 }  // namespace cf

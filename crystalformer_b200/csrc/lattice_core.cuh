@@ -302,7 +302,9 @@ __device__ __forceinline__ bool key_in_box(int key, int pk)
     return ((key >> 11) & 63) <= box_r1(pk) && ((key >> 17) & 63) <= box_r2(pk) && ((key >> 23) & 63) <= box_r3(pk);
 }
 
-struct CandidateRing {
+template <int ENTRIES>
+struct CandidateRingOf {
+    static constexpr int MASK = ENTRIES - 1;
     float2 *buf;
     int head, count, lane;
     __device__ __forceinline__ void init(float *storage, int lane_)
@@ -323,7 +325,7 @@ struct CandidateRing {
         int at = head + count;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            if (cand[u]) buf[(at + __popc(m[u] & lt)) & (RING_ENTRIES - 1)] = make_float2(d2[u], __int_as_float(key[u]));
+            if (cand[u]) buf[(at + __popc(m[u] & lt)) & (MASK)] = make_float2(d2[u], __int_as_float(key[u]));
             at += __popc(m[u]);
         }
         count = at - head;
@@ -334,7 +336,7 @@ struct CandidateRing {
     {
         const unsigned mask = __ballot_sync(FULL, cand);
         if (mask == 0u) return;
-        if (cand) buf[(head + count + __popc(mask & ((1u << lane) - 1u))) & (RING_ENTRIES - 1)] = make_float2(d2, __int_as_float(key));
+        if (cand) buf[(head + count + __popc(mask & ((1u << lane) - 1u))) & (MASK)] = make_float2(d2, __int_as_float(key));
         count += __popc(mask);
         __syncwarp();
     }
@@ -343,15 +345,16 @@ struct CandidateRing {
     __device__ __forceinline__ bool take(float &d2, int &key)
     {
         const int n = min(count, 32);
-        const float2 e = buf[(head + lane) & (RING_ENTRIES - 1)];
+        const float2 e = buf[(head + lane) & (MASK)];
         d2 = e.x;
         key = __float_as_int(e.y);
-        head = (head + n) & (RING_ENTRIES - 1);
+        head = (head + n) & (MASK);
         count -= n;
         __syncwarp();
         return lane < n;
     }
 };
+using CandidateRing = CandidateRingOf<RING_ENTRIES>;
 
 // ---- lane <-> bins ------------------------------------------------------------------------------------------------
 struct BasisParams {

@@ -12,6 +12,7 @@
 // (models/latticeformer.py:211-302 with pooling "avr", a Linear - ReLU - Linear head and LayerNorm = Identity.)
 #include "common.cuh"
 #include "dense_tc.cuh"
+#include "infinite_attn_block.cuh"
 #include "term_list.cuh"
 
 namespace cf {
@@ -242,6 +243,7 @@ struct Saved {
     float *rvlen, *rvecs, *vcell;
     int32_t *row_order;
     unsigned *tickets;
+    void *row_blocks;
     unsigned char *embed;
     float *x[MAX_LAYERS + 1];
     LayerSaved layer[MAX_LAYERS];
@@ -266,6 +268,7 @@ Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64
     s.vcell = c.take<float>(B);
     s.row_order = c.take<int32_t>(N);
     s.tickets = c.take<unsigned>(MAX_LAYERS);
+    s.row_blocks = c.take<unsigned>(row_blocks_words(N));
     s.embed = c.take<unsigned char>(tc_image_bytes(1));
     const size_t image = tc_image_bytes(tc_layer_blocks((int)d.ff_dim));
     for (int l = 0; l < d.num_layers; ++l) {
@@ -576,6 +579,11 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
         rc = launch_term_list_build(tb, prep);
         if (rc != CF_OK) return rc;
     }
+    static_assert(MAX_LAYERS <= ROW_BLOCK_LAYERS, "every layer has a scheduling block of its own");
+    const RowBlocks row_blocks = row_blocks_carve(w.row_blocks, N);
+    const bool by_blocks = listed && b.max_atoms > ROW_BLOCK_MIN_ATOMS && b.max_atoms <= ROW_BLOCK_MAX_ATOMS;
+    if (by_blocks) rc = launch_row_blocks(row_blocks, order, w.row_start, w.edges, N, E, prep);
+    if (rc != CF_OK) return rc;
     if (w.kr != nullptr) rc = cf_reci_phase(w.pos_ij, w.rvecs, w.batch, w.edges, E, w.kr, prep);
     if (rc == CF_OK) rc = join_early_prep(s);
     if (rc == CF_OK) rc = pack_all(d, w, false, prep);  // (joined before the backward, below)
@@ -584,7 +592,11 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
         const LayerSaved &t = w.layer[l];
         const Domain dom = domain_of(d, l);
         const double dist_max = d.scalars[SCALARS * l + 5];
-        if (dom == REAL) {
+        if (dom == REAL && by_blocks) {
+            rc = block_attn_impl(t.q, t.k, t.v, t.a, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, E, d.K, b.max_atoms,
+                                 dist_max, d.wscale, d.weights[PER_LAYER * l + W_PE], d.cutoff_radius, d.lattice_range, d.minimum_range,
+                                 t.attn, t.logit, t.lse, t.psi, list, row_blocks, l, s);
+        } else if (dom == REAL) {
             rc = infinite_attn_fwd_impl(t.q, t.k, t.v, t.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
                                         HEAD_DIM, E, d.K, b.max_atoms, dist_max, d.wscale, d.weights[PER_LAYER * l + W_PE],
                                         d.cutoff_radius, d.lattice_range, d.minimum_range, t.attn, t.logit, t.lse, t.psi, order,
