@@ -17,6 +17,196 @@ namespace cf {
 namespace {
 using namespace tc5;
 
+// The rows of attention outputs, element features or species of a tile as operand 0 (scales: row floats 0).
+__device__ __forceinline__ void load_first_operand(const DenseForward &p, const Shared &s, long long row_base)
+{
+    unsigned char *A0 = s.mem + OFF_A0;
+    if (p.tail != nullptr) {
+        load_operand(s, A0, [&](int row, int ln) {
+            return row_base + row < p.N ? *reinterpret_cast<const float4 *>(p.attn + (row_base + row) * 128 + 4 * ln)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+        });
+    } else {
+        load_operand(s, A0, [&](int row, int ln) {
+            float e[4] = {0.f, 0.f, 0.f, 0.f};
+            if (row_base + row < p.N) {
+                if (p.features != nullptr) {
+                    const float *f = p.features + (row_base + row) * p.feature_dim;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (4 * ln + u < p.feature_dim) e[u] = f[4 * ln + u];
+                } else {
+                    const long long z = p.species[row_base + row] - 4 * ln;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) e[u] = z == u ? 1.0f : 0.0f;
+                }
+            }
+            return make_float4(e[0], e[1], e[2], e[3]);
+        });
+    }
+}
+
+// Constants of the weights: 1 / s of each matrix, and a bound of the hidden units' biases (every epilogue thread calls).
+struct WeightScales {
+    float first = 0.f, w1 = 0.f, w2 = 0.f, head = 0.f, b1_max = 0.f;
+    __device__ __forceinline__ WeightScales(const DenseForward &p, const Shared &s)
+    {
+        const int chunks = p.ff / 128;
+        if (p.weights_fresh) grid_dependency_wait();
+        if (p.tail != nullptr) {
+            const float *inv = reinterpret_cast<const float *>(p.tail);
+            first = inv[0]; w1 = inv[1]; w2 = inv[2 * chunks];
+            for (int i = threadIdx.x; i < p.ff; i += EPI_THREADS) b1_max = fmaxf(b1_max, fabsf(p.b1[i]));
+            b1_max = warp_max(b1_max);
+            if ((threadIdx.x & 31) == 0) s.warp_floats()[threadIdx.x >> 5] = b1_max;
+            epilogue_sync();
+#pragma unroll
+            for (int w = 0; w < EPI_WARPS; ++w) b1_max = fmaxf(b1_max, s.warp_floats()[w]);
+        }
+        if (p.embed != nullptr) first = *reinterpret_cast<const float *>(p.embed);
+        if (p.head != nullptr) head = reinterpret_cast<const float *>(p.head)[1 + 2 * chunks];
+    }
+};
+
+// The thread's 32 features ahead of the feed-forward: x + attn Wo^T + bo, the embedding, or x as it is.
+__device__ __forceinline__ void first_rows(const DenseForward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, long long row_base,
+                                           float w_i, float (&x)[2][16])
+{
+    const bool tail = p.tail != nullptr;
+    if (!tail && p.embed == nullptr) {
+#pragma unroll
+        for (int half = 0; half < 2; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+        return;
+    }
+    load_first_operand(p, s, row_base);
+    fence_async_smem();
+    fence_before();
+    mbar_arrive(s.bar(B_A0));
+    if (tail) {  // the residual and its bias arrive during the product
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 b = *reinterpret_cast<const float2 *>(p.bo + pl.col0 + 8 * j);
+                x[half][4 * j] += b.x; x[half][4 * j + 1] += b.y; x[half][4 * j + 2] += b.x; x[half][4 * j + 3] += b.y;
+            }
+        }
+    }
+    epilogue_sync();  // (the loading warps' scales)
+    float xi[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
+    ph.wait(s, B_D0);
+    fence_after();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float d[16];
+        tmem_load_16x32(pl.tmem(tmem, D0, half), d);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float sc = xi[2 * half + ((i >> 1) & 1)] * w_i;
+            x[half][i] = tail ? fmaf(d[i], sc, x[half][i]) : d[i] * sc;
+        }
+    }
+}
+
+// The hidden units of all chunks share one scale per row (their products with W2 meet in one sum), from a bound known
+// beforehand: |h| <= 128 max|y| max|W1| + max|b1|, with both operands below 2^15 in their scaled form.  A bound some 2^8
+// above the largest unit still leaves 2^-31 of it as resolution.
+__device__ __forceinline__ void hidden_scales(const WeightScales &ws, const float (&xi)[4], float (&hs)[4], float (&hi)[4])
+{
+#pragma unroll
+    for (int i = 0; i < 4; ++i) hs[i] = power_of_two(fmaf(137438953472.0f * xi[i], ws.w1, ws.b1_max), hi[i]);
+}
+
+// Chunk c of the hidden units from its accumulator, as the operand at `a_off` (wait_free: once the previous chunk's has
+// been multiplied).
+__device__ __forceinline__ void hidden_units(const DenseForward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, int d_col,
+                                             int done, int c, long long row_base, const float (&xi)[4], float w1_i, const float (&hs)[4],
+                                             int a_off, int ready, bool wait_free)
+{
+    float2 bias[4];
+    load_columns(p.b1 + 128 * c, pl, bias);
+    ph.wait(s, done);
+    fence_after();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float h[16];
+        tmem_load_16x32(pl.tmem(tmem, d_col, half), h);
+        const float sa = xi[2 * half] * w1_i, sb = xi[2 * half + 1] * w1_i;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 b = bias[j];
+            h[4 * j] = fmaxf(fmaf(h[4 * j], sa, b.x), 0.f);
+            h[4 * j + 1] = fmaxf(fmaf(h[4 * j + 1], sa, b.y), 0.f);
+            h[4 * j + 2] = fmaxf(fmaf(h[4 * j + 2], sb, b.x), 0.f);
+            h[4 * j + 3] = fmaxf(fmaf(h[4 * j + 3], sb, b.y), 0.f);
+        }
+        if (half == 0 && wait_free) ph.wait(s, B_A1_FREE);
+        store_operand(s.mem + a_off, pl, half, h, hs[2 * half], hs[2 * half + 1]);
+        if (p.h_save != nullptr) store_rows(p.h_save + 128 * c, p.ff, row_base, p.N, pl, half, h);
+    }
+    fence_async_smem();
+    fence_before();
+    mbar_arrive(s.bar(ready));
+}
+
+// One of q, k, v (which = 0, 1, 2) from its accumulator, and the Gaussian widths beside q.
+__device__ __forceinline__ void head_out(const DenseForward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, int d_col,
+                                         int done, int which, long long row_base, const float (&xi)[4], float wh_i)
+{
+    float2 bias[4], w[4];
+    load_columns(p.bqkv + 128 * which, pl, bias);
+    if (which == 0) load_columns(p.w_pos, pl, w);
+    ph.wait(s, done);
+    fence_after();
+    float *dst = which == 0 ? p.q : which == 1 ? p.k : p.v;
+    float al[2][4];  // q . w_pos of the thread's columns: (half, 2 head + row)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float d[16];
+        tmem_load_16x32(pl.tmem(tmem, d_col, half), d);
+        const float sa = xi[2 * half] * wh_i, sb = xi[2 * half + 1] * wh_i;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 b = bias[j];
+            d[4 * j] = fmaf(d[4 * j], sa, b.x); d[4 * j + 1] = fmaf(d[4 * j + 1], sa, b.y);
+            d[4 * j + 2] = fmaf(d[4 * j + 2], sb, b.x); d[4 * j + 3] = fmaf(d[4 * j + 3], sb, b.y);
+        }
+        if (which == 0) {
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const float2 wa = w[2 * hh], wb = w[2 * hh + 1];
+                const float *da = d + 8 * hh, *db = da + 4;
+                al[half][2 * hh] = fmaf(db[1], wb.y, fmaf(db[0], wb.x, fmaf(da[1], wa.y, da[0] * wa.x)));
+                al[half][2 * hh + 1] = fmaf(db[3], wb.y, fmaf(db[2], wb.x, fmaf(da[3], wa.y, da[2] * wa.x)));
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) d[i] *= 0.25f;  // q / sqrt(16)
+        }
+        store_rows(dst, 128, row_base, p.N, pl, half, d);
+    }
+    if (which == 0) {
+        // the heads' Gaussian widths from alpha = q . w_pos (…attention_cuda.py:647-722): the four lanes of a row trade
+        // halves of their sums, lane t finishes head t / 2 of row t % 2 (of either half)
+        const float lb = pl.group < 2 ? p.lower_bound : p.lower_bound_hi, factor = pl.group < 2 ? p.a_factor : p.a_factor_hi;
+        const float slope = p.gauss_scale * (p.elu_beta / (1.0f - lb));
+        const int e = pl.t & 1, hh = pl.t >> 1;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const float *v = al[half];
+            const float k0 = (e ? v[1] : v[0]) + __shfl_xor_sync(FULL, e ? v[0] : v[1], 1);
+            const float k1 = (e ? v[3] : v[2]) + __shfl_xor_sync(FULL, e ? v[2] : v[3], 1);
+            const float alpha = (hh ? k1 : k0) + __shfl_xor_sync(FULL, hh ? k0 : k1, 2);
+            const float tt = (alpha + p.gauss_shift) * slope;
+            const float elu = tt > 0.f ? tt : expm1f(tt), f = (1.0f - lb) * elu + 1.0f;
+            const long long row = row_base + pl.row0 + 16 * half + 8 * e;
+            if (row < p.N) p.a[row * HEADS + 2 * pl.group + hh] = p.inverse ? factor / f : f * factor;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const DenseForward p)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
@@ -31,7 +221,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
     if (warp == STREAM_WARP) {
         if (p.weights_fresh) grid_dependency_wait();
         if (lane == 0) {
-            Producer pr;
+            Producer<STAGES> pr;
             for (long long tile = blockIdx.x; tile < tiles && pr.ok; tile += gridDim.x) {
                 if (tail) pr.stream(s, p.tail, 0, 1 + 2 * chunks);
                 else if (embed) pr.stream(s, p.embed, 0, 1);
@@ -43,7 +233,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
     } else if (warp == ISSUE_WARP) {
         grid_dependency_wait();
         if (lane == 0) {
-            Issuer is;
+            Issuer<STAGES> is;
             Phase ph;
             for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
                 bool ok = true;
@@ -80,22 +270,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
         }
     } else {
         const Place pl;
-        unsigned char *A0 = s.mem + OFF_A0, *A1 = s.mem + OFF_A1;
-        const float *tail_inv = reinterpret_cast<const float *>(p.tail), *head_inv = reinterpret_cast<const float *>(p.head);
-        if (p.weights_fresh) grid_dependency_wait();
-        // constants of the weights: 1 / s of each matrix, and a bound of the hidden units' biases
-        float wo_i = 0.f, w1_i = 0.f, w2_i = 0.f, wh_i = 0.f, we_i = 0.f, b1_max = 0.f;
-        if (tail) {
-            wo_i = tail_inv[0]; w1_i = tail_inv[1]; w2_i = tail_inv[2 * chunks];
-            for (int i = threadIdx.x; i < p.ff; i += EPI_THREADS) b1_max = fmaxf(b1_max, fabsf(p.b1[i]));
-            b1_max = warp_max(b1_max);
-            if (lane == 0) s.warp_floats()[warp] = b1_max;
-            epilogue_sync();
-#pragma unroll
-            for (int w = 0; w < EPI_WARPS; ++w) b1_max = fmaxf(b1_max, s.warp_floats()[w]);
-        }
-        if (embed) we_i = *reinterpret_cast<const float *>(p.embed);
-        if (head) wh_i = head_inv[1 + 2 * chunks];
+        const WeightScales ws(p, s);
         grid_dependency_wait();
         Phase ph;
         for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -103,119 +278,17 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             epilogue_sync();  // the previous tile's readers are done with the per-row scales
             float x[2][16];   // the thread's 32 features: x, then y, then x'
             float xi[4];      // 1 / scale of its four rows in the current operand
-            // largest magnitude of the rows -> scales, then operand 0
-            auto publish = [&]() {
-                float m[4] = {0.f, 0.f, 0.f, 0.f}, xs[4];
-#pragma unroll
-                for (int half = 0; half < 2; ++half)
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) m[2 * half + ((i >> 1) & 1)] = fmaxf(m[2 * half + ((i >> 1) & 1)], fabsf(x[half][i]));
-                row_maxima(s, pl, m);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xs[i] = power_of_two(m[i], xi[i]);
-#pragma unroll
-                for (int half = 0; half < 2; ++half) store_operand(A0, pl, half, x[half], xs[2 * half], xs[2 * half + 1]);
-                fence_async_smem();
-                fence_before();
-                mbar_arrive(s.bar(B_A0));
-            };
-            if (tail || embed) {
-                if (tail) {
-                    load_operand(s, A0, [&](int row, int ln) {
-                        return row_base + row < p.N ? *reinterpret_cast<const float4 *>(p.attn + (row_base + row) * 128 + 4 * ln)
-                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-                    });
-                } else {
-                    load_operand(s, A0, [&](int row, int ln) {
-                        float e[4] = {0.f, 0.f, 0.f, 0.f};
-                        if (row_base + row < p.N) {
-                            if (p.features != nullptr) {
-                                const float *f = p.features + (row_base + row) * p.feature_dim;
-#pragma unroll
-                                for (int u = 0; u < 4; ++u)
-                                    if (4 * ln + u < p.feature_dim) e[u] = f[4 * ln + u];
-                            } else {
-                                const long long z = p.species[row_base + row] - 4 * ln;
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) e[u] = z == u ? 1.0f : 0.0f;
-                            }
-                        }
-                        return make_float4(e[0], e[1], e[2], e[3]);
-                    });
-                }
-                fence_async_smem();
-                fence_before();
-                mbar_arrive(s.bar(B_A0));
-                if (tail) {  // the residual and its bias arrive during the product
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 b = *reinterpret_cast<const float2 *>(p.bo + pl.col0 + 8 * j);
-                            x[half][4 * j] += b.x; x[half][4 * j + 1] += b.y; x[half][4 * j + 2] += b.x; x[half][4 * j + 3] += b.y;
-                        }
-                    }
-                }
-                epilogue_sync();  // (the loading warps' scales)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
-                ph.wait(s, B_D0);
-                fence_after();
-                const float wi = tail ? wo_i : we_i;
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float d[16];
-                    tmem_load_16x32(pl.tmem(tmem, D0, half), d);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float sc = xi[2 * half + ((i >> 1) & 1)] * wi;
-                        x[half][i] = tail ? fmaf(d[i], sc, x[half][i]) : d[i] * sc;
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int half = 0; half < 2; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
-            }
+            first_rows(p, s, pl, ph, tmem, row_base, ws.first, x);
             if (tail) {
-                publish();  // y
+                publish_rows(s, pl, x, xi);  // y
                 if (p.y_save != nullptr) {
 #pragma unroll
                     for (int half = 0; half < 2; ++half) store_rows(p.y_save, 128, row_base, p.N, pl, half, x[half]);
                 }
-                // The hidden units of all chunks share one scale per row (their products with W2 meet in one accumulator),
-                // from a bound known beforehand: |h| <= 128 max|y| max|W1| + max|b1|, with both operands below 2^15 in
-                // their scaled form.  A bound some 2^8 above the largest unit still leaves 2^-31 of it as resolution.
                 float hs[4], hi[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) hs[i] = power_of_two(fmaf(137438953472.0f * xi[i], w1_i, b1_max), hi[i]);
-                for (int c = 0; c < chunks; ++c) {
-                    const int d_col = (c & 1) ? D1 : D0;
-                    float2 bias[4];
-                    load_columns(p.b1 + 128 * c, pl, bias);
-                    ph.wait(s, (c & 1) ? B_D1 : B_D0);
-                    fence_after();
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        float h[16];
-                        tmem_load_16x32(pl.tmem(tmem, d_col, half), h);
-                        const float sa = xi[2 * half] * w1_i, sb = xi[2 * half + 1] * w1_i;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 b = bias[j];
-                            h[4 * j] = fmaxf(fmaf(h[4 * j], sa, b.x), 0.f);
-                            h[4 * j + 1] = fmaxf(fmaf(h[4 * j + 1], sa, b.y), 0.f);
-                            h[4 * j + 2] = fmaxf(fmaf(h[4 * j + 2], sb, b.x), 0.f);
-                            h[4 * j + 3] = fmaxf(fmaf(h[4 * j + 3], sb, b.y), 0.f);
-                        }
-                        if (half == 0 && c > 0) ph.wait(s, B_A1_FREE);  // the previous chunk has been multiplied
-                        store_operand(A1, pl, half, h, hs[2 * half], hs[2 * half + 1]);
-                        if (p.h_save != nullptr) store_rows(p.h_save + 128 * c, p.ff, row_base, p.N, pl, half, h);
-                    }
-                    fence_async_smem();
-                    fence_before();
-                    mbar_arrive(s.bar(B_A1));
-                }
+                hidden_scales(ws, xi, hs, hi);
+                for (int c = 0; c < chunks; ++c)
+                    hidden_units(p, s, pl, ph, tmem, (c & 1) ? D1 : D0, (c & 1) ? B_D1 : B_D0, c, row_base, xi, ws.w1, hs, OFF_A1, B_A1, c > 0);
                 float2 bias[4];
                 load_columns(p.b2, pl, bias);
                 ph.wait(s, B_A1_FREE);
@@ -225,7 +298,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                 for (int half = 0; half < 2; ++half) {
                     float d[16];
                     tmem_load_16x32(pl.tmem(tmem, DX, half), d);
-                    const float sa = hi[2 * half] * w2_i, sb = hi[2 * half + 1] * w2_i;
+                    const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float2 b = bias[j];
@@ -236,64 +309,162 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                     }
                 }
             }
-            if (head) publish();
+            if (head) publish_rows(s, pl, x, xi);
             if (tail || embed) {
 #pragma unroll
                 for (int half = 0; half < 2; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!head) continue;
 #pragma unroll
-            for (int which = 0; which < 3; ++which) {
-                float2 bias[4];
-                load_columns(p.bqkv + 128 * which, pl, bias);
-                ph.wait(s, which == 0 ? B_D0 : which == 1 ? B_D1 : B_DX);
-                fence_after();
-                float *dst = which == 0 ? p.q : which == 1 ? p.k : p.v;
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float d[16];
-                    tmem_load_16x32(pl.tmem(tmem, which == 0 ? D0 : which == 1 ? D1 : DX, half), d);
-                    const float sa = xi[2 * half] * wh_i, sb = xi[2 * half + 1] * wh_i;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float2 b = bias[j];
-                        d[4 * j] = fmaf(d[4 * j], sa, b.x); d[4 * j + 1] = fmaf(d[4 * j + 1], sa, b.y);
-                        d[4 * j + 2] = fmaf(d[4 * j + 2], sb, b.x); d[4 * j + 3] = fmaf(d[4 * j + 3], sb, b.y);
-                    }
-                    if (which == 0) {
-                        // the heads' Gaussian widths from alpha = q . w_pos (…attention_cuda.py:647-722), then q / sqrt(16)
-#pragma unroll
-                        for (int hh = 0; hh < 2; ++hh) {
-                            float al[2] = {0.f, 0.f};
-#pragma unroll
-                            for (int jj = 0; jj < 2; ++jj) {
-                                const int j = 2 * hh + jj;
-                                const float2 w = *reinterpret_cast<const float2 *>(p.w_pos + pl.col0 + 8 * j);
-                                al[0] = fmaf(d[4 * j + 1], w.y, fmaf(d[4 * j], w.x, al[0]));
-                                al[1] = fmaf(d[4 * j + 3], w.y, fmaf(d[4 * j + 2], w.x, al[1]));
-                            }
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                al[e] += __shfl_xor_sync(FULL, al[e], 1);
-                                al[e] += __shfl_xor_sync(FULL, al[e], 2);
-                                const long long row = row_base + pl.row0 + 16 * half + 8 * e;
-                                if (pl.t == 0 && row < p.N) {
-                                    const float lb = pl.group < 2 ? p.lower_bound : p.lower_bound_hi;
-                                    const float tt = (al[e] + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - lb));
-                                    const float elu = tt > 0.f ? tt : expm1f(tt), f = (1.0f - lb) * elu + 1.0f;
-                                    const float factor = pl.group < 2 ? p.a_factor : p.a_factor_hi;
-                                    p.a[row * HEADS + 2 * pl.group + hh] = p.inverse ? factor / f : f * factor;
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) d[i] *= 0.25f;
-                    }
-                    store_rows(dst, 128, row_base, p.N, pl, half, d);
-                }
-            }
+            for (int which = 0; which < 3; ++which)
+                head_out(p, s, pl, ph, tmem, which == 0 ? D0 : which == 1 ? D1 : DX, which == 0 ? B_D0 : which == 1 ? B_D1 : B_DX, which,
+                         row_base, xi, ws.head);
         }
     }
+    block_end(s, tmem, &g_dense_forward_status);
+}
+
+// The same for a cluster of four blocks (dense_tc_core.cuh): block r takes hidden chunk r and, of q, k, v, matrix r.  Hidden
+// units go to operand buffer 0 (y has been multiplied by then), buffer 1 takes the shares of the output sum.
+// 2,027 rows, 512 hidden units, a boundary inside the network: 31 us with a block per tile, 20 here (unchained).
+__global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(const DenseForward p)
+{
+    extern __shared__ __align__(1024) unsigned char smem_tc[];
+    uint32_t tmem;
+    const Shared s = block_begin(smem_tc, tmem);
+    const uint32_t rank = cluster_rank();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chunks = p.ff / 128;
+    const long long row_base = (long long)(blockIdx.x / SPLIT) * 128;
+    const bool tail = p.tail != nullptr, embed = p.embed != nullptr, head = p.head != nullptr;
+    const bool has_chunk = tail && (int)rank < chunks, has_head = head && rank < 3;
+    grid_launch_dependents();
+    cluster_sync();  // every block's barriers are ready for the others' arrivals
+
+    if (warp == STREAM_WARP) {
+        if (p.weights_fresh) grid_dependency_wait();
+        if (lane == 0) {
+            Producer<SPLIT_STAGES> pr;
+            if (tail) pr.stream(s, p.tail, 0, 1);
+            else if (embed) pr.stream(s, p.embed, 0, 1);
+            if (has_chunk && pr.ok) pr.stream(s, p.tail, 1 + first_of_chunk(rank), 1);
+            if (has_chunk && pr.ok) pr.stream(s, p.tail, 1 + second_of_chunk(rank, chunks), 1);
+            if (has_head && pr.ok) pr.stream(s, p.head, 1 + 2 * chunks + (int)rank, 1);
+            if (!pr.ok) pr.drain(s);
+        }
+        __syncwarp();
+        grid_dependency_wait();
+    } else if (warp == ISSUE_WARP) {
+        grid_dependency_wait();
+        if (lane == 0) {
+            Issuer<SPLIT_STAGES> is;
+            Phase ph;
+            bool ok = true;
+            auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
+            auto product = [&](int d, bool use, int done) {
+                if (ok && use) is.product(s, tmem, d, OFF_A0, false);
+                ok = ok && is.ok;
+                mma_commit(s.bar(done));
+            };
+            if (tail || embed) {
+                ready(B_A0);
+                product(D0, true, B_D0);
+            }
+            if (tail) {
+                ready(B_A0);
+                if (has_chunk) {
+                    product(D0, true, B_D0);
+                    ready(B_A0);
+                    product(DX, true, B_DX);
+                }
+            }
+            if (has_head) {
+                if (tail) {
+                    ok = ph.wait_cluster(s, B_ROWS) && ok;
+                    fence_async_smem();
+                    fence_after();
+                } else {
+                    ready(B_A0);
+                }
+                product(D1, true, B_D1);
+            }
+            if (!ok) is.drain(s);
+        }
+        __syncwarp();
+    } else {
+        const Place pl;
+        const WeightScales ws(p, s);
+        grid_dependency_wait();
+        Phase ph;
+        if (threadIdx.x == 0 && tail) {
+            expect_shares(s);
+            if (has_head) expect_rows(s);
+        }
+        const bool mine = (warp & 3) == (int)rank;  // this warp's rows of an accumulator are finished by this block
+        float x[2][16], xi[4];
+        first_rows(p, s, pl, ph, tmem, row_base, ws.first, x);
+        if (tail) {
+            publish_rows(s, pl, x, xi);  // y
+            if (p.y_save != nullptr && mine) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) store_rows(p.y_save, 128, row_base, p.N, pl, half, x[half]);
+            }
+            float hs[4], hi[4];
+            hidden_scales(ws, xi, hs, hi);
+            if (has_chunk) hidden_units(p, s, pl, ph, tmem, D0, B_D0, rank, row_base, xi, ws.w1, hs, OFF_A0, B_A0, false);
+            float2 bias[4];
+            load_columns(p.b2, pl, bias);
+            if (has_chunk) {
+                ph.wait(s, B_DX);
+                fence_after();
+            } else {
+                epilogue_sync();  // (buffer 0 is about to take the shares: y is no longer being written)
+            }
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float d[16];
+                if (has_chunk) {
+                    tmem_load_16x32(pl.tmem(tmem, DX, half), d);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) d[i] = 0.f;
+                }
+                const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {  // (the finishing block's own share carries y and the bias)
+                    const float2 b = bias[j];
+                    d[4 * j] = fmaf(d[4 * j], sa, mine ? x[half][4 * j] + b.x : 0.f);
+                    d[4 * j + 1] = fmaf(d[4 * j + 1], sa, mine ? x[half][4 * j + 1] + b.y : 0.f);
+                    d[4 * j + 2] = fmaf(d[4 * j + 2], sb, mine ? x[half][4 * j + 2] + b.x : 0.f);
+                    d[4 * j + 3] = fmaf(d[4 * j + 3], sb, mine ? x[half][4 * j + 3] + b.y : 0.f);
+                }
+                stage_share(s, pl, half, d);
+            }
+            send_share(s, rank);
+            float4 v[2];
+            collect_shares(s, ph, v);
+            if (head) spread_rows(s, ph, rank, v, 3, 0);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const long long row = row_base + 32 * (int)rank + 2 * warp + u;
+                if (row < p.N) *reinterpret_cast<float4 *>(p.x_out + row * 128 + 4 * lane) = v[u];
+            }
+            if (has_head) {
+                ph.wait_cluster(s, B_ROWS);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
+            }
+        } else {
+            if (head) publish_rows(s, pl, x, xi);
+            if (embed && mine) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
+            }
+        }
+        if (has_head) head_out(p, s, pl, ph, tmem, D1, B_D1, (int)rank, row_base, xi, ws.head);
+    }
+    __syncthreads();
+    cluster_sync();  // (no block ends while another may still write to it)
     block_end(s, tmem, &g_dense_forward_status);
 }
 
@@ -343,19 +514,15 @@ int launch_dense_forward(const DenseForward &p, cudaStream_t s)
     if (p.N == 0) return CF_OK;
     if (p.ff <= 0 || p.ff % 128 != 0 || p.ff > TC_MAX_FF)
         return fail(CF_ERR_UNSUPPORTED, "dense forward: ff_dim=%d must be a multiple of 128 up to %d", p.ff, TC_MAX_FF);
-    static thread_local bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!configured[dev & 63]) {
-        if (cudaFuncSetAttribute(dense_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc5::SMEM_BYTES) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(CF_ERR_CUDA, "dense forward: %d bytes of shared memory not available", tc5::SMEM_BYTES);
-        }
-        configured[dev & 63] = true;
-    }
+    static thread_local DenseLaunch launch;
+    int rc = launch.configure(reinterpret_cast<const void *>(dense_forward_kernel), reinterpret_cast<const void *>(dense_forward_split_kernel), "dense forward");
+    if (rc != CF_OK) return rc;
     const long long tiles = (p.N + 127) / 128, cap = sm_count();
-    launch_chained(dense_forward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
-                   p.chained, p);
+    if (split_tiles(tiles, p.ff, launch.clusters()))
+        launch_chained_cluster(dense_forward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, p.chained, p);
+    else
+        launch_chained(dense_forward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
+                       p.chained, p);
     return launch_status("dense_forward_kernel");
 }
 

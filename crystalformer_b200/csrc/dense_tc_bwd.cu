@@ -14,6 +14,63 @@ namespace cf {
 namespace {
 using namespace tc5;
 
+// gq' = gq / 4 + galpha w_pos of one row (lane l: columns 4 l .. 4 l + 3, head l / 4), written with galpha in place of gq and
+// ga: alpha of the head from the saved query (stored divided by 4), then the slope of its width.  The whole warp calls.
+__device__ __forceinline__ float4 query_grad(const DenseBackward &p, const float4 &wp, float4 gq, const float4 &qv, float ga, long long row)
+{
+    const int lane = threadIdx.x & 31;
+    const float lb = lane < 16 ? p.lower_bound : p.lower_bound_hi;
+    const float slope = p.gauss_scale * (lane < 16 ? p.a_factor : p.a_factor_hi) * p.elu_beta;
+    float al = 4.0f * fmaf(qv.w, wp.w, fmaf(qv.z, wp.z, fmaf(qv.y, wp.y, qv.x * wp.x)));
+    al += __shfl_xor_sync(FULL, al, 1);
+    al += __shfl_xor_sync(FULL, al, 2);
+    const float tt = (al + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - lb));
+    float galpha = ga * slope * (tt > 0.f ? 1.0f : expf(tt));
+    if (p.inverse) {
+        const float f = (1.0f - lb) * (tt > 0.f ? tt : expm1f(tt)) + 1.0f;
+        galpha = -galpha / (f * f);
+    }
+    gq.x = fmaf(galpha, wp.x, 0.25f * gq.x); gq.y = fmaf(galpha, wp.y, 0.25f * gq.y);
+    gq.z = fmaf(galpha, wp.z, 0.25f * gq.z); gq.w = fmaf(galpha, wp.w, 0.25f * gq.w);
+    __syncwarp();  // (the lanes of a head have read ga)
+    if (row < p.N) {
+        *reinterpret_cast<float4 *>(p.gq + row * 128 + 4 * lane) = gq;
+        if ((lane & 3) == 0) p.ga[row * HEADS + (lane >> 2)] = galpha;
+    }
+    return gq;
+}
+
+// Chunk c of the hidden units' gradients, gh = (gx W2) [h > 0], as the operand at `a_off` (wait_free: once the previous
+// chunk's has been multiplied).
+__device__ __forceinline__ void hidden_grads(const DenseBackward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, int d_col,
+                                             int done, int c, long long row_base, const float (&xi)[4], float w2_i, const float (&hs)[4],
+                                             int a_off, int ready, bool wait_free)
+{
+    unsigned live = 0u;  // bit 16 half + i: the unit was active
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float h[16];
+        load_rows(p.h + 128 * c, p.ff, row_base, p.N, pl, half, h);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) live |= (h[i] > 0.f ? 1u : 0u) << (16 * half + i);
+    }
+    ph.wait(s, done);
+    fence_after();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float g[16];
+        tmem_load_16x32(pl.tmem(tmem, d_col, half), g);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) g[i] = (live >> (16 * half + i)) & 1u ? g[i] * (xi[2 * half + ((i >> 1) & 1)] * w2_i) : 0.f;
+        if (half == 0 && wait_free) ph.wait(s, B_A1_FREE);
+        store_operand(s.mem + a_off, pl, half, g, hs[2 * half], hs[2 * half + 1]);
+        store_rows(p.gh + 128 * c, p.ff, row_base, p.N, pl, half, g);
+    }
+    fence_async_smem();
+    fence_before();
+    mbar_arrive(s.bar(ready));
+}
+
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const DenseBackward p)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
@@ -28,7 +85,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
 
     if (warp == STREAM_WARP) {
         if (lane == 0) {
-            Producer pr;
+            Producer<STAGES> pr;
             for (long long tile = blockIdx.x; tile < tiles && pr.ok; tile += gridDim.x) {
                 if (head) pr.stream(s, p.head, 0, 3);
                 if (tail) pr.stream(s, p.tail, 3, 1 + 2 * chunks);
@@ -37,7 +94,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
         }
     } else if (warp == ISSUE_WARP) {
         if (lane == 0) {
-            Issuer is;
+            Issuer<STAGES> is;
             Phase ph;
             for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
                 bool ok = true;
@@ -86,27 +143,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             epilogue_sync();  // the previous tile's readers are done with the per-row scales
             float x[2][16];   // the thread's 32 gradients: gx, then gy
             float xi[4];
-            auto publish = [&]() {
-                float m[4] = {0.f, 0.f, 0.f, 0.f}, xs[4];
-#pragma unroll
-                for (int half = 0; half < 2; ++half)
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) m[2 * half + ((i >> 1) & 1)] = fmaxf(m[2 * half + ((i >> 1) & 1)], fabsf(x[half][i]));
-                row_maxima(s, pl, m);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xs[i] = power_of_two(m[i], xi[i]);
-#pragma unroll
-                for (int half = 0; half < 2; ++half) store_operand(A0, pl, half, x[half], xs[2 * half], xs[2 * half + 1]);
-                fence_async_smem();
-                fence_before();
-                mbar_arrive(s.bar(B_A0));
-            };
             if (head) {
                 // ---- gq' and gk as operands 0 and 1, with one scale per row for the three of them (their products meet in
                 //      one accumulator); warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (head l / 4)
                 const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
-                const float lb = lane < 16 ? p.lower_bound : p.lower_bound_hi;
-                const float slope = p.gauss_scale * (lane < 16 ? p.a_factor : p.a_factor_hi) * p.elu_beta;
                 float *inv_out = s.row_floats(0);
                 const uint32_t lane_at = (lane >> 4) * 16384 + (lane & 1) * 8;
                 auto put = [&](unsigned char *buf, int row, const float4 v, float sc) {
@@ -135,23 +175,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                             gvv = *reinterpret_cast<const float4 *>(p.gv + row * 128 + 4 * lane);
                             ga = p.ga[row * HEADS + (lane >> 2)];
                         }
-                        // alpha of the head (q is stored divided by 4), the slope of its width, and gq'
-                        float al = 4.0f * fmaf(qv.w, wp.w, fmaf(qv.z, wp.z, fmaf(qv.y, wp.y, qv.x * wp.x)));
-                        al += __shfl_xor_sync(FULL, al, 1);
-                        al += __shfl_xor_sync(FULL, al, 2);
-                        const float tt = (al + p.gauss_shift) * p.gauss_scale * (p.elu_beta / (1.0f - lb));
-                        float galpha = ga * slope * (tt > 0.f ? 1.0f : expf(tt));
-                        if (p.inverse) {
-                            const float f = (1.0f - lb) * (tt > 0.f ? tt : expm1f(tt)) + 1.0f;
-                            galpha = -galpha / (f * f);
-                        }
-                        gq[u].x = fmaf(galpha, wp.x, 0.25f * gq[u].x); gq[u].y = fmaf(galpha, wp.y, 0.25f * gq[u].y);
-                        gq[u].z = fmaf(galpha, wp.z, 0.25f * gq[u].z); gq[u].w = fmaf(galpha, wp.w, 0.25f * gq[u].w);
-                        __syncwarp();  // (the lanes of a head have read ga)
-                        if (row < p.N) {
-                            *reinterpret_cast<float4 *>(p.gq + row * 128 + 4 * lane) = gq[u];
-                            if ((lane & 3) == 0) p.ga[row * HEADS + (lane >> 2)] = galpha;
-                        }
+                        gq[u] = query_grad(p, wp, gq[u], qv, ga, row);
                         const float mq = fmaxf(fmaxf(fabsf(gq[u].x), fabsf(gq[u].y)), fmaxf(fabsf(gq[u].z), fabsf(gq[u].w)));
                         const float mk = fmaxf(fmaxf(fabsf(gk[u].x), fabsf(gk[u].y)), fmaxf(fabsf(gk[u].z), fabsf(gk[u].w)));
                         const float mv = fmaxf(fmaxf(fabsf(gvv.x), fabsf(gvv.y)), fmaxf(fabsf(gvv.z), fabsf(gvv.w)));
@@ -205,38 +229,13 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 for (int half = 0; half < 2; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!tail) continue;
-            publish();  // gx
+            publish_rows(s, pl, x, xi);  // gx
             // ---- hidden units: one scale per row for all chunks, |gh| <= 128 max|gx| max|W2| (see the forward)
             float hs[4], hi[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) hs[i] = power_of_two(137438953472.0f * xi[i] * w2_i, hi[i]);
-            for (int c = 0; c < chunks; ++c) {
-                const int d_col = (c & 1) ? D1 : D0;
-                unsigned live = 0u;  // bit 16 half + i: the unit was active
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float h[16];
-                    load_rows(p.h + 128 * c, p.ff, row_base, p.N, pl, half, h);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) live |= (h[i] > 0.f ? 1u : 0u) << (16 * half + i);
-                }
-                ph.wait(s, (c & 1) ? B_D1 : B_D0);
-                fence_after();
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float g[16];
-                    tmem_load_16x32(pl.tmem(tmem, d_col, half), g);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        g[i] = (live >> (16 * half + i)) & 1u ? g[i] * (xi[2 * half + ((i >> 1) & 1)] * w2_i) : 0.f;
-                    if (half == 0 && c > 0) ph.wait(s, B_A1_FREE);
-                    store_operand(A1, pl, half, g, hs[2 * half], hs[2 * half + 1]);
-                    store_rows(p.gh + 128 * c, p.ff, row_base, p.N, pl, half, g);
-                }
-                fence_async_smem();
-                fence_before();
-                mbar_arrive(s.bar(B_A1));
-            }
+            for (int c = 0; c < chunks; ++c)
+                hidden_grads(p, s, pl, ph, tmem, (c & 1) ? D1 : D0, (c & 1) ? B_D1 : B_D0, c, row_base, xi, w2_i, hs, OFF_A1, B_A1, c > 0);
             ph.wait(s, B_A1_FREE);
             ph.wait(s, B_DX);
             fence_after();
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
 #pragma unroll
                 for (int i = 0; i < 16; ++i) x[half][i] = fmaf(d[i], hi[2 * half + ((i >> 1) & 1)] * w1_i, x[half][i]);
             }
-            publish();  // gy
+            publish_rows(s, pl, x, xi);  // gy
 #pragma unroll
             for (int half = 0; half < 2; ++half) store_rows(p.gy, 128, row_base, p.N, pl, half, x[half]);
             ph.wait(s, B_D0);
@@ -262,6 +261,203 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             }
         }
     }
+    block_end(s, tmem, &g_dense_backward_status);
+}
+
+// The same for a cluster of four blocks (dense_tc_core.cuh): block 0, 1, 2 multiplies gq', gk, gv, block r hidden chunk r,
+// block 0 the last product; the shares of gx and of gy are collected by rows of 32.
+// 2,400 rows, 512 hidden units, mean of a network's boundaries: 38 us with a block per tile, 27 here.
+__global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(const DenseBackward p)
+{
+    extern __shared__ __align__(1024) unsigned char smem_tc[];
+    uint32_t tmem;
+    const Shared s = block_begin(smem_tc, tmem);
+    const uint32_t rank = cluster_rank();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chunks = p.ff / 128;
+    const long long row_base = (long long)(blockIdx.x / SPLIT) * 128;
+    const bool head = p.head != nullptr, tail = p.tail != nullptr;
+    const bool has_head = head && rank < 3, has_chunk = tail && (int)rank < chunks, has_last = tail && rank == 0;
+    grid_launch_dependents();
+    cluster_sync();  // every block's barriers are ready for the others' arrivals
+    grid_dependency_wait();  // (the images were written by a kernel of this step)
+
+    if (warp == STREAM_WARP) {
+        if (lane == 0) {
+            Producer<SPLIT_STAGES> pr;
+            if (has_head) pr.stream(s, p.head, (int)rank, 1);
+            if (has_chunk && pr.ok) pr.stream(s, p.tail, 3 + first_of_chunk(rank), 1);
+            if (has_chunk && pr.ok) pr.stream(s, p.tail, 3 + second_of_chunk(rank, chunks), 1);
+            if (has_last && pr.ok) pr.stream(s, p.tail, 3 + 2 * chunks, 1);
+            if (!pr.ok) pr.drain(s);
+        }
+        __syncwarp();
+    } else if (warp == ISSUE_WARP) {
+        if (lane == 0) {
+            Issuer<SPLIT_STAGES> is;
+            Phase ph;
+            bool ok = true;
+            auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
+            auto rows_ready = [&]() {
+                ok = ph.wait_cluster(s, B_ROWS) && ok;
+                fence_async_smem();
+                fence_after();
+            };
+            auto product = [&](int d, int done) {
+                if (ok) is.product(s, tmem, d, OFF_A0, false);
+                ok = ok && is.ok;
+                mma_commit(s.bar(done));
+            };
+            if (has_head) {
+                ready(B_A0);
+                product(D0, B_D0);
+            }
+            if (tail) {
+                if (head) rows_ready(); else ready(B_A0);  // gx
+                if (has_chunk) {
+                    product(D1, B_D1);
+                    ready(B_A0);
+                    product(DX, B_DX);
+                }
+                if (has_last) {
+                    rows_ready();  // gy
+                    product(D0, B_D0);
+                }
+            }
+            if (!ok) is.drain(s);
+        }
+        __syncwarp();
+    } else {
+        const Place pl;
+        const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] : 0.f;
+        float w2_i = 0.f, w1_i = 0.f, wo_i = 0.f;
+        if (tail) {
+            const float *inv = reinterpret_cast<const float *>(p.tail);
+            w2_i = inv[3]; w1_i = inv[3 + 2 * chunks - 1]; wo_i = inv[3 + 2 * chunks];
+        }
+        Phase ph;
+        float xi[4];
+        // shares of a sum from the accumulator d_col (or nothing) to the blocks that finish the rows
+        auto send = [&](int d_col, bool any, float w_i, const float (&ri)[4]) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float d[16];
+                if (any) {
+                    tmem_load_16x32(pl.tmem(tmem, d_col, half), d);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) d[i] = 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; ++i) d[i] *= ri[2 * half + ((i >> 1) & 1)] * w_i;
+                stage_share(s, pl, half, d);
+            }
+            send_share(s, rank);
+        };
+        // the rows that this warp finishes: 2 warp + u of the block's 32
+        const long long own = row_base + 32 * (int)rank + 2 * warp;
+        auto load_own = [&](const float *src, float4 (&v)[2]) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                v[u] = own + u < p.N ? *reinterpret_cast<const float4 *>(src + (own + u) * 128 + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        auto collect = [&](float4 (&sum)[2], float *dst) {  // sum += the four shares
+            float4 v[2];
+            if (threadIdx.x == 0) expect_shares(s);
+            collect_shares(s, ph, v);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                sum[u].x += v[u].x; sum[u].y += v[u].y; sum[u].z += v[u].z; sum[u].w += v[u].w;
+                if (own + u < p.N) *reinterpret_cast<float4 *>(dst + (own + u) * 128 + 4 * lane) = sum[u];
+            }
+        };
+        float4 g[2];  // gx, then gy, of the own rows
+        if (head) {
+            if (rank == 0) {
+                const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
+                load_operand(s, s.mem + OFF_A0, [&](int r, int) {
+                    const long long row = row_base + r;
+                    float4 gq = make_float4(0.f, 0.f, 0.f, 0.f), qv = gq;
+                    float ga = 0.f;
+                    if (row < p.N) {
+                        gq = *reinterpret_cast<const float4 *>(p.gq + row * 128 + 4 * lane);
+                        qv = *reinterpret_cast<const float4 *>(p.q + row * 128 + 4 * lane);
+                        ga = p.ga[row * HEADS + (lane >> 2)];
+                    }
+                    return query_grad(p, wp, gq, qv, ga, row);
+                });
+            } else if (rank < 3) {
+                const float *src = rank == 1 ? p.gk : p.gv;
+                load_operand(s, s.mem + OFF_A0, [&](int r, int) {
+                    return row_base + r < p.N ? *reinterpret_cast<const float4 *>(src + (row_base + r) * 128 + 4 * lane)
+                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+                });
+            }
+            load_own(p.g_res, g);
+            if (has_head) {
+                fence_async_smem();
+                fence_before();
+                mbar_arrive(s.bar(B_A0));
+                epilogue_sync();
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
+                ph.wait(s, B_D0);
+                fence_after();
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xi[i] = 0.f;
+            }
+            send(D0, has_head, wh_i, xi);
+            collect(g, p.gx);
+            if (tail) {
+                if (threadIdx.x == 0) expect_rows(s);
+                spread_rows(s, ph, rank, g, SPLIT, 1);
+                ph.wait_cluster(s, B_ROWS);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(1)[pl.row0 + 8 * i];
+            }
+        } else {
+            float x[2][16];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
+            load_own(p.gx, g);
+            publish_rows(s, pl, x, xi);
+        }
+        if (tail) {
+            // ---- hidden units: one scale per row for all chunks, |gh| <= 128 max|gx| max|W2| (see the forward)
+            float hs[4], hi[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) hs[i] = power_of_two(137438953472.0f * xi[i] * w2_i, hi[i]);
+            if (has_chunk) {
+                hidden_grads(p, s, pl, ph, tmem, D1, B_D1, rank, row_base, xi, w2_i, hs, OFF_A0, B_A0, false);
+                ph.wait(s, B_DX);
+                fence_after();
+            } else {
+                epilogue_sync();  // (buffer 0 is about to take the shares: gx is no longer being written)
+            }
+            send(DX, has_chunk, w1_i, hi);
+            collect(g, p.gy);
+            if (threadIdx.x == 0 && has_last) expect_rows(s);
+            spread_rows(s, ph, rank, g, 1, 2);
+            if (has_last) {
+                ph.wait_cluster(s, B_ROWS);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(2)[pl.row0 + 8 * i];
+                ph.wait(s, B_D0);
+                fence_after();
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float d[16];
+                    tmem_load_16x32(pl.tmem(tmem, D0, half), d);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) d[i] *= xi[2 * half + ((i >> 1) & 1)] * wo_i;
+                    store_rows(p.gattn, 128, row_base, p.N, pl, half, d);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    cluster_sync();  // (no block ends while another may still write to it)
     block_end(s, tmem, &g_dense_backward_status);
 }
 
@@ -463,19 +659,15 @@ int grad_splits(int count, long long rows)
 int launch_dense_backward(const DenseBackward &p, cudaStream_t s)
 {
     if (p.N == 0) return CF_OK;
-    static thread_local bool configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!configured[dev & 63]) {
-        if (cudaFuncSetAttribute(dense_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc5::SMEM_BYTES) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(CF_ERR_CUDA, "dense backward: %d bytes of shared memory not available", tc5::SMEM_BYTES);
-        }
-        configured[dev & 63] = true;
-    }
+    static thread_local DenseLaunch launch;
+    int rc = launch.configure(reinterpret_cast<const void *>(dense_backward_kernel), reinterpret_cast<const void *>(dense_backward_split_kernel), "dense backward");
+    if (rc != CF_OK) return rc;
     const long long tiles = (p.N + 127) / 128, cap = sm_count();
-    launch_chained(dense_backward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
-                   p.chained, p);
+    if (split_tiles(tiles, p.ff, launch.clusters()))
+        launch_chained_cluster(dense_backward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, p.chained, p);
+    else
+        launch_chained(dense_backward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
+                       p.chained, p);
     return launch_status("dense_backward_kernel");
 }
 

@@ -12,6 +12,8 @@
 #include "dense_tc.cuh"
 #include "tc5.cuh"
 
+#include "common.cuh"
+
 namespace cf {
 namespace tc5 {
 
@@ -23,7 +25,7 @@ constexpr int OFF_A0 = 0, OFF_A1 = OPERAND_BYTES, OFF_RING = 2 * OPERAND_BYTES, 
 constexpr int OFF_ROW = OFF_MISC + 256;             // 5 x 128 floats: scales of loaded rows, row maxima of the column groups
 constexpr int SMEM_BYTES = OFF_ROW + 5 * 512 + 64;  // (+ a word per epilogue warp)
 static_assert(SMEM_BYTES <= 232448, "shared memory of one SM");
-enum Barrier { B_FULL = 0, B_EMPTY = STAGES, B_D0 = 2 * STAGES, B_D1, B_DX, B_A0, B_A1, B_A1_FREE, B_DRAIN };
+enum Barrier { B_FULL = 0, B_EMPTY = STAGES, B_D0 = 2 * STAGES, B_D1, B_DX, B_A0, B_A1, B_A1_FREE, B_DRAIN, B_PART, B_ROWS, B_GO };
 constexpr int D0 = 0, D1 = 128, DX = 256;           // accumulators (columns of tensor memory)
 
 struct Shared {
@@ -46,9 +48,16 @@ struct Phase {
         bits ^= 1u << b;
         return ok;
     }
+    __device__ __forceinline__ bool wait_cluster(const Shared &s, int b)  // arrivals from other blocks of the cluster
+    {
+        const bool ok = mbar_wait<true>(s.bar(b), (bits >> b) & 1u, s.gave_up);
+        bits ^= 1u << b;
+        return ok;
+    }
 };
 
 // ---- weight stream (one thread) -------------------------------------------------------------------------------------
+template <int STAGES>
 struct Producer {
     int slot = 0;
     int requested = 0;   // stages asked for so far
@@ -76,6 +85,7 @@ struct Producer {
 };
 
 // ---- tensor instructions (one thread) ---------------------------------------------------------------------------------
+template <int STAGES>
 struct Issuer {
     int slot = 0;
     uint32_t phase = 0;
@@ -171,6 +181,24 @@ __device__ __forceinline__ void row_maxima(const Shared &s, const Place &pl, flo
     epilogue_sync();
 }
 
+// The block's rows as operand 0: scales from the largest magnitude of every row (xi: 1 / scale of the thread's rows).
+__device__ __forceinline__ void publish_rows(const Shared &s, const Place &pl, const float (&x)[2][16], float (&xi)[4])
+{
+    float m[4] = {0.f, 0.f, 0.f, 0.f}, xs[4];
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) m[2 * half + ((i >> 1) & 1)] = fmaxf(m[2 * half + ((i >> 1) & 1)], fabsf(x[half][i]));
+    row_maxima(s, pl, m);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xs[i] = power_of_two(m[i], xi[i]);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) store_operand(s.mem + OFF_A0, pl, half, x[half], xs[2 * half], xs[2 * half + 1]);
+    fence_async_smem();
+    fence_before();
+    mbar_arrive(s.bar(B_A0));
+}
+
 // this thread's eight values of a per-column constant (read before the wait for the product that needs them)
 __device__ __forceinline__ void load_columns(const float *src, const Place &pl, float2 (&b)[4])
 {
@@ -245,6 +273,137 @@ __device__ __forceinline__ void load_operand(const Shared &s, unsigned char *buf
     }
 }
 
+// ---- a tile shared by four blocks ---------------------------------------------------------------------------------------
+// A boundary is a chain of twelve products per tile, about a microsecond each on one SM's tensor pipe; with few tiles most
+// SMs have none.  A cluster of four blocks then takes a tile: block r multiplies hidden chunk r and head matrix r, products
+// that precede them are done by all four.  Where the chunks meet in one sum, every block sends its share (already in units
+// of the result) of rows 32 o .. 32 o + 31 to block o (slot r of operand buffer 1, which these blocks do not use
+// otherwise); block o adds the four in rank order, finishes its 32 rows and, where they are the next operand, writes them
+// into operand buffer 0 of every block that needs them.  Both transfers are bulk copies between the blocks' shared
+// memories, from a staging place of the sender (shares: its operand buffer 0; finished rows: the third stage of the weight
+// ring, which these blocks do without) with the bytes counted on the receiver's barrier, B_PART and B_ROWS: 3.5 us for the
+// shares and 2.2 for the rows, against 3.9 and 2.7 with plain stores to the other blocks (48 KB leave every block: about 17
+// bytes per ns, what an SM's link to the others in its cluster gives).  Rows may overwrite a
+// receiver's operand buffer 0 once its own shares have left it: every block tells the others when it has received all of
+// its shares (B_GO).
+constexpr int SPLIT = 4, SPLIT_STAGES = STAGES - 1;
+constexpr int OFF_STAGING = OFF_RING + SPLIT_STAGES * STAGE_BYTES;
+constexpr int SHARE_BYTES = 16384, ROWS_BYTES = 16384 + 128;
+
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t at_rank(uint32_t addr, uint32_t rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync()  // every thread of the four blocks
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void arrive_at(uint32_t bar_of_rank)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_of_rank) : "memory");
+}
+// shared memory of this block -> shared memory of another, the bytes counted on a barrier there
+__device__ __forceinline__ void bulk_send(uint32_t dst_of_rank, uint32_t src, uint32_t bytes, uint32_t bar_of_rank)
+{
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_of_rank),
+                 "r"(src), "r"(bytes), "r"(bar_of_rank)
+                 : "memory");
+}
+// (one thread of the receiver, once per transfer; the bytes may come first)
+__device__ __forceinline__ void expect_shares(const Shared &s) { mbar_expect(s.bar(B_PART), SPLIT * SHARE_BYTES); }
+__device__ __forceinline__ void expect_rows(const Shared &s) { mbar_expect(s.bar(B_ROWS), SPLIT * ROWS_BYTES); }
+
+// One half (16 values) of this thread's part of the share, staged for the block that finishes these rows.  A row of a share
+// is 512 bytes, its 32-byte pieces swizzled by the row so that a warp's stores meet no bank twice.
+__device__ __forceinline__ void stage_share(const Shared &s, const Place &pl, int half, const float (&v)[16])
+{
+    unsigned char *share = s.mem + OFF_A0 + ((threadIdx.x >> 5) & 3) * SHARE_BYTES;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        unsigned char *at = share + (pl.g + 16 * half) * 512 + (((4 * pl.group + j) ^ pl.g) << 5) + pl.t * 8;
+        *reinterpret_cast<float2 *>(at) = make_float2(v[4 * j], v[4 * j + 1]);
+        *reinterpret_cast<float2 *>(at + 8 * 512) = make_float2(v[4 * j + 2], v[4 * j + 3]);
+    }
+}
+// The four warps that staged a share meet, and one thread sends it.
+__device__ __forceinline__ void send_share(const Shared &s, uint32_t rank)
+{
+    const uint32_t to = (threadIdx.x >> 5) & 3u;
+    fence_async_smem();
+    fence_before();
+    asm volatile("bar.sync %0, 128;" ::"r"(2u + to) : "memory");
+    if ((threadIdx.x & 31) == 0 && (threadIdx.x >> 7) == 0)
+        bulk_send(at_rank(s.base + OFF_A1 + rank * SHARE_BYTES, to), s.base + OFF_A0 + to * SHARE_BYTES, SHARE_BYTES, at_rank(s.bar(B_PART), to));
+}
+// The sums of this block's rows, once the four shares are here: row 2 w + u of its 32, columns 4 l .. 4 l + 3.
+__device__ __forceinline__ void collect_shares(const Shared &s, Phase &ph, float4 (&v)[2])
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    ph.wait_cluster(s, B_PART);
+    if (w == 0 && lane < SPLIT) arrive_at(at_rank(s.bar(B_GO), (uint32_t)lane));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int row = 2 * w + u;
+        const unsigned char *at = s.mem + OFF_A1 + row * 512 + (((lane >> 1) ^ (row & 7)) << 5) + (lane & 1) * 16;
+        float4 a = *reinterpret_cast<const float4 *>(at);
+#pragma unroll
+        for (int slot = 1; slot < SPLIT; ++slot) {
+            const float4 b = *reinterpret_cast<const float4 *>(at + slot * SHARE_BYTES);
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+        v[u] = a;
+    }
+}
+// The block's finished rows as operand 0 (and 1 / scale as row floats `which`) of the first `receivers` blocks.
+__device__ __forceinline__ void spread_rows(const Shared &s, Phase &ph, uint32_t rank, const float4 (&v)[2], int receivers, int which)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float m[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) m[u] = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) m[u] = fmaxf(m[u], __shfl_xor_sync(FULL, m[u], o));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int row = 2 * w + u;
+        float inv;
+        const float sc = power_of_two(m[u], inv);
+        uint2 h0, h1;
+        split_pair(v[u].x * sc, v[u].y * sc, h0.x, h1.x);
+        split_pair(v[u].z * sc, v[u].w * sc, h0.y, h1.y);
+        // staged by (k panel, piece): 32 rows x 128 bytes each, as the operand has them
+        unsigned char *at = s.mem + OFF_STAGING + (lane >> 4) * 8192 + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + (lane & 1) * 8;
+        *reinterpret_cast<uint2 *>(at) = h0;
+        *reinterpret_cast<uint2 *>(at + 4096) = h1;
+        if (lane == 0) *reinterpret_cast<float *>(s.mem + OFF_STAGING + 16384 + row * 4) = inv;
+    }
+    fence_async_smem();
+    epilogue_sync();
+    if (w == 0) {
+        const int to = lane >> 2, part = lane & 3;  // (k panel, piece)
+        ph.wait_cluster(s, B_GO);
+        if (to < receivers) {
+            const uint32_t bar = at_rank(s.bar(B_ROWS), (uint32_t)to), from = s.base + OFF_STAGING + part * 4096;
+            bulk_send(at_rank(s.base + OFF_A0 + (part >> 1) * 16384 + (part & 1) * 32768 + rank * 4096u, (uint32_t)to), from, 4096, bar);
+            if (part == 0)
+                bulk_send(at_rank(s.base + OFF_ROW + (uint32_t)(which * 512) + rank * 128u, (uint32_t)to), s.base + OFF_STAGING + 16384, 128, bar);
+        }
+    }
+}
+// positions of a chunk's two blocks in the interleaved order of an image (first the block that makes the hidden units)
+__device__ __forceinline__ int first_of_chunk(int c) { return c < 2 ? c : 2 * c - 1; }
+__device__ __forceinline__ int second_of_chunk(int c, int chunks) { return min(c + 2, chunks) + c; }
+
 // ---- block set-up and end -----------------------------------------------------------------------------------------------
 __device__ __forceinline__ Shared block_begin(unsigned char *mem, uint32_t &tmem)
 {
@@ -257,6 +416,7 @@ __device__ __forceinline__ Shared block_begin(unsigned char *mem, uint32_t &tmem
         mbar_init(s.bar(B_D0), 1); mbar_init(s.bar(B_D1), 1); mbar_init(s.bar(B_DX), 1);
         mbar_init(s.bar(B_A0), EPI_THREADS); mbar_init(s.bar(B_A1), EPI_THREADS); mbar_init(s.bar(B_A1_FREE), 1);
         mbar_init(s.bar(B_DRAIN), 1);
+        mbar_init(s.bar(B_PART), 1); mbar_init(s.bar(B_ROWS), 1); mbar_init(s.bar(B_GO), SPLIT);
         *s.gave_up = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
@@ -276,6 +436,43 @@ __device__ __forceinline__ void block_end(const Shared &s, uint32_t tmem, unsign
     if ((threadIdx.x >> 5) == ISSUE_WARP) tmem_free<512>(tmem);
     if (threadIdx.x == 0 && *s.gave_up != 0u) atomicOr(status, 1u);
 }
+
+// ---- host side ------------------------------------------------------------------------------------------------------------
+// The rule: a cluster per tile while all clusters fit at once (with a second wave, 41 tiles: 52 us against 39 with a block
+// per tile, forward; 56 against 41 backward), and one chunk per block at most.
+inline bool split_tiles(long long tiles, int ff, int clusters) { return ff <= 128 * SPLIT && tiles <= clusters; }
+
+struct DenseLaunch {  // per thread: what a device's set-up of the two kernels gave
+    int clusters_of[64] = {};  // clusters that fit at once; 0: not set up yet
+    int device = 0;
+    int configure(const void *alone, const void *split, const char *what)
+    {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        device = dev & 63;
+        if (clusters_of[device] > 0) return CF_OK;
+        if (cudaFuncSetAttribute(alone, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess ||
+            cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(CF_ERR_CUDA, "%s: %d bytes of shared memory not available", what, SMEM_BYTES);
+        }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(SPLIT); cfg.blockDim = dim3(BLOCK_THREADS); cfg.dynamicSmemBytes = SMEM_BYTES;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = SPLIT; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, split, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = sm_count() / SPLIT;
+        }
+        clusters_of[device] = n;
+        return CF_OK;
+    }
+    int clusters() const { return clusters_of[device]; }
+};
 
 }  // namespace tc5
 }  // namespace cf

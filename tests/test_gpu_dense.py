@@ -39,3 +39,43 @@ def test_one_call_forward_with_images_equals_the_gemm_path(ff, sizes):
             out[fused] = (model(data), model.encoder(emb, data.pos, geo.batch, data.trans_vec, geo.sizes, geometry=geo))
     assert rel_err(out[True][1].cpu().numpy(), out[False][1].cpu().numpy()) < 3e-6
     assert (out[True][0] - out[False][0]).abs().max() < 1e-6  # (embedding, pooling and head included)
+
+
+@pytest.mark.parametrize("ff", [128, 384, 512, 640])
+@pytest.mark.parametrize("atoms", [1, 33, 4737, 9600])
+def test_boundaries_shared_by_a_cluster_or_not(ff, atoms):
+    """A tile per cluster of four blocks (few tiles, at most four hidden chunks) and a tile per block: one row, rows of two of
+    the four blocks, more clusters than fit at once, more tiles than two waves of clusters; with and without blocks idle."""
+    from crystalformer_b200.model import Latticeformer, default_params
+    torch.manual_seed(atoms + ff)
+    model = Latticeformer(default_params(num_layers=2, ff_dim=ff)).cuda()
+    for p in model.parameters():
+        if p.requires_grad:
+            p.data.add_(torch.randn_like(p) * 0.05)
+    sizes = [1] * min(atoms, 7) + [30] * ((atoms - 7) // 30) + [(atoms - 7) % 30 or 1] if atoms > 7 else [1] * atoms
+    cb = make_crystals(4, len(sizes), lambda rng, b: np.array(sizes), length_range=(8.0, 14.0))
+    t = lambda x: torch.as_tensor(x).cuda()
+    data = types.SimpleNamespace(x=t(cb.x), pos=t(cb.pos), trans_vec=t(cb.trans_vec), sizes=t(cb.sizes))
+    model.train()
+    with torch.no_grad():
+        model(data)
+    model.eval()
+    out = {}
+    with torch.no_grad():
+        for fused in (True, False):
+            model.encoder.dense_fused = fused
+            out[fused] = model(data)
+    assert (out[True] - out[False]).abs().max() < 2e-6
+    # the training step's boundaries, forward and backward, against the layer-by-layer step
+    model.encoder.dense_fused = True
+    model.train()
+    grads = {}
+    for native in (True, False):
+        model.native = native
+        model.zero_grad(set_to_none=True)
+        model(data).abs().mean().backward()
+        grads[native] = {n: p.grad for n, p in model.named_parameters() if p.requires_grad}
+    noise = 1e-6 * max(float(g.norm()) for g in grads[False].values())
+    for n, g in grads[False].items():
+        # (a hidden unit within rounding of zero may fall on either side of the ReLU)
+        assert (grads[True][n] - g).norm() <= 2e-3 * g.norm() + noise, n
