@@ -439,8 +439,13 @@ __device__ __forceinline__ void block_end(const Shared &s, uint32_t tmem, unsign
 
 // ---- host side ------------------------------------------------------------------------------------------------------------
 // The rule: a cluster per tile while all clusters fit at once (with a second wave, 41 tiles: 52 us against 39 with a block
-// per tile, forward; 56 against 41 backward), and one chunk per block at most.
-inline bool split_tiles(long long tiles, int ff, int clusters) { return ff <= 128 * SPLIT && tiles <= clusters; }
+// per tile, forward; 56 against 41 backward), one chunk per block at most, and not where the caller asked for the least SM
+// time (dense_tile_rows 32: batches on several streams; four blocks of 20 us take more of the chip than one of 30, and a
+// stream of 128-crystal batches on four streams 3.52 ms instead of 3.31).
+inline bool split_tiles(long long tiles, int ff, int clusters)
+{
+    return ff <= 128 * SPLIT && tiles <= clusters && dense_tile_rows_choice() != 32;
+}
 
 struct DenseLaunch {  // per thread: what a device's set-up of the two kernels gave
     int clusters_of[64] = {};  // clusters that fit at once; 0: not set up yet

@@ -40,7 +40,7 @@ class PipelinedPredictor:
         batch; with a ``gather`` only if it overlaps its collects (its steps must otherwise run in one order on every
         rank's one stream).  ``dense_tile_rows`` (16, 32 or 0 = chosen per launch; default 32 with several streams, else
         0): the row tile of the fused dense blocks when batches are submitted through the library's one-call path:
-        32-row tiles take a little longer per forward and less SM time in total, which pays once streams overlap."""
+        with 32 the blocks take a little longer per forward and less SM time in total, which pays once streams overlap."""
         if depth < 1:
             raise ValueError("depth must be at least 1")
         self.model = model
