@@ -40,7 +40,7 @@ struct BwdRowArgs {
 __host__ __device__ inline size_t bwd_row_smem_floats(int max_atoms, bool with_basis)
 {
     // per atom: rel (4) + c (8) + p (8) + gov (8) + s0 (8); then u (8 x 64), per-warp candidates, ga partials
-    return (size_t)max_atoms * 36 + (with_basis ? HEADS * U_STRIDE : 0) + WARPS * 2 * BWD_RING + WARPS * 8 + 16;
+    return (size_t)max_atoms * 36 + (with_basis ? HEADS * U_STRIDE : 0) + WARPS * 2 * BWD_RING + WARPS * 8;
 }
 
 template <int K>
@@ -56,79 +56,102 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
     float *u = s0 + (size_t)p.max_atoms * 8;                           // [8][64]
     float *rings = u + (K > 0 ? HEADS * U_STRIDE : 0);                 // [WARPS][2 BWD_RING]
     float *ga_part = rings + WARPS * 2 * BWD_RING;                     // [WARPS][8]
-    float *delta_s = ga_part + WARPS * 8;                              // [8]
     CandidateRingOf<BWD_RING> ring;
     ring.init(rings + warp * 2 * BWD_RING, lane);
 
+    // what a row starts from: atom, edges, keys, first key; fetched a row ahead (dependent reads)
+    struct Row {
+        long long i, e0, a0;
+        int n;
+    };
+    auto row_of = [&](long long slot) {
+        Row r{0, 0, 0, 0};
+        if (slot < p.N) {
+            r.i = p.row_order ? p.row_order[slot] : slot;
+            r.e0 = p.row_start[r.i];
+            r.n = (int)(p.row_start[r.i + 1] - r.e0);
+            r.a0 = r.n > 0 ? p.edges[p.E + r.e0] : 0;
+        }
+        return r;
+    };
+    Row next = row_of(blockIdx.x);
     for (long long slot = blockIdx.x; slot < p.N; slot += gridDim.x) {
-        const long long i = p.row_order ? p.row_order[slot] : slot;
+        const long long i = next.i, e0 = next.e0, a0 = next.a0;
+        const int n = next.n;
         const long long c = p.batch[i];
-        const long long e0 = p.row_start[i];
-        const int n = (int)(p.row_start[i + 1] - e0);
-        const long long a0 = n > 0 ? p.edges[p.E + e0] : 0;
+        next = row_of(slot + gridDim.x);
         if (n > p.max_atoms) {
             p.gq[i * HEADS * HEAD_DIM + tid] = __int_as_float(0x7fc00000);
             if (tid < HEADS) p.ga[i * HEADS + tid] = __int_as_float(0x7fc00000);
             continue;
         }
-        // ---- relative positions, delta_i = gout_i . out_i, u_i = W^T gout_i
-        if (p.pos_ij) {
-            for (int j = tid; j < n; j += THREADS) {
-                const float *pp = p.pos_ij + 3 * (e0 + j);
-                rel[j] = make_float4(pp[0], pp[1], pp[2], 0.f);
-            }
-        } else {
-            const float pix = p.pos[3 * i], piy = p.pos[3 * i + 1], piz = p.pos[3 * i + 2];
-            for (int j = tid; j < n; j += THREADS) {
-                const float *pp = p.pos + 3 * (a0 + j);
-                rel[j] = make_float4(__fsub_rn(pp[0], pix), __fsub_rn(pp[1], piy), __fsub_rn(pp[2], piz), 0.f);
+        // ---- per key: (q.k - lse) log2e, p_ij, gout_i.v_j - delta_i.  A key's k and v rows are one coalesced read of a warp
+        //      each (lane l: channels 4 l .. 4 l + 3, head l / 4); the four lanes of a head add their partial products, and
+        //      then take one of the four results each.  delta_i = gout_i . out_i in every warp.  (One key per lane read
+        //      each of its 16-byte pieces from a line of its own: 60 % of the L1's wavefronts.)
+        {
+            const float4 q4 = __ldg(reinterpret_cast<const float4 *>(p.q + i * HEADS * HEAD_DIM) + lane);
+            const float4 go = __ldg(reinterpret_cast<const float4 *>(p.gout + i * HEADS * HEAD_DIM) + lane);
+            const float4 ou = __ldg(reinterpret_cast<const float4 *>(p.out + i * HEADS * HEAD_DIM) + lane);
+            const int h = lane >> 2, t = lane & 3;
+            const float lse = p.lse[i * HEADS + h];
+            const float4 *kp = reinterpret_cast<const float4 *>(p.k + a0 * HEADS * HEAD_DIM) + lane;
+            const float4 *vp = reinterpret_cast<const float4 *>(p.v + a0 * HEADS * HEAD_DIM) + lane;
+            float delta = fmaf(go.w, ou.w, fmaf(go.z, ou.z, fmaf(go.y, ou.y, go.x * ou.x)));
+            delta += __shfl_xor_sync(FULL, delta, 1);
+            delta += __shfl_xor_sync(FULL, delta, 2);
+            for (int j0 = 4 * warp; j0 < n; j0 += 4 * WARPS) {
+                float4 kk[4], vv[4];
+                float lg[4];
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const int j = min(j0 + w, n - 1);
+                    kk[w] = __ldg(kp + (size_t)j * 32);
+                    vv[w] = __ldg(vp + (size_t)j * 32);
+                    lg[w] = t == 2 ? p.logit[(e0 + j) * HEADS + h] : 0.f;
+                }
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    float s = fmaf(q4.w, kk[w].w, fmaf(q4.z, kk[w].z, fmaf(q4.y, kk[w].y, q4.x * kk[w].x)));
+                    float g = fmaf(go.w, vv[w].w, fmaf(go.z, vv[w].z, fmaf(go.y, vv[w].y, go.x * vv[w].x)));
+                    s += __shfl_xor_sync(FULL, s, 1);
+                    g += __shfl_xor_sync(FULL, g, 1);
+                    s += __shfl_xor_sync(FULL, s, 2);
+                    g += __shfl_xor_sync(FULL, g, 2);
+                    const float x = ((t == 0 ? s : lg[w]) - lse) * LOG2E;
+                    const float val = t == 0 ? x : t == 1 ? g - delta : t == 2 ? ex2(x) : 0.f;
+                    float *dst = (t == 0 ? cj : t == 1 ? gov : t == 2 ? pj : s0) + (j0 + w) * 8 + h;
+                    if (j0 + w < n) *dst = val;
+                }
             }
         }
-        {
-            // thread = (h, m): one element of gout_i and out_i; reduce the products over the 16 lanes of a head
-            float prod = p.gout[i * HEADS * HEAD_DIM + tid] * p.out[i * HEADS * HEAD_DIM + tid];
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) prod += __shfl_xor_sync(FULL, prod, o);
-            if ((tid & 15) == 0) delta_s[tid >> 4] = prod;
+        // ---- relative positions (rows without a list), u_i = W^T gout_i: thread = head and four bins
+        const int list_first = (p.list.pool != nullptr && n > 0) ? p.list.start[e0] : -1;
+        if (list_first < 0) {
+            const float pix = p.pos_ij ? 0.f : p.pos[3 * i], piy = p.pos_ij ? 0.f : p.pos[3 * i + 1], piz = p.pos_ij ? 0.f : p.pos[3 * i + 2];
+            for (int j = tid; j < n; j += THREADS) {
+                const float *pp = p.pos_ij ? p.pos_ij + 3 * (e0 + j) : p.pos + 3 * (a0 + j);
+                rel[j] = p.pos_ij ? make_float4(pp[0], pp[1], pp[2], 0.f)
+                                  : make_float4(__fsub_rn(pp[0], pix), __fsub_rn(pp[1], piy), __fsub_rn(pp[2], piz), 0.f);
+            }
         }
         if (K > 0) {
-            for (int idx = tid; idx < HEADS * KBINS; idx += THREADS) {
-                const int h = idx / KBINS, k = idx % KBINS;
-                const float *go = p.gout + (i * HEADS + h) * HEAD_DIM;
-                const float *w = p.W + (size_t)h * HEAD_DIM * KBINS + k;
-                float acc = 0.f;
+            const int h = tid >> 4, k4 = tid & 15;
+            const float4 *go4 = reinterpret_cast<const float4 *>(p.gout + (i * HEADS + h) * HEAD_DIM);
+            const float4 *w4 = reinterpret_cast<const float4 *>(p.W + (size_t)h * HEAD_DIM * KBINS) + k4;
+            float2 lo = make_float2(0.f, 0.f), hi = lo;
 #pragma unroll
-                for (int m = 0; m < HEAD_DIM; ++m) acc = fmaf(__ldg(w + m * KBINS), go[m], acc);
-                u[h * U_STRIDE + k] = acc;
-            }
-        }
-        __syncthreads();
-        // ---- per key: q.k - lse, p_ij, gout_i.v_j - delta_i; warp w owns heads 2w and 2w+1
+            for (int m4 = 0; m4 < HEAD_DIM / 4; ++m4) {
+                const float4 g4 = __ldg(go4 + m4);
+                const float g[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int h = 2 * warp + hh;
-            float4 qv[4], gv4[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                qv[t] = __ldg(reinterpret_cast<const float4 *>(p.q + (i * HEADS + h) * HEAD_DIM) + t);
-                gv4[t] = __ldg(reinterpret_cast<const float4 *>(p.gout + (i * HEADS + h) * HEAD_DIM) + t);
-            }
-            const float lse = p.lse[i * HEADS + h], dl = delta_s[h];
-            for (int j = lane; j < n; j += 32) {
-                const float4 *kp = reinterpret_cast<const float4 *>(p.k + ((a0 + j) * HEADS + h) * HEAD_DIM);
-                const float4 *vp = reinterpret_cast<const float4 *>(p.v + ((a0 + j) * HEADS + h) * HEAD_DIM);
-                float s = 0.f, g = 0.f;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float4 kv = __ldg(kp + t), vv = __ldg(vp + t);
-                    s = fmaf(qv[t].x, kv.x, s); s = fmaf(qv[t].y, kv.y, s); s = fmaf(qv[t].z, kv.z, s); s = fmaf(qv[t].w, kv.w, s);
-                    g = fmaf(gv4[t].x, vv.x, g); g = fmaf(gv4[t].y, vv.y, g); g = fmaf(gv4[t].z, vv.z, g); g = fmaf(gv4[t].w, vv.w, g);
+                for (int m = 0; m < 4; ++m) {
+                    const float4 w = __ldg(w4 + (4 * m4 + m) * (KBINS / 4));
+                    lo = fma2(make_float2(w.x, w.y), make_float2(g[m], g[m]), lo);
+                    hi = fma2(make_float2(w.z, w.w), make_float2(g[m], g[m]), hi);
                 }
-                cj[j * 8 + h] = (s - lse) * LOG2E;
-                pj[j * 8 + h] = ex2((p.logit[(e0 + j) * HEADS + h] - lse) * LOG2E);
-                gov[j * 8 + h] = g - dl;
-                s0[j * 8 + h] = 0.f;
             }
+            *reinterpret_cast<float4 *>(u + h * U_STRIDE + 4 * k4) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
         __syncthreads();
 
@@ -191,7 +214,8 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
                 const int id = got ? j : -1;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const bool same = __shfl_up_sync(FULL, id, o) == id && lane >= o;
+                    const bool same = __shfl_up_sync(FULL, id, o) == id && lane >= o && got;
+                    if (!__any_sync(FULL, same)) break;  // (no run of equal keys is longer than o)
 #pragma unroll
                     for (int h = 0; h < 8; ++h) {
                         const float up = __shfl_up_sync(FULL, pc[h], o);
@@ -215,7 +239,6 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
             const bool got = ring.take(d2, key);
             weigh(got, got ? (key & 2047) : 0, got ? d2 : 0.f, key);  // (a lane without an entry reads whatever the ring held)
         };
-        const int list_first = (p.list.pool != nullptr && n > 0) ? p.list.start[e0] : -1;
         if (list_first >= 0) {
             // ---- terms from the row's list (entries contiguous, keys ascending).  A warp takes whole keys, so that
             //      every per-key sum has one owner: warp w gets the keys whose first entry lies in its equal share
@@ -290,6 +313,7 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
             const int h = tid >> 4;
             float acc = 0.f;
             const float *kp = p.k + a0 * HEADS * HEAD_DIM + tid;
+#pragma unroll 8
             for (int j = 0; j < n; ++j) acc = fmaf(s0[j * 8 + h], __ldg(kp + (size_t)j * HEADS * HEAD_DIM), acc);
             p.gq[i * HEADS * HEAD_DIM + tid] = acc;
         }

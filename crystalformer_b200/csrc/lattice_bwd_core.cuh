@@ -13,27 +13,32 @@ namespace cf {
 
 constexpr int U_STRIDE = 64;                  // floats per head row of the u tile
 
+// Adds four bins' values of all heads: the even and the odd bins' sums of a head share a packed accumulator (one issue slot
+// for two products).
+__device__ __forceinline__ void basis_dot_step(const float *__restrict__ u, float &t, float bin_step, float2 (&c2)[8])
+{
+    const float t1 = t + bin_step, t2 = t1 + bin_step, t3 = t2 + bin_step;
+    const float2 g01 = make_float2(ex2(-t * t), ex2(-t1 * t1)), g23 = make_float2(ex2(-t2 * t2), ex2(-t3 * t3));
+    t = t3 + bin_step;
+#pragma unroll
+    for (int h = 0; h < 8; ++h) {
+        const float4 uv = *reinterpret_cast<const float4 *>(u + h * U_STRIDE);
+        c2[h] = fma2(make_float2(uv.z, uv.w), g23, fma2(make_float2(uv.x, uv.y), g01, c2[h]));
+    }
+}
+
 // c[h] = sum_k u[h][k] 2^(-((k+1) step - x)^2); u in shared memory, [8][U_STRIDE].
 template <int K>
 __device__ __forceinline__ void basis_dot(const float *__restrict__ u, float x, float bin_step, float (&c)[8])
 {
+    float2 c2[8];
 #pragma unroll
-    for (int h = 0; h < 8; ++h) c[h] = 0.f;
+    for (int h = 0; h < 8; ++h) c2[h] = make_float2(0.f, 0.f);
     float t = bin_step - x;
 #pragma unroll 2
-    for (int k = 0; k < K; k += 4) {
-        const float t1 = t + bin_step, t2 = t1 + bin_step, t3 = t2 + bin_step;
-        const float g0 = ex2(-t * t), g1 = ex2(-t1 * t1), g2 = ex2(-t2 * t2), g3 = ex2(-t3 * t3);
-        t = t3 + bin_step;
+    for (int k = 0; k < K; k += 4) basis_dot_step(u + k, t, bin_step, c2);
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-            const float4 uv = *reinterpret_cast<const float4 *>(u + h * U_STRIDE + k);
-            c[h] = fmaf(uv.x, g0, c[h]);
-            c[h] = fmaf(uv.y, g1, c[h]);
-            c[h] = fmaf(uv.z, g2, c[h]);
-            c[h] = fmaf(uv.w, g3, c[h]);
-        }
-    }
+    for (int h = 0; h < 8; ++h) c[h] = c2[h].x + c2[h].y;
 }
 
 // The same for a basis of one bin width (BasisParams::windowed): a value more than 8 bins from the term's centre
@@ -41,26 +46,16 @@ __device__ __forceinline__ void basis_dot(const float *__restrict__ u, float x, 
 // k0 <= floor(xi) - 8 < k0 + 4 (clamped to the table).  The rows of u are then read at lane-dependent offsets.
 __device__ __forceinline__ void basis_dot_window(const float *__restrict__ u, float x, float bin_step, float (&c)[8])
 {
+    float2 c2[8];
 #pragma unroll
-    for (int h = 0; h < 8; ++h) c[h] = 0.f;
+    for (int h = 0; h < 8; ++h) c2[h] = make_float2(0.f, 0.f);
     int k0 = (__float2int_rd(__fdividef(x, bin_step)) - 9) & ~3;
     k0 = max(0, min(k0, 44));
     float t = (float)(k0 + 1) * bin_step - x;
-    const float *uw = u + k0;
 #pragma unroll
-    for (int k = 0; k < 20; k += 4) {
-        const float t1 = t + bin_step, t2 = t1 + bin_step, t3 = t2 + bin_step;
-        const float g0 = ex2(-t * t), g1 = ex2(-t1 * t1), g2 = ex2(-t2 * t2), g3 = ex2(-t3 * t3);
-        t = t3 + bin_step;
+    for (int k = 0; k < 20; k += 4) basis_dot_step(u + k0 + k, t, bin_step, c2);
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-            const float4 uv = *reinterpret_cast<const float4 *>(uw + h * U_STRIDE + k);
-            c[h] = fmaf(uv.x, g0, c[h]);
-            c[h] = fmaf(uv.y, g1, c[h]);
-            c[h] = fmaf(uv.z, g2, c[h]);
-            c[h] = fmaf(uv.w, g3, c[h]);
-        }
-    }
+    for (int h = 0; h < 8; ++h) c[h] = c2[h].x + c2[h].y;
 }
 
 }  // namespace cf
