@@ -10,13 +10,15 @@
 // M_h bounds every exponent from above (a < 0, d2 >= dmin), so no weight overflows and no separate pass for the
 // soft-max statistics is needed: phi, the soft-max and the histogram come out of ONE sweep over the row's entries.
 //
-// A chunk of eight consecutive entries is one k-step of mma.m16n8k8 (TF32 operands, FP32 accumulators in registers):
-//     Psi^T tile [16 bins x 8 heads] += G [16 bins x 8 terms] . E [8 terms x 8 heads]
-//     P^T tile   [16 keys x 8 heads] += 1[j_t = key] [16 keys x 8 terms] . E
+// Two chunks of eight consecutive entries are one k-step of mma.m16n8k16 (half operands, FP32 accumulators in registers):
+//     Psi^T tile [16 bins x 8 heads] += G [16 bins x 16 terms] . E [16 terms x 8 heads]
+//     P^T tile   [16 keys x 8 heads] += 1[j_t = key] [16 keys x 16 terms] . E
 // Every lane computes its fragment elements directly in registers: lane (g = lane / 4, t = lane % 4) owns the terms
-// t and t + 4 of the chunk for head g (two exponentials: the B fragment) and bins g, g + 8 of a tile for the same two
-// terms (four exponentials: the A fragment).  FP32-level accuracy from TF32 products by splitting both operands into a
-// rounded high part and the exact remainder (three products; the one-hot operand of P is exact, two products).
+// 2 t, 2 t + 1 of either chunk for head g (four exponentials: the B fragment) and bins g, g + 8 of a tile for the same
+// terms (eight exponentials: the A fragment).  FP32-level accuracy by splitting both operands into a rounded high part and
+// the remainder (three products; the one-hot operand of P is exact, two products).  Pairs of terms share a register, so
+// splitting, the one-hot compares and the products take about half the instructions of TF32 operands and m16n8k8, which
+// this replaced: 1,024 crystals of 1-60 atoms 674 -> 620 us per call, 128 crystals of 1-30 atoms 41.2 -> 39.7 us.
 // Because the entries are sorted by distance a chunk touches only the one or two bin tiles around its distances, and
 // the sweep ends at the first chunk whose entries are below the weight floor for every head.
 //
@@ -24,6 +26,8 @@
 // left-over list and processed by the enumerating row kernel (infinite_attn_fwd.cu) afterwards.  Without a radial
 // basis (K = 0: PSI = false) the histogram, its tiles and the projection W drop out; the rest is the same (the
 // one-call forwards do not use that variant: there the enumerating kernel with term lists is faster).
+#include <cuda_fp16.h>
+
 #include "lattice_core.cuh"
 #include "row_list.cuh"
 
@@ -56,19 +60,35 @@ struct SortedRowArgs {
     unsigned long long *stats;  // optional: { chunks swept, (chunk, bin tile) pairs computed, rows } are added here
 };
 
-__device__ __forceinline__ void mma_tf32(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1)
+// A k-step is 16 entries (two chunks): m16n8k16 with half operands.
+__device__ __forceinline__ void mma_half(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1)
 {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// x = hi + lo with hi = x cut to the TF32 grid (10 mantissa bits) and lo the exact remainder (0 <= lo < 2^-10 x for the
-// non-negative values split here); products of such pairs, hi.hi + lo.hi + hi.lo, are within 2^-19 of x.y
-__device__ __forceinline__ void split_tf32(float x, unsigned &hi, unsigned &lo)
+// Values of [0, 1], scaled by 2^15, as two halves each: x = hi + lo to 2^-22 relative, and never worse than 2^-39 of the
+// largest value.  Products of such pairs, hi.hi + lo.hi + hi.lo, are within 2^-21 of x.y.  A pair of terms per register.
+constexpr float HALF_SCALE_LOG2 = 15.0f;
+// A head's sum is at least one if its box holds the term that its bound M_h comes from; below this the absolute floor of the
+// halves would show, and the row is left over.
+constexpr float MIN_SUM = 1.5e-5f;
+constexpr float UNSCALE = 1.0f / 32768.0f;
+__device__ __forceinline__ void split_halves(float x, float y, unsigned &hi, unsigned &lo)
 {
-    hi = __float_as_uint(x) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi));
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 back = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - back.x, y - back.y);
+    hi = *reinterpret_cast<const unsigned *>(&h);
+    lo = *reinterpret_cast<const unsigned *>(&l);
+}
+// 1.0 in every half of `pair` that equals `value`: small integers as the bits of halves (subnormal numbers, compared exactly)
+__device__ __forceinline__ unsigned one_where_equal(unsigned pair, unsigned value)
+{
+    const unsigned both = value * 0x10001u;
+    const __half2 r = __heq2(*reinterpret_cast<const __half2 *>(&pair), *reinterpret_cast<const __half2 *>(&both));
+    return *reinterpret_cast<const unsigned *>(&r);
 }
 
 // max over the warp of eight per-lane values, one per head, with nine shuffles: the lanes trade halves of their value
@@ -105,6 +125,7 @@ struct SortedSmem {
     float pj[SR_WARPS][8 * CJ_LD];        // P_h[j]
     float psi[SR_WARPS][PSI ? 8 * PSI_LD : 4];  // Psi_h[k]
     float2 ring[SR_WARPS][RING_SLOTS][64];  // list entries, 8 chunks (512 bytes) per slot
+    float xs[SR_WARPS][PSI ? 64 : 4];       // basis coordinates of the slot being swept
     long long next_task;
 };
 
@@ -210,6 +231,8 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
 #pragma unroll
     for (int m = 0; m < 4; ++m) accPsi[m][0] = accPsi[m][1] = accPsi[m][2] = accPsi[m][3] = 0.f;
     const float *cjg = cj + g * CJ_LD;
+    const float M_scaled = M_g - HALF_SCALE_LOG2;
+    const unsigned g_pair = (unsigned)g * 0x10001u;
     const float ucg = (float)(g + 1) * p.bin_step;          // centre of bin g in basis units
     const float step16 = 16.0f * p.bin_step, step8 = 8.0f * p.bin_step;
     bool more = true;
@@ -223,69 +246,75 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
         __syncwarp();
         const float2 *stage = ring[ring_slot];
         const int in_group = min(8, my_chunks - 8 * grp);
+        float *xs = sm.xs[warp];
+        if (PSI) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (lane + 32 * u < 8 * in_group) {
+                    const float d2 = stage[lane + 32 * u].x;
+                    xs[lane + 32 * u] = d2 * rsqrt_fast(fmaxf(d2, 1e-35f)) * p.bin_scale;
+                }
+            __syncwarp();
+        }
         for (int ch = 0; ch < in_group; ch += 2) {
             const bool two = ch + 1 < in_group;
-            const float2 e0a = stage[8 * ch + t], e0b = stage[8 * ch + t + 4];
-            const float2 e1a = stage[8 * (ch + (two ? 1 : 0)) + t], e1b = stage[8 * (ch + (two ? 1 : 0)) + t + 4];
+            const int chb = ch + (two ? 1 : 0);
             // entries ascend in d2: once a chunk's first entry is below the floor for every head, all that follow are
-            const float d2_first = __shfl_sync(FULL, e0a.x, 0);
-            if (__all_sync(FULL, fmaf(a2g, d2_first, slack_g) < p.floor_log2)) { more = false; break; }
-            const float d2v[4] = {e0a.x, e0b.x, e1a.x, e1b.x};
-            const int keyv[4] = {__float_as_int(e0a.y), __float_as_int(e0b.y), __float_as_int(e1a.y), __float_as_int(e1b.y)};
-            // B fragments: the weights of terms t, t + 4 of either chunk for head g
-            unsigned w_hi[4], w_lo[4];
-            int dj[4];
-            float x[4];
+            if (__all_sync(FULL, fmaf(a2g, stage[8 * ch].x, slack_g) < p.floor_log2)) { more = false; break; }
+            // terms 2 t, 2 t + 1 of either chunk
+            const float4 ea = *reinterpret_cast<const float4 *>(stage + 8 * ch + 2 * t), eb = *reinterpret_cast<const float4 *>(stage + 8 * chb + 2 * t);
+            const float d2v[4] = {ea.x, ea.z, eb.x, eb.z};
+            const int keyv[4] = {__float_as_int(ea.y), __float_as_int(ea.w), __float_as_int(eb.y), __float_as_int(eb.w)};
+            // B fragments: the weights of the four terms for head g
+            float w[4];
+            int jv[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int j = keyv[u] & 255;
-                float w = ex2(fmaf(a2g, d2v[u], cjg[j]) - M_g);
-                w = (row_key_in_box(keyv[u], boxor) && (u < 2 || two)) ? w : 0.f;
-                split_tf32(w, w_hi[u], w_lo[u]);
-                dj[u] = j - g;
-                if (PSI) x[u] = d2v[u] * rsqrt_fast(fmaxf(d2v[u], 1e-35f)) * p.bin_scale;  // basis coordinate of the term
+                jv[u] = keyv[u] & 255;
+                w[u] = ex2(fmaf(a2g, d2v[u], cjg[jv[u]]) - M_scaled);
+                w[u] = (row_key_in_box(keyv[u], boxor) && (u < 2 || two)) ? w[u] : 0.f;
             }
+            unsigned w_hi[2], w_lo[2];
+            split_halves(w[0], w[1], w_hi[0], w_lo[0]);
+            split_halves(w[2], w[3], w_hi[1], w_lo[1]);
             // P^T tiles: one-hot of the terms' keys (rows g, g + 8 of tile u are keys 16 u + g, 16 u + g + 8)
+            const unsigned ja = ((unsigned)jv[0] | ((unsigned)jv[1] << 16)) ^ g_pair, jb = ((unsigned)jv[2] | ((unsigned)jv[3] << 16)) ^ g_pair;
 #pragma unroll
             for (int u = 0; u < NT; ++u) {
-                unsigned o[8];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    o[2 * e] = dj[e] == 16 * u ? 0x3f800000u : 0u;
-                    o[2 * e + 1] = dj[e] == 16 * u + 8 ? 0x3f800000u : 0u;
-                }
-                mma_tf32(accP[u], o[0], o[1], o[2], o[3], w_hi[0], w_hi[1]);
-                mma_tf32(accP[u], o[0], o[1], o[2], o[3], w_lo[0], w_lo[1]);
-                mma_tf32(accP[u], o[4], o[5], o[6], o[7], w_hi[2], w_hi[3]);
-                mma_tf32(accP[u], o[4], o[5], o[6], o[7], w_lo[2], w_lo[3]);
+                const unsigned o0 = one_where_equal(ja, 16 * u), o1 = one_where_equal(ja, 16 * u + 8);
+                const unsigned o2 = one_where_equal(jb, 16 * u), o3 = one_where_equal(jb, 16 * u + 8);
+                mma_half(accP[u], o0, o1, o2, o3, w_hi[0], w_hi[1]);
+                mma_half(accP[u], o0, o1, o2, o3, w_lo[0], w_lo[1]);
             }
             swept += two ? 2 : 1;
             if (PSI) {
             // the bin tiles the two chunks can reach
-            const float x_first = __shfl_sync(FULL, x[0], 0), x_last = __shfl_sync(FULL, x[3], 3);
-            const float b_lo = fmaf(x_first, p.inv_bin_step, -1.0f - p.tile_reach);
-            const float b_hi = fmaf(x_last, p.inv_bin_step, -1.0f + p.tile_reach);
+            const float b_lo = fmaf(xs[8 * ch], p.inv_bin_step, -1.0f - p.tile_reach);
+            const float b_hi = fmaf(xs[8 * chb + 7], p.inv_bin_step, -1.0f + p.tile_reach);
             const int m_lo = max(0, __float2int_rd(b_lo * 0.0625f));
             const int m_hi = b_hi < 0.0f ? -1 : min(3, __float2int_rd(b_hi * 0.0625f));  // (beyond the last bin: only phi needs the terms)
-            const float uu[4] = {x[0] - ucg, x[1] - ucg, x[2] - ucg, x[3] - ucg};
+            const float2 xa = *reinterpret_cast<const float2 *>(xs + 8 * ch + 2 * t), xb = *reinterpret_cast<const float2 *>(xs + 8 * chb + 2 * t);
+            const float uu[4] = {xa.x - ucg, xa.y - ucg, xb.x - ucg, xb.y - ucg};
             tiles_done += max(m_hi - m_lo + 1, 0) * (two ? 2 : 1);
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 if (m < m_lo || m > m_hi) continue;  // (the same for every lane)
                 // A fragments: g_k(d) = exp2(-(c_k - x)^2) at bins 16 m + g, 16 m + g + 8 for the four terms
-                unsigned hi[8], lo[8];
+                float v0[4], v1[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float v0 = fmaf(-(float)m, step16, uu[e]), v1 = v0 - step8;
-                    split_tf32(ex2(-v0 * v0), hi[2 * e], lo[2 * e]);
-                    split_tf32(ex2(-v1 * v1), hi[2 * e + 1], lo[2 * e + 1]);
+                    const float c0 = fmaf(-(float)m, step16, uu[e]), c1 = c0 - step8;
+                    v0[e] = ex2(fmaf(-c0, c0, HALF_SCALE_LOG2));
+                    v1[e] = ex2(fmaf(-c1, c1, HALF_SCALE_LOG2));
                 }
-                mma_tf32(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_hi[0], w_hi[1]);
-                mma_tf32(accPsi[m], lo[0], lo[1], lo[2], lo[3], w_hi[0], w_hi[1]);
-                mma_tf32(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_lo[0], w_lo[1]);
-                mma_tf32(accPsi[m], hi[4], hi[5], hi[6], hi[7], w_hi[2], w_hi[3]);
-                mma_tf32(accPsi[m], lo[4], lo[5], lo[6], lo[7], w_hi[2], w_hi[3]);
-                mma_tf32(accPsi[m], hi[4], hi[5], hi[6], hi[7], w_lo[2], w_lo[3]);
+                unsigned hi[4], lo[4];
+                split_halves(v0[0], v0[1], hi[0], lo[0]);
+                split_halves(v1[0], v1[1], hi[1], lo[1]);
+                split_halves(v0[2], v0[3], hi[2], lo[2]);
+                split_halves(v1[2], v1[3], hi[3], lo[3]);
+                mma_half(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_hi[0], w_hi[1]);
+                mma_half(accPsi[m], lo[0], lo[1], lo[2], lo[3], w_hi[0], w_hi[1]);
+                mma_half(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_lo[0], w_lo[1]);
             }
             }
         }
@@ -303,17 +332,17 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
     __syncwarp();
 #pragma unroll
     for (int m = 0; m < (PSI ? 4 : 0); ++m) {
-        psi[(2 * t) * PSI_LD + 16 * m + g] = accPsi[m][0];
-        psi[(2 * t + 1) * PSI_LD + 16 * m + g] = accPsi[m][1];
-        psi[(2 * t) * PSI_LD + 16 * m + g + 8] = accPsi[m][2];
-        psi[(2 * t + 1) * PSI_LD + 16 * m + g + 8] = accPsi[m][3];
+        psi[(2 * t) * PSI_LD + 16 * m + g] = accPsi[m][0] * (UNSCALE * UNSCALE);
+        psi[(2 * t + 1) * PSI_LD + 16 * m + g] = accPsi[m][1] * (UNSCALE * UNSCALE);
+        psi[(2 * t) * PSI_LD + 16 * m + g + 8] = accPsi[m][2] * (UNSCALE * UNSCALE);
+        psi[(2 * t + 1) * PSI_LD + 16 * m + g + 8] = accPsi[m][3] * (UNSCALE * UNSCALE);
     }
 #pragma unroll
     for (int u = 0; u < NT; ++u) {
-        pj[(2 * t) * CJ_LD + 16 * u + g] = accP[u][0];
-        pj[(2 * t + 1) * CJ_LD + 16 * u + g] = accP[u][1];
-        pj[(2 * t) * CJ_LD + 16 * u + g + 8] = accP[u][2];
-        pj[(2 * t + 1) * CJ_LD + 16 * u + g + 8] = accP[u][3];
+        pj[(2 * t) * CJ_LD + 16 * u + g] = accP[u][0] * UNSCALE;
+        pj[(2 * t + 1) * CJ_LD + 16 * u + g] = accP[u][1] * UNSCALE;
+        pj[(2 * t) * CJ_LD + 16 * u + g + 8] = accP[u][2] * UNSCALE;
+        pj[(2 * t + 1) * CJ_LD + 16 * u + g + 8] = accP[u][3] * UNSCALE;
     }
     sync();
     if (COOP) {
@@ -339,7 +368,7 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
                 S += pw;
             }
         }
-        const bool failed = __syncthreads_or(!(S > 1e-30f));  // a head without a single listed term inside its box
+        const bool failed = __syncthreads_or(!(S > MIN_SUM));  // a head whose box misses the terms that gave its bound
         if (failed) return false;
         const float *ps = sm.psi[0] + h * PSI_LD;
         float o0 = 0.f, o1 = 0.f;
@@ -373,7 +402,7 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
                 S += pw;
             }
         }
-        if (__any_sync(FULL, !(S > 1e-30f))) return false;  // a head without a single listed term inside its box
+        if (__any_sync(FULL, !(S > MIN_SUM))) return false;  // a head whose box misses the terms that gave its bound
         // ---- W_g Psi_g for the lane's four channels 4 l .. 4 l + 3 (head g): W transposed in shared memory, so a
         //      warp reads 512 consecutive bytes per bin
         const float4 *wt4 = reinterpret_cast<const float4 *>(sm.wt) + lane;
