@@ -296,7 +296,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                 RowListBuild rb{};
                 rb.pos_ij = pos_ij; rb.tvecs = tvecs; rb.rvlen = cutoff_radius != 0.0 ? rvlen : nullptr;
                 rb.batch = batch; rb.edges = edges; rb.row_start = row_start; rb.row_order = row_order;
-                rb.N = N; rb.E = E; rb.rule = rule; rb.a_widest = a_widest; rb.window = window; rb.coop_chunks = ROW_COOP_CHUNKS;
+                rb.N = N; rb.E = E; rb.rule = rule; rb.a_widest = a_widest; rb.window = window; rb.coop_chunks = row_coop_chunks(rb.N);
                 rb.out = row_lists = row_list_carve(logit + E * 8 + 64, N, E);
                 rc = launch_row_list_build(rb, forked ? side.stream : s);
             } else {

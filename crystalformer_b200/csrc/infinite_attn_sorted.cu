@@ -1,5 +1,5 @@
 // Fused infinitely connected attention, forward, for batches of small crystals (at most 64 atoms per cell): one warp
-// per atom row (the four warps of a block share a row whose list is long), the row's terms read from its
+// per atom row (the warps of a block share a row whose list is long), the row's terms read from its
 // distance-sorted row list (row_list.cuh), every sum over terms done as tensor-core products.
 //
 // For row i (head h, Gaussian parameter a_h < 0) over its listed terms t = (key j_t, squared distance d2_t):
@@ -34,8 +34,10 @@
 namespace cf {
 namespace {
 
-constexpr int SR_THREADS = 128;
-constexpr int SR_WARPS = SR_THREADS / 32;
+// Warps of a block (they share the staged W): with up to 32 keys four blocks of four warps fit an SM, with up to 64 (larger
+// tables) only three, but two blocks of eight (442 -> 404 us per call, 1,024 crystals of 1-60 atoms).
+__host__ __device__ constexpr int sorted_warps(int NT) { return NT > 2 ? 8 : 4; }
+__host__ __device__ constexpr int sorted_blocks(int NT) { return NT > 2 ? 2 : 4; }
 constexpr int PSI_LD = 68;    // leading dimension of the histogram tile (heads x 64 bins): 4-bank shift per head
 constexpr int RING_SLOTS = 3; // groups of eight chunks staged per warp
 constexpr int CHANNELS = HEADS * HEAD_DIM;
@@ -119,6 +121,7 @@ __device__ __forceinline__ float warp_max_heads(const float (&v)[8], int lane)
 // Shared memory of one thread block (NT key tiles of 16; PSI: with the radial basis).
 template <int NT, bool PSI>
 struct SortedSmem {
+    static constexpr int SR_WARPS = sorted_warps(NT);
     static constexpr int CJ_LD = 16 * NT + 1;  // leading dimension of the per-(head, key) tables (odd: no bank conflicts)
     float wt[PSI ? 64 * CHANNELS : 4];    // W transposed: wt[k][channel], staged once per block
     float cj[SR_WARPS][8 * CJ_LD];        // s_h[j] per (head, key); a block working on one row uses table 0
@@ -130,13 +133,14 @@ struct SortedSmem {
 };
 
 // One row.  COOP = false: the calling warp processes the whole row on its own (only warp-level synchronisation).
-// COOP = true: the four warps of the block share the row - the keys of the q.k table, then the row's chunks dealt
+// COOP = true: the warps of the block share the row - the keys of the q.k table, then the row's chunks dealt
 // round-robin, every warp with its own accumulators; the partial histograms meet in shared memory and every thread
 // finishes one output channel.  Returns false if the row must be left over.
 template <int NT, bool COOP, bool PSI>
 __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT, PSI> &sm, const int4 r0, const int4 r1, int warp, int lane)
 {
     constexpr int CJ_LD = SortedSmem<NT, PSI>::CJ_LD;
+    constexpr int SR_WARPS = sorted_warps(NT), SR_THREADS = 32 * SR_WARPS;
     const int g = lane >> 2, t = lane & 3;
     auto sync = [&]() {
         if (COOP) __syncthreads(); else __syncwarp();
@@ -346,13 +350,21 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
     }
     sync();
     if (COOP) {
-        // ---- the four partial tables are added in a fixed order; one output channel per thread
-        const int tid = 32 * warp + lane;
-        for (int idx = tid; idx < (PSI ? 8 * PSI_LD : 0); idx += SR_THREADS)
-            sm.psi[0][idx] = (sm.psi[0][idx] + sm.psi[1][idx]) + (sm.psi[2][idx] + sm.psi[3][idx]);
-        for (int idx = tid; idx < 8 * CJ_LD; idx += SR_THREADS)
-            sm.pj[0][idx] = (sm.pj[0][idx] + sm.pj[1][idx]) + (sm.pj[2][idx] + sm.pj[3][idx]);
+        // ---- the warps' partial tables are added in a fixed order; one output channel per thread (of the first four warps)
+        for (int idx = 32 * warp + lane; idx < (PSI ? 8 * PSI_LD : 0); idx += SR_THREADS) {
+            float sum = sm.psi[0][idx];
+#pragma unroll
+            for (int w = 1; w < SR_WARPS; ++w) sum += sm.psi[w][idx];
+            sm.psi[0][idx] = sum;
+        }
+        for (int idx = 32 * warp + lane; idx < 8 * CJ_LD; idx += SR_THREADS) {
+            float sum = sm.pj[0][idx];
+#pragma unroll
+            for (int w = 1; w < SR_WARPS; ++w) sum += sm.pj[w][idx];
+            sm.pj[0][idx] = sum;
+        }
         __syncthreads();
+        const int tid = (32 * warp + lane) & (CHANNELS - 1);
         const int h = tid >> 4;
         const float *pg = sm.pj[0] + h * CJ_LD;
         const float *vp = p.v + (size_t)a0 * CHANNELS + tid;
@@ -380,9 +392,9 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
             o0 = fmaf(sm.wt[(k4 + 2) * CHANNELS + tid], pv.z, o0);
             o1 = fmaf(sm.wt[(k4 + 3) * CHANNELS + tid], pv.w, o1);
         }
-        p.out[(size_t)i * CHANNELS + tid] = (acc + (o0 + o1)) * __frcp_rn(S);
+        if (32 * warp < CHANNELS) p.out[(size_t)i * CHANNELS + tid] = (acc + (o0 + o1)) * __frcp_rn(S);
         const float M_h = __shfl_sync(FULL, M_g, 4 * (h & 7));  // (every warp holds the same bounds: head g in lanes 4 g ..)
-        if ((tid & 15) == 0) p.lse[(size_t)i * HEADS + h] = (M_h + log2f(S)) * LN2;
+        if ((tid & 15) == 0 && 32 * warp < CHANNELS) p.lse[(size_t)i * HEADS + h] = (M_h + log2f(S)) * LN2;
         return true;
     } else {
         // ---- sum_j P_g[j] v_j and S_g = sum_j P_g[j]: lane l owns channels 4 l .. 4 l + 3 (head g)
@@ -433,15 +445,16 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
 // compute a row has no influence on which terms are summed, and the choice between the two organisations depends on
 // the row's list alone, so results are repeatable bit for bit.
 template <int NT, bool PSI>
-__global__ void __launch_bounds__(SR_THREADS, NT > 2 ? 3 : 4) infinite_attn_sorted_rows_kernel(const SortedRowArgs p)
+__global__ void __launch_bounds__(32 * sorted_warps(NT), sorted_blocks(NT)) infinite_attn_sorted_rows_kernel(const SortedRowArgs p)
 {
     extern __shared__ __align__(16) unsigned char sorted_smem_raw[];
     SortedSmem<NT, PSI> &sm = *reinterpret_cast<SortedSmem<NT, PSI> *>(sorted_smem_raw);
+    constexpr int SR_WARPS = sorted_warps(NT);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     grid_launch_dependents();
     // W (8,16,64) -> wt[k][channel]: thread = channel, 256 contiguous bytes read, 64 conflict-free stores (W is a
     // constant: in a chained launch this runs while the kernel before this one drains)
-    if (PSI) {
+    if (PSI && tid < CHANNELS) {
         const float4 *src = reinterpret_cast<const float4 *>(p.W + (size_t)tid * 64);
 #pragma unroll 4
         for (int k4 = 0; k4 < 16; ++k4) {
@@ -523,9 +536,9 @@ int launch_sorted_rows(const SortedRowLaunch &l, cudaStream_t s)
         }
         done = true;
     }
-    const long long cap = (long long)sm_count() * (l.max_atoms > 32 ? 3 : 4);
+    const long long cap = (long long)sm_count() * sorted_blocks(l.max_atoms > 32 ? 4 : 2);
     const unsigned blocks = (unsigned)(l.N < cap ? l.N : cap);
-    launch_chained(kernel, dim3(blocks), dim3(SR_THREADS), smem, s, l.chained, p);
+    launch_chained(kernel, dim3(blocks), dim3(32 * sorted_warps(l.max_atoms > 32 ? 4 : 2)), smem, s, l.chained, p);
     return launch_status("infinite_attn_sorted_rows_kernel");
 }
 

@@ -320,7 +320,7 @@ extern "C" int cf_row_list_build(const float *pos_ij, const float *tvecs, const 
     b.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     b.a_widest = (float)a_widest;
     b.window = term_window(weight_floor_log2(), (float)a_widest);
-    b.coop_chunks = ROW_COOP_CHUNKS;
+    b.coop_chunks = row_coop_chunks(b.N);
     b.out = row_list_carve(workspace, N, E);
     return launch_row_list_build(b, as_stream(stream));
 }

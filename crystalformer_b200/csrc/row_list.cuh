@@ -51,7 +51,16 @@ struct RowListView {
     long long capacity;  // entries
 };
 
-constexpr int ROW_COOP_CHUNKS = 64;  // rows listing more chunks than this are shared by the warps of a block
+// Rows that list more chunks than this are shared by the warps of a block: a row of its own warp should not outlast the
+// rest of the launch.  With a row or less per warp in flight (about sixteen warps of an SM) that is from 64 chunks on; the
+// more rows every warp gets, the longer one of them may take, and rows that a block shares cost a barrier per phase: with
+// 31,000 rows sharing from 64 chunks on took 620 us per call, this rule 442.
+constexpr int ROW_COOP_CHUNKS = 64;
+inline int row_coop_chunks(long long N)
+{
+    const long long rows_per_warp_2 = N / (32ll * sm_count());  // half the rows of a warp
+    return ROW_COOP_CHUNKS * (int)(rows_per_warp_2 < 1 ? 1 : rows_per_warp_2 > 16 ? 16 : rows_per_warp_2);
+}
 
 struct RowListBuild {
     const float *pos_ij, *tvecs, *rvlen;
