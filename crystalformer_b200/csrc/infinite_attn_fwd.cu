@@ -76,6 +76,8 @@ __host__ __device__ inline size_t row_group_floats(int max_atoms, bool with_basi
            (max_atoms <= 32 ? 32 * KV_LD + 128 : 0);  // batches of small crystals: a tile for the row's k, then v, rows
                                                       // and the row's query
 }
+// ... and behind them, in the variant that enumerates phi: phi of the row's keys
+__host__ __device__ inline size_t enum_phi_floats(int max_atoms) { return (size_t)max_atoms * HEADS; }
 
 // phi of one edge by enumeration, for the rare edge whose row has no term list or whose listed terms miss a head's
 // box when the row kernel computes phi itself; kept out of line so that the row kernel's registers do not pay for it.
@@ -92,6 +94,23 @@ __device__ __noinline__ void edge_phi_enumerated(const BoxRule rule, const float
     for (int h = 0; h < 8; ++h) z_out[h] = z[h];
 }
 
+// The same for the rows that enumerate phi as a matter of course: TPE consecutive lanes per edge (the whole warp calls).  A
+// thread per edge left most of a block's threads idle through the longest phase of such a row.
+template <int TPE>
+__device__ __noinline__ void edge_phi_by_lanes(const BoxRule rule, const float *a_row, const float *rvlen3, const float *tvecs9,
+                                               const float *pos3, float floor_log2, float *z_out)
+{
+    float a[8], z[8];
+#pragma unroll
+    for (int h = 0; h < 8; ++h) a[h] = a_row[h];
+    Cell cell;
+    cell.load(tvecs9);
+    edge_phi<TPE>(rule, a, rvlen3, cell, pos3[0], pos3[1], pos3[2], floor_log2, (int)(threadIdx.x % TPE), z);
+    if (threadIdx.x % TPE == 0)
+#pragma unroll
+        for (int h = 0; h < 8; ++h) z_out[h] = z[h];
+}
+
 // ROW_WARPS = 4: one thread block per atom (large crystals: the four warps split the translations).
 // ROW_WARPS = 1: one warp per atom, four atoms per thread block (small crystals: a row is a few thousand terms and
 //                its cost is dominated by the latency of its phases, so four rows progress independently per block
@@ -100,7 +119,7 @@ __device__ __noinline__ void edge_phi_enumerated(const BoxRule rule, const float
 // or more than 32 keys): phi of every edge is enumerated inside the row (a variant of its own, so that the ordinary
 // instantiations carry none of its code or registers).
 template <int K, int ROW_WARPS, bool ENUM_PHI = false>
-__global__ void __launch_bounds__(THREADS, ENUM_PHI ? 2 : (K == 0 ? 6 : (ROW_WARPS == 1 ? 3 : 4))) infinite_attn_rows_kernel(const RowArgs p)
+__global__ void __launch_bounds__(THREADS, ENUM_PHI ? 3 : (K == 0 ? 6 : (ROW_WARPS == 1 ? 3 : 4))) infinite_attn_rows_kernel(const RowArgs p)
 {
     extern __shared__ __align__(16) float smem_all[];
     constexpr int GROUPS = WARPS / ROW_WARPS;        // row groups per block
@@ -118,7 +137,9 @@ __global__ void __launch_bounds__(THREADS, ENUM_PHI ? 2 : (K == 0 ? 6 : (ROW_WAR
         else
             asm volatile("bar.sync 2, %0;" ::"n"(32 * ROW_WARPS) : "memory");
     };
-    float *smem = smem_all + (size_t)group * row_group_floats(p.max_atoms, K > 0, ROW_WARPS);
+    const size_t group_floats = row_group_floats(p.max_atoms, K > 0, ROW_WARPS);
+    float *smem = smem_all + (size_t)group * (group_floats + (ENUM_PHI ? enum_phi_floats(p.max_atoms) : 0));
+    float *phis = smem + group_floats;  // [max_atoms][8], ENUM_PHI only
     float4 *rel = reinterpret_cast<float4 *>(smem);                    // [max_atoms]
     // per-key tables are head-major with a leading dimension = 1 (mod 32): lanes over keys and lanes over heads both
     // fall into distinct banks
@@ -201,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, ENUM_PHI ? 2 : (K == 0 ? 6 : (ROW_WAR
         // read its entries sub, sub + ROW_WARPS, ... and combine by a fixed butterfly; lane 0 of the key stores the eight
         // values at dst.  Every thread of the group calls it (keys beyond the row just take part in the shuffles).  The
         // rare edge without a list, or whose listed terms miss a head's box, is enumerated out of line.
-        const bool phi_here = K > 0 && p.phi_in_row != 0;
+        const bool phi_here = K > 0 && !ENUM_PHI && p.phi_in_row != 0;
         auto phi_from_lists = [&](int jk, float *dst) {
             float a8[8], a2p[8];
             int pkp[8];
@@ -257,6 +278,20 @@ __global__ void __launch_bounds__(THREADS, ENUM_PHI ? 2 : (K == 0 ? 6 : (ROW_WAR
             }
         };
 
+        if (ENUM_PHI && n > 0) {
+            // ---- phi of every key by enumeration, as many lanes per key as the row group has (a power of two up to 8)
+            const float *rv = p.rvlen ? p.rvlen + 3 * c : nullptr;
+            auto enumerate = [&](auto fn, int tpe) {
+                for (int j0 = 0; j0 < n; j0 += RT / tpe) {
+                    const int j = j0 + rt / tpe, jc = min(j, n - 1);  // (a repeated last key writes the same values)
+                    fn(p.rule, p.a + i * HEADS, rv, p.tvecs + 9 * c, p.pos_ij + 3 * (e0 + jc), p.basis.floor_log2, phis + 8 * jc);
+                }
+            };
+            if (8 * n <= RT) enumerate(edge_phi_by_lanes<8>, 8);
+            else if (4 * n <= RT) enumerate(edge_phi_by_lanes<4>, 4);
+            else enumerate(edge_phi_by_lanes<2>, 2);
+            row_sync();
+        }
         if (n <= 32) {
             // ---- up to 32 keys: the soft-max in registers, one key per lane, the heads split over the warps of the group
             //      (logits, statistics by shuffles).
@@ -287,14 +322,8 @@ __global__ void __launch_bounds__(THREADS, ENUM_PHI ? 2 : (K == 0 ? 6 : (ROW_WAR
                         rx = __fsub_rn(pp[0], pi[0]); ry = __fsub_rn(pp[1], pi[1]); rz = __fsub_rn(pp[2], pi[2]);
                     }
                 }
-                // phi: left in shared memory by the phase above, or in the logit array by the phi kernel, or - a left-over
-                // row without a basis, for which neither ran - enumerated here
-                __align__(16) float enumerated[8];
-                const bool phi_enum = ENUM_PHI && p.phi_in_row != 0 && !phi_here;
-                if (phi_enum)
-                    edge_phi_enumerated(p.rule, p.a + i * HEADS, p.rvlen ? p.rvlen + 3 * c : nullptr, p.tvecs + 9 * c,
-                                        p.pos_ij + 3 * (e0 + lane), p.basis.floor_log2, enumerated);
-                const float *src = (phi_enum ? enumerated : phi_here ? part + 8 * lane : logit_io + (e0 + lane) * HEADS) + h0;
+                // phi: left in shared memory by a phase above, or in the logit array by the phi kernel
+                const float *src = (ENUM_PHI ? phis + 8 * lane : phi_here ? part + 8 * lane : logit_io + (e0 + lane) * HEADS) + h0;
                 if (HPW == 8) {
                     const float4 v0 = reinterpret_cast<const float4 *>(src)[0], v1 = reinterpret_cast<const float4 *>(src)[1];
                     phi[0] = v0.x; phi[1] = v0.y; phi[2] = v0.z; phi[3] = v0.w;
@@ -397,11 +426,9 @@ __global__ void __launch_bounds__(THREADS, ENUM_PHI ? 2 : (K == 0 ? 6 : (ROW_WAR
                 const float4 *kp = reinterpret_cast<const float4 *>(kmat + (a0 + j) * HEADS * HEAD_DIM);
                 float4 *lp = reinterpret_cast<float4 *>(logit_io + (e0 + j) * HEADS);  // phi was left here by the phi kernel
                 float phi[8];
-                if (ENUM_PHI && p.phi_in_row != 0) {  // (a left-over row: no phi kernel ran)
-                    edge_phi_enumerated(p.rule, p.a + i * HEADS, p.rvlen ? p.rvlen + 3 * c : nullptr, p.tvecs + 9 * c,
-                                        p.pos_ij + 3 * (e0 + j), p.basis.floor_log2, phi);
-                } else {
-                    const float4 ph0 = lp[0], ph1 = lp[1];
+                {
+                    const float4 *src = ENUM_PHI ? reinterpret_cast<const float4 *>(phis + 8 * j) : lp;
+                    const float4 ph0 = src[0], ph1 = src[1];
                     phi[0] = ph0.x; phi[1] = ph0.y; phi[2] = ph0.z; phi[3] = ph0.w;
                     phi[4] = ph1.x; phi[5] = ph1.y; phi[6] = ph1.z; phi[7] = ph1.w;
                 }
@@ -802,12 +829,12 @@ namespace cf {
 int launch_rows(const RowArgs &p, int64_t K, long long grid_rows, cudaStream_t s, bool chained)
 {
     const int max_atoms = p.max_atoms;
-    const int row_warps = max_atoms <= 12 ? 1 : WARPS;
+    // left-over rows of the sorted path (no lists): phi enumerated inside the row
+    const bool enum_phi = p.phi_in_row != 0 && p.list.pool == nullptr;
+    const int row_warps = max_atoms <= 12 && !(enum_phi && K > 0) ? 1 : WARPS;
     const int groups = WARPS / row_warps;
-    const size_t smem = sizeof(float) * groups * row_group_floats(max_atoms, K > 0, row_warps);
+    const size_t smem = sizeof(float) * groups * (row_group_floats(max_atoms, K > 0, row_warps) + (enum_phi ? enum_phi_floats(max_atoms) : 0));
     void (*kernel)(const RowArgs);
-    // left-over rows of the sorted path without a basis, or of more than 32 keys: phi enumerated inside the row
-    const bool enum_phi = p.phi_in_row != 0 && (K == 0 || max_atoms > 32);
     if (enum_phi)
         kernel = K > 0 ? infinite_attn_rows_kernel<64, 4, true>
                        : (row_warps == 1 ? infinite_attn_rows_kernel<0, 1, true> : infinite_attn_rows_kernel<0, 4, true>);
@@ -856,8 +883,9 @@ int launch_leftover_rows(const float *q, const float *k, const float *v, const f
     p.ticket = ticket;
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     p.basis = make_basis_params(K, dist_max, wscale, weight_floor_log2());
-    // left-over rows are rare: a grid of one block per SM draws them through the ticket
-    return launch_rows(p, K, (long long)sm_count() * (max_atoms <= 12 ? WARPS : 1), s, true);
+    // left-over rows are few: a grid of three blocks per SM draws them through the ticket (one per SM was as good without
+    // any, and 400 us together with a thread per edge for phi, instead of 216, with the 1,300 of a screening batch)
+    return launch_rows(p, K, 3ll * sm_count() * (max_atoms <= 12 && K == 0 ? WARPS : 1), s, true);
 }
 
 // The rows that the block kernel (infinite_attn_block.cu) met without a term list: phi is in the logit array already.
