@@ -119,7 +119,7 @@ __device__ __noinline__ void edge_phi_by_lanes(const BoxRule rule, const float *
 // or more than 32 keys): phi of every edge is enumerated inside the row (a variant of its own, so that the ordinary
 // instantiations carry none of its code or registers).
 template <int K, int ROW_WARPS, bool ENUM_PHI = false>
-__global__ void __launch_bounds__(THREADS, ENUM_PHI ? 3 : (K == 0 ? 6 : (ROW_WARPS == 1 ? 3 : 4))) infinite_attn_rows_kernel(const RowArgs p)
+__global__ void __launch_bounds__(THREADS, ENUM_PHI ? (K == 0 ? 3 : 4) : (K == 0 ? 6 : (ROW_WARPS == 1 ? 3 : 4))) infinite_attn_rows_kernel(const RowArgs p)
 {
     extern __shared__ __align__(16) float smem_all[];
     constexpr int GROUPS = WARPS / ROW_WARPS;        // row groups per block
@@ -884,9 +884,9 @@ int launch_leftover_rows(const float *q, const float *k, const float *v, const f
     p.ticket = ticket;
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     p.basis = make_basis_params(K, dist_max, wscale, weight_floor_log2());
-    // left-over rows are few: a grid of three blocks per SM draws them through the ticket (one per SM was as good without
-    // any, and 400 us together with a thread per edge for phi, instead of 216, with the 1,300 of a screening batch)
-    return launch_rows(p, K, 3ll * sm_count() * (max_atoms <= 12 && K == 0 ? WARPS : 1), s, true);
+    // left-over rows are few: a grid of four blocks per SM draws them through the ticket (one per SM was as good without
+    // any, and 400 us together with a thread per edge for phi, instead of 196, with the 1,300 of a screening batch)
+    return launch_rows(p, K, 4ll * sm_count() * (max_atoms <= 12 && K == 0 ? WARPS : 1), s, true);
 }
 
 // The rows that the block kernel (infinite_attn_block.cu) met without a term list: phi is in the logit array already.

@@ -10,24 +10,27 @@ constexpr int RL_THREADS = 256;
 constexpr int RL_WARPS = RL_THREADS / 32;
 constexpr int RL_BUCKETS = 2 * RL_THREADS;  // (the scan below takes two buckets per thread)
 constexpr int RL_MAX_TRANSLATIONS = 4096;  // boxes beyond this are not listed
-constexpr size_t RL_SMEM = sizeof(unsigned long long) * 2 * ROW_LIST_CAP + sizeof(int) * (2 * RL_BUCKETS + 8);
+constexpr size_t RL_SMEM = sizeof(unsigned long long) * ROW_LIST_CAP + sizeof(unsigned short) * 2 * ROW_LIST_CAP + sizeof(int) * (2 * RL_BUCKETS + 8);
 
 // One thread block per row.  Every key's candidate translations (a bounding box of the ball that holds its listed
 // terms) are walked by a warp, one per lane and step; terms within `window` of their edge's nearest image are appended to a
-// shared-memory buffer (one atomic per warp and step) as 64-bit items (d2 bits << 32 | key).  The items are then
-// sorted: distributed over RL_BUCKETS buckets that are equally spaced in d^3 (terms are about uniform in volume, so
-// buckets hold a handful of items each), and placed inside their bucket by counting the smaller items of the same
-// bucket.  The 64-bit items are distinct except for exact duplicates, so the result does not depend on the order in
-// which the atomics arrived.  Four warps per row: most of a row's cost is per thread (set-up, scans, barriers), not
-// per item.
+// shared-memory buffer (one atomic per warp and step) as 64-bit items (d2 bits << 32 | key) and counted in their bucket:
+// RL_BUCKETS buckets, equally spaced in d^3 (terms are about uniform in volume, so buckets hold a handful of items each).
+// The items' indices are then distributed over the buckets and placed inside their bucket by counting the smaller items of
+// the same bucket.  The 64-bit items are distinct except for exact duplicates, so the result does not depend on the order
+// in which the atomics arrived.  Eight warps per row: most of a row's cost is per thread (set-up, scans, barriers), not
+// per item.  Bound by latency (issue slots 40 % busy): what is moved is 16-bit indices and not the items, which makes room
+// for a fourth block per SM; 31,000 rows of 1,000 entries 0.99 -> 0.89 ms, 2,000 of 650 52 -> 47 us.
 __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowListBuild p)
 {
     extern __shared__ __align__(16) unsigned long long rl_smem[];
-    unsigned long long *ent = rl_smem, *ent2 = rl_smem + ROW_LIST_CAP;
-    int *hist = reinterpret_cast<int *>(ent2 + ROW_LIST_CAP);  // [RL_BUCKETS] counts, then running cursors
+    unsigned long long *ent = rl_smem;
+    unsigned short *placed = reinterpret_cast<unsigned short *>(ent + ROW_LIST_CAP);  // item indices by bucket
+    unsigned short *sorted = placed + ROW_LIST_CAP;                                   // item indices in order
+    int *hist = reinterpret_cast<int *>(sorted + ROW_LIST_CAP);  // [RL_BUCKETS] counts, then running cursors
     int *offs = hist + RL_BUCKETS;                             // [RL_BUCKETS] first position of every bucket
     int *wsum = offs + RL_BUCKETS;                             // [RL_WARPS]
-    __shared__ int dmin_s[ROW_LIST_MAX_KEYS];
+    __shared__ float dmin_s[ROW_LIST_MAX_KEYS];
     __shared__ float4 key_s[ROW_LIST_MAX_KEYS];                // relative position of every key, .w = its threshold
     __shared__ int cnt_s;
     __shared__ int4 kbox_s[ROW_LIST_MAX_KEYS];                 // first translation of every key's box, its widths w3 | w2 << 8
@@ -45,7 +48,6 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
         const long long a0 = n > 0 ? p.edges[p.E + e0] : i;
         __syncthreads();  // the previous row's readers are done with the shared buffers
         if (tid == 0) cnt_s = 0;
-        if (tid < ROW_LIST_MAX_KEYS) dmin_s[tid] = 0x7f800000;  // +inf
         for (int b = tid; b < RL_BUCKETS; b += RL_THREADS) hist[b] = 0;
         Cell cell;
         cell.load(p.tvecs + 9 * c);
@@ -125,6 +127,17 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
 #pragma unroll
             for (int u = 0; u < ROW_LIST_MAX_KEYS / 32; ++u) d2_max = fmaxf(d2_max, d2max_s[u]);
         }
+        // ---- bucket of an item: about floor(RL_BUCKETS (d / d_max)^3) - terms are roughly uniform in volume, so such
+        //      buckets fill evenly - with x^1.5 replaced by x (0.35 + 0.65 x), x = d2 / d2_max: within a few
+        //      percent of it on [0, 1] and, evaluated as below, non-decreasing in d2 float by float (products and
+        //      fused multiply-adds of non-negative non-decreasing factors round monotonically), which is all the
+        //      sort needs: the final order is that of the items themselves whatever the partition into buckets
+        const float inv_d2max = 1.0f / d2_max;
+        auto bucket_of = [&](float d2) {
+            const float x = d2 * inv_d2max;
+            return min(RL_BUCKETS - 1, (int)(x * fmaf(0.65f, x, 0.35f) * ((float)RL_BUCKETS * 0.999f)));
+        };
+        auto d2_of = [](unsigned long long item) { return __uint_as_float((unsigned)(item >> 32)); };
         if (fits) {
             // a warp takes a key at a time, its lanes the translations of the key's box (32 per pass)
             for (int j = wr; j < n; j += RL_WARPS) {
@@ -133,6 +146,7 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
                 const int count = kcnt_s[j];
                 const int w3 = kb.w & 255, w2 = kb.w >> 8;
                 const float inv_w3 = __frcp_rn((float)w3), inv_w2 = __frcp_rn((float)w2);
+                float nearest = INFINITY;
                 for (int tr0 = 0; tr0 < count; tr0 += 32) {  // (warp-uniform bounds: the ballots below are safe)
                     const int tr = tr0 + lane;
                     // digits of tr in the mixed radix (w1, w2, w3): quotients by a rounded-down product with the
@@ -147,6 +161,7 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
                     const float dz = fmaf(cell.t3z, f3, fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, r.z)));
                     const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
                     const bool keep = tr < count && d2 <= r.w;
+                    if (keep) nearest = fminf(nearest, d2);
                     const unsigned mask = __ballot_sync(FULL, keep);
                     if (mask == 0u) continue;
                     int base = 0;
@@ -155,9 +170,14 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
                     if (keep) {
                         const int at = base + __popc(mask & lt);
                         const int key123 = (abs(n1) << 8) | (abs(n2) << 16) | (abs(n3) << 24);
-                        if (at < ROW_LIST_CAP) ent[at] = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)(key123 | j);
+                        if (at < ROW_LIST_CAP) {
+                            ent[at] = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)(key123 | j);
+                            atomicAdd(&hist[bucket_of(d2)], 1);
+                        }
                     }
                 }
+                nearest = warp_min(nearest);
+                if (lane == 0) dmin_s[j] = nearest;  // smallest listed d2 of the key
             }
         }
         __syncthreads();
@@ -165,18 +185,6 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
         const bool sortable = fits && total >= 1 && total <= ROW_LIST_CAP;
         const int chunks = (total + 7) >> 3, out_total = chunks << 3;
         if (sortable) {
-            // ---- bucket of an item: about floor(RL_BUCKETS (d / d_max)^3) - terms are roughly uniform in volume, so such
-            //      buckets fill evenly - with x^1.5 replaced by x (0.35 + 0.65 x), x = d2 / d2_max: within a few
-            //      percent of it on [0, 1] and, evaluated as below, non-decreasing in d2 float by float (products and
-            //      fused multiply-adds of non-negative non-decreasing factors round monotonically), which is all the
-            //      sort needs: the final order is that of the items themselves whatever the partition into buckets
-            const float inv_d2max = 1.0f / d2_max;
-            auto bucket_of = [&](unsigned long long item) {
-                const float x = __uint_as_float((unsigned)(item >> 32)) * inv_d2max;
-                return min(RL_BUCKETS - 1, (int)(x * fmaf(0.65f, x, 0.35f) * ((float)RL_BUCKETS * 0.999f)));
-            };
-            for (int t = tid; t < total; t += RL_THREADS) atomicAdd(&hist[bucket_of(ent[t])], 1);
-            __syncthreads();
             // exclusive scan of the counts (two buckets per thread)
             {
                 const int v0 = hist[2 * tid], v1 = hist[2 * tid + 1];
@@ -195,24 +203,20 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
                 hist[2 * tid] = excl; hist[2 * tid + 1] = excl + v0;  // running cursors of the scatter
             }
             __syncthreads();
-            for (int t = tid; t < total; t += RL_THREADS) {
-                const unsigned long long item = ent[t];
-                ent2[atomicAdd(&hist[bucket_of(item)], 1)] = item;
-            }
+            for (int t = tid; t < total; t += RL_THREADS) placed[atomicAdd(&hist[bucket_of(d2_of(ent[t]))], 1)] = (unsigned short)t;
             __syncthreads();
             // an item's place inside its bucket = the number of smaller items there (equal items: by position)
             for (int t = tid; t < total; t += RL_THREADS) {
-                const unsigned long long item = ent2[t];
-                const int b = bucket_of(item);
+                const int mine = placed[t];
+                const unsigned long long item = ent[mine];
+                const int b = bucket_of(d2_of(item));
                 const int lo = offs[b], hi = hist[b];  // (after the scatter the cursor of a bucket is its end)
                 int rank = 0;
                 for (int u = lo; u < hi; ++u) {
-                    const unsigned long long other = ent2[u];
+                    const unsigned long long other = ent[placed[u]];
                     rank += (other < item || (other == item && u < t)) ? 1 : 0;
                 }
-                ent[lo + rank] = item;
-                // smallest listed d2 of the item's key (d2 >= 0: the bit patterns order like the values)
-                atomicMin(&dmin_s[(int)(item & 255u)], (int)(item >> 32));
+                sorted[lo + rank] = (unsigned short)mine;
             }
             if (tid == 0) {
                 const unsigned long long at = atomicAdd(p.out.cursor, (unsigned long long)out_total);
@@ -226,13 +230,13 @@ __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowLis
         }
         const long long base = base_s;
         if (base >= 0) {
-            const unsigned last_d2 = (unsigned)(ent[total - 1] >> 32);
+            const unsigned last_d2 = (unsigned)(ent[sorted[total - 1]] >> 32);
             for (int t = tid; t < out_total; t += RL_THREADS) {
-                const unsigned long long v = ent[t < total ? t : 0];
+                const unsigned long long v = ent[sorted[t < total ? t : 0]];
                 p.out.pool[base + t] = t < total ? make_float2(__uint_as_float((unsigned)(v >> 32)), __uint_as_float((unsigned)v))
                                                  : make_float2(__uint_as_float(last_d2), __int_as_float(ROW_PAD_KEY));
             }
-            if (tid < n) p.out.dmin[e0 + tid] = __int_as_float(dmin_s[tid]);
+            if (tid < n) p.out.dmin[e0 + tid] = dmin_s[tid];
         }
         if (tid == 0) {
             p.out.rowdir[2 * slot] = make_int4((int)i, (int)a0, n, (int)c);
@@ -288,7 +292,7 @@ int launch_row_list_build(const RowListBuild &b, cudaStream_t s)
         }
         configured[dev & 63] = true;
     }
-    const long long cap = (long long)sm_count() * 3;
+    const long long cap = (long long)sm_count() * 4;
     row_list_build_kernel<<<(unsigned)(b.N < cap ? b.N : cap), RL_THREADS, RL_SMEM, s>>>(b);
     return launch_status("row_list_build_kernel");
 }
