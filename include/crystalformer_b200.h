@@ -14,7 +14,9 @@
  *     failure on the calling thread.
  * State kept by the library: the process-wide switches (cf_set_weight_floor_log2, cf_set_sorted_rows,
  * cf_set_chained_launches, cf_set_row_stats), a
- * side stream and two events per (host thread, device) created by the first cf_encoder_forward / cf_model_forward,
+ * side stream and three events per (host thread, device) created by the first cf_encoder_forward / cf_model_forward
+ * / cf_model_begin / cf_train_begin, a pinned staging buffer of at most 8 MiB per host thread for the sizes that the
+ * begin calls read back,
  * the 8 MiB scratch array of cf_lattice_sum_bwd_static, and a pool of row tickets per device: 64 single counters
  * handed round-robin to the cf_infinite_attn_fwd[_listed] calls with K > 0 and 8 blocks of 16 handed round-robin to the
  * one-call forwards that use term lists.  A ticket is reused after 64 calls (8 forwards): at most that many such calls
