@@ -884,9 +884,11 @@ int launch_leftover_rows(const float *q, const float *k, const float *v, const f
     p.ticket = ticket;
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     p.basis = make_basis_params(K, dist_max, wscale, weight_floor_log2());
-    // left-over rows are few: a grid of four blocks per SM draws them through the ticket (one per SM was as good without
-    // any, and 400 us together with a thread per edge for phi, instead of 196, with the 1,300 of a screening batch)
-    return launch_rows(p, K, 4ll * sm_count() * (max_atoms <= 12 && K == 0 ? WARPS : 1), s, true);
+    // left-over rows are few and drawn through the ticket: a block for every eighth row of the batch, at least one and at
+    // most four per SM (with the 1,300 of a screening batch one per SM took, together with a thread per edge for phi,
+    // 400 us instead of 196; a small batch has none as a rule, and each block of the grid costs its launch)
+    const long long sms = sm_count(), blocks = N / 8 < sms ? sms : N / 8 > 4 * sms ? 4 * sms : N / 8;
+    return launch_rows(p, K, blocks * (max_atoms <= 12 && K == 0 ? WARPS : 1), s, true);
 }
 
 // The rows that the block kernel (infinite_attn_block.cu) met without a term list: phi is in the logit array already.

@@ -297,10 +297,11 @@ constexpr int RING_ENTRIES = 256;  // >= 31 left over + 4 x 32 offered + slack, 
 constexpr int RING_FLOATS = 2 * RING_ENTRIES;
 
 __device__ __forceinline__ int pack_key(int j, int i1, int i2, int i3) { return j | (i1 << 11) | (i2 << 17) | (i3 << 23); }
-__device__ __forceinline__ bool key_in_box(int key, int pk)
-{
-    return ((key >> 11) & 63) <= box_r1(pk) && ((key >> 17) & 63) <= box_r2(pk) && ((key >> 23) & 63) <= box_r3(pk);
-}
+// The |n| of a key as bytes, for tests against several boxes; bytes_in_box: 128 + R - |n| keeps a byte's top bit exactly when
+// |n| <= R (|n| <= 63: no borrow).
+__device__ __forceinline__ int key_bytes(int key) { return ((key >> 11) & 63) | (((key >> 17) & 63) << 8) | (((key >> 23) & 63) << 16); }
+__device__ __forceinline__ bool bytes_in_box(int bytes, int pk) { return (((pk | 0x808080) - bytes) & 0x808080) == 0x808080; }
+__device__ __forceinline__ bool key_in_box(int key, int pk) { return bytes_in_box(key_bytes(key), pk); }
 
 template <int ENTRIES>
 struct CandidateRingOf {

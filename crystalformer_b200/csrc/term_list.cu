@@ -192,20 +192,29 @@ __global__ void __launch_bounds__(128) phi_from_list_kernel(const PhiListArgs p)
     const float m = first >= 0 ? p.list.dmin[e] : 0.f;
     const float2 *ent = p.list.pool + (first >= 0 ? first : 0);
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    // entries are requested two steps ahead of their use: the lists stream from memory, and a step is short
-    float2 n0 = make_float2(0.f, 0.f), n1 = n0;
-    if (sub < cnt) n0 = __ldg(ent + sub);
-    if (sub + TPE < cnt) n1 = __ldg(ent + sub + TPE);
-    for (int t = sub; t < cnt; t += TPE) {
-        const float2 en = n0;
-        n0 = n1;
-        if (t + 2 * TPE < cnt) n1 = __ldg(ent + t + 2 * TPE);
-        const float rel = en.x - m;
-        if (a2max * rel < p.floor_log2) continue;  // below the floor for every head
-        const int key = __float_as_int(en.y);
+    // four entries per step, the next four requested meanwhile: the lists stream from memory, and a step is short
+    const float2 none = make_float2(INFINITY, 0.f);
+    float2 nx[4];
 #pragma unroll
-        for (int h = 0; h < 8; ++h)
-            if (key_in_box(key, pk[h])) s[h] += ex2(a2[h] * rel);
+    for (int u = 0; u < 4; ++u) nx[u] = sub + u * TPE < cnt ? __ldg(ent + sub + u * TPE) : none;
+    for (int t = sub; t < cnt; t += 4 * TPE) {
+        float2 en[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            en[u] = nx[u];
+            nx[u] = t + (4 + u) * TPE < cnt ? __ldg(ent + t + (4 + u) * TPE) : none;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float rel = en[u].x - m;
+            if (a2max * rel < p.floor_log2) continue;  // below the floor for every head (or no entry)
+            const int bytes = key_bytes(__float_as_int(en[u].y));
+#pragma unroll
+            for (int h = 0; h < 8; ++h) {
+                const float w = ex2(a2[h] * rel);
+                s[h] += bytes_in_box(bytes, pk[h]) ? w : 0.f;
+            }
+        }
     }
     bool done = cnt > 0;
 #pragma unroll
