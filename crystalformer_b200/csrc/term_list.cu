@@ -274,9 +274,10 @@ int launch_term_list_build(const TermListBuild &b, cudaStream_t s)
 int launch_phi_from_list(const PhiListArgs &p, cudaStream_t s)
 {
     if (p.E == 0) return CF_OK;
-    // lanes per edge: as many as keep the grid at a few waves of the SMs
+    // lanes per edge: as many as keep the grid at about a wave's threads (a wave costs its loads of edge, atom, crystal and
+    // widths, about 3 us, whatever the lists hold: 141,000 edges took 45 us per call with eight lanes, 31 with two)
     const long long per_wave = (long long)sm_count() * 2048;
-    const int tpe = p.E * 8 <= 4 * per_wave ? 8 : (p.E * 4 <= 4 * per_wave ? 4 : (p.E * 2 <= 4 * per_wave ? 2 : 1));
+    const int tpe = p.E * 8 <= per_wave ? 8 : (p.E * 4 <= per_wave ? 4 : (p.E * 2 <= per_wave ? 2 : 1));
     const unsigned blocks = (unsigned)((p.E * tpe + 127) / 128);
     switch (tpe) {
         case 8: phi_from_list_kernel<8><<<blocks, 128, 0, s>>>(p); break;
