@@ -404,7 +404,9 @@ def run_b200(args):
         y_direct = model(resident, counts=(n_atoms, n_edges, max_atoms), **({} if peers is None else {"gather": peers}))
     if peers is not None:
         peers.wait_ready()
-    e2e_equal = bool(torch.equal(y_served, y_direct.cpu()))
+    # (the served forward keeps one dense block per tile, the direct one shares a tile between four: sums in another order)
+    e2e_difference = float((y_served - y_direct.cpu()).abs().max() / y_direct.abs().max())
+    e2e_equal = e2e_difference < 2e-6
     # ---- the same stream with the species as indices (z: the position of the 1 in every one-hot row of x), the
     #      predictor's compact input: 8 bytes per atom go to the device instead of 4 x 98; a shorter run, reported beside
     #      the figure above, which uses the reference's input format
@@ -497,7 +499,7 @@ def run_b200(args):
                     "host_issue_ms_per_step": e2e_issue * 1e3 / e2e_steps,
                     "clock": "host wall clock (perf_counter) from the first submit to the last result of one uninterrupted "
                              "stream of timed_steps batches (pipeline fill and drain inside the clock), max over ranks",
-                    "outputs_equal_direct_forward": e2e_equal,
+                    "outputs_equal_direct_forward": e2e_equal, "outputs_max_rel_difference": e2e_difference,
                     "api": f"crystalformer_b200.serving.PipelinedPredictor, {e2e_depth} batches in flight on {e2e_streams} compute stream(s)"},
             "e2e_species_indices": e2e_z,
             "gpu_launches": None if launches is None else launches * args.steps,
@@ -557,14 +559,14 @@ def attention_roofline(ops, device, model, step, wl, n_atoms, n_edges, max_atoms
         finally:
             ops.set_row_stats(None)
         chunks, tiles, rows = (int(v) / layers for v in words[:3].tolist())
-        # per lane and chunk: 2 ex2 (weights) + 2 rsqrt; per (chunk, tile): 4 ex2 (basis values).  FP32-pipe: about 18
-        # per chunk (exponents, basis coordinates, operand splits) and 20 per (chunk, tile).
-        sfu_ops = 32 * (4 * chunks + 4 * tiles)
+        # per lane and chunk: 2 ex2 (weights), and a quarter of an rsqrt; per (chunk, tile): 4 ex2 (basis values).  FP32-pipe:
+        # about 18 per chunk (exponents, basis coordinates, operand splits) and 20 per (chunk, tile).
+        sfu_ops = 32 * (2.25 * chunks + 4 * tiles)
         fp32_ops = 32 * (18 * chunks + 20 * tiles)
         t_sfu, t_fp32 = sfu_ops / nominal["sfu"], fp32_ops / nominal["fp32"]
         executed = {"chunks_per_call": chunks, "bin_tiles_per_call": tiles, "rows_per_call": rows,
                     "entries_per_call": 8 * chunks, "sfu_lane_ops": sfu_ops, "fp32_lane_instr": fp32_ops,
-                    "mma_m16n8k8_per_call": 4 * chunks + 3 * tiles,
+                    "mma_m16n8k16_per_call": (4 * chunks + 3 * tiles) / 2,
                     "sfu_frac": t_sfu / t_call, "fp32_frac": t_fp32 / t_call,
                     "sfu_frac_of_probe": sfu_ops / peaks["sfu"] / t_call}
         # bytes the call has to move at least: the list entries it sweeps, the row directory and per-edge minima, and
@@ -822,11 +824,12 @@ def train_step_case(ops, device, crystals=None):
     return {"case": "train", "workload": "cfg3", "metric": "training step (fwd + bwd, L1 loss)", "crystals": cb.num_crystals,
             "atoms": cb.num_atoms, "edges": cb.num_edges,
             "ms_per_step": ms, "crystals_per_s": cb.num_crystals / (ms * 1e-3), "host_issue_ms": host * 1e3 / reps,
-            "attention_fwd_us": per["fwd"] * 1e3, "attention_bwd_us": per["bwd"] * 1e3,
+            "attention_fwd_us": per["fwd"] * 1e3 if events["fwd"] else None, "attention_bwd_us": per["bwd"] * 1e3 if events["bwd"] else None,
             "attention_calls_per_step": len(events["fwd"]) // 3, "loss": float(loss.item()),
             "timing": "20 steps back to back between one CUDA-event pair (no L2 flush: the step's working set of "
                       "activations exceeds what survives between uses anyway)",
-            "note": "term lists built once per step inside the first forward call; the rest of the step is torch autograd"}
+            "note": "the whole step is two library calls behind one autograd node; attention_*_us only where the step goes through "
+                    "the operators (autograd path)"}
 
 
 def lattice_microbench(ops, device, peaks, pairs=250000):
@@ -868,7 +871,7 @@ def lattice_microbench(ops, device, peaks, pairs=250000):
                     "over the enumeration, not a pipe utilisation (ncu: XU 37 %, ALU 43 %, FMA 22 % of peak, "
                     "profiles/ncu_full_lattice_psi_microbench80k.md)",
             "hbm_gbs": out_bytes / t / 1e9, "hbm_frac": out_bytes / t / 6558.7e9,
-            "kernels": "lattice_phi_kernel + lattice_psi_kernel", "l2": "output 520 MB per launch exceeds L2"}
+            "kernels": "lattice_edge_kernel", "l2": "output 520 MB per launch exceeds L2"}
 
 
 def cpu_baseline(model, params, cb, seconds_budget=10.0):
