@@ -36,7 +36,7 @@ __device__ __forceinline__ void digit_range(float rho, float len, float s, int R
     hi = (int)floorf(fminf(m - s, (float)R));
 }
 
-// One warp per row, one key per lane: threshold, box and terms of a key are its lane's own work (two walks of the box, to
+// One warp per row, one key per lane (rows of few keys: several lanes, which deal the columns of the key's box): threshold, box and terms of a key are its lane's own work (two walks of the box, to
 // count and to fill), the offsets of a chunk of 32 keys come from a scan over the lanes.  A box holds about twice the
 // listed terms, whatever the cell: the walk of the rule's box by columns that this replaces took 0.53 ms for 64 crystals
 // of 100-200 atoms (1.5 M edges, 3 terms each), this one 0.15 ms.
@@ -64,9 +64,9 @@ __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const Te
         // the lane's key: position, threshold (an upper bound of the smallest squared distance ANY head's box can contain,
         // plus the window; boxes of half-width >= 1 contain the 27 nearest translations, otherwise only n = 0 is certain),
         // and visit(d2, n1, n2, n3) for every listed term
-        auto walk_key = [&](int j, auto &&visit) {
-            const float *pp = p.pos_ij + 3 * (e0 + j);
-            const float rx = pp[0], ry = pp[1], rz = pp[2];
+        const int lanes = n > 16 ? 1 : n > 8 ? 2 : n > 4 ? 4 : n > 2 ? 8 : n > 1 ? 16 : 32;  // of a key
+        const int sub = lane & (lanes - 1), first_key = lane / lanes;
+        auto threshold = [&](float rx, float ry, float rz) {
             float m = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
             if (near27) {
                 const int q1 = min(R1, 1), q2 = min(R2, 1), q3 = min(R3, 1);
@@ -80,7 +80,9 @@ __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const Te
                             m = fminf(m, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
                         }
             }
-            const float thr = m + p.window;
+            return m + p.window;
+        };
+        auto walk_key = [&](float rx, float ry, float rz, float thr, auto &&visit) {
             int lo1 = -R1, hi1 = R1, lo2 = -R2, hi2 = R2, lo3 = -R3, hi3 = R3;
             if (dual.prune) {
                 const float rho = sqrtf(fmaxf(thr, 0.f)) * 1.0001f;
@@ -88,31 +90,46 @@ __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const Te
                 digit_range(rho, dual.l2, rx * dual.b2x + ry * dual.b2y + rz * dual.b2z, R2, lo2, hi2);
                 digit_range(rho, dual.l3, rx * dual.b3x + ry * dual.b3y + rz * dual.b3z, R3, lo3, hi3);
             }
-            for (int n1 = lo1; n1 <= hi1; ++n1)
-                for (int n2 = lo2; n2 <= hi2; ++n2) {
-                    // r + n1 t1 + n2 t2 + n3 t3, contracted like the reference's expression
-                    const float f1 = (float)n1, f2 = (float)n2;
-                    const float ex = fmaf(cell.t2x, f2, fmaf(cell.t1x, f1, rx));
-                    const float ey = fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, ry));
-                    const float ez = fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, rz));
-                    for (int n3 = lo3; n3 <= hi3; ++n3) {
-                        const float f3 = (float)n3;
-                        const float dx = fmaf(cell.t3x, f3, ex), dy = fmaf(cell.t3y, f3, ey), dz = fmaf(cell.t3z, f3, ez);
-                        const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        if (d2 <= thr) visit(d2, n1, n2, n3);
-                    }
+            const int w2 = hi2 - lo2 + 1;
+            if (w2 <= 0) return;
+            int n1 = lo1, n2 = lo2 + sub;
+            while (n2 > hi2) { n2 -= w2; ++n1; }
+            while (n1 <= hi1) {
+                // r + n1 t1 + n2 t2 + n3 t3, contracted like the reference's expression
+                const float f1 = (float)n1, f2 = (float)n2;
+                const float ex = fmaf(cell.t2x, f2, fmaf(cell.t1x, f1, rx));
+                const float ey = fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, ry));
+                const float ez = fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, rz));
+                for (int n3 = lo3; n3 <= hi3; ++n3) {
+                    const float f3 = (float)n3;
+                    const float dx = fmaf(cell.t3x, f3, ex), dy = fmaf(cell.t3y, f3, ey), dz = fmaf(cell.t3z, f3, ez);
+                    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                    if (d2 <= thr) visit(d2, n1, n2, n3);
                 }
+                n2 += lanes;
+                while (n2 > hi2) { n2 -= w2; ++n1; }
+            }
         };
-        // ---- count
-        int total = 0;
-        for (int j = lane; j < n; j += 32) {
+        // ---- count (a key's threshold waits in its dmin for the second walk)
+        int total = 0, own = 0;  // own: terms of this lane, where a key has several lanes (the row is one chunk then)
+        for (int j0 = 0; j0 < n; j0 += 32) {
+            const int j = j0 + first_key;
             int cnt = 0;
-            float dm = INFINITY;
-            walk_key(j, [&](float d2, int, int, int) { ++cnt; dm = fminf(dm, d2); });
-            p.count[e0 + j] = cnt;
-            p.dmin[e0 + j] = dm;
+            float thr = 0.f;
+            if (j < n) {
+                const float *pp = p.pos_ij + 3 * (e0 + j);
+                thr = threshold(pp[0], pp[1], pp[2]);
+                walk_key(pp[0], pp[1], pp[2], thr, [&](float, int, int, int) { ++cnt; });
+            }
+            own = cnt;
             total += cnt;
+            for (int o = 1; o < lanes; o <<= 1) cnt += __shfl_xor_sync(FULL, cnt, o);
+            if (j < n && sub == 0) {
+                p.count[e0 + j] = cnt;
+                p.dmin[e0 + j] = thr;
+            }
         }
+        __syncwarp();  // (the other lanes of a key read its threshold)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(FULL, total, o);
         long long base = 0;
@@ -128,22 +145,28 @@ __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const Te
         // ---- fill, keys ascending
         long long run = base;
         for (int j0 = 0; j0 < n; j0 += 32) {
-            const int j = j0 + lane;
-            const int cnt = j < n ? p.count[e0 + j] : 0;  // (this lane's own store)
+            const int j = j0 + first_key;
+            const int cnt = j >= n ? 0 : lanes > 1 ? own : p.count[e0 + j];  // (this lane's own store)
+            const float thr = j < n ? p.dmin[e0 + j] : 0.f;
             int incl = cnt;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int up = __shfl_up_sync(FULL, incl, o);
                 if (lane >= o) incl += up;
             }
+            float dm = INFINITY;
             if (j < n) {
                 const long long first = run + incl - cnt;
-                p.start[e0 + j] = (int)first;
+                if (sub == 0) p.start[e0 + j] = (int)first;
                 float2 *out = p.pool + first;
-                walk_key(j, [&](float d2, int n1, int n2, int n3) {
+                const float *pp = p.pos_ij + 3 * (e0 + j);
+                walk_key(pp[0], pp[1], pp[2], thr, [&](float d2, int n1, int n2, int n3) {
                     *out++ = make_float2(d2, __int_as_float(pack_key(j, abs(n1), abs(n2), abs(n3))));
+                    dm = fminf(dm, d2);
                 });
             }
+            for (int o = 1; o < lanes; o <<= 1) dm = fminf(dm, __shfl_xor_sync(FULL, dm, o));
+            if (j < n && sub == 0) p.dmin[e0 + j] = dm;
             run += __shfl_sync(FULL, incl, 31);
         }
     }
