@@ -68,17 +68,21 @@ __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const Te
         const int sub = lane & (lanes - 1), first_key = lane / lanes;
         auto threshold = [&](float rx, float ry, float rz) {
             float m = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
-            if (near27) {
-                const int q1 = min(R1, 1), q2 = min(R2, 1), q3 = min(R3, 1);
-                for (int n1 = -q1; n1 <= q1; ++n1)
-                    for (int n2 = -q2; n2 <= q2; ++n2)
-                        for (int n3 = -q3; n3 <= q3; ++n3) {
-                            const float f1 = (float)n1, f2 = (float)n2, f3 = (float)n3;
-                            const float dx = fmaf(cell.t3x, f3, fmaf(cell.t2x, f2, fmaf(cell.t1x, f1, rx)));
-                            const float dy = fmaf(cell.t3y, f3, fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, ry)));
-                            const float dz = fmaf(cell.t3z, f3, fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, rz)));
-                            m = fminf(m, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
-                        }
+            auto image = [&](float f1, float f2, float f3) {
+                const float dx = fmaf(cell.t3x, f3, fmaf(cell.t2x, f2, fmaf(cell.t1x, f1, rx)));
+                const float dy = fmaf(cell.t3y, f3, fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, ry)));
+                const float dz = fmaf(cell.t3z, f3, fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, rz)));
+                m = fminf(m, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+            };
+            if (near27 && R1 > 0 && R2 > 0 && R3 > 0) {  // (unrolled: independent terms, nine at a time)
+#pragma unroll 1
+                for (int n1 = -1; n1 <= 1; ++n1)
+#pragma unroll
+                    for (int t = 0; t < 9; ++t) image((float)n1, (float)(t / 3 - 1), (float)(t % 3 - 1));
+            } else if (near27) {
+                for (int n1 = -min(R1, 1); n1 <= min(R1, 1); ++n1)
+                    for (int n2 = -min(R2, 1); n2 <= min(R2, 1); ++n2)
+                        for (int n3 = -min(R3, 1); n3 <= min(R3, 1); ++n3) image((float)n1, (float)n2, (float)n3);
             }
             return m + p.window;
         };
@@ -100,6 +104,7 @@ __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const Te
                 const float ex = fmaf(cell.t2x, f2, fmaf(cell.t1x, f1, rx));
                 const float ey = fmaf(cell.t2y, f2, fmaf(cell.t1y, f1, ry));
                 const float ez = fmaf(cell.t2z, f2, fmaf(cell.t1z, f1, rz));
+#pragma unroll 2
                 for (int n3 = lo3; n3 <= hi3; ++n3) {
                     const float f3 = (float)n3;
                     const float dx = fmaf(cell.t3x, f3, ex), dy = fmaf(cell.t3y, f3, ey), dz = fmaf(cell.t3z, f3, ez);
