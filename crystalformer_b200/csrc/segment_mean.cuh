@@ -17,24 +17,39 @@ __device__ __forceinline__ float segment_mean_channel(const float *__restrict__ 
     else if (len > 2) {
         float part[12];
         unsigned occupied = 0;
-        const long long groups = (len + 3) / 4;
-        for (long long g = 0; g < groups; ++g) {
-            const long long r = 4 * g;
+        auto carry = [&](float val, int from) {  // (static indices: the partial sums stay in registers)
+#pragma unroll
+            for (int level = 0; level < 12; ++level) {
+                if (level < from) continue;
+                if (!(occupied & (1u << level))) {
+                    part[level] = val;
+                    occupied |= 1u << level;
+                    break;
+                }
+                val = part[level] + val;
+                occupied &= ~(1u << level);
+            }
+        };
+        long long r = 0;
+        // sixteen rows at a time: their loads are in flight together (four at a time took 22 us for crystals of 200 atoms,
+        // sixteen 14), their subtree is complete
+        for (; r + 16 <= len; r += 16) {
+            float m[16], g[4];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) m[u] = src[(r + u) * D];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) g[u] = (m[4 * u] + m[4 * u + 1]) + (m[4 * u + 2] + m[4 * u + 3]);
+            carry((g[0] + g[1]) + (g[2] + g[3]), 2);
+        }
+        for (; r < len; r += 4) {
             const float m0 = src[r * D];
             const float m1 = (r + 1 < len) ? src[(r + 1) * D] : 0.f;
             const float m2 = (r + 2 < len) ? src[(r + 2) * D] : 0.f;
             const float m3 = (r + 3 < len) ? src[(r + 3) * D] : 0.f;
-            float val = (m0 + m1) + (m2 + m3);
-            int level = 0;
-            while (occupied & (1u << level)) {
-                val = part[level] + val;
-                occupied &= ~(1u << level);
-                ++level;
-            }
-            part[level] = val;
-            occupied |= 1u << level;
+            carry((m0 + m1) + (m2 + m3), 0);
         }
         bool first = true;
+#pragma unroll
         for (int level = 0; level < 12; ++level)
             if (occupied & (1u << level)) {
                 total = first ? part[level] : part[level] + total;
