@@ -79,3 +79,22 @@ def test_step_follows_the_model():
         model.mlp[0].bias.add_(1.0)
     with pytest.raises(RuntimeError, match="in-place"):
         loss.backward()
+
+
+@pytest.mark.parametrize("bins", [0, 64])
+@pytest.mark.parametrize("sizes,lengths", [([64, 65], (8.0, 14.0)), ([200], (10.0, 20.0)), ([201, 65, 1], (10.0, 20.0)),
+                                           ([1, 2, 3, 4, 5, 8, 9, 16, 17], (3.0, 4.0)), ([33] * 40, (5.0, 11.0)),
+                                           ([30] * 320, (5.0, 11.0))])
+def test_forward_at_the_edges_of_its_dispatch(sizes, lengths, bins):
+    """The one-call forward and the training step's against the autograd path: blocks of rows (65 to 200 atoms) or not, rows of
+    few keys whose boxes are dealt over lanes, two warps per row (1,200 rows), heavy rows to one warp each (9,500 rows)."""
+    model, data, target = setup(sizes, lengths=lengths, num_layers=2, value_pe_dist_real=bins)
+    model.native = False
+    y0 = model(data).detach()
+    model.native = True
+    y1 = model(data).detach()
+    with torch.no_grad():
+        y2 = model.eval()(data)
+    scale = max(1.0, float(y0.abs().max()))
+    assert (y0 - y1).abs().max() < 2e-6 * scale
+    assert (y0 - y2).abs().max() < 2e-6 * scale
