@@ -32,7 +32,7 @@ _REF = {}
 def build(ref: bool = True) -> None:
     """Compile the oracle (and the CPU build of the reference kernels when the reference tree is present)."""
     subprocess.run(["make", "-s", "-C", _HERE], check=True)
-    if ref and os.path.isdir(os.environ.get("CF_REFERENCE_ROOT", "/root/reference")):
+    if ref and os.path.isdir(os.path.join(os.environ.get("CF_REFERENCE_ROOT", "/root/reference"), "models", "kernels")):
         subprocess.run(["make", "-s", "-C", _HERE, "ref",
                         "REFERENCE=" + os.environ.get("CF_REFERENCE_ROOT", "/root/reference")], check=True)
 
