@@ -97,6 +97,8 @@ class BatchGeometry:
         if num_atoms is None or num_edges is None or max_atoms is None:
             host = sizes.tolist()  # the one device->host read per batch (the reference does the same, :201)
             num_atoms, num_edges, max_atoms = sum(host), sum(n * n for n in host), max(host) if host else 1
+        if pos.numel() < 3 * num_atoms or trans.numel() < 9 * sizes.shape[0]:
+            raise ValueError(f"pos {tuple(pos.shape)} and trans {tuple(trans.shape)} do not hold {num_atoms} atoms in {sizes.shape[0]} crystals")
         self.atom_start, self.edge_start = ops.crystal_offsets(sizes)
         prep = ops.batch_prepare(pos.float(), trans.float(), sizes, self.atom_start, self.edge_start, num_atoms, num_edges)
         self.batch, self.edges, self.row_start = prep["batch"], prep["edges"], prep["row_start"]

@@ -39,6 +39,17 @@ def max_pool(x, batch, sizes):
     return out.scatter_reduce(0, batch[:, None].expand_as(x), x, reduce="amax", include_self=True)
 
 
+def check_batch(data, atoms: int) -> None:
+    """Raises unless the tensors of ``data`` lie on one device and hold ``atoms`` atoms and the crystals of ``sizes``: the
+    library gets their addresses and cannot see how long they are."""
+    x, pos, trans, sizes = data.x, data.pos, data.trans_vec, data.sizes
+    if x.device != pos.device or trans.device != pos.device:
+        raise RuntimeError(f"x, pos and trans_vec must be on one device, not on {x.device}, {pos.device} and {trans.device}")
+    if x.dim() != 2 or sizes.dim() != 1 or x.shape[0] < atoms or pos.numel() < 3 * atoms or trans.numel() < 9 * sizes.shape[0]:
+        raise ValueError(f"x {tuple(x.shape)}, pos {tuple(pos.shape)}, trans_vec {tuple(trans.shape)} and sizes {tuple(sizes.shape)} do not "
+                         f"hold a batch of {atoms} atoms")
+
+
 class Latticeformer(nn.Module):
     def __init__(self, params):
         super().__init__()
@@ -210,12 +221,19 @@ class Latticeformer(nn.Module):
         if plan is None:
             plan = self._current_plan(dev)
         if counts is None:
-            if "desc" in plan and plan["images"] and data.pos.shape[0] > 0 and data.sizes.device == dev \
-                    and data.sizes.dtype == torch.int64 and data.sizes.is_contiguous() and data.sizes.shape[0] > 0:
+            # (the first block reads all rows of pos and x before the sizes are known, at the width of the model)
+            if "desc" in plan and plan["images"] and data.pos.dim() == 2 and data.pos.shape[0] > 0 and data.sizes.device == dev \
+                    and data.sizes.dtype == torch.int64 and data.sizes.is_contiguous() and data.sizes.dim() == 1 \
+                    and data.sizes.shape[0] > 0 and data.x.dim() == 2 and data.x.shape[1] == plan["emb"].shape[1] \
+                    and data.x.shape[0] >= data.pos.shape[0]:
                 return self._forward_begun(data, gather, plan)
             host = data.sizes.tolist()  # the one device->host read per batch (the reference does the same)
             counts = (sum(host), sum(n * n for n in host), max(host) if host else 1)
         n_atoms, n_edges, max_atoms = (int(v) for v in counts)
+        check_batch(data, n_atoms)
+        width = plan["emb"].shape[1]  # (the packed embedding has 128 input columns, of which a narrower x uses the first)
+        if data.x.shape[1] != width and (plan["emb_packed"] is None or data.x.shape[1] > 128):
+            raise ValueError(f"x has {data.x.shape[1]} columns, the model embeds {width}")
         f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()
         feats, pos, trans = f32(data.x), f32(data.pos), f32(data.trans_vec)
         sizes = data.sizes
@@ -254,6 +272,7 @@ class Latticeformer(nn.Module):
         """The one-call forward for sizes that only the device knows: their read-back and the first dense block are queued
         together, and the host waits for the former while the latter runs."""
         dev = data.pos.device
+        check_batch(data, data.pos.shape[0])
         f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()
         feats, pos, trans, sizes = f32(data.x), f32(data.pos), f32(data.trans_vec), data.sizes
         N, B = pos.shape[0], sizes.shape[0]
@@ -299,6 +318,7 @@ class Latticeformer(nn.Module):
         if geometry is None:
             geometry = BatchGeometry(data.pos, data.trans_vec, data.sizes, *(counts if counts is not None else ()))
         g = geometry
+        check_batch(data, g.batch.shape[0])
         x = self.encoder(x, data.pos, g.batch, data.trans_vec, g.sizes, geometry=g)
         x = self.proj_before_pooling(x)
         x = self.pooling_layer(x, g.batch, g.sizes)

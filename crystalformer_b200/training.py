@@ -198,10 +198,14 @@ def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[
         return None
     if any(t.requires_grad for t in (data.x, data.pos, data.trans_vec)) or torch.is_autocast_enabled():
         return None
+    # the kernels get addresses: what does not have the model's shapes, or lies elsewhere, is left to the operators' own checks
+    dev, sizes = data.pos.device, data.sizes
+    if data.x.device != dev or data.trans_vec.device != dev or sizes.dim() != 1 or sizes.shape[0] < 1 or data.pos.dim() != 2 \
+            or data.pos.shape[1] != 3 or tuple(data.x.shape) != (data.pos.shape[0], plan.desc.feature_dim) \
+            or data.trans_vec.numel() != 9 * sizes.shape[0]:
+        return None
     f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()
     feats, pos, trans = f32(data.x), f32(data.pos), f32(data.trans_vec)
-    dev = pos.device
-    sizes = data.sizes
     if sizes.device != dev or sizes.dtype != torch.int64 or not sizes.is_contiguous():
         sizes = sizes.to(device=dev, dtype=torch.int64).contiguous()
     if pos.shape[0] < 1 or feats.data_ptr() % 16 or plan.params[0].device != dev or (counts is not None and (
