@@ -55,6 +55,7 @@ SIGNATURES = {
     "cf_dense_pack_embedding": [P, I64, P, P],
     "cf_model_head_floats": [I64],
     "cf_model_begin": [P, P, P, I64, I64, P, P, P, P],
+    "cf_begin_abandon": [P, P],
     "cf_model_finish": [P, P, P, P, P, I64, I64, I64, I64, P, P, P, P, P, P, P],
     "cf_train_saved_bytes": [P, I64, I64],
     "cf_train_edge_bytes": [P, I64, I64, I64],

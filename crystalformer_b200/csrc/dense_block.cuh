@@ -45,7 +45,7 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
                        const double *scalars, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius, int lattice_range,
                        int minimum_range, const float *W1, const float *b1, int64_t hidden, const float *W2, const float *b2,
                        int64_t targets, double order_reach, void *workspace, float *y, void *const *attn_events,
-                       const cf_peer_gather *gather, void *inputs_ready, void *slot_free, void *stream, float *head = nullptr);
+                       const cf_peer_gather *gather, void *inputs_ready, void *slot_free, void *stream, const HeadStage *begun = nullptr);
 
 inline bool dense_path_available(int num_layers, const float *const *weights, long long ff_dim)
 {

@@ -77,10 +77,12 @@ int launch_dense_forward(const DenseForward &p, cudaStream_t s);
 // wrote; head_stage carves it from N (4 x 128 + 8) floats.
 struct HeadStage {
     float *x, *q, *k, *v, *a;
+    void *event;  // after which it has been written
 };
-inline HeadStage head_stage(float *memory, long long N)
+inline HeadStage head_stage(float *memory, long long N, void *event)
 {
     HeadStage h;
+    h.event = event;
     h.x = memory; h.q = h.x + N * 128; h.k = h.q + N * 128; h.v = h.k + N * 128; h.a = h.v + N * 128;
     return h;
 }
@@ -92,8 +94,10 @@ inline void dense_head_of(DenseForward &d, const float *const *w, const double *
     d.elu_beta = (float)sc[3]; d.lower_bound = (float)sc[4];
     d.a_factor_hi = d.a_factor; d.lower_bound_hi = d.lower_bound;
 }
-// Host read of a batch's sizes beside the work that `launch` queues (encoder_forward.cu).
-int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *), void *arg, void **inputs_event);
+// Host read of a batch's sizes beside the work that `launch` queues on the side stream (encoder_forward.cu).
+int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *, cudaStream_t), void *arg,
+                      void **begun_event);
+int join_begun(void *begun_event, cudaStream_t s);
 
 // ---- training (dense_tc_bwd.cu) ---------------------------------------------------------------------------------------
 // The blocks of one layer in the backward kernel's order, every one transposed: [Wq, Wk, Wv] and

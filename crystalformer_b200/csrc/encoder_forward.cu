@@ -46,11 +46,11 @@ int sorted_attn_impl(const float *q, const float *k, const float *v, const float
                      const RowListView &view, int sched_slot, bool zeroed, int64_t K, cudaStream_t s);
 namespace {
 
-// A second stream and two events per (host thread, device), created on first use and kept for the life of the
+// A second stream and its events per (host thread, device), created on first use and kept for the life of the
 // process: the term-list build of a forward depends on the geometry only and runs beside the first dense block.
 struct SideStream {
     cudaStream_t stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr, inputs = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, inputs = nullptr, begun = nullptr;
     bool ok = false;
 };
 SideStream &side_stream()
@@ -63,7 +63,8 @@ SideStream &side_stream()
         s.ok = cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) == cudaSuccess &&
                cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) == cudaSuccess &&
                cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) == cudaSuccess &&
-               cudaEventCreateWithFlags(&s.inputs, cudaEventDisableTiming) == cudaSuccess;
+               cudaEventCreateWithFlags(&s.inputs, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&s.begun, cudaEventDisableTiming) == cudaSuccess;
         if (!s.ok) {
             cudaGetLastError();
             s.stream = reinterpret_cast<cudaStream_t>(1);  // do not try again
@@ -75,9 +76,13 @@ SideStream &side_stream()
 }  // namespace
 
 // The host's copy of a batch's sizes, for callers that only have them on the device: the copy is queued first, then
-// `launch` queues work that needs the number of atoms only, and the host waits for the copy while that runs.  counts =
-// { atoms, edges, largest crystal }.  Pinned staging memory and the event are this thread's (at most 8 MiB, returned
-// when the thread ends).
+// `launch` queues work that needs the number of atoms only on the side stream, and the host waits for the copy while that
+// runs.  counts = { atoms, edges, largest crystal }.  Pinned staging memory and the event are this thread's (at most 8 MiB,
+// returned when the thread ends).
+// It is the early work that goes to the side stream and the rest of the batch's that stays on `s`: the memory of the rest is
+// allocated after the wait, in the order of `s`, when other host threads may have queued work on `s` and freed their
+// memory to it, so nothing but `s` itself may touch that memory first.  The early work writes only what was allocated
+// before the fork.
 namespace {
 struct PinnedSizes {
     int64_t *at = nullptr;
@@ -96,7 +101,13 @@ struct PinnedSizes {
     }
 };
 }  // namespace
-int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *), void *arg, void **inputs_event)
+// `s` made to wait for the early work of a batch.
+int join_begun(void *begun_event, cudaStream_t s)
+{
+    return cudaStreamWaitEvent(s, reinterpret_cast<cudaEvent_t>(begun_event), 0) == cudaSuccess ? CF_OK : launch_status("first block");
+}
+int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *, cudaStream_t), void *arg,
+                      void **begun_event)
 {
     static thread_local PinnedSizes pinned;
     SideStream &side = side_stream();
@@ -107,10 +118,16 @@ int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStre
         CF_REQUIRE(pinned.reserve(B), CF_ERR_CUDA, "no pinned memory for %lld sizes", (long long)B);
         if (cudaMemcpyAsync(pinned.at, sizes, sizeof(int64_t) * (size_t)B, cudaMemcpyDeviceToHost, s) != cudaSuccess) return launch_status("sizes to the host");
     }
-    if (cudaEventRecord(side.inputs, s) != cudaSuccess) return launch_status("sizes to the host");
-    *inputs_event = side.inputs;
-    const int rc = launch(arg);
-    if (rc != CF_OK || !read) return rc;
+    if (cudaEventRecord(side.inputs, s) != cudaSuccess || cudaStreamWaitEvent(side.stream, side.inputs, 0) != cudaSuccess)
+        return launch_status("sizes to the host");
+    const int rc = launch(arg, side.stream);
+    if (cudaEventRecord(side.begun, side.stream) != cudaSuccess) return launch_status("first block");
+    *begun_event = side.begun;
+    if (rc != CF_OK) {
+        join_begun(side.begun, s);  // (what was launched may still write to the caller's memory)
+        return rc;
+    }
+    if (!read) return rc;
     if (cudaEventSynchronize(side.inputs) != cudaSuccess) return launch_status("sizes to the host");
     int64_t n = 0, e = 0, m = 0;
     for (int64_t c = 0; c < B; ++c) {
@@ -217,6 +234,12 @@ __global__ void ffn_post_kernel(float *__restrict__ h, const float *__restrict__
 }  // namespace
 }  // namespace cf
 
+extern "C" int cf_begin_abandon(void *begun_event, void *stream)
+{
+    CF_REQUIRE(begun_event != nullptr, CF_ERR_INVALID, "cf_begin_abandon: null pointer");
+    return cf::join_begun(begun_event, cf::as_stream(stream));
+}
+
 extern "C" int64_t cf_encoder_workspace_floats(int64_t N, int64_t E, int64_t ff_dim)
 {
     // qkv (384) + q,k,v (3 x 128) + attention output (128) + a (8) + lse (8) + hidden (ff) per atom, logits per edge,
@@ -274,7 +297,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     bool sorted_rows = false;  // batches of crystals of at most 32 atoms with a value encoding: row lists + sorted row kernel
     // The build runs on the side stream and the first attention waits for it.  early_prep: the caller has already put the
     // geometry launch on the side stream (cf_model_forward with an inputs-ready event), so the side stream is not made
-    // to wait for this stream here.
+    // to wait for this stream here.  begun: the first dense block is on the side stream already and the build stays here.
     bool forked = early_prep;
     unsigned *tickets = nullptr;
     RowBlocks row_blocks{};
@@ -286,7 +309,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
             const BoxRule rule{(float)cutoff_radius, lattice_range, minimum_range};
             const float window = term_window(weight_floor_log2(), a_widest);
             SideStream &side = side_stream();
-            if (!early_prep)
+            if (!early_prep && begun == nullptr)
                 forked = side.ok && cudaEventRecord(side.fork, s) == cudaSuccess &&
                          cudaStreamWaitEvent(side.stream, side.fork, 0) == cudaSuccess;
             // (without a basis the enumerating kernel with term lists is faster - 0.62 against 0.79 ms for a 7-layer
@@ -360,6 +383,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
             return launch_dense_forward(d, s);
         };
         rc = boundary(0);
+        if (begun != nullptr && rc == CF_OK) rc = join_begun(begun->event, s);
         if (forked) cudaStreamWaitEvent(s, side_stream().join, 0);
         for (int l = 0; l < num_layers && rc == CF_OK; ++l) {
             if (attn_events) cudaEventRecord(reinterpret_cast<cudaEvent_t>(attn_events[2 * l]), s);

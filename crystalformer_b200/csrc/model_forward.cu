@@ -145,7 +145,7 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
                        int lattice_range, int minimum_range, const float *W1, const float *b1, int64_t hidden,
                        const float *W2, const float *b2, int64_t targets, double order_reach, void *workspace,
                        float *y, void *const *attn_events, const cf_peer_gather *gather, void *inputs_ready,
-                       void *slot_free, void *stream, float *head)
+                       void *slot_free, void *stream, const HeadStage *begun)
 {
     CF_REQUIRE(N >= 0 && B >= 0 && E >= 0 && feature_dim > 0, CF_ERR_INVALID, "cf_model_forward: bad size");
     if (gather != nullptr) {
@@ -166,8 +166,7 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
     CF_REQUIRE(embed_fused || features, CF_ERR_UNSUPPORTED, "cf_model_forward: species indices need the packed weights");
     cudaStream_t s = as_stream(stream);
     Scratch w = carve(workspace, N, B, E, ff_dim);
-    const HeadStage begun = head_stage(head, N);
-    if (head != nullptr) w.x = begun.x;
+    if (begun != nullptr) w.x = begun->x;
 
     CF_REQUIRE(B <= (1 << 20), CF_ERR_RANGE, "cf_model_forward: B=%lld above 2^20 crystals", (long long)B);
     // Early preparation: given an event after which the inputs are valid, the geometry launch and the list build go to
@@ -193,7 +192,7 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
     rc = encoder_forward_impl(cublas_handle, num_layers, weights, scalars, w.x, w.pos_ij, trans,
                               cutoff_radius != 0.0 ? w.rvlen : nullptr, w.batch, w.edges, w.row_start, N, B, E, max_atoms, K,
                               ff_dim, wscale, cutoff_radius, lattice_range, minimum_range, w.encoder, order, attn_events,
-                              stream, embed_fused ? &embed : nullptr, early, head != nullptr ? &begun : nullptr);
+                              stream, embed_fused ? &embed : nullptr, early, begun);
     if (rc != CF_OK) return rc;
     const bool chained = num_layers > 0 && N > 0;  // behind the encoder's last dense block
     if (gather != nullptr)
@@ -231,42 +230,42 @@ struct BeginArgs {
     const float *features;
     int64_t N;
     float *head;
-    cudaStream_t s;
 };
-int begin_launch(void *arg)
+int begin_launch(void *arg, cudaStream_t s)
 {
     const BeginArgs &b = *static_cast<const BeginArgs *>(arg);
-    const HeadStage h = head_stage(b.head, b.N);
+    const HeadStage h = head_stage(b.head, b.N, nullptr);
     DenseForward d{};
     d.N = b.N; d.ff = (int)b.d->ff_dim; d.x_out = h.x; d.q = h.q; d.k = h.k; d.v = h.v; d.a = h.a;
     dense_embed_of(d, EmbedStage{b.features, nullptr, (int)b.d->feature_dim, reinterpret_cast<const float4 *>(b.d->W_embed_packed)});
     dense_head_of(d, b.d->weights, b.d->scalars);
-    return launch_dense_forward(d, b.s);
+    return launch_dense_forward(d, s);
 }
 }  // namespace
 }  // namespace cf
 
 extern "C" int cf_model_begin(const cf_model_desc *desc, const float *features, const int64_t *sizes, int64_t N, int64_t B,
-                              float *head, int64_t *counts, void **inputs_event, void *stream)
+                              float *head, int64_t *counts, void **begun_event, void *stream)
 {
     using namespace cf;
-    CF_REQUIRE(desc && features && sizes && head && counts && inputs_event, CF_ERR_INVALID, "cf_model_begin: null pointer");
+    CF_REQUIRE(desc && features && sizes && head && counts && begun_event, CF_ERR_INVALID, "cf_model_begin: null pointer");
     CF_REQUIRE(N >= 1 && B >= 1, CF_ERR_INVALID, "cf_model_begin: empty batch");
     CF_REQUIRE(desc->num_layers >= 1 && desc->feature_dim >= 1 && desc->feature_dim <= 128 && is_tc_image(desc->W_embed_packed) &&
                    dense_tc_images(desc->num_layers, desc->weights),
                CF_ERR_UNSUPPORTED, "cf_model_begin: needs weight images");
-    BeginArgs args{desc, features, N, head, as_stream(stream)};
-    return read_sizes_beside(sizes, B, counts, as_stream(stream), begin_launch, &args, inputs_event);
+    BeginArgs args{desc, features, N, head};
+    return read_sizes_beside(sizes, B, counts, as_stream(stream), begin_launch, &args, begun_event);
 }
 
 extern "C" int cf_model_finish(const cf_model_desc *d, const float *features, const float *pos, const float *trans, const int64_t *sizes,
-                               int64_t N, int64_t B, int64_t E, int64_t max_atoms, float *head, void *inputs_event, void *workspace,
+                               int64_t N, int64_t B, int64_t E, int64_t max_atoms, float *head, void *begun_event, void *workspace,
                                float *y, void *const *attn_events, const cf_peer_gather *gather, void *stream)
 {
     using namespace cf;
-    CF_REQUIRE(d && features && head && inputs_event, CF_ERR_INVALID, "cf_model_finish: null pointer");
+    CF_REQUIRE(d && features && head && begun_event, CF_ERR_INVALID, "cf_model_finish: null pointer");
+    const HeadStage begun = head_stage(head, N, begun_event);
     return model_forward_impl(nullptr, features, nullptr, d->feature_dim, pos, trans, sizes, N, B, E, max_atoms, d->W_embed,
                               d->W_embed_packed, d->num_layers, d->weights, d->scalars, d->K, d->ff_dim, d->wscale, d->cutoff_radius,
                               d->lattice_range, d->minimum_range, d->W1, d->b1, d->hidden, d->W2, d->b2, d->targets, d->order_reach,
-                              workspace, y, attn_events, gather, inputs_event, nullptr, stream, head);
+                              workspace, y, attn_events, gather, nullptr, nullptr, stream, &begun);
 }

@@ -513,13 +513,12 @@ struct TrainBegin {
     const cf_train_desc *d;
     const cf_train_batch *b;
     const Saved *w;
-    cudaStream_t s;
 };
-int train_begin_launch(void *arg)
+int train_begin_launch(void *arg, cudaStream_t s)
 {
     const TrainBegin &t = *static_cast<const TrainBegin *>(arg);
-    const int rc = pack_all(*t.d, *t.w, true, t.s);
-    return rc == CF_OK ? forward_boundary(*t.d, *t.b, *t.w, 0, t.s) : rc;
+    const int rc = pack_all(*t.d, *t.w, true, s);
+    return rc == CF_OK ? forward_boundary(*t.d, *t.b, *t.w, 0, s) : rc;
 }
 
 unsigned blocks_of(long long threads) { return (unsigned)((threads + 255) / 256); }
@@ -527,25 +526,25 @@ unsigned blocks_of(long long threads) { return (unsigned)((threads + 255) / 256)
 }  // namespace
 }  // namespace cf
 
-extern "C" int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **inputs_event, void *stream)
+extern "C" int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **begun_event, void *stream)
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_begin");
     if (rc == CF_OK) rc = check_batch(batch, "cf_train_begin", false);
     if (rc != CF_OK) return rc;
-    CF_REQUIRE(counts && inputs_event, CF_ERR_INVALID, "cf_train_begin: null pointer");
+    CF_REQUIRE(counts && begun_event, CF_ERR_INVALID, "cf_train_begin: null pointer");
     const Saved w = carve_saved(*desc, batch->saved, nullptr, batch->N, batch->B, 0);
-    TrainBegin arg{desc, batch, &w, as_stream(stream)};
-    return read_sizes_beside(batch->sizes, batch->B, counts, as_stream(stream), train_begin_launch, &arg, inputs_event);
+    TrainBegin arg{desc, batch, &w};
+    return read_sizes_beside(batch->sizes, batch->B, counts, as_stream(stream), train_begin_launch, &arg, begun_event);
 }
 
-extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *inputs_event, float *y, void *stream)
+extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *begun_event, float *y, void *stream)
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_forward");
     if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward", true);
     if (rc != CF_OK) return rc;
-    CF_REQUIRE(y && inputs_event, CF_ERR_INVALID, "cf_train_forward: null pointer");
+    CF_REQUIRE(y && begun_event, CF_ERR_INVALID, "cf_train_forward: null pointer");
     const cf_train_desc &d = *desc;
     const cf_train_batch &b = *batch;
     const int64_t N = b.N, B = b.B, E = b.E;
@@ -554,13 +553,14 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
     const Saved w = carve_saved(d, b.saved, b.saved_edges, N, B, E);
     const float *const *tail_weights = d.weights + PER_LAYER * L;
 
-    // ---- geometry, term lists and the backward's weight images beside the first dense block
-    cudaStream_t prep = early_prep_stream(inputs_event, nullptr);
-    CF_REQUIRE(prep != nullptr, CF_ERR_CUDA, "cf_train_forward: the side stream could not be created");
-    if (cudaMemsetAsync(w.tickets, 0, sizeof(unsigned) * MAX_LAYERS, prep) != cudaSuccess) return launch_status("cf_train_forward: tickets");
+    // ---- the backward's weight images behind the first dense block on the side stream (into memory that cf_train_begin has
+    //      had), geometry and term lists here, beside both
+    cudaStream_t side = early_prep_stream(nullptr, nullptr);
+    CF_REQUIRE(side != nullptr, CF_ERR_CUDA, "cf_train_forward: the side stream could not be created");
+    if (cudaMemsetAsync(w.tickets, 0, sizeof(unsigned) * MAX_LAYERS, s) != cudaSuccess) return launch_status("cf_train_forward: tickets");
     bool ordered = false;
     rc = launch_prepare_all(b.pos, b.trans, b.sizes, w.atom_start, w.edge_start, B, N, E, w.batch, w.edges, w.row_start, w.pos_ij, w.rvlen,
-                            d.order_reach, w.row_order, &ordered, prep, w.rvecs, w.vcell);
+                            d.order_reach, w.row_order, &ordered, s, w.rvecs, w.vcell);
     if (rc != CF_OK) return rc;
     const int32_t *order = ordered ? w.row_order : nullptr;
     const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
@@ -576,17 +576,17 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
         tb.window = list.window;
         term_list_carve(w.lists, N, E, &tb.start, &tb.count, &tb.dmin, &tb.cursor, &tb.pool);
         tb.capacity = (long long)term_pool_entries(N, E);
-        rc = launch_term_list_build(tb, prep);
+        rc = launch_term_list_build(tb, s);
         if (rc != CF_OK) return rc;
     }
     static_assert(MAX_LAYERS <= ROW_BLOCK_LAYERS, "every layer has a scheduling block of its own");
     const RowBlocks row_blocks = row_blocks_carve(w.row_blocks, N);
     const bool by_blocks = listed && b.max_atoms > ROW_BLOCK_MIN_ATOMS && b.max_atoms <= ROW_BLOCK_MAX_ATOMS;
-    if (by_blocks) rc = launch_row_blocks(row_blocks, order, w.row_start, w.edges, N, E, prep);
+    if (by_blocks) rc = launch_row_blocks(row_blocks, order, w.row_start, w.edges, N, E, s);
     if (rc != CF_OK) return rc;
-    if (w.kr != nullptr) rc = cf_reci_phase(w.pos_ij, w.rvecs, w.batch, w.edges, E, w.kr, prep);
-    if (rc == CF_OK) rc = join_early_prep(s);
-    if (rc == CF_OK) rc = pack_all(d, w, false, prep);  // (joined before the backward, below)
+    if (w.kr != nullptr) rc = cf_reci_phase(w.pos_ij, w.rvecs, w.batch, w.edges, E, w.kr, s);
+    if (rc == CF_OK) rc = join_begun(begun_event, s);
+    if (rc == CF_OK) rc = pack_all(d, w, false, side);  // (joined below)
     // ---- layers
     for (int l = 0; l < L && rc == CF_OK; ++l) {
         const LayerSaved &t = w.layer[l];
@@ -620,7 +620,8 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
     if (rc == CF_OK)
         rc = launch_pool_head(w.x[L], w.atom_start, tail_weights[1], tail_weights[2], tail_weights[3], tail_weights[4], (int)d.hidden,
                               (int)d.targets, B, y, w.pooled, w.hid, true, s);
-    return rc == CF_OK ? join_early_prep(s) : rc;
+    const int joined = join_early_prep(s);  // (after an error too: the images may still be being written)
+    return rc == CF_OK ? joined : rc;
 }
 
 extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, const float *gy, void *scratch,

@@ -285,13 +285,18 @@ class Latticeformer(nn.Module):
             _lib.call("cf_model_begin", desc, feats.data_ptr(), sizes.data_ptr(), N, B, head.data_ptr(), counts, ctypes.byref(event), stream)
             n_atoms, n_edges, max_atoms = counts
             if n_atoms != N:  # (atoms beyond the crystals: their rows are not part of the batch)
+                _lib.call("cf_begin_abandon", event, stream)
                 return self._forward_native(data, (n_atoms, n_edges, max_atoms), gather, plan)
-            work = torch.empty(int(lib.cf_model_workspace_bytes(N, B, n_edges, plan["w"]["ff"])), dtype=torch.uint8, device=dev)
-            y = torch.empty((B, plan["targets"]), dtype=torch.float32, device=dev)
-            step = None if gather is None else gather.next_descriptor()
-            _lib.call("cf_model_finish", desc, feats.data_ptr(), pos.data_ptr(), trans.data_ptr(), sizes.data_ptr(), N, B, n_edges,
-                      max_atoms, head.data_ptr(), event, work.data_ptr(), y.data_ptr(), self.encoder._attention_events(),
-                      None if step is None else ctypes.byref(step), stream)
+            try:
+                work = torch.empty(int(lib.cf_model_workspace_bytes(N, B, n_edges, plan["w"]["ff"])), dtype=torch.uint8, device=dev)
+                y = torch.empty((B, plan["targets"]), dtype=torch.float32, device=dev)
+                step = None if gather is None else gather.next_descriptor()
+                _lib.call("cf_model_finish", desc, feats.data_ptr(), pos.data_ptr(), trans.data_ptr(), sizes.data_ptr(), N, B, n_edges,
+                          max_atoms, head.data_ptr(), event, work.data_ptr(), y.data_ptr(), self.encoder._attention_events(),
+                          None if step is None else ctypes.byref(step), stream)
+            except BaseException:  # (the first block still writes to `head`, on a stream of the library's)
+                _lib.load().cf_begin_abandon(event, stream)
+                raise
         return y if gather is None else gather.collect()
 
     def forward(self, data, geometry: Optional[BatchGeometry] = None, counts: Optional[Tuple[int, int, int]] = None,

@@ -153,12 +153,16 @@ class TrainStep(torch.autograd.Function):
         with torch.cuda.device(dev):
             stream = torch.cuda.current_stream(dev).cuda_stream
             _lib.call("cf_train_begin", desc, ctypes.byref(batch), known, ctypes.byref(event), stream)
-            if known[0] != N or known[2] > 1024:
-                raise NotThisBatch
-            batch.E, batch.max_atoms = known[1], known[2]
-            edges = torch.empty(int(lib.cf_train_edge_bytes(desc, N, B, batch.E)), dtype=torch.uint8, device=dev)
-            batch.saved_edges = edges.data_ptr()
-            _lib.call("cf_train_forward", desc, ctypes.byref(batch), event, y.data_ptr(), stream)
+            try:
+                if known[0] != N or known[2] > 1024:
+                    raise NotThisBatch
+                batch.E, batch.max_atoms = known[1], known[2]
+                edges = torch.empty(int(lib.cf_train_edge_bytes(desc, N, B, batch.E)), dtype=torch.uint8, device=dev)
+                batch.saved_edges = edges.data_ptr()
+                _lib.call("cf_train_forward", desc, ctypes.byref(batch), event, y.data_ptr(), stream)
+            except BaseException:  # (the first block still writes to `saved`, on a stream of the library's)
+                lib.cf_begin_abandon(event, stream)
+                raise
         ctx.save_for_backward(saved, edges, feats, pos, trans, sizes)
         ctx.step = (plan, batch, plan.versions())
         return y

@@ -14,7 +14,7 @@
  *     failure on the calling thread.
  * State kept by the library: the process-wide switches (cf_set_weight_floor_log2, cf_set_sorted_rows,
  * cf_set_chained_launches, cf_set_row_stats), a
- * side stream and three events per (host thread, device) created by the first cf_encoder_forward / cf_model_forward
+ * side stream and four events per (host thread, device) created by the first cf_encoder_forward / cf_model_forward
  * / cf_model_begin / cf_train_begin, a pinned staging buffer of at most 8 MiB per host thread for the sizes that the
  * begin calls read back,
  * the 8 MiB scratch array of cf_lattice_sum_bwd_static, and a pool of row tickets per device: 64 single counters
@@ -427,13 +427,18 @@ int cf_model_forward(void *cublas_handle, const float *features, int64_t feature
 
 /* ------------------------------------------------------------------------------------------------------------
  * cf_model_forward in two halves, for callers whose sizes are on the device only (declared below cf_model_desc):
- * cf_model_begin queues the read-back of the sizes, then the first dense block (which needs the number of atoms only),
- * waits for the sizes while that runs and returns counts = { atoms, edges, largest crystal } (nothing is read or waited
- * for if counts[0] >= 0 on entry); cf_model_finish queues the rest, its batch preparation beside the first block.  Only
- * with weight images.  head: cf_model_head_floats(N) floats of device memory, kept between the two; inputs_event: an
- * event of the library's, valid until this thread's next cf_model_begin / cf_train_begin.
+ * cf_model_begin queues the read-back of the sizes, then, on the library's side stream, the first dense block (which needs
+ * the number of atoms only), waits for the sizes while that runs and returns counts = { atoms, edges, largest crystal }
+ * (nothing is read or waited for if counts[0] >= 0 on entry); cf_model_finish queues the rest on `stream`, its batch
+ * preparation beside the first block.  Only with weight images.  head: cf_model_head_floats(N) floats of device memory,
+ * kept between the two; begun_event: an event of the library's that the first block is followed by, valid until this
+ * thread's next cf_model_begin / cf_train_begin.  Memory that cf_model_finish / cf_train_forward alone are given may be
+ * allocated after the begin call, in the order of `stream`, also when other host threads use that stream meanwhile.
+ * A batch that has been begun and is not finished is given up by cf_begin_abandon: `stream` waits for its first block, after
+ * which the memory may be reused in the order of `stream`.
  * ---------------------------------------------------------------------------------------------------------- */
 int64_t cf_model_head_floats(int64_t N);
+int cf_begin_abandon(void *begun_event, void *stream);
 
 /* ------------------------------------------------------------------------------------------------------------
  * A training step of the whole model (what autograd does through Latticeformer.forward and its backward,
@@ -451,7 +456,7 @@ int64_t cf_model_head_floats(int64_t N);
  *                    backward reads: `saved`, cf_train_saved_bytes(desc, N, B) bytes, and `saved_edges`,
  *                    cf_train_edge_bytes(desc, N, B, E) bytes (E = sum n^2 >= 1, largest crystal max_atoms <= 1024).
  * cf_train_begin needs N, B and `saved` only: it queues the read-back of the sizes, packs the weights and runs the first
- * dense block, and returns counts and inputs_event as cf_model_begin does; cf_train_forward then writes y (B, targets).
+ * dense block, and returns counts and begun_event as cf_model_begin does; cf_train_forward then writes y (B, targets).
  * cf_train_backward takes gy (B, targets), scratch of cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of
  * device pointers to the gradients, in the order of the weights (the entry of a NULL weight is not used); every gradient
  * is written, none accumulated.  The weights must not change between the calls.
@@ -472,8 +477,8 @@ typedef struct cf_train_batch {
 int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B);
 int64_t cf_train_edge_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
 int64_t cf_train_scratch_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
-int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **inputs_event, void *stream);
-int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *inputs_event, float *y, void *stream);
+int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **begun_event, void *stream);
+int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *begun_event, float *y, void *stream);
 int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, const float *gy, void *scratch,
                       float *const *grads, void *stream);
 
@@ -527,9 +532,9 @@ typedef struct cf_model_desc {
     double order_reach;
 } cf_model_desc;
 int cf_model_begin(const cf_model_desc *desc, const float *features, const int64_t *sizes, int64_t N, int64_t B, float *head,
-                   int64_t *counts, void **inputs_event, void *stream);
+                   int64_t *counts, void **begun_event, void *stream);
 int cf_model_finish(const cf_model_desc *desc, const float *features, const float *pos, const float *trans, const int64_t *sizes,
-                    int64_t N, int64_t B, int64_t E, int64_t max_atoms, float *head, void *inputs_event, void *workspace, float *y,
+                    int64_t N, int64_t B, int64_t E, int64_t max_atoms, float *head, void *begun_event, void *workspace, float *y,
                     void *const *attn_events, const cf_peer_gather *gather, void *stream);
 typedef struct cf_serve_slot {
     void *copy_stream, *compute_stream;
