@@ -387,12 +387,13 @@ int check_desc(const cf_train_desc *d, const char *who)
                "%s: lattice_range %d outside [0,%d]", who, (int)d->lattice_range, CF_MAX_RANGE);
     return CF_OK;
 }
-int check_batch(const cf_train_batch *b, const char *who, bool edges_known)
+enum Half { BEGIN, FORWARD, BACKWARD };
+int check_batch(const cf_train_batch *b, const char *who, Half half)
 {
     CF_REQUIRE(b != nullptr, CF_ERR_INVALID, "%s: null batch", who);
     CF_REQUIRE(b->N >= 1 && b->B >= 1 && b->B <= (1 << 20), CF_ERR_INVALID, "%s: empty batch or too many crystals", who);
-    CF_REQUIRE(b->features && b->pos && b->trans && b->sizes && b->saved, CF_ERR_INVALID, "%s: null pointer", who);
-    if (!edges_known) return CF_OK;
+    CF_REQUIRE(b->features && b->trans && b->saved && (half == BACKWARD || (b->pos && b->sizes)), CF_ERR_INVALID, "%s: null pointer", who);
+    if (half == BEGIN) return CF_OK;
     CF_REQUIRE(b->E >= 1 && b->max_atoms >= 1 && b->max_atoms <= 1024, CF_ERR_RANGE, "%s: E=%lld, max_atoms=%lld (1..1024)", who,
                (long long)b->E, (long long)b->max_atoms);
     CF_REQUIRE(b->saved_edges, CF_ERR_INVALID, "%s: null pointer", who);
@@ -530,7 +531,7 @@ extern "C" int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *b
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_begin");
-    if (rc == CF_OK) rc = check_batch(batch, "cf_train_begin", false);
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_begin", BEGIN);
     if (rc != CF_OK) return rc;
     CF_REQUIRE(counts && begun_event, CF_ERR_INVALID, "cf_train_begin: null pointer");
     const Saved w = carve_saved(*desc, batch->saved, nullptr, batch->N, batch->B, 0);
@@ -542,7 +543,7 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_forward");
-    if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward", true);
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward", FORWARD);
     if (rc != CF_OK) return rc;
     CF_REQUIRE(y && begun_event, CF_ERR_INVALID, "cf_train_forward: null pointer");
     const cf_train_desc &d = *desc;
@@ -629,7 +630,7 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_backward");
-    if (rc == CF_OK) rc = check_batch(batch, "cf_train_backward", true);
+    if (rc == CF_OK) rc = check_batch(batch, "cf_train_backward", BACKWARD);
     if (rc != CF_OK) return rc;
     CF_REQUIRE(gy && scratch && grads, CF_ERR_INVALID, "cf_train_backward: null pointer");
     const cf_train_desc &d = *desc;

@@ -92,7 +92,8 @@ class TrainPlan:
         where = iter(range(len(self.params)))
         self.slots = [None if p is None else next(where) for p in ordered]
         self.offsets = offsets
-        self.pointers = (ctypes.c_void_p * len(ordered))(*[None if p is None else p.data_ptr() for p in ordered])
+        self.addresses = [p.data_ptr() for p in self.params]
+        self.pointers = self.table(self.addresses)
         self.scalars = (ctypes.c_double * len(scalars))(*scalars)
         self.targets = model.mlp[3].out_features
         order_reach = model.native_reach()
@@ -103,11 +104,31 @@ class TrainPlan:
             targets=self.targets, wscale=float(P.value_pe_width_scale), cutoff_radius=enc._cutoff(), order_reach=order_reach,
             weights=ctypes.cast(self.pointers, ctypes.c_void_p), scalars=ctypes.cast(self.scalars, ctypes.c_void_p))
 
+    def table(self, addresses):
+        """Addresses of the parameters, one after the other, as the library's array with its empty places."""
+        return (ctypes.c_void_p * len(self.slots))(*[None if s is None else addresses[s] for s in self.slots])
+
+    def desc_now(self) -> _lib.TrainDesc:
+        """The description with the parameters where they lie now: their storage may have been replaced since the forward."""
+        addresses = [p.data_ptr() for p in self.params]
+        if addresses == self.addresses:
+            return self.desc
+        if not all(p.shape == q.shape and usable(p, q.device) for p, q in zip(self.params, self.like)):
+            raise RuntimeError("a parameter of the model was moved or changed its type between the forward and the backward of a training step")
+        desc = _lib.TrainDesc.from_buffer_copy(self.desc)
+        desc.keep = self.table(addresses)
+        desc.weights = ctypes.cast(desc.keep, ctypes.c_void_p)
+        return desc
+
     def current(self) -> bool:
         return self.watch.current() and [g._version for g in self.scales] == self.scale_versions
 
     def versions(self) -> list:
         return [p._version for p in self.params]
+
+
+def usable(p: torch.Tensor, device) -> bool:
+    return p.dtype == torch.float32 and p.is_contiguous() and p.device == device
 
 
 def supported(model) -> bool:
@@ -130,7 +151,7 @@ def supported(model) -> bool:
             return False
         if any(isinstance(m, torch.nn.Dropout) and m.p > 0 for m in (layer.dropout, layer.dropout1, layer.dropout2)) or att.dropout > 0:
             return False
-    return all(p.dtype == torch.float32 and p.is_contiguous() and p.device == dev for p in model.parameters())
+    return all(usable(p, dev) for p in model.parameters())
 
 
 class NotThisBatch(Exception):
@@ -163,29 +184,31 @@ class TrainStep(torch.autograd.Function):
             except BaseException:  # (the first block still writes to `saved`, on a stream of the library's)
                 lib.cf_begin_abandon(event, stream)
                 raise
-        ctx.save_for_backward(saved, edges, feats, pos, trans, sizes)
-        ctx.step = (plan, batch, plan.versions())
+        # (no address is kept: what saved-tensor hooks give back in the backward may lie elsewhere, or be a recomputation)
+        ctx.save_for_backward(saved, edges, feats, trans)
+        ctx.step = (plan, (N, B, batch.E, batch.max_atoms), plan.versions())
         return y
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, gy):
-        plan, batch, versions = ctx.step
-        keep = ctx.saved_tensors  # (the memory `batch` points into; released with the graph)
+        plan, (N, B, E, max_atoms), versions = ctx.step
+        saved, edges, feats, trans = ctx.saved_tensors
         if plan.versions() != versions:
             raise RuntimeError("a parameter of the model was modified by an in-place operation between the forward and the "
                                "backward of a training step")
         dev = gy.device
         gy = gy.contiguous()
-        scratch = torch.empty(int(_lib.load().cf_train_scratch_bytes(ctypes.byref(plan.desc), batch.N, batch.B, batch.E)),
-                              dtype=torch.uint8, device=dev)
+        desc = plan.desc_now()
+        batch = _lib.TrainBatch(features=feats.data_ptr(), trans=trans.data_ptr(), N=N, B=B, E=E, max_atoms=max_atoms,
+                                saved=saved.data_ptr(), saved_edges=edges.data_ptr())
+        scratch = torch.empty(int(_lib.load().cf_train_scratch_bytes(ctypes.byref(desc), N, B, E)), dtype=torch.uint8, device=dev)
         flat = torch.empty(plan.floats, dtype=torch.float32, device=dev)
         base = flat.data_ptr()
         where = (ctypes.c_void_p * len(plan.slots))(*[None if s is None else base + 4 * plan.offsets[s] for s in plan.slots])
         with torch.cuda.device(dev):
-            _lib.call("cf_train_backward", ctypes.byref(plan.desc), ctypes.byref(batch), gy.data_ptr(), scratch.data_ptr(),
+            _lib.call("cf_train_backward", ctypes.byref(desc), ctypes.byref(batch), gy.data_ptr(), scratch.data_ptr(),
                       ctypes.cast(where, ctypes.c_void_p), torch.cuda.current_stream(dev).cuda_stream)
-        del keep
         return (None, None, None, *torch._utils._unflatten_dense_tensors(flat, plan.like))
 
 

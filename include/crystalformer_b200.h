@@ -457,7 +457,8 @@ int cf_begin_abandon(void *begun_event, void *stream);
  *                    cf_train_edge_bytes(desc, N, B, E) bytes (E = sum n^2 >= 1, largest crystal max_atoms <= 1024).
  * cf_train_begin needs N, B and `saved` only: it queues the read-back of the sizes, packs the weights and runs the first
  * dense block, and returns counts and begun_event as cf_model_begin does; cf_train_forward then writes y (B, targets).
- * cf_train_backward takes gy (B, targets), scratch of cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of
+ * cf_train_backward (of the batch: features, trans, the sizes N, B, E, max_atoms and the two blocks of memory, which hold no
+ * addresses and may have been copied elsewhere since) takes gy (B, targets), scratch of cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of
  * device pointers to the gradients, in the order of the weights (the entry of a NULL weight is not used); every gradient
  * is written, none accumulated.  The weights must not change between the calls.
  * ---------------------------------------------------------------------------------------------------------- */

@@ -98,3 +98,41 @@ def test_forward_at_the_edges_of_its_dispatch(sizes, lengths, bins):
     scale = max(1.0, float(y0.abs().max()))
     assert (y0 - y1).abs().max() < 2e-6 * scale
     assert (y0 - y2).abs().max() < 2e-6 * scale
+
+
+def test_saved_tensors_that_come_back_elsewhere():
+    """Saved-tensor hooks (offloading, checkpointing) and parameters whose storage is replaced between forward and backward."""
+    from torch.autograd.graph import save_on_cpu, saved_tensors_hooks
+    from torch.utils.checkpoint import checkpoint
+    model, data, target = setup([9, 20, 5, 66], lengths=(8.0, 14.0), num_layers=2)
+    ref = step(model, data, target, native=True)[1]
+
+    def grads(y):
+        for p in model.parameters():
+            p.grad = None
+        fill = [torch.full((64 << 20,), 255, dtype=torch.uint8, device="cuda") for _ in range(2)]  # what the forward freed is reused
+        (y - target).abs().mean().backward()
+        del fill
+        return {n: p.grad for n, p in model.named_parameters() if p.requires_grad}
+
+    def with_hooks():
+        with save_on_cpu():
+            return model(data)
+
+    def with_copies():
+        with saved_tensors_hooks(lambda t: t.clone(), lambda t: t.clone()):
+            return model(data)
+
+    def replaced():
+        y = model(data)
+        for p in model.parameters():
+            p.data = p.data.clone()
+        return y
+
+    for forward in (with_hooks, with_copies, lambda: checkpoint(model, data, use_reentrant=False), replaced, lambda: model(data)):
+        got = grads(forward())
+        assert all(torch.equal(got[n], ref[n]) for n in ref)
+    # the positions are not needed any more after the forward
+    y = model(data)
+    data.pos.add_(0.0)
+    assert all(torch.equal(g, ref[n]) for n, g in grads(y).items())
