@@ -1,14 +1,17 @@
 """Training step of the model shell in two library calls (cf_train_forward / cf_train_backward) behind one autograd node.
 
-``Latticeformer.forward`` takes it whenever gradients are enabled and the configuration is the one the calls implement:
-the node's inputs are the model's parameters, its backward returns all of their gradients.  Same values as the
+``Latticeformer.forward`` takes it whenever gradients are enabled, the configuration is the one the calls implement and the
+submodules are the model's own (they are not called: a hook, a parametrisation or another class in their place would not
+take effect): the node's inputs are the model's parameters, its backward returns all of their gradients.  Same values as the
 operation-by-operation autograd path (models/latticeformer.py:211-302 and its backward), which stays for everything else."""
 from __future__ import annotations
 
 import ctypes
 from typing import Optional, Tuple
 
+import numpy as np
 import torch
+from torch.autograd.forward_ad import unpack_dual
 
 from . import _lib
 
@@ -38,6 +41,8 @@ class ModelWatch:
         self.versions = versions
         self.settings = model.encoder.lattice_params
         self.layer_settings = [layer.self_attn.params for layer in model.encoder.layers]
+        self.dropouts = [m for m in model.modules() if isinstance(m, torch.nn.Dropout)]
+        self.attentions = [layer.self_attn for layer in model.encoder.layers]
         self.key = self.now()
 
     def now(self) -> list:
@@ -46,6 +51,7 @@ class ModelWatch:
                P.value_pe_width_scale, P.value_pe_dist_max]
         for Q in self.layer_settings:
             key += (Q.positive_func, Q.gauss_lb_real, Q.scale_real, Q.value_pe_dist_max, Q.gauss_lb_reci, Q.scale_reci)
+        key += [m.p for m in self.dropouts] + [m.dropout for m in self.attentions]
         key += [t.data_ptr() for t in self.tensors]
         return key + [t._version for t in self.tensors] if self.versions else key
 
@@ -79,6 +85,7 @@ class TrainPlan:
         ordered += [model.input_embeddings.weight, model.mlp[0].weight, model.mlp[0].bias, model.mlp[3].weight, model.mlp[3].bias]
         self.params = [p for p in ordered if p is not None]
         self.watch = ModelWatch(model, versions=False)
+        self.submodules = [m.__dict__ for m in model.modules() if m is not model]
         self.scales = [layer.self_attn.gauss_scale for layer in enc.layers]
         self.scale_versions = [g._version for g in self.scales]
         sizes = [p.numel() for p in self.params]
@@ -91,7 +98,9 @@ class TrainPlan:
         self.like = [p.detach() for p in self.params]
         where = iter(range(len(self.params)))
         self.slots = [None if p is None else next(where) for p in ordered]
-        self.offsets = offsets
+        # the gradients' places as byte offsets in the library's order (0 and not `present` for a parameter that is not there)
+        self.present = np.array([s is not None for s in self.slots], dtype=np.int64)
+        self.offsets = np.array([0 if s is None else 4 * offsets[s] for s in self.slots], dtype=np.int64)
         self.addresses = [p.data_ptr() for p in self.params]
         self.pointers = self.table(self.addresses)
         self.scalars = (ctypes.c_double * len(scalars))(*scalars)
@@ -123,6 +132,13 @@ class TrainPlan:
     def current(self) -> bool:
         return self.watch.current() and [g._version for g in self.scales] == self.scale_versions
 
+    def untouched(self) -> bool:
+        """Whether calling the submodules would do nothing but their own forward (hooks of the model itself run in any case)."""
+        for d in self.submodules:
+            if d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or "forward" in d:
+                return False
+        return not torch.nn.modules.module._has_any_global_hook()
+
     def versions(self) -> list:
         return [p._version for p in self.params]
 
@@ -132,7 +148,14 @@ def usable(p: torch.Tensor, device) -> bool:
 
 
 def supported(model) -> bool:
-    """Whether the parameters are what the kernels read: float32, contiguous, on one GPU, one projection per head."""
+    """Whether the submodules are the model's own (a parametrised one has a class of its own) and the parameters what the
+    kernels read: float32, contiguous, on one GPU, one projection per head."""
+    from .attention import CrystalformerMultiheadAttentionCUDA, NonDynamicallyQuantizableLinear
+    from .encoder import CrystalformerEncoderCUDA, CrystalformerEncoderLayerCUDA
+    own = {torch.nn.Linear, NonDynamicallyQuantizableLinear, torch.nn.Identity, torch.nn.ReLU, torch.nn.Dropout, torch.nn.Sequential,
+           torch.nn.ModuleList, CrystalformerEncoderCUDA, CrystalformerEncoderLayerCUDA, CrystalformerMultiheadAttentionCUDA}
+    if any(type(m) not in own for m in model.modules() if m is not model):
+        return False
     enc = model.encoder
     ff = enc.layers[0].linear1.out_features if len(enc.layers) else 0
     hidden = model.mlp[0].out_features
@@ -204,11 +227,10 @@ class TrainStep(torch.autograd.Function):
                                 saved=saved.data_ptr(), saved_edges=edges.data_ptr())
         scratch = torch.empty(int(_lib.load().cf_train_scratch_bytes(ctypes.byref(desc), N, B, E)), dtype=torch.uint8, device=dev)
         flat = torch.empty(plan.floats, dtype=torch.float32, device=dev)
-        base = flat.data_ptr()
-        where = (ctypes.c_void_p * len(plan.slots))(*[None if s is None else base + 4 * plan.offsets[s] for s in plan.slots])
+        where = plan.offsets + flat.data_ptr() * plan.present
         with torch.cuda.device(dev):
             _lib.call("cf_train_backward", ctypes.byref(desc), ctypes.byref(batch), gy.data_ptr(), scratch.data_ptr(),
-                      ctypes.cast(where, ctypes.c_void_p), torch.cuda.current_stream(dev).cuda_stream)
+                      where.ctypes.data, torch.cuda.current_stream(dev).cuda_stream)
         return (None, None, None, *torch._utils._unflatten_dense_tensors(flat, plan.like))
 
 
@@ -221,9 +243,9 @@ def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[
             return None
         plan = TrainPlan(model)
         model._train_plan = OfThisModel(plan)
-    if not all(layer.self_attn.term_lists for layer in model.encoder.layers):
+    if not plan.untouched() or not all(layer.self_attn.term_lists for layer in model.encoder.layers):
         return None
-    if any(t.requires_grad for t in (data.x, data.pos, data.trans_vec)) or torch.is_autocast_enabled():
+    if any(t.requires_grad or unpack_dual(t).tangent is not None for t in (data.x, data.pos, data.trans_vec)) or torch.is_autocast_enabled():
         return None
     # the kernels get addresses: what does not have the model's shapes, or lies elsewhere, is left to the operators' own checks
     dev, sizes = data.pos.device, data.sizes

@@ -136,3 +136,92 @@ def test_saved_tensors_that_come_back_elsewhere():
     y = model(data)
     data.pos.add_(0.0)
     assert all(torch.equal(g, ref[n]) for n, g in grads(y).items())
+
+
+class Scaled(torch.nn.Linear):
+    def forward(self, x):
+        return 1.5 * super().forward(x)
+
+
+class Doubled(torch.nn.Module):
+    def forward(self, W):
+        return 2.0 * W
+
+
+def _hook(model, seen):
+    model.encoder.layers[1].linear1.register_forward_hook(lambda m, i, o: (seen.append(1), o * 1.5)[1])
+
+
+def _pre_hook(model, seen):
+    model.encoder.register_forward_pre_hook(lambda m, i: seen.append(1))
+
+
+def _backward_hook(model, seen):
+    model.encoder.layers[0].linear2.register_full_backward_hook(lambda m, gi, go: seen.append(1))
+
+
+def _parametrised(model, seen):
+    torch.nn.utils.parametrize.register_parametrization(model.encoder.layers[0].linear2, "weight", Doubled())
+
+
+def _subclass(model, seen):
+    old = model.encoder.layers[0].linear1
+    new = Scaled(old.in_features, old.out_features).cuda()
+    new.load_state_dict(old.state_dict())
+    model.encoder.layers[0].linear1 = new
+
+
+def _own_forward(model, seen):
+    layer = model.encoder.layers[1].linear2
+    layer.forward = lambda x: (seen.append(1), 0.5 * torch.nn.functional.linear(x, layer.weight, layer.bias))[1]
+
+
+def _layer_norm(model, seen):
+    model.encoder.layers[0].norm2 = torch.nn.LayerNorm(128).cuda()
+
+
+@pytest.mark.parametrize("change", [_hook, _pre_hook, _backward_hook, _parametrised, _subclass, _own_forward, _layer_norm])
+def test_changed_submodules_take_effect(change):
+    """What a user hangs on a submodule after the first step: the steps follow it, with updates of the weights in between."""
+    import torch.nn.utils.parametrize  # noqa: F401
+    model, data, target = setup([9, 20, 5], num_layers=2)
+    step(model, data, target, native=True)
+    assert model._train_plan is not None
+    seen = []
+    change(model, seen)
+    for _ in range(2):
+        (y0, ref), calls = step(model, data, target, native=False), len(seen)
+        y1, got = step(model, data, target, native=True)
+        assert len(seen) == 2 * calls
+        seen.clear()
+        assert torch.equal(y0, y1) and all(torch.equal(ref[n], got[n]) for n in ref)
+        with torch.no_grad():
+            for n, p in model.named_parameters():
+                if p.requires_grad:
+                    p.sub_(0.01 * got[n])
+
+
+def test_hooks_of_all_modules_and_dropout():
+    model, data, target = setup([9, 20, 5], num_layers=2)
+    for layer in model.encoder.layers:
+        layer.dropout2 = torch.nn.Dropout(0.0)
+    step(model, data, target, native=True)
+    assert model._train_plan is not None
+    seen = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: seen.append(type(m)))
+    step(model, data, target, native=True)
+    handle.remove()
+    assert torch.nn.Linear in seen
+    model.encoder.layers[1].dropout2.p = 0.9  # the next step drops units
+    a, b = (step(model, data, target, native=True)[0] for _ in range(2))
+    assert not torch.equal(a, b)
+
+
+def test_directional_derivatives_are_not_dropped():
+    """A tangent on an input is refused by the operators (they define none) and not ignored."""
+    import torch.autograd.forward_ad as fwad
+    model, data, target = setup([9, 5], num_layers=1)
+    with fwad.dual_level():
+        data.x = fwad.make_dual(data.x, torch.ones_like(data.x))
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            model(data)
