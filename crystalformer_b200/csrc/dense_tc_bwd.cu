@@ -464,9 +464,13 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(
 // ---- weight gradients ---------------------------------------------------------------------------------------------------
 // A block owns one 128 x 128 gradient block (GradJob) and a share of the atom rows, and contracts 64 rows at a time on the
 // tensor cores.  The contraction runs over rows, so rows cannot carry scales of their own; the operands are three bfloat16
-// pieces (24 bits, the exponent range of float) and a product the six piece products down to 2^-16 relative, summed smallest
-// first.  In memory a chunk of rows is already what the transposed (MN-major) operand wants: row n of a panel = 64
-// features of atom n in 128 swizzled bytes.  Sixteen warps load and convert, one thread issues; two chunks in flight.
+// pieces (24 bits, the exponent range of float) and a product the six piece products down to 2^-16 relative.  In memory a
+// chunk of rows is already what the transposed (MN-major) operand wants: row n of a panel = 64 features of atom n in 128
+// swizzled bytes.  Sixteen warps load and convert, one thread issues; two chunks in flight.
+// The tensor pipe drops what does not fit when it adds to an accumulator, always towards zero, so a sum that stays in one
+// loses half a unit per instruction: 7e-6 of the gradient after 5,000 rows (a float32 GEMM: 3e-7).  Here an accumulator
+// holds one chunk, its small products added first, so that four additions are of full size; the chunks are added in
+// registers, rounded to nearest (two accumulators, so that the additions of a chunk lie beside the next one's products).
 constexpr int GR_ROWS = 64;                                  // atoms per chunk
 constexpr int GR_PIECE = GR_ROWS * 256;                      // bytes of one piece of one operand (two 64-feature panels)
 constexpr int GR_BUFFER = 6 * GR_PIECE;                      // g pieces, x pieces
@@ -502,14 +506,17 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
     }
-    if (warp == 16) tmem_alloc<128>(base + GR_MISC + 56);
+    if (warp == 16) tmem_alloc<256>(base + GR_MISC + 56);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem_tc + GR_MISC + 56);
     const long long all = (job.rows + GR_ROWS - 1) / GR_ROWS;  // chunks of the job, and this block's share
     const long long c_lo = all * blockIdx.y / splits, c_hi = all * (blockIdx.y + 1) / splits;
-    float4 sums = make_float4(0.f, 0.f, 0.f, 0.f);
+    const Place pl;
+    float acc[2][16];  // the accumulator's chunks so far: thread = 4 rows x 8 columns, as in the chain kernels
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i >> 4][i & 15] = 0.f;
     if (warp == 16) {
         if (lane == 0) {
             constexpr uint32_t IDESC = instr_desc<128, 128, 1, true>();
@@ -527,19 +534,32 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
                     g[i] = smem_desc(base + b * GR_BUFFER + i * GR_PIECE, GR_PIECE / 2, 1024);
                     x[i] = smem_desc(base + b * GR_BUFFER + (3 + i) * GR_PIECE, GR_PIECE / 2, 1024);
                 }
+                const uint32_t d = tmem + 128u * (uint32_t)b;
 #pragma unroll
                 for (int ks = 0; ks < GR_ROWS / 16; ++ks) {
                     const uint64_t at = (uint64_t)(ks * 2048 >> 4);
-                    mma_f16(tmem, g[2] + at, x[0] + at, IDESC, c > c_lo || ks > 0);
-                    mma_f16(tmem, g[0] + at, x[2] + at, IDESC, true);
-                    mma_f16(tmem, g[1] + at, x[1] + at, IDESC, true);
-                    mma_f16(tmem, g[1] + at, x[0] + at, IDESC, true);
-                    mma_f16(tmem, g[0] + at, x[1] + at, IDESC, true);
-                    mma_f16(tmem, g[0] + at, x[0] + at, IDESC, true);
+                    mma_f16(d, g[2] + at, x[0] + at, IDESC, ks > 0);
+                    mma_f16(d, g[0] + at, x[2] + at, IDESC, true);
+                    mma_f16(d, g[1] + at, x[1] + at, IDESC, true);
+                }
+#pragma unroll
+                for (int ks = 0; ks < GR_ROWS / 16; ++ks) {
+                    const uint64_t at = (uint64_t)(ks * 2048 >> 4);
+                    mma_f16(d, g[1] + at, x[0] + at, IDESC, true);
+                    mma_f16(d, g[0] + at, x[1] + at, IDESC, true);
+                }
+#pragma unroll
+                for (int ks = 0; ks < GR_ROWS / 16; ++ks) {
+                    const uint64_t at = (uint64_t)(ks * 2048 >> 4);
+                    mma_f16(d, g[0] + at, x[0] + at, IDESC, true);
                 }
                 mma_commit(bar(G_EMPTY + b));
             }
-            mma_commit(bar(G_DONE));
+            if (!ok) {  // a wait has run out: the instructions issued so far
+                unsigned mine = 0u;
+                mma_commit(bar(G_DONE));
+                mbar_wait(bar(G_DONE), 0, &mine);
+            }
         }
     } else {
         // loader: warp w converts rows 4 w .. 4 w + 3 of either operand, lane l the columns 4 l .. 4 l + 3
@@ -567,11 +587,35 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
             }
         };
         fetch(c_lo);
-        for (long long c = c_lo; c < c_hi; ++c) {
+        float4 sums = make_float4(0.f, 0.f, 0.f, 0.f), lost = sums;  // column sums of g, and what their roundings dropped
+        auto add = [](float v, float &sum, float &low) {  // (compensated: the rows of a share are thousands)
+            const float t = sum + v, back = t - sum;
+            low += (sum - (t - back)) + (v - back);
+            sum = t;
+        };
+        for (long long c = c_lo; c < c_hi + 2; ++c) {  // (the last two only collect)
             const int b = (int)((c - c_lo) & 1);
             unsigned char *gb = smem_tc + b * GR_BUFFER + lane_at, *xb = gb + 3 * GR_PIECE;
-            mbar_wait(bar(G_EMPTY + b), phase, gave_up);  // (a failed wait is reported at the end; nothing depends on it here)
+            if (c < c_hi || c >= c_lo + 2) mbar_wait(bar(G_EMPTY + b), phase, gave_up);  // (a failed wait is reported at the end)
             if (b) phase ^= 1u;
+            if (c >= c_lo + 2) {  // the products of chunk c - 2 are complete
+                fence_after();
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float d[16];
+                    tmem_load_16x32(pl.tmem(tmem, 128 * b, half), d);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) acc[half][i] += d[i];
+                }
+                fence_before();
+            }
+            if (c >= c_hi) continue;
+            if (with_bias) {
+                add((gv[0].x + gv[1].x) + (gv[2].x + gv[3].x), sums.x, lost.x);
+                add((gv[0].y + gv[1].y) + (gv[2].y + gv[3].y), sums.y, lost.y);
+                add((gv[0].z + gv[1].z) + (gv[2].z + gv[3].z), sums.z, lost.z);
+                add((gv[0].w + gv[1].w) + (gv[2].w + gv[3].w), sums.w, lost.w);
+            }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int row = 4 * warp + u;
@@ -585,44 +629,35 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
                 split3(xv[u].z, xv[u].w, hi);
 #pragma unroll
                 for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2 *>(xb + i * GR_PIECE + at) = make_uint2(lo[i], hi[i]);
-                if (with_bias) { sums.x += gv[u].x; sums.y += gv[u].y; sums.z += gv[u].z; sums.w += gv[u].w; }
             }
             fence_async_smem();
             mbar_arrive(bar(G_FULL + b));
             fetch(c + 1);
         }
         float4 *mine = reinterpret_cast<float4 *>(smem_tc + GR_MISC + 64) + warp * 32 + lane;
-        *mine = sums;
-        // the accumulator: thread = 4 rows x 8 columns, as in the chain kernels
-        mbar_wait(bar(G_DONE), 0, gave_up);
-        fence_after();
+        *mine = make_float4(sums.x + lost.x, sums.y + lost.y, sums.z + lost.z, sums.w + lost.w);
     }
     __syncthreads();
     if (warp < 16) {
-        const Place pl;
         float *out = partial + ((size_t)blockIdx.x * splits + blockIdx.y) * GRAD_PARTIAL;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float d[16];
-            tmem_load_16x32(pl.tmem(tmem, 0, half), d);
-            if (c_lo >= c_hi) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) d[i] = 0.f;
-            }
-            store_rows(out, 128, 0, 128, pl, half, d);
-        }
+        for (int half = 0; half < 2; ++half) store_rows(out, 128, 0, 128, pl, half, acc[half]);
         if (job.bias != nullptr && threadIdx.x < 128) {
             const float *col = reinterpret_cast<const float *>(smem_tc + GR_MISC + 64) + threadIdx.x;
-            float t = 0.f;
+            float t[16];
 #pragma unroll
-            for (int w = 0; w < 16; ++w) t += col[128 * w];
-            out[128 * 128 + threadIdx.x] = t;
+            for (int w = 0; w < 16; ++w) t[w] = col[128 * w];
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int w = 0; w < o; ++w) t[w] += t[w + o];
+            out[128 * 128 + threadIdx.x] = t[0];
         }
     }
     fence_before();
     __syncthreads();
     fence_after();
-    if (warp == 16) tmem_free<128>(tmem);
+    if (warp == 16) tmem_free<256>(tmem);
     if (threadIdx.x == 0 && *gave_up != 0u) atomicOr(&g_dense_backward_status, 1u);
 }
 
