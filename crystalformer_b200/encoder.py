@@ -213,7 +213,8 @@ class CrystalformerEncoderCUDA(Module):
         if self.norm is not None or self.d_model != 128 or self.nhead != 8:
             return False
         for layer in self.layers:
-            att, P = layer.self_attn, layer.self_attn.params
+            att = layer.self_attn
+            P = att.params
             if not (P.domain in domains and P.positive_func.startswith("elu") and P.gauss_state == "q" and P.normalize_gauss and att.fused
                     and P.value_pe_condproj == "no" and P.norm_func_mode == 0 and att.kdim == 128 and att.vdim == 128
                     and att.in_proj_bias is not None and layer.activation is F.relu and not layer.norm_first

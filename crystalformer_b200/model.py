@@ -128,10 +128,12 @@ class Latticeformer(nn.Module):
         """Whether embedding, pooling and head are what the one-call paths implement (inference and training)."""
         if not getattr(self, "native", True) or self.pooling != "avr" or isinstance(self.proj_before_pooling, nn.Module):
             return False
-        m = self.mlp
-        if not (len(m) == 4 and isinstance(m[0], nn.Linear) and isinstance(m[1], nn.Identity)
-                and isinstance(m[2], nn.ReLU) and isinstance(m[3], nn.Linear) and m[0].in_features == 128
-                and m[0].out_features <= 1024 and m[0].bias is not None and m[3].bias is not None):
+        m = list(self.mlp)
+        if len(m) != 4:
+            return False
+        first, norm, act, last = m
+        if not (isinstance(first, nn.Linear) and isinstance(norm, nn.Identity) and isinstance(act, nn.ReLU) and isinstance(last, nn.Linear)
+                and first.in_features == 128 and first.out_features <= 1024 and first.bias is not None and last.bias is not None):
             return False
         return self.input_embeddings.out_features == 128 and self.encoder.native
 

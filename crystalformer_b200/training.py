@@ -7,11 +7,12 @@ operation-by-operation autograd path (models/latticeformer.py:211-302 and its ba
 from __future__ import annotations
 
 import ctypes
+from operator import is_
 from typing import Optional, Tuple
 
 import numpy as np
 import torch
-from torch.autograd.forward_ad import unpack_dual
+from torch.autograd import forward_ad
 
 from . import _lib
 
@@ -35,9 +36,10 @@ class ModelWatch:
     (with ``versions``) modified in place, or a setting changed."""
 
     def __init__(self, model, versions: bool):
-        self.children = [(m._modules, n, c) for m in model.modules() for n, c in m._modules.items()]
-        self.places = [(d, n, t) for m in model.modules() for d in (m._parameters, m._buffers) for n, t in d.items() if t is not None]
-        self.tensors = [t for _, _, t in self.places]
+        children = [(m._modules, n, c) for m in model.modules() for n, c in m._modules.items()]
+        places = [(d, n, t) for m in model.modules() for d in (m._parameters, m._buffers) for n, t in d.items() if t is not None]
+        self.tensors = [t for _, _, t in places]
+        self.dicts, self.names, self.values = zip(*(children + places))
         self.versions = versions
         self.settings = model.encoder.lattice_params
         self.layer_settings = [layer.self_attn.params for layer in model.encoder.layers]
@@ -52,12 +54,11 @@ class ModelWatch:
         for Q in self.layer_settings:
             key += (Q.positive_func, Q.gauss_lb_real, Q.scale_real, Q.value_pe_dist_max, Q.gauss_lb_reci, Q.scale_reci)
         key += [m.p for m in self.dropouts] + [m.dropout for m in self.attentions]
-        key += [t.data_ptr() for t in self.tensors]
+        key += map(torch.Tensor.data_ptr, self.tensors)
         return key + [t._version for t in self.tensors] if self.versions else key
 
     def current(self) -> bool:
-        return all([d.get(n) is c for d, n, c in self.children]) and all([d.get(n) is t for d, n, t in self.places]) \
-            and self.now() == self.key
+        return all(map(is_, map(dict.get, self.dicts, self.names), self.values)) and self.now() == self.key
 
 
 DOMAINS = ("real", "reci", "RECI", "multihead")  # in the order of the library's codes
@@ -95,14 +96,13 @@ class TrainPlan:
             offsets.append(at)
             at += n
         self.floats = at
-        self.like = [p.detach() for p in self.params]
+        self.like = [p.detach() for p in self.params]  # (and keeps the storage that the addresses name)
         where = iter(range(len(self.params)))
         self.slots = [None if p is None else next(where) for p in ordered]
         # the gradients' places as byte offsets in the library's order (0 and not `present` for a parameter that is not there)
         self.present = np.array([s is not None for s in self.slots], dtype=np.int64)
         self.offsets = np.array([0 if s is None else 4 * offsets[s] for s in self.slots], dtype=np.int64)
-        self.addresses = [p.data_ptr() for p in self.params]
-        self.pointers = self.table(self.addresses)
+        self.pointers = (ctypes.c_void_p * len(ordered))(*[None if p is None else p.data_ptr() for p in ordered])
         self.scalars = (ctypes.c_double * len(scalars))(*scalars)
         self.targets = model.mlp[3].out_features
         order_reach = model.native_reach()
@@ -112,22 +112,6 @@ class TrainPlan:
             K=int(P.value_pe_dist_real), ff_dim=enc.layers[0].linear1.out_features, hidden=model.mlp[0].out_features,
             targets=self.targets, wscale=float(P.value_pe_width_scale), cutoff_radius=enc._cutoff(), order_reach=order_reach,
             weights=ctypes.cast(self.pointers, ctypes.c_void_p), scalars=ctypes.cast(self.scalars, ctypes.c_void_p))
-
-    def table(self, addresses):
-        """Addresses of the parameters, one after the other, as the library's array with its empty places."""
-        return (ctypes.c_void_p * len(self.slots))(*[None if s is None else addresses[s] for s in self.slots])
-
-    def desc_now(self) -> _lib.TrainDesc:
-        """The description with the parameters where they lie now: their storage may have been replaced since the forward."""
-        addresses = [p.data_ptr() for p in self.params]
-        if addresses == self.addresses:
-            return self.desc
-        if not all(p.shape == q.shape and usable(p, q.device) for p, q in zip(self.params, self.like)):
-            raise RuntimeError("a parameter of the model was moved or changed its type between the forward and the backward of a training step")
-        desc = _lib.TrainDesc.from_buffer_copy(self.desc)
-        desc.keep = self.table(addresses)
-        desc.weights = ctypes.cast(desc.keep, ctypes.c_void_p)
-        return desc
 
     def current(self) -> bool:
         return self.watch.current() and [g._version for g in self.scales] == self.scale_versions
@@ -222,9 +206,8 @@ class TrainStep(torch.autograd.Function):
                                "backward of a training step")
         dev = gy.device
         gy = gy.contiguous()
-        desc = plan.desc_now()
-        batch = _lib.TrainBatch(features=feats.data_ptr(), trans=trans.data_ptr(), N=N, B=B, E=E, max_atoms=max_atoms,
-                                saved=saved.data_ptr(), saved_edges=edges.data_ptr())
+        desc = plan.desc
+        batch = _lib.TrainBatch(feats.data_ptr(), None, trans.data_ptr(), None, N, B, E, max_atoms, saved.data_ptr(), edges.data_ptr())
         scratch = torch.empty(int(_lib.load().cf_train_scratch_bytes(ctypes.byref(desc), N, B, E)), dtype=torch.uint8, device=dev)
         flat = torch.empty(plan.floats, dtype=torch.float32, device=dev)
         where = plan.offsets + flat.data_ptr() * plan.present
@@ -243,9 +226,10 @@ def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[
             return None
         plan = TrainPlan(model)
         model._train_plan = OfThisModel(plan)
-    if not plan.untouched() or not all(layer.self_attn.term_lists for layer in model.encoder.layers):
+    if not plan.untouched() or not all([att.term_lists for att in plan.watch.attentions]):
         return None
-    if any(t.requires_grad or unpack_dual(t).tangent is not None for t in (data.x, data.pos, data.trans_vec)) or torch.is_autocast_enabled():
+    if data.x.requires_grad or data.pos.requires_grad or data.trans_vec.requires_grad or torch.is_autocast_enabled() \
+            or forward_ad._current_level >= 0:  # (forward-mode derivatives are on: an input may carry a tangent)
         return None
     # the kernels get addresses: what does not have the model's shapes, or lies elsewhere, is left to the operators' own checks
     dev, sizes = data.pos.device, data.sizes
