@@ -94,6 +94,14 @@ __device__ __forceinline__ float warp_sum(float v)
     return v;
 }
 
+// sum += v with what the rounding dropped kept in `low` (two-sum): long sums of one thread, sum + low at the end.
+__device__ __forceinline__ void add_compensated(float v, float &sum, float &low)
+{
+    const float t = __fadd_rn(sum, v), back = __fsub_rn(t, sum);
+    low += __fadd_rn(__fsub_rn(sum, __fsub_rn(t, back)), __fsub_rn(v, back));
+    sum = t;
+}
+
 // Picks x[idx] from eight registers without dynamic indexing.
 __device__ __forceinline__ float pick8(const float (&x)[8], int idx)
 {

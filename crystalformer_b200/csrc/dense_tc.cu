@@ -55,7 +55,7 @@ struct WeightScales {
         if (p.weights_fresh) grid_dependency_wait();
         if (p.tail != nullptr) {
             const float *inv = reinterpret_cast<const float *>(p.tail);
-            first = inv[0]; w1 = inv[1]; w2 = inv[2 * chunks];
+            first = inv[0] * GIVEN_BACK; w1 = inv[1] * GIVEN_BACK; w2 = inv[2 * chunks] * GIVEN_BACK;
             for (int i = threadIdx.x; i < p.ff; i += EPI_THREADS) b1_max = fmaxf(b1_max, fabsf(p.b1[i]));
             b1_max = warp_max(b1_max);
             if ((threadIdx.x & 31) == 0) s.warp_floats()[threadIdx.x >> 5] = b1_max;
@@ -64,7 +64,7 @@ struct WeightScales {
             for (int w = 0; w < EPI_WARPS; ++w) b1_max = fmaxf(b1_max, s.warp_floats()[w]);
         }
         if (p.embed != nullptr) first = *reinterpret_cast<const float *>(p.embed);
-        if (p.head != nullptr) head = reinterpret_cast<const float *>(p.head)[1 + 2 * chunks];
+        if (p.head != nullptr) head = reinterpret_cast<const float *>(p.head)[1 + 2 * chunks] * GIVEN_BACK;
     }
 };
 
@@ -82,16 +82,11 @@ __device__ __forceinline__ void first_rows(const DenseForward &p, const Shared &
     fence_async_smem();
     fence_before();
     mbar_arrive(s.bar(B_A0));
-    if (tail) {  // the residual and its bias arrive during the product
+    float2 bias[4];
+    if (tail) {  // the residual and the bias arrive during the product
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 b = *reinterpret_cast<const float2 *>(p.bo + pl.col0 + 8 * j);
-                x[half][4 * j] += b.x; x[half][4 * j + 1] += b.y; x[half][4 * j + 2] += b.x; x[half][4 * j + 3] += b.y;
-            }
-        }
+        for (int half = 0; half < 2; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+        load_columns(p.bo, pl, bias);
     }
     epilogue_sync();  // (the loading warps' scales)
     float xi[4];
@@ -106,7 +101,7 @@ __device__ __forceinline__ void first_rows(const DenseForward &p, const Shared &
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const float sc = xi[2 * half + ((i >> 1) & 1)] * w_i;
-            x[half][i] = tail ? fmaf(d[i], sc, x[half][i]) : d[i] * sc;
+            x[half][i] = tail ? x[half][i] + fmaf(d[i], sc, (i & 1) ? bias[i >> 2].y : bias[i >> 2].x) : d[i] * sc;
         }
     }
 }
@@ -224,8 +219,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             Producer<STAGES> pr;
             for (long long tile = blockIdx.x; tile < tiles && pr.ok; tile += gridDim.x) {
                 if (tail) pr.stream(s, p.tail, 0, 1 + 2 * chunks);
-                else if (embed) pr.stream(s, p.embed, 0, 1);
-                if (head) pr.stream(s, p.head, 1 + 2 * chunks, 3);
+                else if (embed) pr.stream(s, p.embed, 0, 1, TC_EMBED_PIECES);
+                if (head && pr.ok) pr.stream(s, p.head, 1 + 2 * chunks, 3);
             }
             if (!pr.ok) pr.drain(s);
         }
@@ -238,31 +233,30 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
                 bool ok = true;
                 auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
-                auto product = [&](int d, int a, bool acc, int done) {
-                    if (ok) is.product(s, tmem, d, a, acc);
+                auto product = [&](int d, int a, int done, int pieces = 2) {
+                    if (ok) is.product(s, tmem, d, a, pieces);
                     ok = ok && is.ok;
                     mma_commit(s.bar(done));
                 };
                 if (tail || embed) {
                     ready(B_A0);
-                    product(D0, OFF_A0, false, B_D0);
+                    product(D0, OFF_A0, B_D0, tail ? 2 : TC_EMBED_PIECES);
                 }
                 if (tail) {
                     ready(B_A0);
-                    product(D0, OFF_A0, false, B_D0);
-                    if (chunks > 1) product(D1, OFF_A0, false, B_D1);
+                    product(D0, OFF_A0, B_D0);
+                    if (chunks > 1) product(D1, OFF_A0, B_D1);
                     for (int c = 0; c < chunks && ok; ++c) {
                         ready(B_A1);
-                        product(DX, OFF_A1, c > 0, B_A1_FREE);
-                        if (c + 1 == chunks) mma_commit(s.bar(B_DX));
-                        if (c + 2 < chunks) product((c & 1) ? D1 : D0, OFF_A0, false, (c & 1) ? B_D1 : B_D0);
+                        product((c & 1) ? DY : DX, OFF_A1, B_A1_FREE);
+                        if (c + 2 < chunks) product((c & 1) ? D1 : D0, OFF_A0, (c & 1) ? B_D1 : B_D0);
                     }
                 }
                 if (head) {
                     ready(B_A0);
-                    product(D0, OFF_A0, false, B_D0);
-                    product(D1, OFF_A0, false, B_D1);
-                    product(DX, OFF_A0, false, B_DX);
+                    product(D0, OFF_A0, B_D0);
+                    product(D1, OFF_A0, B_D1);
+                    product(DX, OFF_A0, B_DX);
                 }
                 is.ok = is.ok && ok;
             }
@@ -281,31 +275,36 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             first_rows(p, s, pl, ph, tmem, row_base, ws.first, x);
             if (tail) {
                 publish_rows(s, pl, x, xi);  // y
-                if (p.y_save != nullptr) {
+                // (y lies in memory while the registers take the sum of the chunks, whose hidden units share their scales)
+                float *y_rows = p.y_save != nullptr ? p.y_save : p.x_out;
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) store_rows(p.y_save, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < 2; ++half) {
+                    store_rows(y_rows, 128, row_base, p.N, pl, half, x[half]);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) x[half][i] = 0.f;
                 }
                 float hs[4], hi[4];
                 hidden_scales(ws, xi, hs, hi);
-                for (int c = 0; c < chunks; ++c)
+                for (int c = 0; c < chunks; ++c) {
                     hidden_units(p, s, pl, ph, tmem, (c & 1) ? D1 : D0, (c & 1) ? B_D1 : B_D0, c, row_base, xi, ws.w1, hs, OFF_A1, B_A1, c > 0);
+                    if (c > 0) add_accumulator(pl, tmem, (c & 1) ? DX : DY, x);  // of chunk c - 1, beside chunk c's product
+                }
                 float2 bias[4];
                 load_columns(p.b2, pl, bias);
                 ph.wait(s, B_A1_FREE);
-                ph.wait(s, B_DX);
-                fence_after();
+                add_accumulator(pl, tmem, (chunks & 1) ? DX : DY, x);
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    float d[16];
-                    tmem_load_16x32(pl.tmem(tmem, DX, half), d);
+                    float y[16];
+                    load_rows(y_rows, 128, row_base, p.N, pl, half, y);
                     const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float2 b = bias[j];
-                        x[half][4 * j] += fmaf(d[4 * j], sa, b.x);
-                        x[half][4 * j + 1] += fmaf(d[4 * j + 1], sa, b.y);
-                        x[half][4 * j + 2] += fmaf(d[4 * j + 2], sb, b.x);
-                        x[half][4 * j + 3] += fmaf(d[4 * j + 3], sb, b.y);
+                        x[half][4 * j] = y[4 * j] + fmaf(x[half][4 * j], sa, b.x);
+                        x[half][4 * j + 1] = y[4 * j + 1] + fmaf(x[half][4 * j + 1], sa, b.y);
+                        x[half][4 * j + 2] = y[4 * j + 2] + fmaf(x[half][4 * j + 2], sb, b.x);
+                        x[half][4 * j + 3] = y[4 * j + 3] + fmaf(x[half][4 * j + 3], sb, b.y);
                     }
                 }
             }
@@ -346,7 +345,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
         if (lane == 0) {
             Producer<SPLIT_STAGES> pr;
             if (tail) pr.stream(s, p.tail, 0, 1);
-            else if (embed) pr.stream(s, p.embed, 0, 1);
+            else if (embed) pr.stream(s, p.embed, 0, 1, TC_EMBED_PIECES);
             if (has_chunk && pr.ok) pr.stream(s, p.tail, 1 + first_of_chunk(rank), 1);
             if (has_chunk && pr.ok) pr.stream(s, p.tail, 1 + second_of_chunk(rank, chunks), 1);
             if (has_head && pr.ok) pr.stream(s, p.head, 1 + 2 * chunks + (int)rank, 1);
@@ -361,21 +360,21 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
             Phase ph;
             bool ok = true;
             auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
-            auto product = [&](int d, bool use, int done) {
-                if (ok && use) is.product(s, tmem, d, OFF_A0, false);
+            auto product = [&](int d, int done, int pieces = 2) {
+                if (ok) is.product(s, tmem, d, OFF_A0, pieces);
                 ok = ok && is.ok;
                 mma_commit(s.bar(done));
             };
             if (tail || embed) {
                 ready(B_A0);
-                product(D0, true, B_D0);
+                product(D0, B_D0, tail ? 2 : TC_EMBED_PIECES);
             }
             if (tail) {
                 ready(B_A0);
                 if (has_chunk) {
-                    product(D0, true, B_D0);
+                    product(D0, B_D0);
                     ready(B_A0);
-                    product(DX, true, B_DX);
+                    product(DX, B_DX);
                 }
             }
             if (has_head) {
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
                 } else {
                     ready(B_A0);
                 }
-                product(D1, true, B_D1);
+                product(D1, B_D1);
             }
             if (!ok) is.drain(s);
         }
@@ -404,6 +403,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
         float x[2][16], xi[4];
         first_rows(p, s, pl, ph, tmem, row_base, ws.first, x);
         if (tail) {
+            if (mine) {  // (read back by the threads that finish the rows, behind the barriers of publish_rows)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) stage_rows(s.mem + OFF_OWN, pl, half, x[half]);
+            }
             publish_rows(s, pl, x, xi);  // y
             if (p.y_save != nullptr && mine) {
 #pragma unroll
@@ -412,8 +415,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
             float hs[4], hi[4];
             hidden_scales(ws, xi, hs, hi);
             if (has_chunk) hidden_units(p, s, pl, ph, tmem, D0, B_D0, rank, row_base, xi, ws.w1, hs, OFF_A0, B_A0, false);
-            float2 bias[4];
-            load_columns(p.b2, pl, bias);
+            const float2 b2_lo = *reinterpret_cast<const float2 *>(p.b2 + 4 * lane), b2_hi = *reinterpret_cast<const float2 *>(p.b2 + 4 * lane + 2);
             if (has_chunk) {
                 ph.wait(s, B_DX);
                 fence_after();
@@ -431,18 +433,21 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
                 }
                 const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {  // (the finishing block's own share carries y and the bias)
-                    const float2 b = bias[j];
-                    d[4 * j] = fmaf(d[4 * j], sa, mine ? x[half][4 * j] + b.x : 0.f);
-                    d[4 * j + 1] = fmaf(d[4 * j + 1], sa, mine ? x[half][4 * j + 1] + b.y : 0.f);
-                    d[4 * j + 2] = fmaf(d[4 * j + 2], sb, mine ? x[half][4 * j + 2] + b.x : 0.f);
-                    d[4 * j + 3] = fmaf(d[4 * j + 3], sb, mine ? x[half][4 * j + 3] + b.y : 0.f);
+                for (int j = 0; j < 4; ++j) {
+                    d[4 * j] *= sa; d[4 * j + 1] *= sa;
+                    d[4 * j + 2] *= sb; d[4 * j + 3] *= sb;
                 }
                 stage_share(s, pl, half, d);
             }
             send_share(s, rank);
             float4 v[2];
             collect_shares(s, ph, v);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float4 y = staged_row(s.mem + OFF_OWN, 2 * warp + u, lane);
+                v[u].x = y.x + (v[u].x + b2_lo.x); v[u].y = y.y + (v[u].y + b2_lo.y);
+                v[u].z = y.z + (v[u].z + b2_hi.x); v[u].w = y.w + (v[u].w + b2_hi.y);
+            }
             if (head) spread_rows(s, ph, rank, v, 3, 0);
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -513,14 +518,18 @@ __global__ void __launch_bounds__(PACK_THREADS) dense_pack_kernel(const PackJob 
             const int k = k0 + u;
             v[u] = (n < b.rows && k < b.cols) ? (b.trans ? b.src[(size_t)k * b.ld + n] : b.src[(size_t)n * b.ld + k]) * sc : 0.f;
         }
-        uint4 h0, h1;
-        split_pair(v[0], v[1], h0.x, h1.x);
-        split_pair(v[2], v[3], h0.y, h1.y);
-        split_pair(v[4], v[5], h0.z, h1.z);
-        split_pair(v[6], v[7], h0.w, h1.w);
-        unsigned char *at = out + (k0 >> 6) * STAGE_BYTES + n * 128 + ((((k0 & 63) >> 3) ^ (n & 7)) << 4);
-        *reinterpret_cast<uint4 *>(at) = h0;
-        *reinterpret_cast<uint4 *>(at + 16384) = h1;
+        uint4 h0, h1, h2;
+        split_three(v[0], v[1], h0.x, h1.x, h2.x);
+        split_three(v[2], v[3], h0.y, h1.y, h2.y);
+        split_three(v[4], v[5], h0.z, h1.z, h2.z);
+        split_three(v[6], v[7], h0.w, h1.w, h2.w);
+        unsigned char *at = out + (k0 >> 6) * (TC_PIECE_BYTES / 2) + n * 128 + ((((k0 & 63) >> 3) ^ (n & 7)) << 4);
+        if (b.pieces == 3) {
+            *reinterpret_cast<uint4 *>(at) = h2;
+            at += TC_PIECE_BYTES;
+        }
+        *reinterpret_cast<uint4 *>(at) = h1;
+        *reinterpret_cast<uint4 *>(at + TC_PIECE_BYTES) = h0;
     }
 }
 
@@ -554,7 +563,7 @@ static PackBlock &pack_add(PackJob &job, int &count, unsigned char *image, int b
 {
     PackBlock &b = job.b[count++];
     b = PackBlock{};
-    b.src = src; b.ld = ld; b.trans = (short)trans; b.rows = 128; b.cols = 128; b.block = (short)block; b.image = image;
+    b.src = src; b.ld = ld; b.trans = (short)trans; b.rows = 128; b.cols = 128; b.block = (short)block; b.pieces = 2; b.image = image;
     return b;
 }
 
@@ -606,13 +615,14 @@ void pack_embedding(PackJob &job, int &count, unsigned char *image, const float 
 {
     PackBlock &b = pack_add(job, count, image, 0, W, feature_dim, 0);
     b.cols = (short)feature_dim;
+    b.pieces = TC_EMBED_PIECES;
     b.group[0] = W;
     b.group_elems = 128 * feature_dim;
 }
 
 }  // namespace cf
 
-extern "C" int64_t cf_dense_image_bytes(int64_t ff_dim) { return (int64_t)cf::tc_image_bytes(ff_dim > 0 ? cf::tc_layer_blocks((int)ff_dim) : 1); }
+extern "C" int64_t cf_dense_image_bytes(int64_t ff_dim) { return (int64_t)(ff_dim > 0 ? cf::tc_image_bytes(cf::tc_layer_blocks((int)ff_dim)) : cf::TC_EMBED_BYTES); }
 
 extern "C" int cf_dense_pack_layer(const float *Wq, const float *Wk, const float *Wv, const float *Wo, const float *W1,
                                    const float *W2, int64_t ff_dim, void *image, void *stream)

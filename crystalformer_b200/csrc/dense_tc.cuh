@@ -7,11 +7,16 @@
 namespace cf {
 
 // Weight images.  A layer's projections are cut into 128 x 128 blocks; a block is 64 KB, the shared-memory image that
-// the tensor instruction reads: two 64-deep k panels, each { h0, h1 } of 128 rows x 128 bytes with the 128-byte swizzle
-// (tc5.cuh), so that a stage of the weight stream is one contiguous 32 KB copy.  Blocks are stored in the order in
-// which the kernel consumes them; in front of them 1 KB of scales (float, 1 / s of every block).
-constexpr int TC_BLOCK_BYTES = 65536;
+// the tensor instruction reads: the pieces h1 and h0 (tc5.cuh) one after the other, each two 64-deep k panels of 128 rows x
+// 128 bytes with the 128-byte swizzle, so that a stage of the weight stream is one contiguous 32 KB copy of one piece, the
+// small one first (Issuer::product).  Blocks are stored in the order in which the kernel consumes them; in front of them
+// 1 KB of scales (float, 1 / s of every block).  The embedding has a third piece in front, so that an element's row comes
+// out as the weight's column bit for bit.
+constexpr int TC_PIECE_BYTES = 32768;
+constexpr int TC_BLOCK_BYTES = 2 * TC_PIECE_BYTES;
 constexpr int TC_HEADER_BYTES = 1024;
+constexpr int TC_EMBED_PIECES = 3;
+constexpr size_t TC_EMBED_BYTES = TC_HEADER_BYTES + TC_EMBED_PIECES * TC_PIECE_BYTES;
 inline size_t tc_image_bytes(int blocks) { return (size_t)TC_HEADER_BYTES + (size_t)blocks * TC_BLOCK_BYTES; }
 inline int tc_tail_blocks(int ff) { return 1 + 2 * (ff / 128); }  // Wo, then W1 / W2 chunks interleaved
 inline int tc_layer_blocks(int ff) { return tc_tail_blocks(ff) + 3; }
@@ -22,6 +27,7 @@ struct PackBlock {
     const float *src, *group[3];
     int group_elems, ld;
     short rows, cols, trans, block;   // block: index in the image
+    int pieces;
     unsigned char *image;
 };
 constexpr int PACK_MAX = 56;                          // blocks of one launch (the job is a kernel parameter)

@@ -99,30 +99,29 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
                 bool ok = true;
                 auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
-                auto product = [&](int d, int a, bool acc, int done) {
-                    if (ok) is.product(s, tmem, d, a, acc);
+                auto product = [&](int d, int a, int done) {
+                    if (ok) is.product(s, tmem, d, a);
                     ok = ok && is.ok;
                     if (done >= 0) mma_commit(s.bar(done));
                 };
                 if (head) {
-                    ready(B_A0);                            // gq' and gk
-                    product(D0, OFF_A0, false, B_D0);       // (operand 0 is free again)
-                    product(D0, OFF_A1, true, -1);
-                    ready(B_A0);                            // gv
-                    product(D0, OFF_A0, true, B_D0);
+                    ready(B_A0);                     // gq' and gk
+                    product(D0, OFF_A0, B_D0);       // (operand 0 is free again)
+                    product(D1, OFF_A1, -1);
+                    ready(B_A0);                     // gv
+                    product(DX, OFF_A0, B_D0);
                 }
                 if (tail) {
                     ready(B_A0);
-                    product(D0, OFF_A0, false, B_D0);
-                    if (chunks > 1) product(D1, OFF_A0, false, B_D1);
+                    product(D0, OFF_A0, B_D0);
+                    if (chunks > 1) product(D1, OFF_A0, B_D1);
                     for (int c = 0; c < chunks && ok; ++c) {
                         ready(B_A1);
-                        product(DX, OFF_A1, c > 0, B_A1_FREE);
-                        if (c + 1 == chunks) mma_commit(s.bar(B_DX));
-                        if (c + 2 < chunks) product((c & 1) ? D1 : D0, OFF_A0, false, (c & 1) ? B_D1 : B_D0);
+                        product((c & 1) ? DY : DX, OFF_A1, B_A1_FREE);
+                        if (c + 2 < chunks) product((c & 1) ? D1 : D0, OFF_A0, (c & 1) ? B_D1 : B_D0);
                     }
                     ready(B_A0);
-                    product(D0, OFF_A0, false, B_D0);
+                    product(D0, OFF_A0, B_D0);
                 }
                 is.ok = is.ok && ok;
             }
@@ -131,11 +130,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
     } else {
         const Place pl;
         unsigned char *A0 = s.mem + OFF_A0, *A1 = s.mem + OFF_A1;
-        const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] : 0.f;
+        const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] * GIVEN_BACK : 0.f;
         float w2_i = 0.f, w1_i = 0.f, wo_i = 0.f;
         if (tail) {
             const float *inv = reinterpret_cast<const float *>(p.tail);
-            w2_i = inv[3]; w1_i = inv[3 + 2 * chunks - 1]; wo_i = inv[3 + 2 * chunks];
+            w2_i = inv[3] * GIVEN_BACK; w1_i = inv[3 + 2 * chunks - 1] * GIVEN_BACK; wo_i = inv[3 + 2 * chunks] * GIVEN_BACK;
         }
         Phase ph;
         for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -145,7 +144,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             float xi[4];
             if (head) {
                 // ---- gq' and gk as operands 0 and 1, with one scale per row for the three of them (their products meet in
-                //      one accumulator); warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (head l / 4)
+                //      one sum); warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (head l / 4)
                 const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
                 float *inv_out = s.row_floats(0);
                 const uint32_t lane_at = (lane >> 4) * 16384 + (lane & 1) * 8;
@@ -218,10 +217,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 fence_after();
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    float d[16];
+                    float d[16], e[16];
                     tmem_load_16x32(pl.tmem(tmem, D0, half), d);
+                    tmem_load_16x32(pl.tmem(tmem, D1, half), e);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) x[half][i] = fmaf(d[i], xi[2 * half + ((i >> 1) & 1)] * wh_i, x[half][i]);
+                    for (int i = 0; i < 16; ++i) d[i] += e[i];
+                    tmem_load_16x32(pl.tmem(tmem, DX, half), e);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) x[half][i] = fmaf(d[i] + e[i], xi[2 * half + ((i >> 1) & 1)] * wh_i, x[half][i]);
                     store_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
                 }
             } else {
@@ -229,22 +232,27 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 for (int half = 0; half < 2; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!tail) continue;
-            publish_rows(s, pl, x, xi);  // gx
+            publish_rows(s, pl, x, xi);  // gx (read again from memory behind the chunks, whose sum takes its registers)
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[half][i] = 0.f;
             // ---- hidden units: one scale per row for all chunks, |gh| <= 128 max|gx| max|W2| (see the forward)
             float hs[4], hi[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) hs[i] = power_of_two(137438953472.0f * xi[i] * w2_i, hi[i]);
-            for (int c = 0; c < chunks; ++c)
+            for (int c = 0; c < chunks; ++c) {
                 hidden_grads(p, s, pl, ph, tmem, (c & 1) ? D1 : D0, (c & 1) ? B_D1 : B_D0, c, row_base, xi, w2_i, hs, OFF_A1, B_A1, c > 0);
+                if (c > 0) add_accumulator(pl, tmem, (c & 1) ? DX : DY, x);  // of chunk c - 1, beside chunk c's product
+            }
             ph.wait(s, B_A1_FREE);
-            ph.wait(s, B_DX);
-            fence_after();
+            add_accumulator(pl, tmem, (chunks & 1) ? DX : DY, x);
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                float d[16];
-                tmem_load_16x32(pl.tmem(tmem, DX, half), d);
+                float g[16];
+                load_rows(p.gx, 128, row_base, p.N, pl, half, g);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) x[half][i] = fmaf(d[i], hi[2 * half + ((i >> 1) & 1)] * w1_i, x[half][i]);
+                for (int i = 0; i < 16; ++i) x[half][i] = fmaf(x[half][i], hi[2 * half + ((i >> 1) & 1)] * w1_i, g[i]);
             }
             publish_rows(s, pl, x, xi);  // gy
 #pragma unroll
@@ -304,7 +312,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(
                 fence_after();
             };
             auto product = [&](int d, int done) {
-                if (ok) is.product(s, tmem, d, OFF_A0, false);
+                if (ok) is.product(s, tmem, d, OFF_A0);
                 ok = ok && is.ok;
                 mma_commit(s.bar(done));
             };
@@ -329,11 +337,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(
         __syncwarp();
     } else {
         const Place pl;
-        const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] : 0.f;
+        const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] * GIVEN_BACK : 0.f;
         float w2_i = 0.f, w1_i = 0.f, wo_i = 0.f;
         if (tail) {
             const float *inv = reinterpret_cast<const float *>(p.tail);
-            w2_i = inv[3]; w1_i = inv[3 + 2 * chunks - 1]; wo_i = inv[3 + 2 * chunks];
+            w2_i = inv[3] * GIVEN_BACK; w1_i = inv[3 + 2 * chunks - 1] * GIVEN_BACK; wo_i = inv[3 + 2 * chunks] * GIVEN_BACK;
         }
         Phase ph;
         float xi[4];
@@ -588,11 +596,6 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
         };
         fetch(c_lo);
         float4 sums = make_float4(0.f, 0.f, 0.f, 0.f), lost = sums;  // column sums of g, and what their roundings dropped
-        auto add = [](float v, float &sum, float &low) {  // (compensated: the rows of a share are thousands)
-            const float t = sum + v, back = t - sum;
-            low += (sum - (t - back)) + (v - back);
-            sum = t;
-        };
         for (long long c = c_lo; c < c_hi + 2; ++c) {  // (the last two only collect)
             const int b = (int)((c - c_lo) & 1);
             unsigned char *gb = smem_tc + b * GR_BUFFER + lane_at, *xb = gb + 3 * GR_PIECE;
@@ -611,10 +614,10 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
             }
             if (c >= c_hi) continue;
             if (with_bias) {
-                add((gv[0].x + gv[1].x) + (gv[2].x + gv[3].x), sums.x, lost.x);
-                add((gv[0].y + gv[1].y) + (gv[2].y + gv[3].y), sums.y, lost.y);
-                add((gv[0].z + gv[1].z) + (gv[2].z + gv[3].z), sums.z, lost.z);
-                add((gv[0].w + gv[1].w) + (gv[2].w + gv[3].w), sums.w, lost.w);
+                add_compensated((gv[0].x + gv[1].x) + (gv[2].x + gv[3].x), sums.x, lost.x);
+                add_compensated((gv[0].y + gv[1].y) + (gv[2].y + gv[3].y), sums.y, lost.y);
+                add_compensated((gv[0].z + gv[1].z) + (gv[2].z + gv[3].z), sums.z, lost.z);
+                add_compensated((gv[0].w + gv[1].w) + (gv[2].w + gv[3].w), sums.w, lost.w);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {

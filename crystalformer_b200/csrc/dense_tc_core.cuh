@@ -4,10 +4,18 @@
 // A thread block carries a tile of 128 atom rows through its chain of products.  Warps 0-15 are the epilogue warps
 // (thread = 4 rows x 8 columns of a 128 x 128 accumulator, in the layout of tmem_load_16x32: warp w covers rows
 // 32 (w % 4) .., columns 32 (w / 4) ..; with eight warps an epilogue took 2 us instead of 1), one thread of warp 16
-// issues the tensor instructions, one thread of warp 17 streams the weight images through a ring of three 32 KB stages.  Operands: two 64 KB buffers in shared memory, each
-// { h0, h1 } of two 64-deep k panels.  A product of two-piece operands is three fp16 products, h0 h1 + h1 h0 + h0 h0
-// (h1 h1 is below 2^-22 of the result), accumulated in fp32 in tensor memory: error about 2^-22 per term, less than the
-// 2^-20 of the TF32 + bfloat16 split of the warp-level version.
+// issues the tensor instructions, one thread of warp 17 streams the weight images through a ring of three 32 KB stages.
+// Operands: two 64 KB buffers in shared memory, each { h0, h1 } of two 64-deep k panels.  A product of two-piece operands is
+// three fp16 products, h0 h1 + h1 h0 + h0 h0 (h1 h1 is below 2^-24 of a term), accumulated in fp32 in tensor memory.
+// The tensor pipe drops what does not fit when it adds to an accumulator, always towards zero: half a unit of the sum per
+// instruction.  So the small products come first, while the sum is 2^-11 of what it will be, and the eight instructions of
+// h0 h0 last; and a sum of several products (feed-forward chunks, the three of the head's gradient) is made in registers,
+// rounded to nearest, from an accumulator per product.  What is still lost is mostly a factor: the eight additions take
+// 1.6e-7 of the result on average (regression on the operands of training steps, 1.2e-7 to 1.6e-7), of which the scales of
+// the weights give 2^-23 back (not the embedding's: sums of one element per row lose nothing).
+// Relative errors against 64 bits, float32 GEMMs on the same operands in brackets: 128-deep product 1.3e-7 (2.0e-7), 512-deep
+// sum of chunks 2.3e-7 (3.5e-7); with the piece products in turn and the chunks in one accumulator 4.8e-7 and 1.8e-6; the
+// TF32 + bfloat16 split of the warp-level version has 2^-20 per term.
 #pragma once
 #include "dense_tc.cuh"
 #include "tc5.cuh"
@@ -26,7 +34,8 @@ constexpr int OFF_ROW = OFF_MISC + 256;             // 5 x 128 floats: scales of
 constexpr int SMEM_BYTES = OFF_ROW + 5 * 512 + 64;  // (+ a word per epilogue warp)
 static_assert(SMEM_BYTES <= 232448, "shared memory of one SM");
 enum Barrier { B_FULL = 0, B_EMPTY = STAGES, B_D0 = 2 * STAGES, B_D1, B_DX, B_A0, B_A1, B_A1_FREE, B_DRAIN, B_PART, B_ROWS, B_GO };
-constexpr int D0 = 0, D1 = 128, DX = 256;           // accumulators (columns of tensor memory)
+constexpr float GIVEN_BACK = 1.0f + 0x1p-23f;  // see above; a factor of the weights' scales (powers of two: exact)
+constexpr int D0 = 0, D1 = 128, DX = 256, DY = 384;  // accumulators (columns of tensor memory)
 
 struct Shared {
     uint32_t base;              // shared address of the block's memory
@@ -63,10 +72,10 @@ struct Producer {
     int requested = 0;   // stages asked for so far
     uint32_t phase = 1;  // the stages start out empty
     bool ok = true;
-    __device__ __forceinline__ void stream(const Shared &s, const unsigned char *image, int first_block, int blocks)
+    __device__ __forceinline__ void stream(const Shared &s, const unsigned char *image, int first_block, int blocks, int pieces = 2)
     {
         const unsigned char *src = image + TC_HEADER_BYTES + (size_t)first_block * TC_BLOCK_BYTES;
-        for (int i = 0; i < 2 * blocks && ok; ++i) {
+        for (int i = 0; i < pieces * blocks && ok; ++i) {
             ok = mbar_wait(s.bar(B_EMPTY + slot), phase, s.gave_up);
             if (!ok) return;
             mbar_expect(s.bar(B_FULL + slot), STAGE_BYTES);
@@ -90,22 +99,23 @@ struct Issuer {
     int slot = 0;
     uint32_t phase = 0;
     bool ok = true;
-    // D (+)= A . B^T for the operand buffer at a_off and the next block of the stream
-    __device__ __forceinline__ void product(const Shared &s, uint32_t tmem, int d_col, int a_off, bool accumulate)
+    // D = A . B^T for the operand buffer at a_off and the next block of the stream, whose pieces come smallest first
+    __device__ __forceinline__ void product(const Shared &s, uint32_t tmem, int d_col, int a_off, int pieces = 2)
     {
         constexpr uint32_t IDESC = instr_desc<128, 128, 0, false>();
-        for (int p = 0; p < 2 && ok; ++p) {
+        const uint64_t a0 = smem_desc(s.base + a_off, 16, 1024), a1 = smem_desc(s.base + a_off + 32768, 16, 1024);
+        for (int left = pieces - 1; left >= 0 && ok; --left) {
             ok = mbar_wait(s.bar(B_FULL + slot), phase, s.gave_up);
             if (!ok) return;
-            const uint32_t a = s.base + a_off + p * 16384, b = s.base + OFF_RING + slot * STAGE_BYTES;
-            const uint64_t a0 = smem_desc(a, 16, 1024), a1 = smem_desc(a + 32768, 16, 1024);
-            const uint64_t b0 = smem_desc(b, 16, 1024), b1 = smem_desc(b + 16384, 16, 1024);
+            const uint64_t b = smem_desc(s.base + OFF_RING + slot * STAGE_BYTES, 16, 1024);
+            // step ks: 16 k = 32 bytes = 2 units of the descriptor's address field, four to a panel of 16 KB = 1024 units
+            auto at = [](int ks) { return (uint64_t)((ks >> 2) * 1024 + (ks & 3) * 2); };
+            if (left == 0) {
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {  // 16 k = 32 bytes = 2 units of the descriptor's address field
-                mma_f16(tmem + d_col, a0 + 2 * ks, b1 + 2 * ks, IDESC, accumulate || p > 0 || ks > 0);
-                mma_f16(tmem + d_col, a1 + 2 * ks, b0 + 2 * ks, IDESC, true);
-                mma_f16(tmem + d_col, a0 + 2 * ks, b0 + 2 * ks, IDESC, true);
+                for (int ks = 0; ks < 8; ++ks) mma_f16(tmem + d_col, a1 + at(ks), b + at(ks), IDESC, true);
             }
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) mma_f16(tmem + d_col, a0 + at(ks), b + at(ks), IDESC, left < pieces - 1 || ks > 0);
             mma_commit(s.bar(B_EMPTY + slot));
             if (++slot == STAGES) { slot = 0; phase ^= 1u; }
         }
@@ -155,6 +165,19 @@ __device__ __forceinline__ void store_operand(unsigned char *buf, const Place &p
         split_pair(v[4 * j + 2] * s1, v[4 * j + 3] * s1, h0, h1);
         *reinterpret_cast<uint32_t *>(c + 1024) = h0;          // 8 rows further: the same swizzle phase
         *reinterpret_cast<uint32_t *>(c + 1024 + 32768) = h1;
+    }
+}
+
+// sum += this thread's part of an accumulator whose product is known to be complete
+__device__ __forceinline__ void add_accumulator(const Place &pl, uint32_t tmem, int d_col, float (&sum)[2][16])
+{
+    fence_after();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        float d[16];
+        tmem_load_16x32(pl.tmem(tmem, d_col, half), d);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum[half][i] += d[i];
     }
 }
 
@@ -288,6 +311,8 @@ __device__ __forceinline__ void load_operand(const Shared &s, unsigned char *buf
 // its shares (B_GO).
 constexpr int SPLIT = 4, SPLIT_STAGES = STAGES - 1;
 constexpr int OFF_STAGING = OFF_RING + SPLIT_STAGES * STAGE_BYTES;
+constexpr int OFF_OWN = OFF_STAGING + 16384;     // the forward's residual of the rows that this block finishes
+constexpr int OFF_STAGED_INV = OFF_ROW + 4 * 512;  // (row floats 4)
 constexpr int SHARE_BYTES = 16384, ROWS_BYTES = 16384 + 128;
 
 __device__ __forceinline__ uint32_t cluster_rank()
@@ -321,17 +346,25 @@ __device__ __forceinline__ void bulk_send(uint32_t dst_of_rank, uint32_t src, ui
 __device__ __forceinline__ void expect_shares(const Shared &s) { mbar_expect(s.bar(B_PART), SPLIT * SHARE_BYTES); }
 __device__ __forceinline__ void expect_rows(const Shared &s) { mbar_expect(s.bar(B_ROWS), SPLIT * ROWS_BYTES); }
 
-// One half (16 values) of this thread's part of the share, staged for the block that finishes these rows.  A row of a share
-// is 512 bytes, its 32-byte pieces swizzled by the row so that a warp's stores meet no bank twice.
-__device__ __forceinline__ void stage_share(const Shared &s, const Place &pl, int half, const float (&v)[16])
+// 32 rows of 128 floats as they are staged: a row is 512 bytes, its 32-byte pieces swizzled by the row so that a warp's
+// stores meet no bank twice.  One half (16 values) of this thread's part, and four columns of a row.
+__device__ __forceinline__ void stage_rows(unsigned char *share, const Place &pl, int half, const float (&v)[16])
 {
-    unsigned char *share = s.mem + OFF_A0 + ((threadIdx.x >> 5) & 3) * SHARE_BYTES;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         unsigned char *at = share + (pl.g + 16 * half) * 512 + (((4 * pl.group + j) ^ pl.g) << 5) + pl.t * 8;
         *reinterpret_cast<float2 *>(at) = make_float2(v[4 * j], v[4 * j + 1]);
         *reinterpret_cast<float2 *>(at + 8 * 512) = make_float2(v[4 * j + 2], v[4 * j + 3]);
     }
+}
+__device__ __forceinline__ const float4 &staged_row(const unsigned char *share, int row, int lane)
+{
+    return *reinterpret_cast<const float4 *>(share + row * 512 + (((lane >> 1) ^ (row & 7)) << 5) + (lane & 1) * 16);
+}
+// A half of this thread's part of the share, for the block that finishes these rows.
+__device__ __forceinline__ void stage_share(const Shared &s, const Place &pl, int half, const float (&v)[16])
+{
+    stage_rows(s.mem + OFF_A0 + ((threadIdx.x >> 5) & 3) * SHARE_BYTES, pl, half, v);
 }
 // The four warps that staged a share meet, and one thread sends it.
 __device__ __forceinline__ void send_share(const Shared &s, uint32_t rank)
@@ -352,11 +385,10 @@ __device__ __forceinline__ void collect_shares(const Shared &s, Phase &ph, float
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
         const int row = 2 * w + u;
-        const unsigned char *at = s.mem + OFF_A1 + row * 512 + (((lane >> 1) ^ (row & 7)) << 5) + (lane & 1) * 16;
-        float4 a = *reinterpret_cast<const float4 *>(at);
+        float4 a = staged_row(s.mem + OFF_A1, row, lane);
 #pragma unroll
         for (int slot = 1; slot < SPLIT; ++slot) {
-            const float4 b = *reinterpret_cast<const float4 *>(at + slot * SHARE_BYTES);
+            const float4 b = staged_row(s.mem + OFF_A1 + slot * SHARE_BYTES, row, lane);
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
         }
         v[u] = a;
@@ -385,7 +417,7 @@ __device__ __forceinline__ void spread_rows(const Shared &s, Phase &ph, uint32_t
         unsigned char *at = s.mem + OFF_STAGING + (lane >> 4) * 8192 + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + (lane & 1) * 8;
         *reinterpret_cast<uint2 *>(at) = h0;
         *reinterpret_cast<uint2 *>(at + 4096) = h1;
-        if (lane == 0) *reinterpret_cast<float *>(s.mem + OFF_STAGING + 16384 + row * 4) = inv;
+        if (lane == 0) *reinterpret_cast<float *>(s.mem + OFF_STAGED_INV + row * 4) = inv;
     }
     fence_async_smem();
     epilogue_sync();
@@ -396,7 +428,7 @@ __device__ __forceinline__ void spread_rows(const Shared &s, Phase &ph, uint32_t
             const uint32_t bar = at_rank(s.bar(B_ROWS), (uint32_t)to), from = s.base + OFF_STAGING + part * 4096;
             bulk_send(at_rank(s.base + OFF_A0 + (part >> 1) * 16384 + (part & 1) * 32768 + rank * 4096u, (uint32_t)to), from, 4096, bar);
             if (part == 0)
-                bulk_send(at_rank(s.base + OFF_ROW + (uint32_t)(which * 512) + rank * 128u, (uint32_t)to), s.base + OFF_STAGING + 16384, 128, bar);
+                bulk_send(at_rank(s.base + OFF_ROW + (uint32_t)(which * 512) + rank * 128u, (uint32_t)to), s.base + OFF_STAGED_INV, 128, bar);
         }
     }
 }

@@ -132,9 +132,10 @@ __device__ __forceinline__ void mma_commit(uint32_t bar)
 
 // ---- two-piece operands -----------------------------------------------------------------------------------------------
 // A value v is stored as h0 + h1, two halves of v s with s a power of two: h0 = half(v s), h1 = half(v s - h0).
-// s is chosen so that the largest value of the row (or matrix) that shares it lands in [2^14, 2^15): 22 bits of
-// mantissa, and an absolute floor of 2^-25, i.e. 2^-39 of that largest value.  power_of_two gives s and 1 / s for a
-// largest magnitude m (exponents clamped so that both are normal numbers; m = 0 is fine).
+// s is chosen so that the largest value of the row (or matrix) that shares it lands in [2^14, 2^15): what is left out is at
+// most one unit of v's 24 bits (h0 takes 11, and the rest, which has a sign, needs 12 where h1 has 11: one value in four is
+// off, by that unit), with an absolute floor of 2^-25, i.e. 2^-39 of that largest value.  power_of_two gives s and 1 / s for
+// a largest magnitude m (exponents clamped so that both are normal numbers; m = 0 is fine).
 __device__ __forceinline__ float power_of_two(float m, float &inv)
 {
     int e = (int)(__float_as_uint(m) >> 23) & 255;
@@ -149,6 +150,14 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t &h0, uint3
     const __half2 lo = __floats2half2_rn(a - back.x, b - back.y);
     h0 = *reinterpret_cast<const uint32_t *>(&hi);
     h1 = *reinterpret_cast<const uint32_t *>(&lo);
+}
+// ... and what is left as a third half: all 24 bits
+__device__ __forceinline__ void split_three(float a, float b, uint32_t &h0, uint32_t &h1, uint32_t &h2)
+{
+    split_pair(a, b, h0, h1);
+    const float2 f0 = __half22float2(*reinterpret_cast<const __half2 *>(&h0)), f1 = __half22float2(*reinterpret_cast<const __half2 *>(&h1));
+    const __half2 rest = __floats2half2_rn((a - f0.x) - f1.x, (b - f0.y) - f1.y);
+    h2 = *reinterpret_cast<const uint32_t *>(&rest);
 }
 
 }  // namespace tc5

@@ -72,24 +72,28 @@ __global__ void __launch_bounds__(128) head_backward_kernel(const float *__restr
 }
 
 // gradient of the head's last layer: gW2[t][u] = sum_c gy[c][t] hid[c][u], gb2[t] = sum_c gy[c][t].  Block = (32 units,
-// target); the warps take every eighth crystal and meet in shared memory in a fixed order.
+// target); the warps take every eighth crystal (compensated sums: a batch may have thousands) and meet in shared memory in a
+// fixed order.
 __global__ void __launch_bounds__(256) head_weight_grad_kernel(const float *__restrict__ gy, const float *__restrict__ hid, long long B,
                                                                int hidden, int targets, float *__restrict__ gW2, float *__restrict__ gb2)
 {
     __shared__ float part[2][8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, u = blockIdx.x * 32 + lane, t = blockIdx.y;
-    float acc = 0.f, bias = 0.f;
+    float acc = 0.f, acc_low = 0.f, bias = 0.f, bias_low = 0.f;
     for (long long c = w; c < B; c += 8) {
         const float g = gy[c * targets + t];
-        acc = fmaf(g, u < hidden ? hid[c * hidden + u] : 0.f, acc);
-        bias += g;
+        add_compensated(g * (u < hidden ? hid[c * hidden + u] : 0.f), acc, acc_low);
+        add_compensated(g, bias, bias_low);
     }
-    part[0][w][lane] = acc;
-    part[1][w][lane] = bias;
+    part[0][w][lane] = acc + acc_low;
+    part[1][w][lane] = bias + bias_low;
     __syncthreads();
     if (w == 0) {
-        float a = 0.f, b = 0.f;
-        for (int i = 0; i < 8; ++i) { a += part[0][i][lane]; b += part[1][i][lane]; }
+        auto eight = [&](int which) {
+            const float(*v)[32] = part[which];
+            return ((v[0][lane] + v[1][lane]) + (v[2][lane] + v[3][lane])) + ((v[4][lane] + v[5][lane]) + (v[6][lane] + v[7][lane]));
+        };
+        const float a = eight(0), b = eight(1);
         if (u < hidden) gW2[(size_t)t * hidden + u] = a;
         if (blockIdx.x == 0 && lane == 0) gb2[t] = b;
     }
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(512) pe_grad_kernel(const PeArgs p)
     const int tid = threadIdx.x, l = blockIdx.y, h = tid >> 6;
     const long long lo = p.N * blockIdx.x / p.shares, hi = p.N * (blockIdx.x + 1) / p.shares;
     const float *gattn = p.gattn[l], *psi = PSI ? p.psi[l] : nullptr, *q = p.q[l], *galpha = p.galpha[l];
-    float acc[16], wpos = 0.f;
+    float acc[16], wpos = 0.f, wpos_low = 0.f;
 #pragma unroll
     for (int m = 0; m < 16; ++m) acc[m] = 0.f;
     for (long long n0 = lo; n0 < hi; n0 += PE_ROWS) {
@@ -142,14 +146,15 @@ __global__ void __launch_bounds__(512) pe_grad_kernel(const PeArgs p)
             }
         }
         if (tid < CH && q != nullptr)
-            for (int r = 0; r < rows; ++r) wpos = fmaf(galpha[(n0 + r) * HEADS + (tid >> 4)], 4.0f * q[(n0 + r) * CH + tid], wpos);
+            for (int r = 0; r < rows; ++r)
+                add_compensated(galpha[(n0 + r) * HEADS + (tid >> 4)] * (4.0f * q[(n0 + r) * CH + tid]), wpos, wpos_low);
     }
     float *out = p.partial + ((size_t)l * p.shares + blockIdx.x) * PE_PARTIAL;
     if (PSI) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) out[(h * 16 + m) * 64 + (tid & 63)] = acc[m];
     }
-    if (tid < CH) out[CH * 64 + tid] = wpos;
+    if (tid < CH) out[CH * 64 + tid] = wpos + wpos_low;
 }
 
 // the shares added in a fixed order: block = 32 values, warp w the shares w, w + 8, ..., then the eight partial sums
@@ -269,7 +274,7 @@ Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64
     s.row_order = c.take<int32_t>(N);
     s.tickets = c.take<unsigned>(MAX_LAYERS);
     s.row_blocks = c.take<unsigned>(row_blocks_words(N));
-    s.embed = c.take<unsigned char>(tc_image_bytes(1));
+    s.embed = c.take<unsigned char>(TC_EMBED_BYTES);
     const size_t image = tc_image_bytes(tc_layer_blocks((int)d.ff_dim));
     for (int l = 0; l < d.num_layers; ++l) {
         LayerSaved &y = s.layer[l];

@@ -61,9 +61,11 @@ def test_errors_are_those_of_float32_products(ff, layers, atoms, spread):
             if p.grad is not None and n in g64 and float(g64[n].norm()) > 0 and "in_proj" not in n:
                 off[native][n] = rel(p.grad, g64[n])
     assert model._train_plan is not None
+    print({n: (f"{e:.2e}", f"{e / off[False][n]:.2f}") for n, e in off[True].items()})
     for n, e in off[True].items():
         assert e <= BOUND(off[False][n]), (n, e, off[False][n])
 
 
-# A weight gradient is a sum over thousands of rows: adding its products in one tensor-core accumulator is 7e-6 off.
-BOUND = lambda float32: 4e-6
+# No further off than the float32 products, a tenth for chance (norms over thousands of values; a bias gradient is a few
+# values or a hundred, each a few roundings of 2^-24).  Sums in a tensor-core accumulator are 2 to 40 times as far off.
+BOUND = lambda float32: max(1.1 * float32, 4 * 2.0 ** -24)
