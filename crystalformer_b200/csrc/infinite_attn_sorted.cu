@@ -70,13 +70,16 @@ __device__ __forceinline__ void mma_half(float (&c)[4], unsigned a0, unsigned a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Values of [0, 1], scaled by 2^15, as two halves each: x = hi + lo to 2^-22 relative, and never worse than 2^-39 of the
-// largest value.  Products of such pairs, hi.hi + lo.hi + hi.lo, are within 2^-21 of x.y.  A pair of terms per register.
-constexpr float HALF_SCALE_LOG2 = 15.0f;
+// Values of [0, 1] as two halves each, a pair of terms per register: x = hi + lo up to one unit of x's 24 bits, with a floor of
+// 2^-25 of the largest value, 2^-40 for the weights, which are scaled by 2^15 first (a row's sum may hold thousands of small
+// ones; the basis, whose values enter beside larger ones of the same term, is not).  The scale is a product and not part of
+// the exponent: there it would round the exponents of the largest weights at 2^-20 instead of 2^-25 (error of the output
+// against 64 bits 1.63e-7 instead of 1.34e-7; TF32 operands had 1.45e-7).
+constexpr float HALF_SCALE = 32768.0f;
 // A head's sum is at least one if its box holds the term that its bound M_h comes from; below this the absolute floor of the
 // halves would show, and the row is left over.
 constexpr float MIN_SUM = 1.5e-5f;
-constexpr float UNSCALE = 1.0f / 32768.0f;
+constexpr float UNSCALE = 1.0f / HALF_SCALE;
 __device__ __forceinline__ void split_halves(float x, float y, unsigned &hi, unsigned &lo)
 {
     const __half2 h = __floats2half2_rn(x, y);
@@ -235,7 +238,6 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
 #pragma unroll
     for (int m = 0; m < 4; ++m) accPsi[m][0] = accPsi[m][1] = accPsi[m][2] = accPsi[m][3] = 0.f;
     const float *cjg = cj + g * CJ_LD;
-    const float M_scaled = M_g - HALF_SCALE_LOG2;
     const unsigned g_pair = (unsigned)g * 0x10001u;
     const float ucg = (float)(g + 1) * p.bin_step;          // centre of bin g in basis units
     const float step16 = 16.0f * p.bin_step, step8 = 8.0f * p.bin_step;
@@ -275,12 +277,14 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 jv[u] = keyv[u] & 255;
-                w[u] = ex2(fmaf(a2g, d2v[u], cjg[jv[u]]) - M_scaled);
+                w[u] = ex2(fmaf(a2g, d2v[u], cjg[jv[u]]) - M_g);
                 w[u] = (row_key_in_box(keyv[u], boxor) && (u < 2 || two)) ? w[u] : 0.f;
             }
             unsigned w_hi[2], w_lo[2];
-            split_halves(w[0], w[1], w_hi[0], w_lo[0]);
-            split_halves(w[2], w[3], w_hi[1], w_lo[1]);
+            const float2 scale = make_float2(HALF_SCALE, HALF_SCALE);
+            const float2 wa = __fmul2_rn(make_float2(w[0], w[1]), scale), wb = __fmul2_rn(make_float2(w[2], w[3]), scale);
+            split_halves(wa.x, wa.y, w_hi[0], w_lo[0]);
+            split_halves(wb.x, wb.y, w_hi[1], w_lo[1]);
             // P^T tiles: one-hot of the terms' keys (rows g, g + 8 of tile u are keys 16 u + g, 16 u + g + 8)
             const unsigned ja = ((unsigned)jv[0] | ((unsigned)jv[1] << 16)) ^ g_pair, jb = ((unsigned)jv[2] | ((unsigned)jv[3] << 16)) ^ g_pair;
 #pragma unroll
@@ -308,8 +312,8 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float c0 = fmaf(-(float)m, step16, uu[e]), c1 = c0 - step8;
-                    v0[e] = ex2(fmaf(-c0, c0, HALF_SCALE_LOG2));
-                    v1[e] = ex2(fmaf(-c1, c1, HALF_SCALE_LOG2));
+                    v0[e] = ex2(-c0 * c0);
+                    v1[e] = ex2(-c1 * c1);
                 }
                 unsigned hi[4], lo[4];
                 split_halves(v0[0], v0[1], hi[0], lo[0]);
@@ -336,10 +340,10 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
     __syncwarp();
 #pragma unroll
     for (int m = 0; m < (PSI ? 4 : 0); ++m) {
-        psi[(2 * t) * PSI_LD + 16 * m + g] = accPsi[m][0] * (UNSCALE * UNSCALE);
-        psi[(2 * t + 1) * PSI_LD + 16 * m + g] = accPsi[m][1] * (UNSCALE * UNSCALE);
-        psi[(2 * t) * PSI_LD + 16 * m + g + 8] = accPsi[m][2] * (UNSCALE * UNSCALE);
-        psi[(2 * t + 1) * PSI_LD + 16 * m + g + 8] = accPsi[m][3] * (UNSCALE * UNSCALE);
+        psi[(2 * t) * PSI_LD + 16 * m + g] = accPsi[m][0] * UNSCALE;
+        psi[(2 * t + 1) * PSI_LD + 16 * m + g] = accPsi[m][1] * UNSCALE;
+        psi[(2 * t) * PSI_LD + 16 * m + g + 8] = accPsi[m][2] * UNSCALE;
+        psi[(2 * t + 1) * PSI_LD + 16 * m + g + 8] = accPsi[m][3] * UNSCALE;
     }
 #pragma unroll
     for (int u = 0; u < NT; ++u) {

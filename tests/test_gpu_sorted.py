@@ -248,3 +248,28 @@ def test_sorted_rows_at_bench_size_match_the_listed_kernel(ops):
                                      rvlen=rvlen, cutoff_radius=-3.5, minimum_range=2, precision="f64")
     _, ref = oracle.fused_attn_fwd(q[:n_s], k[:n_s], v[:n_s], z, psiW, edges, precision="f64")
     assert rel_err(out[:n_s].cpu().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("crystals,nmax", [(24, 30), (14, 60)])
+def test_error_against_64_bits(ops, crystals, nmax):
+    """The half-precision pairs of the sorted kernel keep float32's precision: 2-norm error against the float64 chain beside the
+    enumerating kernel's, which works in float32 throughout.  A pair leaves out one unit of 2^-24 in one value of four, 4e-8
+    for either operand beside the 1.2e-7 of the float32 sums: a tenth more, and as much again for chance."""
+    cb = make_crystals(11, crystals, uniform_atoms(1, nmax), length_range=(3.0, 15.0))
+    prep = prepare(ops, cb)
+    N, max_atoms = cb.num_atoms, int(cb.sizes.max())
+    rng = np.random.default_rng(3)
+    q = (rng.standard_normal((N, H, D)) * 0.25).astype(np.float32)
+    k, v = (rng.standard_normal((N, H, D)).astype(np.float32) for _ in range(2))
+    W = (rng.standard_normal((H, D, K)) * 0.1).astype(np.float32)
+    a = (-0.5 / (1.4 * (0.5 + rng.random((N, H)))) ** 2).astype(np.float32)
+    a_widest = -0.5 / (1.4 * 1.5) ** 2
+    host = lambda t: t.cpu().numpy()
+    z, vals = oracle.lattice_sum_fwd(a, host(prep["pos_ij"]), cb.trans_vec, cb.batch, host(prep["edges"]), K, DIST_MAX, WSCALE, W=W,
+                                     rvlen=host(prep["rvlen"]), cutoff_radius=-3.5, lattice_range=2, minimum_range=2, precision="f64")
+    _, exact = oracle.fused_attn_fwd(q, k, v, z, vals, host(prep["edges"]), precision="f64")
+    out, _, _ = sorted_forward(ops, cb, prep, q, k, v, a, W, -3.5, 2, a_widest)
+    plain = ops.infinite_attn_fwd(dev(q), dev(k), dev(v), dev(a), prep["pos_ij"], dev(cb.trans_vec), prep["rvlen"], prep["batch"],
+                                  prep["edges"], prep["row_start"], max_atoms, K, DIST_MAX, WSCALE, dev(W), -3.5, 2, 2)[0]
+    off = lambda t: float(np.linalg.norm(host(t).astype(np.float64).ravel() - exact.ravel()) / np.linalg.norm(exact))
+    assert off(out) <= 1.25 * off(plain), (off(out), off(plain))
