@@ -32,6 +32,8 @@ SIGNATURES = {
                              I32, P, P, P, P, P, P],
     "cf_infinite_attn_bwd": [P, P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, F64, F64, P, F64, I32,
                              I32, P, P, P, P, P, P, P, P, P, P, P],
+    "cf_check_waits": [],
+    "cf_wait_probe": [I64, P],
     "cf_pipe_probe": [I32, I32, I32, I64, P, P],
     "cf_model_forward": [P, P, I64, P, P, P, I64, I64, I64, I64, P, P, I32, P, P, I64, I64, F64, F64, I32, I32, P, P, I64, P,
                          P, I64, F64, P, P, P, P, P, P, P],

@@ -33,6 +33,41 @@ int launch_status(const char *what)
     return CF_OK;
 }
 
+namespace {
+struct WaitStatus {
+    unsigned *words = nullptr;  // one per device; kernels of any device may write to it
+    WaitStatus()
+    {
+        // (may be the first call of a capture: pinned memory has no part in it)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(unsigned) * 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            words = static_cast<unsigned *>(p);
+            for (int i = 0; i < 64; ++i) words[i] = 0u;
+        } else {
+            cudaGetLastError();
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+};
+}  // namespace
+
+unsigned *wait_status()
+{
+    static WaitStatus status;
+    int dev = 0;
+    if (status.words == nullptr || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    return status.words + (dev & 63);
+}
+
+int check_waits(const char *who)
+{
+    unsigned *word = wait_status();
+    if (word == nullptr || __atomic_load_n(word, __ATOMIC_RELAXED) == 0u || __atomic_exchange_n(word, 0u, __ATOMIC_ACQUIRE) == 0u) return CF_OK;
+    return fail(CF_ERR_WAIT, "%s: a wait of an earlier dense kernel on this device ran out; what that call returned is void", who);
+}
+
 float weight_floor_log2()
 {
     const double f = g_floor_log2.load();
@@ -70,6 +105,8 @@ int sm_count()
 extern "C" {
 
 int cf_version(void) { return 100; }
+
+int cf_check_waits(void) { return cf::check_waits("cf_check_waits"); }
 
 const char *cf_last_error(void) { return cf::g_error; }
 

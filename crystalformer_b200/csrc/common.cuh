@@ -16,6 +16,10 @@ constexpr float LN2 = 0.6931471805599453f;
 // ---- host-side error plumbing (api.cu) --------------------------------------------------------------------
 int fail(int code, const char *fmt, ...);
 int launch_status(const char *what);
+// The word of the current device in which kernels report bounded waits that ran out (pinned host memory, null if there is
+// none), and whether one has: CF_OK or, once per report, CF_ERR_WAIT.
+unsigned *wait_status();
+int check_waits(const char *who);
 float weight_floor_log2();  // log2 of the weight below which a term is left out of the basis accumulation
 unsigned long long *row_stats_words();  // device words that the sorted row kernel adds its work counts to, or NULL
 int &dense_tile_rows_choice();  // this thread's row tile of the dense blocks: 0 = chosen per launch, 16, 32

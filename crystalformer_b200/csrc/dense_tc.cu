@@ -11,8 +11,6 @@
 // units, DX for the output), so the tensor pipe only waits at y, at x' and at the end of a tile.
 #include "dense_tc_core.cuh"
 
-__device__ unsigned g_dense_forward_status;  // set by a block whose waits ran out (never in a working build)
-
 namespace cf {
 namespace {
 using namespace tc5;
@@ -320,7 +318,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                          row_base, xi, ws.head);
         }
     }
-    block_end(s, tmem, &g_dense_forward_status);
+    block_end(s, tmem, p.status);
 }
 
 // The same for a cluster of four blocks (dense_tc_core.cuh): block r takes hidden chunk r and, of q, k, v, matrix r.  Hidden
@@ -470,7 +468,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
     }
     __syncthreads();
     cluster_sync();  // (no block ends while another may still write to it)
-    block_end(s, tmem, &g_dense_forward_status);
+    block_end(s, tmem, p.status);
 }
 
 // ---- packing -------------------------------------------------------------------------------------------------------
@@ -535,9 +533,13 @@ __global__ void __launch_bounds__(PACK_THREADS) dense_pack_kernel(const PackJob 
 
 }  // namespace
 
-int launch_dense_forward(const DenseForward &p, cudaStream_t s)
+int launch_dense_forward(const DenseForward &args, cudaStream_t s)
 {
-    if (p.N == 0) return CF_OK;
+    if (args.N == 0) return CF_OK;
+    const int waits = check_waits("dense forward");
+    if (waits != CF_OK) return waits;
+    DenseForward p = args;
+    p.status = wait_status();
     if (p.ff <= 0 || p.ff % 128 != 0 || p.ff > TC_MAX_FF)
         return fail(CF_ERR_UNSUPPORTED, "dense forward: ff_dim=%d must be a multiple of 128 up to %d", p.ff, TC_MAX_FF);
     static thread_local DenseLaunch launch;

@@ -64,6 +64,7 @@ struct DenseForward {
     float *x_out;        // (N,128) features after the tail / embedding
     float *q, *k, *v, *a;
     float *y_save, *h_save;  // training: y (N,128) and the hidden units (N, ff), or null
+    unsigned *status;        // (set by the launch: wait_status)
 };
 
 // The packed-weight pointers of the one-call forwards (slot 10 of a layer, W_embed_packed) carry bit 0 set when they name
@@ -128,6 +129,7 @@ struct DenseBackward {
     const unsigned char *tail;
     const float *h;              // (N, ff) the saved hidden units
     float *gh, *gy, *gattn;
+    unsigned *status;            // (set by the launch: wait_status)
 };
 int launch_dense_backward(const DenseBackward &p, cudaStream_t s);
 

@@ -8,8 +8,6 @@
 // gh, gy, gq') is written on the way.
 #include "dense_tc_core.cuh"
 
-__device__ unsigned g_dense_backward_status;  // set by a block whose waits ran out (never in a working build)
-
 namespace cf {
 namespace {
 using namespace tc5;
@@ -269,7 +267,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             }
         }
     }
-    block_end(s, tmem, &g_dense_backward_status);
+    block_end(s, tmem, p.status);
 }
 
 // The same for a cluster of four blocks (dense_tc_core.cuh): block 0, 1, 2 multiplies gq', gk, gv, block r hidden chunk r,
@@ -466,7 +464,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(
     }
     __syncthreads();
     cluster_sync();  // (no block ends while another may still write to it)
-    block_end(s, tmem, &g_dense_backward_status);
+    block_end(s, tmem, p.status);
 }
 
 // ---- weight gradients ---------------------------------------------------------------------------------------------------
@@ -498,7 +496,7 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t (&w)[3])
     }
 }
 
-__global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJobs jobs, int splits, float *partial)
+__global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJobs jobs, int splits, float *partial, unsigned *status)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
     const GradJob &job = jobs.j[blockIdx.x];
@@ -661,7 +659,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
     __syncthreads();
     fence_after();
     if (warp == 16) tmem_free<256>(tmem);
-    if (threadIdx.x == 0 && *gave_up != 0u) atomicOr(&g_dense_backward_status, 1u);
+    if (threadIdx.x == 0) report_waits(gave_up, status);
 }
 
 // The splits of a job added in their order and written where the gradient belongs; 16 blocks per job.
@@ -694,9 +692,13 @@ int grad_splits(int count, long long rows)
 
 }  // namespace
 
-int launch_dense_backward(const DenseBackward &p, cudaStream_t s)
+int launch_dense_backward(const DenseBackward &args, cudaStream_t s)
 {
-    if (p.N == 0) return CF_OK;
+    if (args.N == 0) return CF_OK;
+    const int waits = check_waits("dense backward");
+    if (waits != CF_OK) return waits;
+    DenseBackward p = args;
+    p.status = wait_status();
     static thread_local DenseLaunch launch;
     int rc = launch.configure(reinterpret_cast<const void *>(dense_backward_kernel), reinterpret_cast<const void *>(dense_backward_split_kernel), "dense backward");
     if (rc != CF_OK) return rc;
@@ -714,6 +716,8 @@ size_t grad_partial_floats(int count, long long rows) { return (size_t)count * g
 int launch_weight_grads(const GradJobs &jobs, int count, float *partial, cudaStream_t s)
 {
     if (count == 0) return CF_OK;
+    const int waits = check_waits("weight gradients");
+    if (waits != CF_OK) return waits;
     static thread_local bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -725,7 +729,7 @@ int launch_weight_grads(const GradJobs &jobs, int count, float *partial, cudaStr
         configured[dev & 63] = true;
     }
     const int splits = grad_splits(count, jobs.j[0].rows);
-    weight_grad_kernel<<<dim3(count, splits), GR_THREADS, GR_SMEM, s>>>(jobs, splits, partial);
+    weight_grad_kernel<<<dim3(count, splits), GR_THREADS, GR_SMEM, s>>>(jobs, splits, partial, wait_status());
     weight_grad_sum_kernel<<<dim3(count, 16), 256, 0, s>>>(jobs, splits, partial);
     return launch_status("weight_grad_kernel");
 }

@@ -466,7 +466,7 @@ __device__ __forceinline__ void block_end(const Shared &s, uint32_t tmem, unsign
     __syncthreads();
     fence_after();
     if ((threadIdx.x >> 5) == ISSUE_WARP) tmem_free<512>(tmem);
-    if (threadIdx.x == 0 && *s.gave_up != 0u) atomicOr(status, 1u);
+    if (threadIdx.x == 0) report_waits(s.gave_up, status);
 }
 
 // ---- host side ------------------------------------------------------------------------------------------------------------

@@ -1,9 +1,26 @@
 // Throughput probes for the two pipes that bound the lattice-sum kernels: FP32 FMA and MUFU (ex2).
 // They give the roofline denominators measured on the device at hand instead of datasheet numbers.
 #include "common.cuh"
+#include "tc5.cuh"
 
 namespace cf {
 namespace {
+
+// A bounded wait that runs out: nothing ever arrives at the barrier.
+__global__ void wait_probe_kernel(unsigned long long limit_ns, unsigned *status)
+{
+    __shared__ __align__(8) unsigned long long barrier;
+    __shared__ unsigned gave_up;
+    const uint32_t bar = tc5::smem_u32(&barrier);
+    if (threadIdx.x == 0) {
+        tc5::mbar_init(bar, 1);
+        gave_up = 0u;
+    }
+    __syncthreads();
+    tc5::mbar_wait(bar, 0, &gave_up, limit_ns);
+    __syncthreads();
+    if (threadIdx.x == 0) tc5::report_waits(&gave_up, status);
+}
 
 template <int KIND>
 __global__ void pipe_probe_kernel(long long iters, float *sink)
@@ -27,6 +44,15 @@ __global__ void pipe_probe_kernel(long long iters, float *sink)
 
 }  // namespace
 }  // namespace cf
+
+extern "C" int cf_wait_probe(int64_t limit_ns, void *stream)
+{
+    using namespace cf;
+    CF_REQUIRE(limit_ns >= 0 && limit_ns <= (int64_t)tc5::WAIT_NS, CF_ERR_RANGE, "cf_wait_probe: limit of %lld ns (0 to %llu)", (long long)limit_ns,
+               tc5::WAIT_NS);
+    wait_probe_kernel<<<1, 32, 0, as_stream(stream)>>>((unsigned long long)limit_ns, wait_status());
+    return launch_status("cf_wait_probe");
+}
 
 extern "C" int cf_pipe_probe(int kind, int blocks, int threads, int64_t iters, float *sink, void *stream)
 {

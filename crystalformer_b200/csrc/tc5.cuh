@@ -49,7 +49,7 @@ __device__ __forceinline__ unsigned long long global_ns()
 // caller then leaves its loop, and the block drains its copies, frees its tensor memory and returns.
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 template <bool CLUSTER = false>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile unsigned *gave_up)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile unsigned *gave_up, unsigned long long limit_ns = WAIT_NS)
 {
     auto ready = [&]() { return CLUSTER ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity); };
     if (ready()) return true;
@@ -57,10 +57,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     for (int tries = 0; tries < (1 << 28); ++tries) {
         if (ready()) return true;
         if (*gave_up != 0u) return false;
-        if (global_ns() - t0 > WAIT_NS) break;
+        if (global_ns() - t0 > limit_ns) break;
     }
     *gave_up = 1u;
     return false;
+}
+
+// One thread of a block, at its end: a wait that ran out is reported to the host (wait_status).
+__device__ __forceinline__ void report_waits(volatile unsigned *gave_up, unsigned *status)
+{
+    if (*gave_up != 0u && status != nullptr) atomicOr_system(status, 1u);
 }
 
 // ---- copies and proxies ----------------------------------------------------------------------------------------------

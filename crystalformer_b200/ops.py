@@ -44,6 +44,13 @@ def _check_projection(W: Optional[torch.Tensor], H: int, K: int, name: str) -> N
         raise ValueError(f"{name}: W must end in (H={H}, Dv, K={K}), got {tuple(W.shape)}")
 
 
+def check_waits(device=None) -> None:
+    """Raises if a bounded wait of a kernel launched earlier on the device has run out, so that what its call returned is void
+    (cf_check_waits).  Covers what has finished: synchronise first.  The next forward or backward raises it too."""
+    with torch.cuda.device(device if device is not None else torch.cuda.current_device()):
+        _lib.call("cf_check_waits")
+
+
 def set_sorted_rows(enabled: bool) -> None:
     """Whether the one-call forwards may use row lists and the sorted row kernel (cf_set_sorted_rows)."""
     _lib.load().cf_set_sorted_rows(c_int(1 if enabled else 0))

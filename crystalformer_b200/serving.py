@@ -232,11 +232,14 @@ class PipelinedPredictor:
     def result(self, ticket: int) -> torch.Tensor:
         """Waits for the oldest batch in flight (``ticket`` must be its ticket) and returns its output on the host.
         The returned tensor is a view of a ring buffer that is reused ``depth`` submissions later: copy it to keep it.
-        Raises if the batch's peer gather gave up waiting for a rank (its rows would be NaN)."""
+        Raises if the batch's peer gather gave up waiting for a rank (its rows would be NaN) or a bounded wait of a kernel ran
+        out (``ops.check_waits``)."""
         if not self._inflight or self._inflight[0][0] != ticket:
             raise RuntimeError("results must be collected in submission order")
         _, done, out, status = self._inflight.popleft()
         done.synchronize()
+        with torch.cuda.device(self.device):
+            _lib.call("cf_check_waits")  # (this batch's, or of one still in flight)
         if status is not None and int(status[0]) != 0:
             raise RuntimeError(f"peer gather: gave up waiting for the outputs of rank {int(status[0]) - 1}")
         return out

@@ -16,7 +16,7 @@
  * cf_set_chained_launches, cf_set_row_stats), a
  * side stream and four events per (host thread, device) created by the first cf_encoder_forward / cf_model_forward
  * / cf_model_begin / cf_train_begin, a pinned staging buffer of at most 8 MiB per host thread for the sizes that the
- * begin calls read back,
+ * begin calls read back, a word of pinned host memory per device in which kernels report waits that ran out,
  * the 8 MiB scratch array of cf_lattice_sum_bwd_static, and a pool of row tickets per device: 64 single counters
  * handed round-robin to the cf_infinite_attn_fwd[_listed] calls with K > 0 and 8 blocks of 16 handed round-robin to the
  * one-call forwards that use term lists.  A ticket is reused after 64 calls (8 forwards): at most that many such calls
@@ -47,6 +47,7 @@ extern "C" {
 #define CF_ERR_UNSUPPORTED (-2) /* shape outside the compiled set (H, D, K) */
 #define CF_ERR_CUDA (-3)        /* a CUDA runtime call failed; message in cf_last_error() */
 #define CF_ERR_RANGE (-4)       /* a size exceeds a documented limit */
+#define CF_ERR_WAIT (-5)        /* a bounded wait of an earlier launch on the device ran out: its outputs are void */
 
 /* Largest half-width of the translation box in any direction.  The reference loops over whatever the cut-off rule
  * yields; here a box wider than this is clamped so that a degenerate width (a -> 0) cannot stall the GPU. */
@@ -595,6 +596,16 @@ int cf_reci_sum_fwd(const float *a, const float *kr_base, const float *rvecs, co
 int cf_reci_sum_bwd(const float *a, const float *kr_base, const float *rvecs, const int64_t *batch,
                     const int64_t *row_start, const float *gz, const float *sumexp, int64_t N, int64_t H, int64_t E,
                     int lattice_range, float *ga, void *stream);
+
+/* ------------------------------------------------------------------------------------------------------------
+ * The dense kernels' waits (for copies and tensor instructions, at most two seconds each) end by themselves if what they wait
+ * for never comes; the launch then finishes with void outputs and reports it.  As the launches are asynchronous, the report
+ * is returned as CF_ERR_WAIT by the next call that launches such a kernel on the device, or by cf_check_waits, which does
+ * nothing else: after a synchronisation it covers everything before it.  A report is returned once.
+ * cf_wait_probe launches one warp that waits limit_ns (up to two seconds) for something that never comes, and reports.
+ * ---------------------------------------------------------------------------------------------------------- */
+int cf_check_waits(void);
+int cf_wait_probe(int64_t limit_ns, void *stream);
 
 /* ------------------------------------------------------------------------------------------------------------
  * Pipe-throughput probes for the roofline denominators: `iters` dependent-free FFMA (kind 0) or MUFU.EX2 (kind 1)
