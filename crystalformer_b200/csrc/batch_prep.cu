@@ -164,7 +164,6 @@ __global__ void row_cost_kernel(const int64_t *__restrict__ atom_start, const fl
 // (cost, crystal) keys in shared memory, exclusive scan of the sorted atom counts, then every crystal's atoms are
 // written as one run.
 constexpr int ORDER_THREADS = 1024;
-constexpr int ORDER_MAX_CRYSTALS = 2048;
 
 __device__ __forceinline__ void row_order_body(const int64_t *__restrict__ atom_start, const float *__restrict__ trans,
                                                int B, int padded, float sphere, int32_t *__restrict__ order)
@@ -315,7 +314,7 @@ int launch_prepare_all(const float *pos, const float *trans, const int64_t *size
         crystal_offsets_kernel<<<1, SCAN_THREADS, 0, s>>>(sizes, B, atom_start, edge_start);
     }
     p.batch = batch; p.edges = edges; p.row_start = row_start; p.pos_ij = pos_ij; p.rvlen = rvlen; p.rvecs = rvecs; p.vcell = vcell;
-    *ordered = row_order != nullptr && B <= ORDER_MAX_CRYSTALS && N < (1ll << 31);
+    *ordered = row_order != nullptr && rows_are_ordered(B, N);
     p.order = *ordered ? row_order : nullptr;
     p.padded = 2;
     while (p.padded < B) p.padded <<= 1;

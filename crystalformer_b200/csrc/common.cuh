@@ -158,6 +158,11 @@ inline cudaError_t launch_chained_cluster(void (*kernel)(KArgs...), unsigned blo
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Whether a batch's rows are ordered by their cost (batch_prep.cu: a sort of its crystals in one block): the preparation writes
+// the order, and whoever reads it later, only then.
+constexpr int ORDER_MAX_CRYSTALS = 2048;
+inline bool rows_are_ordered(long long B, long long N) { return B <= ORDER_MAX_CRYSTALS && N < (1ll << 31); }
+
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 int sm_count();
 

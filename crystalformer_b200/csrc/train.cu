@@ -647,8 +647,7 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
     Scratch g = carve_scratch(d, scratch, N, B, E);
     const float *const *tail_weights = d.weights + PER_LAYER * L;
     float *const *tail_grads = grads + PER_LAYER * L;
-    const bool ordered = N < (1ll << 31) && B <= 2048;
-    const int32_t *order = ordered ? w.row_order : nullptr;
+    const int32_t *order = rows_are_ordered(B, N) ? w.row_order : nullptr;
     const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
     TermList list{};
     float a_widest;

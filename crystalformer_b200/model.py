@@ -280,7 +280,7 @@ class Latticeformer(nn.Module):
         N, B = pos.shape[0], sizes.shape[0]
         lib = _lib.load()
         desc = ctypes.byref(plan["desc"])
-        head = torch.empty(N * 520, dtype=torch.float32, device=dev)  # cf_model_head_floats(N)
+        head = torch.empty(int(lib.cf_model_head_floats(N)), dtype=torch.float32, device=dev)
         counts, event = (ctypes.c_int64 * 3)(-1, 0, 0), ctypes.c_void_p()
         with torch.cuda.device(dev):
             stream = torch.cuda.current_stream(dev).cuda_stream

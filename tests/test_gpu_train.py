@@ -58,6 +58,16 @@ def test_gradients_equal_the_autograd_path(params, sizes):
     assert all(torch.equal(got[n], again[n]) for n in got)  # no atomics in any sum
 
 
+@pytest.mark.parametrize("crystals", [2048, 2049])
+def test_batches_with_and_without_an_order_of_rows(crystals):
+    """The preparation orders the rows of up to 2048 crystals; forward and backward agree on whether it has."""
+    model, data, target = setup([2] * crystals, num_layers=1)
+    ref, got = step(model, data, target, native=False)[1], step(model, data, target, native=True)[1]
+    assert model._train_plan is not None
+    for name in ref:
+        assert (got[name] - ref[name]).norm() <= 2e-3 * ref[name].norm() + 1e-9, name
+
+
 def test_step_follows_the_model():
     """In-place updates, replaced parameters, copies and frozen parameters; a modified weight between the two halves."""
     model, data, target = setup([9, 20, 5], num_layers=2)
