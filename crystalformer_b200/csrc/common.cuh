@@ -106,6 +106,30 @@ __device__ __forceinline__ void add_compensated(float v, float &sum, float &low)
     sum = t;
 }
 
+// Eight per-lane values reduced over the warp with nine shuffles: the lanes trade halves of their value sets across lane bits
+// 4, 3, 2 (keeping the values whose index bits match their own), then finish over bits 1, 0.  Lane l ends with value l / 4.
+template <class Op>
+__device__ __forceinline__ float warp_reduce_of_8(const float (&v)[8], int lane, Op op)
+{
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
+    float w4[4], w2[2];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) w4[u] = op(b4 ? v[4 + u] : v[u], __shfl_xor_sync(FULL, b4 ? v[u] : v[4 + u], 16));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) w2[u] = op(b3 ? w4[2 + u] : w4[u], __shfl_xor_sync(FULL, b3 ? w4[u] : w4[2 + u], 8));
+    float r = op(b2 ? w2[1] : w2[0], __shfl_xor_sync(FULL, b2 ? w2[0] : w2[1], 4));
+    r = op(r, __shfl_xor_sync(FULL, r, 2));
+    return op(r, __shfl_xor_sync(FULL, r, 1));
+}
+__device__ __forceinline__ float warp_max_of_8(const float (&v)[8], int lane)
+{
+    return warp_reduce_of_8(v, lane, [](float a, float b) { return fmaxf(a, b); });
+}
+__device__ __forceinline__ float warp_sum_of_8(const float (&v)[8], int lane)
+{
+    return warp_reduce_of_8(v, lane, [](float a, float b) { return a + b; });
+}
+
 // Picks x[idx] from eight registers without dynamic indexing.
 __device__ __forceinline__ float pick8(const float (&x)[8], int idx)
 {
@@ -162,6 +186,19 @@ inline cudaError_t launch_chained_cluster(void (*kernel)(KArgs...), unsigned blo
 // the order, and whoever reads it later, only then.
 constexpr int ORDER_MAX_CRYSTALS = 2048;
 inline bool rows_are_ordered(long long B, long long N) { return B <= ORDER_MAX_CRYSTALS && N < (1ll << 31); }
+
+// Places in a block of memory, 256-byte aligned, one after the other; with a null base only their sum.
+struct Carver {
+    char *base;
+    size_t used = 0;
+    template <class T>
+    T *take(size_t count)
+    {
+        T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (count * sizeof(T) + 255) & ~(size_t)255;
+        return p;
+    }
+};
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 int sm_count();

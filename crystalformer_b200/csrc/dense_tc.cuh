@@ -116,7 +116,6 @@ void pack_layer_backward(PackJob &job, int &count, unsigned char *image, int ff,
 struct DenseBackward {
     long long N;
     int ff;
-    bool chained;
     // head (image null: none): gx = g_res + gq' Wq + gk Wk + gv Wv, gq' = gq / 4 + galpha w_pos
     const unsigned char *head;
     const float *q, *w_pos;      // the saved query (scaled by 1/4)

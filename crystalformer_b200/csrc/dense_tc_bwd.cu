@@ -78,8 +78,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
     const long long tiles = (p.N + 127) / 128;
     const int chunks = p.ff / 128;
     const bool head = p.head != nullptr, tail = p.tail != nullptr;
-    grid_launch_dependents();
-    grid_dependency_wait();  // (the images were written by a kernel of this step)
 
     if (warp == STREAM_WARP) {
         if (lane == 0) {
@@ -284,9 +282,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(
     const long long row_base = (long long)(blockIdx.x / SPLIT) * 128;
     const bool head = p.head != nullptr, tail = p.tail != nullptr;
     const bool has_head = head && rank < 3, has_chunk = tail && (int)rank < chunks, has_last = tail && rank == 0;
-    grid_launch_dependents();
     cluster_sync();  // every block's barriers are ready for the others' arrivals
-    grid_dependency_wait();  // (the images were written by a kernel of this step)
 
     if (warp == STREAM_WARP) {
         if (lane == 0) {
@@ -704,10 +700,9 @@ int launch_dense_backward(const DenseBackward &args, cudaStream_t s)
     if (rc != CF_OK) return rc;
     const long long tiles = (p.N + 127) / 128, cap = sm_count();
     if (split_tiles(tiles, p.ff, launch.clusters()))
-        launch_chained_cluster(dense_backward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, p.chained, p);
+        launch_chained_cluster(dense_backward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, false, p);
     else
-        launch_chained(dense_backward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
-                       p.chained, p);
+        dense_backward_kernel<<<(unsigned)(tiles < cap ? tiles : cap), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
     return launch_status("dense_backward_kernel");
 }
 

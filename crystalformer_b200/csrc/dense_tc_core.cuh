@@ -252,21 +252,6 @@ __device__ __forceinline__ void store_rows(float *dst, int ld, long long row_bas
     }
 }
 
-// max over the warp of eight per-lane values with nine shuffles: the lanes trade halves of their value sets across lane
-// bits 4, 3, 2, then finish over bits 1, 0.  Lane l ends with the maximum of value l / 4.
-__device__ __forceinline__ float warp_max_of_8(const float (&v)[8], int lane)
-{
-    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
-    float w4[4], w2[2];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) w4[u] = fmaxf(b4 ? v[4 + u] : v[u], __shfl_xor_sync(FULL, b4 ? v[u] : v[4 + u], 16));
-#pragma unroll
-    for (int u = 0; u < 2; ++u) w2[u] = fmaxf(b3 ? w4[2 + u] : w4[u], __shfl_xor_sync(FULL, b3 ? w4[u] : w4[2 + u], 8));
-    float r = fmaxf(b2 ? w2[1] : w2[0], __shfl_xor_sync(FULL, b2 ? w2[0] : w2[1], 4));
-    r = fmaxf(r, __shfl_xor_sync(FULL, r, 2));
-    return fmaxf(r, __shfl_xor_sync(FULL, r, 1));
-}
-
 // Loads a tile of rows as an operand: warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (fetch(row,
 // lane) returns them); the row's scale comes from its own largest magnitude, 1 / scale goes to row_floats(0).
 template <class Fetch>

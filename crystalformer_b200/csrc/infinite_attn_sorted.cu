@@ -96,31 +96,6 @@ __device__ __forceinline__ unsigned one_where_equal(unsigned pair, unsigned valu
     return *reinterpret_cast<const unsigned *>(&r);
 }
 
-// max over the warp of eight per-lane values, one per head, with nine shuffles: the lanes trade halves of their value
-// sets across lane bits 4, 3, 2 (keeping the heads whose index bits match their own), then finish over bits 1, 0.
-// Lane l ends with the maximum of head l / 4.
-__device__ __forceinline__ float warp_max_heads(const float (&v)[8], int lane)
-{
-    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
-    float w4[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const float keep = b4 ? v[4 + u] : v[u], send = b4 ? v[u] : v[4 + u];
-        w4[u] = fmaxf(keep, __shfl_xor_sync(FULL, send, 16));
-    }
-    float w2[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const float keep = b3 ? w4[2 + u] : w4[u], send = b3 ? w4[u] : w4[2 + u];
-        w2[u] = fmaxf(keep, __shfl_xor_sync(FULL, send, 8));
-    }
-    const float keep = b2 ? w2[1] : w2[0], send = b2 ? w2[0] : w2[1];
-    float r = fmaxf(keep, __shfl_xor_sync(FULL, send, 4));
-    r = fmaxf(r, __shfl_xor_sync(FULL, r, 2));
-    r = fmaxf(r, __shfl_xor_sync(FULL, r, 1));
-    return r;
-}
-
 // Shared memory of one thread block (NT key tiles of 16; PSI: with the radial basis).
 template <int NT, bool PSI>
 struct SortedSmem {
@@ -227,8 +202,8 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
                 m8[h] = fmaxf(m8[h], fmaf(a8[h] * LOG2E, dm2, s2));
             }
         }
-        M_g = warp_max_heads(m8, lane);
-        slack_g = warp_max_heads(s8, lane) - M_g;
+        M_g = warp_max_of_8(m8, lane);  // (of head lane / 4 = g)
+        slack_g = warp_max_of_8(s8, lane) - M_g;
     }
 
     // ---- the sweep: two chunks per step (their instruction streams are independent up to the accumulators)

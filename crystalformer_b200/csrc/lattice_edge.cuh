@@ -11,20 +11,6 @@
 
 namespace cf {
 
-// Sums of eight per-lane values over the warp with nine shuffles: lane l ends with the sum of value l / 4.
-__device__ __forceinline__ float warp_sum_of_8(const float (&v)[8], int lane)
-{
-    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
-    float w4[4], w2[2];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) w4[u] = (b4 ? v[4 + u] : v[u]) + __shfl_xor_sync(FULL, b4 ? v[u] : v[4 + u], 16);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) w2[u] = (b3 ? w4[2 + u] : w4[u]) + __shfl_xor_sync(FULL, b3 ? w4[u] : w4[2 + u], 8);
-    float r = (b2 ? w2[1] : w2[0]) + __shfl_xor_sync(FULL, b2 ? w2[0] : w2[1], 4);
-    r += __shfl_xor_sync(FULL, r, 2);
-    return r + __shfl_xor_sync(FULL, r, 1);
-}
-
 // The constants of a warp's edges e, e + stride, ...: lanes 0-8 carry the lattice rows, 9-11 the relative position, 12-14
 // the reciprocal row lengths, every lane the width of head lane % 8.  Three edges are under way at a time.
 struct EdgeStream {

@@ -77,20 +77,6 @@ __global__ void __launch_bounds__(HEAD_THREADS) pool_head_kernel(const float *__
     }
 }
 
-inline size_t align_up(size_t v) { return (v + 255) & ~(size_t)255; }
-
-struct Carve {
-    char *base;
-    size_t used = 0;
-    template <class T>
-    T *take(size_t count)
-    {
-        T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
-        used += align_up(count * sizeof(T));
-        return p;
-    }
-};
-
 struct Scratch {
     int64_t *atom_start, *edge_start, *batch, *row_start, *edges;
     float *pos_ij, *rvlen, *x, *encoder;
@@ -100,7 +86,7 @@ struct Scratch {
 
 Scratch carve(void *workspace, int64_t N, int64_t B, int64_t E, int64_t ff_dim)
 {
-    Carve c{static_cast<char *>(workspace)};
+    Carver c{static_cast<char *>(workspace)};
     Scratch s{};
     s.atom_start = c.take<int64_t>(B + 1);
     s.edge_start = c.take<int64_t>(B + 1);

@@ -219,18 +219,6 @@ int projection_shares(long long rows)
 }
 
 // ---- memory ----------------------------------------------------------------------------------------------------------------
-struct Carver {
-    char *base;
-    size_t used = 0;
-    template <class T>
-    T *take(size_t count)
-    {
-        T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
-        used += (count * sizeof(T) + 255) & ~(size_t)255;
-        return p;
-    }
-};
-
 enum Domain { REAL = 0, RECI = 1, RECI_INVERSE = 2, MULTIHEAD = 3 };
 constexpr int SCALARS = 9;  // gauss_scale, gauss_shift, a_factor, elu_beta, lower_bound, dist_max, a_factor_hi, lower_bound_hi, domain
 Domain domain_of(const cf_train_desc &d, int l) { return (Domain)(int)d.scalars[SCALARS * l + 8]; }
