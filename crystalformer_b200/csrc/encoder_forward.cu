@@ -301,7 +301,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     bool forked = early_prep;
     unsigned *tickets = nullptr;
     RowBlocks row_blocks{};
-    bool by_blocks = false;  // term lists and crystals of up to ROW_BLOCK_MAX_ATOMS: the row block kernel
+    bool by_blocks = false;  // term lists and rows that pay: the row block kernel
     if (pos_ij != nullptr && weight_floor_log2() > -200.0f) {
         float a_widest = -INFINITY;
         for (int l = 0; l < num_layers; ++l) a_widest = fmaxf(a_widest, (float)(scalars[6 * l + 4] * scalars[6 * l + 2]));
@@ -333,7 +333,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                 term_list_carve(logit + E * 8 + 64, N, E, &tb.start, &tb.count, &tb.dmin, &tb.cursor, &tb.pool);
                 tb.capacity = (long long)term_pool_entries(N, E);
                 rc = launch_term_list_build(tb, forked ? side.stream : s);
-                by_blocks = max_atoms > ROW_BLOCK_MIN_ATOMS && max_atoms <= ROW_BLOCK_MAX_ATOMS && num_layers <= ROW_BLOCK_LAYERS && N < (1ll << 31);
+                by_blocks = by_row_blocks(N, B, max_atoms) && num_layers <= ROW_BLOCK_LAYERS;
                 if (by_blocks && rc == CF_OK) {
                     row_blocks = row_blocks_carve(workspace + ((cf_encoder_workspace_floats(N, E, ff_dim) - (int64_t)row_blocks_words(N) - 32) & ~3ll), N);
                     rc = launch_row_blocks(row_blocks, row_order, row_start, edges, N, E, forked ? side.stream : s);

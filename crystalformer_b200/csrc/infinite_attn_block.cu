@@ -48,15 +48,18 @@ struct BlockArgs {
     BasisParams basis;
 };
 
-__host__ __device__ inline int key_stride(int max_atoms) { return (max_atoms + 1) & ~1; }
+__host__ __device__ constexpr int key_stride(int max_atoms) { return (max_atoms + 1) & ~1; }
 template <bool PSI>
-__host__ __device__ inline size_t block_floats(int max_atoms)
+__host__ __device__ constexpr size_t block_floats(int max_atoms)
 {
     // s / p table; Psi tile (before it: the partial soft-max statistics, 32 x 8 x 8 x 2); per warp the staging area and the
     // candidate ring (before them: the queries); per (row, head): a log2e, box, -lse log2e
     return (size_t)HEADS * key_stride(max_atoms) * BR_LD + (PSI ? BR_ROWS * HEADS * PSI_LD : 2 * 32 * BR_ROWS * HEADS) +
            (PSI ? BR_WARPS * BR_WARP_FLOATS : BR_ROWS * CH) + 3 * BR_ROWS * HEADS;
 }
+// two blocks per SM (228 KB, of which a block takes 1 KB for itself) up to ROW_BLOCK_MAX_ATOMS, and no further
+constexpr size_t two_blocks(int max_atoms) { return 2 * (sizeof(float) * block_floats<true>(max_atoms) + 16 + 1024); }
+static_assert(two_blocks(ROW_BLOCK_MAX_ATOMS) <= 233472 && two_blocks(ROW_BLOCK_MAX_ATOMS + 1) > 233472, "the largest crystal of two blocks per SM");
 static_assert(BR_ROWS * CH <= BR_WARPS * BR_WARP_FLOATS, "the queries fit where the warps' buffers will be");
 static_assert(2 * 32 * BR_ROWS * HEADS <= BR_ROWS * HEADS * PSI_LD, "the statistics fit where the Psi tile will be");
 

@@ -575,7 +575,7 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
     }
     static_assert(MAX_LAYERS <= ROW_BLOCK_LAYERS, "every layer has a scheduling block of its own");
     const RowBlocks row_blocks = row_blocks_carve(w.row_blocks, N);
-    const bool by_blocks = listed && b.max_atoms > ROW_BLOCK_MIN_ATOMS && b.max_atoms <= ROW_BLOCK_MAX_ATOMS;
+    const bool by_blocks = listed && by_row_blocks(N, B, b.max_atoms);
     if (by_blocks) rc = launch_row_blocks(row_blocks, order, w.row_start, w.edges, N, E, s);
     if (rc != CF_OK) return rc;
     if (w.kr != nullptr) rc = cf_reci_phase(w.pos_ij, w.rvecs, w.batch, w.edges, E, w.kr, s);

@@ -148,6 +148,14 @@ def test_saved_tensors_that_come_back_elsewhere():
     assert all(torch.equal(g, ref[n]) for n, g in grads(y).items())
 
 
+@pytest.mark.parametrize("bins", [0, 64])
+@pytest.mark.parametrize("sizes", [[65] * 12, [64] * 12, [210, 100, 1] * 4, [211, 100, 1] * 4, [66] + [31] * 30, [66] + [32] * 30, [150] * 4 + [139],
+                                   [150] * 4 + [140], [200, 3, 77] * 8])
+def test_forward_by_blocks_of_rows_or_not(sizes, bins):
+    """Both sides of every line of the rule: crystals of 64 and 65, of 210 and 211 atoms, 32 atoms on average, 740 rows."""
+    test_forward_at_the_edges_of_its_dispatch(sizes, (10.0, 20.0), bins)
+
+
 class Scaled(torch.nn.Linear):
     def forward(self, x):
         return 1.5 * super().forward(x)
