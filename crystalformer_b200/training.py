@@ -128,12 +128,13 @@ class TrainPlan:
 
 
 def usable(p: torch.Tensor, device) -> bool:
-    return p.dtype == torch.float32 and p.is_contiguous() and p.device == device
+    return p.dtype == torch.float32 and p.is_contiguous() and p.device == device and p.data_ptr() % 16 == 0
 
 
 def supported(model) -> bool:
     """Whether the submodules are the model's own (a parametrised one has a class of its own) and the parameters what the
-    kernels read: float32, contiguous, on one GPU, one projection per head."""
+    kernels read: float32, contiguous, 16-byte aligned (a parameter may be a view into a longer one), on one GPU, one
+    projection per head."""
     from .attention import CrystalformerMultiheadAttentionCUDA, NonDynamicallyQuantizableLinear
     from .encoder import CrystalformerEncoderCUDA, CrystalformerEncoderLayerCUDA
     own = {torch.nn.Linear, NonDynamicallyQuantizableLinear, torch.nn.Identity, torch.nn.ReLU, torch.nn.Dropout, torch.nn.Sequential,

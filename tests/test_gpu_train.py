@@ -156,6 +156,25 @@ def test_forward_by_blocks_of_rows_or_not(sizes, bins):
     test_forward_at_the_edges_of_its_dispatch(sizes, (10.0, 20.0), bins)
 
 
+def test_parameters_that_are_views_at_odd_places():
+    """Parameters flattened into one vector: what the kernels' wide loads cannot read takes the operation-by-operation path."""
+    model, data, target = setup([9, 20, 5], num_layers=2, value_pe_dist_real=0)
+    ref = step(model, data, target, native=False)
+    trained = [p for p in model.parameters() if p.requires_grad]
+    flat = torch.empty(sum(p.numel() for p in trained) + 1, device="cuda")
+    at = 1
+    for p in trained:
+        flat[at:at + p.numel()] = p.data.reshape(-1)
+        p.data = flat[at:at + p.numel()].view(p.shape)
+        at += p.numel()
+    model._train_plan = None
+    got = step(model, data, target, native=True)
+    assert model._train_plan is None
+    assert (got[0] - ref[0]).abs().max() < 2e-6
+    for n, g in ref[1].items():
+        assert (got[1][n] - g).norm() <= 2e-3 * g.norm() + 1e-9, n
+
+
 class Scaled(torch.nn.Linear):
     def forward(self, x):
         return 1.5 * super().forward(x)
