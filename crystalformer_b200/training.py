@@ -232,10 +232,11 @@ def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[
     if data.x.requires_grad or data.pos.requires_grad or data.trans_vec.requires_grad or torch.is_autocast_enabled() \
             or forward_ad._current_level >= 0:  # (forward-mode derivatives are on: an input may carry a tangent)
         return None
-    # the kernels get addresses: what does not have the model's shapes, or lies elsewhere, is left to the operators' own checks
+    # the kernels get addresses: what does not have the model's shapes and types, or lies elsewhere, is left to the operators' own checks
     dev, sizes = data.pos.device, data.sizes
-    if data.x.device != dev or data.trans_vec.device != dev or sizes.dim() != 1 or sizes.shape[0] < 1 or data.pos.dim() != 2 \
-            or data.pos.shape[1] != 3 or tuple(data.x.shape) != (data.pos.shape[0], plan.desc.feature_dim) \
+    if data.x.device != dev or data.trans_vec.device != dev or data.x.dtype != torch.float32 or data.trans_vec.dtype != torch.float32 \
+            or sizes.dim() != 1 or sizes.shape[0] < 1 or data.pos.dim() != 2 or data.pos.shape[1] != 3 \
+            or tuple(data.x.shape) != (data.pos.shape[0], plan.desc.feature_dim) \
             or data.trans_vec.numel() != 9 * sizes.shape[0]:
         return None
     f32 = lambda t: t if (t.dtype == torch.float32 and t.is_contiguous()) else t.detach().float().contiguous()

@@ -59,6 +59,17 @@ def test_narrow_features(model_and_batch):
         assert torch.allclose(model(narrow), model(padded), rtol=0.0, atol=1e-6)
 
 
+@pytest.mark.parametrize("name", ["x", "trans_vec"])
+def test_other_types_in_training(model_and_batch, name):
+    """Training refuses features and cells of another type, as its operators do; positions are converted."""
+    model, data = model_and_batch
+    model.train()
+    with pytest.raises((RuntimeError, TypeError)):
+        model(types.SimpleNamespace(**dict(data, **{name: data[name].double()})))
+    y = model(types.SimpleNamespace(**dict(data, pos=data["pos"].double())))
+    assert torch.equal(y, model(types.SimpleNamespace(**data)))
+
+
 def test_atoms_beyond_the_crystals(model_and_batch):
     """Rows that no crystal owns are not part of the batch (inference)."""
     model, data = model_and_batch
