@@ -169,8 +169,12 @@ __global__ void __launch_bounds__(512) project_back_kernel(const float *__restri
     for (long long e0 = (long long)blockIdx.x * UP_ROWS; e0 < E; e0 += (long long)gridDim.x * UP_ROWS) {
         const int rows = (int)min((long long)UP_ROWS, E - e0);
         __syncthreads();
-        for (int i = tid; i < rows * 32; i += 512)
-            reinterpret_cast<float4 *>(go)[i] = __ldg(reinterpret_cast<const float4 *>(gv + e0 * HEADS * HEAD_DIM) + i);
+        const float *src = gv + e0 * HEADS * HEAD_DIM;
+        if ((reinterpret_cast<uintptr_t>(gv) & 15) == 0) {
+            for (int i = tid; i < rows * 32; i += 512) reinterpret_cast<float4 *>(go)[i] = __ldg(reinterpret_cast<const float4 *>(src) + i);
+        } else {  // (a view into something longer)
+            for (int i = tid; i < rows * 128; i += 512) go[i] = __ldg(src + i);
+        }
         __syncthreads();
 #pragma unroll 4
         for (int r = 0; r < rows; ++r) {

@@ -126,3 +126,17 @@ def test_fused_backward_against_oracle_chain(ops, cutoff, minimum, nmax, Kbins):
         assert rel_err(gW.cpu().numpy(), rW[0]) < TOL
     again = fused_grads(ops, cb, edges, pos_ij, rvlen, q, k, v, a, Wn, go, Kbins, cutoff, minimum)
     assert torch.equal(ga, again[4]) and torch.equal(gq, again[1]) and torch.equal(gk, again[2])
+
+
+def test_lattice_sum_backward_takes_gradients_that_are_views(ops):
+    """A contiguous gradient that lies at an odd place of a longer tensor: the same bits as the aligned one."""
+    cb, edges, pos_ij, rvlen, a, W, rng = random_case(73, 4, 7)
+    N, E = cb.num_atoms, edges.shape[1]
+    base = (dev(a), dev(pos_ij), dev(cb.trans_vec), dev(cb.batch), dev(edges))
+    kw = dict(W=dev(W), rvlen=dev(rvlen), cutoff_radius=-3.5, lattice_range=2, minimum_range=2)
+    z, _ = ops.lattice_sum_fwd(*base, K, DIST_MAX, WSCALE, **kw)
+    gz, gv = dev(rng.standard_normal((E, H)).astype(np.float32)), dev(rng.standard_normal((E, H, D)).astype(np.float32))
+    odd = torch.empty(gv.numel() + 1, device="cuda")[1:].view(gv.shape).copy_(gv)
+    row_start = dev(oracle.row_starts(edges, N))
+    ref, got = (ops.lattice_sum_bwd(*base, row_start, z, gz, g, K, DIST_MAX, WSCALE, **kw) for g in (gv, odd))
+    assert odd.data_ptr() % 16 == 4 and all(torch.equal(r, o) for r, o in zip(ref, got))
