@@ -404,9 +404,7 @@ def run_b200(args):
         y_direct = model(resident, counts=(n_atoms, n_edges, max_atoms), **({} if peers is None else {"gather": peers}))
     if peers is not None:
         peers.wait_ready()
-    # (the served forward keeps one dense block per tile, the direct one shares a tile between four: sums in another order)
-    e2e_difference = float((y_served - y_direct.cpu()).abs().max() / y_direct.abs().max())
-    e2e_equal = e2e_difference < 2e-6
+    e2e_equal = bool(torch.equal(y_served, y_direct.cpu()))
     # ---- the same stream with the species as indices (z: the position of the 1 in every one-hot row of x), the
     #      predictor's compact input: 8 bytes per atom go to the device instead of 4 x 98; a shorter run, reported beside
     #      the figure above, which uses the reference's input format
@@ -499,7 +497,7 @@ def run_b200(args):
                     "host_issue_ms_per_step": e2e_issue * 1e3 / e2e_steps,
                     "clock": "host wall clock (perf_counter) from the first submit to the last result of one uninterrupted "
                              "stream of timed_steps batches (pipeline fill and drain inside the clock), max over ranks",
-                    "outputs_equal_direct_forward": e2e_equal, "outputs_max_rel_difference": e2e_difference,
+                    "outputs_equal_direct_forward": e2e_equal,
                     "api": f"crystalformer_b200.serving.PipelinedPredictor, {e2e_depth} batches in flight on {e2e_streams} compute stream(s)"},
             "e2e_species_indices": e2e_z,
             "gpu_launches": None if launches is None else launches * args.steps,

@@ -322,7 +322,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
 }
 
 // The same for a cluster of four blocks (dense_tc_core.cuh): block r takes hidden chunk r and, of q, k, v, matrix r.  Hidden
-// units go to operand buffer 0 (y has been multiplied by then), buffer 1 takes the shares of the output sum.
+// units go to operand buffer 0 (y has been multiplied by then), buffer 1 takes the shares of the output sum.  Every value
+// comes from the same operations in the same order as in a block per tile: the outputs are the same bits.
 // 2,027 rows, 512 hidden units, a boundary inside the network: 31 us with a block per tile, 20 here (unchained).
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(const DenseForward p)
 {
@@ -413,27 +414,24 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
             float hs[4], hi[4];
             hidden_scales(ws, xi, hs, hi);
             if (has_chunk) hidden_units(p, s, pl, ph, tmem, D0, B_D0, rank, row_base, xi, ws.w1, hs, OFF_A0, B_A0, false);
+            if (mine && pl.group == 0 && pl.t == 0) {  // the scales of the finished rows, for the threads that finish them
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s.row_floats(3)[pl.g + 8 * i] = hi[i] * ws.w2;
+            }
+            epilogue_sync();  // (and y is no longer being written to buffer 0, which is about to take the shares)
             const float2 b2_lo = *reinterpret_cast<const float2 *>(p.b2 + 4 * lane), b2_hi = *reinterpret_cast<const float2 *>(p.b2 + 4 * lane + 2);
             if (has_chunk) {
                 ph.wait(s, B_DX);
                 fence_after();
-            } else {
-                epilogue_sync();  // (buffer 0 is about to take the shares: y is no longer being written)
             }
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
+            for (int half = 0; half < 2; ++half) {  // (the shares are the accumulators as they are: all chunks have one scale per row)
                 float d[16];
                 if (has_chunk) {
                     tmem_load_16x32(pl.tmem(tmem, DX, half), d);
                 } else {
 #pragma unroll
                     for (int i = 0; i < 16; ++i) d[i] = 0.f;
-                }
-                const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    d[4 * j] *= sa; d[4 * j + 1] *= sa;
-                    d[4 * j + 2] *= sb; d[4 * j + 3] *= sb;
                 }
                 stage_share(s, pl, half, d);
             }
@@ -443,8 +441,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(c
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const float4 y = staged_row(s.mem + OFF_OWN, 2 * warp + u, lane);
-                v[u].x = y.x + (v[u].x + b2_lo.x); v[u].y = y.y + (v[u].y + b2_lo.y);
-                v[u].z = y.z + (v[u].z + b2_hi.x); v[u].w = y.w + (v[u].w + b2_hi.y);
+                const float sc = s.row_floats(3)[2 * warp + u];
+                v[u].x = y.x + fmaf(v[u].x, sc, b2_lo.x); v[u].y = y.y + fmaf(v[u].y, sc, b2_lo.y);
+                v[u].z = y.z + fmaf(v[u].z, sc, b2_hi.x); v[u].w = y.w + fmaf(v[u].w, sc, b2_hi.y);
             }
             if (head) spread_rows(s, ph, rank, v, 3, 0);
 #pragma unroll

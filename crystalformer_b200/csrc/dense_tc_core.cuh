@@ -284,10 +284,10 @@ __device__ __forceinline__ void load_operand(const Shared &s, unsigned char *buf
 // ---- a tile shared by four blocks ---------------------------------------------------------------------------------------
 // A boundary is a chain of twelve products per tile, about a microsecond each on one SM's tensor pipe; with few tiles most
 // SMs have none.  A cluster of four blocks then takes a tile: block r multiplies hidden chunk r and head matrix r, products
-// that precede them are done by all four.  Where the chunks meet in one sum, every block sends its share (already in units
-// of the result) of rows 32 o .. 32 o + 31 to block o (slot r of operand buffer 1, which these blocks do not use
-// otherwise); block o adds the four in rank order, finishes its 32 rows and, where they are the next operand, writes them
-// into operand buffer 0 of every block that needs them.  Both transfers are bulk copies between the blocks' shared
+// that precede them are done by all four.  Where the chunks meet in one sum, every block sends its share of rows
+// 32 o .. 32 o + 31 to block o (slot r of operand buffer 1, which these blocks do not use otherwise); block o adds the four
+// in rank order, finishes its 32 rows and, where they are the next operand, writes them into operand buffer 0 of every
+// block that needs them.  Both transfers are bulk copies between the blocks' shared
 // memories, from a staging place of the sender (shares: its operand buffer 0; finished rows: the third stage of the weight
 // ring, which these blocks do without) with the bytes counted on the receiver's barrier, B_PART and B_ROWS: 3.5 us for the
 // shares and 2.2 for the rows, against 3.9 and 2.7 with plain stores to the other blocks (48 KB leave every block: about 17

@@ -79,3 +79,26 @@ def test_boundaries_shared_by_a_cluster_or_not(ff, atoms):
     for n, g in grads[False].items():
         # (a hidden unit within rounding of zero may fall on either side of the ReLU)
         assert (grads[True][n] - g).norm() <= 2e-3 * g.norm() + noise, n
+
+
+@pytest.mark.parametrize("ff", [128, 384, 512])
+@pytest.mark.parametrize("atoms", [1, 33, 200, 2000])
+def test_outputs_do_not_depend_on_how_a_batch_is_issued(ff, atoms):
+    """A forward whose tiles are shared by four blocks, and the serving pipeline on several streams, which keeps a block per tile."""
+    from crystalformer_b200.model import Latticeformer, default_params
+    from crystalformer_b200.serving import PipelinedPredictor
+    torch.manual_seed(atoms + ff)
+    model = Latticeformer(default_params(num_layers=2, ff_dim=ff)).cuda()
+    for p in model.parameters():
+        if p.requires_grad:
+            p.data.add_(torch.randn_like(p) * 0.05)
+    sizes = [min(atoms, 20)] * max(1, atoms // 20)
+    cb = make_crystals(4, len(sizes), lambda rng, b: np.array(sizes), length_range=(4.0, 12.0))
+    host = types.SimpleNamespace(x=torch.as_tensor(cb.x).pin_memory(), pos=torch.as_tensor(cb.pos).pin_memory(),
+                                 trans_vec=torch.as_tensor(cb.trans_vec).pin_memory(), sizes=torch.as_tensor(cb.sizes).pin_memory())
+    data = types.SimpleNamespace(**{n: t.cuda() for n, t in vars(host).items()})
+    with torch.no_grad():
+        model.train()(data)
+        direct = model.eval()(data)
+    runner = PipelinedPredictor(model, depth=2, streams=2)
+    assert torch.equal(runner.result(runner.submit(host)), direct.cpu())
