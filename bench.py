@@ -866,8 +866,8 @@ def lattice_microbench(ops, device, peaks, pairs=250000):
             "algorithmic_sfu_rate_over_probe": terms * sfu_per_term(64) / t / peaks["sfu"],
             "note": "algorithmic = every (edge, translation) term of the boxes x the reference's per-term instruction "
                     "count, divided by the time: the kernels skip terms below the weight floor, so this is a speed-up "
-                    "over the enumeration, not a pipe utilisation (ncu: XU 37 %, ALU 43 %, FMA 22 % of peak, "
-                    "profiles/ncu_full_lattice_psi_microbench80k.md)",
+                    "over the enumeration, not a pipe utilisation (ncu, 218,302 pairs: XU 27 %, ALU 37 %, FMA 30 % of "
+                    "peak, profiles/ncu_attention_large_cells_training_lattice.md)",
             "hbm_gbs": out_bytes / t / 1e9, "hbm_frac": out_bytes / t / 6558.7e9,
             "kernels": "lattice_edge_kernel", "l2": "output 520 MB per launch exceeds L2"}
 

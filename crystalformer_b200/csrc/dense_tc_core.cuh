@@ -13,8 +13,8 @@
 // rounded to nearest, from an accumulator per product.  What is still lost is mostly a factor: the eight additions take
 // 1.6e-7 of the result on average (regression on the operands of training steps, 1.2e-7 to 1.6e-7), of which the scales of
 // the weights give 2^-23 back (not the embedding's: sums of one element per row lose nothing).
-// Relative errors against 64 bits, float32 GEMMs on the same operands in brackets: 128-deep product 1.3e-7 (2.0e-7), 512-deep
-// sum of chunks 2.3e-7 (3.5e-7); with the piece products in turn and the chunks in one accumulator 4.8e-7 and 1.8e-6; the
+// Relative errors against 64 bits, float32 GEMMs on the same operands in brackets: 128-deep product 1.4e-7 (2.0e-7), 512-deep
+// sum of chunks 2.5e-7 (3.5e-7); with the piece products in turn and the chunks in one accumulator 4.8e-7 and 1.8e-6; the
 // TF32 + bfloat16 split of the warp-level version has 2^-20 per term.
 #pragma once
 #include "dense_tc.cuh"

@@ -312,8 +312,9 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
             if (!early_prep && begun == nullptr)
                 forked = side.ok && cudaEventRecord(side.fork, s) == cudaSuccess &&
                          cudaStreamWaitEvent(side.stream, side.fork, 0) == cudaSuccess;
-            // (without a basis the enumerating kernel with term lists is faster - 0.62 against 0.79 ms for a 7-layer
-            // forward of 256 crystals of up to 60 atoms - so K = 0 keeps it)
+            // (K = 0 keeps the row kernel with term lists: a 7-layer forward of 256 crystals of log-normal size up to 60 atoms
+            // takes 569 us that way and 595 sorted, 128 of 1-30 468 and 456, 256 of 1-40 880 and 1,084, 64 of 40-64 822 and 994;
+            // only 1,024 of 1-60 would gain, 4.39 and 3.62 ms)
             sorted_rows = sorted_rows_enabled() && K == 64 && max_atoms <= ROW_LIST_MAX_KEYS && N < (1ll << 31) && E < (1ll << 31);
             if (sorted_rows) {
                 RowListBuild rb{};

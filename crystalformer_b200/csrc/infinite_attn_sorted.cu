@@ -25,7 +25,7 @@
 // Rows without a list, rows of more than 16 NT keys and rows where a head's sum comes out empty are appended to the
 // left-over list and processed by the enumerating row kernel (infinite_attn_fwd.cu) afterwards.  Without a radial
 // basis (K = 0: PSI = false) the histogram, its tiles and the projection W drop out; the rest is the same (the
-// one-call forwards do not use that variant: there the enumerating kernel with term lists is faster).
+// one-call forwards do not use that variant, see encoder_forward.cu).
 #include <cuda_fp16.h>
 
 #include "lattice_core.cuh"

@@ -15,12 +15,13 @@ constexpr size_t RL_SMEM = sizeof(unsigned long long) * ROW_LIST_CAP + sizeof(un
 // One thread block per row.  Every key's candidate translations (a bounding box of the ball that holds its listed
 // terms) are walked by a warp, one per lane and step; terms within `window` of their edge's nearest image are appended to a
 // shared-memory buffer (one atomic per warp and step) as 64-bit items (d2 bits << 32 | key) and counted in their bucket:
-// RL_BUCKETS buckets, equally spaced in d^3 (terms are about uniform in volume, so buckets hold a handful of items each).
-// The items' indices are then distributed over the buckets and placed inside their bucket by counting the smaller items of
-// the same bucket.  The 64-bit items are distinct except for exact duplicates, so the result does not depend on the order
-// in which the atomics arrived.  Eight warps per row: most of a row's cost is per thread (set-up, scans, barriers), not
-// per item.  Bound by latency (issue slots 40 % busy): what is moved is 16-bit indices and not the items, which makes room
-// for a fourth block per SM; 31,000 rows of 1,000 entries 0.99 -> 0.89 ms, 2,000 of 650 52 -> 47 us.
+// RL_BUCKETS buckets, about equally spaced in d^3 (terms are about uniform in volume, so buckets hold a handful of items
+// each).  The items stay where they are: their 16-bit indices are distributed over the buckets and placed inside their
+// bucket by counting the smaller items of the same bucket.  The 64-bit items are distinct except for exact duplicates, so
+// the result does not depend on the order in which the atomics arrived.  Eight warps per row: most of a row's cost is per
+// thread (set-up, scans, barriers), not per item.  Bound by latency (issue slots 40 % busy); 16-bit indices in place of a
+// second copy of the items leave room for four blocks per SM instead of three: 31,000 rows of 1,000 entries 0.99 -> 0.89 ms,
+// 2,000 of 650 52 -> 47 us.
 __global__ void __launch_bounds__(RL_THREADS) row_list_build_kernel(const RowListBuild p)
 {
     extern __shared__ __align__(16) unsigned long long rl_smem[];

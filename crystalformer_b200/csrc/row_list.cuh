@@ -19,8 +19,8 @@
 //   sched   [ROW_SCHED_SLOTS][4] unsigned: per attention call { ticket of the shared rows, rows left over, ticket of
 //           the left-over launch, ticket of the one-warp rows }; zeroed by the build
 //   leftover[N] int: atoms whose row the sorted kernel could not process (no list, or a head whose box misses the list)
-//   tasks   [2][N] int + two counters: the slots of the rows with long lists (shared by the four warps of a block) and
-//           of all other rows (one warp each), in the order in which the build finished them
+//   tasks   [2][N] int + two counters: the slots of the rows with long lists (shared by the warps of a block) and of
+//           all other rows (one warp each), in the order in which the build finished them
 //   pool    entries (d2, key) with key = j | |n1| << 8 | |n2| << 16 | |n3| << 24; a row's entries are contiguous,
 //           ascending in d2, padded to a multiple of eight with copies of the last d2 whose key (0x7f7f7f00) lies
 //           outside every box

@@ -36,8 +36,9 @@ __device__ __forceinline__ void digit_range(float rho, float len, float s, int R
     hi = (int)floorf(fminf(m - s, (float)R));
 }
 
-// One warp per row, one key per lane (rows of few keys: several lanes, which deal the columns of the key's box): threshold, box and terms of a key are its lane's own work (two walks of the box, to
-// count and to fill), the offsets of a chunk of 32 keys come from a scan over the lanes.  A box holds about twice the
+// One warp per row, one key per lane, or several lanes where the row has few keys (they deal the columns of the key's box
+// among themselves).  Threshold, box and terms of a key are its lanes' own work (two walks of the box, to count and to
+// fill); the offsets of a chunk of keys come from a scan over the lanes.  A box holds about twice the
 // listed terms, whatever the cell: the walk of the rule's box by columns that this replaces took 0.53 ms for 64 crystals
 // of 100-200 atoms (1.5 M edges, 3 terms each), this one 0.15 ms.
 __global__ void __launch_bounds__(32 * TL_WARPS) term_list_build_kernel(const TermListBuild p)

@@ -39,8 +39,9 @@ class PipelinedPredictor:
         side and fill each other's idle issue slots (they are latency-bound), at the price of a longer latency per
         batch; with a ``gather`` only if it overlaps its collects (its steps must otherwise run in one order on every
         rank's one stream).  ``dense_tile_rows`` (16, 32 or 0 = chosen per launch; default 32 with several streams, else
-        0): the row tile of the fused dense blocks when batches are submitted through the library's one-call path:
-        with 32 the blocks take a little longer per forward and less SM time in total, which pays once streams overlap."""
+        0): how the dense boundaries are launched when batches are submitted through the library's one-call path
+        (cf_model_desc): with 32 they take a little longer per forward and less SM time in total, which pays once streams
+        overlap.  The outputs are the same bits."""
         if depth < 1:
             raise ValueError("depth must be at least 1")
         self.model = model

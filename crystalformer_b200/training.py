@@ -35,15 +35,16 @@ class ModelWatch:
     """Notices when a model is no longer the one a plan was made for: a submodule, parameter or buffer replaced, moved or
     (with ``versions``) modified in place, or a setting changed."""
 
-    def __init__(self, model, versions: bool):
-        children = [(m._modules, n, c) for m in model.modules() for n, c in m._modules.items()]
-        places = [(d, n, t) for m in model.modules() for d in (m._parameters, m._buffers) for n, t in d.items() if t is not None]
+    def __init__(self, model, versions: bool, modules=None):
+        modules = list(model.modules()) if modules is None else modules
+        children = [(m._modules, n, c) for m in modules for n, c in m._modules.items()]
+        places = [(d, n, t) for m in modules for d in (m._parameters, m._buffers) for n, t in d.items() if t is not None]
         self.tensors = [t for _, _, t in places]
         self.dicts, self.names, self.values = zip(*(children + places))
         self.versions = versions
         self.settings = model.encoder.lattice_params
         self.layer_settings = [layer.self_attn.params for layer in model.encoder.layers]
-        self.dropouts = [m for m in model.modules() if isinstance(m, torch.nn.Dropout)]
+        self.dropouts = [m for m in modules if isinstance(m, torch.nn.Dropout)]
         self.attentions = [layer.self_attn for layer in model.encoder.layers]
         self.key = self.now()
 
@@ -68,7 +69,7 @@ class TrainPlan:
     """What a step needs and the batch does not change: the parameters in the library's order with their addresses, the
     scalar settings, and where every gradient lies in one flat buffer.  Valid while the parameters keep their storage."""
 
-    def __init__(self, model):
+    def __init__(self, model, modules):
         enc = model.encoder
         P = enc.lattice_params
         ordered, scalars = [], []
@@ -85,8 +86,8 @@ class TrainPlan:
             scalars += [gs[0], gs[1], low[0], beta, low[1], dist_max, *high, DOMAINS.index(Q.domain)]
         ordered += [model.input_embeddings.weight, model.mlp[0].weight, model.mlp[0].bias, model.mlp[3].weight, model.mlp[3].bias]
         self.params = [p for p in ordered if p is not None]
-        self.watch = ModelWatch(model, versions=False)
-        self.submodules = [m.__dict__ for m in model.modules() if m is not model]
+        self.watch = ModelWatch(model, False, modules)
+        self.submodules = [m.__dict__ for m in modules if m is not model]
         self.scales = [layer.self_attn.gauss_scale for layer in enc.layers]
         self.scale_versions = [g._version for g in self.scales]
         sizes = [p.numel() for p in self.params]
@@ -131,7 +132,7 @@ def usable(p: torch.Tensor, device) -> bool:
     return p.dtype == torch.float32 and p.is_contiguous() and p.device == device and p.data_ptr() % 16 == 0
 
 
-def supported(model) -> bool:
+def supported(model, modules) -> bool:
     """Whether the submodules are the model's own (a parametrised one has a class of its own) and the parameters what the
     kernels read: float32, contiguous, 16-byte aligned (a parameter may be a view into a longer one), on one GPU, one
     projection per head."""
@@ -139,7 +140,7 @@ def supported(model) -> bool:
     from .encoder import CrystalformerEncoderCUDA, CrystalformerEncoderLayerCUDA
     own = {torch.nn.Linear, NonDynamicallyQuantizableLinear, torch.nn.Identity, torch.nn.ReLU, torch.nn.Dropout, torch.nn.Sequential,
            torch.nn.ModuleList, CrystalformerEncoderCUDA, CrystalformerEncoderLayerCUDA, CrystalformerMultiheadAttentionCUDA}
-    if any(type(m) not in own for m in model.modules() if m is not model):
+    if any(type(m) not in own for m in modules if m is not model):
         return False
     enc = model.encoder
     ff = enc.layers[0].linear1.out_features if len(enc.layers) else 0
@@ -159,7 +160,7 @@ def supported(model) -> bool:
             return False
         if any(isinstance(m, torch.nn.Dropout) and m.p > 0 for m in (layer.dropout, layer.dropout1, layer.dropout2)) or att.dropout > 0:
             return False
-    return all(usable(p, dev) for p in model.parameters())
+    return all(usable(p, dev) for m in modules for p in m._parameters.values() if p is not None)
 
 
 class NotThisBatch(Exception):
@@ -223,9 +224,10 @@ def train_step(model, data, counts: Optional[Tuple[int, int, int]]) -> Optional[
     cache = getattr(model, "_train_plan", None)
     plan = None if cache is None else cache.values[0]
     if plan is None or not plan.current():
-        if not supported(model):
+        modules = list(model.modules())
+        if not supported(model, modules):
             return None
-        plan = TrainPlan(model)
+        plan = TrainPlan(model, modules)
         model._train_plan = OfThisModel(plan)
     if not plan.untouched() or not all([att.term_lists for att in plan.watch.attentions]):
         return None
