@@ -77,6 +77,7 @@ class PipelinedPredictor:
                                                              and native_ok_without_grad(self.model)) else None
         if self._plan is not None and "desc" in self._plan:
             self._plan["desc"].dense_tile_rows = self.dense_tile_rows
+        torch.cuda.current_stream(self.device).synchronize()  # (the weights are packed on this stream and read on others)
 
     def _device_inputs(self, slot: int, batch):
         """Device tensors of the slot with the batch's shapes (allocated once per shape, not per batch)."""

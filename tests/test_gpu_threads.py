@@ -102,3 +102,45 @@ def test_two_threads_on_one_stream(training):
         th.join()
     torch.cuda.synchronize()
     assert not wrong, wrong[:3]
+
+
+def test_weights_packed_behind_other_work():
+    """A pipeline is built on a stream that is busy, and its streams of its own do not wait for that one."""
+    from crystalformer_b200.serving import PipelinedPredictor
+    model, data, cb = setup(64)
+    with torch.no_grad():
+        ref = model.eval()(data).cpu()
+        model.input_embeddings.weight.mul_(1.0)  # (a new version: the embedding is packed again)
+    host = types.SimpleNamespace(x=torch.as_tensor(cb.x).pin_memory(), pos=torch.as_tensor(cb.pos).pin_memory(),
+                                 trans_vec=torch.as_tensor(cb.trans_vec).pin_memory(), sizes=torch.as_tensor(cb.sizes).pin_memory())
+    torch.cuda.synchronize()
+    torch.cuda._sleep(4_000_000)
+    runner = PipelinedPredictor(model, depth=2, streams=2)
+    assert torch.equal(runner.result(runner.submit(host)), ref)
+
+
+@pytest.mark.parametrize("bins", [0, 64])
+def test_steps_in_a_graph(bins):
+    """With the sizes given a training step queues work only, on two streams that meet again: it can be captured."""
+    model, data, cb = setup(bins)
+    model.train()
+    counts = (cb.num_atoms, cb.num_edges, int(cb.sizes.max()))
+    weights = [p for p in model.parameters() if p.requires_grad]
+
+    def step():
+        y = model(data, counts=counts)
+        return [y.detach(), *torch.autograd.grad(y.abs().mean(), weights)]
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    with torch.no_grad():
+        data.pos.mul_(1.01)
+        weights[0].mul_(1.1)
+    graph.replay()
+    assert all(torch.equal(a, b) for a, b in zip(captured, step()))
