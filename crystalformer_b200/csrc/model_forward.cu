@@ -143,6 +143,8 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
                (long long)targets, HEAD_MAX_HIDDEN);
     CF_REQUIRE(N < (1ll << 31) / 512, CF_ERR_RANGE, "cf_model_forward: N=%lld too large for 32-bit GEMM sizes", (long long)N);
     if (B == 0) return CF_OK;
+    const int waits = check_waits("cf_model_forward");  // (before anything of the batch is queued)
+    if (waits != CF_OK) return waits;
     CF_REQUIRE((features || species) && pos && trans && sizes && W_embed && W1 && b1 && W2 && b2 && workspace && y, CF_ERR_INVALID,
                "cf_model_forward: null pointer");
     // With packed weights everywhere the whole forward runs in this library's kernels and cuBLAS is not touched.

@@ -34,6 +34,8 @@ extern "C" int cf_serve_submit(const cf_model_desc *model, const cf_serve_slot *
     CF_REQUIRE(slot->copied && slot->inputs_free && slot->done && slot->x && slot->pos && slot->trans && slot->sizes &&
                    slot->workspace && slot->y && slot->y_host,
                CF_ERR_INVALID, "cf_serve_submit: incomplete slot");
+    const int waits = check_waits("cf_serve_submit");  // (before anything of the batch is queued)
+    if (waits != CF_OK) return waits;
     cudaStream_t copy = as_stream(slot->copy_stream), compute = as_stream(slot->compute_stream);
     cudaEvent_t copied = reinterpret_cast<cudaEvent_t>(slot->copied), inputs_free = reinterpret_cast<cudaEvent_t>(slot->inputs_free);
     cudaEvent_t done = reinterpret_cast<cudaEvent_t>(slot->done);

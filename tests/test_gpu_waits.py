@@ -73,6 +73,9 @@ def test_results_of_a_pipeline_raise_it(setup):
     run_out()
     with pytest.raises(_lib.CrystalformerB200Error, match="ran out"):
         runner.result(ticket)
+    run_out()
+    with pytest.raises(_lib.CrystalformerB200Error, match="ran out"):
+        runner.submit(host)
     out = runner.result(runner.submit(host))
     with torch.no_grad():
-        assert torch.allclose(out, model(data).cpu(), rtol=0.0, atol=2e-6)
+        assert torch.equal(out, model(data).cpu())
