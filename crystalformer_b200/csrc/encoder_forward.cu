@@ -75,10 +75,16 @@ SideStream &side_stream()
 
 }  // namespace
 
+// `s` made to wait for the early work of a batch.
+int join_begun(void *begun_event, cudaStream_t s)
+{
+    return cudaStreamWaitEvent(s, reinterpret_cast<cudaEvent_t>(begun_event), 0) == cudaSuccess ? CF_OK : launch_status("first block");
+}
+
 // The host's copy of a batch's sizes, for callers that only have them on the device: the copy is queued first, then
 // `launch` queues work that needs the number of atoms only on the side stream, and the host waits for the copy while that
-// runs.  counts = { atoms, edges, largest crystal }.  Pinned staging memory and the event are this thread's (at most 8 MiB,
-// returned when the thread ends).
+// runs.  counts = { atoms, edges, largest crystal }.  Pinned staging memory (at most 8 MiB, returned when the thread ends)
+// and the events are this thread's.
 // It is the early work that goes to the side stream and the rest of the batch's that stays on `s`: the memory of the rest is
 // allocated after the wait, in the order of `s`, when other host threads may have queued work on `s` and freed their
 // memory to it, so nothing but `s` itself may touch that memory first.  The early work writes only what was allocated
@@ -101,11 +107,6 @@ struct PinnedSizes {
     }
 };
 }  // namespace
-// `s` made to wait for the early work of a batch.
-int join_begun(void *begun_event, cudaStream_t s)
-{
-    return cudaStreamWaitEvent(s, reinterpret_cast<cudaEvent_t>(begun_event), 0) == cudaSuccess ? CF_OK : launch_status("first block");
-}
 int read_sizes_beside(const int64_t *sizes, int64_t B, int64_t *counts, cudaStream_t s, int (*launch)(void *, cudaStream_t), void *arg,
                       void **begun_event)
 {
