@@ -58,6 +58,8 @@ WORKLOADS = {
 FIXED_BOX_TERMS = 125  # (2 R + 1)^3 with the default lattice_range R = 2
 PARITY_TOL = 1e-4
 SM_FP32_LANES, SM_SFU_LANES = 128, 16  # FP32 and MUFU lane-instructions per clock and SM
+SM_SHARED_BYTES = 128  # shared memory, per clock and SM
+HBM_BYTES_PER_S = 6558.7e9  # measured copy
 
 
 def fp32_instr_per_term(K, H=8):
@@ -544,21 +546,35 @@ def attention_roofline(ops, device, model, step, wl, n_atoms, n_edges, max_atoms
                    "note": "work of the reference's enumeration of every (edge, translation) term divided by this "
                            "kernel's time: a speed-up over that algorithm, not a utilisation (the kernel reads "
                            "precomputed lists and skips terms below the weight floor)"}
-    sorted_path = K == 64 and max_atoms <= 32
-    executed = None
-    traffic = None
-    if sorted_path:
-        # counters of the sorted row kernel over one extra, untimed forward
-        words = torch.zeros(4, dtype=torch.int64, device=device)
-        ops.set_row_stats(words)
-        try:
-            step()
-            torch.cuda.synchronize()
-        finally:
-            ops.set_row_stats(None)
-        chunks, tiles, rows = (int(v) / layers for v in words[:3].tolist())
-        # per lane and chunk: 2 ex2 (weights), and a quarter of an rsqrt; per (chunk, tile): 4 ex2 (basis values).  FP32-pipe:
-        # about 18 per chunk (exponents, basis coordinates, operand splits) and 20 per (chunk, tile).
+    # counters of the attention kernel over one extra, untimed forward
+    words = torch.zeros(4, dtype=torch.int64, device=device)
+    ops.set_row_stats(words)
+    try:
+        step()
+        torch.cuda.synchronize()
+    finally:
+        ops.set_row_stats(None)
+    chunks, tiles, rows, products = (int(v) / layers for v in words.tolist())
+    atoms_io = n_atoms * 4 * (3 * 128 + 8 + 128 + 8)  # q, k, v, a in / out, lse out once per atom
+    common = {"algorithmic": algorithmic, "launches": op_calls, "avg_launch_us": t_call * 1e6,
+              "share_of_step": t_call * 1e3 * layers / ms_step, "peaks": peaks,
+              "traffic_unit": "bytes per call, from the run's own sizes and counters (see profiles/ for the ncu dram__bytes figure "
+                              "of the same kernel)"}
+    if products > 0:
+        # attention over pair grids: a product of 16 keys and 16 nodes moves 1 KB of half pairs into shared memory and out of it
+        # twice (both orientations), and is six tensor instructions
+        moved, peak = 3 * 1024 * products, sms * SM_SHARED_BYTES * clock_hz
+        traffic = 1024 * products + atoms_io
+        return {"kernel": "pair_attn_kernel (+ the launch for left-over rows): one attention call", "bound": "shared memory", "unit": "GB/s",
+                "achieved": moved / t_call / 1e9, "peak": peak / 1e9, "frac": moved / t_call / peak,
+                "peak_source": f"{sms} SMs x {SM_SHARED_BYTES} bytes x {clock_hz / 1e9:.3f} GHz (nominal)",
+                "executed": {"products_per_call": products, "rows_per_call": rows, "mma_m16n8k16_per_call": 6 * products,
+                             "shared_memory_bytes": moved},
+                "traffic": traffic, "hbm_frac_if_streamed": traffic / t_call / HBM_BYTES_PER_S, **common}
+    executed = traffic = None
+    if chunks > 0:
+        # sorted row kernel.  Per lane and chunk: 2 ex2 (weights), and a quarter of an rsqrt; per (chunk, tile): 4 ex2 (basis
+        # values).  FP32-pipe: about 18 per chunk (exponents, basis coordinates, operand splits) and 20 per (chunk, tile).
         sfu_ops = 32 * (2.25 * chunks + 4 * tiles)
         fp32_ops = 32 * (18 * chunks + 20 * tiles)
         t_sfu, t_fp32 = sfu_ops / nominal["sfu"], fp32_ops / nominal["fp32"]
@@ -567,25 +583,19 @@ def attention_roofline(ops, device, model, step, wl, n_atoms, n_edges, max_atoms
                     "mma_m16n8k16_per_call": (4 * chunks + 3 * tiles) / 2,
                     "sfu_frac": t_sfu / t_call, "fp32_frac": t_fp32 / t_call,
                     "sfu_frac_of_probe": sfu_ops / peaks["sfu"] / t_call}
-        # bytes the call has to move at least: the list entries it sweeps, the row directory and per-edge minima, and
-        # q, k, v, a in / out, lse out once per atom
-        traffic = 64 * chunks + 32 * n_atoms + 4 * n_edges + n_atoms * 4 * (3 * 128 + 8 + 128 + 8)
-    frac = executed["sfu_frac"] if executed else None
+        # bytes the call has to move at least: the list entries it sweeps, the row directory and per-edge minima, the atoms
+        traffic = 64 * chunks + 32 * n_atoms + 4 * n_edges + atoms_io
     return {
         "kernel": ("infinite_attn_sorted_rows_kernel (+ the launch for left-over rows): one attention call"
-                   if sorted_path else "phi_from_list_kernel + infinite_attn_rows_kernel: one attention call"),
+                   if chunks > 0 else "phi_from_list_kernel + infinite_attn_rows_kernel: one attention call"),
         "bound": "sfu", "unit": "G MUFU lane-ops/s",
         "achieved": None if executed is None else executed["sfu_lane_ops"] / t_call / 1e9,
-        "peak": nominal["sfu"] / 1e9, "frac": frac,
+        "peak": nominal["sfu"] / 1e9, "frac": executed["sfu_frac"] if executed else None,
         "peak_source": f"{sms} SMs x {SM_SFU_LANES} MUFU lanes x {clock_hz / 1e9:.3f} GHz (nominal); cf_pipe_probe measured "
                        f"{peaks['sfu'] / 1e9:.0f} G MUFU/s and {peaks['fp32'] / 1e9:.0f} G FFMA/s in this run "
                        "(MEASURED_PEAKS.json holds HBM and bf16 figures only)",
-        "executed": executed, "algorithmic": algorithmic, "launches": op_calls, "avg_launch_us": t_call * 1e6,
-        "share_of_step": t_call * 1e3 * layers / ms_step,
-        "traffic": traffic, "traffic_unit": "bytes per call, from the run's own sizes and counters (see profiles/ for the "
-                                            "ncu dram__bytes figure of the same kernel)",
-        "hbm_frac_if_streamed": None if traffic is None else traffic / t_call / 6558.7e9,
-        "peaks": peaks,
+        "executed": executed, "traffic": traffic,
+        "hbm_frac_if_streamed": None if traffic is None else traffic / t_call / HBM_BYTES_PER_S, **common,
     }
 
 

@@ -21,6 +21,7 @@
 #include "dense_block.cuh"
 #include "dense_tc.cuh"
 #include "infinite_attn_block.cuh"
+#include "pair_grid.cuh"
 #include "row_list.cuh"
 #include "term_list.cuh"
 
@@ -30,7 +31,8 @@ int encoder_forward_impl(void *cublas_handle, int num_layers, const float *const
                          const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t E,
                          int64_t max_atoms, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius,
                          int lattice_range, int minimum_range, float *workspace, const int32_t *row_order,
-                         void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun);
+                         void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun,
+                         const GridMemory *grid_memory);
 int infinite_attn_fwd_impl(const float *q, const float *k, const float *v, const float *a, const float *pos,
                            const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *batch,
                            const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t H, int64_t D,
@@ -260,7 +262,7 @@ extern "C" int cf_encoder_forward(void *cublas_handle, int num_layers, const flo
 {
     return cf::encoder_forward_impl(cublas_handle, num_layers, weights, scalars, x, pos_ij, tvecs, rvlen, batch, edges,
                                     row_start, N, B, E, max_atoms, K, ff_dim, wscale, cutoff_radius, lattice_range,
-                                    minimum_range, workspace, row_order, attn_events, stream, nullptr, false, nullptr);
+                                    minimum_range, workspace, row_order, attn_events, stream, nullptr, false, nullptr, nullptr);
 }
 
 // cf_encoder_forward with an optional embedding stage (dense path only): x is then written by the first dense block.
@@ -269,7 +271,8 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                              const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t E,
                              int64_t max_atoms, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius,
                              int lattice_range, int minimum_range, float *workspace, const int32_t *row_order,
-                             void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun)
+                             void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun,
+                             const GridMemory *grid_memory)
 {
     CF_REQUIRE(N >= 0 && E >= 0 && num_layers >= 0, CF_ERR_INVALID, "cf_encoder_forward: negative size");
     CF_REQUIRE(ff_dim > 0 && ff_dim % 4 == 0, CF_ERR_UNSUPPORTED, "cf_encoder_forward: ff_dim must be a positive multiple of 4");
@@ -303,6 +306,8 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     unsigned *tickets = nullptr;
     RowBlocks row_blocks{};
     bool by_blocks = false;  // term lists and rows that pay: the row block kernel
+    PairAttn by_grid{};      // (call: -1 where there are no pair grids)
+    by_grid.call = -1;
     if (pos_ij != nullptr && weight_floor_log2() > -200.0f) {
         float a_widest = -INFINITY;
         for (int l = 0; l < num_layers; ++l) a_widest = fmaxf(a_widest, (float)(scalars[6 * l + 4] * scalars[6 * l + 2]));
@@ -313,11 +318,24 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
             if (!early_prep && begun == nullptr)
                 forked = side.ok && cudaEventRecord(side.fork, s) == cudaSuccess &&
                          cudaStreamWaitEvent(side.stream, side.fork, 0) == cudaSuccess;
-            // (K = 0 keeps the row kernel with term lists: a 7-layer forward of 256 crystals of log-normal size up to 60 atoms
-            // takes 569 us that way and 595 sorted, 128 of 1-30 468 and 456, 256 of 1-40 880 and 1,084, 64 of 40-64 822 and 994;
-            // only 1,024 of 1-60 would gain, 4.39 and 3.62 ms)
-            sorted_rows = sorted_rows_enabled() && K == 64 && max_atoms <= ROW_LIST_MAX_KEYS && N < (1ll << 31) && E < (1ll << 31);
-            if (sorted_rows) {
+            // (sorted rows where neither pair grids nor larger crystals say otherwise; K = 0 keeps the row kernel with term lists: a
+            // 7-layer forward of 256 crystals of log-normal size up to 60 atoms took 569 us that way and 595 sorted)
+            bool one_basis = true;  // (the vectors' nodes are those of one basis)
+            for (int l = 1; l < num_layers; ++l) one_basis = one_basis && (K == 0 || scalars[6 * l + 5] == scalars[5]);
+            const bool gridded = grid_memory != nullptr && one_basis && sorted_rows_enabled() && num_layers <= PG_LAYERS &&
+                                 pair_grid_pays(N, B, E, max_atoms, K) &&
+                                 pair_grid_params(K, scalars[5], wscale, a_widest, weight_floor_log2(), by_grid.par);
+            sorted_rows = !gridded && sorted_rows_enabled() && K == 64 && max_atoms <= ROW_LIST_MAX_KEYS && N < (1ll << 31) && E < (1ll << 31);
+            if (gridded) {
+                by_grid.q = q; by_grid.k = k; by_grid.v = v; by_grid.a = a; by_grid.rvlen = cutoff_radius != 0.0 ? rvlen : nullptr;
+                by_grid.atom_start = grid_memory->atom_start; by_grid.edge_start = grid_memory->edge_start;
+                by_grid.N = N; by_grid.B = B; by_grid.E = E; by_grid.K = K; by_grid.max_atoms = (int)max_atoms; by_grid.rule = rule;
+                by_grid.dist_max = scalars[5]; by_grid.wscale = wscale; by_grid.call = 0;
+                by_grid.grid = pair_grid_carve(grid_memory->memory, N, B, E);
+                by_grid.leftover = by_grid.grid.leftover;
+                rc = launch_pair_grid_build(by_grid, pos_ij, tvecs, a_widest, weights + 3, 11, num_layers, forked ? side.stream : s);
+                by_grid.projected = K > 0;
+            } else if (sorted_rows) {
                 RowListBuild rb{};
                 rb.pos_ij = pos_ij; rb.tvecs = tvecs; rb.rvlen = cutoff_radius != 0.0 ? rvlen : nullptr;
                 rb.batch = batch; rb.edges = edges; rb.row_start = row_start; rb.row_order = row_order;
@@ -354,6 +372,11 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
     if (forked && cudaEventRecord(side_stream().join, side_stream().stream) != cudaSuccess) return launch_status("side stream join");
     // one attention call of layer l (dist_max, W of that layer)
     auto attention = [&](int l, double dist_max, const float *W, float *attn_out, float *lse_out) {
+        if (by_grid.call >= 0) {
+            PairAttn p = by_grid;
+            p.W = W; p.out = attn_out; p.call = l; p.lse = lse_out;
+            return grid_attn_impl(p, pos_ij, tvecs, batch, edges, row_start, cutoff_radius, lattice_range, minimum_range, s);
+        }
         if (sorted_rows)
             return sorted_attn_impl(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, N, E, max_atoms, dist_max, wscale,
                                     W, cutoff_radius, lattice_range, minimum_range, attn_out, lse_out, row_lists,

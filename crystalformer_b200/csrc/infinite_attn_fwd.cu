@@ -866,20 +866,20 @@ int launch_rows(const RowArgs &p, int64_t K, long long grid_rows, cudaStream_t s
     return launch_status("cf_infinite_attn_fwd");
 }
 
-// The rows that the sorted row kernel (infinite_attn_sorted.cu) left over: atoms rows[0 .. *count), processed by the
+// The rows that the sorted row kernel (infinite_attn_sorted.cu) or the kernel over pair grids (pair_attn.cu) left over: atoms rows[0 .. *count), processed by the
 // row kernel above without lists (phi and the candidates by enumeration).  `ticket` must be zero on entry.
 int launch_leftover_rows(const float *q, const float *k, const float *v, const float *a, const float *pos_ij,
                          const float *tvecs, const float *rvlen, const int64_t *batch, const int64_t *edges,
                          const int64_t *row_start, int64_t N, int64_t E, int64_t max_atoms, double dist_max,
                          double wscale, const float *W, double cutoff_radius, int lattice_range, int minimum_range,
-                         float *out, float *lse, const int *rows, const unsigned *count, unsigned *ticket, int64_t K,
-                         cudaStream_t s)
+                         float *out, float *logit, float *lse, float *psi_row, const int *rows, const unsigned *count,
+                         unsigned *ticket, int64_t K, cudaStream_t s)
 {
     RowArgs p{};
     p.q = q; p.k = k; p.v = v; p.a = a; p.pos_ij = pos_ij; p.tvecs = tvecs; p.rvlen = rvlen; p.W = W;
     p.batch = batch; p.edges = edges; p.row_start = row_start; p.row_order = rows; p.rows_on_device = count; p.E = E;
-    p.out = out; p.logit = nullptr; p.lse = lse; p.psi_row = nullptr; p.N = N; p.max_atoms = (int)max_atoms;
-    p.keep_logit = 0;
+    p.out = out; p.logit = logit; p.lse = lse; p.psi_row = psi_row; p.N = N; p.max_atoms = (int)max_atoms;
+    p.keep_logit = logit != nullptr;  // (inference: neither logits nor psi_row)
     p.phi_in_row = 1;  // no list: every edge's phi is enumerated inside the row kernel
     p.ticket = ticket;
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};

@@ -528,8 +528,8 @@ int launch_leftover_rows(const float *q, const float *k, const float *v, const f
                          const float *tvecs, const float *rvlen, const int64_t *batch, const int64_t *edges,
                          const int64_t *row_start, int64_t N, int64_t E, int64_t max_atoms, double dist_max,
                          double wscale, const float *W, double cutoff_radius, int lattice_range, int minimum_range,
-                         float *out, float *lse, const int *rows, const unsigned *count, unsigned *ticket, int64_t K,
-                         cudaStream_t s);
+                         float *out, float *logit, float *lse, float *psi_row, const int *rows, const unsigned *count,
+                         unsigned *ticket, int64_t K, cudaStream_t s);
 
 // One attention call over a batch's row lists: the sorted row kernel, then the enumerating row kernel for whatever it
 // left over (normally nothing: that launch then finds a zero count and returns).  sched_slot: which of the
@@ -553,7 +553,7 @@ int sorted_attn_impl(const float *q, const float *k, const float *v, const float
     int rc = launch_sorted_rows(l, s);
     if (rc != CF_OK) return rc;
     return launch_leftover_rows(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, N, E, max_atoms, dist_max, wscale,
-                                W, cutoff_radius, lattice_range, minimum_range, out, lse, view.leftover, sched + 1, sched + 2, K, s);
+                                W, cutoff_radius, lattice_range, minimum_range, out, nullptr, lse, nullptr, view.leftover, sched + 1, sched + 2, K, s);
 }
 }  // namespace cf
 

@@ -10,6 +10,7 @@
 #include "blas_dyn.cuh"
 #include "common.cuh"
 #include "dense_block.cuh"
+#include "pair_grid.cuh"
 #include "peer_gather.cuh"
 #include "segment_mean.cuh"
 
@@ -24,7 +25,8 @@ int encoder_forward_impl(void *cublas_handle, int num_layers, const float *const
                          const int64_t *edges, const int64_t *row_start, int64_t N, int64_t B, int64_t E,
                          int64_t max_atoms, int64_t K, int64_t ff_dim, double wscale, double cutoff_radius,
                          int lattice_range, int minimum_range, float *workspace, const int32_t *row_order,
-                         void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun);
+                         void *const *attn_events, void *stream, const EmbedStage *embed, bool early_prep, const HeadStage *begun,
+                         const GridMemory *grid_memory);
 cudaStream_t early_prep_stream(void *inputs_ready, void *slot_free);
 namespace {
 
@@ -81,6 +83,7 @@ struct Scratch {
     int64_t *atom_start, *edge_start, *batch, *row_start, *edges;
     float *pos_ij, *rvlen, *x, *encoder;
     int32_t *row_order;
+    char *grid;  // pair grids (null: more pairs than they are kept for)
     size_t bytes;
 };
 
@@ -98,6 +101,8 @@ Scratch carve(void *workspace, int64_t N, int64_t B, int64_t E, int64_t ff_dim)
     s.row_order = c.take<int32_t>(N);
     s.x = c.take<float>(N * MODEL_DIM);
     s.encoder = c.take<float>((size_t)cf_encoder_workspace_floats(N, E, ff_dim));
+    const size_t grid = pair_grid_bytes(N, B, E, N > 0 ? E / N : 0);  // (the largest crystal has at least E / N atoms)
+    s.grid = grid > 0 ? c.take<char>(grid) : nullptr;
     s.bytes = c.used;
     return s;
 }
@@ -177,10 +182,11 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
         if (st != CUBLAS_STATUS_SUCCESS) return fail(CF_ERR_CUDA, "cf_model_forward: cuBLAS SGEMM failed with status %d", (int)st);
     }
     const EmbedStage embed{features, species, (int)feature_dim, reinterpret_cast<const float4 *>(W_embed_packed)};
+    const GridMemory grid{w.grid, w.atom_start, w.edge_start};
     rc = encoder_forward_impl(cublas_handle, num_layers, weights, scalars, w.x, w.pos_ij, trans,
                               cutoff_radius != 0.0 ? w.rvlen : nullptr, w.batch, w.edges, w.row_start, N, B, E, max_atoms, K,
                               ff_dim, wscale, cutoff_radius, lattice_range, minimum_range, w.encoder, order, attn_events,
-                              stream, embed_fused ? &embed : nullptr, early, begun);
+                              stream, embed_fused ? &embed : nullptr, early, begun, w.grid != nullptr ? &grid : nullptr);
     if (rc != CF_OK) return rc;
     const bool chained = num_layers > 0 && N > 0;  // behind the encoder's last dense block
     if (gather != nullptr)

@@ -1,0 +1,132 @@
+// Pair grids: the lattice sums of a batch as short vectors, one per pair of atoms, made once per batch for all layers.
+//
+// Every sum over the images of a pair (i, j) that an attention layer needs is of the form sum_n f(d_n) with f smooth on the
+// scale of the radial basis: exp(a d^2) for the weights, exp(a d^2) g_k(d) for the basis sums, exp(a d^2) c(d) and
+// exp(a d^2) d^2 in the backward.  The distances d_n belong to the geometry, f to the layer.  With nodes d_m of spacing h and
+// interpolation weights L_q(y) that reproduce such functions from the POINTS nearest nodes,
+//     sum_n f(d_n) = sum_m rho_m f(d_m),     rho_m = sum_n L_{m - floor(d_n / h)}(y_n)
+// so the images enter once, in rho, and a layer evaluates its functions at the nodes only: two small matrix products per row
+// instead of a sweep of its terms (3 to 1,000 images per pair).  rho_ij = rho_ji, so pairs i <= j are kept.
+//
+// Nodes: h is a third of the radial basis' standard deviation, twelve points.  The weights are the best ones for functions of
+// a Gaussian spectrum of that width (simple kriging with its autocorrelation, conditional on y; polynomials of degree nine in
+// y fit them to 1e-10).  For rows of random cells of 3-9 A the basis sums come out within 2.6e-8 (2-norm, arithmetic in 64
+// bits) and the weights within 9e-9, a fraction of what float32 sums lose; ten points would give 1.8e-7, a spacing of
+// 1 / 2.5 with fourteen points 5e-8, 1 / 4 with ten 9e-9 at a third more memory.  Without a basis the widths themselves set
+// the scale: h = 0.1 of the widest standard deviation that the model can produce.
+//
+// Boxes: the cut-off rule gives every (atom, head) its own box of images, between the box of an infinitely narrow Gaussian and
+// that of the widest.  A crystal has one set of vectors per box in that range (its variants: one for four cells of five, two
+// for most others), and a head uses its own.
+//
+// A vector is stored as half-precision pairs (value, remainder), scaled by RHO_SCALE: per 16 nodes 32 bytes of values and 32
+// of remainders, which is what the matrix instructions' operands are loaded from.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+
+namespace cf {
+
+constexpr int PG_POINTS = 12, PG_BELOW = 5;  // nodes floor(x) - 5 ... floor(x) + 6; node m sits at (m - 5) h
+constexpr int PG_TILE = 16;                  // nodes per tile
+constexpr int PG_TILES_BASIS = 11, PG_TILES_PLAIN = 5;
+constexpr float PG_RHO_SCALE = 32.0f;
+constexpr int PG_MAX_VARIANTS = 32;
+constexpr int PG_UNIT = 8;                   // pairs of a unit of the build
+constexpr int PG_ROWS = 8;                   // rows of a crystal that a block of the attention kernels takes
+constexpr int PG_ALL_BOXES = 1 << 24;         // in PairGrid::info: the variants are all the boxes up to the widest Gaussian's
+constexpr int PG_MAX_ATOMS = 64;             // (tables of eight rows in shared memory, two blocks per SM)
+constexpr int PG_LAYERS = 32;                // calls per batch that find zeroed counters
+constexpr size_t PG_MAX_BYTES = 24ull << 30;
+
+__host__ __device__ inline int pg_tiles(long long K) { return K > 0 ? PG_TILES_BASIS : PG_TILES_PLAIN; }
+__host__ __device__ inline int pg_slot_bytes(long long K) { return 64 * pg_tiles(K); }
+
+// Fragments of the matrix g_k(d_m) of the basis at the nodes, in halves (value, remainder) scaled by PG_BASIS_SCALE: per (node
+// tile, bin tile) 32 lanes x (4 + 4) words; first with bins as rows, then with nodes as rows.
+constexpr float PG_BASIS_SCALE = 16384.0f;
+constexpr int PG_FRAGS = PG_TILES_BASIS * 4;
+constexpr size_t PG_BASIS_WORDS = (size_t)PG_FRAGS * 32 * 8;
+
+struct PairGrid {
+    unsigned char *slots;        // vectors: pair (i <= j) of crystal c at (edge_start[c] + atom_start[c]) / 2 + its index
+    int4 *info;                  // per crystal: smallest box (packed), variants per axis (packed), first extra slot, atoms
+    int *unit_start;             // (B + 1): build units (PG_UNIT pairs of one variant) before a crystal
+    int4 *tiles;                 // row tiles of the attention kernels: { crystal, first row, atoms (negative: no vectors), first
+                                 // atom }, { first vector, first extra vector, smallest box, variants per axis }
+    unsigned *counters;          // { tiles, -, -, - }, then per call { rows left over, ticket of their launch, -, - }
+    int *leftover;               // rows left over by a call
+    uint4 *basis;                // fragments, bins as rows
+    uint4 *basis_nodes;          // fragments, nodes as rows
+    uint4 *projected;            // W_h g(d_m) of every call: per (call, head, node tile) a fragment, channels as rows
+    float *projected_scale;      // (call, head): what the products with them are divided by
+    long long slot_count;
+};
+// Memory of a batch's grids and the offsets that only the model's entry points have.
+struct GridMemory {
+    void *memory;
+    const int64_t *atom_start, *edge_start;
+};
+struct PairGridParams {
+    int tiles;                   // node tiles of a vector
+    float inv_h2, inv_h2_low;    // 1 / h^2 in two floats
+    float gauss;                 // exp(a d_m^2) = 2^(a gauss (m - 5)^2)
+    float a_widest;              // no layer has a wider Gaussian
+    float a_least;               // rows with a narrower Gaussian (a below) are left over
+    float floor_log2;
+};
+
+// Bytes for a batch, and whether a batch can go this way at all.
+size_t pair_grid_bytes(long long N, long long B, long long E, long long max_atoms_or_0);
+PairGrid pair_grid_carve(void *memory, long long N, long long B, long long E);
+bool pair_grid_params(long long K, double dist_max, double wscale, float a_widest, float floor_log2, PairGridParams &out);
+inline bool pair_grid_fits(long long N, long long B, long long E, long long max_atoms)
+{
+    return N > 0 && max_atoms <= PG_MAX_ATOMS && N < (1ll << 28) && pair_grid_bytes(N, B, E, max_atoms) > 0;
+}
+// Whether an inference batch gains by them.  The plan, the vectors and a block's fixed work (a row's Gaussians at the nodes, whatever
+// its keys) want
+// - enough pairs: forwards of 1, 4, 16, 64, 128 crystals of up to 30 atoms 196, 208, 220, 236, 291 us against 214, 208, 228, 266,
+//   367 by row lists, 1, 16, 64 of up to 60 atoms 217, 250, 292 against 191, 293, 475; without a basis (seven layers, term
+//   lists) 255, 270, 293, 307, 361 against 250, 257, 278, 337, 417;
+// - enough keys per row: 256, 1,024 crystals of up to 8 atoms 254, 443 against 254, 372, 483 and 596 of up to 12 377, 388 against
+//   349, 357, 118 and 436 of up to 18 234, 399 against 270, 397.
+// With several forwards in flight it is not latency that counts, and they pay later: sixteen batches of 64, 128, 256 crystals of up
+// to 24 atoms 2,389, 2,605, 3,461 us against 1,978, 2,497, 3,905, of up to 40 2,603, 3,282, 5,885 against 3,589, 5,689, 10,453, 16
+// of up to 60 2,193 against 2,723; without a basis 64, 128, 256 of up to 24 2,584, 2,941, 3,587 against 2,067, 2,882, 4,448.  The
+// line is drawn there for all, so that a batch has the same bits however it is issued.
+inline bool pair_grid_pays(long long N, long long B, long long E, long long max_atoms, long long K)
+{
+    if (!pair_grid_fits(N, B, E, max_atoms) || E < 11 * N) return false;
+    return E >= 30000 || (K > 0 && E >= 18000 && E >= 24 * N);
+}
+
+// One attention call over a batch's grids, and its backward.
+struct PairAttn {
+    const float *q, *k, *v, *a, *rvlen, *W;
+    const int64_t *atom_start, *edge_start;
+    long long N, B, E, K;
+    int max_atoms;
+    BoxRule rule;
+    double dist_max, wscale;
+    PairGridParams par;
+    PairGrid grid;
+    int call;
+    float *out, *lse, *psi_row, *logit;  // psi_row, logit: or null
+    unsigned char *left;         // per row: 1 if it was left over (or null)
+    bool projected;              // the build had this call's W: no psi_row
+    int *leftover;               // the rows, and their number in counters[4 (call + 1)]
+    // backward
+    const float *gout;
+    float *gq, *gk, *gv, *ga, *glogit, *prob;
+};
+// The plan and the vectors (geometry, rule, sizes and parameters of `p`; a_widest: the widest Gaussian of any layer), and either the
+// basis at the nodes (W null: for calls with psi_row) or the calls' projections at the nodes (W of call c at W[c * W_stride]).
+int launch_pair_grid_build(const PairAttn &p, const float *pos_ij, const float *tvecs, float a_widest, const float *const *W, int W_stride,
+                           int calls, cudaStream_t s);
+// The attention, and the rows that it leaves over by enumeration (their logits too, where p.logit is given).
+int grid_attn_impl(const PairAttn &p, const float *pos_ij, const float *tvecs, const int64_t *batch, const int64_t *edges,
+                   const int64_t *row_start, double cutoff_radius, int lattice_range, int minimum_range, cudaStream_t s);
+
+}  // namespace cf

@@ -62,7 +62,7 @@ def set_chained_launches(enabled: bool) -> None:
 
 
 def set_row_stats(words: Optional[torch.Tensor]) -> None:
-    """Work counters of the sorted row kernel (cf_set_row_stats): a zeroed CUDA int64 tensor of four words, or None to
+    """Work counters of the sorted row kernel and of the attention over pair grids (cf_set_row_stats): a zeroed CUDA int64 tensor of four words, or None to
     switch the counting off.  The tensor must stay alive while set."""
     _lib.load().cf_set_row_stats(_ptr(words))
 
@@ -301,6 +301,49 @@ def infinite_attn_fwd_sorted(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row
                   c_double(cutoff_radius or 0.0), c_int(lattice_range), c_int(minimum_range), _ptr(out), _ptr(lse),
                   _ptr(row_lists), _stream(dev))
     return out, lse
+
+
+def pair_grid_build(pos_ij, tvecs, rvlen, atom_start, edge_start, num_atoms, max_atoms, K, dist_max, wscale, cutoff_radius,
+                    lattice_range, minimum_range, a_widest):
+    """Pair grids of a batch (see cf_pair_grid_build): (workspace tensor, atom_start, edge_start, a_widest), to be handed to
+    ``infinite_attn_fwd_grid`` for every layer of the batch."""
+    dev = pos_ij.device
+    pos_ij, tvecs, rvlen = (_want(t, torch.float32, n, dev) for t, n in ((pos_ij, "pos_ij"), (tvecs, "tvecs"), (rvlen, "rvlen")))
+    atom_start, edge_start = _want(atom_start, torch.int64, "atom_start", dev), _want(edge_start, torch.int64, "edge_start", dev)
+    N, B, E = num_atoms, tvecs.shape[0], pos_ij.shape[0]
+    work = torch.empty(int(_lib.load().cf_pair_grid_bytes(N, B, E)), dtype=torch.uint8, device=dev)
+    with torch.cuda.device(dev):
+        _lib.call("cf_pair_grid_build", _ptr(pos_ij), _ptr(tvecs), _ptr(rvlen), _ptr(atom_start), _ptr(edge_start), c_int64(N),
+                  c_int64(B), c_int64(E), c_int64(max_atoms), c_int64(K), c_double(dist_max), c_double(wscale),
+                  c_double(cutoff_radius or 0.0), c_int(lattice_range), c_int(minimum_range), c_double(a_widest), _ptr(work),
+                  _stream(dev))
+    return work, atom_start, edge_start, a_widest
+
+
+def infinite_attn_fwd_grid(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, max_atoms, K, dist_max, wscale, W,
+                           cutoff_radius, lattice_range, minimum_range, grids, want_psi_row=False):
+    """Fused attention forward over a batch's pair grids.  Returns (out (N,H,D), logit (E,H), of the rows left over only, lse (N,H),
+    psi_row (N,H,K) or None, left (N) uint8: 1 where a row was left over)."""
+    dev = q.device
+    q, k, v, a, tvecs = (_want(t, torch.float32, n, dev) for t, n in
+                         ((q, "q"), (k, "k"), (v, "v"), (a, "a"), (tvecs, "tvecs")))
+    pos_ij, rvlen, W = (_want(t, torch.float32, n, dev) for t, n in ((pos_ij, "pos_ij"), (rvlen, "rvlen"), (W, "W")))
+    batch, edges, row_start = (_want(t, torch.int64, n, dev) for t, n in
+                               ((batch, "batch"), (edges, "edges"), (row_start, "row_start")))
+    N, H, D = q.shape
+    _check_projection(W, H, K, "infinite_attn_fwd_grid")
+    E, B = edges.shape[1], tvecs.shape[0]
+    work, atom_start, edge_start, a_widest = grids
+    out, logit = torch.empty((N, H, D), dtype=torch.float32, device=dev), torch.empty((E, H), dtype=torch.float32, device=dev)
+    lse, left = torch.empty((N, H), dtype=torch.float32, device=dev), torch.empty(N, dtype=torch.uint8, device=dev)
+    psi_row = torch.empty((N, H, K), dtype=torch.float32, device=dev) if (want_psi_row and K > 0) else None
+    with torch.cuda.device(dev):
+        _lib.call("cf_infinite_attn_fwd_grid", _ptr(q), _ptr(k), _ptr(v), _ptr(a), _ptr(pos_ij), _ptr(tvecs), _ptr(rvlen),
+                  _ptr(batch), _ptr(edges), _ptr(row_start), _ptr(atom_start), _ptr(edge_start), c_int64(N), c_int64(B), c_int64(H),
+                  c_int64(D), c_int64(E), c_int64(K), c_int64(max_atoms), c_double(dist_max), c_double(wscale), _ptr(W),
+                  c_double(cutoff_radius or 0.0), c_int(lattice_range), c_int(minimum_range), c_double(a_widest), _ptr(out),
+                  _ptr(logit), _ptr(lse), _ptr(psi_row), _ptr(left), _ptr(work), _stream(dev))
+    return out, logit, lse, psi_row, left
 
 
 def infinite_attn_fwd(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, max_atoms, K, dist_max, wscale, W,

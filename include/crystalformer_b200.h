@@ -71,8 +71,9 @@ void cf_set_weight_floor_log2(double log2_floor);
 double cf_get_weight_floor_log2(void);
 
 /* Whether cf_encoder_forward / cf_model_forward may take the row-list path (cf_row_list_build +
- * cf_infinite_attn_fwd_sorted, below) for batches whose crystals have at most 64 atoms; 1 by default, 0 keeps the
- * term-list kernels for every batch.  Process-wide, read at launch time. */
+ * cf_infinite_attn_fwd_sorted, below) and, from some thousand pairs on, cf_model_forward and cf_model_finish the pair grids
+ * (cf_pair_grid_build + cf_infinite_attn_fwd_grid) for batches whose crystals have at most 64 atoms; 1 by default, 0 keeps
+ * the term-list kernels for every batch.  Process-wide, read at launch time. */
 void cf_set_sorted_rows(int enabled);
 int cf_get_sorted_rows(void);
 
@@ -81,10 +82,11 @@ int cf_get_sorted_rows(void);
  * drains, then wait for it to complete); 1 by default, 0 launches them the ordinary way.  Results are identical. */
 void cf_set_chained_launches(int enabled);
 
-/* Work counters of the sorted row kernel (diagnostic, for roofline accounting): while `device_words` (DEVICE memory,
- * four uint64, zeroed by the caller) is set, every cf_infinite_attn_fwd_sorted launch - also inside the one-call
- * forwards - adds { chunks of eight entries swept, (chunk, 16-bin tile) pairs whose basis values were evaluated,
- * rows processed, 0 }.  NULL (the default) switches the counting off.  Process-wide; the memory must stay valid
+/* Work counters of the sorted row kernel and of the attention over pair grids (diagnostic, for roofline accounting): while
+ * `device_words` (DEVICE memory, four uint64, zeroed by the caller) is set, every cf_infinite_attn_fwd_sorted and
+ * cf_infinite_attn_fwd_grid launch - also inside the one-call forwards - adds { chunks of eight entries swept, (chunk, 16-bin
+ * tile) pairs whose basis values were evaluated, rows processed, products of 16 keys and 16 nodes }, the first two from the
+ * former, the last from the latter.  NULL (the default) switches the counting off.  Process-wide; the memory must stay valid
  * while set. */
 void cf_set_row_stats(void *device_words);
 
@@ -285,6 +287,35 @@ int cf_infinite_attn_bwd_listed(const float *q, const float *k, const float *v, 
                                 const float *lse, const float *out, const float *gout, float *gq, float *gk, float *gv,
                                 float *ga, float *glogit, const int32_t *row_order, void *term_lists, double a_widest,
                                 void *stream);
+
+/* ------------------------------------------------------------------------------------------------------------
+ * Pair grids: the lattice sums of a batch reduced to one vector per pair of atoms (and box of the cut-off rule), made once
+ * per batch, and the fused attention over them.  Same function as cf_infinite_attn_fwd (real_enc_proj_fwd +
+ * fused_dpa_fwd of the reference, models/kernels/real_enc_proj_fwd.cu:63-169, models/kernels/fused_dpa_fwd_v3.cu); the cost of a
+ * row depends on its keys, no longer on the images in reach.  The functions of the distance that a layer sums over the images
+ * (Gaussians, times the radial basis) are interpolated between nodes a third of the basis' standard deviation apart (twelve
+ * points, 3e-8 of a row's sums); K = 0: 0.1 of the widest Gaussian's.  Rows that this does not serve - a Gaussian
+ * narrower than 3 standard deviations of the basis (K = 0: 0.5 of the widest), reach beyond the nodes, a box that is not among
+ * the crystal's variants, logits more than 16 bits above the atom's own, an infinity or a NaN - are processed by the enumerating
+ * kernel of cf_infinite_attn_fwd inside the same call, and marked in `left`.
+ *   a_widest: the a (< 0) closest to zero that any layer can produce, as for cf_term_list_build.
+ *   grids: cf_pair_grid_bytes(N, B, E) bytes (0: more pairs than grids are kept for), 256-byte aligned; it also holds the
+ *   counters of the calls that use it, so calls sharing it must be ordered (one stream).
+ *   logit (E,H): or NULL; written for the rows left over only.  psi_row (N,H,K): or NULL.  left (N): or NULL.
+ *   max_atoms <= 64.  CF_ERR_UNSUPPORTED where the nodes of (dist_max, wscale) do not cover ordinary Gaussians.
+ * ---------------------------------------------------------------------------------------------------------- */
+int64_t cf_pair_grid_bytes(int64_t N, int64_t B, int64_t E);
+int cf_pair_grid_build(const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *atom_start,
+                       const int64_t *edge_start, int64_t N, int64_t B, int64_t E, int64_t max_atoms, int64_t K,
+                       double dist_max, double wscale, double cutoff_radius, int lattice_range, int minimum_range,
+                       double a_widest, void *grids, void *stream);
+int cf_infinite_attn_fwd_grid(const float *q, const float *k, const float *v, const float *a, const float *pos_ij,
+                              const float *tvecs, const float *rvlen, const int64_t *batch, const int64_t *edges,
+                              const int64_t *row_start, const int64_t *atom_start, const int64_t *edge_start, int64_t N,
+                              int64_t B, int64_t H, int64_t D, int64_t E, int64_t K, int64_t max_atoms, double dist_max,
+                              double wscale, const float *W, double cutoff_radius, int lattice_range, int minimum_range,
+                              double a_widest, float *out, float *logit, float *lse, float *psi_row, uint8_t *left,
+                              void *grids, void *stream);
 
 /* ------------------------------------------------------------------------------------------------------------
  * Row lists and the tensor-core row kernel for batches of small crystals (max_atoms <= 64; K = 64, or K = 0: no

@@ -1,0 +1,141 @@
+"""Fused attention over pair grids (csrc/pair_grid.cu, pair_attn.cu) against the float64 oracle chain and the enumerating kernel.
+
+Tolerance: the 2-norm error against 64 bits may be 1.25 times the enumerating kernel's on the same rows plus 3e-8, what the
+interpolation between the nodes leaves of a row's sums (the weights reproduce the basis functions within 2.6e-8)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from crystalformer_b200.synthetic import make_crystals, uniform_atoms
+
+pytestmark = pytest.mark.gpu
+H, D, DIST_MAX, WSCALE, A_WIDEST = 8, 16, 14.0, 1.0, -0.5 * 0.5 / 1.4 ** 2
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from crystalformer_b200 import ops as o
+    return o
+
+
+def dev(x):
+    return torch.as_tensor(np.ascontiguousarray(x)).cuda()
+
+
+def inputs(cb, sigma, scale=0.3, seed=3):
+    rng = np.random.default_rng(seed)
+    N = cb.num_atoms
+    a = (-0.5 / (sigma[0] + (sigma[1] - sigma[0]) * rng.random((N, H))) ** 2).astype(np.float32)
+    W = (rng.standard_normal((H, D, 64)) * 0.1).astype(np.float32)
+    q = (rng.standard_normal((N, H, D)) * scale).astype(np.float32)
+    k, v = (rng.standard_normal((N, H, D)).astype(np.float32) for _ in range(2))
+    return q, k, v, a, W
+
+
+def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE):
+    """(grid results, enumerating kernel's results)"""
+    q, k, v, a, W = x
+    sizes = dev(cb.sizes)
+    atom_start, edge_start = ops.crystal_offsets(sizes)
+    g = ops.batch_prepare(dev(cb.pos if pos is None else pos), dev(cb.trans_vec), sizes, atom_start, edge_start, cb.num_atoms, cb.num_edges)
+    nmax = int(cb.sizes.max())
+    W = dev(W) if K else None
+    args = (dev(q), dev(k), dev(v), dev(a), g["pos_ij"], dev(cb.trans_vec), g["rvlen"], g["batch"], g["edges"], g["row_start"],
+            nmax, K, DIST_MAX, wscale, W, cutoff, 2, minimum)
+    grids = ops.pair_grid_build(g["pos_ij"], dev(cb.trans_vec), g["rvlen"], atom_start, edge_start, cb.num_atoms, nmax, K, DIST_MAX,
+                                wscale, cutoff, 2, minimum, A_WIDEST)
+    return (ops.infinite_attn_fwd_grid(*args, grids, want_psi_row=K > 0), ops.infinite_attn_fwd(*args, want_psi_row=K > 0),
+            lambda: ops.infinite_attn_fwd_grid(*args, grids, want_psi_row=K > 0))
+
+
+def reference(cb, x, K, cutoff, minimum, wscale=WSCALE):
+    q, k, v, a, W = x
+    edges = oracle.edge_index(cb.sizes)
+    pos_ij, _, _, rvlen = oracle.geometry(cb.pos, cb.trans_vec, edges)
+    z, psiW = oracle.lattice_sum_fwd(a, pos_ij, cb.trans_vec, cb.batch, edges, K, DIST_MAX, wscale, W=W[None] if K else None, rvlen=rvlen,
+                                     cutoff_radius=cutoff, lattice_range=2, minimum_range=minimum, precision="f64")
+    _, out = oracle.fused_attn_fwd(q, k, v, z, psiW, edges, precision="f64")
+    logit = np.einsum("ehd,ehd->eh", q[edges[0]].astype(np.float64), k[edges[1]].astype(np.float64)) + z
+    lse = np.full((cb.num_atoms, H), -np.inf)
+    np.logaddexp.at(lse, edges[0], logit)
+    return np.asarray(out).reshape(cb.num_atoms, H, D), lse
+
+
+def close(x, ref, plain, rows, what):
+    err, err0 = (np.linalg.norm(t.cpu().numpy().astype(np.float64)[rows] - ref[rows]) / np.linalg.norm(ref[rows]) for t in (x, plain))
+    assert err <= 1.25 * err0 + 3e-8, (what, err, err0)
+
+
+# sizes about the tiles of 16 keys and 8 rows; one, two and four key tiles; cells with one box per width and with several; the three
+# cut-off rules; another width of the basis
+@pytest.mark.parametrize("lo,hi,K,cutoff,minimum,lengths,sigma,wscale", [
+    (1, 9, 64, -3.5, 2, (3.0, 9.0), (1.18, 1.6), 1.0), (15, 17, 64, -3.5, 2, (4.0, 12.0), (1.18, 1.6), 1.0),
+    (31, 33, 64, -3.5, 2, (4.0, 12.0), (1.0, 1.6), 1.0), (63, 64, 64, -3.5, 2, (6.0, 12.0), (1.18, 1.6), 1.0),
+    (8, 24, 64, -3.5, 0, (3.0, 9.0), (1.18, 1.6), 1.0), (4, 12, 64, 0.0, 2, (3.0, 9.0), (1.18, 1.6), 1.0),
+    (4, 12, 64, 6.5, 2, (3.0, 9.0), (1.18, 1.6), 1.0), (4, 20, 64, -3.5, 2, (3.0, 4.5), (1.2, 1.7), 1.0),
+    (4, 20, 64, -3.5, 2, (4.0, 9.0), (1.18, 1.6), 1.1), (1, 1, 64, -3.5, 2, (5.0, 9.0), (1.18, 1.6), 1.0),
+    (1, 17, 0, -3.5, 2, (3.0, 9.0), (1.18, 1.6), 1.0), (33, 64, 0, -3.5, 2, (4.0, 12.0), (1.18, 1.9), 1.0),
+    (4, 20, 0, 0.0, 2, (3.0, 9.0), (1.18, 1.6), 1.0), (4, 20, 0, -3.5, 2, (3.0, 4.5), (1.2, 1.7), 1.0)])
+def test_grid_forward_against_oracle_chain(ops, lo, hi, K, cutoff, minimum, lengths, sigma, wscale):
+    cb = make_crystals(41, 9, uniform_atoms(lo, hi), length_range=lengths)
+    x = inputs(cb, sigma)
+    (out, _, lse, psi, left), (out0, _, lse0, psi0), again = run(ops, cb, x, K, cutoff, minimum, wscale=wscale)
+    ref, ref_lse = reference(cb, x, K, cutoff, minimum, wscale)
+    rows = left.cpu().numpy() == 0
+    assert rows.mean() > 0.9
+    close(out, ref, out0, rows, "rows by nodes")
+    close(out, ref, out0, slice(None), "all rows")
+    # float32 logarithms of sums: a few units in the last place of either, and of the largest logit
+    assert np.abs(lse.cpu().numpy() - ref_lse).max() < 1e-6 * max(1.0, np.abs(ref_lse).max()) + 1.5e-6
+    if K:  # 64 sums per (row, head), each within a few units of the row's largest
+        assert float((psi - psi0).abs().max() / psi0.abs().max()) < 2e-6
+    repeat = again()
+    assert torch.equal(out, repeat[0]) and torch.equal(lse, repeat[2])
+
+
+@pytest.mark.parametrize("K", [64, 0])
+def test_rows_that_nodes_do_not_serve_are_left_over(ops, K):
+    """Gaussians too narrow and too wide for the nodes, logits far above the atom's own: marked, and as good as the others."""
+    cb = make_crystals(43, 8, uniform_atoms(3, 20), length_range=(4.0, 9.0))
+    x = inputs(cb, (1.2, 1.5))
+    rng = np.random.default_rng(1)
+    kind = rng.integers(0, 4, cb.num_atoms)
+    x[3][kind == 1, 5] = -0.5 / 0.3 ** 2
+    x[0][kind == 2] *= 40.0
+    x[3][kind == 3, 2] = -0.5 / 2.6 ** 2  # (wider than a_widest: a box beyond the crystal's, or reach beyond the nodes)
+    (out, _, lse, _, left), (out0, _, lse0, _), _ = run(ops, cb, x, K)
+    left = left.cpu().numpy()
+    assert left[kind == 1].all() and left[kind == 3].all() and left[kind == 2].any() and not left[kind == 0].any()
+    ref, _ = reference(cb, x, K, -3.5, 2)
+    close(out, ref, out0, slice(None), "all rows")
+
+
+@pytest.mark.parametrize("K", [64, 0])
+def test_numbers_that_are_not_finite_stay_visible(ops, K):
+    """A NaN or an infinity in an input shows in the rows that the enumerating kernel shows it in."""
+    cb = make_crystals(44, 6, uniform_atoms(4, 18), length_range=(4.0, 9.0))
+    starts = np.concatenate([[0], np.cumsum(cb.sizes)])
+    x = inputs(cb, (1.2, 1.5))
+    x[0][starts[0] + 1, 2, 3] = np.nan
+    x[1][starts[1] + 1, 1, 0] = np.nan
+    x[2][starts[2] + 2, 4, 5] = np.nan
+    x[1][starts[3] + 1, 3, 3] = np.inf
+    x[3][starts[4] + 1, 6] = np.nan
+    pos = cb.pos.copy()
+    pos[starts[5] + 2] = np.nan
+    (out, *_), (out0, *_), _ = run(ops, cb, x, K, pos=pos)
+    bad, bad0 = (~torch.isfinite(t).flatten(1).all(dim=1) for t in (out, out0))
+    assert torch.equal(bad, bad0)
+
+
+def test_crystals_beyond_the_extra_vectors(ops):
+    """Cells so flat that a head's box varies by dozens: only the smallest box has vectors, all other rows are left over."""
+    cb = make_crystals(45, 3, uniform_atoms(3, 6), length_range=(3.0, 6.0))
+    cb.trans_vec[0] *= np.float32(0.2)
+    cb.pos[:cb.sizes[0]] *= np.float32(0.2)
+    x = inputs(cb, (1.2, 1.6), scale=0.1)
+    (out, _, _, _, left), (out0, *_), _ = run(ops, cb, x, 64)
+    assert left[:int(cb.sizes[0])].all()
+    ref, _ = reference(cb, x, 64, -3.5, 2)
+    close(out, ref, out0, slice(None), "all rows")
