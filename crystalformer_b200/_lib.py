@@ -53,6 +53,8 @@ SIGNATURES = {
     "cf_pair_grid_build": [P, P, P, P, P, I64, I64, I64, I64, I64, F64, F64, F64, I32, I32, F64, P, P],
     "cf_infinite_attn_fwd_grid": [P, P, P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, F64, F64, P, F64, I32, I32, F64,
                                   P, P, P, P, P, P, P],
+    "cf_infinite_attn_bwd_grid": [P, P, P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, F64, F64, P, F64, I32, I32, F64,
+                                  P, P, P, P, P, P, P, P, P, P, P, P, P],
     "cf_infinite_attn_fwd_sorted": [P, P, P, P, P, P, P, P, P, P, I64, I64, I64, I64, I64, I64, I64, F64, F64, P, F64, I32,
                                     I32, P, P, P, P],
     "cf_serve_submit": [P, P, P, P, P, P, I64, I64, I64, I64, I32, P, P],

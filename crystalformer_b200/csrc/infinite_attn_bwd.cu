@@ -15,6 +15,7 @@
 //                                  per key).  Writes glogit (E,H), ga (N,H), gq (N,H,D).
 //   infinite_attn_bwd_cols_kernel  gk_j, gv_j from glogit and p_ij = exp(logit - lse_i), eight keys per block.
 #include "lattice_bwd_core.cuh"
+#include "pair_grid.cuh"
 #include "term_list.cuh"
 
 namespace cf {
@@ -35,6 +36,8 @@ struct BwdRowArgs {
     BoxRule rule;
     BasisParams basis;
     TermList list;  // optional (pool == NULL: none): the rows' terms, found once per batch (term_list.cuh)
+    const unsigned *rows_on_device;  // optional: the number of rows to process (entries of row_order), read on the device
+    float *prob;    // optional (E,H): p_ij, written by the rows and read by the columns instead of exp(logit - lse)
 };
 
 __host__ __device__ inline size_t bwd_row_smem_floats(int max_atoms, bool with_basis)
@@ -43,7 +46,7 @@ __host__ __device__ inline size_t bwd_row_smem_floats(int max_atoms, bool with_b
     return (size_t)max_atoms * 36 + (with_basis ? HEADS * U_STRIDE : 0) + WARPS * 2 * BWD_RING + WARPS * 8;
 }
 
-template <int K>
+template <int K, bool LEFT>
 __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(const BwdRowArgs p)
 {
     extern __shared__ __align__(16) float smem[];
@@ -59,6 +62,7 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
     CandidateRingOf<BWD_RING> ring;
     ring.init(rings + warp * 2 * BWD_RING, lane);
 
+    const long long rows = LEFT ? (long long)*p.rows_on_device : p.N;
     // what a row starts from: atom, edges, keys, first key; fetched a row ahead (dependent reads)
     struct Row {
         long long i, e0, a0;
@@ -66,7 +70,7 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
     };
     auto row_of = [&](long long slot) {
         Row r{0, 0, 0, 0};
-        if (slot < p.N) {
+        if (slot < rows) {
             r.i = p.row_order ? p.row_order[slot] : slot;
             r.e0 = p.row_start[r.i];
             r.n = (int)(p.row_start[r.i + 1] - r.e0);
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
         return r;
     };
     Row next = row_of(blockIdx.x);
-    for (long long slot = blockIdx.x; slot < p.N; slot += gridDim.x) {
+    for (long long slot = blockIdx.x; slot < rows; slot += gridDim.x) {
         const long long i = next.i, e0 = next.e0, a0 = next.a0;
         const int n = next.n;
         const long long c = p.batch[i];
@@ -307,6 +311,7 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
             const float g = fmaf(pj[idx], gov[idx], s0[idx]);
             s0[idx] = g;
             p.glogit[e0 * HEADS + idx] = g;
+            if (LEFT) p.prob[e0 * HEADS + idx] = pj[idx];
         }
         __syncthreads();
         {
@@ -321,12 +326,13 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
     }
 }
 
-// gk_j = sum_i glogit_ij q_i, gv_j = sum_i p_ij gout_i with p_ij = exp(logit_ij - lse_i).  Block = eight consecutive keys (of
+// gk_j = sum_i glogit_ij q_i, gv_j = sum_i p_ij gout_i with p_ij = exp(logit_ij - lse_i) (PROB: as the rows left it).  Block = eight consecutive keys (of
 // one crystal at a time), warp = head: a row's values of the eight keys are contiguous in the n x n block, so they are read
 // coalesced, thirty-two rows at a time, and q and gout once for the eight keys (a warp per key and head read them, and the
 // columns with a stride, once per key: 0.11 ms against 0.02 ms at crystals of 100-200 atoms).
 constexpr int COL_KEYS = 8, COL_ROWS = 32;
 constexpr int COL_LD = COL_ROWS * COL_KEYS + 4;  // floats per head (bank skew)
+template <bool PROB>
 __global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRowArgs p)
 {
     __shared__ __align__(16) float gs[HEADS * COL_LD], ps[HEADS * COL_LD];
@@ -354,7 +360,7 @@ __global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRo
                     if (jj < keys) {
                         const long long e = (c0 + (long long)(i0 + i) * n + jl + jj) * HEADS + hh;
                         g = p.glogit[e];
-                        pr = ex2((p.logit[e] - p.lse[(first + i0 + i) * HEADS + hh]) * LOG2E);
+                        pr = PROB ? p.prob[e] : ex2((p.logit[e] - p.lse[(first + i0 + i) * HEADS + hh]) * LOG2E);
                     }
                     gs[hh * COL_LD + i * COL_KEYS + jj] = g;
                     ps[hh * COL_LD + i * COL_KEYS + jj] = pr;
@@ -385,6 +391,28 @@ __global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRo
     }
 }
 
+// LEFT: only the rows that a call over pair grids left over (p.rows_on_device of them), which also leave their probabilities
+template <bool LEFT>
+int launch_bwd(const BwdRowArgs &p, int64_t K, cudaStream_t s)
+{
+    const size_t smem = sizeof(float) * bwd_row_smem_floats(p.max_atoms, K > 0);
+    const long long grid_rows = LEFT ? p.N / 8 + 1 : p.N;
+    auto kernel = K > 0 ? infinite_attn_bwd_rows_kernel<64, LEFT> : infinite_attn_bwd_rows_kernel<0, LEFT>;
+    if (smem > 48 * 1024) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(CF_ERR_RANGE, "cf_infinite_attn_bwd: %zu bytes of shared memory for max_atoms=%d not available", smem, p.max_atoms);
+        }
+    }
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, smem) != cudaSuccess || occ <= 0) occ = 1;
+    const long long cap = (long long)sm_count() * occ;
+    kernel<<<(int)(grid_rows < cap ? grid_rows : cap), THREADS, smem, s>>>(p);
+    const long long tiles = (p.N + COL_KEYS - 1) / COL_KEYS, cap2 = (long long)sm_count() * 8;
+    infinite_attn_bwd_cols_kernel<LEFT><<<(int)(tiles < cap2 ? tiles : cap2), 256, 0, s>>>(p);
+    return launch_status("cf_infinite_attn_bwd");
+}
+
 }  // namespace
 
 int infinite_attn_bwd_impl(const float *q, const float *k, const float *v, const float *a, const float *pos,
@@ -394,6 +422,23 @@ int infinite_attn_bwd_impl(const float *q, const float *k, const float *v, const
                            double cutoff_radius, int lattice_range, int minimum_range, const float *logit,
                            const float *lse, const float *out, const float *gout, float *gq, float *gk, float *gv,
                            float *ga, float *glogit, const int32_t *row_order, const TermList *list, void *stream);
+
+// The backward over pair grids, by enumeration for the rows that the forward left over (p.leftover, counted in the grid's counters of
+// the call), then the sums over the rows for k and v.
+int grid_attn_bwd_impl(const PairAttn &l, const float *pos_ij, const float *tvecs, const int64_t *batch, const int64_t *edges,
+                       const int64_t *row_start, cudaStream_t s)
+{
+    const int rc = launch_pair_attn_bwd(l, s);
+    if (rc != CF_OK || l.N == 0) return rc;
+    BwdRowArgs p{};
+    p.q = l.q; p.k = l.k; p.v = l.v; p.a = l.a; p.pos_ij = pos_ij; p.tvecs = tvecs; p.rvlen = l.rvlen; p.W = l.W;
+    p.logit = l.logit; p.lse = l.lse; p.out = l.out; p.gout = l.gout; p.batch = batch; p.edges = edges; p.row_start = row_start;
+    p.gq = l.gq; p.gk = l.gk; p.gv = l.gv; p.ga = l.ga; p.glogit = l.glogit; p.prob = l.prob; p.N = l.N; p.E = l.E; p.max_atoms = l.max_atoms;
+    p.row_order = l.leftover; p.rows_on_device = l.grid.counters + 4 * (l.call + 1);
+    p.rule = l.rule;
+    p.basis = make_basis_params(l.K, l.dist_max, l.wscale, weight_floor_log2());
+    return launch_bwd<true>(p, l.K, s);
+}
 
 }  // namespace cf
 
@@ -468,20 +513,5 @@ int cf::infinite_attn_bwd_impl(const float *q, const float *k, const float *v, c
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     p.basis = make_basis_params(K, dist_max, wscale, weight_floor_log2());
     if (list != nullptr) p.list = *list;
-    const size_t smem = sizeof(float) * bwd_row_smem_floats((int)max_atoms, K > 0);
-    auto kernel = K > 0 ? infinite_attn_bwd_rows_kernel<64> : infinite_attn_bwd_rows_kernel<0>;
-    if (smem > 48 * 1024) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(CF_ERR_RANGE, "cf_infinite_attn_bwd: %zu bytes of shared memory for max_atoms=%lld not available",
-                        smem, (long long)max_atoms);
-        }
-    }
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, THREADS, smem) != cudaSuccess || occ <= 0) occ = 1;
-    const long long cap = (long long)sm_count() * occ;
-    kernel<<<(int)(N < cap ? N : cap), THREADS, smem, s>>>(p);
-    const long long tiles = (N + COL_KEYS - 1) / COL_KEYS, cap2 = (long long)sm_count() * 8;
-    infinite_attn_bwd_cols_kernel<<<(int)(tiles < cap2 ? tiles : cap2), 256, 0, s>>>(p);
-    return launch_status("cf_infinite_attn_bwd");
+    return launch_bwd<false>(p, K, s);
 }

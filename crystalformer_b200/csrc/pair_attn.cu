@@ -139,7 +139,7 @@ __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool 
         copy_wait<0>();
         __syncwarp();
         row.variant = __shfl_sync(FULL, hd.variant, __ffs(left) - 1);
-        ring.start(row.vectors(), first, N, 0);
+        ring.start(row.vectors(), first, N, PASS);
     }
     // heads 2t and 2t + 1 at nodes g and g + 8 of a tile
     const float2 aa = make_float2(__shfl_sync(FULL, a2h2, 8 * t), __shfl_sync(FULL, a2h2, 8 * t + 4));
@@ -226,12 +226,12 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     ring.init((unsigned)__cvta_generic_to_shared(smem + warp * L::REGION), i, n, row.slot_bytes, lane);
     auto start = [&]() {
         count = min(tiles, PASS);
-        ring.start(row.vectors(), 0, count, one_box ? tiles - count : 0);
+        ring.start(row.vectors(), 0, one_box ? tiles : count, PASS);
     };
     if (good) start();
 
     // ---- logits in bits
-    head_products(ops, p.k + a0 * (HEADS * HEAD_DIM) + warp * HEAD_DIM, n, warp, 0, 1, row.key_tiles, LOG2E, -INFINITY, tables, row_words, lane);
+    head_products<false>(ops, p.k + a0 * (HEADS * HEAD_DIM) + warp * HEAD_DIM, n, warp, 0, 1, row.key_tiles, LOG2E, -INFINITY, tables, row_words, lane);
     __syncthreads();
 
     // ---- a row per warp, or half of one
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
                     copy_wait<0>();
                     __syncwarp();
                     row.variant = __shfl_sync(FULL, hd.variant, 0);
-                    ring.start(row.vectors(), PASS, more, 0);
+                    ring.start(row.vectors(), PASS, more, PASS);
                 }
                 BY_TILES(more, node_pass<N>(row, ring, false, PASS, hd, lane, E, z, largest); copy_wait<0>(); __syncwarp();
                          store_e<N>(E, scale, smem + warp * L::REGION, lane);)
@@ -535,6 +535,12 @@ int grid_call(PairAttn &p, const char *who, const float *rvlen, const int64_t *a
     p.leftover = p.grid.leftover;
     return CF_OK;
 }
+// The rows that a forward marked, listed again for its backward
+__global__ void list_left_kernel(const unsigned char *__restrict__ left, long long N, int *__restrict__ list, unsigned *__restrict__ count)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N && left[i] != 0) list[atomicAdd(count, 1u)] = (int)i;
+}
 }  // namespace
 }  // namespace cf
 
@@ -578,4 +584,32 @@ extern "C" int cf_infinite_attn_fwd_grid(const float *q, const float *k, const f
     cudaStream_t s = as_stream(stream);
     if (cudaMemsetAsync(p.grid.counters + 4 * PG_LAYERS, 0, 4 * sizeof(unsigned), s) != cudaSuccess) return launch_status("cf_infinite_attn_fwd_grid");
     return grid_attn_impl(p, pos_ij, tvecs, batch, edges, row_start, cutoff_radius, lattice_range, minimum_range, s);
+}
+
+extern "C" int cf_infinite_attn_bwd_grid(const float *q, const float *k, const float *v, const float *a, const float *pos_ij,
+                                         const float *tvecs, const float *rvlen, const int64_t *batch, const int64_t *edges,
+                                         const int64_t *row_start, const int64_t *atom_start, const int64_t *edge_start, int64_t N, int64_t B,
+                                         int64_t H, int64_t D, int64_t E, int64_t K, int64_t max_atoms, double dist_max, double wscale,
+                                         const float *W, double cutoff_radius, int lattice_range, int minimum_range, double a_widest,
+                                         const float *logit, const float *lse, const uint8_t *left, const float *out, const float *gout,
+                                         float *gq, float *gk, float *gv, float *ga, float *glogit, float *prob, void *grids, void *stream)
+{
+    using namespace cf;
+    CF_REQUIRE(H == HEADS && D == HEAD_DIM, CF_ERR_UNSUPPORTED, "cf_infinite_attn_bwd_grid: H=%lld D=%lld, only H=8 D=16 is compiled",
+               (long long)H, (long long)D);
+    PairAttn p{};
+    const int rc = grid_call(p, "cf_infinite_attn_bwd_grid", rvlen, atom_start, edge_start, N, B, E, K, max_atoms, dist_max, wscale,
+                             cutoff_radius, lattice_range, minimum_range, a_widest, grids);
+    if (rc != CF_OK || N == 0) return rc;
+    CF_REQUIRE(q && k && v && a && pos_ij && tvecs && batch && edges && row_start && logit && lse && left && out && gout && gq && gk && gv &&
+               ga && glogit && prob && (K == 0 || W), CF_ERR_INVALID, "cf_infinite_attn_bwd_grid: null pointer");
+    p.q = q; p.k = k; p.v = v; p.a = a; p.W = W; p.out = const_cast<float *>(out); p.lse = const_cast<float *>(lse);
+    p.logit = const_cast<float *>(logit); p.left = const_cast<uint8_t *>(left); p.gout = gout;
+    p.gq = gq; p.gk = gk; p.gv = gv; p.ga = ga; p.glogit = glogit; p.prob = prob;
+    p.call = PG_LAYERS - 1;
+    cudaStream_t s = as_stream(stream);
+    unsigned *count = p.grid.counters + 4 * PG_LAYERS;
+    if (cudaMemsetAsync(count, 0, 4 * sizeof(unsigned), s) != cudaSuccess) return launch_status("cf_infinite_attn_bwd_grid");
+    list_left_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(left, N, p.leftover, count);
+    return grid_attn_bwd_impl(p, pos_ij, tvecs, batch, edges, row_start, s);
 }

@@ -30,8 +30,8 @@ struct KeyRing {
     static constexpr int KEY_LD = PA_STEP * 64 + 16, STAGE = PA_KEYS * KEY_LD, BYTES = STAGES * STAGE;
     const unsigned char *base, *k0, *k1;  // vectors of the crystal and variant, of the lane's keys
     int i, n, slot_bytes, key_tiles, lane_key, lane_byte;
-    int ft, fs, tiles, put, got;          // next step to fetch (key tile, first node tile of so many), stages
-    int next_first, next_tiles;           // the pass after this one, if it is of the same vectors (tiles > 0)
+    int ft, fs, tiles, put, got;          // next step to fetch (key tile, first node tile of the pass's so many), stages
+    int pass, remaining;                  // node tiles of a pass; those of the passes to come
     unsigned ring, dst, plain, trans;     // the lane's place in a stage: copies, ldmatrix, ldmatrix transposed
     __device__ __forceinline__ void init(unsigned ring_, int i_, int n_, int slot_bytes_, int lane)
     {
@@ -69,21 +69,23 @@ struct KeyRing {
             fs += PA_STEP;
             if (fs >= tiles) {
                 fs = 0;
-                if (++ft == key_tiles && next_tiles > 0) {  // on to the next pass
-                    base += next_first * 64;
-                    tiles = next_tiles;
-                    next_tiles = 0;
+                if (++ft == key_tiles && remaining > 0) {  // on to the next pass over the keys
+                    base += pass * 64;
+                    tiles = min(pass, remaining);
+                    remaining -= tiles;
                     ft = 0;
                 }
             }
         }
         copy_commit();
     }
-    // `more`: after these node tiles come so many more of the same vectors, another pass over the keys
-    __device__ __forceinline__ void start(const unsigned char *vectors, int first_tile, int tiles_, int more)
+    // `total` node tiles of a variant's vectors from `first_tile`, in passes over the keys of up to `pass` tiles
+    __device__ __forceinline__ void start(const unsigned char *vectors, int first_tile, int total, int pass_)
     {
         base = vectors + first_tile * 64 + lane_byte;
-        tiles = tiles_; next_first = tiles_; next_tiles = more;
+        pass = pass_;
+        tiles = min(pass, total);
+        remaining = total - tiles;
         ft = fs = put = got = 0;
 #pragma unroll
         for (int u = 0; u < STAGES - 1; ++u) fetch();
@@ -191,6 +193,7 @@ __device__ __forceinline__ HeadOperands head_operands(const float *__restrict__ 
     o.k1 = kp[min(first * PA_KEYS + g + 8, n - 1) * (HEADS * HEAD_DIM / 4)];
     return o;
 }
+template <bool SUM_ORDER>
 __device__ __forceinline__ void head_products(const HeadOperands &op, const float *__restrict__ keys, int n, int head, int first, int stride,
                                               int key_tiles, float scale, float pad, float *table, int row_words, int lane)
 {
@@ -201,7 +204,8 @@ __device__ __forceinline__ void head_products(const HeadOperands &op, const floa
     const float4 *kp = reinterpret_cast<const float4 *>(keys) + t;
     auto key = [&](int j) { return kp[min(j, n - 1) * (HEADS * HEAD_DIM / 4)]; };
     float4 k0 = op.k0, k1 = op.k1;
-    float *o = table + 2 * t * row_words + first * 128 + pa_key_word(head, g);
+    const int slot = SUM_ORDER ? pa_sum_slot(g, head >> 1) * 4 + (head & 1) : pa_key_word(head, g);  // (SUM_ORDER: that of the sums S)
+    float *o = table + 2 * t * row_words + first * 128 + slot;
     for (int T = first; T < key_tiles; T += stride, o += stride * 128) {
         const float4 a0 = k0, a1 = k1;
         const int j = T * PA_KEYS + g;

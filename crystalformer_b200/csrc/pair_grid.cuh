@@ -102,6 +102,16 @@ inline bool pair_grid_pays(long long N, long long B, long long E, long long max_
     return E >= 30000 || (K > 0 && E >= 18000 && E >= 24 * N);
 }
 
+// ... and whether a training step does: device time of a step (four layers), term lists against grids.  With a basis what it saves
+// grows with the rows: 495, 653, 962, 1,271 rows (crystals of up to 30 or 40 atoms) 527, 657, 689, 926 us against 545, 596, 594,
+// 685, few keys per row or many alike (1,173 rows of 6 keys 830 against 613, 504 of 41 650 against 630, 283 of 46 535 against 614).
+// Without one a row by lists costs little: 653, 962, 1,271, 5,321 rows 521, 521, 642, 1,564 against 513, 501, 548, 1,200, and 1,693
+// rows of 8 keys 576 against 584.
+inline bool pair_grid_pays_training(long long N, long long B, long long E, long long max_atoms, long long K)
+{
+    return pair_grid_fits(N, B, E, max_atoms) && (K > 0 ? N >= 640 && E >= 5 * N : N >= 960 && E >= 11 * N);
+}
+
 // One attention call over a batch's grids, and its backward.
 struct PairAttn {
     const float *q, *k, *v, *a, *rvlen, *W;
@@ -125,6 +135,9 @@ struct PairAttn {
 // basis at the nodes (W null: for calls with psi_row) or the calls' projections at the nodes (W of call c at W[c * W_stride]).
 int launch_pair_grid_build(const PairAttn &p, const float *pos_ij, const float *tvecs, float a_widest, const float *const *W, int W_stride,
                            int calls, cudaStream_t s);
+int launch_pair_attn_bwd(const PairAttn &p, cudaStream_t s);
+int grid_attn_bwd_impl(const PairAttn &p, const float *pos_ij, const float *tvecs, const int64_t *batch, const int64_t *edges,
+                       const int64_t *row_start, cudaStream_t s);
 // The attention, and the rows that it leaves over by enumeration (their logits too, where p.logit is given).
 int grid_attn_impl(const PairAttn &p, const float *pos_ij, const float *tvecs, const int64_t *batch, const int64_t *edges,
                    const int64_t *row_start, double cutoff_radius, int lattice_range, int minimum_range, cudaStream_t s);

@@ -4,15 +4,16 @@
 // The autograd path records some sixty framework operations per layer; on a batch of crystals each of them is a few
 // microseconds of device work, and the host needs about 5 ms to issue them.  Here a step is about forty launches of this
 // library's kernels:
-//   forward    weight images (both directions), batch geometry, term lists, then per layer the dense boundary
-//              (dense_tc.cu) and the fused attention (infinite_attn_fwd.cu), pooling + head
+//   forward    weight images (both directions), batch geometry, pair grids or term lists, then per layer the dense boundary
+//              (dense_tc.cu) and the fused attention (pair_attn.cu or infinite_attn_fwd.cu), pooling + head
 //   backward   head and pooling, then per layer the dense boundary (dense_tc_bwd.cu) and the attention backward
-//              (infinite_attn_bwd.cu), and at the end every weight gradient of the model in one launch each for the
+//              (pair_attn_bwd.cu, infinite_attn_bwd.cu), and at the end every weight gradient of the model in one launch each for the
 //              projections and for the value encoding
 // (models/latticeformer.py:211-302 with pooling "avr", a Linear - ReLU - Linear head and LayerNorm = Identity.)
 #include "common.cuh"
 #include "dense_tc.cuh"
 #include "infinite_attn_block.cuh"
+#include "pair_grid.cuh"
 #include "term_list.cuh"
 
 namespace cf {
@@ -228,6 +229,8 @@ struct LayerSaved {
     unsigned char *forward, *backward;  // weight images
     float *q, *k, *v, *a, *attn, *psi, *y, *h;
     float *lse, *logit;                              // domain real: the fused attention
+    unsigned char *left;                             // ... over pair grids: the rows left over, marked and listed
+    int *leftover;
     float *phi_real, *sum_reci, *phi, *values, *prob;  // others: the operator pair
 };
 struct Saved {
@@ -245,7 +248,7 @@ struct Saved {
     // memory whose size depends on the edges
     int64_t *edges;
     float *pos_ij, *kr, *phi_reci;
-    void *lists;
+    void *lists, *grid;
     size_t edge_bytes;
 };
 Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64_t N, int64_t B, int64_t E)
@@ -272,6 +275,8 @@ Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64
         y.q = c.take<float>(N * CH); y.k = c.take<float>(N * CH); y.v = c.take<float>(N * CH);
         y.a = c.take<float>(N * HEADS); y.lse = c.take<float>(N * HEADS);
         y.attn = c.take<float>(N * CH);
+        y.left = domain_of(d, l) == REAL ? c.take<unsigned char>(N) : nullptr;
+        y.leftover = domain_of(d, l) == REAL ? c.take<int>(N) : nullptr;
         y.psi = d.K > 0 && domain_of(d, l) == REAL ? c.take<float>(N * HEADS * d.K) : nullptr;
         y.y = c.take<float>(N * CH);
         y.h = c.take<float>(N * d.ff_dim);
@@ -302,6 +307,8 @@ Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64
     s.kr = split ? e.take<float>(3 * E) : nullptr;
     s.phi_reci = split ? e.take<float>(E * HEADS) : nullptr;
     s.lists = fused ? e.take<char>(term_list_workspace_bytes(N, E)) : nullptr;
+    const size_t grid = fused && N > 0 ? pair_grid_bytes(N, B, E, E / N) : 0;  // (the largest crystal has at least E / N atoms)
+    s.grid = grid > 0 ? e.take<char>(grid) : nullptr;
     s.edge_bytes = e.used;
     return s;
 }
@@ -312,7 +319,7 @@ struct LayerGrads {
 struct Scratch {
     float *gx[MAX_LAYERS + 1];
     LayerGrads layer[MAX_LAYERS];
-    float *glogit, *ghid, *partial, *pe_partial;
+    float *glogit, *prob, *ghid, *partial, *pe_partial;
     float *gphi, *g_real, *g_reci, *gvalues, *ga_reci, *pair;  // the operator pair's backward
     int shares;
     size_t bytes;
@@ -332,6 +339,7 @@ Scratch carve_scratch(const cf_train_desc &d, void *memory, int64_t N, int64_t B
     }
     s.gx[d.num_layers] = c.take<float>(N * CH);
     s.glogit = c.take<float>(E * HEADS);
+    s.prob = d.num_layers > 0 && N > 0 && pair_grid_bytes(N, B, E, E / N) > 0 ? c.take<float>(E * HEADS) : nullptr;
     bool split = false, values = false;
     for (int l = 0; l < d.num_layers; ++l) {
         split = split || domain_of(d, l) != REAL;
@@ -410,6 +418,38 @@ bool lists_of(const cf_train_desc &d, const Saved &s, int64_t N, int64_t E, Term
     list.pool = pool; list.start = start; list.count = count; list.dmin = dmin;
     list.window = term_window(weight_floor_log2(), a_widest);
     return true;
+}
+
+// Whether a batch's layers of domain real go by pair grids, and what their calls share.  Both halves of a step decide alike, from the
+// description and the sizes only (not from the process-wide floor, which may change in between: nodes in reach are chosen for
+// 2^-40 at least where terms are to be kept below 2^-30).
+bool grid_of(const cf_train_desc &d, const cf_train_batch &b, const Saved &w, PairAttn &p, float &a_widest)
+{
+    a_widest = -INFINITY;
+    double dist_max = 0.0;
+    for (int l = 0; l < d.num_layers; ++l) {
+        if (domain_of(d, l) != REAL) continue;
+        const double dm = d.scalars[SCALARS * l + 5];
+        if (d.K > 0 && dist_max != 0.0 && dm != dist_max) return false;  // (the nodes are those of one basis)
+        dist_max = dm;
+        a_widest = fmaxf(a_widest, (float)(d.scalars[SCALARS * l + 4] * d.scalars[SCALARS * l + 2]));
+    }
+    if (w.grid == nullptr || d.num_layers > PG_LAYERS || !pair_grid_pays_training(b.N, b.B, b.E, b.max_atoms, d.K)) return false;
+    const float floor = weight_floor_log2();
+    if (!pair_grid_params(d.K, dist_max, d.wscale, a_widest, -30.0f, p.par)) return false;
+    p.par.floor_log2 = floor < -30.0f ? -40.0f : -30.0f;
+    p.rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
+    p.atom_start = w.atom_start; p.edge_start = w.edge_start; p.N = b.N; p.B = b.B; p.E = b.E; p.K = d.K; p.max_atoms = (int)b.max_atoms;
+    p.rule = BoxRule{(float)d.cutoff_radius, d.lattice_range, d.minimum_range};
+    p.dist_max = dist_max; p.wscale = d.wscale;
+    p.grid = pair_grid_carve(w.grid, b.N, b.B, b.E);
+    return true;
+}
+// ... and one layer's
+void grid_layer(PairAttn &p, const cf_train_desc &d, const LayerSaved &t, int l)
+{
+    p.q = t.q; p.k = t.k; p.v = t.v; p.a = t.a; p.W = d.weights[PER_LAYER * l + W_PE]; p.call = l; p.out = t.attn; p.lse = t.lse;
+    p.psi_row = t.psi; p.logit = t.logit; p.left = t.left; p.leftover = t.leftover;
 }
 
 }  // namespace
@@ -559,8 +599,14 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
     const int32_t *order = ordered ? w.row_order : nullptr;
     const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
     TermList list{};
+    PairAttn by_grid{};
     float a_widest;
-    const bool listed = lists_of(d, w, N, E, list, a_widest);
+    const bool gridded = grid_of(d, b, w, by_grid, a_widest);
+    const bool listed = !gridded && lists_of(d, w, N, E, list, a_widest);
+    if (gridded) {
+        rc = launch_pair_grid_build(by_grid, w.pos_ij, b.trans, a_widest, nullptr, 0, 0, s);
+        if (rc != CF_OK) return rc;
+    }
     if (listed) {
         TermListBuild tb{};
         tb.pos_ij = w.pos_ij; tb.tvecs = b.trans; tb.rvlen = rvlen; tb.batch = w.batch; tb.edges = w.edges; tb.row_start = w.row_start;
@@ -586,7 +632,10 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
         const LayerSaved &t = w.layer[l];
         const Domain dom = domain_of(d, l);
         const double dist_max = d.scalars[SCALARS * l + 5];
-        if (dom == REAL && by_blocks) {
+        if (dom == REAL && gridded) {
+            grid_layer(by_grid, d, t, l);
+            rc = grid_attn_impl(by_grid, w.pos_ij, b.trans, w.batch, w.edges, w.row_start, d.cutoff_radius, d.lattice_range, d.minimum_range, s);
+        } else if (dom == REAL && by_blocks) {
             rc = block_attn_impl(t.q, t.k, t.v, t.a, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, E, d.K, b.max_atoms,
                                  dist_max, d.wscale, d.weights[PER_LAYER * l + W_PE], d.cutoff_radius, d.lattice_range, d.minimum_range,
                                  t.attn, t.logit, t.lse, t.psi, list, row_blocks, l, s);
@@ -638,8 +687,10 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
     const int32_t *order = rows_are_ordered(B, N) ? w.row_order : nullptr;
     const float *rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
     TermList list{};
+    PairAttn by_grid{};
     float a_widest;
-    const bool listed = lists_of(d, w, N, E, list, a_widest);
+    const bool gridded = grid_of(d, b, w, by_grid, a_widest);
+    const bool listed = !gridded && lists_of(d, w, N, E, list, a_widest);
 
     head_backward_kernel<<<(unsigned)B, 128, 0, s>>>(gy, w.hid, tail_weights[1], tail_weights[3], w.atom_start, hidden, targets, g.ghid, g.gx[L]);
     head_weight_grad_kernel<<<dim3((hidden + 31) / 32, targets), 256, 0, s>>>(gy, w.hid, B, hidden, targets, tail_grads[3], tail_grads[4]);
@@ -664,6 +715,13 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
         const LayerSaved &y = w.layer[l];
         const LayerGrads &gg = g.layer[l];
         const double dist_max = d.scalars[SCALARS * l + 5];
+        if (domain_of(d, l) == REAL && gridded) {
+            grid_layer(by_grid, d, y, l);
+            by_grid.gout = gg.gattn; by_grid.gq = gg.gq; by_grid.gk = gg.gk; by_grid.gv = gg.gv; by_grid.ga = gg.ga;
+            by_grid.glogit = g.glogit; by_grid.prob = g.prob;
+            rc = grid_attn_bwd_impl(by_grid, w.pos_ij, b.trans, w.batch, w.edges, w.row_start, s);
+            continue;
+        }
         if (domain_of(d, l) == REAL) {
             rc = infinite_attn_bwd_impl(y.q, y.k, y.v, y.a, nullptr, w.pos_ij, b.trans, rvlen, w.batch, w.edges, w.row_start, N, B, HEADS,
                                         HEAD_DIM, E, d.K, b.max_atoms, dist_max, d.wscale, d.weights[PER_LAYER * l + W_PE],

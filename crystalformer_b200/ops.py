@@ -346,6 +346,33 @@ def infinite_attn_fwd_grid(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_s
     return out, logit, lse, psi_row, left
 
 
+def infinite_attn_bwd_grid(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, max_atoms, K, dist_max, wscale, W,
+                           cutoff_radius, lattice_range, minimum_range, grids, logit, lse, left, out, gout):
+    """Backward of infinite_attn_fwd_grid: (gq, gk, gv, ga).  ``logit``, ``lse``, ``left``, ``out``: the forward's."""
+    dev = q.device
+    q, k, v, a, tvecs, logit, lse, out, gout = (_want(t, torch.float32, n, dev) for t, n in (
+        (q, "q"), (k, "k"), (v, "v"), (a, "a"), (tvecs, "tvecs"), (logit, "logit"), (lse, "lse"), (out, "out"), (gout, "gout")))
+    pos_ij, rvlen, W = (_want(t, torch.float32, n, dev) for t, n in ((pos_ij, "pos_ij"), (rvlen, "rvlen"), (W, "W")))
+    batch, edges, row_start = (_want(t, torch.int64, n, dev) for t, n in
+                               ((batch, "batch"), (edges, "edges"), (row_start, "row_start")))
+    left = _want(left, torch.uint8, "left", dev)
+    N, H, D = q.shape
+    _check_projection(W, H, K, "infinite_attn_bwd_grid")
+    E, B = edges.shape[1], tvecs.shape[0]
+    work, atom_start, edge_start, a_widest = grids
+    gq, gk, gv = (torch.empty_like(q) for _ in range(3))
+    ga = torch.empty((N, H), dtype=torch.float32, device=dev)
+    glogit, prob = (torch.empty((E, H), dtype=torch.float32, device=dev) for _ in range(2))
+    with torch.cuda.device(dev):
+        _lib.call("cf_infinite_attn_bwd_grid", _ptr(q), _ptr(k), _ptr(v), _ptr(a), _ptr(pos_ij), _ptr(tvecs), _ptr(rvlen),
+                  _ptr(batch), _ptr(edges), _ptr(row_start), _ptr(atom_start), _ptr(edge_start), c_int64(N), c_int64(B), c_int64(H),
+                  c_int64(D), c_int64(E), c_int64(K), c_int64(max_atoms), c_double(dist_max), c_double(wscale), _ptr(W),
+                  c_double(cutoff_radius or 0.0), c_int(lattice_range), c_int(minimum_range), c_double(a_widest), _ptr(logit),
+                  _ptr(lse), _ptr(left), _ptr(out), _ptr(gout), _ptr(gq), _ptr(gk), _ptr(gv), _ptr(ga), _ptr(glogit), _ptr(prob),
+                  _ptr(work), _stream(dev))
+    return gq, gk, gv, ga
+
+
 def infinite_attn_fwd(q, k, v, a, pos_ij, tvecs, rvlen, batch, edges, row_start, max_atoms, K, dist_max, wscale, W,
                       cutoff_radius, lattice_range, minimum_range, want_psi_row=False, pos=None, row_order=None,
                       term_lists=None):

@@ -302,6 +302,8 @@ int cf_infinite_attn_bwd_listed(const float *q, const float *k, const float *v, 
  *   grids: cf_pair_grid_bytes(N, B, E) bytes (0: more pairs than grids are kept for), 256-byte aligned; it also holds the
  *   counters of the calls that use it, so calls sharing it must be ordered (one stream).
  *   logit (E,H): or NULL; written for the rows left over only.  psi_row (N,H,K): or NULL.  left (N): or NULL.
+ *   cf_infinite_attn_bwd_grid is the backward as cf_infinite_attn_bwd's, from the same grids and the forward's logit, lse, left
+ *   and out; prob (E,H) is scratch (the probabilities, handed from its rows to its columns).
  *   max_atoms <= 64.  CF_ERR_UNSUPPORTED where the nodes of (dist_max, wscale) do not cover ordinary Gaussians.
  * ---------------------------------------------------------------------------------------------------------- */
 int64_t cf_pair_grid_bytes(int64_t N, int64_t B, int64_t E);
@@ -315,6 +317,14 @@ int cf_infinite_attn_fwd_grid(const float *q, const float *k, const float *v, co
                               int64_t B, int64_t H, int64_t D, int64_t E, int64_t K, int64_t max_atoms, double dist_max,
                               double wscale, const float *W, double cutoff_radius, int lattice_range, int minimum_range,
                               double a_widest, float *out, float *logit, float *lse, float *psi_row, uint8_t *left,
+                              void *grids, void *stream);
+int cf_infinite_attn_bwd_grid(const float *q, const float *k, const float *v, const float *a, const float *pos_ij,
+                              const float *tvecs, const float *rvlen, const int64_t *batch, const int64_t *edges,
+                              const int64_t *row_start, const int64_t *atom_start, const int64_t *edge_start, int64_t N,
+                              int64_t B, int64_t H, int64_t D, int64_t E, int64_t K, int64_t max_atoms, double dist_max,
+                              double wscale, const float *W, double cutoff_radius, int lattice_range, int minimum_range,
+                              double a_widest, const float *logit, const float *lse, const uint8_t *left, const float *out,
+                              const float *gout, float *gq, float *gk, float *gv, float *ga, float *glogit, float *prob,
                               void *grids, void *stream);
 
 /* ------------------------------------------------------------------------------------------------------------

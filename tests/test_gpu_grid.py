@@ -33,8 +33,8 @@ def inputs(cb, sigma, scale=0.3, seed=3):
     return q, k, v, a, W
 
 
-def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE):
-    """(grid results, enumerating kernel's results)"""
+def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE, gout=None):
+    """(grid results, enumerating kernel's results, the call again); with gout: the backward's, and the rows left over"""
     q, k, v, a, W = x
     sizes = dev(cb.sizes)
     atom_start, edge_start = ops.crystal_offsets(sizes)
@@ -45,6 +45,11 @@ def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE):
             nmax, K, DIST_MAX, wscale, W, cutoff, 2, minimum)
     grids = ops.pair_grid_build(g["pos_ij"], dev(cb.trans_vec), g["rvlen"], atom_start, edge_start, cb.num_atoms, nmax, K, DIST_MAX,
                                 wscale, cutoff, 2, minimum, A_WIDEST)
+    if gout is not None:
+        out, logit, lse, _, left = ops.infinite_attn_fwd_grid(*args, grids)
+        out0, logit0, lse0, _ = ops.infinite_attn_fwd(*args)
+        by_grid = lambda: ops.infinite_attn_bwd_grid(*args, grids, logit, lse, left, out, dev(gout))
+        return by_grid(), ops.infinite_attn_bwd(*args, logit0, lse0, out0, dev(gout)), by_grid, left
     return (ops.infinite_attn_fwd_grid(*args, grids, want_psi_row=K > 0), ops.infinite_attn_fwd(*args, want_psi_row=K > 0),
             lambda: ops.infinite_attn_fwd_grid(*args, grids, want_psi_row=K > 0))
 
@@ -139,3 +144,49 @@ def test_crystals_beyond_the_extra_vectors(ops):
     assert left[:int(cb.sizes[0])].all()
     ref, _ = reference(cb, x, 64, -3.5, 2)
     close(out, ref, out0, slice(None), "all rows")
+
+
+def backward_reference(cb, x, go, K, cutoff, minimum, wscale):
+    q, k, v, a, W = x
+    edges = oracle.edge_index(cb.sizes)
+    pos_ij, _, _, rvlen = oracle.geometry(cb.pos, cb.trans_vec, edges)
+    Wn = W[None] if K else None
+    common = dict(rvlen=rvlen, cutoff_radius=cutoff, lattice_range=2, minimum_range=minimum, precision="f64")
+    z, psiW = oracle.lattice_sum_fwd(a, pos_ij, cb.trans_vec, cb.batch, edges, K, DIST_MAX, wscale, W=Wn, **common)
+    prob, out = oracle.fused_attn_fwd(q, k, v, z, psiW, edges, precision="f64")
+    gq, gk, gv, g_phi, g_psiW = oracle.fused_attn_bwd(q, k, v, psiW, edges, prob, out, go, precision="f64")
+    ga, _ = oracle.lattice_sum_bwd(a, pos_ij, cb.trans_vec, cb.batch, edges, z, g_phi, g_psiW, K, DIST_MAX, wscale, W=Wn, **common)
+    return [np.asarray(t, np.float64).reshape(cb.num_atoms, -1) for t in (gq, gk, gv, ga)]
+
+
+# as the forward's, with gradients from 1e-10 to 1e10 (the columns of the products are scaled by the gradient's own size)
+@pytest.mark.parametrize("lo,hi,K,cutoff,minimum,lengths,sigma,wscale,size", [
+    (1, 9, 64, -3.5, 2, (3.0, 9.0), (1.18, 1.6), 1.0, 1.0), (15, 17, 64, -3.5, 2, (4.0, 12.0), (1.18, 1.6), 1.0, 1e-10),
+    (31, 33, 64, -3.5, 2, (4.0, 12.0), (1.0, 1.6), 1.0, 1e10), (40, 64, 64, -3.5, 2, (6.0, 12.0), (1.18, 1.6), 1.0, 1.0),
+    (8, 24, 64, -3.5, 0, (3.0, 9.0), (1.18, 1.6), 1.0, 1.0), (4, 12, 64, 0.0, 2, (3.0, 9.0), (1.18, 1.6), 1.0, 1.0),
+    (4, 20, 64, -3.5, 2, (3.0, 4.5), (1.2, 1.7), 1.0, 1.0), (4, 20, 64, -3.5, 2, (4.0, 9.0), (1.18, 1.6), 1.1, 1.0),
+    (1, 1, 64, -3.5, 2, (5.0, 9.0), (1.18, 1.6), 1.0, 1.0), (4, 20, 64, -3.5, 2, (3.0, 9.0), (0.3, 1.6), 1.0, 1.0),
+    (1, 17, 0, -3.5, 2, (3.0, 9.0), (1.18, 1.6), 1.0, 1e-10), (33, 64, 0, -3.5, 2, (4.0, 12.0), (1.18, 1.9), 1.0, 1.0),
+    (4, 20, 0, -3.5, 2, (3.0, 4.5), (1.2, 1.7), 1.0, 1e10)])
+def test_grid_backward_against_oracle_chain(ops, lo, hi, K, cutoff, minimum, lengths, sigma, wscale, size):
+    cb = make_crystals(41, 9, uniform_atoms(lo, hi), length_range=lengths)
+    x = inputs(cb, sigma)
+    go = (np.random.default_rng(5).standard_normal((cb.num_atoms, H, D)) * size).astype(np.float32)
+    got, plain, again, left = run(ops, cb, x, K, cutoff, minimum, wscale=wscale, gout=go)
+    assert 0.1 < left.float().mean() if sigma[0] < 0.5 else left.float().mean() < 0.1
+    for name, t, t0, ref in zip(("gq", "gk", "gv", "ga"), got, plain, backward_reference(cb, x, go, K, cutoff, minimum, wscale)):
+        close(t.flatten(1), ref, t0.flatten(1), slice(None), name)
+    assert all(torch.equal(s, t) for s, t in zip(got, again()))
+
+
+@pytest.mark.parametrize("K", [64, 0])
+def test_gradients_that_are_not_finite_stay_visible(ops, K):
+    """A NaN or an infinity in the gradient shows where the enumerating kernel shows it."""
+    cb = make_crystals(47, 4, uniform_atoms(4, 18), length_range=(4.0, 9.0))
+    starts = np.concatenate([[0], np.cumsum(cb.sizes)])
+    go = np.random.default_rng(5).standard_normal((cb.num_atoms, H, D)).astype(np.float32)
+    go[starts[0] + 1, 2, 3] = np.nan
+    go[starts[1] + 2, 5, 0] = np.inf
+    got, plain, _, _ = run(ops, cb, inputs(cb, (1.2, 1.5)), K, gout=go)
+    for t, t0 in zip(got, plain):
+        assert torch.equal(torch.isfinite(t), torch.isfinite(t0))
