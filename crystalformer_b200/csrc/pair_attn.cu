@@ -14,6 +14,8 @@
 // matters), three products each with the small ones first, or TF32 pairs where the range is the caller's (q, k, v, W, w S).
 // (Logits and sum p v by a row's own warp, with float32 sums, cost 10-20 % more: keys and values then come through the L1 once per
 // row instead of once per block, and shared memory, which shares its pipe, is what bounds the second phase.)
+#include <initializer_list>
+
 #include "pair_attn.cuh"
 
 namespace cf {
@@ -535,6 +537,13 @@ int grid_call(PairAttn &p, const char *who, const float *rvlen, const int64_t *a
     p.leftover = p.grid.leftover;
     return CF_OK;
 }
+// The kernels read rows in pieces of 16 bytes; a caller's tensors may lie anywhere
+bool in_pieces(std::initializer_list<const void *> pointers)
+{
+    uintptr_t any = 0;
+    for (const void *p : pointers) any |= (uintptr_t)p;
+    return (any & 15) == 0;
+}
 // The rows that a forward marked, listed again for its backward
 __global__ void list_left_kernel(const unsigned char *__restrict__ left, long long N, int *__restrict__ list, unsigned *__restrict__ count)
 {
@@ -579,6 +588,8 @@ extern "C" int cf_infinite_attn_fwd_grid(const float *q, const float *k, const f
     if (rc != CF_OK || N == 0) return rc;
     CF_REQUIRE(q && k && v && a && pos_ij && tvecs && batch && edges && row_start && out && lse && (K == 0 || W), CF_ERR_INVALID,
                "cf_infinite_attn_fwd_grid: null pointer");
+    CF_REQUIRE(in_pieces({q, k, v, out, lse, psi_row, W, grids}), CF_ERR_INVALID,
+               "cf_infinite_attn_fwd_grid: q, k, v, W, out, lse, psi_row and grids must start on 16 bytes");
     p.q = q; p.k = k; p.v = v; p.a = a; p.W = W; p.out = out; p.lse = lse; p.psi_row = psi_row; p.logit = logit; p.left = left;
     p.call = PG_LAYERS - 1;  // (its counters are cleared here: any number of calls per build, in one stream's order)
     cudaStream_t s = as_stream(stream);
@@ -603,6 +614,8 @@ extern "C" int cf_infinite_attn_bwd_grid(const float *q, const float *k, const f
     if (rc != CF_OK || N == 0) return rc;
     CF_REQUIRE(q && k && v && a && pos_ij && tvecs && batch && edges && row_start && logit && lse && left && out && gout && gq && gk && gv &&
                ga && glogit && prob && (K == 0 || W), CF_ERR_INVALID, "cf_infinite_attn_bwd_grid: null pointer");
+    CF_REQUIRE(in_pieces({q, k, v, out, gout, lse, W, gq, ga, glogit, prob, grids}), CF_ERR_INVALID,
+               "cf_infinite_attn_bwd_grid: q, k, v, W, out, gout, lse, gq, ga, glogit, prob and grids must start on 16 bytes");
     p.q = q; p.k = k; p.v = v; p.a = a; p.W = W; p.out = const_cast<float *>(out); p.lse = const_cast<float *>(lse);
     p.logit = const_cast<float *>(logit); p.left = const_cast<uint8_t *>(left); p.gout = gout;
     p.gq = gq; p.gk = gk; p.gv = gv; p.ga = ga; p.glogit = glogit; p.prob = prob;

@@ -304,7 +304,7 @@ int cf_infinite_attn_bwd_listed(const float *q, const float *k, const float *v, 
  *   logit (E,H): or NULL; written for the rows left over only.  psi_row (N,H,K): or NULL.  left (N): or NULL.
  *   cf_infinite_attn_bwd_grid is the backward as cf_infinite_attn_bwd's, from the same grids and the forward's logit, lse, left
  *   and out; prob (E,H) is scratch (the probabilities, handed from its rows to its columns).
- *   max_atoms <= 64.  CF_ERR_UNSUPPORTED where the nodes of (dist_max, wscale) do not cover ordinary Gaussians.
+ *   max_atoms <= 64; arrays of (N,...) and (E,...) floats, W and grids on 16 bytes.  CF_ERR_UNSUPPORTED where the nodes of (dist_max, wscale) do not cover ordinary Gaussians.
  * ---------------------------------------------------------------------------------------------------------- */
 int64_t cf_pair_grid_bytes(int64_t N, int64_t B, int64_t E);
 int cf_pair_grid_build(const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *atom_start,

@@ -20,7 +20,7 @@ def ops():
 
 
 def dev(x):
-    return torch.as_tensor(np.ascontiguousarray(x)).cuda()
+    return x if isinstance(x, torch.Tensor) else torch.as_tensor(np.ascontiguousarray(x)).cuda()
 
 
 def inputs(cb, sigma, scale=0.3, seed=3):
@@ -190,3 +190,13 @@ def test_gradients_that_are_not_finite_stay_visible(ops, K):
     got, plain, _, _ = run(ops, cb, inputs(cb, (1.2, 1.5)), K, gout=go)
     for t, t0 in zip(got, plain):
         assert torch.equal(torch.isfinite(t), torch.isfinite(t0))
+
+
+def test_tensors_off_sixteen_bytes_are_refused(ops):
+    cb = make_crystals(48, 2, uniform_atoms(4, 8), length_range=(5.0, 9.0))
+    x = inputs(cb, (1.2, 1.5))
+    off = torch.empty(x[0].size + 1, device="cuda")[1:].copy_(dev(x[0]).flatten()).view(x[0].shape)
+    with pytest.raises(RuntimeError, match="16 bytes"):
+        run(ops, cb, (off,) + x[1:], 64)
+    with pytest.raises(RuntimeError, match="16 bytes"):
+        run(ops, cb, x, 64, gout=off)
