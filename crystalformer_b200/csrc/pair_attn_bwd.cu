@@ -10,10 +10,11 @@
 // products, three node tiles at a time (their columns are 48 registers), every pass over all keys; p and glogit add up in the
 // tables.  (3) warp = head: gq.
 //
-// Bound: issue and latency of a warp's chain (128 registers, 16 warps on an SM, or 8 beyond 40 atoms where the tables fill it); the
-// vectors come from L2.  256 crystals of up to 40 atoms: 113 us per layer, 169 by term lists (infinite_attn_bwd.cu), whose work
-// grows with the images.  Error against 64 bits on 24 crystals of up to 30 atoms (gq, gk, gv, ga): 1.4, 1.4, 1.0, 1.8e-7, by lists
-// 2.2, 2.1, 1.0, 2.4e-7; S0's small products add up apart from the large ones (gv 1.04e-7 without).
+// Bound: issue and latency of a warp's chain (128 registers: 16 warps on an SM; 8 beyond 48 atoms, where the tables of one block
+// fill it); the vectors come from L2.  256 crystals of up to 40 atoms: 78 us per layer (112 with 8 warps on an SM, u apart from the
+// sums), 169 by term lists (infinite_attn_bwd.cu), whose work grows with the images.  Error against 64 bits on 24 crystals of up to
+// 30 atoms (gq, gk, gv, ga): 1.4, 1.4, 1.0, 1.8e-7, by lists 2.2, 2.1, 1.0, 2.4e-7; S0's small products add up apart from the large
+// ones (gv 1.04e-7 without).
 #include "pair_attn.cuh"
 
 namespace cf {
@@ -41,9 +42,14 @@ struct Args {
 
 // logits, gout.v, p and glogit of a row, each in the order of the sums S
 __host__ __device__ constexpr int table_words(int max_atoms) { return ((max_atoms + PA_KEYS - 1) / PA_KEYS) * 128 + 4; }
+// p and glogit of a row lie side by side, and there its u before
+__host__ __device__ constexpr int sums_words(int max_atoms, bool basis)
+{
+    return basis && 2 * table_words(max_atoms) - 4 < U_LD ? U_LD : 2 * table_words(max_atoms) - 4;
+}
 size_t smem_bytes(int max_atoms, bool basis)
 {
-    return (size_t)WARPS * RING + sizeof(float) * (4 * PG_ROWS * table_words(max_atoms) + (basis ? PG_ROWS * U_LD : 0));
+    return (size_t)WARPS * RING + sizeof(float) * PG_ROWS * (2 * table_words(max_atoms) + sums_words(max_atoms, basis));
 }
 
 // x f as the operand of a product over the nodes (nodes x heads), f given at nodes g, g + 8 and heads 2t, 2t + 1
@@ -62,7 +68,8 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0), g = lane >> 2, t = lane & 3;
     const int row_words = table_words(p.max_atoms);
     float *logits = reinterpret_cast<float *>(smem + WARPS * RING), *dvs = logits + PG_ROWS * row_words;
-    float *probs = dvs + PG_ROWS * row_words, *glogits = probs + PG_ROWS * row_words, *us = glogits + PG_ROWS * row_words;
+    const int sums_ld = sums_words(p.max_atoms, BASIS);
+    float *probs = dvs + PG_ROWS * row_words, *glogits = probs + row_words, *us = probs;
     __shared__ int there[PG_ROWS];
     if (blockIdx.x >= p.counters[0]) return;
     const int4 tile = p.tiles[2 * blockIdx.x], place = p.tiles[2 * blockIdx.x + 1];
@@ -103,8 +110,8 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
             for (int c = 0; c < 4; ++c) { ax[c][0] = __ldg(w + c * 64 + bt * 16); ax[c][1] = __ldg(w + c * 64 + bt * 16 + 8); }
             float c[4];
             mma_exact(c, {ax[0][0], ax[0][1], ax[1][0], ax[1][1]}, {ax[2][0], ax[2][1], ax[3][0], ax[3][1]}, bh, bl, b3);
-            float *o = us + 2 * t * U_LD + warp * 64 + bt * 16 + g;
-            o[0] = c[0]; o[U_LD] = c[1]; o[8] = c[2]; o[U_LD + 8] = c[3];
+            float *o = us + 2 * t * sums_ld + warp * 64 + bt * 16 + g;
+            o[0] = c[0]; o[sums_ld] = c[1]; o[8] = c[2]; o[sums_ld + 8] = c[3];
         }
     }
     if (lane == 0) there[warp] = mine_here ? 1 : 0;
@@ -114,8 +121,8 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
     if (mine_here) {
         float4 *lg = reinterpret_cast<float4 *>(logits + warp * row_words) + pa_sum_slot(g, t);
         float4 *dv = reinterpret_cast<float4 *>(dvs + warp * row_words) + pa_sum_slot(g, t);
-        float4 *pr = reinterpret_cast<float4 *>(probs + warp * row_words) + pa_sum_slot(g, t);
-        float4 *gl = reinterpret_cast<float4 *>(glogits + warp * row_words) + pa_sum_slot(g, t);
+        float4 *pr = reinterpret_cast<float4 *>(probs + warp * sums_ld) + pa_sum_slot(g, t);
+        float4 *gl = reinterpret_cast<float4 *>(glogits + warp * sums_ld) + pa_sum_slot(g, t);
         // the nodes in reach, as the forward chose them
         float top0 = -INFINITY, top1 = -INFINITY;
         for (int T = 0; T < key_tiles; ++T) {
@@ -151,7 +158,6 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
             const float4 l = lg[T * 32], d = dv[T * 32];
             lg[T * 32] = make_float4(ex2(l.x - lse0) * 0x1p-20f, ex2(l.y - lse1) * 0x1p-20f, ex2(l.z - lse0) * 0x1p-20f, ex2(l.w - lse1) * 0x1p-20f);
             dv[T * 32] = make_float4(d.x - d0, d.y - d1, d.z - d0, d.w - d1);
-            if (!one_box) pr[T * 32] = gl[T * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         // u of head g as the operand of c (bins x heads), scaled to a largest value between 2^10 and 2^11
         unsigned uh[4][2], ul[4][2];
@@ -163,7 +169,7 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
             for (int bt = 0; bt < 4; ++bt)
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    u[bt][x] = *reinterpret_cast<const float2 *>(us + warp * U_LD + g * 64 + bt * 16 + 8 * x + 2 * t);
+                    u[bt][x] = *reinterpret_cast<const float2 *>(us + warp * sums_ld + g * 64 + bt * 16 + 8 * x + 2 * t);
                     most = fmaxf(most, fmaxf(fabsf(u[bt][x].x), fabsf(u[bt][x].y)));
                 }
             most = fmaxf(most, __shfl_xor_sync(FULL, most, 1));
@@ -176,6 +182,10 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
                 for (int x = 0; x < 2; ++x) split_f16(u[bt][x].x * scale, u[bt][x].y * scale, uh[bt][x], ul[bt][x]);
             c_scale0 = __shfl_sync(FULL, inv, 8 * t);
             c_scale1 = __shfl_sync(FULL, inv, 8 * t + 4);
+        }
+        if (!one_box) {
+            __syncwarp();  // (u has been read)
+            for (int T = 0; T < key_tiles; ++T) pr[T * 32] = gl[T * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         // The columns are x, x c, x n^2 and x c n^2 (n: nodes from zero), scaled: x by 2^15, c by u's scale and 2^2 over the
         // basis' (c is at most 2.6 of u's largest), n^2 by 2^-9 (x n^2 is at most 2 / e of sigma^2 in node spacings: 550)
@@ -336,7 +346,7 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
     {
         const float *k0 = kp + g;
         const bool in = there[g] != 0;
-        const float *gr = glogits + g * row_words + (warp & 1);
+        const float *gr = glogits + g * sums_ld + (warp & 1);
         const int slot0 = pa_sum_slot(2 * t, warp >> 1) * 4, slot1 = pa_sum_slot(2 * t + 1, warp >> 1) * 4;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         for (int T = 0; T < key_tiles; ++T) {
