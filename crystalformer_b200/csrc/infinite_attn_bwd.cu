@@ -37,6 +37,7 @@ struct BwdRowArgs {
     BasisParams basis;
     TermList list;  // optional (pool == NULL: none): the rows' terms, found once per batch (term_list.cuh)
     const unsigned *rows_on_device;  // optional: the number of rows to process (entries of row_order), read on the device
+    bool pieces;    // logit, lse, glogit and prob start on 16 bytes (a caller's may lie anywhere)
     float *prob;    // optional (E,H): p_ij, written by the rows and read by the columns instead of exp(logit - lse)
 };
 
@@ -326,18 +327,22 @@ __global__ void __launch_bounds__(THREADS, 4) infinite_attn_bwd_rows_kernel(cons
     }
 }
 
-// gk_j = sum_i glogit_ij q_i, gv_j = sum_i p_ij gout_i with p_ij = exp(logit_ij - lse_i) (PROB: as the rows left it).  Block = eight consecutive keys (of
-// one crystal at a time), warp = head: a row's values of the eight keys are contiguous in the n x n block, so they are read
-// coalesced, thirty-two rows at a time, and q and gout once for the eight keys (a warp per key and head read them, and the
-// columns with a stride, once per key: 0.11 ms against 0.02 ms at crystals of 100-200 atoms).
-constexpr int COL_KEYS = 8, COL_ROWS = 32;
+// gk_j = sum_i glogit_ij q_i, gv_j = sum_i p_ij gout_i with p_ij = exp(logit_ij - lse_i) (PROB: as the rows left it).  Block = eight
+// consecutive keys (of one crystal at a time), warp = head: a row's values of the eight keys are contiguous in the n x n block, so
+// they are read coalesced, thirty-two rows at a time, and q and gout once for the eight keys (a warp per key and head read them, and
+// the columns with a stride, once per key: 0.11 ms against 0.02 ms at crystals of 100-200 atoms).
+// Bound by latency (27 MB at 16 crystals of 100-200 atoms, 4 us) and issue: the next rows' values, two 16-byte pieces per thread and
+// array, are on their way while these are summed, and q and gout are read sixteen rows at a time at constant offsets.  There 27 us
+// (a word per thread and wait, offsets by row: 47; the pieces alone: 37), 256 crystals of up to 40 atoms 16.6 us (18.5).
+constexpr int COL_KEYS = 8, COL_ROWS = 32, COL_PIECES = COL_ROWS * COL_KEYS * HEADS / 4 / 256;
 constexpr int COL_LD = COL_ROWS * COL_KEYS + 4;  // floats per head (bank skew)
 template <bool PROB>
-__global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRowArgs p)
+__global__ void __launch_bounds__(256, 3) infinite_attn_bwd_cols_kernel(const BwdRowArgs p)
 {
     __shared__ __align__(16) float gs[HEADS * COL_LD], ps[HEADS * COL_LD];
     const int tid = threadIdx.x, lane = tid & 31, h = tid >> 5;
     const int d = lane & 15, par = lane >> 4;
+    const int pi = tid >> 4, pj = (tid >> 1) & 7, ph = (tid & 1) * 4;  // the thread's piece: row, key, four heads
     for (long long tile = blockIdx.x; tile * COL_KEYS < p.N; tile += gridDim.x) {
         long long j0 = tile * COL_KEYS;
         const long long tile_end = min(j0 + COL_KEYS, p.N);
@@ -348,37 +353,65 @@ __global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRo
             const long long first = p.edges[p.E + r0];
             const long long c0 = p.row_start[first];
             const int jl = (int)(j0 - first), keys = (int)(min(tile_end, first + n) - j0);
+            const size_t at = ((size_t)c0 + jl + pj) * HEADS + ph;
+            auto four = [&](const float *x) { return p.pieces ? *reinterpret_cast<const float4 *>(x) : make_float4(x[0], x[1], x[2], x[3]); };
+            float4 g[COL_PIECES], w[COL_PIECES], ls[COL_PIECES];
+            auto fetch = [&](int i0) {
+#pragma unroll
+                for (int u = 0; u < COL_PIECES; ++u) {
+                    const int i = i0 + pi + 16 * u;
+                    g[u] = w[u] = ls[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (i < n && pj < keys) {
+                        const size_t e = at + (size_t)i * n * HEADS;
+                        g[u] = four(p.glogit + e);
+                        w[u] = four((PROB ? p.prob : p.logit) + e);
+                        if (!PROB) ls[u] = four(p.lse + (first + i) * HEADS + ph);
+                    }
+                }
+            };
             float ak[COL_KEYS], av[COL_KEYS];
 #pragma unroll
             for (int u = 0; u < COL_KEYS; ++u) ak[u] = av[u] = 0.f;
+            fetch(0);
             for (int i0 = 0; i0 < n; i0 += COL_ROWS) {
                 const int rows = min(COL_ROWS, n - i0);
                 __syncthreads();  // (the previous chunk has been read)
-                for (int idx = tid; idx < rows * 64; idx += 256) {
-                    const int i = idx >> 6, jj = (idx >> 3) & 7, hh = idx & 7;
-                    float g = 0.f, pr = 0.f;
-                    if (jj < keys) {
-                        const long long e = (c0 + (long long)(i0 + i) * n + jl + jj) * HEADS + hh;
-                        g = p.glogit[e];
-                        pr = PROB ? p.prob[e] : ex2((p.logit[e] - p.lse[(first + i0 + i) * HEADS + hh]) * LOG2E);
-                    }
-                    gs[hh * COL_LD + i * COL_KEYS + jj] = g;
-                    ps[hh * COL_LD + i * COL_KEYS + jj] = pr;
+#pragma unroll
+                for (int u = 0; u < COL_PIECES; ++u) {
+                    const int o = ph * COL_LD + (pi + 16 * u) * COL_KEYS + pj;
+                    const float4 x = w[u];
+                    auto prob = [&](float v, float l) { return PROB ? v : ex2((v - l) * LOG2E); };
+                    gs[o] = g[u].x; gs[o + COL_LD] = g[u].y; gs[o + 2 * COL_LD] = g[u].z; gs[o + 3 * COL_LD] = g[u].w;
+                    ps[o] = prob(x.x, ls[u].x); ps[o + COL_LD] = prob(x.y, ls[u].y);
+                    ps[o + 2 * COL_LD] = prob(x.z, ls[u].z); ps[o + 3 * COL_LD] = prob(x.w, ls[u].w);
                 }
                 __syncthreads();
-                const float *qp = p.q + (first + i0) * HEADS * HEAD_DIM + h * HEAD_DIM + d;
-                const float *gp = p.gout + (first + i0) * HEADS * HEAD_DIM + h * HEAD_DIM + d;
-#pragma unroll 4
-                for (int i = par; i < rows; i += 2) {
-                    const float qv = __ldg(qp + (size_t)i * HEADS * HEAD_DIM), gv = __ldg(gp + (size_t)i * HEADS * HEAD_DIM);
-                    const float4 *g4 = reinterpret_cast<const float4 *>(gs + h * COL_LD + i * COL_KEYS);
-                    const float4 *p4 = reinterpret_cast<const float4 *>(ps + h * COL_LD + i * COL_KEYS);
-                    const float4 g0 = g4[0], g1 = g4[1], p0 = p4[0], p1 = p4[1];
+                if (i0 + COL_ROWS < n) fetch(i0 + COL_ROWS);
+                const float *qp = p.q + (first + i0 + par) * HEADS * HEAD_DIM + h * HEAD_DIM + d;
+                const float *gp = p.gout + (first + i0 + par) * HEADS * HEAD_DIM + h * HEAD_DIM + d;
+                const float4 *g4 = reinterpret_cast<const float4 *>(gs + h * COL_LD + par * COL_KEYS);
+                const float4 *p4 = reinterpret_cast<const float4 *>(ps + h * COL_LD + par * COL_KEYS);
+                auto sum = [&](int u, float qv, float gv) {  // row 2u + par
+                    const float4 g0 = g4[4 * u], g1 = g4[4 * u + 1], p0 = p4[4 * u], p1 = p4[4 * u + 1];
                     ak[0] = fmaf(g0.x, qv, ak[0]); ak[1] = fmaf(g0.y, qv, ak[1]); ak[2] = fmaf(g0.z, qv, ak[2]); ak[3] = fmaf(g0.w, qv, ak[3]);
                     ak[4] = fmaf(g1.x, qv, ak[4]); ak[5] = fmaf(g1.y, qv, ak[5]); ak[6] = fmaf(g1.z, qv, ak[6]); ak[7] = fmaf(g1.w, qv, ak[7]);
                     av[0] = fmaf(p0.x, gv, av[0]); av[1] = fmaf(p0.y, gv, av[1]); av[2] = fmaf(p0.z, gv, av[2]); av[3] = fmaf(p0.w, gv, av[3]);
                     av[4] = fmaf(p1.x, gv, av[4]); av[5] = fmaf(p1.y, gv, av[5]); av[6] = fmaf(p1.z, gv, av[6]); av[7] = fmaf(p1.w, gv, av[7]);
+                };
+                constexpr int STEP = 2 * HEADS * HEAD_DIM;
+                int u0 = 0;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {  // sixteen rows at a time: constant offsets
+                    if (rows < 16 * (half + 1)) break;
+                    float qv[8], gv[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) { qv[u] = __ldg(qp + (8 * half + u) * STEP); gv[u] = __ldg(gp + (8 * half + u) * STEP); }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) sum(8 * half + u, qv[u], gv[u]);
+                    u0 = 8 * (half + 1);
                 }
+#pragma unroll 4
+                for (int u = u0; 2 * u + par < rows; ++u) sum(u, __ldg(qp + u * STEP), __ldg(gp + u * STEP));
             }
 #pragma unroll
             for (int u = 0; u < COL_KEYS; ++u) {
@@ -393,8 +426,9 @@ __global__ void __launch_bounds__(256) infinite_attn_bwd_cols_kernel(const BwdRo
 
 // LEFT: only the rows that a call over pair grids left over (p.rows_on_device of them), which also leave their probabilities
 template <bool LEFT>
-int launch_bwd(const BwdRowArgs &p, int64_t K, cudaStream_t s)
+int launch_bwd(BwdRowArgs p, int64_t K, cudaStream_t s)
 {
+    p.pieces = (((uintptr_t)p.logit | (uintptr_t)p.lse | (uintptr_t)p.glogit | (uintptr_t)p.prob) & 15) == 0;
     const size_t smem = sizeof(float) * bwd_row_smem_floats(p.max_atoms, K > 0);
     const long long grid_rows = LEFT ? p.N / 8 + 1 : p.N;
     auto kernel = K > 0 ? infinite_attn_bwd_rows_kernel<64, LEFT> : infinite_attn_bwd_rows_kernel<0, LEFT>;

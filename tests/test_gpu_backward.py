@@ -140,3 +140,31 @@ def test_lattice_sum_backward_takes_gradients_that_are_views(ops):
     row_start = dev(oracle.row_starts(edges, N))
     ref, got = (ops.lattice_sum_bwd(*base, row_start, z, gz, g, K, DIST_MAX, WSCALE, **kw) for g in (gv, odd))
     assert odd.data_ptr() % 16 == 4 and all(torch.equal(r, o) for r, o in zip(ref, got))
+
+
+@pytest.mark.parametrize("sizes", [[1, 8, 9, 15, 16, 17], [31, 32, 33, 1, 65], [7, 48, 3, 130]])
+def test_gradients_of_keys_and_values_from_the_logits(ops, sizes):
+    """The sums over the rows, in float64 from the forward's own logits: around the chunks of 16 and 32 rows and tiles of 8 keys, and
+    with logits and lse that do not lie on 16 bytes.  Tolerance: an exponent of up to 20 carries 2^-24 of it into a probability, and
+    the differences gout.v - delta cancel to a few tenths of their terms."""
+    cb = make_crystals(74, len(sizes), lambda rng, b: np.array(sizes), length_range=(6.0, 14.0))
+    N, E, m = cb.num_atoms, cb.num_edges, max(sizes)
+    sz = dev(cb.sizes)
+    atom_start, edge_start = ops.crystal_offsets(sz)
+    g = ops.batch_prepare(dev(cb.pos), dev(cb.trans_vec), sz, atom_start, edge_start, N, E)
+    rng = np.random.default_rng(9)
+    q, k, v, go = (dev((rng.standard_normal((N, H, D)) * s).astype(np.float32)) for s in (0.5, 1.0, 1.0, 1.0))
+    a = dev((-0.5 / (1.0 + 0.6 * rng.random((N, H))) ** 2).astype(np.float32))
+    args = (q, k, v, a, g["pos_ij"], dev(cb.trans_vec), g["rvlen"], g["batch"], g["edges"], g["row_start"], m, 0, DIST_MAX, WSCALE, None, -3.5, 2, 2)
+    out, logit, lse, _ = ops.infinite_attn_fwd(*args)
+    _, gk, gv, _ = ops.infinite_attn_bwd(*args, logit, lse, out, go)
+    i, j = g["edges"]
+    d = lambda t: t.double()
+    p = torch.exp(d(logit) - d(lse)[i])
+    gl = p * ((d(go)[i] * d(v)[j]).sum(-1) - (d(go) * d(out)).sum(-1)[i])
+    for t, w, x in ((gk, gl, q), (gv, p, go)):
+        ref = torch.zeros((N, H, D), device="cuda", dtype=torch.float64).index_add_(0, j, w[:, :, None] * d(x)[i])
+        assert float((d(t) - ref).norm() / ref.norm()) < 4e-6
+    shifted = [torch.empty(t.numel() + 1, device="cuda")[1:].copy_(t.flatten()).view(t.shape) for t in (logit, lse)]
+    again = ops.infinite_attn_bwd(*args, *shifted, out, go)
+    assert torch.equal(gk, again[1]) and torch.equal(gv, again[2])
