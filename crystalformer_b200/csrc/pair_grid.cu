@@ -219,8 +219,9 @@ __device__ constexpr Coefs COEF_BASIS = {{
 
 constexpr int UNIT = PG_UNIT;                   // pairs of a warp, four lanes each
 constexpr int LIST = 24;                        // places of a lane waiting for their nodes
+constexpr int AT_ONCE = 2;                      // places that a lane works on at a time
 constexpr int ROOM = 5;                         // images between two looks at the lists: the usual box's column
-constexpr int BUILD_WARPS = 4;
+constexpr int BUILD_WARPS = 4, BUILD_BLOCKS = 5;
 constexpr int MAX_RUN = 4;                      // units in a row that a warp takes
 __host__ __device__ constexpr size_t build_smem(int tiles) { return BUILD_WARPS * sizeof(float) * ((size_t)(tiles * PG_TILE + PG_POINTS) * UNIT + LIST * 32); }
 
@@ -251,10 +252,13 @@ __device__ __forceinline__ int crystal_of_unit(const int *unit_start, int B, int
 // the nodes of one place are disjoint, places come one after the other, so there are no conflicts and no atomics, and a pair's
 // images add in a fixed order.  In shared memory node m of pair p lies in bank 8 m + p: a quarter's nodes are 3 apart from the next
 // one's, so the 32 lanes meet no bank twice.
-// Bound by instruction issue.  One pair per lane, with all twelve nodes in its own column, left room for seven warps on an SM:
-// 591 us for 0.8 M vectors of 1,024 crystals of up to 60 atoms, 63 us for 128 of up to 30.
+// Bound by instruction issue and the waits of a lane's chain (0.73 M vectors of 1,024 crystals of up to 60 atoms: 410 us; their
+// bytes 80).  So two places are worked on at a time, without spills (95 registers, twenty warps on an SM; at 80 and twenty-four
+// 465 us, three or four places at 114 and sixteen 415 and 425), and since a unit's images differ by a factor of ten, warps take
+// units as they come free: 256 crystals of up to 40 atoms 80 us, 190 with equal shares and one place at a time; 128 of up to 30 30
+// and 36 us.  One pair per lane, with all twelve nodes in its own column, left room for seven warps: 591 us and 63.
 template <int TILES>
-__global__ void __launch_bounds__(32 * BUILD_WARPS, 6) pair_grid_kernel(const BuildArgs p)
+__global__ void __launch_bounds__(32 * BUILD_WARPS, BUILD_BLOCKS) pair_grid_kernel(const BuildArgs p)
 {
     extern __shared__ __align__(16) float build_mem[];
     const int lane = threadIdx.x & 31, quarter = lane >> 3, mine = lane & 7;
@@ -275,12 +279,19 @@ __global__ void __launch_bounds__(32 * BUILD_WARPS, 6) pair_grid_kernel(const Bu
                                   PG_RHO_SCALE * (quarter < 2 ? (quarter == 0 ? o0 : o1) : (quarter == 2 ? o2 : o3)));
         }
     const int units = p.grid.unit_start[p.B], warps = gridDim.x * BUILD_WARPS;
-    const int length = max(1, min(MAX_RUN, units / warps)), turn = warps * length;
+    const int length = max(1, min(MAX_RUN, units / (4 * warps)));
     int c = 0, c_begin = 0, c_end = 0;  // the crystal and its units
     int4 info = make_int4(0, 0, 0, 0);
     Cell cell;
     float inv_t3sq = 0.f;
-    for (int run = (blockIdx.x * BUILD_WARPS + (threadIdx.x >> 5)) * length, u = run; u < units; u = u + 1 < run + length ? u + 1 : (run += turn)) {
+    // runs of units: the first by the warp's number, the others as warps come free (a unit's images differ by a factor of ten)
+    int run = (blockIdx.x * BUILD_WARPS + (threadIdx.x >> 5)) * length, u = run, ticket = 0;
+    auto next_unit = [&]() {
+        if (++u < run + length) return;
+        u = run = warps * length + __shfl_sync(FULL, ticket, 0);
+    };
+    for (; u < units; next_unit()) {
+        if (u == run && lane == 0) ticket = (int)atomicAdd(p.grid.counters + 1, (unsigned)length);
         if (u < c_begin || u >= c_end) {
             c = crystal_of_unit(p.grid.unit_start, (int)p.B, u, lane);
             c_begin = p.grid.unit_start[c];
@@ -317,7 +328,7 @@ __global__ void __launch_bounds__(32 * BUILD_WARPS, 6) pair_grid_kernel(const Bu
         auto spread = [&]() {
             // x = d / h to a few 2^-24 of a node spacing, not of d: the square root of d2 / h^2 in two floats, one Newton step in
             // the remainder; kept as node and 24 bits of the rest
-            const int longest = __reduce_max_sync(FULL, count);
+            const int longest = (__reduce_max_sync(FULL, count) + AT_ONCE - 1) / AT_ONCE * AT_ONCE;
             for (int t = 0; t < longest; ++t) {  // (shorter lists end in places beyond the nodes)
                 const float d2 = __uint_as_float(list[t * 32 + lane]);
                 const float s = d2 * p.inv_h2, s_low = fmaf(d2, p.inv_h2_low, fmaf(d2, p.inv_h2, -s));
@@ -332,23 +343,34 @@ __global__ void __launch_bounds__(32 * BUILD_WARPS, 6) pair_grid_kernel(const Bu
                 const int most = __reduce_max_sync(FULL, __shfl_sync(FULL, count, from * 8 + mine));
                 const unsigned *at = list + from * 8 + mine;
 #pragma unroll 1
-                for (int t = 0; t < most; ++t, at += 32) {
-                    const unsigned place = *at;
-                    float *node = hist + ((place >> 24) + 3 * quarter) * UNIT + mine;
-                    const float y = fmaf((float)(place & 0xffffffu), 0x1p-24f, -0.5f), y2 = y * y;
-                    const float2 yy = make_float2(y2, y2);
-                    float2 v[3];
+                for (int t = 0; t < most; t += AT_ONCE, at += 32 * AT_ONCE) {  // AT_ONCE at a time: one's sums of products fill the other's waits
+                    unsigned place[AT_ONCE];
+                    float2 v[AT_ONCE][3], yy[AT_ONCE];
+                    float y[AT_ONCE];
 #pragma unroll
-                    for (int q = 0; q < 3; ++q) v[q] = fma2(k[q][4], yy, k[q][3]);
+                    for (int w = 0; w < AT_ONCE; ++w) place[w] = at[32 * w];
+#pragma unroll
+                    for (int w = 0; w < AT_ONCE; ++w) {
+                        y[w] = fmaf((float)(place[w] & 0xffffffu), 0x1p-24f, -0.5f);
+                        yy[w] = make_float2(y[w] * y[w], y[w] * y[w]);
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) v[w][q] = fma2(k[q][4], yy[w], k[q][3]);
+                    }
 #pragma unroll
                     for (int d = 2; d >= 0; --d)
 #pragma unroll
-                        for (int q = 0; q < 3; ++q) v[q] = fma2(v[q], yy, k[q][d]);
-                    const float h0 = node[0], h1 = node[UNIT], h2 = node[2 * UNIT];
-                    node[0] = h0 + fmaf(v[0].y, y, v[0].x);
-                    node[UNIT] = h1 + fmaf(v[1].y, y, v[1].x);
-                    node[2 * UNIT] = h2 + fmaf(v[2].y, y, v[2].x);
-                    __syncwarp();  // (the next place may share nodes with this one, in another lane)
+                        for (int w = 0; w < AT_ONCE; ++w)
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) v[w][q] = fma2(v[w][q], yy[w], k[q][d]);
+#pragma unroll
+                    for (int w = 0; w < AT_ONCE; ++w) {
+                        float *node = hist + ((place[w] >> 24) + 3 * quarter) * UNIT + mine;
+                        const float h0 = node[0], h1 = node[UNIT], h2 = node[2 * UNIT];
+                        node[0] = h0 + fmaf(v[w][0].y, y[w], v[w][0].x);
+                        node[UNIT] = h1 + fmaf(v[w][1].y, y[w], v[w][1].x);
+                        node[2 * UNIT] = h2 + fmaf(v[w][2].y, y[w], v[w][2].x);
+                        __syncwarp();  // (the next place may share nodes with this one, in another lane)
+                    }
                 }
             }
             count = 0;
@@ -365,21 +387,18 @@ __global__ void __launch_bounds__(32 * BUILD_WARPS, 6) pair_grid_kernel(const Bu
             const float line2 = fmaf(bz, bz, fmaf(by, by, bx * bx)) - bt * bt * inv_t3sq;
             const bool in = n1 <= R1 && line2 * 0.9999f - 1e-6f < d2_end;
             if (__any_sync(FULL, in)) {
-                auto image = [&](float f3) {
+                auto image = [&](int n3) {
+                    const float f3 = (float)n3;
                     const float dx = fmaf(cell.t3x, f3, bx), dy = fmaf(cell.t3y, f3, by), dz = fmaf(cell.t3z, f3, bz);
                     const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
                     list[count * 32 + lane] = __float_as_uint(d2);  // (stays where it counts)
-                    count += in && d2 < d2_end ? 1 : 0;
+                    count += in && n3 <= R3 && d2 < d2_end ? 1 : 0;
                 };
-                if (R3 == 2) {
+                // (five images between two looks at the lists: the usual box's column)
+                for (int n3 = -R3; n3 <= R3; n3 += ROOM) {
                     if (__any_sync(FULL, count >= LIST - ROOM)) spread();
 #pragma unroll
-                    for (int w = -2; w <= 2; ++w) image((float)w);
-                } else {
-                    for (int n3 = -R3; n3 <= R3; ++n3) {
-                        if (__any_sync(FULL, count >= LIST - ROOM)) spread();
-                        image((float)n3);
-                    }
+                    for (int w = 0; w < ROOM; ++w) image(n3 + w);
                 }
             }
             n2 += 4;
@@ -485,10 +504,11 @@ int launch_pair_grid_build(const PairAttn &b, const float *pos_ij, const float *
     a.grid = b.grid;
     auto kernel = b.K > 0 ? pair_grid_kernel<PG_TILES_BASIS> : pair_grid_kernel<PG_TILES_PLAIN>;
     const size_t smem = build_smem(b.par.tiles);
+    static_assert(LIST % AT_ONCE == 0, "places at once");
     static_assert(build_smem(PG_TILES_BASIS) <= 48 * 1024, "no more shared memory than any kernel has");
     // (a crystal has at least one unit; those of the extra variants are not known here: the loop takes them)
     const long long units = ((b.E + b.N) / 2 + PG_UNIT - 1) / PG_UNIT + b.B, blocks = (units + BUILD_WARPS - 1) / BUILD_WARPS;
-    const long long cap = (long long)sm_count() * 6;
+    const long long cap = (long long)sm_count() * BUILD_BLOCKS;
     kernel<<<(unsigned)(blocks < cap ? blocks : cap), 32 * BUILD_WARPS, smem, s>>>(a);
     return launch_status("pair_grid_kernel");
 }

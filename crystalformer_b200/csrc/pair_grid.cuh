@@ -55,7 +55,7 @@ struct PairGrid {
     int *unit_start;             // (B + 1): build units (PG_UNIT pairs of one variant) before a crystal
     int4 *tiles;                 // row tiles of the attention kernels: { crystal, first row, atoms (negative: no vectors), first
                                  // atom }, { first vector, first extra vector, smallest box, variants per axis }
-    unsigned *counters;          // { tiles, -, -, - }, then per call { rows left over, ticket of their launch, -, - }
+    unsigned *counters;          // { tiles, units given out, -, - }, then per call { rows left over, ticket of their launch, -, - }
     int *leftover;               // rows left over by a call
     uint4 *basis;                // fragments, bins as rows
     uint4 *basis_nodes;          // fragments, nodes as rows
