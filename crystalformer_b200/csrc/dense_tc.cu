@@ -16,16 +16,17 @@ namespace {
 using namespace tc5;
 
 // The rows of attention outputs, element features or species of a tile as operand 0 (scales: row floats 0).
+template <class P>
 __device__ __forceinline__ void load_first_operand(const DenseForward &p, const Shared &s, long long row_base)
 {
     unsigned char *A0 = s.mem + OFF_A0;
     if (p.tail != nullptr) {
-        load_operand(s, A0, [&](int row, int ln) {
+        load_operand<P>(s, A0, [&](int row, int ln) {
             return row_base + row < p.N ? *reinterpret_cast<const float4 *>(p.attn + (row_base + row) * 128 + 4 * ln)
                                         : make_float4(0.f, 0.f, 0.f, 0.f);
         });
     } else {
-        load_operand(s, A0, [&](int row, int ln) {
+        load_operand<P>(s, A0, [&](int row, int ln) {
             float e[4] = {0.f, 0.f, 0.f, 0.f};
             if (row_base + row < p.N) {
                 if (p.features != nullptr) {
@@ -67,33 +68,34 @@ struct WeightScales {
 };
 
 // The thread's 32 features ahead of the feed-forward: x + attn Wo^T + bo, the embedding, or x as it is.
-__device__ __forceinline__ void first_rows(const DenseForward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, long long row_base,
+template <class P>
+__device__ __forceinline__ void first_rows(const DenseForward &p, const Shared &s, const P &pl, Phase &ph, uint32_t tmem, long long row_base,
                                            float w_i, float (&x)[2][16])
 {
     const bool tail = p.tail != nullptr;
     if (!tail && p.embed == nullptr) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+        for (int half = 0; half < P::HALVES; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
         return;
     }
-    load_first_operand(p, s, row_base);
+    load_first_operand<P>(p, s, row_base);
     fence_async_smem();
     fence_before();
     mbar_arrive(s.bar(B_A0));
     float2 bias[4];
     if (tail) {  // the residual and the bias arrive during the product
 #pragma unroll
-        for (int half = 0; half < 2; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
+        for (int half = 0; half < P::HALVES; ++half) load_rows(p.x_in, 128, row_base, p.N, pl, half, x[half]);
         load_columns(p.bo, pl, bias);
     }
     epilogue_sync();  // (the loading warps' scales)
     float xi[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
+    for (int i = 0; i < 2 * P::HALVES; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
     ph.wait(s, B_D0);
     fence_after();
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < P::HALVES; ++half) {
         float d[16];
         tmem_load_16x32(pl.tmem(tmem, D0, half), d);
 #pragma unroll
@@ -115,7 +117,8 @@ __device__ __forceinline__ void hidden_scales(const WeightScales &ws, const floa
 
 // Chunk c of the hidden units from its accumulator, as the operand at `a_off` (wait_free: once the previous chunk's has
 // been multiplied).
-__device__ __forceinline__ void hidden_units(const DenseForward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, int d_col,
+template <class P>
+__device__ __forceinline__ void hidden_units(const DenseForward &p, const Shared &s, const P &pl, Phase &ph, uint32_t tmem, int d_col,
                                              int done, int c, long long row_base, const float (&xi)[4], float w1_i, const float (&hs)[4],
                                              int a_off, int ready, bool wait_free)
 {
@@ -124,7 +127,7 @@ __device__ __forceinline__ void hidden_units(const DenseForward &p, const Shared
     ph.wait(s, done);
     fence_after();
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < P::HALVES; ++half) {
         float h[16];
         tmem_load_16x32(pl.tmem(tmem, d_col, half), h);
         const float sa = xi[2 * half] * w1_i, sb = xi[2 * half + 1] * w1_i;
@@ -146,7 +149,8 @@ __device__ __forceinline__ void hidden_units(const DenseForward &p, const Shared
 }
 
 // One of q, k, v (which = 0, 1, 2) from its accumulator, and the Gaussian widths beside q.
-__device__ __forceinline__ void head_out(const DenseForward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, int d_col,
+template <class P>
+__device__ __forceinline__ void head_out(const DenseForward &p, const Shared &s, const P &pl, Phase &ph, uint32_t tmem, int d_col,
                                          int done, int which, long long row_base, const float (&xi)[4], float wh_i)
 {
     float2 bias[4], w[4];
@@ -157,7 +161,7 @@ __device__ __forceinline__ void head_out(const DenseForward &p, const Shared &s,
     float *dst = which == 0 ? p.q : which == 1 ? p.k : p.v;
     float al[2][4];  // q . w_pos of the thread's columns: (half, 2 head + row)
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < P::HALVES; ++half) {
         float d[16];
         tmem_load_16x32(pl.tmem(tmem, d_col, half), d);
         const float sa = xi[2 * half] * wh_i, sb = xi[2 * half + 1] * wh_i;
@@ -187,26 +191,27 @@ __device__ __forceinline__ void head_out(const DenseForward &p, const Shared &s,
         const float slope = p.gauss_scale * (p.elu_beta / (1.0f - lb));
         const int e = pl.t & 1, hh = pl.t >> 1;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int half = 0; half < P::HALVES; ++half) {
             const float *v = al[half];
             const float k0 = (e ? v[1] : v[0]) + __shfl_xor_sync(FULL, e ? v[0] : v[1], 1);
             const float k1 = (e ? v[3] : v[2]) + __shfl_xor_sync(FULL, e ? v[2] : v[3], 1);
             const float alpha = (hh ? k1 : k0) + __shfl_xor_sync(FULL, hh ? k0 : k1, 2);
             const float tt = (alpha + p.gauss_shift) * slope;
             const float elu = tt > 0.f ? tt : expm1f(tt), f = (1.0f - lb) * elu + 1.0f;
-            const long long row = row_base + pl.row0 + 16 * half + 8 * e;
+            const long long row = row_base + pl.tile0 + 16 * half + 8 * e;
             if (row < p.N) p.a[row * HEADS + 2 * pl.group + hh] = p.inverse ? factor / f : f * factor;
         }
     }
 }
 
+template <int HALVES>
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const DenseForward p)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
     uint32_t tmem;
     const Shared s = block_begin(smem_tc, tmem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long tiles = (p.N + 127) / 128;
+    const long long tiles = (p.N + 64 * HALVES - 1) / (64 * HALVES);
     const int chunks = p.ff / 128;
     const bool tail = p.tail != nullptr, embed = p.embed != nullptr, head = p.head != nullptr;
     grid_launch_dependents();
@@ -261,22 +266,22 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             if (!is.ok) is.drain(s);
         }
     } else {
-        const Place pl;
+        const PlaceOf<HALVES> pl;
         const WeightScales ws(p, s);
         grid_dependency_wait();
         Phase ph;
         for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            const long long row_base = tile * 128;
+            const long long row_base = tile * (64 * HALVES);
             epilogue_sync();  // the previous tile's readers are done with the per-row scales
             float x[2][16];   // the thread's 32 features: x, then y, then x'
-            float xi[4];      // 1 / scale of its four rows in the current operand
+            float xi[4] = {1.f, 1.f, 1.f, 1.f};  // 1 / scale of its four rows in the current operand
             first_rows(p, s, pl, ph, tmem, row_base, ws.first, x);
             if (tail) {
                 publish_rows(s, pl, x, xi);  // y
                 // (y lies in memory while the registers take the sum of the chunks, whose hidden units share their scales)
                 float *y_rows = p.y_save != nullptr ? p.y_save : p.x_out;
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
+                for (int half = 0; half < HALVES; ++half) {
                     store_rows(y_rows, 128, row_base, p.N, pl, half, x[half]);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) x[half][i] = 0.f;
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                 ph.wait(s, B_A1_FREE);
                 add_accumulator(pl, tmem, (chunks & 1) ? DX : DY, x);
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
+                for (int half = 0; half < HALVES; ++half) {
                     float y[16];
                     load_rows(y_rows, 128, row_base, p.N, pl, half, y);
                     const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
@@ -309,7 +314,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             if (head) publish_rows(s, pl, x, xi);
             if (tail || embed) {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < HALVES; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!head) continue;
 #pragma unroll
@@ -542,13 +547,16 @@ int launch_dense_forward(const DenseForward &args, cudaStream_t s)
     if (p.ff <= 0 || p.ff % 128 != 0 || p.ff > TC_MAX_FF)
         return fail(CF_ERR_UNSUPPORTED, "dense forward: ff_dim=%d must be a multiple of 128 up to %d", p.ff, TC_MAX_FF);
     static thread_local DenseLaunch launch;
-    int rc = launch.configure(reinterpret_cast<const void *>(dense_forward_kernel), reinterpret_cast<const void *>(dense_forward_split_kernel), "dense forward");
+    int rc = launch.configure(reinterpret_cast<const void *>(dense_forward_kernel<2>), reinterpret_cast<const void *>(dense_forward_kernel<1>),
+                              reinterpret_cast<const void *>(dense_forward_split_kernel), "dense forward");
     if (rc != CF_OK) return rc;
     const long long tiles = (p.N + 127) / 128, cap = sm_count();
     if (split_tiles(tiles, p.ff, launch.clusters()))
         launch_chained_cluster(dense_forward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, p.chained, p);
+    else if (half_tiles(p.N))
+        launch_chained(dense_forward_kernel<1>, dim3((unsigned)((p.N + 63) / 64)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s, p.chained, p);
     else
-        launch_chained(dense_forward_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
+        launch_chained(dense_forward_kernel<2>, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
                        p.chained, p);
     return launch_status("dense_forward_kernel");
 }

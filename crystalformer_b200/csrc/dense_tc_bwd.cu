@@ -40,13 +40,14 @@ __device__ __forceinline__ float4 query_grad(const DenseBackward &p, const float
 
 // Chunk c of the hidden units' gradients, gh = (gx W2) [h > 0], as the operand at `a_off` (wait_free: once the previous
 // chunk's has been multiplied).
-__device__ __forceinline__ void hidden_grads(const DenseBackward &p, const Shared &s, const Place &pl, Phase &ph, uint32_t tmem, int d_col,
+template <class P>
+__device__ __forceinline__ void hidden_grads(const DenseBackward &p, const Shared &s, const P &pl, Phase &ph, uint32_t tmem, int d_col,
                                              int done, int c, long long row_base, const float (&xi)[4], float w2_i, const float (&hs)[4],
                                              int a_off, int ready, bool wait_free)
 {
     unsigned live = 0u;  // bit 16 half + i: the unit was active
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < P::HALVES; ++half) {
         float h[16];
         load_rows(p.h + 128 * c, p.ff, row_base, p.N, pl, half, h);
 #pragma unroll
@@ -55,7 +56,7 @@ __device__ __forceinline__ void hidden_grads(const DenseBackward &p, const Share
     ph.wait(s, done);
     fence_after();
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < P::HALVES; ++half) {
         float g[16];
         tmem_load_16x32(pl.tmem(tmem, d_col, half), g);
 #pragma unroll
@@ -69,13 +70,14 @@ __device__ __forceinline__ void hidden_grads(const DenseBackward &p, const Share
     mbar_arrive(s.bar(ready));
 }
 
+template <int HALVES>
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const DenseBackward p)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
     uint32_t tmem;
     const Shared s = block_begin(smem_tc, tmem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long tiles = (p.N + 127) / 128;
+    const long long tiles = (p.N + 64 * HALVES - 1) / (64 * HALVES);
     const int chunks = p.ff / 128;
     const bool head = p.head != nullptr, tail = p.tail != nullptr;
 
@@ -124,7 +126,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             if (!is.ok) is.drain(s);
         }
     } else {
-        const Place pl;
+        using P = PlaceOf<HALVES>;
+        const P pl;
         unsigned char *A0 = s.mem + OFF_A0, *A1 = s.mem + OFF_A1;
         const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] * GIVEN_BACK : 0.f;
         float w2_i = 0.f, w1_i = 0.f, wo_i = 0.f;
@@ -134,13 +137,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
         }
         Phase ph;
         for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            const long long row_base = tile * 128;
+            const long long row_base = tile * (64 * HALVES);
             epilogue_sync();  // the previous tile's readers are done with the per-row scales
             float x[2][16];   // the thread's 32 gradients: gx, then gy
-            float xi[4];
+            float xi[4] = {1.f, 1.f, 1.f, 1.f};
             if (head) {
                 // ---- gq' and gk as operands 0 and 1, with one scale per row for the three of them (their products meet in
-                //      one sum); warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (head l / 4)
+                //      one sum); warp w takes EACH rows, lane l the columns 4 l .. 4 l + 3 (head l / 4)
+                constexpr int EACH = 4 * HALVES;
                 const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
                 float *inv_out = s.row_floats(0);
                 const uint32_t lane_at = (lane >> 4) * 16384 + (lane & 1) * 8;
@@ -153,12 +157,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                     *reinterpret_cast<uint2 *>(c + 32768) = h1;
                 };
 #pragma unroll
-                for (int r0 = 0; r0 < 8; r0 += 4) {
+                for (int r0 = 0; r0 < EACH; r0 += 4) {
                     float4 gq[4], gk[4];
                     float m[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const long long row = row_base + 8 * warp + r0 + u;
+                        const long long row = row_base + EACH * warp + r0 + u;
                         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                         float4 qv = zero, gvv = zero;
                         gq[u] = gk[u] = zero;
@@ -182,7 +186,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                         for (int u = 0; u < 4; ++u) m[u] = fmaxf(m[u], __shfl_xor_sync(FULL, m[u], o));
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const int row = 8 * warp + r0 + u;
+                        const int row = P::accumulator_row(EACH * warp + r0 + u);
                         float inv;
                         const float sc = power_of_two(m[u], inv);
                         if (lane == 0) inv_out[row] = inv;
@@ -194,16 +198,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 fence_before();
                 mbar_arrive(s.bar(B_A0));
 #pragma unroll
-                for (int half = 0; half < 2; ++half) load_rows(p.g_res, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < HALVES; ++half) load_rows(p.g_res, 128, row_base, p.N, pl, half, x[half]);
                 epilogue_sync();
 #pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = inv_out[pl.row0 + 8 * i];
+                for (int i = 0; i < 2 * HALVES; ++i) xi[i] = inv_out[pl.row0 + 8 * i];
                 ph.wait(s, B_D0);  // gq' has been multiplied
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int row = 8 * warp + u;
+                for (int u = 0; u < EACH; ++u) {
+                    const int of_tile = EACH * warp + u, row = P::accumulator_row(of_tile);
                     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (row_base + row < p.N) v = *reinterpret_cast<const float4 *>(p.gv + (row_base + row) * 128 + 4 * lane);
+                    if (row_base + of_tile < p.N) v = *reinterpret_cast<const float4 *>(p.gv + (row_base + of_tile) * 128 + 4 * lane);
                     put(A0, row, v, 1.0f / inv_out[row]);  // (powers of two: exact)
                 }
                 fence_async_smem();
@@ -212,7 +216,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 ph.wait(s, B_D0);
                 fence_after();
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
+                for (int half = 0; half < HALVES; ++half) {
                     float d[16], e[16];
                     tmem_load_16x32(pl.tmem(tmem, D0, half), d);
                     tmem_load_16x32(pl.tmem(tmem, D1, half), e);
@@ -225,12 +229,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 }
             } else {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < HALVES; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!tail) continue;
             publish_rows(s, pl, x, xi);  // gx (read again from memory behind the chunks, whose sum takes its registers)
 #pragma unroll
-            for (int half = 0; half < 2; ++half)
+            for (int half = 0; half < HALVES; ++half)
 #pragma unroll
                 for (int i = 0; i < 16; ++i) x[half][i] = 0.f;
             // ---- hidden units: one scale per row for all chunks, |gh| <= 128 max|gx| max|W2| (see the forward)
@@ -244,7 +248,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             ph.wait(s, B_A1_FREE);
             add_accumulator(pl, tmem, (chunks & 1) ? DX : DY, x);
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
+            for (int half = 0; half < HALVES; ++half) {
                 float g[16];
                 load_rows(p.gx, 128, row_base, p.N, pl, half, g);
 #pragma unroll
@@ -252,11 +256,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             }
             publish_rows(s, pl, x, xi);  // gy
 #pragma unroll
-            for (int half = 0; half < 2; ++half) store_rows(p.gy, 128, row_base, p.N, pl, half, x[half]);
+            for (int half = 0; half < HALVES; ++half) store_rows(p.gy, 128, row_base, p.N, pl, half, x[half]);
             ph.wait(s, B_D0);
             fence_after();
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
+            for (int half = 0; half < HALVES; ++half) {
                 float d[16];
                 tmem_load_16x32(pl.tmem(tmem, D0, half), d);
 #pragma unroll
@@ -696,13 +700,16 @@ int launch_dense_backward(const DenseBackward &args, cudaStream_t s)
     DenseBackward p = args;
     p.status = wait_status();
     static thread_local DenseLaunch launch;
-    int rc = launch.configure(reinterpret_cast<const void *>(dense_backward_kernel), reinterpret_cast<const void *>(dense_backward_split_kernel), "dense backward");
+    int rc = launch.configure(reinterpret_cast<const void *>(dense_backward_kernel<2>), reinterpret_cast<const void *>(dense_backward_kernel<1>),
+                              reinterpret_cast<const void *>(dense_backward_split_kernel), "dense backward");
     if (rc != CF_OK) return rc;
     const long long tiles = (p.N + 127) / 128, cap = sm_count();
     if (split_tiles(tiles, p.ff, launch.clusters()))
         launch_chained_cluster(dense_backward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, false, p);
+    else if (half_tiles(p.N))
+        dense_backward_kernel<1><<<(unsigned)((p.N + 63) / 64), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
     else
-        dense_backward_kernel<<<(unsigned)(tiles < cap ? tiles : cap), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
+        dense_backward_kernel<2><<<(unsigned)(tiles < cap ? tiles : cap), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
     return launch_status("dense_backward_kernel");
 }
 

@@ -1,7 +1,7 @@
 // What the forward and backward dense kernels share (dense_tc.cu, dense_tc_bwd.cu): block roles, the weight stream, one
 // 128 x 128 x 128 product, and the conversion of accumulator fragments into operands.
 //
-// A thread block carries a tile of 128 atom rows through its chain of products.  Warps 0-15 are the epilogue warps
+// A thread block carries a tile of 128 atom rows (or 64: half_tiles below) through its chain of products.  Warps 0-15 are the epilogue warps
 // (thread = 4 rows x 8 columns of a 128 x 128 accumulator, in the layout of tmem_load_16x32: warp w covers rows
 // 32 (w % 4) .., columns 32 (w / 4) ..; with eight warps an epilogue took 2 us instead of 1), one thread of warp 16
 // issues the tensor instructions, one thread of warp 17 streams the weight images through a ring of three 32 KB stages.
@@ -132,15 +132,23 @@ struct Issuer {
 // ---- epilogue threads ---------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
-// this thread's place in a 128 x 128 accumulator: row(half, e) = row0 + 16 half + 8 e, columns col0 + 8 j + {0, 1}, j < 4
-struct Place {
+// this thread's place in a 128 x 128 accumulator: row(half, e) = row0 + 16 half + 8 e, columns col0 + 8 j + {0, 1}, j < 4.
+// HALVES = 1: a tile of 64 rows, sixteen in each quarter of the accumulator (the rest is multiplied and never looked at: the tensor
+// pipe is not what a tile waits for, and every epilogue is half as long).
+template <int HALVES_>
+struct PlaceOf {
+    static constexpr int HALVES = HALVES_, ROWS = 64 * HALVES;
     int row0, col0, g, t, group;  // group: column group of 32
+    int tile0;                    // row0 in the tile
+    // the accumulator's row of a tile's row
+    static __device__ __forceinline__ int accumulator_row(int row) { return HALVES == 2 ? row : (row >> 4) * 32 + (row & 15); }
     uint32_t tmem_off;            // lane and column offset of this warp's part (half 0)
-    __device__ __forceinline__ Place()
+    __device__ __forceinline__ PlaceOf()
     {
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         g = lane >> 2; t = lane & 3; group = w >> 2;
         row0 = 32 * (w & 3) + g;
+        tile0 = 16 * HALVES * (w & 3) + g;
         col0 = 32 * group + 2 * t;
         tmem_off = ((uint32_t)(32 * (w & 3)) << 16) + 32u * (uint32_t)group;
     }
@@ -149,9 +157,11 @@ struct Place {
         return base + tmem_off + ((uint32_t)(16 * half) << 16) + (uint32_t)d_col;
     }
 };
+using Place = PlaceOf<2>;
 
 // 16 values of `half` (rows scaled by s0 / s1) into an operand buffer
-__device__ __forceinline__ void store_operand(unsigned char *buf, const Place &pl, int half, const float (&v)[16], float s0, float s1)
+template <class P>
+__device__ __forceinline__ void store_operand(unsigned char *buf, const P &pl, int half, const float (&v)[16], float s0, float s1)
 {
     unsigned char *at = buf + (pl.group >> 1) * 16384 + (pl.row0 + 16 * half) * 128 + pl.t * 4;
     const int chunk0 = 4 * (pl.group & 1);
@@ -169,11 +179,12 @@ __device__ __forceinline__ void store_operand(unsigned char *buf, const Place &p
 }
 
 // sum += this thread's part of an accumulator whose product is known to be complete
-__device__ __forceinline__ void add_accumulator(const Place &pl, uint32_t tmem, int d_col, float (&sum)[2][16])
+template <class P>
+__device__ __forceinline__ void add_accumulator(const P &pl, uint32_t tmem, int d_col, float (&sum)[2][16])
 {
     fence_after();
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
+    for (int half = 0; half < P::HALVES; ++half) {
         float d[16];
         tmem_load_16x32(pl.tmem(tmem, d_col, half), d);
 #pragma unroll
@@ -184,55 +195,59 @@ __device__ __forceinline__ void add_accumulator(const Place &pl, uint32_t tmem, 
 // largest magnitude of each of the thread's four rows over all 128 columns (the four column groups of the block);
 // m[2 half + e].  Two barriers of the epilogue threads: the second one keeps a later call from overwriting maxima
 // still being read.
-__device__ __forceinline__ void row_maxima(const Shared &s, const Place &pl, float (&m)[4])
+template <class P>
+__device__ __forceinline__ void row_maxima(const Shared &s, const P &pl, float (&m)[4])
 {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2 * P::HALVES; ++i) {
         m[i] = fmaxf(m[i], __shfl_xor_sync(FULL, m[i], 1));
         m[i] = fmaxf(m[i], __shfl_xor_sync(FULL, m[i], 2));
     }
     if (pl.t == 0) {
         float *mine = s.row_floats(1 + pl.group);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mine[pl.row0 + 8 * i] = m[i];
+        for (int i = 0; i < 2 * P::HALVES; ++i) mine[pl.row0 + 8 * i] = m[i];
     }
     epilogue_sync();
     const float *all = s.row_floats(1) + pl.row0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2 * P::HALVES; ++i)
         m[i] = fmaxf(fmaxf(all[8 * i], all[128 + 8 * i]), fmaxf(all[256 + 8 * i], all[384 + 8 * i]));
     epilogue_sync();
 }
 
 // The block's rows as operand 0: scales from the largest magnitude of every row (xi: 1 / scale of the thread's rows).
-__device__ __forceinline__ void publish_rows(const Shared &s, const Place &pl, const float (&x)[2][16], float (&xi)[4])
+template <class P>
+__device__ __forceinline__ void publish_rows(const Shared &s, const P &pl, const float (&x)[2][16], float (&xi)[4])
 {
     float m[4] = {0.f, 0.f, 0.f, 0.f}, xs[4];
 #pragma unroll
-    for (int half = 0; half < 2; ++half)
+    for (int half = 0; half < P::HALVES; ++half)
 #pragma unroll
         for (int i = 0; i < 16; ++i) m[2 * half + ((i >> 1) & 1)] = fmaxf(m[2 * half + ((i >> 1) & 1)], fabsf(x[half][i]));
     row_maxima(s, pl, m);
 #pragma unroll
     for (int i = 0; i < 4; ++i) xs[i] = power_of_two(m[i], xi[i]);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) store_operand(s.mem + OFF_A0, pl, half, x[half], xs[2 * half], xs[2 * half + 1]);
+    for (int half = 0; half < P::HALVES; ++half) store_operand(s.mem + OFF_A0, pl, half, x[half], xs[2 * half], xs[2 * half + 1]);
     fence_async_smem();
     fence_before();
     mbar_arrive(s.bar(B_A0));
 }
 
 // this thread's eight values of a per-column constant (read before the wait for the product that needs them)
-__device__ __forceinline__ void load_columns(const float *src, const Place &pl, float2 (&b)[4])
+template <class P>
+__device__ __forceinline__ void load_columns(const float *src, const P &pl, float2 (&b)[4])
 {
 #pragma unroll
     for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float2 *>(src + pl.col0 + 8 * j);
 }
 
 // two columns of a row-major (N, ld) array at this thread's fragment positions of `half`, zero beyond row N
-__device__ __forceinline__ void load_rows(const float *src, int ld, long long row_base, long long N, const Place &pl, int half, float (&v)[16])
+template <class P>
+__device__ __forceinline__ void load_rows(const float *src, int ld, long long row_base, long long N, const P &pl, int half, float (&v)[16])
 {
-    const long long r0 = row_base + pl.row0 + 16 * half, r1 = r0 + 8;
+    const long long r0 = row_base + pl.tile0 + 16 * half, r1 = r0 + 8;
     const float *p0 = src + r0 * ld + pl.col0, *p1 = src + r1 * ld + pl.col0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -241,9 +256,10 @@ __device__ __forceinline__ void load_rows(const float *src, int ld, long long ro
         v[4 * j] = a.x; v[4 * j + 1] = a.y; v[4 * j + 2] = b.x; v[4 * j + 3] = b.y;
     }
 }
-__device__ __forceinline__ void store_rows(float *dst, int ld, long long row_base, long long N, const Place &pl, int half, const float (&v)[16])
+template <class P>
+__device__ __forceinline__ void store_rows(float *dst, int ld, long long row_base, long long N, const P &pl, int half, const float (&v)[16])
 {
-    const long long r0 = row_base + pl.row0 + 16 * half, r1 = r0 + 8;
+    const long long r0 = row_base + pl.tile0 + 16 * half, r1 = r0 + 8;
     float *p0 = dst + r0 * ld + pl.col0, *p1 = dst + r1 * ld + pl.col0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -252,23 +268,24 @@ __device__ __forceinline__ void store_rows(float *dst, int ld, long long row_bas
     }
 }
 
-// Loads a tile of rows as an operand: warp w takes rows 8 w .. 8 w + 7, lane l the columns 4 l .. 4 l + 3 (fetch(row,
+// Loads a tile of rows as an operand: warp w takes eight (four) rows from 8 w (4 w) on, lane l the columns 4 l .. 4 l + 3 (fetch(row,
 // lane) returns them); the row's scale comes from its own largest magnitude, 1 / scale goes to row_floats(0).
-template <class Fetch>
+template <class P = Place, class Fetch>
 __device__ __forceinline__ void load_operand(const Shared &s, unsigned char *buf, Fetch &&fetch)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float *inv_out = s.row_floats(0);
-    float4 v[8];
-    float m[8];
+    constexpr int EACH = 4 * P::HALVES;
+    float4 v[EACH];
+    float m[8] = {};
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = fetch(8 * w + u, lane);
+    for (int u = 0; u < EACH; ++u) v[u] = fetch(EACH * w + u, lane);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) m[u] = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
+    for (int u = 0; u < EACH; ++u) m[u] = fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w)));
     const float row_max = warp_max_of_8(m, lane);  // of row lane / 4
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int row = 8 * w + u;
+    for (int u = 0; u < EACH; ++u) {
+        const int row = P::accumulator_row(EACH * w + u);
         float inv;
         const float sc = power_of_two(__shfl_sync(FULL, row_max, 4 * u), inv);
         if (lane == 0) inv_out[row] = inv;
@@ -464,16 +481,23 @@ inline bool split_tiles(long long tiles, int ff, int clusters)
     return ff <= 128 * SPLIT && tiles <= clusters && dense_tile_rows_choice() != 32;
 }
 
-struct DenseLaunch {  // per thread: what a device's set-up of the two kernels gave
+// Otherwise tiles of 64 rows while there is an SM for each (and SM time is not what counts): every epilogue of the chain is half as
+// long, and the products, which are not what it waits for, take as long as before.  Median of a network's boundaries with tiles
+// of 128 and of 64: 4,881 rows 31 and 24 us (inference), 39 and 30 (training, forward), 48 and 33 (backward); 9,301 rows 32 and 32, 49
+// and 34, 52 and 35.  Beyond 64 rows per SM a second tile would follow: 35 us twice against 50.
+inline bool half_tiles(long long rows) { return (rows + 63) / 64 <= sm_count() && dense_tile_rows_choice() != 32; }
+
+struct DenseLaunch {  // per thread: what a device's set-up of the kernels gave
     int clusters_of[64] = {};  // clusters that fit at once; 0: not set up yet
     int device = 0;
-    int configure(const void *alone, const void *split, const char *what)
+    int configure(const void *alone, const void *half, const void *split, const char *what)
     {
         int dev = 0;
         cudaGetDevice(&dev);
         device = dev & 63;
         if (clusters_of[device] > 0) return CF_OK;
         if (cudaFuncSetAttribute(alone, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess ||
+            cudaFuncSetAttribute(half, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess ||
             cudaFuncSetAttribute(split, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) {
             cudaGetLastError();
             return fail(CF_ERR_CUDA, "%s: %d bytes of shared memory not available", what, SMEM_BYTES);

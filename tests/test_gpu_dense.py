@@ -81,6 +81,27 @@ def test_boundaries_shared_by_a_cluster_or_not(ff, atoms):
         assert (grads[True][n] - g).norm() <= 2e-3 * g.norm() + noise, n
 
 
+@pytest.mark.parametrize("ff", [128, 512, 640])
+def test_tiles_of_64_and_of_128_rows(ff):
+    """A tile of 64 rows on every SM, and one row more (tiles of 128): the same bits for the rows that both have, and for a batch whose
+    last tile has one row or 63."""
+    from crystalformer_b200.model import Latticeformer, default_params
+    torch.manual_seed(ff)
+    model = Latticeformer(default_params(num_layers=2, ff_dim=ff)).cuda()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    cb = make_crystals(6, 64 * sms + 1, lambda rng, b: np.ones(b, dtype=np.int64), length_range=(8.0, 14.0))
+    t = lambda x: torch.as_tensor(x).cuda()
+    batch = lambda n: types.SimpleNamespace(x=t(cb.x)[:n], pos=t(cb.pos)[:n], trans_vec=t(cb.trans_vec)[:n], sizes=t(cb.sizes)[:n])
+    model.train()
+    with torch.no_grad():
+        model(batch(64 * sms))
+    model.eval()
+    with torch.no_grad():
+        whole = model(batch(64 * sms + 1))
+        for n in (64 * sms, 64 * sms - 1, 64 * sms - 63):
+            assert torch.equal(model(batch(n)), whole[:n]), n
+
+
 @pytest.mark.parametrize("ff", [128, 384, 512])
 @pytest.mark.parametrize("atoms", [1, 33, 200, 2000])
 def test_outputs_do_not_depend_on_how_a_batch_is_issued(ff, atoms):
