@@ -166,22 +166,6 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-template <typename... KArgs, typename... Args>
-inline cudaError_t launch_chained_cluster(void (*kernel)(KArgs...), unsigned blocks, unsigned cluster, unsigned threads, size_t smem,
-                                          cudaStream_t stream, bool chained, Args &&...args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (chained && chained_launches_enabled()) ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 // Whether a batch's rows are ordered by their cost (batch_prep.cu: a sort of its crystals in one block): the preparation writes
 // the order, and whoever reads it later, only then.
 constexpr int ORDER_MAX_CRYSTALS = 2048;

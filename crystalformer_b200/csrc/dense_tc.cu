@@ -91,7 +91,7 @@ __device__ __forceinline__ void first_rows(const DenseForward &p, const Shared &
     epilogue_sync();  // (the loading warps' scales)
     float xi[4];
 #pragma unroll
-    for (int i = 0; i < 2 * P::HALVES; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
+    for (int i = 0; i < P::HALVES * P::PAIRS; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
     ph.wait(s, B_D0);
     fence_after();
 #pragma unroll
@@ -199,27 +199,26 @@ __device__ __forceinline__ void head_out(const DenseForward &p, const Shared &s,
             const float tt = (alpha + p.gauss_shift) * slope;
             const float elu = tt > 0.f ? tt : expm1f(tt), f = (1.0f - lb) * elu + 1.0f;
             const long long row = row_base + pl.tile0 + 16 * half + 8 * e;
-            if (row < p.N) p.a[row * HEADS + 2 * pl.group + hh] = p.inverse ? factor / f : f * factor;
+            if (row < p.N && (P::PAIRS == 2 || e == 0)) p.a[row * HEADS + 2 * pl.group + hh] = p.inverse ? factor / f : f * factor;
         }
     }
 }
 
-template <int HALVES>
+template <int ROWS>
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const DenseForward p)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
     uint32_t tmem;
     const Shared s = block_begin(smem_tc, tmem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long tiles = (p.N + 64 * HALVES - 1) / (64 * HALVES);
+    const long long tiles = (p.N + ROWS - 1) / ROWS;
     const int chunks = p.ff / 128;
     const bool tail = p.tail != nullptr, embed = p.embed != nullptr, head = p.head != nullptr;
-    grid_launch_dependents();
 
     if (warp == STREAM_WARP) {
         if (p.weights_fresh) grid_dependency_wait();
         if (lane == 0) {
-            Producer<STAGES> pr;
+            Producer pr;
             for (long long tile = blockIdx.x; tile < tiles && pr.ok; tile += gridDim.x) {
                 if (tail) pr.stream(s, p.tail, 0, 1 + 2 * chunks);
                 else if (embed) pr.stream(s, p.embed, 0, 1, TC_EMBED_PIECES);
@@ -231,7 +230,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
     } else if (warp == ISSUE_WARP) {
         grid_dependency_wait();
         if (lane == 0) {
-            Issuer<STAGES> is;
+            Issuer is;
             Phase ph;
             for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
                 bool ok = true;
@@ -266,12 +265,16 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             if (!is.ok) is.drain(s);
         }
     } else {
-        const PlaceOf<HALVES> pl;
+        using P = PlaceOf<ROWS>;
+        const P pl;
         const WeightScales ws(p, s);
         grid_dependency_wait();
+        // (not before: the blocks that follow would be packed onto the few SMs that the kernel ahead has left; pooling and head of
+        // 128 crystals 30 us behind the last boundary instead of 9)
+        grid_launch_dependents();
         Phase ph;
         for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            const long long row_base = tile * (64 * HALVES);
+            const long long row_base = tile * ROWS;
             epilogue_sync();  // the previous tile's readers are done with the per-row scales
             float x[2][16];   // the thread's 32 features: x, then y, then x'
             float xi[4] = {1.f, 1.f, 1.f, 1.f};  // 1 / scale of its four rows in the current operand
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                 // (y lies in memory while the registers take the sum of the chunks, whose hidden units share their scales)
                 float *y_rows = p.y_save != nullptr ? p.y_save : p.x_out;
 #pragma unroll
-                for (int half = 0; half < HALVES; ++half) {
+                for (int half = 0; half < P::HALVES; ++half) {
                     store_rows(y_rows, 128, row_base, p.N, pl, half, x[half]);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) x[half][i] = 0.f;
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                 ph.wait(s, B_A1_FREE);
                 add_accumulator(pl, tmem, (chunks & 1) ? DX : DY, x);
 #pragma unroll
-                for (int half = 0; half < HALVES; ++half) {
+                for (int half = 0; half < P::HALVES; ++half) {
                     float y[16];
                     load_rows(y_rows, 128, row_base, p.N, pl, half, y);
                     const float sa = hi[2 * half] * ws.w2, sb = hi[2 * half + 1] * ws.w2;
@@ -314,7 +317,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
             if (head) publish_rows(s, pl, x, xi);
             if (tail || embed) {
 #pragma unroll
-                for (int half = 0; half < HALVES; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < P::HALVES; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!head) continue;
 #pragma unroll
@@ -323,155 +326,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_kernel(const D
                          row_base, xi, ws.head);
         }
     }
-    block_end(s, tmem, p.status);
-}
-
-// The same for a cluster of four blocks (dense_tc_core.cuh): block r takes hidden chunk r and, of q, k, v, matrix r.  Hidden
-// units go to operand buffer 0 (y has been multiplied by then), buffer 1 takes the shares of the output sum.  Every value
-// comes from the same operations in the same order as in a block per tile: the outputs are the same bits.
-// 2,027 rows, 512 hidden units, a boundary inside the network: 31 us with a block per tile, 20 here (unchained).
-__global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_forward_split_kernel(const DenseForward p)
-{
-    extern __shared__ __align__(1024) unsigned char smem_tc[];
-    uint32_t tmem;
-    const Shared s = block_begin(smem_tc, tmem);
-    const uint32_t rank = cluster_rank();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int chunks = p.ff / 128;
-    const long long row_base = (long long)(blockIdx.x / SPLIT) * 128;
-    const bool tail = p.tail != nullptr, embed = p.embed != nullptr, head = p.head != nullptr;
-    const bool has_chunk = tail && (int)rank < chunks, has_head = head && rank < 3;
-    grid_launch_dependents();
-    cluster_sync();  // every block's barriers are ready for the others' arrivals
-
-    if (warp == STREAM_WARP) {
-        if (p.weights_fresh) grid_dependency_wait();
-        if (lane == 0) {
-            Producer<SPLIT_STAGES> pr;
-            if (tail) pr.stream(s, p.tail, 0, 1);
-            else if (embed) pr.stream(s, p.embed, 0, 1, TC_EMBED_PIECES);
-            if (has_chunk && pr.ok) pr.stream(s, p.tail, 1 + first_of_chunk(rank), 1);
-            if (has_chunk && pr.ok) pr.stream(s, p.tail, 1 + second_of_chunk(rank, chunks), 1);
-            if (has_head && pr.ok) pr.stream(s, p.head, 1 + 2 * chunks + (int)rank, 1);
-            if (!pr.ok) pr.drain(s);
-        }
-        __syncwarp();
-        grid_dependency_wait();
-    } else if (warp == ISSUE_WARP) {
-        grid_dependency_wait();
-        if (lane == 0) {
-            Issuer<SPLIT_STAGES> is;
-            Phase ph;
-            bool ok = true;
-            auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
-            auto product = [&](int d, int done, int pieces = 2) {
-                if (ok) is.product(s, tmem, d, OFF_A0, pieces);
-                ok = ok && is.ok;
-                mma_commit(s.bar(done));
-            };
-            if (tail || embed) {
-                ready(B_A0);
-                product(D0, B_D0, tail ? 2 : TC_EMBED_PIECES);
-            }
-            if (tail) {
-                ready(B_A0);
-                if (has_chunk) {
-                    product(D0, B_D0);
-                    ready(B_A0);
-                    product(DX, B_DX);
-                }
-            }
-            if (has_head) {
-                if (tail) {
-                    ok = ph.wait_cluster(s, B_ROWS) && ok;
-                    fence_async_smem();
-                    fence_after();
-                } else {
-                    ready(B_A0);
-                }
-                product(D1, B_D1);
-            }
-            if (!ok) is.drain(s);
-        }
-        __syncwarp();
-    } else {
-        const Place pl;
-        const WeightScales ws(p, s);
-        grid_dependency_wait();
-        Phase ph;
-        if (threadIdx.x == 0 && tail) {
-            expect_shares(s);
-            if (has_head) expect_rows(s);
-        }
-        const bool mine = (warp & 3) == (int)rank;  // this warp's rows of an accumulator are finished by this block
-        float x[2][16], xi[4];
-        first_rows(p, s, pl, ph, tmem, row_base, ws.first, x);
-        if (tail) {
-            if (mine) {  // (read back by the threads that finish the rows, behind the barriers of publish_rows)
-#pragma unroll
-                for (int half = 0; half < 2; ++half) stage_rows(s.mem + OFF_OWN, pl, half, x[half]);
-            }
-            publish_rows(s, pl, x, xi);  // y
-            if (p.y_save != nullptr && mine) {
-#pragma unroll
-                for (int half = 0; half < 2; ++half) store_rows(p.y_save, 128, row_base, p.N, pl, half, x[half]);
-            }
-            float hs[4], hi[4];
-            hidden_scales(ws, xi, hs, hi);
-            if (has_chunk) hidden_units(p, s, pl, ph, tmem, D0, B_D0, rank, row_base, xi, ws.w1, hs, OFF_A0, B_A0, false);
-            if (mine && pl.group == 0 && pl.t == 0) {  // the scales of the finished rows, for the threads that finish them
-#pragma unroll
-                for (int i = 0; i < 4; ++i) s.row_floats(3)[pl.g + 8 * i] = hi[i] * ws.w2;
-            }
-            epilogue_sync();  // (and y is no longer being written to buffer 0, which is about to take the shares)
-            const float2 b2_lo = *reinterpret_cast<const float2 *>(p.b2 + 4 * lane), b2_hi = *reinterpret_cast<const float2 *>(p.b2 + 4 * lane + 2);
-            if (has_chunk) {
-                ph.wait(s, B_DX);
-                fence_after();
-            }
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {  // (the shares are the accumulators as they are: all chunks have one scale per row)
-                float d[16];
-                if (has_chunk) {
-                    tmem_load_16x32(pl.tmem(tmem, DX, half), d);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) d[i] = 0.f;
-                }
-                stage_share(s, pl, half, d);
-            }
-            send_share(s, rank);
-            float4 v[2];
-            collect_shares(s, ph, v);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const float4 y = staged_row(s.mem + OFF_OWN, 2 * warp + u, lane);
-                const float sc = s.row_floats(3)[2 * warp + u];
-                v[u].x = y.x + fmaf(v[u].x, sc, b2_lo.x); v[u].y = y.y + fmaf(v[u].y, sc, b2_lo.y);
-                v[u].z = y.z + fmaf(v[u].z, sc, b2_hi.x); v[u].w = y.w + fmaf(v[u].w, sc, b2_hi.y);
-            }
-            if (head) spread_rows(s, ph, rank, v, 3, 0);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const long long row = row_base + 32 * (int)rank + 2 * warp + u;
-                if (row < p.N) *reinterpret_cast<float4 *>(p.x_out + row * 128 + 4 * lane) = v[u];
-            }
-            if (has_head) {
-                ph.wait_cluster(s, B_ROWS);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
-            }
-        } else {
-            if (head) publish_rows(s, pl, x, xi);
-            if (embed && mine) {
-#pragma unroll
-                for (int half = 0; half < 2; ++half) store_rows(p.x_out, 128, row_base, p.N, pl, half, x[half]);
-            }
-        }
-        if (has_head) head_out(p, s, pl, ph, tmem, D1, B_D1, (int)rank, row_base, xi, ws.head);
-    }
-    __syncthreads();
-    cluster_sync();  // (no block ends while another may still write to it)
     block_end(s, tmem, p.status);
 }
 
@@ -547,17 +401,14 @@ int launch_dense_forward(const DenseForward &args, cudaStream_t s)
     if (p.ff <= 0 || p.ff % 128 != 0 || p.ff > TC_MAX_FF)
         return fail(CF_ERR_UNSUPPORTED, "dense forward: ff_dim=%d must be a multiple of 128 up to %d", p.ff, TC_MAX_FF);
     static thread_local DenseLaunch launch;
-    int rc = launch.configure(reinterpret_cast<const void *>(dense_forward_kernel<2>), reinterpret_cast<const void *>(dense_forward_kernel<1>),
-                              reinterpret_cast<const void *>(dense_forward_split_kernel), "dense forward");
+    const void *const kernels[3] = {reinterpret_cast<const void *>(dense_forward_kernel<128>), reinterpret_cast<const void *>(dense_forward_kernel<64>),
+                                    reinterpret_cast<const void *>(dense_forward_kernel<32>)};
+    int rc = launch.configure(kernels, "dense forward");
     if (rc != CF_OK) return rc;
-    const long long tiles = (p.N + 127) / 128, cap = sm_count();
-    if (split_tiles(tiles, p.ff, launch.clusters()))
-        launch_chained_cluster(dense_forward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, p.chained, p);
-    else if (half_tiles(p.N))
-        launch_chained(dense_forward_kernel<1>, dim3((unsigned)((p.N + 63) / 64)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s, p.chained, p);
-    else
-        launch_chained(dense_forward_kernel<2>, dim3((unsigned)(tiles < cap ? tiles : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s,
-                       p.chained, p);
+    const int rows = tile_rows(p.N);
+    const long long blocks = (p.N + rows - 1) / rows, cap = sm_count();
+    auto kernel = rows == 128 ? dense_forward_kernel<128> : rows == 64 ? dense_forward_kernel<64> : dense_forward_kernel<32>;
+    launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(tc5::BLOCK_THREADS), tc5::SMEM_BYTES, s, p.chained, p);
     return launch_status("dense_forward_kernel");
 }
 

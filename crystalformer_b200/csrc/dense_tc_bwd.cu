@@ -70,20 +70,20 @@ __device__ __forceinline__ void hidden_grads(const DenseBackward &p, const Share
     mbar_arrive(s.bar(ready));
 }
 
-template <int HALVES>
+template <int ROWS>
 __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const DenseBackward p)
 {
     extern __shared__ __align__(1024) unsigned char smem_tc[];
     uint32_t tmem;
     const Shared s = block_begin(smem_tc, tmem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long tiles = (p.N + 64 * HALVES - 1) / (64 * HALVES);
+    const long long tiles = (p.N + ROWS - 1) / ROWS;
     const int chunks = p.ff / 128;
     const bool head = p.head != nullptr, tail = p.tail != nullptr;
 
     if (warp == STREAM_WARP) {
         if (lane == 0) {
-            Producer<STAGES> pr;
+            Producer pr;
             for (long long tile = blockIdx.x; tile < tiles && pr.ok; tile += gridDim.x) {
                 if (head) pr.stream(s, p.head, 0, 3);
                 if (tail) pr.stream(s, p.tail, 3, 1 + 2 * chunks);
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
         }
     } else if (warp == ISSUE_WARP) {
         if (lane == 0) {
-            Issuer<STAGES> is;
+            Issuer is;
             Phase ph;
             for (long long tile = blockIdx.x; tile < tiles && is.ok; tile += gridDim.x) {
                 bool ok = true;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             if (!is.ok) is.drain(s);
         }
     } else {
-        using P = PlaceOf<HALVES>;
+        using P = PlaceOf<ROWS>;
         const P pl;
         unsigned char *A0 = s.mem + OFF_A0, *A1 = s.mem + OFF_A1;
         const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] * GIVEN_BACK : 0.f;
@@ -137,14 +137,14 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
         }
         Phase ph;
         for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            const long long row_base = tile * (64 * HALVES);
+            const long long row_base = tile * ROWS;
             epilogue_sync();  // the previous tile's readers are done with the per-row scales
             float x[2][16];   // the thread's 32 gradients: gx, then gy
             float xi[4] = {1.f, 1.f, 1.f, 1.f};
             if (head) {
                 // ---- gq' and gk as operands 0 and 1, with one scale per row for the three of them (their products meet in
                 //      one sum); warp w takes EACH rows, lane l the columns 4 l .. 4 l + 3 (head l / 4)
-                constexpr int EACH = 4 * HALVES;
+                constexpr int EACH = P::EACH, STEP = EACH < 4 ? EACH : 4;
                 const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
                 float *inv_out = s.row_floats(0);
                 const uint32_t lane_at = (lane >> 4) * 16384 + (lane & 1) * 8;
@@ -157,11 +157,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                     *reinterpret_cast<uint2 *>(c + 32768) = h1;
                 };
 #pragma unroll
-                for (int r0 = 0; r0 < EACH; r0 += 4) {
-                    float4 gq[4], gk[4];
-                    float m[4];
+                for (int r0 = 0; r0 < EACH; r0 += STEP) {
+                    float4 gq[STEP], gk[STEP];
+                    float m[STEP];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < STEP; ++u) {
                         const long long row = row_base + EACH * warp + r0 + u;
                         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
                         float4 qv = zero, gvv = zero;
@@ -183,9 +183,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) m[u] = fmaxf(m[u], __shfl_xor_sync(FULL, m[u], o));
+                        for (int u = 0; u < STEP; ++u) m[u] = fmaxf(m[u], __shfl_xor_sync(FULL, m[u], o));
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < STEP; ++u) {
                         const int row = P::accumulator_row(EACH * warp + r0 + u);
                         float inv;
                         const float sc = power_of_two(m[u], inv);
@@ -198,10 +198,10 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 fence_before();
                 mbar_arrive(s.bar(B_A0));
 #pragma unroll
-                for (int half = 0; half < HALVES; ++half) load_rows(p.g_res, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < P::HALVES; ++half) load_rows(p.g_res, 128, row_base, p.N, pl, half, x[half]);
                 epilogue_sync();
 #pragma unroll
-                for (int i = 0; i < 2 * HALVES; ++i) xi[i] = inv_out[pl.row0 + 8 * i];
+                for (int i = 0; i < P::HALVES * P::PAIRS; ++i) xi[i] = inv_out[pl.row0 + 8 * i];
                 ph.wait(s, B_D0);  // gq' has been multiplied
 #pragma unroll
                 for (int u = 0; u < EACH; ++u) {
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 ph.wait(s, B_D0);
                 fence_after();
 #pragma unroll
-                for (int half = 0; half < HALVES; ++half) {
+                for (int half = 0; half < P::HALVES; ++half) {
                     float d[16], e[16];
                     tmem_load_16x32(pl.tmem(tmem, D0, half), d);
                     tmem_load_16x32(pl.tmem(tmem, D1, half), e);
@@ -229,12 +229,12 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
                 }
             } else {
 #pragma unroll
-                for (int half = 0; half < HALVES; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
+                for (int half = 0; half < P::HALVES; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
             }
             if (!tail) continue;
             publish_rows(s, pl, x, xi);  // gx (read again from memory behind the chunks, whose sum takes its registers)
 #pragma unroll
-            for (int half = 0; half < HALVES; ++half)
+            for (int half = 0; half < P::HALVES; ++half)
 #pragma unroll
                 for (int i = 0; i < 16; ++i) x[half][i] = 0.f;
             // ---- hidden units: one scale per row for all chunks, |gh| <= 128 max|gx| max|W2| (see the forward)
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             ph.wait(s, B_A1_FREE);
             add_accumulator(pl, tmem, (chunks & 1) ? DX : DY, x);
 #pragma unroll
-            for (int half = 0; half < HALVES; ++half) {
+            for (int half = 0; half < P::HALVES; ++half) {
                 float g[16];
                 load_rows(p.gx, 128, row_base, p.N, pl, half, g);
 #pragma unroll
@@ -256,11 +256,11 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             }
             publish_rows(s, pl, x, xi);  // gy
 #pragma unroll
-            for (int half = 0; half < HALVES; ++half) store_rows(p.gy, 128, row_base, p.N, pl, half, x[half]);
+            for (int half = 0; half < P::HALVES; ++half) store_rows(p.gy, 128, row_base, p.N, pl, half, x[half]);
             ph.wait(s, B_D0);
             fence_after();
 #pragma unroll
-            for (int half = 0; half < HALVES; ++half) {
+            for (int half = 0; half < P::HALVES; ++half) {
                 float d[16];
                 tmem_load_16x32(pl.tmem(tmem, D0, half), d);
 #pragma unroll
@@ -269,201 +269,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_kernel(const 
             }
         }
     }
-    block_end(s, tmem, p.status);
-}
-
-// The same for a cluster of four blocks (dense_tc_core.cuh): block 0, 1, 2 multiplies gq', gk, gv, block r hidden chunk r,
-// block 0 the last product; the shares of gx and of gy are collected by rows of 32.
-// 2,400 rows, 512 hidden units, mean of a network's boundaries: 38 us with a block per tile, 27 here.
-__global__ void __launch_bounds__(BLOCK_THREADS, 1) dense_backward_split_kernel(const DenseBackward p)
-{
-    extern __shared__ __align__(1024) unsigned char smem_tc[];
-    uint32_t tmem;
-    const Shared s = block_begin(smem_tc, tmem);
-    const uint32_t rank = cluster_rank();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int chunks = p.ff / 128;
-    const long long row_base = (long long)(blockIdx.x / SPLIT) * 128;
-    const bool head = p.head != nullptr, tail = p.tail != nullptr;
-    const bool has_head = head && rank < 3, has_chunk = tail && (int)rank < chunks, has_last = tail && rank == 0;
-    cluster_sync();  // every block's barriers are ready for the others' arrivals
-
-    if (warp == STREAM_WARP) {
-        if (lane == 0) {
-            Producer<SPLIT_STAGES> pr;
-            if (has_head) pr.stream(s, p.head, (int)rank, 1);
-            if (has_chunk && pr.ok) pr.stream(s, p.tail, 3 + first_of_chunk(rank), 1);
-            if (has_chunk && pr.ok) pr.stream(s, p.tail, 3 + second_of_chunk(rank, chunks), 1);
-            if (has_last && pr.ok) pr.stream(s, p.tail, 3 + 2 * chunks, 1);
-            if (!pr.ok) pr.drain(s);
-        }
-        __syncwarp();
-    } else if (warp == ISSUE_WARP) {
-        if (lane == 0) {
-            Issuer<SPLIT_STAGES> is;
-            Phase ph;
-            bool ok = true;
-            auto ready = [&](int b) { ok = ph.wait(s, b) && ok; fence_after(); };
-            auto rows_ready = [&]() {
-                ok = ph.wait_cluster(s, B_ROWS) && ok;
-                fence_async_smem();
-                fence_after();
-            };
-            auto product = [&](int d, int done) {
-                if (ok) is.product(s, tmem, d, OFF_A0);
-                ok = ok && is.ok;
-                mma_commit(s.bar(done));
-            };
-            if (has_head) {
-                ready(B_A0);
-                product(D0, B_D0);
-            }
-            if (tail) {
-                if (head) rows_ready(); else ready(B_A0);  // gx
-                if (has_chunk) {
-                    product(D1, B_D1);
-                    ready(B_A0);
-                    product(DX, B_DX);
-                }
-                if (has_last) {
-                    rows_ready();  // gy
-                    product(D0, B_D0);
-                }
-            }
-            if (!ok) is.drain(s);
-        }
-        __syncwarp();
-    } else {
-        const Place pl;
-        const float wh_i = head ? reinterpret_cast<const float *>(p.head)[0] * GIVEN_BACK : 0.f;
-        float w2_i = 0.f, w1_i = 0.f, wo_i = 0.f;
-        if (tail) {
-            const float *inv = reinterpret_cast<const float *>(p.tail);
-            w2_i = inv[3] * GIVEN_BACK; w1_i = inv[3 + 2 * chunks - 1] * GIVEN_BACK; wo_i = inv[3 + 2 * chunks] * GIVEN_BACK;
-        }
-        Phase ph;
-        float xi[4];
-        // shares of a sum from the accumulator d_col (or nothing) to the blocks that finish the rows
-        auto send = [&](int d_col, bool any, float w_i, const float (&ri)[4]) {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                float d[16];
-                if (any) {
-                    tmem_load_16x32(pl.tmem(tmem, d_col, half), d);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) d[i] = 0.f;
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) d[i] *= ri[2 * half + ((i >> 1) & 1)] * w_i;
-                stage_share(s, pl, half, d);
-            }
-            send_share(s, rank);
-        };
-        // the rows that this warp finishes: 2 warp + u of the block's 32
-        const long long own = row_base + 32 * (int)rank + 2 * warp;
-        auto load_own = [&](const float *src, float4 (&v)[2]) {
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-                v[u] = own + u < p.N ? *reinterpret_cast<const float4 *>(src + (own + u) * 128 + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-        };
-        auto collect = [&](float4 (&sum)[2], float *dst) {  // sum += the four shares
-            float4 v[2];
-            if (threadIdx.x == 0) expect_shares(s);
-            collect_shares(s, ph, v);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                sum[u].x += v[u].x; sum[u].y += v[u].y; sum[u].z += v[u].z; sum[u].w += v[u].w;
-                if (own + u < p.N) *reinterpret_cast<float4 *>(dst + (own + u) * 128 + 4 * lane) = sum[u];
-            }
-        };
-        float4 g[2];  // gx, then gy, of the own rows
-        if (head) {
-            if (rank == 0) {
-                const float4 wp = *reinterpret_cast<const float4 *>(p.w_pos + 4 * lane);
-                load_operand(s, s.mem + OFF_A0, [&](int r, int) {
-                    const long long row = row_base + r;
-                    float4 gq = make_float4(0.f, 0.f, 0.f, 0.f), qv = gq;
-                    float ga = 0.f;
-                    if (row < p.N) {
-                        gq = *reinterpret_cast<const float4 *>(p.gq + row * 128 + 4 * lane);
-                        qv = *reinterpret_cast<const float4 *>(p.q + row * 128 + 4 * lane);
-                        ga = p.ga[row * HEADS + (lane >> 2)];
-                    }
-                    return query_grad(p, wp, gq, qv, ga, row);
-                });
-            } else if (rank < 3) {
-                const float *src = rank == 1 ? p.gk : p.gv;
-                load_operand(s, s.mem + OFF_A0, [&](int r, int) {
-                    return row_base + r < p.N ? *reinterpret_cast<const float4 *>(src + (row_base + r) * 128 + 4 * lane)
-                                              : make_float4(0.f, 0.f, 0.f, 0.f);
-                });
-            }
-            load_own(p.g_res, g);
-            if (has_head) {
-                fence_async_smem();
-                fence_before();
-                mbar_arrive(s.bar(B_A0));
-                epilogue_sync();
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(0)[pl.row0 + 8 * i];
-                ph.wait(s, B_D0);
-                fence_after();
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = 0.f;
-            }
-            send(D0, has_head, wh_i, xi);
-            collect(g, p.gx);
-            if (tail) {
-                if (threadIdx.x == 0) expect_rows(s);
-                spread_rows(s, ph, rank, g, SPLIT, 1);
-                ph.wait_cluster(s, B_ROWS);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(1)[pl.row0 + 8 * i];
-            }
-        } else {
-            float x[2][16];
-#pragma unroll
-            for (int half = 0; half < 2; ++half) load_rows(p.gx, 128, row_base, p.N, pl, half, x[half]);
-            load_own(p.gx, g);
-            publish_rows(s, pl, x, xi);
-        }
-        if (tail) {
-            // ---- hidden units: one scale per row for all chunks, |gh| <= 128 max|gx| max|W2| (see the forward)
-            float hs[4], hi[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) hs[i] = power_of_two(137438953472.0f * xi[i] * w2_i, hi[i]);
-            if (has_chunk) {
-                hidden_grads(p, s, pl, ph, tmem, D1, B_D1, rank, row_base, xi, w2_i, hs, OFF_A0, B_A0, false);
-                ph.wait(s, B_DX);
-                fence_after();
-            } else {
-                epilogue_sync();  // (buffer 0 is about to take the shares: gx is no longer being written)
-            }
-            send(DX, has_chunk, w1_i, hi);
-            collect(g, p.gy);
-            if (threadIdx.x == 0 && has_last) expect_rows(s);
-            spread_rows(s, ph, rank, g, 1, 2);
-            if (has_last) {
-                ph.wait_cluster(s, B_ROWS);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) xi[i] = s.row_floats(2)[pl.row0 + 8 * i];
-                ph.wait(s, B_D0);
-                fence_after();
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    float d[16];
-                    tmem_load_16x32(pl.tmem(tmem, D0, half), d);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) d[i] *= xi[2 * half + ((i >> 1) & 1)] * wo_i;
-                    store_rows(p.gattn, 128, row_base, p.N, pl, half, d);
-                }
-            }
-        }
-    }
-    __syncthreads();
-    cluster_sync();  // (no block ends while another may still write to it)
     block_end(s, tmem, p.status);
 }
 
@@ -519,7 +324,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1) weight_grad_kernel(const GradJo
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem_tc + GR_MISC + 56);
     const long long all = (job.rows + GR_ROWS - 1) / GR_ROWS;  // chunks of the job, and this block's share
     const long long c_lo = all * blockIdx.y / splits, c_hi = all * (blockIdx.y + 1) / splits;
-    const Place pl;
+    const PlaceOf<128> pl;
     float acc[2][16];  // the accumulator's chunks so far: thread = 4 rows x 8 columns, as in the chain kernels
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i >> 4][i & 15] = 0.f;
@@ -700,16 +505,14 @@ int launch_dense_backward(const DenseBackward &args, cudaStream_t s)
     DenseBackward p = args;
     p.status = wait_status();
     static thread_local DenseLaunch launch;
-    int rc = launch.configure(reinterpret_cast<const void *>(dense_backward_kernel<2>), reinterpret_cast<const void *>(dense_backward_kernel<1>),
-                              reinterpret_cast<const void *>(dense_backward_split_kernel), "dense backward");
+    const void *const kernels[3] = {reinterpret_cast<const void *>(dense_backward_kernel<128>), reinterpret_cast<const void *>(dense_backward_kernel<64>),
+                                    reinterpret_cast<const void *>(dense_backward_kernel<32>)};
+    int rc = launch.configure(kernels, "dense backward");
     if (rc != CF_OK) return rc;
-    const long long tiles = (p.N + 127) / 128, cap = sm_count();
-    if (split_tiles(tiles, p.ff, launch.clusters()))
-        launch_chained_cluster(dense_backward_split_kernel, (unsigned)(tiles * SPLIT), SPLIT, tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s, false, p);
-    else if (half_tiles(p.N))
-        dense_backward_kernel<1><<<(unsigned)((p.N + 63) / 64), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
-    else
-        dense_backward_kernel<2><<<(unsigned)(tiles < cap ? tiles : cap), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
+    const int rows = tile_rows(p.N);
+    const long long blocks = (p.N + rows - 1) / rows, cap = sm_count();
+    auto kernel = rows == 128 ? dense_backward_kernel<128> : rows == 64 ? dense_backward_kernel<64> : dense_backward_kernel<32>;
+    kernel<<<(unsigned)(blocks < cap ? blocks : cap), tc5::BLOCK_THREADS, tc5::SMEM_BYTES, s>>>(p);
     return launch_status("dense_backward_kernel");
 }
 

@@ -31,14 +31,6 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// (acquires what other blocks of the cluster wrote before they arrived)
-__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ unsigned long long global_ns()
 {
     unsigned long long t;
@@ -48,10 +40,9 @@ __device__ __forceinline__ unsigned long long global_ns()
 // Every wait is bounded: after two seconds (or once another thread of the block has given up) it returns false; the
 // caller then leaves its loop, and the block drains its copies, frees its tensor memory and returns.
 constexpr unsigned long long WAIT_NS = 2000000000ull;
-template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile unsigned *gave_up, unsigned long long limit_ns = WAIT_NS)
 {
-    auto ready = [&]() { return CLUSTER ? mbar_try_cluster(bar, parity) : mbar_try(bar, parity); };
+    auto ready = [&]() { return mbar_try(bar, parity); };
     if (ready()) return true;
     const unsigned long long t0 = global_ns();
     for (int tries = 0; tries < (1 << 28); ++tries) {

@@ -82,24 +82,36 @@ def test_boundaries_shared_by_a_cluster_or_not(ff, atoms):
 
 
 @pytest.mark.parametrize("ff", [128, 512, 640])
-def test_tiles_of_64_and_of_128_rows(ff):
-    """A tile of 64 rows on every SM, and one row more (tiles of 128): the same bits for the rows that both have, and for a batch whose
-    last tile has one row or 63."""
+@pytest.mark.parametrize("rows", [32, 64])
+def test_tiles_of_32_64_and_128_rows(ff, rows):
+    """A tile of so many rows on every SM, and one row more (tiles of twice as many): the same bits for the rows that both have, and for
+    batches whose last tile has one row or all but one."""
     from crystalformer_b200.model import Latticeformer, default_params
     torch.manual_seed(ff)
     model = Latticeformer(default_params(num_layers=2, ff_dim=ff)).cuda()
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    cb = make_crystals(6, 64 * sms + 1, lambda rng, b: np.ones(b, dtype=np.int64), length_range=(8.0, 14.0))
+    most = rows * torch.cuda.get_device_properties(0).multi_processor_count
+    cb = make_crystals(6, most + 1, lambda rng, b: np.ones(b, dtype=np.int64), length_range=(8.0, 14.0))
     t = lambda x: torch.as_tensor(x).cuda()
     batch = lambda n: types.SimpleNamespace(x=t(cb.x)[:n], pos=t(cb.pos)[:n], trans_vec=t(cb.trans_vec)[:n], sizes=t(cb.sizes)[:n])
     model.train()
     with torch.no_grad():
-        model(batch(64 * sms))
+        model(batch(most))
     model.eval()
     with torch.no_grad():
-        whole = model(batch(64 * sms + 1))
-        for n in (64 * sms, 64 * sms - 1, 64 * sms - 63):
+        whole = model(batch(most + 1))
+        for n in (most, most - 1, most - rows + 1):
             assert torch.equal(model(batch(n)), whole[:n]), n
+    # the step's gradients: sums over the rows in float32, in another order of shares
+    model.train()
+    grads = {}
+    for n in (most, most + 1):
+        x = batch(n)
+        model.zero_grad(set_to_none=True)
+        (model(x)[:most].abs().sum()).backward()
+        grads[n] = {k: p.grad.clone() for k, p in model.named_parameters() if p.requires_grad}
+    noise = 1e-6 * max(float(g.norm()) for g in grads[most].values())
+    for k, g in grads[most].items():
+        assert (grads[most + 1][k] - g).norm() <= 2e-6 * g.norm() + noise, k
 
 
 @pytest.mark.parametrize("ff", [128, 384, 512])
