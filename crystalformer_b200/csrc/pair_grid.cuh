@@ -86,20 +86,19 @@ inline bool pair_grid_fits(long long N, long long B, long long E, long long max_
     return N > 0 && max_atoms <= PG_MAX_ATOMS && N < (1ll << 28) && pair_grid_bytes(N, B, E, max_atoms) > 0;
 }
 // Whether an inference batch gains by them.  The plan, the vectors and a block's fixed work (a row's Gaussians at the nodes, whatever
-// its keys) want
-// - enough pairs: forwards of 1, 4, 16, 64, 128 crystals of up to 30 atoms 196, 208, 220, 236, 291 us against 214, 208, 228, 266,
-//   367 by row lists, 1, 16, 64 of up to 60 atoms 217, 250, 292 against 191, 293, 475; without a basis (seven layers, term
-//   lists) 255, 270, 293, 307, 361 against 250, 257, 278, 337, 417;
-// - enough keys per row: 256, 1,024 crystals of up to 8 atoms 254, 443 against 254, 372, 483 and 596 of up to 12 377, 388 against
-//   349, 357, 118 and 436 of up to 18 234, 399 against 270, 397.
-// With several forwards in flight it is not latency that counts, and they pay later: sixteen batches of 64, 128, 256 crystals of up
-// to 24 atoms 2,389, 2,605, 3,461 us against 1,978, 2,497, 3,905, of up to 40 2,603, 3,282, 5,885 against 3,589, 5,689, 10,453, 16
-// of up to 60 2,193 against 2,723; without a basis 64, 128, 256 of up to 24 2,584, 2,941, 3,587 against 2,067, 2,882, 4,448.  The
-// line is drawn there for all, so that a batch has the same bits however it is issued.
+// its keys) want enough pairs and enough keys per row.  Times by row lists (without a basis: term lists), then over grids:
+// - one forward at a time: 1, 4, 16, 64, 128 crystals of up to 30 atoms 211, 205, 218, 248, 354 us and 199, 200, 203, 220, 276; 1, 16,
+//   64 of up to 60 182, 280, 462 and 216, 227, 273; 16, 64, 1,024 of up to 8 161, 182, 363 and 200, 199, 407; without a basis (seven
+//   layers) 16, 64, 128 of up to 30 260, 316, 390 and 261, 285, 325, 16, 64 of up to 60 330, 503 and 288, 334;
+// - sixteen batches in flight, where it is not latency that counts: 64, 128, 256 of up to 16 1,662, 1,876, 2,539 and 1,731, 2,075, 2,590;
+//   16, 64, 128, 256 of up to 24 (16 keys per row) 1,924, 1,855, 2,459, 3,866 and 1,829, 1,853, 2,391, 3,389; 16, 64, 256 of up to
+//   40 2,018, 3,166, 10,329 and 1,618, 2,355, 5,441; without a basis 64, 128, 256 of up to 24 2,080, 2,849, 4,566 and 2,248, 2,680,
+//   3,673, 32 of up to 40 2,233 and 2,193, 256 of up to 16 (11 keys per row) 3,101 and 2,970.
+// One line for all, so that a batch has the same bits however it is issued.
 inline bool pair_grid_pays(long long N, long long B, long long E, long long max_atoms, long long K)
 {
-    if (!pair_grid_fits(N, B, E, max_atoms) || E < 11 * N) return false;
-    return E >= 30000 || (K > 0 && E >= 18000 && E >= 24 * N);
+    if (!pair_grid_fits(N, B, E, max_atoms)) return false;
+    return K > 0 ? (E >= 5000 && E >= 16 * N) || (E >= 30000 && E >= 11 * N) : E >= 20000 && E >= 11 * N;
 }
 
 // ... and whether a training step does: device time of a step (four layers), term lists against grids.  With a basis what it saves
