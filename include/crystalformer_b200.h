@@ -329,8 +329,8 @@ int cf_infinite_attn_bwd_grid(const float *q, const float *k, const float *v, co
 
 /* ------------------------------------------------------------------------------------------------------------
  * Row lists and the tensor-core row kernel for batches of small crystals (max_atoms <= 64; K = 64, or K = 0: no
- * radial basis, W may be NULL; inference).  The one-call forwards use them for K = 64 (without a basis the
- * enumerating kernel with term lists is the faster one).
+ * radial basis, W may be NULL; inference).  The one-call forwards use them for K = 64 where there are too few pairs for
+ * pair grids (without a basis the enumerating kernel with term lists is the faster one there).
  * Same function as cf_infinite_attn_fwd (real_enc_proj_fwd + fused_dpa_fwd of the reference,
  * models/kernels/real_enc_proj_fwd.cu:63-169, models/kernels/fused_dpa_fwd_v3.cu), other organisation:
  * cf_row_list_build stores, per ATOM ROW, all (key, translation) terms within the term-list window of their edge's
