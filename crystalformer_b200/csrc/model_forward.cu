@@ -83,7 +83,7 @@ struct Scratch {
     int64_t *atom_start, *edge_start, *batch, *row_start, *edges;
     float *pos_ij, *rvlen, *x, *encoder;
     int32_t *row_order;
-    char *grid;  // pair grids (null: more pairs than they are kept for)
+    char *grid;  // pair grids
     size_t bytes;
 };
 
@@ -101,8 +101,7 @@ Scratch carve(void *workspace, int64_t N, int64_t B, int64_t E, int64_t ff_dim)
     s.row_order = c.take<int32_t>(N);
     s.x = c.take<float>(N * MODEL_DIM);
     s.encoder = c.take<float>((size_t)cf_encoder_workspace_floats(N, E, ff_dim));
-    const size_t grid = pair_grid_bytes(N, B, E, N > 0 ? E / N : 0);  // (the largest crystal has at least E / N atoms)
-    s.grid = grid > 0 ? c.take<char>(grid) : nullptr;
+    s.grid = c.take<char>(pair_grid_reserve(N, B, E));
     s.bytes = c.used;
     return s;
 }
@@ -186,7 +185,7 @@ int model_forward_impl(void *cublas_handle, const float *features, const int64_t
     rc = encoder_forward_impl(cublas_handle, num_layers, weights, scalars, w.x, w.pos_ij, trans,
                               cutoff_radius != 0.0 ? w.rvlen : nullptr, w.batch, w.edges, w.row_start, N, B, E, max_atoms, K,
                               ff_dim, wscale, cutoff_radius, lattice_range, minimum_range, w.encoder, order, attn_events,
-                              stream, embed_fused ? &embed : nullptr, early, begun, w.grid != nullptr ? &grid : nullptr);
+                              stream, embed_fused ? &embed : nullptr, early, begun, &grid);
     if (rc != CF_OK) return rc;
     const bool chained = num_layers > 0 && N > 0;  // behind the encoder's last dense block
     if (gather != nullptr)

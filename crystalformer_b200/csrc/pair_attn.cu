@@ -555,7 +555,9 @@ __global__ void list_left_kernel(const unsigned char *__restrict__ left, long lo
 
 extern "C" int64_t cf_pair_grid_bytes(int64_t N, int64_t B, int64_t E)
 {
-    return N > 0 && B > 0 && E >= 0 ? (int64_t)cf::pair_grid_bytes(N, B, E, 0) : 0;
+    if (N <= 0 || B <= 0 || E < 0) return 0;
+    const size_t bytes = cf::pair_grid_bytes(N, B, E);
+    return bytes <= cf::PG_MAX_BYTES ? (int64_t)bytes : 0;
 }
 
 extern "C" int cf_pair_grid_build(const float *pos_ij, const float *tvecs, const float *rvlen, const int64_t *atom_start,

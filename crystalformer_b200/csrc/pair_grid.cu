@@ -452,10 +452,8 @@ PairGrid carve(Carver &c, long long N, long long B, long long E)
 
 }  // namespace
 
-size_t pair_grid_bytes(long long N, long long B, long long E, long long max_atoms)
+size_t pair_grid_bytes(long long N, long long B, long long E)
 {
-    const long long pairs = (E + N) / 2;
-    if (max_atoms > PG_MAX_ATOMS || N <= 0 || (size_t)(pairs + extra_slots(pairs)) * 64 * PG_TILES_BASIS > PG_MAX_BYTES) return 0;
     Carver c{nullptr};
     carve(c, N, B, E);
     return c.used;

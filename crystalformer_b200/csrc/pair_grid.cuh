@@ -78,12 +78,20 @@ struct PairGridParams {
 };
 
 // Bytes for a batch, and whether a batch can go this way at all.
-size_t pair_grid_bytes(long long N, long long B, long long E, long long max_atoms_or_0);
+size_t pair_grid_bytes(long long N, long long B, long long E);
 PairGrid pair_grid_carve(void *memory, long long N, long long B, long long E);
 bool pair_grid_params(long long K, double dist_max, double wscale, float a_widest, float floor_log2, PairGridParams &out);
 inline bool pair_grid_fits(long long N, long long B, long long E, long long max_atoms)
 {
-    return N > 0 && max_atoms <= PG_MAX_ATOMS && N < (1ll << 28) && pair_grid_bytes(N, B, E, max_atoms) > 0;
+    return N > 0 && N < (1ll << 28) && max_atoms <= PG_MAX_ATOMS && E <= PG_MAX_ATOMS * N && pair_grid_bytes(N, B, E) <= PG_MAX_BYTES;
+}
+// What memory for batches of up to N atoms, B crystals and E edges holds for grids: those of any such batch, whether they are this
+// one's or not (a batch that fits has at most 64 edges per atom), so that a workspace grows with each of its sizes.
+inline size_t pair_grid_reserve(long long N, long long B, long long E)
+{
+    if (N <= 0) return 0;
+    const size_t most = pair_grid_bytes(N, B, E < PG_MAX_ATOMS * N ? E : PG_MAX_ATOMS * N);
+    return most < PG_MAX_BYTES ? most : PG_MAX_BYTES;
 }
 // Whether an inference batch gains by them.  The plan, the vectors and a block's fixed work (a row's Gaussians at the nodes, whatever
 // its keys) want enough pairs and enough keys per row.  Times by row lists (without a basis: term lists), then over grids:

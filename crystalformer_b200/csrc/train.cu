@@ -307,8 +307,7 @@ Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64
     s.kr = split ? e.take<float>(3 * E) : nullptr;
     s.phi_reci = split ? e.take<float>(E * HEADS) : nullptr;
     s.lists = fused ? e.take<char>(term_list_workspace_bytes(N, E)) : nullptr;
-    const size_t grid = fused && N > 0 ? pair_grid_bytes(N, B, E, E / N) : 0;  // (the largest crystal has at least E / N atoms)
-    s.grid = grid > 0 ? e.take<char>(grid) : nullptr;
+    s.grid = fused ? e.take<char>(pair_grid_reserve(N, B, E)) : nullptr;
     s.edge_bytes = e.used;
     return s;
 }
@@ -339,7 +338,7 @@ Scratch carve_scratch(const cf_train_desc &d, void *memory, int64_t N, int64_t B
     }
     s.gx[d.num_layers] = c.take<float>(N * CH);
     s.glogit = c.take<float>(E * HEADS);
-    s.prob = d.num_layers > 0 && N > 0 && pair_grid_bytes(N, B, E, E / N) > 0 ? c.take<float>(E * HEADS) : nullptr;
+    s.prob = c.take<float>(E * HEADS);
     bool split = false, values = false;
     for (int l = 0; l < d.num_layers; ++l) {
         split = split || domain_of(d, l) != REAL;

@@ -91,3 +91,22 @@ def test_peer_gather_descriptor_matches_the_header_layout():
     D = _lib.PeerGatherDescriptor
     assert ctypes.sizeof(D) == 24 + 8 * peers
     assert (D.world.offset, D.rank.offset, D.rows_per_rank.offset, D.step.offset, D.cells.offset) == (0, 4, 8, 16, 24)
+
+
+def test_workspace_of_the_maxima_holds_every_batch_below_them(lib):
+    """A slot has the workspace of its three maxima (serving): no batch within them may need more, whatever kernels it takes.  Sizes on
+    both sides of 64 atoms per crystal, of the smallest batch with pair grids and of the most that grids may take."""
+    import numpy as np
+    rng = np.random.default_rng(1)
+    size = lambda n, b, e: int(lib.cf_model_workspace_bytes(n, b, e, 512))
+    crystals = lambda b, n: (b * n, b, b * n * n)
+    for b, large, small in ((16, 70, 60), (20, 88, 64), (64, 70, 60), (128, 70, 60), (1, 65, 64), (40000, 64, 32), (100, 1024, 64)):
+        outer = np.maximum(crystals(b, large), crystals(b, small))
+        assert size(*crystals(b, small)) <= size(*(int(v) for v in outer)), (b, large, small)
+    for _ in range(20000):
+        b = int(np.exp(rng.uniform(0, np.log(50000))))
+        n = b * int(rng.integers(1, 100))
+        e = int(n * rng.uniform(1, 100))
+        outer = [int(v * f) for v, f in zip((n, b, e), rng.choice([1.0, 1.01, 1.25, 4.0], 3))]
+        assert size(n, b, e) <= size(*outer), ((n, b, e), outer)
+        assert size(n, b, min(e, 64 * n)) <= size(*outer), ((n, b, e), outer)

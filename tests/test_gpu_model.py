@@ -221,3 +221,25 @@ def test_pipelined_predictor_equals_direct_calls(golden_model, depth, streams, c
                       h.pos.data_ptr(), h.trans_vec.data_ptr(), h.sizes.data_ptr(), int(h.x.shape[0]), int(h.sizes.shape[0]),
                       int((h.sizes ** 2).sum()), int(h.sizes.max()), 1, None, None)
         assert "exceeds the slot's buffers" in str(e.value)
+
+
+@pytest.mark.parametrize("bins", [64, 0])
+def test_one_slot_serves_batches_of_different_kinds(bins):
+    """Batches of one slot that take different kernels (crystals of 70 atoms: term lists; of 60: pair grids; of 8: row lists) in the
+    workspace of the largest: the direct forward's bits, in any order."""
+    from crystalformer_b200.model import Latticeformer, default_params
+    from crystalformer_b200.serving import PipelinedPredictor
+    torch.manual_seed(5)
+    model = Latticeformer(default_params(num_layers=2, value_pe_dist_real=bins)).cuda().train()
+    batches = [make_crystals(60 + s, 16, uniform_atoms(n, n), length_range=(8.0, 14.0)) for s, n in enumerate((70, 60, 70, 64, 8, 60))]
+    host = [types.SimpleNamespace(**{name: torch.from_numpy(getattr(b, name)).pin_memory() for name in ("x", "pos", "trans_vec", "sizes")})
+            for b in batches]
+    on_gpu = [types.SimpleNamespace(**{k: v.cuda() for k, v in vars(h).items()}) for h in host]
+    with torch.no_grad():
+        model(on_gpu[0])  # sets the width statistics
+        model.eval()
+        direct = [model(d).cpu() for d in on_gpu]
+    runner = PipelinedPredictor(model, depth=1)
+    for h, ref in zip(host, direct):
+        assert torch.equal(runner.result(runner.submit(h)), ref)
+    assert runner._native[0] is not None
