@@ -35,7 +35,8 @@ struct Args {
     const unsigned *counters;
     const unsigned char *left;
     const uint4 *basis_nodes;
-    float inv_wscale, node2;  // h^2: ga is in units of it
+    float inv_wscale;
+    float c_scale, c_unit, n2_scale, ga_unit;  // see column_scales
     float *gq, *ga, *glogit, *prob;
     int max_atoms;
 };
@@ -59,6 +60,27 @@ __device__ __forceinline__ void node_operand(const float (&f)[4], unsigned (&h)[
     split_f16(f[2], f[3], h[1], l[1]);
 #pragma unroll
     for (int u = 0; u < 2; ++u) { h[u] = transpose_8x8(h[u]); l[u] = transpose_8x8(l[u]); }
+}
+
+// Powers of two that keep the columns within half precision (65,504) whatever the widths.  x comes as 2^15 at most, u as 2^11, the
+// basis as 2^14.
+// c = sum_k u_k g_k(d) <= u_max sum_k g_k(d), and sum_k exp(-(y - k)^2 / 2 w^2) <= 1 + sqrt(2 pi) w for any y (the largest term, and the
+// integral of the others): x c is at most 2^13 (1 + sqrt(2 pi) w) after 2^-27, which fits up to w = 2.75 and is halved from there on
+// as often as it takes.
+// x n^2 is at most 2 / e of s^2, s the Gaussian's standard deviation in node spacings; a row's nodes reach down to 2^floor with
+// PA_USUAL_LAG bits to spare, so s^2 <= (nodes)^2 / (2 ln 2 (PA_USUAL_LAG - floor)): 420 at the floor of 2^-30, 2^-9 then.  Scaled to 1 at
+// most, it leaves x c n^2 below x c.
+void column_scales(Args &p, double wscale)
+{
+    int down = 27;
+    for (double most = 8192.0 * (1.0 + 2.5066282746310002 * wscale); most > 65000.0; most *= 0.5) ++down;
+    p.c_scale = (float)ldexp(1.0, -down);
+    p.c_unit = (float)ldexp(1.0, down);
+    const double nodes = p.par.tiles * PG_TILE - PG_POINTS, s2 = nodes * nodes / (2.0 * 0.6931471805599453 * fmax(PA_USUAL_LAG - (double)p.par.floor_log2, 1.0));
+    int n2 = 9;
+    while (0.7357588823428847 * s2 > ldexp(1.0, n2)) ++n2;
+    p.n2_scale = (float)ldexp(1.0, -n2);
+    p.ga_unit = (float)ldexp(1.0 / ((double)p.par.inv_h2 + (double)p.par.inv_h2_low), n2);
 }
 
 template <bool BASIS>
@@ -187,9 +209,7 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
             __syncwarp();  // (u has been read)
             for (int T = 0; T < key_tiles; ++T) pr[T * 32] = gl[T * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        // The columns are x, x c, x n^2 and x c n^2 (n: nodes from zero), scaled: x by 2^15, c by u's scale and 2^2 over the
-        // basis' (c is at most 2.6 of u's largest), n^2 by 2^-9 (x n^2 is at most 2 / e of sigma^2 in node spacings: 550)
-        constexpr float N2_SCALE = 0x1p-9f;
+        // The columns are x, x c, x n^2 and x c n^2 (n: nodes from zero), scaled (column_scales)
         const float2 aa = make_float2(__shfl_sync(FULL, hd.a2h2, 8 * t), __shfl_sync(FULL, hd.a2h2, 8 * t + 4));
         const int var0 = __shfl_sync(FULL, hd.variant, 8 * t), var1 = __shfl_sync(FULL, hd.variant, 8 * t + 4);
         float ga0 = 0.f, ga1 = 0.f, m0 = 0.f, m1 = 0.f;  // m: sum_j w S2
@@ -203,7 +223,7 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
                 const float n0 = (float)(mt * PG_TILE - PG_BELOW + g), n1 = n0 + 8.0f, q0 = n0 * n0, q1 = n1 * n1;
                 const float2 e0 = mul2(aa, make_float2(q0, q0)), e1 = mul2(aa, make_float2(q1, q1));
                 float x[4] = {ex2(e0.x) * PA_W_SCALE, ex2(e0.y) * PA_W_SCALE, ex2(e1.x) * PA_W_SCALE, ex2(e1.y) * PA_W_SCALE};
-                const float s0 = q0 * N2_SCALE, s1 = q1 * N2_SCALE;
+                const float s0 = q0 * p.n2_scale, s1 = q1 * p.n2_scale;
                 node_operand(x, xh[u], xl[u]);
                 const float z[4] = {x[0] * s0, x[1] * s0, x[2] * s1, x[3] * s1};
                 node_operand(z, zh[u], zl[u]);
@@ -221,9 +241,8 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
 #pragma unroll
                         for (int w = 0; w < 4; ++w) c[w] += b[w];
                     }
-                    // x c: 2^15 2^11 2.6 2^14 at most, brought to 2^14
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) c[w] *= x[w] * 0x1p-27f;
+                    for (int w = 0; w < 4; ++w) c[w] *= x[w] * p.c_scale;
                     node_operand(c, yh[u], yl[u]);
                     const float tt[4] = {c[0] * s0, c[1] * s0, c[2] * s1, c[3] * s1};
                     node_operand(tt, th[u], tl[u]);
@@ -274,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
                     ga0 += fmaf(ww.x, d.x, ww.z * d.z);
                     ga1 += fmaf(ww.y, d.y, ww.w * d.w);
                     if (BASIS) {
-                        const float k0 = c_scale0 * 0x1p27f, k1 = c_scale1 * 0x1p27f;
+                        const float k0 = c_scale0 * p.c_unit, k1 = c_scale1 * p.c_unit;
                         gg.x = fmaf(w.x * k0, S1[0], gg.x); gg.y = fmaf(w.y * k1, S1[1], gg.y);
                         gg.z = fmaf(w.z * k0, S1[2], gg.z); gg.w = fmaf(w.w * k1, S1[3], gg.w);
                         ga0 = fmaf(w.x * k0, S3[0], fmaf(w.z * k0, S3[2], ga0));
@@ -324,8 +343,7 @@ __global__ void __launch_bounds__(THREADS, 2) pair_attn_bwd_kernel(const Args p)
         }
         off0 = -off0 / sum0;
         off1 = -off1 / sum1;
-        const float unit = p.node2 / N2_SCALE;
-        if (g == 0) *reinterpret_cast<float2 *>(p.ga + (a0 + i) * HEADS + 2 * t) = make_float2(fmaf(off0, m0, ga0) / sum0 * unit, fmaf(off1, m1, ga1) / sum1 * unit);
+        if (g == 0) *reinterpret_cast<float2 *>(p.ga + (a0 + i) * HEADS + 2 * t) = make_float2(fmaf(off0, m0, ga0) / sum0 * p.ga_unit, fmaf(off1, m1, ga1) / sum1 * p.ga_unit);
         // per edge, for the sums over the rows
         float2 *po = reinterpret_cast<float2 *>(p.prob + (e0 + g) * HEADS + 2 * t), *go2 = reinterpret_cast<float2 *>(p.glogit + (e0 + g) * HEADS + 2 * t);
         const float norm0 = 1.0f / sum0, norm1 = 1.0f / sum1;
@@ -382,7 +400,7 @@ int launch_pair_attn_bwd(const PairAttn &l, cudaStream_t s)
     p.edge_start = l.edge_start; p.rule = l.rule; p.par = l.par; p.slots = l.grid.slots; p.tiles = l.grid.tiles; p.counters = l.grid.counters;
     p.left = l.left; p.basis_nodes = l.grid.basis_nodes;
     p.inv_wscale = l.wscale > 0 ? (float)(1.0 / (double)(float)l.wscale) : 1.0f;
-    p.node2 = (float)(1.0 / ((double)l.par.inv_h2 + (double)l.par.inv_h2_low));
+    column_scales(p, (double)(float)l.wscale);
     p.gq = l.gq; p.ga = l.ga; p.glogit = l.glogit; p.prob = l.prob; p.max_atoms = l.max_atoms;
     auto kernel = l.K > 0 ? pair_attn_bwd_kernel<true> : pair_attn_bwd_kernel<false>;
     static thread_local bool configured[64][2] = {};

@@ -33,7 +33,7 @@ def inputs(cb, sigma, scale=0.3, seed=3):
     return q, k, v, a, W
 
 
-def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE, gout=None):
+def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE, gout=None, dist_max=DIST_MAX):
     """(grid results, enumerating kernel's results, the call again); with gout: the backward's, and the rows left over"""
     q, k, v, a, W = x
     sizes = dev(cb.sizes)
@@ -42,8 +42,8 @@ def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE, gout=Non
     nmax = int(cb.sizes.max())
     W = dev(W) if K else None
     args = (dev(q), dev(k), dev(v), dev(a), g["pos_ij"], dev(cb.trans_vec), g["rvlen"], g["batch"], g["edges"], g["row_start"],
-            nmax, K, DIST_MAX, wscale, W, cutoff, 2, minimum)
-    grids = ops.pair_grid_build(g["pos_ij"], dev(cb.trans_vec), g["rvlen"], atom_start, edge_start, cb.num_atoms, nmax, K, DIST_MAX,
+            nmax, K, dist_max, wscale, W, cutoff, 2, minimum)
+    grids = ops.pair_grid_build(g["pos_ij"], dev(cb.trans_vec), g["rvlen"], atom_start, edge_start, cb.num_atoms, nmax, K, dist_max,
                                 wscale, cutoff, 2, minimum, A_WIDEST)
     if gout is not None:
         out, logit, lse, _, left = ops.infinite_attn_fwd_grid(*args, grids)
@@ -54,11 +54,11 @@ def run(ops, cb, x, K, cutoff=-3.5, minimum=2, pos=None, wscale=WSCALE, gout=Non
             lambda: ops.infinite_attn_fwd_grid(*args, grids, want_psi_row=K > 0))
 
 
-def reference(cb, x, K, cutoff, minimum, wscale=WSCALE):
+def reference(cb, x, K, cutoff, minimum, wscale=WSCALE, dist_max=DIST_MAX):
     q, k, v, a, W = x
     edges = oracle.edge_index(cb.sizes)
     pos_ij, _, _, rvlen = oracle.geometry(cb.pos, cb.trans_vec, edges)
-    z, psiW = oracle.lattice_sum_fwd(a, pos_ij, cb.trans_vec, cb.batch, edges, K, DIST_MAX, wscale, W=W[None] if K else None, rvlen=rvlen,
+    z, psiW = oracle.lattice_sum_fwd(a, pos_ij, cb.trans_vec, cb.batch, edges, K, dist_max, wscale, W=W[None] if K else None, rvlen=rvlen,
                                      cutoff_radius=cutoff, lattice_range=2, minimum_range=minimum, precision="f64")
     _, out = oracle.fused_attn_fwd(q, k, v, z, psiW, edges, precision="f64")
     logit = np.einsum("ehd,ehd->eh", q[edges[0]].astype(np.float64), k[edges[1]].astype(np.float64)) + z
@@ -146,16 +146,16 @@ def test_crystals_beyond_the_extra_vectors(ops):
     close(out, ref, out0, slice(None), "all rows")
 
 
-def backward_reference(cb, x, go, K, cutoff, minimum, wscale):
+def backward_reference(cb, x, go, K, cutoff, minimum, wscale, dist_max=DIST_MAX):
     q, k, v, a, W = x
     edges = oracle.edge_index(cb.sizes)
     pos_ij, _, _, rvlen = oracle.geometry(cb.pos, cb.trans_vec, edges)
     Wn = W[None] if K else None
     common = dict(rvlen=rvlen, cutoff_radius=cutoff, lattice_range=2, minimum_range=minimum, precision="f64")
-    z, psiW = oracle.lattice_sum_fwd(a, pos_ij, cb.trans_vec, cb.batch, edges, K, DIST_MAX, wscale, W=Wn, **common)
+    z, psiW = oracle.lattice_sum_fwd(a, pos_ij, cb.trans_vec, cb.batch, edges, K, dist_max, wscale, W=Wn, **common)
     prob, out = oracle.fused_attn_fwd(q, k, v, z, psiW, edges, precision="f64")
     gq, gk, gv, g_phi, g_psiW = oracle.fused_attn_bwd(q, k, v, psiW, edges, prob, out, go, precision="f64")
-    ga, _ = oracle.lattice_sum_bwd(a, pos_ij, cb.trans_vec, cb.batch, edges, z, g_phi, g_psiW, K, DIST_MAX, wscale, W=Wn, **common)
+    ga, _ = oracle.lattice_sum_bwd(a, pos_ij, cb.trans_vec, cb.batch, edges, z, g_phi, g_psiW, K, dist_max, wscale, W=Wn, **common)
     return [np.asarray(t, np.float64).reshape(cb.num_atoms, -1) for t in (gq, gk, gv, ga)]
 
 
@@ -200,3 +200,33 @@ def test_tensors_off_sixteen_bytes_are_refused(ops):
         run(ops, cb, (off,) + x[1:], 64)
     with pytest.raises(RuntimeError, match="16 bytes"):
         run(ops, cb, x, 64, gout=off)
+
+
+@pytest.mark.parametrize("dist_max,wscale", [(7.0, 4.0), (5.0, 5.0), (2.0, 10.0), (3.0, 8.0), (14.0, 2.0)])
+def test_wide_bases_stay_within_half_precision(ops, dist_max, wscale):
+    """Bases whose functions overlap by dozens, and a gradient of one sign over all bins: sum_k u_k g_k(d) grows with the width."""
+    cb = make_crystals(49, 6, uniform_atoms(6, 20), length_range=(4.0, 9.0))
+    q, k, v, a, W = inputs(cb, (1.85, 1.98))
+    W[:] = 0.1
+    go = np.full((cb.num_atoms, H, D), 1.2437, np.float32)  # (u = 1.98995: just below a power of two)
+    x = (q, k, v, a, W)
+    got, plain, _, left = run(ops, cb, x, 64, wscale=wscale, gout=go, dist_max=dist_max)
+    assert left.float().mean() < 0.1
+    for name, t, t0, ref in zip(("gq", "gk", "gv", "ga"), got, plain, backward_reference(cb, x, go, 64, -3.5, 2, wscale, dist_max)):
+        close(t.flatten(1), ref, t0.flatten(1), slice(None), name)
+
+
+def test_a_high_floor_stays_within_half_precision(ops):
+    """With a floor of 2^-8 the nodes reach Gaussians of 40 node spacings, whose x n^2 is beyond 1,023: nothing overflows.  The kernels leave
+    terms below 2^-8 out by rules of their own, beyond 3.3 standard deviations at the least: up to P(chi2_5 > 2 ln 2 * 8) = 5 % of a sum
+    weighted by d^2, of which ga is a difference of two per kernel: a fifth in all, P(chi2_3) = 1.1 % and a twentieth without d^2."""
+    cb = make_crystals(49, 6, uniform_atoms(6, 20), length_range=(4.0, 9.0))
+    go = np.random.default_rng(5).standard_normal((cb.num_atoms, H, D)).astype(np.float32)
+    ops.set_weight_floor_log2(-8.0)
+    try:
+        got, plain, _, left = run(ops, cb, inputs(cb, (1.55, 1.6), scale=0.05), 64, gout=go, dist_max=8.0)
+    finally:
+        ops.set_weight_floor_log2(-30.0)
+    assert left.float().mean() < 0.1
+    for name, t, t0 in zip(("gq", "gk", "gv", "ga"), got, plain):
+        assert float((t - t0).norm() / t0.norm()) < (0.2 if name == "ga" else 0.05), name
