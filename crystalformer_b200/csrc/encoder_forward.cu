@@ -333,8 +333,11 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                 by_grid.dist_max = scalars[5]; by_grid.wscale = wscale; by_grid.call = 0;
                 by_grid.grid = pair_grid_carve(grid_memory->memory, N, B, E);
                 by_grid.leftover = by_grid.grid.leftover;
-                rc = launch_pair_grid_build(by_grid, pos_ij, tvecs, a_widest, weights + 3, 11, num_layers, forked ? side.stream : s);
                 by_grid.projected = K > 0;
+                // (early: ordered after the inputs only, so the weights are read on this stream)
+                rc = launch_pair_grid_build(by_grid, pos_ij, tvecs, a_widest, early_prep ? nullptr : weights + 3, 11, num_layers,
+                                            forked ? side.stream : s);
+                if (rc == CF_OK && early_prep && K > 0) rc = launch_projected_basis(by_grid, weights + 3, 11, num_layers, s);
             } else if (sorted_rows) {
                 RowListBuild rb{};
                 rb.pos_ij = pos_ij; rb.tvecs = tvecs; rb.rvlen = cutoff_radius != 0.0 ? rvlen : nullptr;

@@ -69,6 +69,14 @@ __device__ __forceinline__ void projected_basis(const PlanArgs &p, int at, float
     if (tid == 0) p.grid.projected_scale[at] = __uint_as_float(x - (13u << 23));
 }
 
+// ... by itself, for batches that are prepared ahead of the weights' stream
+__global__ void __launch_bounds__(32 * PG_TILES_BASIS) projected_basis_kernel(const PlanArgs p)
+{
+    __shared__ float w_sh[HEAD_DIM * 65];
+    __shared__ unsigned largest;
+    projected_basis(p, blockIdx.x, w_sh, &largest);
+}
+
 __device__ __forceinline__ float basis_at_node(int m, int k, double wscale)
 {
     const double u = ((double)(m - PG_BELOW) * wscale - 3.0 * (double)(k + 1)) / (3.0 * wscale);  // in standard deviations
@@ -484,18 +492,35 @@ bool pair_grid_params(long long K, double dist_max, double wscale, float a_wides
     return range >= need && sigma_least <= 0.75 * sigma_widest;
 }
 
+namespace {
+void projections(PlanArgs &p, const PairAttn &b, const float *const *W, int W_stride, int calls)
+{
+    p.grid = b.grid;
+    p.calls = calls;
+    for (int c = 0; c < calls; ++c) p.W[c] = W[c * W_stride];
+    p.wscale = (double)(float)b.wscale;
+    p.wscale_f = (float)b.wscale;
+    p.bits = (float)(-0.72134752044448170 / (9.0 * p.wscale * p.wscale));
+}
+}  // namespace
+
+int launch_projected_basis(const PairAttn &b, const float *const *W, int W_stride, int calls, cudaStream_t s)
+{
+    PlanArgs p{};
+    projections(p, b, W, W_stride, calls);
+    projected_basis_kernel<<<calls * HEADS, 32 * PG_TILES_BASIS, 0, s>>>(p);
+    return launch_status("projected_basis_kernel");
+}
+
 int launch_pair_grid_build(const PairAttn &b, const float *pos_ij, const float *tvecs, float a_widest, const float *const *W, int W_stride, int calls,
                            cudaStream_t s)
 {
     PlanArgs p{};
+    projections(p, b, W, W_stride, b.K > 0 && W != nullptr ? calls : 0);
     p.atom_start = b.atom_start; p.edge_start = b.edge_start; p.rvlen = b.rvlen; p.N = b.N; p.B = b.B; p.E = b.E;
     p.tile_cap = b.N / PG_ROWS + b.B; p.extra_cap = b.grid.slot_count - (b.E + b.N) / 2;
-    p.rule = b.rule; p.a_widest = a_widest; p.wscale = (double)(float)b.wscale; p.grid = b.grid;
-    p.basis_blocks = b.K > 0 && W == nullptr ? (2 * PG_FRAGS * 32 + PLAN_THREADS - 1) / PLAN_THREADS : 0;
-    p.calls = b.K > 0 && W != nullptr ? calls : 0;
-    for (int c = 0; c < p.calls; ++c) p.W[c] = W[c * W_stride];
-    p.wscale_f = (float)b.wscale;
-    p.bits = (float)(-0.72134752044448170 / (9.0 * p.wscale * p.wscale));
+    p.rule = b.rule; p.a_widest = a_widest;
+    p.basis_blocks = b.K > 0 && !b.projected ? (2 * PG_FRAGS * 32 + PLAN_THREADS - 1) / PLAN_THREADS : 0;
     pair_plan_kernel<<<1 + p.basis_blocks + p.calls * HEADS, PLAN_THREADS, 0, s>>>(p);
     BuildArgs a{};
     a.pos_ij = pos_ij; a.tvecs = tvecs; a.atom_start = b.atom_start; a.edge_start = b.edge_start; a.B = b.B; a.inv_h2 = b.par.inv_h2; a.inv_h2_low = b.par.inv_h2_low;

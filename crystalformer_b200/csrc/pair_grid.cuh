@@ -132,16 +132,18 @@ struct PairAttn {
     int call;
     float *out, *lse, *psi_row, *logit;  // psi_row, logit: or null
     unsigned char *left;         // per row: 1 if it was left over (or null)
-    bool projected;              // the build had this call's W: no psi_row
+    bool projected;              // the calls' projections at the nodes are made: no psi_row
     int *leftover;               // the rows, and their number in counters[4 (call + 1)]
     // backward
     const float *gout;
     float *gq, *gk, *gv, *ga, *glogit, *prob;
 };
-// The plan and the vectors (geometry, rule, sizes and parameters of `p`; a_widest: the widest Gaussian of any layer), and either the
-// basis at the nodes (W null: for calls with psi_row) or the calls' projections at the nodes (W of call c at W[c * W_stride]).
+// The plan and the vectors (geometry, rule, sizes and parameters of `p`; a_widest: the widest Gaussian of any layer), and the basis at
+// the nodes (for calls with psi_row) or, with p.projected, the calls' projections there: W of call c at W[c * W_stride], or by
+// launch_projected_basis if W is null (a preparation that runs ahead of the weights' stream must not read them).
 int launch_pair_grid_build(const PairAttn &p, const float *pos_ij, const float *tvecs, float a_widest, const float *const *W, int W_stride,
                            int calls, cudaStream_t s);
+int launch_projected_basis(const PairAttn &p, const float *const *W, int W_stride, int calls, cudaStream_t s);
 int launch_pair_attn_bwd(const PairAttn &p, cudaStream_t s);
 int grid_attn_bwd_impl(const PairAttn &p, const float *pos_ij, const float *tvecs, const int64_t *batch, const int64_t *edges,
                        const int64_t *row_start, cudaStream_t s);

@@ -243,3 +243,28 @@ def test_one_slot_serves_batches_of_different_kinds(bins):
     for h, ref in zip(host, direct):
         assert torch.equal(runner.result(runner.submit(h)), ref)
     assert runner._native[0] is not None
+
+
+@pytest.mark.parametrize("sizes", [[12] * 80, [3] * 20])
+def test_early_preparation_reads_the_inputs_only(sizes):
+    """With an inputs-ready event the preparation is not ordered behind the stream; the weights still are: a projection that the stream
+    writes just before the forward is the one that counts (80 crystals: pair grids, 20 small ones: row lists)."""
+    from crystalformer_b200.model import Latticeformer, default_params
+    torch.manual_seed(6)
+    model = Latticeformer(default_params(num_layers=2)).cuda().train()
+    cb = make_crystals(71, len(sizes), lambda rng, b: np.array(sizes), length_range=(4.0, 9.0))
+    data = types.SimpleNamespace(**{name: torch.from_numpy(getattr(cb, name)).cuda() for name in ("x", "pos", "trans_vec", "sizes")})
+    counts = (sum(sizes), sum(n * n for n in sizes), max(sizes))
+    with torch.no_grad():
+        model(data)  # sets the width statistics
+        model.eval()
+        ready = torch.cuda.Event()
+        ready.record()
+        plan = model._current_plan(data.pos.device)
+        before = model._forward_native(data, counts, None, plan, inputs_ready=ready)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(40_000_000)  # (some 20 ms before the weights change)
+        for layer in model.encoder.layers:
+            layer.self_attn.pe_dist_proj.mul_(-2.0)
+        y = model._forward_native(data, counts, None, plan, inputs_ready=ready)
+        assert torch.equal(y, model(data)) and not torch.equal(y, before)
