@@ -28,27 +28,7 @@ __device__ __forceinline__ void split_tf32(float x, unsigned &hi, unsigned &lo)
     hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     lo = __float_as_uint(x - __uint_as_float(hi));
 }
-// Of lo the tensor pipe takes the leading eleven bits: what it cuts off is made symmetric first (1.5 2^-12, the mean of half a unit
-// in the last of the eleven), 2^-23 of x in all; or it is a third piece.
-__device__ __forceinline__ unsigned rounded_lo(unsigned lo) { return __float_as_uint(__uint_as_float(lo) * 1.0003662f); }
 __device__ __forceinline__ unsigned third_piece(unsigned lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
-// c += A B of float32 operands: three products, the small ones first
-__device__ __forceinline__ void mma_split(float (&c)[4], const float (&a)[4], float b0, float b1)
-{
-    unsigned ah[4], al[4], bh0, bl0, bh1, bl1;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        split_tf32(a[u], ah[u], al[u]);
-        al[u] = rounded_lo(al[u]);
-    }
-    split_tf32(b0, bh0, bl0);
-    split_tf32(b1, bh1, bl1);
-    bl0 = rounded_lo(bl0);
-    bl1 = rounded_lo(bl1);
-    mma_tf32(c, al, bh0, bh1);
-    mma_tf32(c, ah, bl0, bl1);
-    mma_tf32(c, ah, bh0, bh1);
-}
 // What the tensor pipe cuts off a sum is half a unit in its last place on average: MMA_LOST of its value, 2^-24 times the mean of 1 /
 // m over mantissas m.
 constexpr float MMA_LOST = 4.3e-8f;

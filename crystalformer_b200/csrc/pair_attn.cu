@@ -11,7 +11,7 @@
 // in passes of up to six node tiles whose sums a warp holds in registers.  (3) warp = head again: sum p v, and E of the eight rows
 // times the projected basis (TAIL = PROJECTED: W_h g(d_m), made once per call), or Psi, which the backward needs, and its
 // projection (TAIL = KEEP_PSI).  Operands are half pairs (nodes, weights: scaled by 2^15, exact to 22 bits over the range that
-// matters), three products each with the small ones first, or TF32 pairs where the range is the caller's (q, k, v, W, w S).
+// matters), three products each with the small ones first, or three TF32 pieces where the range is the caller's (q, k, v, W, w S).
 // (Logits and sum p v by a row's own warp, with float32 sums, cost 10-20 % more: keys and values then come through the L1 once per
 // row instead of once per block, and shared memory, which shares its pipe, is what bounds the second phase.)
 #include <initializer_list>
@@ -434,14 +434,17 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
                 if (row_tiles[r] > 0)
                     reinterpret_cast<float4 *>(p.psi_row + (a0 + i0 + r) * 512)[x] = *reinterpret_cast<const float4 *>(ps + r * PSI_LD + 4 * x);
             }
-        // ---- projection: head h over the bins, in the order of the lane's pieces, by TF32 pairs
+        // ---- projection: head h over the bins, in the order of the lane's pieces (by TF32 pairs 1.5 times a float32 product's error in
+        // rows of few terms, and a tenth more than by three pieces on average)
 #pragma unroll
         for (int bb = 0; bb < 4; ++bb) {
             const float4 w0 = wf[bb][0], w1 = wf[bb][1];
             const float4 x = *reinterpret_cast<const float4 *>(ps + g * PSI_LD + h * 64 + bb * 16 + 4 * t);
-            float pr[4] = {0.f, 0.f, 0.f, 0.f};
-            mma_split(pr, {w0.x, w1.x, w0.y, w1.y}, x.x, x.y);
-            mma_split(pr, {w0.z, w1.z, w0.w, w1.w}, x.z, x.w);
+            const float bv[4] = {x.x, x.y, x.z, x.w};
+            unsigned bh[4], bl[4], b3[4];
+            split3_tf32(bv, bh, bl, b3);
+            float pr[4];
+            mma_exact(pr, {w0.x, w1.x, w0.y, w1.y}, {w0.z, w1.z, w0.w, w1.w}, bh, bl, b3);
 #pragma unroll
             for (int u = 0; u < 4; ++u) proj[u] += pr[u];
         }

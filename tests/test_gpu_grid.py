@@ -230,3 +230,17 @@ def test_a_high_floor_stays_within_half_precision(ops):
     assert left.float().mean() < 0.1
     for name, t, t0 in zip(("gq", "gk", "gv", "ga"), got, plain):
         assert float((t - t0).norm() / t0.norm()) < (0.2 if name == "ga" else 0.05), name
+
+
+def test_projected_sums_are_as_good_as_float32(ops):
+    """The value encoding's part of the rows by itself (v = 0), small logits and large cells: the products with W lose no more than float32
+    sums do (a tenth for chance: 240 atoms of 8 heads and 16 channels)."""
+    cb = make_crystals(52, 60, uniform_atoms(1, 7), length_range=(8.0, 15.0))
+    q, k, v, a, W = inputs(cb, (0.95, 1.4), scale=0.12)
+    v[:] = 0.0
+    x = (q, k, v, a, W)
+    (out, _, _, _, left), (out0, *_), _ = run(ops, cb, x, 64)
+    assert not left.any()
+    ref, _ = reference(cb, x, 64, -3.5, 2)
+    err, err0 = (np.linalg.norm(t.cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref) for t in (out, out0))
+    assert err <= 1.1 * err0, (err, err0)
