@@ -28,6 +28,7 @@ __device__ __forceinline__ void split_tf32(float x, unsigned &hi, unsigned &lo)
     hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     lo = __float_as_uint(x - __uint_as_float(hi));
 }
+// Of lo the tensor pipe takes the leading eleven bits; what is left is a third piece.
 __device__ __forceinline__ unsigned third_piece(unsigned lo) { return __float_as_uint(__uint_as_float(lo) - __uint_as_float(lo & 0xffffe000u)); }
 // What the tensor pipe cuts off a sum is half a unit in its last place on average: MMA_LOST of its value, 2^-24 times the mean of 1 /
 // m over mantissas m.

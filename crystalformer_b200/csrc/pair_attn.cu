@@ -82,7 +82,7 @@ struct Row {
 // E.
 template <int N, int STAGES>
 __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool fresh, int first, const RowHeads &hd, int lane, float (&E)[PASS][4],
-                                          float2 &z, unsigned &largest)
+                                          float2 &z, float2 &largest)
 {
     const int g = lane >> 2, t = lane & 3;
     const float a2h2 = hd.a2h2;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool 
     }
     // heads 2t and 2t + 1 at nodes g and g + 8 of a tile
     const float2 aa = make_float2(__shfl_sync(FULL, a2h2, 8 * t), __shfl_sync(FULL, a2h2, 8 * t + 4));
-    float most = 0.f;
+    float2 most = make_float2(0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < N; ++u) {
         const float n0 = (float)((first + u) * PG_TILE - PG_BELOW + g), n1 = n0 + 8.0f;
@@ -154,18 +154,20 @@ __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool 
         const float2 r1 = mul2(make_float2(E[u][2], E[u][3]), make_float2(ex2(e1.x), ex2(e1.y)));
         E[u][0] = r0.x; E[u][1] = r0.y; E[u][2] = r1.x; E[u][3] = r1.y;
         z = add2(z, add2(r0, r1));
-        most = fmaxf(most, fmaxf(fmaxf(fabsf(r0.x), fabsf(r0.y)), fmaxf(fabsf(r1.x), fabsf(r1.y))));
+        most = make_float2(fmaxf(most.x, fmaxf(fabsf(r0.x), fabsf(r1.x))), fmaxf(most.y, fmaxf(fabsf(r0.y), fabsf(r1.y))));
     }
-    largest = __reduce_max_sync(FULL, __float_as_uint(most));
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) most = make_float2(fmaxf(most.x, __shfl_xor_sync(FULL, most.x, o)), fmaxf(most.y, __shfl_xor_sync(FULL, most.y, o)));
+    largest = most;
 }
 
-// E as the operand of the product with the basis (nodes x heads), half pairs
+// E as the operand of the product with the basis (nodes x heads), half pairs; scales of heads 2t, 2t + 1
 template <int N>
-__device__ __forceinline__ void store_e(const float (&E)[PASS][4], float scale, unsigned char *at, int lane)
+__device__ __forceinline__ void store_e(const float (&E)[PASS][4], float2 scale, unsigned char *at, int lane)
 {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-        const float2 r0 = mul2(make_float2(E[u][0], E[u][1]), make_float2(scale, scale)), r1 = mul2(make_float2(E[u][2], E[u][3]), make_float2(scale, scale));
+        const float2 r0 = mul2(make_float2(E[u][0], E[u][1]), scale), r1 = mul2(make_float2(E[u][2], E[u][3]), scale);
         unsigned h0, l0, h1, l1;
         split_f16(r0.x, r0.y, h0, l0);
         split_f16(r1.x, r1.y, h1, l1);
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0), g = lane >> 2, t = lane & 3;
     const int row_words = pa_row_words(p.max_atoms);
     float *tables = reinterpret_cast<float *>(smem + L::TABLES), *sums = tables + PG_ROWS * row_words;
-    __shared__ float zs[PG_ROWS][HEADS], e_scale[PG_ROWS];
+    __shared__ float e_unit[PG_ROWS][HEADS];  // one of E as stored, over Z
     __shared__ int row_tiles[PG_ROWS];  // node tiles of a row; 0: it is not there or left over
     grid_launch_dependents();
     grid_dependency_wait();  // q, k, v, a
@@ -257,18 +259,20 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     float2 z = make_float2(0.f, 0.f);
     if (good) {
         float E[PASS][4];
-        unsigned largest = 0u;
+        float2 largest, unit = make_float2(1.f, 1.f);
         if (!one_box) {
             for (int T = 0; T < row.key_tiles; ++T) reinterpret_cast<float4 *>(row.sums)[T * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncwarp();
         }
         BY_TILES(count, node_pass<N>(row, ring, one_box, 0, hd, lane, E, z, largest);)
         if (BASIS) {
-            // scaled to a largest value between 2^10 and 2^11: the second pass has 2^5 to exceed the first
-            const unsigned x = min(max(largest & 0x7f800000u, 30u << 23), 230u << 23);
-            const float scale = __uint_as_float((264u << 23) - x);
+            // every head scaled to a largest value between 2^10 and 2^11: the second pass has 2^5 to exceed the first.  (One scale for the
+            // row left 20 bits to a head 2^15 below the others: 1e-6 of its sums.)
+            auto exponent = [](float v) { return min(max(__float_as_uint(v) & 0x7f800000u, 30u << 23), 230u << 23); };
+            const unsigned x0 = exponent(largest.x), x1 = exponent(largest.y);
+            const float2 scale = make_float2(__uint_as_float((264u << 23) - x0), __uint_as_float((264u << 23) - x1));
+            unit = make_float2(__uint_as_float(x0 - (10u << 23)), __uint_as_float(x1 - (10u << 23)));
             BY_TILES(count, store_e<N>(E, scale, smem + L::WARPS * L::REGION + warp * E_ROW, lane);)
-            if (lane == 0) e_scale[warp] = __uint_as_float(x - (10u << 23));
             const int more = tiles - count;
             if (more > 0) {
                 if (!one_box) {
@@ -279,7 +283,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
                 }
                 BY_TILES(more, node_pass<N>(row, ring, false, PASS, hd, lane, E, z, largest); copy_wait<0>(); __syncwarp();
                          store_e<N>(E, scale, smem + warp * L::REGION, lane);)
-                good = __uint_as_float(largest) * scale < 60000.0f;
+                good = __all_sync(FULL, largest.x * scale.x < 60000.0f && largest.y * scale.y < 60000.0f);
             }
         }
 #pragma unroll
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
             z.x += __shfl_xor_sync(FULL, z.x, o);
             z.y += __shfl_xor_sync(FULL, z.y, o);
         }
-        if (g == 0) *reinterpret_cast<float2 *>(&zs[warp][2 * t]) = z;
+        if (BASIS && g == 0) *reinterpret_cast<float2 *>(&e_unit[warp][2 * t]) = make_float2(unit.x / z.x, unit.y / z.y);
     }
     copy_wait<0>();
     // (an infinity or a NaN anywhere in the row, or sums that overflow: the row kernel's)
@@ -382,7 +386,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
             for (int u = 0; u < 4; ++u) proj[u] += c[u];
         }
         const float vs = p.projected_scale[h];
-        const float f0 = in0 ? vs * e_scale[2 * t] / zs[2 * t][h] : 0.f, f1 = in1 ? vs * e_scale[2 * t + 1] / zs[2 * t + 1][h] : 0.f;
+        const float f0 = in0 ? vs * e_unit[2 * t][h] : 0.f, f1 = in1 ? vs * e_unit[2 * t + 1][h] : 0.f;
         proj[0] *= f0; proj[1] *= f1; proj[2] *= f0; proj[3] *= f1;
     } else {
         // ---- Psi: C[bin][row] of bin tile bt and NH heads; the node tiles in reach of the bins are consecutive
@@ -419,10 +423,9 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
             for (int u = 0; u < 2; ++u)
                 wf[bb][u] = __ldg(reinterpret_cast<const float4 *>(p.W + (h * HEAD_DIM + g + 8 * u) * 64 + bb * 16 + 4 * t));
         __syncthreads();  // (E has been read)
-        const float es0 = in0 ? e_scale[2 * t] * (1.0f / PG_BASIS_SCALE) : 0.f, es1 = in1 ? e_scale[2 * t + 1] * (1.0f / PG_BASIS_SCALE) : 0.f;
 #pragma unroll
         for (int u = 0; u < NH; ++u) {
-            const float s0 = in0 ? es0 / zs[2 * t][h0 + u] : 0.f, s1 = in1 ? es1 / zs[2 * t + 1][h0 + u] : 0.f;
+            const float s0 = in0 ? e_unit[2 * t][h0 + u] * (1.0f / PG_BASIS_SCALE) : 0.f, s1 = in1 ? e_unit[2 * t + 1][h0 + u] * (1.0f / PG_BASIS_SCALE) : 0.f;
             float *o = ps + (h0 + u) * 64 + bt * 16 + g;
             o[(2 * t) * PSI_LD] = psi[u][0] * s0; o[(2 * t + 1) * PSI_LD] = psi[u][1] * s1;
             o[(2 * t) * PSI_LD + 8] = psi[u][2] * s0; o[(2 * t + 1) * PSI_LD + 8] = psi[u][3] * s1;

@@ -244,3 +244,22 @@ def test_projected_sums_are_as_good_as_float32(ops):
     ref, _ = reference(cb, x, 64, -3.5, 2)
     err, err0 = (np.linalg.norm(t.cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref) for t in (out, out0))
     assert err <= 1.1 * err0, (err, err0)
+
+
+def test_heads_far_below_the_others_keep_their_bits(ops):
+    """One head whose weights at the nodes lie 2^15 below the other heads' in every row: two atoms 5.4 to 5.7 A apart, each with its largest
+    logit (14.8 bits ahead) for the other."""
+    cb = make_crystals(50, 40, uniform_atoms(2, 2), length_range=(14.0, 15.0))
+    cb.trans_vec[:] = np.eye(3, dtype=np.float32) * 14.5
+    cb.pos[:] = 0.0
+    cb.pos[1::2, 0] = np.random.default_rng(7).uniform(5.4, 5.7, 40)
+    q, k, v, a, W = inputs(cb, (1.18, 1.2))
+    v[:] = 0.0  # (the rows are the projected sums alone)
+    q[:, 0] = k[:, 0] = 0.0
+    q[0::2, 0, 0] = k[1::2, 0, 0] = q[1::2, 0, 1] = k[0::2, 0, 1] = 3.2
+    x = (q, k, v, a, W)
+    (out, _, _, _, left), (out0, *_), _ = run(ops, cb, x, 64)
+    assert not left.any()
+    ref, _ = reference(cb, x, 64, -3.5, 2)
+    close(out[:, 0], ref[:, 0], out0[:, 0], slice(None), "the head below")
+    close(out, ref, out0, slice(None), "all heads")
