@@ -80,7 +80,8 @@ struct Row {
 
 // One pass: N node tiles from `first`.  S of all keys into the table (`fresh`: what it held does not count), E = x sum_j w rho in
 // E.
-template <int N, int STAGES>
+// PER_TILE: a node tile's large products have a sum of their own, added in registers.
+template <bool PER_TILE, int N, int STAGES>
 __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool fresh, int first, const RowHeads &hd, int lane, float (&E)[PASS][4],
                                           float2 &z, float2 &largest)
 {
@@ -105,7 +106,8 @@ __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool 
         for (int T = 0; T < row.key_tiles; ++T, o += 32, wp += 32) {
             uint4 w = *wp;
             if (!mine) w = make_uint4(0u, 0u, 0u, 0u);
-            // (the tensor pipe truncates what it adds to: the small products have a sum of their own)
+            // (the tensor pipe truncates what it adds to: the small products have a sum of their own, and what it cut off the large ones'
+            // last addition is given back)
             float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int f = 0; f < N; f += PA_STEP) {
@@ -118,7 +120,14 @@ __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool 
                     ldmatrix4(hi, plain + (u - f) * 64);
                     mma_f16(small, lo[0], lo[1], lo[2], lo[3], xh[u][0], xh[u][1]);
                     mma_f16(small, hi[0], hi[1], hi[2], hi[3], xl[u][0], xl[u][1]);
-                    mma_f16(sum, hi[0], hi[1], hi[2], hi[3], xh[u][0], xh[u][1]);
+                    if (PER_TILE) {
+                        float c[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma_f16(c, hi[0], hi[1], hi[2], hi[3], xh[u][0], xh[u][1]);
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) sum[x] += c[x];
+                    } else {
+                        mma_f16(sum, hi[0], hi[1], hi[2], hi[3], xh[u][0], xh[u][1]);
+                    }
                     ldmatrix4_trans(lo, trans + (u - f) * 64 + 32);
                     ldmatrix4_trans(hi, trans + (u - f) * 64);
                     mma_f16(E[u], lo[0], lo[1], lo[2], lo[3], w.x, w.y);
@@ -128,7 +137,11 @@ __device__ __forceinline__ void node_pass(Row &row, KeyRing<STAGES> &ring, bool 
                 ring.done();
             }
             // S of keys g and g + 8, heads 2t and 2t + 1
-            float4 sum = make_float4((small[0] + sb[0]) + sa[0], (small[1] + sb[1]) + sa[1], (small[2] + sb[2]) + sa[2], (small[3] + sb[3]) + sa[3]);
+            auto whole = [&](int x) {
+                const float large = sb[x] + sa[x];
+                return large + fmaf(large, MMA_LOST, small[x]);
+            };
+            float4 sum = make_float4(whole(0), whole(1), whole(2), whole(3));
             if (!fresh) {
                 const float4 v = *o;
                 sum = make_float4(v.x + (mine0 ? sum.x : 0.f), v.y + (mine1 ? sum.y : 0.f), v.z + (mine0 ? sum.z : 0.f), v.w + (mine1 ? sum.w : 0.f));
@@ -196,7 +209,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(FULL, tid >> 5, 0), g = lane >> 2, t = lane & 3;
     const int row_words = pa_row_words(p.max_atoms);
     float *tables = reinterpret_cast<float *>(smem + L::TABLES), *sums = tables + PG_ROWS * row_words;
-    __shared__ float e_unit[PG_ROWS][HEADS];  // one of E as stored, over Z
+    __shared__ float e_unit[PG_ROWS][HEADS], tops[PG_ROWS][HEADS];  // one of E as stored, over Z; largest logits
     __shared__ int row_tiles[PG_ROWS];  // node tiles of a row; 0: it is not there or left over
     grid_launch_dependents();
     grid_dependency_wait();  // q, k, v, a
@@ -264,7 +277,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
             for (int T = 0; T < row.key_tiles; ++T) reinterpret_cast<float4 *>(row.sums)[T * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncwarp();
         }
-        BY_TILES(count, node_pass<N>(row, ring, one_box, 0, hd, lane, E, z, largest);)
+        BY_TILES(count, node_pass<!BASIS, N>(row, ring, one_box, 0, hd, lane, E, z, largest);)
         if (BASIS) {
             // every head scaled to a largest value between 2^10 and 2^11: the second pass has 2^5 to exceed the first.  (One scale for the
             // row left 20 bits to a head 2^15 below the others: 1e-6 of its sums.)
@@ -281,7 +294,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
                     row.variant = __shfl_sync(FULL, hd.variant, 0);
                     ring.start(row.vectors(), PASS, more, PASS);
                 }
-                BY_TILES(more, node_pass<N>(row, ring, false, PASS, hd, lane, E, z, largest); copy_wait<0>(); __syncwarp();
+                BY_TILES(more, node_pass<!BASIS, N>(row, ring, false, PASS, hd, lane, E, z, largest); copy_wait<0>(); __syncwarp();
                          store_e<N>(E, scale, smem + warp * L::REGION, lane);)
                 good = __all_sync(FULL, largest.x * scale.x < 60000.0f && largest.y * scale.y < 60000.0f);
             }
@@ -296,11 +309,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     copy_wait<0>();
     // (an infinity or a NaN anywhere in the row, or sums that overflow: the row kernel's)
     good = good && __all_sync(FULL, z.x > 1e-30f && z.x < 1e30f && z.y > 1e-30f && z.y < 1e30f);
-    if (good && p.lse != nullptr) {
-        const float top0 = __shfl_sync(FULL, top, 8 * t), top1 = __shfl_sync(FULL, top, 8 * t + 4);
-        if (g == 0)  // (scales: weights 2^15, vectors 2^5)
-            *reinterpret_cast<float2 *>(p.lse + (a0 + i) * HEADS + 2 * t) = make_float2((top0 + log2f(z.x * 0x1p-20f)) * LN2, (top1 + log2f(z.y * 0x1p-20f)) * LN2);
-    }
+    if (t == 0) tops[warp][g] = top;
     if (lane == 0) {
         row_tiles[warp] = good ? tiles : 0;
         if (p.stats != nullptr && good) {
@@ -355,6 +364,8 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
         // divided by the sum of these very weights, of row g in the lanes of g
         total += __shfl_xor_sync(FULL, total, 1);
         total += __shfl_xor_sync(FULL, total, 2);
+        // (their sum is closer than Z, which the tensor pipe adds key tile by key tile; scales: weights and Gaussians 2^15, vectors 2^5)
+        if (p.lse != nullptr && t == 0 && tiles_g > 0) p.lse[(a0 + i0 + g) * HEADS + h] = (tops[g][h] + log2f(total * 0x1p-35f)) * LN2;
         total0 = __shfl_sync(FULL, total, 8 * t);
         total1 = __shfl_sync(FULL, total, 8 * t + 4);
         const float f0 = in0 ? 1.0f / total0 : 0.f, f1 = in1 ? 1.0f / total1 : 0.f;

@@ -93,6 +93,8 @@ def test_grid_forward_against_oracle_chain(ops, lo, hi, K, cutoff, minimum, leng
     close(out, ref, out0, slice(None), "all rows")
     # float32 logarithms of sums: a few units in the last place of either, and of the largest logit
     assert np.abs(lse.cpu().numpy() - ref_lse).max() < 1e-6 * max(1.0, np.abs(ref_lse).max()) + 1.5e-6
+    # ... and on average no more than 2^-24 of a sum, half a unit in its last place, beyond twice the enumerating kernel's
+    assert np.abs(lse.cpu().numpy() - ref_lse).mean() < 2 * np.abs(lse0.cpu().numpy() - ref_lse).mean() + 2.0 ** -24
     if K:  # 64 sums per (row, head), each within a few units of the row's largest
         assert float((psi - psi0).abs().max() / psi0.abs().max()) < 2e-6
     repeat = again()
