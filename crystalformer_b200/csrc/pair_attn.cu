@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     float *tables = reinterpret_cast<float *>(smem + L::TABLES), *sums = tables + PG_ROWS * row_words;
     __shared__ float e_unit[PG_ROWS][HEADS], tops[PG_ROWS][HEADS];  // one of E as stored, over Z; largest logits
     __shared__ int row_tiles[PG_ROWS];  // node tiles of a row; 0: it is not there or left over
+    __shared__ unsigned odd[PG_ROWS];   // 1: a row's result is not finite
     grid_launch_dependents();
     grid_dependency_wait();  // q, k, v, a
     const int4 tile = p.tiles[2 * blockIdx.x], place = p.tiles[2 * blockIdx.x + 1];
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     good = good && __all_sync(FULL, z.x > 1e-30f && z.x < 1e30f && z.y > 1e-30f && z.y < 1e30f);
     if (t == 0) tops[warp][g] = top;
     if (lane == 0) {
+        odd[warp] = 0u;
         row_tiles[warp] = good ? tiles : 0;
         if (p.stats != nullptr && good) {
             atomicAdd(p.stats + 2, 1ull);
@@ -468,6 +470,14 @@ __global__ void __launch_bounds__(Layout<TAIL, STAGES>::THREADS, 2) pair_attn_ke
     float *o = p.out + (a0 + i0 + 2 * t) * (HEADS * HEAD_DIM) + h * HEAD_DIM + g;
     if (in0) { o[0] = val[0]; o[8] = val[2]; }
     if (in1) { o[128] = val[1]; o[136] = val[3]; }
+    // An operand in pieces turns an infinity (of a value or of W) into a NaN: such rows are the row kernel's, whose products keep it.
+    auto look = [&](bool in, int r, float sum) {
+        if (!in || sum < INFINITY || atomicExch(odd + r, 1u) != 0u) return;
+        p.leftover[atomicAdd(p.left_count, 1u)] = (int)(a0 + i0 + r);
+        if (p.left != nullptr) p.left[a0 + i0 + r] = 1;
+    };
+    look(in0, 2 * t, fabsf(val[0]) + fabsf(val[2]));
+    look(in1, 2 * t + 1, fabsf(val[1]) + fabsf(val[3]));
 }
 
 template <int TAIL, int STAGES>

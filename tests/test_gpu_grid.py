@@ -265,3 +265,21 @@ def test_heads_far_below_the_others_keep_their_bits(ops):
     ref, _ = reference(cb, x, 64, -3.5, 2)
     close(out[:, 0], ref[:, 0], out0[:, 0], slice(None), "the head below")
     close(out, ref, out0, slice(None), "all heads")
+
+
+@pytest.mark.parametrize("K", [64, 0])
+def test_infinities_stay_infinities(ops, K):
+    """An infinity in a value, or in the value encoding's projection: the rows that meet it are the enumerating kernel's, infinite with its
+    sign, and marked as left over."""
+    cb = make_crystals(51, 5, uniform_atoms(4, 18), length_range=(4.0, 9.0))
+    starts = np.concatenate([[0], np.cumsum(cb.sizes)])
+    x = inputs(cb, (1.2, 1.5))
+    x[2][starts[0] + 1, 2, 3] = np.inf
+    x[2][starts[2] + 1, 7, 0] = -np.inf
+    if K:
+        x[4][4, 5, 9] = np.inf
+    (out, _, _, _, left), (out0, *_), _ = run(ops, cb, x, K)
+    assert torch.isinf(out0).any()
+    for of in (torch.isposinf, torch.isneginf, torch.isnan):
+        assert torch.equal(of(out), of(out0))
+    assert bool(left[~torch.isfinite(out).flatten(1).all(dim=1)].all())
