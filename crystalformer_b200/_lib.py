@@ -111,7 +111,8 @@ class TrainDesc(ctypes.Structure):
 class TrainBatch(ctypes.Structure):
     """``cf_train_batch``: a batch and the memory its step keeps between forward and backward."""
     _fields_ = [("features", c_void_p), ("pos", c_void_p), ("trans", c_void_p), ("sizes", c_void_p), ("N", c_int64), ("B", c_int64),
-                ("E", c_int64), ("max_atoms", c_int64), ("saved", c_void_p), ("saved_edges", c_void_p)]
+                ("E", c_int64), ("max_atoms", c_int64), ("saved", c_void_p), ("saved_edges", c_void_p),
+                ("floor_log2", c_double)]
 
 
 class ServeSlot(ctypes.Structure):

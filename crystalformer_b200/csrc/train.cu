@@ -403,25 +403,26 @@ int check_batch(const cf_train_batch *b, const char *who, Half half)
 // Weights of layer l: Wq Wk Wv b_in w_pos Wpe Wo bo W1 b1 W2 b2; after the layers: W_embed, the head's W1 b1 W2 b2.
 enum { W_Q, W_K, W_V, B_IN, W_POS, W_PE, W_O, B_O, W_1, B_1, W_2, B_2, PER_LAYER };
 
-bool lists_of(const cf_train_desc &d, const Saved &s, int64_t N, int64_t E, TermList &list, float &a_widest)
+bool lists_of(const cf_train_desc &d, const cf_train_batch &b, const Saved &s, TermList &list, float &a_widest)
 {
     a_widest = -INFINITY;
     for (int l = 0; l < d.num_layers; ++l)
         if (domain_of(d, l) == REAL) a_widest = fmaxf(a_widest, (float)(d.scalars[SCALARS * l + 4] * d.scalars[SCALARS * l + 2]));
-    if (s.lists == nullptr || !(weight_floor_log2() > -200.0f) || !(a_widest < 0.0f)) return false;
+    const float floor = (float)b.floor_log2;
+    if (s.lists == nullptr || !(floor > -200.0f) || !(a_widest < 0.0f)) return false;
     int *start, *count;
     float *dmin;
     unsigned long long *cursor;
     float2 *pool;
-    term_list_carve(s.lists, N, E, &start, &count, &dmin, &cursor, &pool);
+    term_list_carve(s.lists, b.N, b.E, &start, &count, &dmin, &cursor, &pool);
     list.pool = pool; list.start = start; list.count = count; list.dmin = dmin;
-    list.window = term_window(weight_floor_log2(), a_widest);
+    list.window = term_window(floor, a_widest);
     return true;
 }
 
 // Whether a batch's layers of domain real go by pair grids, and what their calls share.  Both halves of a step decide alike, from the
-// description and the sizes only (not from the process-wide floor, which may change in between: nodes in reach are chosen for
-// 2^-40 at least where terms are to be kept below 2^-30).
+// description, the sizes and the floor that the forward left in the batch (the process-wide one may change in between).  Nodes in
+// reach are chosen for 2^-30, or for 2^-40 where terms are to be kept below 2^-30; a floor below that is not for nodes.
 bool grid_of(const cf_train_desc &d, const cf_train_batch &b, const Saved &w, PairAttn &p, float &a_widest)
 {
     a_widest = -INFINITY;
@@ -434,8 +435,8 @@ bool grid_of(const cf_train_desc &d, const cf_train_batch &b, const Saved &w, Pa
         a_widest = fmaxf(a_widest, (float)(d.scalars[SCALARS * l + 4] * d.scalars[SCALARS * l + 2]));
     }
     if (w.grid == nullptr || d.num_layers > PG_LAYERS || !pair_grid_pays_training(b.N, b.B, b.E, b.max_atoms, d.K)) return false;
-    const float floor = weight_floor_log2();
-    if (!pair_grid_params(d.K, dist_max, d.wscale, a_widest, -30.0f, p.par)) return false;
+    const float floor = (float)b.floor_log2;
+    if (!(floor >= -40.0f) || !pair_grid_params(d.K, dist_max, d.wscale, a_widest, -30.0f, p.par)) return false;
     p.par.floor_log2 = floor < -30.0f ? -40.0f : -30.0f;
     p.rvlen = d.cutoff_radius != 0.0 ? w.rvlen : nullptr;
     p.atom_start = w.atom_start; p.edge_start = w.edge_start; p.N = b.N; p.B = b.B; p.E = b.E; p.K = d.K; p.max_atoms = (int)b.max_atoms;
@@ -571,13 +572,14 @@ extern "C" int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *b
     return read_sizes_beside(batch->sizes, batch->B, counts, as_stream(stream), train_begin_launch, &arg, begun_event);
 }
 
-extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *begun_event, float *y, void *stream)
+extern "C" int cf_train_forward(const cf_train_desc *desc, cf_train_batch *batch, void *begun_event, float *y, void *stream)
 {
     using namespace cf;
     int rc = check_desc(desc, "cf_train_forward");
     if (rc == CF_OK) rc = check_batch(batch, "cf_train_forward", FORWARD);
     if (rc != CF_OK) return rc;
     CF_REQUIRE(y && begun_event, CF_ERR_INVALID, "cf_train_forward: null pointer");
+    batch->floor_log2 = weight_floor_log2();
     const cf_train_desc &d = *desc;
     const cf_train_batch &b = *batch;
     const int64_t N = b.N, B = b.B, E = b.E;
@@ -601,7 +603,7 @@ extern "C" int cf_train_forward(const cf_train_desc *desc, const cf_train_batch 
     PairAttn by_grid{};
     float a_widest;
     const bool gridded = grid_of(d, b, w, by_grid, a_widest);
-    const bool listed = !gridded && lists_of(d, w, N, E, list, a_widest);
+    const bool listed = !gridded && lists_of(d, b, w, list, a_widest);
     if (gridded) {
         rc = launch_pair_grid_build(by_grid, w.pos_ij, b.trans, a_widest, nullptr, 0, 0, s);
         if (rc != CF_OK) return rc;
@@ -689,7 +691,7 @@ extern "C" int cf_train_backward(const cf_train_desc *desc, const cf_train_batch
     PairAttn by_grid{};
     float a_widest;
     const bool gridded = grid_of(d, b, w, by_grid, a_widest);
-    const bool listed = !gridded && lists_of(d, w, N, E, list, a_widest);
+    const bool listed = !gridded && lists_of(d, b, w, list, a_widest);
 
     head_backward_kernel<<<(unsigned)B, 128, 0, s>>>(gy, w.hid, tail_weights[1], tail_weights[3], w.atom_start, hidden, targets, g.ghid, g.gx[L]);
     head_weight_grad_kernel<<<dim3((hidden + 31) / 32, targets), 256, 0, s>>>(gy, w.hid, B, hidden, targets, tail_grads[3], tail_grads[4]);

@@ -195,13 +195,13 @@ class TrainStep(torch.autograd.Function):
                 raise
         # (no address is kept: what saved-tensor hooks give back in the backward may lie elsewhere, or be a recomputation)
         ctx.save_for_backward(saved, edges, feats, trans)
-        ctx.step = (plan, (N, B, batch.E, batch.max_atoms), plan.versions())
+        ctx.step = (plan, (N, B, batch.E, batch.max_atoms), batch.floor_log2, plan.versions())
         return y
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, gy):
-        plan, (N, B, E, max_atoms), versions = ctx.step
+        plan, (N, B, E, max_atoms), floor, versions = ctx.step
         saved, edges, feats, trans = ctx.saved_tensors
         if plan.versions() != versions:
             raise RuntimeError("a parameter of the model was modified by an in-place operation between the forward and the "
@@ -209,7 +209,7 @@ class TrainStep(torch.autograd.Function):
         dev = gy.device
         gy = gy.contiguous()
         desc = plan.desc
-        batch = _lib.TrainBatch(feats.data_ptr(), None, trans.data_ptr(), None, N, B, E, max_atoms, saved.data_ptr(), edges.data_ptr())
+        batch = _lib.TrainBatch(feats.data_ptr(), None, trans.data_ptr(), None, N, B, E, max_atoms, saved.data_ptr(), edges.data_ptr(), floor)
         scratch = torch.empty(int(_lib.load().cf_train_scratch_bytes(ctypes.byref(desc), N, B, E)), dtype=torch.uint8, device=dev)
         flat = torch.empty(plan.floats, dtype=torch.float32, device=dev)
         where = plan.offsets + flat.data_ptr() * plan.present

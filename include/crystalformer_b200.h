@@ -497,10 +497,12 @@ int cf_begin_abandon(void *begun_event, void *stream);
  *   cf_train_batch : the inputs of cf_model_forward and 256-byte aligned device memory that the forward fills and the
  *                    backward reads: `saved`, cf_train_saved_bytes(desc, N, B) bytes, and `saved_edges`,
  *                    cf_train_edge_bytes(desc, N, B, E) bytes (E = sum n^2 >= 1, largest crystal max_atoms <= 1024).
+ *                    floor_log2 is written by cf_train_forward: the weight floor in force then (cf_set_weight_floor_log2),
+ *                    by which both halves of the step choose their kernels; cf_train_backward is given it back.
  * cf_train_begin needs N, B and `saved` only: it queues the read-back of the sizes, packs the weights and runs the first
  * dense block, and returns counts and begun_event as cf_model_begin does; cf_train_forward then writes y (B, targets).
- * cf_train_backward (of the batch: features, trans, the sizes N, B, E, max_atoms and the two blocks of memory, which hold no
- * addresses and may have been copied elsewhere since) takes gy (B, targets), scratch of cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of
+ * cf_train_backward (of the batch: features, trans, the sizes N, B, E, max_atoms, floor_log2 and the two blocks of memory, which
+ * hold no addresses and may have been copied elsewhere since) takes gy (B, targets), scratch of cf_train_scratch_bytes(desc, N, B, E) bytes and a HOST array of
  * device pointers to the gradients, in the order of the weights (the entry of a NULL weight is not used); every gradient
  * is written, none accumulated.  The weights must not change between the calls.
  * ---------------------------------------------------------------------------------------------------------- */
@@ -516,12 +518,13 @@ typedef struct cf_train_batch {
     const int64_t *sizes;
     int64_t N, B, E, max_atoms;
     void *saved, *saved_edges;
+    double floor_log2;
 } cf_train_batch;
 int64_t cf_train_saved_bytes(const cf_train_desc *desc, int64_t N, int64_t B);
 int64_t cf_train_edge_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
 int64_t cf_train_scratch_bytes(const cf_train_desc *desc, int64_t N, int64_t B, int64_t E);
 int cf_train_begin(const cf_train_desc *desc, const cf_train_batch *batch, int64_t *counts, void **begun_event, void *stream);
-int cf_train_forward(const cf_train_desc *desc, const cf_train_batch *batch, void *begun_event, float *y, void *stream);
+int cf_train_forward(const cf_train_desc *desc, cf_train_batch *batch, void *begun_event, float *y, void *stream);
 int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, const float *gy, void *scratch,
                       float *const *grads, void *stream);
 

@@ -290,3 +290,37 @@ def test_directional_derivatives_are_not_dropped():
         data.x = fwad.make_dual(data.x, torch.ones_like(data.x))
         with pytest.raises((RuntimeError, NotImplementedError)):
             model(data)
+
+
+@pytest.mark.parametrize("sizes", [[12] * 80, [9, 20, 5]])
+def test_the_weight_floor_of_a_step(sizes):
+    """A floor that nodes cannot serve (-1000: every term) keeps a step off the pair grids, and a floor that changes between the halves
+    of a step does not change the way that its second half takes (80 crystals: grids, three: term lists)."""
+    from crystalformer_b200 import ops
+    model, data, target = setup(sizes, lengths=(4.0, 9.0), num_layers=2)
+    rows = torch.zeros(4, dtype=torch.int64, device="cuda")
+
+    def gradients(first, second):
+        rows.zero_()
+        ops.set_row_stats(rows)
+        try:
+            ops.set_weight_floor_log2(first)
+            for p in model.parameters():
+                p.grad = None
+            loss = (model(data) - target).abs().mean()
+            ops.set_weight_floor_log2(second)
+            loss.backward()
+        finally:
+            ops.set_weight_floor_log2(-30.0)
+            ops.set_row_stats(None)
+        return {n: p.grad for n, p in model.named_parameters() if p.requires_grad}, int(rows[2])
+
+    usual, by_grid = gradients(-30.0, -30.0)
+    whole, enumerated = gradients(-1000.0, -1000.0)
+    assert model._train_plan is not None
+    assert enumerated == 0 and (by_grid > 0) == (len(sizes) > 3)
+    noise = 1e-6 * max(float(g.norm()) for g in whole.values())
+    for halves, ref in (((-30.0, -1000.0), usual), ((-1000.0, -30.0), whole), ((-40.0, -30.0), usual)):
+        got, _ = gradients(*halves)
+        for n in ref:  # (as between two kernels: a hidden unit within rounding of zero)
+            assert (got[n] - ref[n]).norm() <= 2e-3 * ref[n].norm() + noise, (halves, n)
