@@ -249,9 +249,12 @@ extern "C" int64_t cf_encoder_workspace_floats(int64_t N, int64_t E, int64_t ff_
     // then the term lists: directory (2 ints per edge), allocation cursor, pool (2 floats per entry)
     // (or, for batches of small crystals, the row lists: whichever is larger)
     const size_t lists = cf::term_list_workspace_bytes(N, E), rows = cf::row_list_workspace_bytes(N, E);
-    return N * (384 + 384 + 128 + 8 + 8 + ff_dim) + E * 8 + 64 + (int64_t)((lists > rows ? lists : rows) + 3) / 4 +
+    return N * (912 + ff_dim) + E * 8 + 64 + (int64_t)((lists > rows ? lists : rows) + 3) / 4 +
            (int64_t)cf::row_blocks_words(N) + 64;
 }
+
+// Where a forward's logits and lists begin, in bytes: a batch with pair grids has neither, so the grids may lie there.
+size_t cf::encoder_lists_at(int64_t N, int64_t ff_dim) { return (sizeof(float) * (size_t)(N * (912 + ff_dim)) + 255) & ~(size_t)255; }
 
 extern "C" int cf_encoder_forward(void *cublas_handle, int num_layers, const float *const *weights, const double *scalars,
                                   float *x, const float *pos_ij, const float *tvecs, const float *rvlen,
@@ -331,7 +334,7 @@ int cf::encoder_forward_impl(void *cublas_handle, int num_layers, const float *c
                 by_grid.atom_start = grid_memory->atom_start; by_grid.edge_start = grid_memory->edge_start;
                 by_grid.N = N; by_grid.B = B; by_grid.E = E; by_grid.K = K; by_grid.max_atoms = (int)max_atoms; by_grid.rule = rule;
                 by_grid.dist_max = scalars[5]; by_grid.wscale = wscale; by_grid.call = 0;
-                by_grid.grid = pair_grid_carve(grid_memory->memory, N, B, E);
+                by_grid.grid = pair_grid_carve(grid_memory->memory, N, B, E, K);
                 by_grid.leftover = by_grid.grid.leftover;
                 by_grid.projected = K > 0;
                 // (early: ordered after the inputs only, so the weights are read on this stream)

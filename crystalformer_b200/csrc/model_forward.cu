@@ -83,7 +83,7 @@ struct Scratch {
     int64_t *atom_start, *edge_start, *batch, *row_start, *edges;
     float *pos_ij, *rvlen, *x, *encoder;
     int32_t *row_order;
-    char *grid;  // pair grids
+    char *grid;  // pair grids, in the place of the encoder's logits and lists
     size_t bytes;
 };
 
@@ -100,8 +100,12 @@ Scratch carve(void *workspace, int64_t N, int64_t B, int64_t E, int64_t ff_dim)
     s.rvlen = c.take<float>(3 * B);
     s.row_order = c.take<int32_t>(N);
     s.x = c.take<float>(N * MODEL_DIM);
-    s.encoder = c.take<float>((size_t)cf_encoder_workspace_floats(N, E, ff_dim));
-    s.grid = c.take<char>(pair_grid_reserve(N, B, E));
+    // (K is not among the sizes: room for grids with a basis)
+    const size_t at = encoder_lists_at(N, ff_dim), lists = sizeof(float) * (size_t)cf_encoder_workspace_floats(N, E, ff_dim);
+    const size_t grids = at + pair_grid_reserve(N, B, E, 64);
+    char *encoder = c.take<char>(lists > grids ? lists : grids);
+    s.encoder = reinterpret_cast<float *>(encoder);
+    s.grid = encoder != nullptr ? encoder + at : nullptr;
     s.bytes = c.used;
     return s;
 }

@@ -552,7 +552,7 @@ int grid_call(PairAttn &p, const char *who, const float *rvlen, const int64_t *a
     CF_REQUIRE(max_atoms >= 1 && max_atoms <= PG_MAX_ATOMS, CF_ERR_RANGE, "%s: max_atoms=%lld outside [1,%d]", who, (long long)max_atoms, PG_MAX_ATOMS);
     if (N == 0) return CF_OK;
     CF_REQUIRE(atom_start && edge_start && grids && (rvlen || cutoff_radius == 0), CF_ERR_INVALID, "%s: null pointer", who);
-    CF_REQUIRE(pair_grid_fits(N, B, E, max_atoms), CF_ERR_RANGE, "%s: %lld edges are more than grids are kept for", who, (long long)E);
+    CF_REQUIRE(pair_grid_fits(N, B, E, max_atoms, 64), CF_ERR_RANGE, "%s: %lld edges are more than grids are kept for", who, (long long)E);
     CF_REQUIRE(pair_grid_params(K, dist_max, wscale, (float)a_widest, weight_floor_log2(), p.par), CF_ERR_UNSUPPORTED,
                "%s: the nodes do not cover Gaussians of a_widest=%g (dist_max=%g, wscale=%g, floor 2^%g)", who, a_widest, dist_max, wscale,
                (double)weight_floor_log2());
@@ -560,7 +560,7 @@ int grid_call(PairAttn &p, const char *who, const float *rvlen, const int64_t *a
     p.atom_start = atom_start; p.edge_start = edge_start; p.N = N; p.B = B; p.E = E; p.K = K; p.max_atoms = (int)max_atoms;
     p.rule = BoxRule{(float)cutoff_radius, lattice_range, minimum_range};
     p.dist_max = dist_max; p.wscale = wscale;
-    p.grid = pair_grid_carve(grids, N, B, E);
+    p.grid = pair_grid_carve(grids, N, B, E, K);
     p.leftover = p.grid.leftover;
     return CF_OK;
 }
@@ -583,7 +583,7 @@ __global__ void list_left_kernel(const unsigned char *__restrict__ left, long lo
 extern "C" int64_t cf_pair_grid_bytes(int64_t N, int64_t B, int64_t E)
 {
     if (N <= 0 || B <= 0 || E < 0) return 0;
-    const size_t bytes = cf::pair_grid_bytes(N, B, E);
+    const size_t bytes = cf::pair_grid_bytes(N, B, E, 64);  // (for any K)
     return bytes <= cf::PG_MAX_BYTES ? (int64_t)bytes : 0;
 }
 

@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(32 * BUILD_WARPS, BUILD_BLOCKS) pair_grid_kern
 
 long long extra_slots(long long pairs) { return pairs / 2 + 8192; }
 
-PairGrid carve(Carver &c, long long N, long long B, long long E)
+PairGrid carve(Carver &c, long long N, long long B, long long E, long long K)
 {
     PairGrid g{};
     const long long pairs = (E + N) / 2;
@@ -454,23 +454,23 @@ PairGrid carve(Carver &c, long long N, long long B, long long E)
     g.basis_nodes = reinterpret_cast<uint4 *>(c.take<unsigned>(PG_BASIS_WORDS));
     g.projected = c.take<uint4>((size_t)PG_LAYERS * HEADS * PG_TILES_BASIS * 64);
     g.projected_scale = c.take<float>((size_t)PG_LAYERS * HEADS);
-    g.slots = c.take<unsigned char>((size_t)g.slot_count * 64 * PG_TILES_BASIS);
+    g.slots = c.take<unsigned char>((size_t)g.slot_count * pg_slot_bytes(K));
     return g;
 }
 
 }  // namespace
 
-size_t pair_grid_bytes(long long N, long long B, long long E)
+size_t pair_grid_bytes(long long N, long long B, long long E, long long K)
 {
     Carver c{nullptr};
-    carve(c, N, B, E);
+    carve(c, N, B, E, K);
     return c.used;
 }
 
-PairGrid pair_grid_carve(void *memory, long long N, long long B, long long E)
+PairGrid pair_grid_carve(void *memory, long long N, long long B, long long E, long long K)
 {
     Carver c{static_cast<char *>(memory)};
-    return carve(c, N, B, E);
+    return carve(c, N, B, E, K);
 }
 
 // Whether vectors of these nodes serve the model: their range must cover an ordinary Gaussian (twice as narrow in variance as the

@@ -38,7 +38,11 @@ constexpr int PG_ROWS = 8;                   // rows of a crystal that a block o
 constexpr int PG_ALL_BOXES = 1 << 24;         // in PairGrid::info: the variants are all the boxes up to the widest Gaussian's
 constexpr int PG_MAX_ATOMS = 64;             // (tables of eight rows in shared memory, two blocks per SM)
 constexpr int PG_LAYERS = 32;                // calls per batch that find zeroed counters
-constexpr size_t PG_MAX_BYTES = 24ull << 30;
+// Grids lie where the batch would have its lists, and with a basis take more: 528 bytes per edge, lists and logits 300 (without one
+// 240).  1,024 crystals of up to 60 atoms have a workspace of 923 MB for it, 649 MB with lists alone.  Beyond 16 M edges (thirteen
+// times those crystals) a batch keeps its lists, so that no workspace is more than 4 GB larger for the grids.
+constexpr size_t PG_MAX_BYTES = 8ull << 30;
+constexpr long long PG_LEAST_EDGES = 5000, PG_LEAST_ROWS = 640;  // no smaller batch, no smaller training step goes this way
 
 __host__ __device__ inline int pg_tiles(long long K) { return K > 0 ? PG_TILES_BASIS : PG_TILES_PLAIN; }
 __host__ __device__ inline int pg_slot_bytes(long long K) { return 64 * pg_tiles(K); }
@@ -68,6 +72,7 @@ struct GridMemory {
     void *memory;
     const int64_t *atom_start, *edge_start;
 };
+size_t encoder_lists_at(int64_t N, int64_t ff_dim);  // (encoder_forward.cu)
 struct PairGridParams {
     int tiles;                   // node tiles of a vector
     float inv_h2, inv_h2_low;    // 1 / h^2 in two floats
@@ -78,20 +83,24 @@ struct PairGridParams {
 };
 
 // Bytes for a batch, and whether a batch can go this way at all.
-size_t pair_grid_bytes(long long N, long long B, long long E);
-PairGrid pair_grid_carve(void *memory, long long N, long long B, long long E);
+size_t pair_grid_bytes(long long N, long long B, long long E, long long K);
+PairGrid pair_grid_carve(void *memory, long long N, long long B, long long E, long long K);
 bool pair_grid_params(long long K, double dist_max, double wscale, float a_widest, float floor_log2, PairGridParams &out);
-inline bool pair_grid_fits(long long N, long long B, long long E, long long max_atoms)
+inline bool pair_grid_fits(long long N, long long B, long long E, long long max_atoms, long long K)
 {
-    return N > 0 && N < (1ll << 28) && max_atoms <= PG_MAX_ATOMS && E <= PG_MAX_ATOMS * N && pair_grid_bytes(N, B, E) <= PG_MAX_BYTES;
+    return N > 0 && N < (1ll << 28) && max_atoms <= PG_MAX_ATOMS && E <= PG_MAX_ATOMS * N && pair_grid_bytes(N, B, E, K) <= PG_MAX_BYTES;
 }
 // What memory for batches of up to N atoms, B crystals and E edges holds for grids: those of any such batch, whether they are this
 // one's or not (a batch that fits has at most 64 edges per atom), so that a workspace grows with each of its sizes.
-inline size_t pair_grid_reserve(long long N, long long B, long long E)
+inline size_t pair_grid_reserve(long long N, long long B, long long E, long long K)
 {
-    if (N <= 0) return 0;
-    const size_t most = pair_grid_bytes(N, B, E < PG_MAX_ATOMS * N ? E : PG_MAX_ATOMS * N);
+    if (N <= 0 || E < PG_LEAST_EDGES) return 0;
+    const size_t most = pair_grid_bytes(N, B, E < PG_MAX_ATOMS * N ? E : PG_MAX_ATOMS * N, K);
     return most < PG_MAX_BYTES ? most : PG_MAX_BYTES;
+}
+inline size_t pair_grid_reserve_training(long long N, long long B, long long E, long long K)
+{
+    return N < PG_LEAST_ROWS ? 0 : pair_grid_reserve(N, B, E > PG_LEAST_EDGES ? E : PG_LEAST_EDGES, K);
 }
 // Whether an inference batch gains by them.  The plan, the vectors and a block's fixed work (a row's Gaussians at the nodes, whatever
 // its keys) want enough pairs and enough keys per row.  Times by row lists (without a basis: term lists), then over grids:
@@ -105,8 +114,8 @@ inline size_t pair_grid_reserve(long long N, long long B, long long E)
 // One line for all, so that a batch has the same bits however it is issued.
 inline bool pair_grid_pays(long long N, long long B, long long E, long long max_atoms, long long K)
 {
-    if (!pair_grid_fits(N, B, E, max_atoms)) return false;
-    return K > 0 ? (E >= 5000 && E >= 16 * N) || (E >= 30000 && E >= 11 * N) : E >= 20000 && E >= 11 * N;
+    if (!pair_grid_fits(N, B, E, max_atoms, K)) return false;
+    return K > 0 ? (E >= PG_LEAST_EDGES && E >= 16 * N) || (E >= 30000 && E >= 11 * N) : E >= 20000 && E >= 11 * N;
 }
 
 // ... and whether a training step does: device time of a step (four layers), term lists against grids.  With a basis what it saves
@@ -116,7 +125,7 @@ inline bool pair_grid_pays(long long N, long long B, long long E, long long max_
 // rows of 8 keys 576 against 584.
 inline bool pair_grid_pays_training(long long N, long long B, long long E, long long max_atoms, long long K)
 {
-    return pair_grid_fits(N, B, E, max_atoms) && (K > 0 ? N >= 640 && E >= 5 * N : N >= 960 && E >= 11 * N);
+    return pair_grid_fits(N, B, E, max_atoms, K) && (K > 0 ? N >= PG_LEAST_ROWS && E >= 5 * N : N >= 960 && E >= 11 * N);
 }
 
 // One attention call over a batch's grids, and its backward.

@@ -306,8 +306,8 @@ Saved carve_saved(const cf_train_desc &d, void *memory, void *edge_memory, int64
     }
     s.kr = split ? e.take<float>(3 * E) : nullptr;
     s.phi_reci = split ? e.take<float>(E * HEADS) : nullptr;
-    s.lists = fused ? e.take<char>(term_list_workspace_bytes(N, E)) : nullptr;
-    s.grid = fused ? e.take<char>(pair_grid_reserve(N, B, E)) : nullptr;
+    const size_t lists = term_list_workspace_bytes(N, E), grid = pair_grid_reserve_training(N, B, E, d.K);
+    s.lists = s.grid = fused ? e.take<char>(lists > grid ? lists : grid) : nullptr;  // (a step has one or the other)
     s.edge_bytes = e.used;
     return s;
 }
@@ -338,7 +338,7 @@ Scratch carve_scratch(const cf_train_desc &d, void *memory, int64_t N, int64_t B
     }
     s.gx[d.num_layers] = c.take<float>(N * CH);
     s.glogit = c.take<float>(E * HEADS);
-    s.prob = c.take<float>(E * HEADS);
+    s.prob = N >= PG_LEAST_ROWS ? c.take<float>(E * HEADS) : nullptr;
     bool split = false, values = false;
     for (int l = 0; l < d.num_layers; ++l) {
         split = split || domain_of(d, l) != REAL;
@@ -442,7 +442,7 @@ bool grid_of(const cf_train_desc &d, const cf_train_batch &b, const Saved &w, Pa
     p.atom_start = w.atom_start; p.edge_start = w.edge_start; p.N = b.N; p.B = b.B; p.E = b.E; p.K = d.K; p.max_atoms = (int)b.max_atoms;
     p.rule = BoxRule{(float)d.cutoff_radius, d.lattice_range, d.minimum_range};
     p.dist_max = dist_max; p.wscale = d.wscale;
-    p.grid = pair_grid_carve(w.grid, b.N, b.B, b.E);
+    p.grid = pair_grid_carve(w.grid, b.N, b.B, b.E, d.K);
     return true;
 }
 // ... and one layer's

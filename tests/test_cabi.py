@@ -110,3 +110,14 @@ def test_workspace_of_the_maxima_holds_every_batch_below_them(lib):
         outer = [int(v * f) for v, f in zip((n, b, e), rng.choice([1.0, 1.01, 1.25, 4.0], 3))]
         assert size(n, b, e) <= size(*outer), ((n, b, e), outer)
         assert size(n, b, min(e, 64 * n)) <= size(*outer), ((n, b, e), outer)
+
+
+def test_pair_grids_lie_in_the_memory_of_the_lists(lib):
+    """A batch has term lists or grids: together they take the larger one's memory, and grids are not kept for batches that never
+    have them (fewer than 5,000 pairs)."""
+    grid = lambda n, b, e: int(lib.cf_pair_grid_bytes(n, b, e))
+    lists = lambda n, e: max(int(lib.cf_term_list_workspace_bytes(n, e)), int(lib.cf_row_list_workspace_bytes(n, e)))
+    for n, b, e in ((32000, 1024, 1270000), (500000, 16000, 20000000), (9600, 64, 1500000), (2000, 128, 41000), (100, 10, 1000)):
+        rest = int(lib.cf_encoder_workspace_floats(n, e, 512)) * 4 - lists(n, e) + n * 1024 + 28 * e + 100 * b + 16384
+        most = max(lists(n, e), (grid(n, b, min(e, 64 * n)) or 8 << 30) if e >= 5000 else 0)
+        assert int(lib.cf_model_workspace_bytes(n, b, e, 512)) <= rest + most, (n, b, e)
