@@ -866,8 +866,9 @@ int launch_rows(const RowArgs &p, int64_t K, long long grid_rows, cudaStream_t s
     return launch_status("cf_infinite_attn_fwd");
 }
 
-// The rows that the sorted row kernel (infinite_attn_sorted.cu) or the kernel over pair grids (pair_attn.cu) left over: atoms rows[0 .. *count), processed by the
-// row kernel above without lists (phi and the candidates by enumeration).  `ticket` must be zero on entry.
+// The rows that the sorted row kernel (infinite_attn_sorted.cu) or the kernel over pair grids (pair_attn.cu) left over: atoms
+// rows[0 .. *count), processed by the row kernel above without lists (phi and the candidates by enumeration).  `ticket` must be zero
+// on entry.
 int launch_leftover_rows(const float *q, const float *k, const float *v, const float *a, const float *pos_ij,
                          const float *tvecs, const float *rvlen, const int64_t *batch, const int64_t *edges,
                          const int64_t *row_start, int64_t N, int64_t E, int64_t max_atoms, double dist_max,

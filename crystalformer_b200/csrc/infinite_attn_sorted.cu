@@ -29,6 +29,7 @@
 #include <cuda_fp16.h>
 
 #include "lattice_core.cuh"
+#include "mma_frag.cuh"
 #include "row_list.cuh"
 
 namespace cf {
@@ -62,14 +63,6 @@ struct SortedRowArgs {
     unsigned long long *stats;  // optional: { chunks swept, (chunk, bin tile) pairs computed, rows } are added here
 };
 
-// A k-step is 16 entries (two chunks): m16n8k16 with half operands.
-__device__ __forceinline__ void mma_half(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1)
-{
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // Values of [0, 1] as two halves each, a pair of terms per register: x = hi + lo up to one unit of x's 24 bits, with a floor of
 // 2^-25 of the largest value, 2^-40 for the weights, which are scaled by 2^15 first (a row's sum may hold thousands of small
 // ones; the basis, whose values enter beside larger ones of the same term, is not).  The scale is a product and not part of
@@ -80,14 +73,6 @@ constexpr float HALF_SCALE = 32768.0f;
 // halves would show, and the row is left over.
 constexpr float MIN_SUM = 1.5e-5f;
 constexpr float UNSCALE = 1.0f / HALF_SCALE;
-__device__ __forceinline__ void split_halves(float x, float y, unsigned &hi, unsigned &lo)
-{
-    const __half2 h = __floats2half2_rn(x, y);
-    const float2 back = __half22float2(h);
-    const __half2 l = __floats2half2_rn(x - back.x, y - back.y);
-    hi = *reinterpret_cast<const unsigned *>(&h);
-    lo = *reinterpret_cast<const unsigned *>(&l);
-}
 // 1.0 in every half of `pair` that equals `value`: small integers as the bits of halves (subnormal numbers, compared exactly)
 __device__ __forceinline__ unsigned one_where_equal(unsigned pair, unsigned value)
 {
@@ -258,16 +243,16 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
             unsigned w_hi[2], w_lo[2];
             const float2 scale = make_float2(HALF_SCALE, HALF_SCALE);
             const float2 wa = __fmul2_rn(make_float2(w[0], w[1]), scale), wb = __fmul2_rn(make_float2(w[2], w[3]), scale);
-            split_halves(wa.x, wa.y, w_hi[0], w_lo[0]);
-            split_halves(wb.x, wb.y, w_hi[1], w_lo[1]);
+            split_f16(wa.x, wa.y, w_hi[0], w_lo[0]);
+            split_f16(wb.x, wb.y, w_hi[1], w_lo[1]);
             // P^T tiles: one-hot of the terms' keys (rows g, g + 8 of tile u are keys 16 u + g, 16 u + g + 8)
             const unsigned ja = ((unsigned)jv[0] | ((unsigned)jv[1] << 16)) ^ g_pair, jb = ((unsigned)jv[2] | ((unsigned)jv[3] << 16)) ^ g_pair;
 #pragma unroll
             for (int u = 0; u < NT; ++u) {
                 const unsigned o0 = one_where_equal(ja, 16 * u), o1 = one_where_equal(ja, 16 * u + 8);
                 const unsigned o2 = one_where_equal(jb, 16 * u), o3 = one_where_equal(jb, 16 * u + 8);
-                mma_half(accP[u], o0, o1, o2, o3, w_hi[0], w_hi[1]);
-                mma_half(accP[u], o0, o1, o2, o3, w_lo[0], w_lo[1]);
+                mma_f16(accP[u], o0, o1, o2, o3, w_hi[0], w_hi[1]);
+                mma_f16(accP[u], o0, o1, o2, o3, w_lo[0], w_lo[1]);
             }
             swept += two ? 2 : 1;
             if (PSI) {
@@ -291,13 +276,13 @@ __device__ __forceinline__ bool sorted_row(const SortedRowArgs &p, SortedSmem<NT
                     v1[e] = ex2(-c1 * c1);
                 }
                 unsigned hi[4], lo[4];
-                split_halves(v0[0], v0[1], hi[0], lo[0]);
-                split_halves(v1[0], v1[1], hi[1], lo[1]);
-                split_halves(v0[2], v0[3], hi[2], lo[2]);
-                split_halves(v1[2], v1[3], hi[3], lo[3]);
-                mma_half(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_hi[0], w_hi[1]);
-                mma_half(accPsi[m], lo[0], lo[1], lo[2], lo[3], w_hi[0], w_hi[1]);
-                mma_half(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_lo[0], w_lo[1]);
+                split_f16(v0[0], v0[1], hi[0], lo[0]);
+                split_f16(v1[0], v1[1], hi[1], lo[1]);
+                split_f16(v0[2], v0[3], hi[2], lo[2]);
+                split_f16(v1[2], v1[3], hi[3], lo[3]);
+                mma_f16(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_hi[0], w_hi[1]);
+                mma_f16(accPsi[m], lo[0], lo[1], lo[2], lo[3], w_hi[0], w_hi[1]);
+                mma_f16(accPsi[m], hi[0], hi[1], hi[2], hi[3], w_lo[0], w_lo[1]);
             }
             }
         }

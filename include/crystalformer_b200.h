@@ -558,8 +558,8 @@ int cf_train_backward(const cf_train_desc *desc, const cf_train_batch *batch, co
  *   cf_model_desc.dense_tile_rows : 0 = the dense blocks choose their row tile themselves (16 rows while that fills
  *                   one wave of SMs: shortest latency of a single forward); 32 = 32-row tiles (fewer, longer blocks
  *                   that read the weights half as often: more forwards per second when several streams keep the GPU
- *                   full); 16 = always 16.  With weight images the tile has 128 rows; small batches share it between
- *                   four blocks (shortest latency) unless the value is 32.
+ *                   full); 16 = always 16.  With weight images 32 means tiles of 128 rows, and any other value the
+ *                   fewest of 32, 64 and 128 rows that leave an SM for each tile.  Same outputs, bit for bit.
  * x_host .. sizes_host: HOST memory (pinned for the copies to be asynchronous) of the batch: one-hot species (N x
  * feature_dim), positions, lattice rows, atoms per crystal; E = sum of sizes^2, max_atoms = largest size.
  * ---------------------------------------------------------------------------------------------------------- */

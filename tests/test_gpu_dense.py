@@ -43,9 +43,9 @@ def test_one_call_forward_with_images_equals_the_gemm_path(ff, sizes):
 
 @pytest.mark.parametrize("ff", [128, 384, 512, 640])
 @pytest.mark.parametrize("atoms", [1, 33, 4737, 9600])
-def test_boundaries_shared_by_a_cluster_or_not(ff, atoms):
-    """A tile per cluster of four blocks (few tiles, at most four hidden chunks) and a tile per block: one row, rows of two of
-    the four blocks, more clusters than fit at once, more tiles than two waves of clusters; with and without blocks idle."""
+def test_boundaries_of_every_tile_height(ff, atoms):
+    """Tiles of 32 rows (one row; a tile and one row), of 64 (the first batch with more than 32 rows per SM) and of 128 (more than 64 per
+    SM); one to five chunks of hidden units."""
     from crystalformer_b200.model import Latticeformer, default_params
     torch.manual_seed(atoms + ff)
     model = Latticeformer(default_params(num_layers=2, ff_dim=ff)).cuda()
@@ -117,7 +117,7 @@ def test_tiles_of_32_64_and_128_rows(ff, rows):
 @pytest.mark.parametrize("ff", [128, 384, 512])
 @pytest.mark.parametrize("atoms", [1, 33, 200, 2000])
 def test_outputs_do_not_depend_on_how_a_batch_is_issued(ff, atoms):
-    """A forward whose tiles are shared by four blocks, and the serving pipeline on several streams, which keeps a block per tile."""
+    """A forward in tiles of 32 rows, and the serving pipeline on several streams, whose tiles have 128."""
     from crystalformer_b200.model import Latticeformer, default_params
     from crystalformer_b200.serving import PipelinedPredictor
     torch.manual_seed(atoms + ff)
