@@ -12,9 +12,9 @@
 //
 // Bound: issue and latency of a warp's chain (128 registers: 16 warps on an SM; 8 beyond 48 atoms, where the tables of one block
 // fill it); the vectors come from L2.  256 crystals of up to 40 atoms: 78 us per layer (112 with 8 warps on an SM, u apart from the
-// sums), 169 by term lists (infinite_attn_bwd.cu), whose work grows with the images.  Error against 64 bits on 24 crystals of up to
-// 30 atoms (gq, gk, gv, ga): 1.4, 1.4, 1.0, 1.8e-7, by lists 2.2, 2.1, 1.0, 2.4e-7; S0's small products add up apart from the large
-// ones (gv 1.04e-7 without).
+// sums), 169 by term lists (infinite_attn_bwd.cu), whose work grows with the images.  Issue slots 48 %, tensor
+// pipe 32 %, LSU wavefronts 38 %.  Error against 64 bits over 40 draws (gq, gk, gv, ga): 2.4, 2.4, 1.0, 3.3e-7, by enumeration 3.9, 3.8,
+// 1.1, 4.2e-7; S0's small products add up apart from the large ones (gv 1.04e-7 instead of 1.0 without, small logits).
 #include "pair_attn.cuh"
 
 namespace cf {
