@@ -104,7 +104,7 @@ int sm_count()
 
 extern "C" {
 
-int cf_version(void) { return 100; }
+int cf_version(void) { return 200; }
 
 int cf_check_waits(void) { return cf::check_waits("cf_check_waits"); }
 

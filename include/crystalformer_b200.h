@@ -53,7 +53,7 @@ extern "C" {
  * yields; here a box wider than this is clamped so that a degenerate width (a -> 0) cannot stall the GPU. */
 #define CF_MAX_RANGE 32
 
-/* Library version as major*10000 + minor*100 + patch. */
+/* Library version as major*10000 + minor*100 + patch.  0.2: cf_train_batch ends with floor_log2. */
 int cf_version(void);
 
 /* Message of the last error raised on the calling thread ("" if none). The pointer stays valid until the next

@@ -121,3 +121,31 @@ def test_pair_grids_lie_in_the_memory_of_the_lists(lib):
         rest = int(lib.cf_encoder_workspace_floats(n, e, 512)) * 4 - lists(n, e) + n * 1024 + 28 * e + 100 * b + 16384
         most = max(lists(n, e), (grid(n, b, min(e, 64 * n)) or 8 << 30) if e >= 5000 else 0)
         assert int(lib.cf_model_workspace_bytes(n, b, e, 512)) <= rest + most, (n, b, e)
+
+
+def test_memory_of_a_training_step_grows_with_its_sizes(lib):
+    """The edge memory of a step holds its lists or its grids, whichever it takes, and never shrinks with a size (640 rows, 5,000 edges and 64
+    edges per atom on both sides); without a basis the lists are the larger."""
+    from crystalformer_b200 import _lib
+    import numpy as np
+    weights, scalars = (ctypes.c_void_p * 29)(), (ctypes.c_double * 18)()
+
+    def desc(K):
+        return _lib.TrainDesc(num_layers=2, lattice_range=2, minimum_range=2, feature_dim=98, K=K, ff_dim=512, hidden=128, targets=1, wscale=1.0,
+                              weights=ctypes.cast(weights, ctypes.c_void_p), scalars=ctypes.cast(scalars, ctypes.c_void_p))
+
+    size = lambda K, n, b, e: int(lib.cf_train_edge_bytes(ctypes.byref(desc(K)), n, b, e))
+    lists = lambda n, e: int(lib.cf_term_list_workspace_bytes(n, e))
+    rest = lambda e: 2 * e * 32 + 28 * e
+    for n, b, e in ((5248, 256, 141696), (640, 20, 20480), (30000, 1000, 1200000)):
+        grid = int(lib.cf_pair_grid_bytes(n, b, e))
+        assert max(lists(n, e), grid) <= size(64, n, b, e) - rest(e) <= max(lists(n, e), grid) + 4096
+        assert size(0, n, b, e) - rest(e) <= lists(n, e) + 4096
+    rng = np.random.default_rng(2)
+    for _ in range(2000):
+        b = int(np.exp(rng.uniform(0, np.log(3000))))
+        n = b * int(rng.integers(1, 100))
+        e = int(n * rng.uniform(1, 100))
+        outer = [int(v * f) for v, f in zip((n, b, e), rng.choice([1.0, 1.01, 1.25, 4.0], 3))]
+        for K in (0, 64):
+            assert size(K, n, b, e) <= size(K, *outer) and size(K, n, b, min(e, 64 * n)) <= size(K, *outer), (K, (n, b, e), outer)
